@@ -17,8 +17,13 @@
 //               computes the next scores while the softmax warps work on the current ones
 //   warps 2..9  softmax: two threads per query row (64 score columns each), TMEM -> registers,
 //               pass 1: running max / sum of exp;  pass 2: p -> shared memory (the A operand)
-// V is consumed as V^T ([head][dim][key], keys contiguous): a K-major B operand that TMA can
-// load directly; the rotary kernels emit it (rowops.cu: *_qkv_post).
+// V is read as it lies in the qkv buffer or the KV cache ([key][dim]): the B operand of P.V is then MN-major (dims
+// contiguous), which tcgen05 takes from the same 128-byte-swizzled 64-dim blocks that K uses.  So nothing transposes V:
+// a segment may start at any token (keys are a TMA coordinate without an alignment rule) and a later portion of a prompt
+// reads the cached keys and values where they are.  (V^T, [head][dim][key], is still taken by b200_attention_fa.)
+// Measured against the kernel without TMA that such calls fell back to (attention_tc.cu): 2048 queries behind 2048 cached
+// keys, 28 heads of 128: 1094 -> 354 us; four pictures and a clip of four frames (6012 patches, 16 heads of 80), which start
+// at odd offsets: 773 us in eight launches -> 236 us in one.
 #include <mutex>
 #include <unordered_map>
 
@@ -60,10 +65,12 @@ __device__ __forceinline__ void f_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void f_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(f_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void f_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t done;
+// Bounded: a wait that does not end (about a second) gives up, and so does every later one of the thread; the rows that it
+// would have stored become NaN.
+__device__ __forceinline__ void f_wait(uint64_t* bar, uint32_t parity, bool& dead) {
+  uint32_t done = 0;
   const uint32_t addr = f_u32(bar);
-  do {
+  for (int i = 0; !done && !dead; ++i) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -71,7 +78,8 @@ __device__ __forceinline__ void f_wait(uint64_t* bar, uint32_t parity) {
         : "=r"(done)
         : "r"(addr), "r"(parity)
         : "memory");
-  } while (!done);
+    if (i > (1 << 24)) dead = true;
+  }
 }
 __device__ __forceinline__ void f_tma_3d(void* dst, const CUtensorMap* tmap, uint64_t* bar, int c0, int c1,
                                          int c2) {
@@ -99,6 +107,9 @@ __device__ __forceinline__ void f_commit(uint64_t* bar) {
                : "memory");
 }
 __device__ __forceinline__ uint32_t f_desc_lo(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | (1u << 16); }
+// MN-major with the 128-byte swizzle: 64-element blocks along MN are FA_BLK bytes apart (the leading offset), groups of 8
+// along K 1024 bytes (the stride offset in F_DESC_HI)
+__device__ __forceinline__ uint32_t f_desc_lo_mn(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | ((uint32_t)(FA_BLK >> 4) << 16); }
 constexpr uint32_t F_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 
 __device__ __forceinline__ void f_tmem_ld32(uint32_t taddr, uint32_t* r) {
@@ -132,6 +143,8 @@ __device__ __forceinline__ float f_ex2(float x) {
   return y;
 }
 
+// VT: V arrives transposed (K-major B operand), else as [key][dim] rows (MN-major B operand)
+template <bool VT>
 __global__ void __launch_bounds__(FA_THREADS, 1)
 attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const FaParams p_in) {
@@ -149,7 +162,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                                            ~static_cast<uintptr_t>(1023));
   uint8_t* Qs = sm;                          // [128 q][128 d]            2 k-blocks
   uint8_t* Ks = sm + 2 * FA_BLK;             // 2 slots x [128 keys][128 d]
-  uint8_t* Vs = sm + 6 * FA_BLK;             // 2 slots x 2 key-blocks x [hdp d][64 keys]
+  uint8_t* Vs = sm + 6 * FA_BLK;             // 2 slots x (VT: 2 key-blocks x [hdp d][64 keys], else 2 dim-blocks x [128 keys][64 d])
   uint8_t* Ps = sm + 10 * FA_BLK;            // [128 q][128 keys]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = blockIdx.y, kvh = h / (p.n_heads / p.n_kv);
@@ -192,6 +205,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   f_fence_after();
   const uint32_t tmem = tmem_slot;
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  bool dead = false;
 
   if (warp == 0) {
     if (lane == 0) {  // ===== TMA producer =====
@@ -199,44 +213,55 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       for (int c = 0; c < kbq; ++c) f_tma_3d(Qs + c * FA_BLK, &tmQ, &bars.q_full, c * 64, h, p.q0 + row0);
       for (int i = 0; i < 2 * n_tiles; ++i) {
         const int j = i % n_tiles, s = i & 1;
-        f_wait(&bars.k_empty[s], ((i >> 1) & 1) ^ 1);
+        f_wait(&bars.k_empty[s], ((i >> 1) & 1) ^ 1, dead);
         f_expect_tx(&bars.k_full[s], (uint32_t)kbq * FA_BLK);
         for (int c = 0; c < kbq; ++c)
           f_tma_3d(Ks + s * 2 * FA_BLK + c * FA_BLK, &tmK, &bars.k_full[s], c * 64, kvh, p.k0 + j * FA_TK);
         if (i >= n_tiles) {
           const int sv = j & 1;
-          f_wait(&bars.v_empty[sv], ((j >> 1) & 1) ^ 1);
-          f_expect_tx(&bars.v_full[sv], 2u * (uint32_t)vblk);
-          for (int c = 0; c < 2; ++c)
-            f_tma_3d(Vs + sv * 2 * FA_BLK + c * vblk, &tmV, &bars.v_full[sv], p.k0 + j * FA_TK + c * 64, 0, kvh);
+          f_wait(&bars.v_empty[sv], ((j >> 1) & 1) ^ 1, dead);
+          if constexpr (VT) {
+            f_expect_tx(&bars.v_full[sv], 2u * (uint32_t)vblk);
+            for (int c = 0; c < 2; ++c)
+              f_tma_3d(Vs + sv * 2 * FA_BLK + c * vblk, &tmV, &bars.v_full[sv], p.k0 + j * FA_TK + c * 64, 0, kvh);
+          } else {
+            f_expect_tx(&bars.v_full[sv], (uint32_t)kbq * FA_BLK);
+            for (int c = 0; c < kbq; ++c)
+              f_tma_3d(Vs + sv * 2 * FA_BLK + c * FA_BLK, &tmV, &bars.v_full[sv], c * 64, kvh, p.k0 + j * FA_TK);
+          }
         }
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {  // ===== MMA issuer =====
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(FA_TK >> 3) << 17) | (8u << 24);
-      const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.hdp >> 3) << 17) | (8u << 24);
+      // (bit 16: the B operand is MN-major)
+      const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (VT ? 0u : 1u << 16) | ((uint32_t)(p.hdp >> 3) << 17) |
+                               (8u << 24);
       const uint32_t q_lo = f_desc_lo(f_u32(Qs)), p_lo = f_desc_lo(f_u32(Ps));
       const int ksteps = p.hdp >> 4;
       auto do_pv = [&](int j) {
         const int sv = j & 1;
-        f_wait(&bars.p_full, j & 1);
-        f_wait(&bars.v_full[sv], (j >> 1) & 1);
+        f_wait(&bars.p_full, j & 1, dead);
+        f_wait(&bars.v_full[sv], (j >> 1) & 1, dead);
         f_fence_after();
-        const uint32_t v_lo = f_desc_lo(f_u32(Vs + sv * 2 * FA_BLK));
-        for (int ks = 0; ks < FA_TK / 16; ++ks) {
+        const uint32_t v_lo = VT ? f_desc_lo(f_u32(Vs + sv * 2 * FA_BLK)) : f_desc_lo_mn(f_u32(Vs + sv * 2 * FA_BLK));
+        // (groups of 16 keys that lie wholly behind the segment's last key are left out)
+        const int ks_n = VT ? FA_TK / 16 : min(FA_TK / 16, (S - j * FA_TK + 15) >> 4);
+        for (int ks = 0; ks < ks_n; ++ks) {
           const uint32_t a = p_lo + (uint32_t)((ks >> 2) * (FA_BLK >> 4) + (ks & 3) * 2);
-          const uint32_t b = v_lo + (uint32_t)((ks >> 2) * (vblk >> 4) + (ks & 3) * 2);
+          // VT: 32 bytes along a 64-key row; else 16 rows of 128 bytes
+          const uint32_t b = VT ? v_lo + (uint32_t)((ks >> 2) * (vblk >> 4) + (ks & 3) * 2) : v_lo + (uint32_t)(ks * (2048 >> 4));
           f_umma(tmem + 256, a, b, F_DESC_HI, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
         }
         f_commit(&bars.p_empty);
         f_commit(&bars.v_empty[sv]);
       };
-      f_wait(&bars.q_full, 0);
+      f_wait(&bars.q_full, 0, dead);
       for (int i = 0; i < 2 * n_tiles; ++i) {
         const int s = i & 1;
-        f_wait(&bars.k_full[s], (i >> 1) & 1);
-        f_wait(&bars.s_empty[s], ((i >> 1) & 1) ^ 1);
+        f_wait(&bars.k_full[s], (i >> 1) & 1, dead);
+        f_wait(&bars.s_empty[s], ((i >> 1) & 1) ^ 1, dead);
         f_fence_after();
         const uint32_t k_lo = f_desc_lo(f_u32(Ks + s * 2 * FA_BLK));
         for (int ks = 0; ks < ksteps; ++ks) {
@@ -264,7 +289,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     float m = -INFINITY, l = 0.f;
     for (int i = 0; i < n_tiles; ++i) {  // ---- pass 1: row max and sum of exp over bf16 scores ----
       const int s = i & 1;
-      f_wait(&bars.s_full[s], (i >> 1) & 1);
+      f_wait(&bars.s_full[s], (i >> 1) & 1, dead);
       f_fence_after();
       const int jbase = i * FA_TK + half * 64;
 #pragma unroll 1
@@ -310,9 +335,9 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const float nbm = -m * LOG2E;
     for (int j = 0; j < n_tiles; ++j) {  // ---- pass 2: p = bf16(exp(s - m) / l) -> shared memory ----
       const int i = n_tiles + j, s = i & 1;
-      f_wait(&bars.s_full[s], (i >> 1) & 1);
+      f_wait(&bars.s_full[s], (i >> 1) & 1, dead);
       f_fence_after();
-      f_wait(&bars.p_empty, (j & 1) ^ 1);  // the previous P.V has consumed the P tile
+      f_wait(&bars.p_empty, (j & 1) ^ 1, dead);  // the previous P.V has consumed the P tile
       uint8_t* prow = Ps + half * FA_BLK + row * 128;
       const int jbase = j * FA_TK + half * 64;
 #pragma unroll 1
@@ -336,16 +361,32 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       f_fence_before();
       f_arrive(&bars.s_empty[s]);
+      if constexpr (!VT) {
+        // V rows behind the segment's last key (another segment's, or a cache's unused rows) meet p = 0, but 0 times a NaN
+        // or an infinity would still reach O: those of the last group of 16 keys that is multiplied are cleared
+        const int first = S - j * FA_TK, end = (first + 15) & ~15;
+        if (first < FA_TK && first != end) {
+          f_wait(&bars.v_full[j & 1], (j >> 1) & 1, dead);
+          const int per = kbq * 8;
+          for (int idx = threadIdx.x - 64; idx < (end - first) * per; idx += 256) {
+            const int r = first + idx / per, ch = idx % per;
+            *reinterpret_cast<uint4*>(Vs + (j & 1) * 2 * FA_BLK + (ch >> 3) * FA_BLK + r * 128 + (ch & 7) * 16) =
+                make_uint4(0, 0, 0, 0);
+          }
+        }
+      }
       f_fence_async();  // generic-proxy writes of P -> visible to the tensor core (async proxy)
       f_arrive(&bars.p_full);
     }
     // ---- epilogue: O row -> bf16 -> global (16-column chunks alternate between the row's two threads) ----
-    f_wait(&bars.o_full, 0);
+    f_wait(&bars.o_full, 0, dead);
     f_fence_after();
     bf16* orow = p.out + (long)(p.q0 + qi) * p.o_ts + (long)h * p.hd;
     for (int c0 = 16 * half; c0 < p.hd; c0 += 32) {
       uint32_t r[16];
       f_tmem_ld16(t_row + 256u + (uint32_t)c0, r);
+      if (dead)
+        for (int e = 0; e < 16; ++e) r[e] = 0x7FC00000u;
       if (qi < p.Lq) {
         if (c0 + 16 <= p.hd) {
           uint4 o0, o1;
@@ -449,6 +490,7 @@ int fa_tmap3(const void* ptr, int d0, int d1, long s1, int d2, long s2, int b0, 
 
 }  // namespace
 
+// v: V^T (strides head, dim) or V rows (strides token, head): the same alignment rules
 bool attention_fa_supported(const void* q, long q_ts, long q_hs, const void* k, long k_ts, long k_hs,
                             const void* vt, long vt_hs, long vt_ds, const void* out, long o_ts, int hd) {
   auto al = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
@@ -459,16 +501,19 @@ bool attention_fa_supported(const void* q, long q_ts, long q_hs, const void* k, 
 
 // q: PRE-SCALED queries (bf16(q * bf16(scale))), element (t, h, d) at q + t*q_ts + h*q_hs + d
 // k: keys, element (s, kvh, d) at k + s*k_ts + kvh*k_hs + d
-// vt: values transposed, element (kvh, d, s) at vt + kvh*vt_hs + d*vt_ds + s   (keys contiguous)
+// v: values like the keys, element (s, kvh, d) at v + s*v_s0 + kvh*v_s1 + d; v_transposed: element (kvh, d, s) at
+//    v + kvh*v_s0 + d*v_s1 + s (keys contiguous; k0 a multiple of 8: TMA starts on 16-byte boundaries)
 // The tensors hold q_tot query tokens / k_tot keys; this call attends queries [q0, q0+Lq) to keys
-// [k0, k0+S) (one vision segment, or the whole prompt); out row t is written at out + t*o_ts.
-int attention_fa(const void* q, long q_ts, long q_hs, const void* k, long k_ts, long k_hs, const void* vt,
-                 long vt_hs, long vt_ds, void* out, long o_ts, int n_heads, int n_kv, int hd, int Lq, int S,
-                 int causal, cudaStream_t st, int q0, int q_tot, int k0, int k_tot, const void* segs, int n_seg) {
+// [k0, k0+S) (or, segs: a device table of (q0, Lq, k0, S) per segment, Lq / S then the longest of them); out row t is
+// written at out + t*o_ts.
+int attention_fa(const void* q, long q_ts, long q_hs, const void* k, long k_ts, long k_hs, const void* v,
+                 long v_s0, long v_s1, void* out, long o_ts, int n_heads, int n_kv, int hd, int Lq, int S,
+                 int causal, cudaStream_t st, int q0, int q_tot, int k0, int k_tot, const void* segs, int n_seg,
+                 bool v_transposed) {
   if (q_tot <= 0) q_tot = q0 + Lq;
   if (k_tot <= 0) k_tot = k0 + S;
   B200_REQUIRE(!segs || n_seg > 0, "attention_fa: segment table without segments");
-  B200_REQUIRE(attention_fa_supported(q, q_ts, q_hs, k, k_ts, k_hs, vt, vt_hs, vt_ds, out, o_ts, hd),
+  B200_REQUIRE(attention_fa_supported(q, q_ts, q_hs, k, k_ts, k_hs, v, v_s0, v_s1, out, o_ts, hd),
                "attention_fa: unsupported layout (hd=%d)", hd);
   B200_REQUIRE(Lq > 0 && S > 0 && n_heads % n_kv == 0, "attention_fa: bad shape");
   const int hdp = (hd + 15) & ~15;
@@ -476,30 +521,19 @@ int attention_fa(const void* q, long q_ts, long q_hs, const void* k, long k_ts, 
   int rc;
   if ((rc = fa_tmap3(q, hd, n_heads, q_hs, q_tot, q_ts, 64, 1, FA_TQ, &tq))) return rc;
   if ((rc = fa_tmap3(k, hd, n_kv, k_hs, k_tot, k_ts, 64, 1, FA_TK, &tk))) return rc;
-  if ((rc = fa_tmap3(vt, k_tot, hd, vt_ds, n_kv, vt_hs, 64, hdp, 1, &tv))) return rc;
-  static unsigned long long set_mask = 0ull;
-  int dev = 0;
-  B200_CUDA(cudaGetDevice(&dev));
+  if (v_transposed) rc = fa_tmap3(v, k_tot, hd, v_s1, n_kv, v_s0, 64, hdp, 1, &tv);
+  else rc = fa_tmap3(v, hd, n_kv, v_s1, k_tot, v_s0, 64, 1, FA_TK, &tv);
+  if (rc) return rc;
+  const auto kern = v_transposed ? attention_fa_kernel<true> : attention_fa_kernel<false>;
+  static unsigned long long set_mask[2] = {0ull, 0ull};
   const size_t smem = 12 * FA_BLK + 1024;
-  if (!(set_mask >> (dev & 63) & 1ull)) {
-    B200_CUDA(cudaFuncSetAttribute(attention_fa_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    set_mask |= 1ull << (dev & 63);
-  }
+  if (first_use_on_device(&set_mask[v_transposed]))
+    B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   FaParams p;
   p.out = (bf16*)out; p.o_ts = o_ts; p.n_heads = n_heads; p.n_kv = n_kv; p.hd = hd; p.hdp = hdp;
   p.Lq = Lq; p.S = S; p.causal = causal; p.q0 = q0; p.k0 = k0;
   p.segs = (const int4*)segs;
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3(cdiv(Lq, FA_TQ), n_heads, segs ? n_seg : 1);
-  lc.blockDim = dim3(FA_THREADS);
-  lc.dynamicSmemBytes = smem;
-  lc.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  lc.attrs = at;
-  lc.numAttrs = 1;
-  B200_CUDA(cudaLaunchKernelEx(&lc, attention_fa_kernel, tq, tk, tv, p));
+  B200_CUDA(launch_pdl(kern, dim3(cdiv(Lq, FA_TQ), n_heads, segs ? n_seg : 1), dim3(FA_THREADS), smem, st, tq, tk, tv, p));
   return B200_OK;
 }
 
@@ -509,5 +543,5 @@ extern "C" int b200_attention_fa(const void* q, long q_ts, long q_hs, const void
                                  const void* vt, long vt_hs, long vt_ds, void* out, long o_ts, int n_heads,
                                  int n_kv, int hd, int Lq, int S, int causal, void* stream) {
   return b200::attention_fa(q, q_ts, q_hs, k, k_ts, k_hs, vt, vt_hs, vt_ds, out, o_ts, n_heads, n_kv, hd, Lq, S,
-                            causal, (cudaStream_t)stream, 0, Lq, 0, S, nullptr, 0);
+                            causal, (cudaStream_t)stream, 0, Lq, 0, S, nullptr, 0, true);
 }

@@ -157,19 +157,19 @@ int vision_rope(void* qkv, const int* pos_hw, const float* inv_freq, int n_tok, 
                 int hd, cudaStream_t st);
 int mrope_kv_write(void* qkv, const int* pos3, const float* inv_freq, const int* axis_sel,
                    void* kc, void* vc, int T, int ctx0, int cap, int n_heads, int n_kv, int hd,
-                   cudaStream_t st, float q_scale = 0.f, void* vt = nullptr, int t_ld = 0,
-                   const KvRef* ref = nullptr, int layer = 0, void* kws = nullptr, const void* tok_loc = nullptr,
-                   long row_stride = 0);
+                   cudaStream_t st, float q_scale = 0.f, const KvRef* ref = nullptr, int layer = 0,
+                   bool k_in_place = false, const void* tok_loc = nullptr, long row_stride = 0);
 int vision_qkv_post(void* qkv, const int* pos_hw, const float* inv_freq, int n_tok, int n_heads, int hd,
                     float scale, void* vt, int t_ld, cudaStream_t st, const void* cs = nullptr);
 // cos / sin table [n_tok][hd / 2] float2 for vision_qkv_post (computed once per tower call)
 int vision_rope_table(const int* pos_hw, const float* inv_freq, int n_tok, int hd, void* cs, cudaStream_t st);
 bool attention_fa_supported(const void* q, long q_ts, long q_hs, const void* k, long k_ts, long k_hs,
                             const void* vt, long vt_hs, long vt_ds, const void* out, long o_ts, int hd);
-int attention_fa(const void* q, long q_ts, long q_hs, const void* k, long k_ts, long k_hs, const void* vt,
-                 long vt_hs, long vt_ds, void* out, long o_ts, int n_heads, int n_kv, int hd, int Lq, int S,
+int attention_fa(const void* q, long q_ts, long q_hs, const void* k, long k_ts, long k_hs, const void* v,
+                 long v_s0, long v_s1, void* out, long o_ts, int n_heads, int n_kv, int hd, int Lq, int S,
                  int causal, cudaStream_t st, int q0 = 0, int q_tot = 0, int k0 = 0, int k_tot = 0,
-                 const void* segs = nullptr, int n_seg = 0);   // segs: device int4 (q0, Lq, k0, S) per segment; Lq / S = the longest
+                 const void* segs = nullptr, int n_seg = 0,    // segs: device int4 (q0, Lq, k0, S) per segment; Lq / S = the longest
+                 bool v_transposed = false);                   // V rows (token, head strides) or V^T (head, dim strides)
 int swiglu(const void* gu, void* out, int rows, int inter, cudaStream_t st);
 int embed_merge(const int* ids, int B, int T, const void* table, int hidden, const void* feats,
                 int n_feats, int image_token, int video_token, void* out, int* src_out,

@@ -433,6 +433,20 @@ static int upload_loc(b200_engine* e, const std::vector<int>& loc, cudaStream_t 
 }
 
 // rot_pos_emb ids (vision.py:219-249), host side, merge-group-major order
+// the attention segments behind the ids: (first token, tokens, first key, keys) of every frame (vision.py:270-281)
+static void append_frames(const int* grid, int n_img, std::vector<int>* out, int* n_frames, int* longest) {
+  int off = 0;
+  *n_frames = *longest = 0;
+  for (int i = 0; i < n_img; ++i) {
+    const int n = grid[i * 3 + 1] * grid[i * 3 + 2];
+    for (int tt = 0; tt < grid[i * 3]; ++tt, off += n) {
+      for (int v : {off, n, off, n}) out->push_back(v);
+      *n_frames += 1;
+      *longest = n > *longest ? n : *longest;
+    }
+  }
+}
+
 static void build_pos_hw(const int* grid, int n_img, int ms, std::vector<int>* out) {
   out->clear();
   for (int i = 0; i < n_img; ++i) {
@@ -497,7 +511,7 @@ static int seq_run(b200_engine* e, std::vector<b200_engine::SeqGraph>& cache, co
 }
 
 static int vision_v2_body(b200_engine* e, const float* pixel_values, const int* grid, int n_images, long N,
-                          void* feats_out, cudaStream_t s);
+                          void* feats_out, int n_frames, int longest, cudaStream_t s);
 
 static int vision_v2(b200_engine* e, const float* pixel_values, const int* grid, int n_images, long N,
                      void* feats_out, cudaStream_t s) {
@@ -505,30 +519,31 @@ static int vision_v2(b200_engine* e, const float* pixel_values, const int* grid,
   // graph input / output live at fixed workspace addresses: stage them around the captured body
   uint8_t* p = e->ws;
   p += align256(N * (long)c.v_patch_dim * 2) + 2 * align256(N * (long)c.v_embed * 2) +
-       align256(N * 3L * c.v_embed * 2) + align256(N * (long)c.v_mlp * 2) + align256(N * (long)c.v_embed * 2) +
-       align256((long)c.v_embed * round8(N) * 2);
+       align256(N * 3L * c.v_embed * 2) + align256(N * (long)c.v_mlp * 2) + align256(N * (long)c.v_embed * 2);
   float* xin = (float*)p; p += align256(N * (long)c.v_patch_dim * 4);
   bf16* fout = (bf16*)p;
   const long Nm = N / ((long)c.v_merge * c.v_merge);
   int rc;
   std::vector<int> pos;
   build_pos_hw(grid, n_images, c.v_merge, &pos);
+  while (pos.size() % 4) pos.push_back(0);   // the table of segments behind the 2 N ids is read as int4
+  int n_frames = 0, longest = 0;
+  append_frames(grid, n_images, &pos, &n_frames, &longest);
   if ((rc = v2_upload_pos(e, pos, s))) return rc;
   B200_CUDA(cudaMemcpyAsync(xin, pixel_values, (size_t)N * c.v_patch_dim * 4, cudaMemcpyDeviceToDevice, s));
   std::vector<long> key = {(long)(uintptr_t)e->ws, (long)e->ws_bytes, N, (long)n_images, (long)(uintptr_t)e->pos_hw};
   for (int i = 0; i < n_images * 3; ++i) key.push_back(grid[i]);
-  rc = seq_run(e, e->vis_graphs, key, s, [&]() { return vision_v2_body(e, xin, grid, n_images, N, fout, s); });
+  rc = seq_run(e, e->vis_graphs, key, s, [&]() { return vision_v2_body(e, xin, grid, n_images, N, fout, n_frames, longest, s); });
   if (rc) return rc;
   B200_CUDA(cudaMemcpyAsync(feats_out, fout, (size_t)Nm * c.v_out * 2, cudaMemcpyDeviceToDevice, s));
   return B200_OK;
 }
 
 static int vision_v2_body(b200_engine* e, const float* pixel_values, const int* grid, int n_images, long N,
-                          void* feats_out, cudaStream_t s) {
+                          void* feats_out, int n_frames, int longest, cudaStream_t s) {
   const auto& c = e->cfg;
   const long E = c.v_embed, Em = c.v_mlp;
   const int nh = c.v_heads, hd = c.v_embed / c.v_heads;
-  const int t_ld = (int)round8(N);
   uint8_t* p = e->ws;
   bf16* x = (bf16*)p; p += align256(N * (long)c.v_patch_dim * 2);
   bf16* h = (bf16*)p; p += align256(N * E * 2);
@@ -536,7 +551,6 @@ static int vision_v2_body(b200_engine* e, const float* pixel_values, const int* 
   bf16* qkv = (bf16*)p; p += align256(N * 3 * E * 2);
   bf16* mlp = (bf16*)p; p += align256(N * Em * 2);
   bf16* att = (bf16*)p; p += align256(N * E * 2);
-  bf16* vt = (bf16*)p; p += align256(E * (long)t_ld * 2);
   int rc;
   if ((rc = cast_f32_bf16(pixel_values, x, N * c.v_patch_dim, s))) return rc;
   if ((rc = v2_linear(e, x, c.v_patch_dim, e->v_patch, nullptr, h, E, (int)N, (int)E, c.v_patch_dim, B200_EPI_NONE, s)))
@@ -551,42 +565,30 @@ static int vision_v2_body(b200_engine* e, const float* pixel_values, const int* 
     if ((rc = vision_rope_table(e->pos_hw, e->v_inv_freq, (int)N, hd, rope_cs, s))) return rc;
     e->launches += 1;
   }
-  bool fa = attention_fa_supported(qkv, 3 * E, hd, qkv + E, 3 * E, hd, vt, (long)hd * t_ld, t_ld, att, E, hd);
-  {  // the pipelined kernel loads V^T tiles with tokens innermost: a segment must start on a 16-byte boundary
-     // (8 tokens); frames with other offsets (e.g. a 6 x 6-patch image followed by another) take the round-1 kernel
-    long o = 0;
-    for (int im = 0; im < n_images && fa; ++im)
-      for (int tt = 0; tt < grid[im * 3]; ++tt) {
-        if (o % 8) fa = false;
-        o += (long)grid[im * 3 + 1] * grid[im * 3 + 2];
-      }
-  }
+  const bool fa = n_frames <= 65535 && attention_fa_supported(qkv, 3 * E, hd, qkv + E, 3 * E, hd, qkv + 2 * E, 3 * E, hd, att, E, hd);
+  const int* frames = e->pos_hw + (2 * N + 3) / 4 * 4;
   for (int i = 0; i < c.v_depth; ++i) {
     const VBlk& b = e->vblk[i];
     if ((rc = v2_linear(e, y, E, b.qkvw, b.qkvb, qkv, 3 * E, (int)N, (int)(3 * E), (int)E, B200_EPI_NONE, s))) return rc;
-    if (fa) {
-      if ((rc = vision_qkv_post(qkv, e->pos_hw, e->v_inv_freq, (int)N, nh, hd, scale, vt, t_ld, s, rope_cs))) return rc;
+    e->launches += 2;
+    if (fa) {   // every frame of every image in ONE launch: the segment of blockIdx.z
+      if ((rc = vision_qkv_post(qkv, e->pos_hw, e->v_inv_freq, (int)N, nh, hd, scale, nullptr, 0, s, rope_cs))) return rc;
+      if ((rc = attention_fa(qkv, 3 * E, hd, qkv + E, 3 * E, hd, qkv + 2 * E, 3 * E, hd, att, E, nh, nh, hd, longest,
+                             longest, 0, s, 0, (int)N, 0, (int)N, frames, n_frames)))
+        return rc;
     } else {
       if ((rc = vision_rope(qkv, e->pos_hw, e->v_inv_freq, (int)N, nh, hd, s))) return rc;
-    }
-    e->launches += 1;
-    long off = 0;
-    for (int im = 0; im < n_images; ++im) {
-      const int t = grid[im * 3];
-      const int seg = grid[im * 3 + 1] * grid[im * 3 + 2];
-      for (int tt = 0; tt < t; ++tt) {  // one attention segment per frame (vision.py:270-281)
-        if (fa) {
-          rc = attention_fa(qkv, 3 * E, hd, qkv + E, 3 * E, hd, vt, (long)hd * t_ld, t_ld, att, E, nh, nh, hd, seg,
-                            seg, 0, s, (int)off, (int)N, (int)off, (int)N);
-        } else {
+      long off = 0;
+      for (int im = 0; im < n_images; ++im) {
+        const int seg = grid[im * 3 + 1] * grid[im * 3 + 2];
+        for (int tt = 0; tt < grid[im * 3]; ++tt, off += seg) {
           const bf16* qb = qkv + off * 3 * E;
-          rc = attention(qb, 3 * E, hd, qb + E, 3 * E, hd, qb + 2 * E, 3 * E, hd, att + off * E, E, nh, nh, hd,
-                         seg, seg, 0, scale, s);
+          if ((rc = attention(qb, 3 * E, hd, qb + E, 3 * E, hd, qb + 2 * E, 3 * E, hd, att + off * E, E, nh, nh, hd, seg,
+                              seg, 0, scale, s)))
+            return rc;
         }
-        if (rc) return rc;
-        off += seg;
-        e->launches += 1;
       }
+      e->launches += n_frames - 1;
     }
     if ((rc = v2_linear_residual_norm(e, att, E, b.projw, b.projb, h, E, B200_NORM_LN, b.ln2w, b.ln2b, c.v_ln_eps,
                                       y, E, (int)N, (int)E, (int)E, s)))
@@ -661,7 +663,7 @@ static int prefill_layers_v2_body(b200_engine* e, const int* pos3, int T, int ct
   const auto& c = e->cfg;
   const long H = c.hidden, I = c.inter, QH = (long)c.n_heads * c.head_dim;
   const long QKV = (long)(c.n_heads + 2 * c.n_kv_heads) * c.head_dim;
-  const int hd = c.head_dim, t_ld = (int)round8(T);
+  const int hd = c.head_dim;
   uint8_t* p = e->ws;
   bf16* h = (bf16*)p; p += align256((long)T * H * 2);
   bf16* xn = (bf16*)p; p += align256((long)T * H * 2);
@@ -669,9 +671,6 @@ static int prefill_layers_v2_body(b200_engine* e, const int* pos3, int T, int ct
   bf16* att = (bf16*)p; p += align256((long)T * QH * 2);
   p += align256((long)T * 2 * I * 2);  // (gate/up buffer of the round-1 path)
   bf16* act = (bf16*)p; p += align256((long)T * I * 2);
-  p += align256(3L * T * 4);
-  bf16* vt = (bf16*)p; p += align256((long)c.n_kv_heads * hd * t_ld * 2);
-  bf16* kws = (bf16*)p; p += align256((long)c.n_kv_heads * hd * T * 2);
   int rc;
   if ((rc = rms_norm(h, e->layers[0].ln1, xn, T, (int)H, c.rms_eps, s))) return rc;
   e->launches += 1;
@@ -683,39 +682,36 @@ static int prefill_layers_v2_body(b200_engine* e, const int* pos3, int T, int ct
     bf16* kc = e->kptr(l, e->kv_row);
     bf16* vc = e->vptr(l, e->kv_row);
     if ((rc = v2_linear(e, xn, H, lw.wqkv, lw.bqkv, qkv, QKV, T, (int)QKV, (int)H, B200_EPI_NONE, s))) return rc;
-    // the pipelined kernel needs V^T of EVERY key: available for a fresh prompt (ctx0 == 0).  It then
-    // reads the chunk's own rotated K copy and V^T from the workspace, and the cache is addressed through
-    // e->kvref: nothing about the KV pool is baked into the captured graph.
-    const bool fa = ctx0 == 0 && attention_fa_supported(qkv, QKV, hd, kws, hd, (long)T * hd, vt, (long)hd * t_ld,
-                                                        t_ld, att, QH, hd);
+    // A fresh prompt's keys (rotated in place) and values are read from its qkv rows, so nothing about the KV pool is baked
+    // into the captured graph (the cache is written through e->kvref); a later portion reads the cached ones where they are.
+    const bool fresh = ctx0 == 0;
+    const bf16 *ka = fresh ? qkv + QH : kc, *va = fresh ? qkv + QH + (long)c.n_kv_heads * hd : vc;
+    const long kv_ts = fresh ? QKV : hd, kv_hs = fresh ? hd : (long)e->kv_cap * hd;
+    const bool fa = attention_fa_supported(qkv, QKV, hd, ka, kv_ts, kv_hs, va, kv_ts, kv_hs, att, QH, hd);
+    e->launches += 2;
     if (segs) {
       B200_REQUIRE(fa, "prefill_batch: the pipelined attention kernel does not support this geometry");
       const long row_stride = (long)c.n_kv_heads * e->kv_cap * hd;
       if ((rc = mrope_kv_write(qkv, pos3, e->lm_inv_freq, e->axis_sel, e->kptr(l, 0), e->vptr(l, 0), T, 0, e->kv_cap,
-                               c.n_heads, c.n_kv_heads, hd, s, scale_bf, vt, t_ld, nullptr, l, kws, tok_loc, row_stride)))
+                               c.n_heads, c.n_kv_heads, hd, s, scale_bf, nullptr, l, true, tok_loc, row_stride)))
         return rc;
       // all sequences in ONE launch: the (q0, Lq, k0, S) table follows the (row, position) table in `tok_loc`
       int longest = 0;
       for (int g = 0; g < n_seg; ++g) longest = segs[g].T > longest ? segs[g].T : longest;
-      if ((rc = attention_fa(qkv, QKV, hd, kws, hd, (long)T * hd, vt, (long)hd * t_ld, t_ld, att, QH, c.n_heads,
-                             c.n_kv_heads, hd, longest, longest, 1, s, 0, T, 0, T, (const int*)tok_loc + 2L * T, n_seg)))
+      rc = attention_fa(qkv, QKV, hd, ka, kv_ts, kv_hs, va, kv_ts, kv_hs, att, QH, c.n_heads, c.n_kv_heads, hd, longest,
+                        longest, 1, s, 0, T, 0, T, (const int*)tok_loc + 2L * T, n_seg);
+    } else {
+      if ((rc = mrope_kv_write(qkv, pos3, e->lm_inv_freq, e->axis_sel, kc, vc, T, ctx0, e->kv_cap, c.n_heads,
+                               c.n_kv_heads, hd, s, fa ? scale_bf : 0.f, fa && fresh ? e->kvref : nullptr, l, fa && fresh)))
         return rc;
-      e->launches += 2;
-    } else {
-    if ((rc = mrope_kv_write(qkv, pos3, e->lm_inv_freq, e->axis_sel, kc, vc, T, ctx0, e->kv_cap, c.n_heads,
-                             c.n_kv_heads, hd, s, fa ? scale_bf : 0.f, fa ? vt : nullptr, t_ld,
-                             fa ? e->kvref : nullptr, l, fa ? kws : nullptr)))
-      return rc;
-    if (fa) {
-      rc = attention_fa(qkv, QKV, hd, kws, hd, (long)T * hd, vt, (long)hd * t_ld, t_ld, att, QH, c.n_heads,
-                        c.n_kv_heads, hd, T, S, 1, s, 0, T, 0, S);
-    } else {
-      rc = attention(qkv, QKV, hd, kc, hd, (long)e->kv_cap * hd, vc, hd, (long)e->kv_cap * hd, att, QH, c.n_heads,
-                     c.n_kv_heads, hd, T, S, 1, scale, s);
+      if (fa)
+        rc = attention_fa(qkv, QKV, hd, ka, kv_ts, kv_hs, va, kv_ts, kv_hs, att, QH, c.n_heads, c.n_kv_heads, hd, T, S, 1, s,
+                          0, T, 0, S);
+      else
+        rc = attention(qkv, QKV, hd, kc, hd, (long)e->kv_cap * hd, vc, hd, (long)e->kv_cap * hd, att, QH, c.n_heads,
+                       c.n_kv_heads, hd, T, S, 1, scale, s);
     }
     if (rc) return rc;
-    e->launches += 2;
-    }
     if ((rc = v2_linear_residual_norm(e, att, QH, lw.wo, nullptr, h, H, B200_NORM_RMS, lw.ln2, nullptr, c.rms_eps, xn,
                                       H, T, (int)H, (int)QH, s)))
       return rc;
@@ -879,9 +875,6 @@ long b200_engine_workspace_bytes(const b200_engine* e, int max_tokens, int max_p
   long v = align256(N * (long)c.v_patch_dim * 2) + align256(N * (long)c.v_embed * 2) * 2 +
            align256(N * 3L * c.v_embed * 2) + align256(N * (long)c.v_mlp * 2) +
            align256(N * (long)c.v_embed * 2);
-  lm += align256((long)c.n_kv_heads * c.head_dim * round8(T) * 2);  // V^T of the prompt chunk
-  lm += align256((long)c.n_kv_heads * c.head_dim * T * 2);          // rotated K of the prompt chunk
-  v += align256((long)c.v_embed * round8(N) * 2);                   // V^T of the vision tower
   v += align256(N * (long)c.v_patch_dim * 4);                       // staged fp32 pixel_values (graph input)
   v += align256((N / ((long)c.v_merge * c.v_merge) + 1) * c.v_out * 2);  // staged features (graph output)
   return (lm > v ? lm : v) + WT_PARTIAL_BYTES + 4096;
@@ -1102,8 +1095,7 @@ int b200_engine_prefill_batch(b200_engine* e, const void* embeds, const int* pos
                  "engine_prefill_batch: sequence %d: %d tokens into row %d (capacity %d, %d rows)", g, seq_len[g], rows[g],
                  e->kv_cap, e->kv_batch);
     segs[g] = PreSeg{(int)T, seq_len[g], rows[g]};
-    T += round8(seq_len[g]);   // every sequence starts at a multiple of 8 tokens: the V^T tiles are loaded by TMA
-                               // with tokens innermost, and a box must start on a 16-byte boundary
+    T += round8(seq_len[g]);   // every sequence starts at a multiple of 8 tokens (the layout of `embeds` and `pos3`)
   }
   B200_REQUIRE(e->ws && b200_engine_workspace_bytes(e, (int)T, 1) <= e->ws_bytes,
                "engine_prefill_batch: workspace too small for %ld tokens", T);

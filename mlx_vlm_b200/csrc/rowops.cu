@@ -149,10 +149,8 @@ __global__ void mrope_kv_write_kernel(bf16* __restrict__ qkv, const int* __restr
                                       const float* __restrict__ inv_freq,
                                       const int* __restrict__ axis_sel, bf16* __restrict__ kc,
                                       bf16* __restrict__ vc, int T, int ctx0, int cap, int n_heads,
-                                      int n_kv, int hd, float q_scale, bf16* __restrict__ vt,
-                                      int t_ld, const KvRef* __restrict__ ref, int layer,
-                                      bf16* __restrict__ kws, const int2* __restrict__ tok_loc,
-                                      long row_stride) {
+                                      int n_kv, int hd, float q_scale, const KvRef* __restrict__ ref, int layer,
+                                      bool k_in_place, const int2* __restrict__ tok_loc, long row_stride) {
   // tok_loc (batched prefill of several sequences in one pass): token t belongs to pool row tok_loc[t].x and
   // lands at cache position tok_loc[t].y; kc / vc then point at row 0 and rows are row_stride elements apart
   pdl_prologue();
@@ -181,10 +179,6 @@ __global__ void mrope_kv_write_kernel(bf16* __restrict__ qkv, const int* __restr
         dst[j] = base[j];
         dst[j + half] = base[j + half];
       }
-      if (vt) {  // V^T [kv head][dim][token] for the pipelined attention kernel (attention_fa.cu)
-        vt[((long)kvh * hd + j) * t_ld + t] = base[j];
-        vt[((long)kvh * hd + j + half) * t_ld + t] = base[j + half];
-      }
       continue;
     }
     const float ang = (float)pos3[axis_sel[j] * T + t] * inv_freq[j];
@@ -203,120 +197,88 @@ __global__ void mrope_kv_write_kernel(bf16* __restrict__ qkv, const int* __restr
         dst[j] = f2bf(o1);
         dst[j + half] = f2bf(o2);
       }
-      if (kws) {  // the prompt chunk's rotated keys [kv head][token][dim] for the pipelined attention
-        bf16* d2 = kws + ((long)kvh * T + t) * hd;
-        d2[j] = f2bf(o1);
-        d2[j + half] = f2bf(o2);
+      if (k_in_place) {  // the pipelined attention reads a fresh prompt's keys from the qkv rows
+        base[j] = f2bf(o1);
+        base[j + half] = f2bf(o2);
       }
     }
   }
 }
 
 // The same operation, tiled (head_dim a multiple of 16): a CTA takes 32 tokens x a group of head slots; thread (token,
-// chunk of 8 rotary pairs) computes its 8 cos / sin ONCE and re-uses them for every head of the group, all loads and
-// stores are 16-byte vectors, and V^T goes through a shared-memory tile so that its stores are contiguous along the
-// token axis.  Identical arithmetic, element for element, to the scalar kernel above (which evaluated cosf / sinf per
-// element and wrote V^T with 2-byte stores a row apart: 329 us per layer at T = 4864 on the Llama-7B geometry = 13 % of
-// the batched C3 prefill, profiles/r2_launches_c3_prefill_ncu.txt).  grid (ceil(T / 32), slot groups), 256 threads.
+// chunk of 8 rotary pairs) computes its 8 cos / sin ONCE and re-uses them for every head of the group; loads and stores
+// are 16-byte vectors, the loads of four heads in flight before the first store (a head's load waits for the one before
+// it otherwise: the stores may alias).  Identical arithmetic, element for element, to the scalar kernel above.  Bound by
+// memory: 2 B read and 2 (V) or 2 + 2 (q in place; K in place and cached) written per element.
+// grid (ceil(T / 32), slot groups), 256 threads.
 __global__ void __launch_bounds__(256)
 mrope_kv_write_tiled_kernel(bf16* __restrict__ qkv, const int* __restrict__ pos3, const float* __restrict__ inv_freq,
                             const int* __restrict__ axis_sel, bf16* __restrict__ kc, bf16* __restrict__ vc, int T, int ctx0,
-                            int cap, int n_heads, int n_kv, int hd, float q_scale, bf16* __restrict__ vt, int t_ld,
-                            const KvRef* __restrict__ ref, int layer, bf16* __restrict__ kws,
-                            const int2* __restrict__ tok_loc, long row_stride, int slots_per_cta) {
+                            int cap, int n_heads, int n_kv, int hd, float q_scale, const KvRef* __restrict__ ref, int layer,
+                            bool k_in_place, const int2* __restrict__ tok_loc, long row_stride, int slots_per_cta) {
   pdl_prologue();
   if (ref) {
     kc = ref->k0 + (long)layer * ref->layer_stride;
     vc = kc + ref->v_off;
     cap = ref->cap;
   }
-  __shared__ bf16 tile[32][136];
-  const int half = hd >> 1, nc = half >> 3, nv = hd >> 3;
+  constexpr int U = 4;   // heads in flight
+  const int half = hd >> 1, nc = half >> 3;
   const int slots = n_heads + 2 * n_kv;
-  const long row_elems = (long)slots * hd;
-  const int t0 = blockIdx.x * 32;
-  const int tl = threadIdx.x / nc, c = threadIdx.x % nc;
-  const int t = t0 + tl;
-  const bool act = threadIdx.x < 32 * nc && t < T;
+  const int c = threadIdx.x % nc;
+  const int t = blockIdx.x * 32 + threadIdx.x / nc;
+  if (threadIdx.x >= 32 * nc || t >= T) return;
   float cs[8], sn[8];
-  int2 loc = make_int2(-1, 0);
-  if (act) {
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int j = c * 8 + u;
-      const float ang = (float)pos3[axis_sel[j] * T + t] * inv_freq[j];
-      cs[u] = rbf(cosf(ang));
-      sn[u] = rbf(sinf(ang));
-    }
-    loc = tok_loc ? tok_loc[t] : make_int2(0, ctx0 + t);
+  for (int u = 0; u < 8; ++u) {
+    const int j = c * 8 + u;
+    const float ang = (float)pos3[axis_sel[j] * T + t] * inv_freq[j];
+    cs[u] = rbf(cosf(ang));
+    sn[u] = rbf(sinf(ang));
   }
+  const int2 loc = tok_loc ? tok_loc[t] : make_int2(0, ctx0 + t);   // (row -1: a padding token of a batched prefill)
+  const long at = (long)loc.x * row_stride + (long)loc.y * hd + c * 8;
+  bf16* row = qkv + (long)t * slots * hd + c * 8;
   const int s_begin = blockIdx.y * slots_per_cta;
   const int s_end = min(slots, s_begin + slots_per_cta);
-  for (int slot = s_begin; slot < s_end; ++slot) {
-    if (slot < n_heads + n_kv) {   // q or k head: rotate
-      if (!act) continue;
-      bf16* base = qkv + (long)t * row_elems + (long)slot * hd;
-      float x1[8], x2[8], o1[8], o2[8];
-      unpack8(*reinterpret_cast<const uint4*>(base + c * 8), x1);
-      unpack8(*reinterpret_cast<const uint4*>(base + half + c * 8), x2);
-      const bool is_q = slot < n_heads;
+  for (int s0 = s_begin; s0 < s_end; s0 += U) {
+    uint4 a[U], b[U];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        o1[u] = rbf(rbf(x1[u] * cs[u]) + rbf((-x2[u]) * sn[u]));
-        o2[u] = rbf(rbf(x2[u] * cs[u]) + rbf(x1[u] * sn[u]));
-        if (is_q && q_scale != 0.f) {   // qs = bf16(q * bf16(scale)) of the SDPA (base.py:305-373)
-          o1[u] *= q_scale;
-          o2[u] *= q_scale;
-        }
+    for (int i = 0; i < U; ++i)
+      if (s0 + i < s_end) {
+        a[i] = *reinterpret_cast<const uint4*>(row + (long)(s0 + i) * hd);
+        b[i] = *reinterpret_cast<const uint4*>(row + (long)(s0 + i) * hd + half);
       }
-      uint4 w1, w2;
-      w1.x = pack2(o1[0], o1[1]); w1.y = pack2(o1[2], o1[3]); w1.z = pack2(o1[4], o1[5]); w1.w = pack2(o1[6], o1[7]);
-      w2.x = pack2(o2[0], o2[1]); w2.y = pack2(o2[2], o2[3]); w2.z = pack2(o2[4], o2[5]); w2.w = pack2(o2[6], o2[7]);
-      if (is_q) {
-        *reinterpret_cast<uint4*>(base + c * 8) = w1;
-        *reinterpret_cast<uint4*>(base + half + c * 8) = w2;
-      } else {
-        const int kvh = slot - n_heads;
-        if (loc.x >= 0) {   // (row -1: a padding token of a batched prefill)
-          bf16* dst = kc + (long)loc.x * row_stride + ((long)kvh * cap + loc.y) * hd;
-          *reinterpret_cast<uint4*>(dst + c * 8) = w1;
-          *reinterpret_cast<uint4*>(dst + half + c * 8) = w2;
-        }
-        if (kws) {
-          bf16* d2 = kws + ((long)kvh * T + t) * hd;
-          *reinterpret_cast<uint4*>(d2 + c * 8) = w1;
-          *reinterpret_cast<uint4*>(d2 + half + c * 8) = w2;
-        }
-      }
-    } else {   // V head: copy into the cache, and transposed into V^T [kv head][dim][token]
-      const int kvh = slot - n_heads - n_kv;
-      for (int idx = threadIdx.x; idx < 32 * nv; idx += blockDim.x) {
-        const int tl2 = idx / nv, c2 = idx % nv;
-        const int t2 = t0 + tl2;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (t2 < T) {
-          v = *reinterpret_cast<const uint4*>(qkv + (long)t2 * row_elems + (long)slot * hd + c2 * 8);
-          const int2 l2 = tok_loc ? tok_loc[t2] : make_int2(0, ctx0 + t2);
-          if (l2.x >= 0)
-            *reinterpret_cast<uint4*>(vc + (long)l2.x * row_stride + ((long)kvh * cap + l2.y) * hd + c2 * 8) = v;
-        }
-        *reinterpret_cast<uint4*>(&tile[tl2][c2 * 8]) = v;
-      }
-      __syncthreads();
-      if (vt) {
-        for (int idx = threadIdx.x; idx < hd * 4; idx += blockDim.x) {
-          const int d = idx >> 2, ch = idx & 3;
-          if (t0 + ch * 8 >= t_ld) continue;
-          unsigned short e[8];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) e[u] = __bfloat16_as_ushort(tile[ch * 8 + u][d]);
-          uint4 o;
-          o.x = e[0] | ((uint32_t)e[1] << 16); o.y = e[2] | ((uint32_t)e[3] << 16);
-          o.z = e[4] | ((uint32_t)e[5] << 16); o.w = e[6] | ((uint32_t)e[7] << 16);
-          *reinterpret_cast<uint4*>(vt + ((long)kvh * hd + d) * t_ld + t0 + ch * 8) = o;
+    for (int i = 0; i < U; ++i) {
+      const int slot = s0 + i;
+      if (slot >= s_end) continue;
+      const bool is_q = slot < n_heads, is_v = slot >= n_heads + n_kv;
+      if (!is_v) {   // rotate
+        float x1[8], x2[8], o1[8], o2[8];
+        unpack8(a[i], x1);
+        unpack8(b[i], x2);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          o1[u] = rbf(rbf(x1[u] * cs[u]) + rbf((-x2[u]) * sn[u]));
+          o2[u] = rbf(rbf(x2[u] * cs[u]) + rbf(x1[u] * sn[u]));
+          if (is_q && q_scale != 0.f) {   // qs = bf16(q * bf16(scale)) of the SDPA (base.py:305-373)
+            o1[u] *= q_scale;
+            o2[u] *= q_scale;
+          }
+        }
+        a[i] = make_uint4(pack2(o1[0], o1[1]), pack2(o1[2], o1[3]), pack2(o1[4], o1[5]), pack2(o1[6], o1[7]));
+        b[i] = make_uint4(pack2(o2[0], o2[1]), pack2(o2[2], o2[3]), pack2(o2[4], o2[5]), pack2(o2[6], o2[7]));
+        if (is_q || k_in_place) {   // (in place: the pipelined attention reads a fresh prompt's keys from the qkv rows)
+          *reinterpret_cast<uint4*>(row + (long)slot * hd) = a[i];
+          *reinterpret_cast<uint4*>(row + (long)slot * hd + half) = b[i];
         }
       }
-      __syncthreads();
+      if (!is_q && loc.x >= 0) {
+        bf16* dst = (is_v ? vc + (long)(slot - n_heads - n_kv) * cap * hd : kc + (long)(slot - n_heads) * cap * hd) + at;
+        *reinterpret_cast<uint4*>(dst) = a[i];
+        *reinterpret_cast<uint4*>(dst + half) = b[i];
+      }
     }
   }
 }
@@ -459,35 +421,34 @@ int vision_rope(void* qkv, const int* pos_hw, const float* inv_freq, int n_tok, 
 
 int mrope_kv_write(void* qkv, const int* pos3, const float* inv_freq, const int* axis_sel,
                    void* kc, void* vc, int T, int ctx0, int cap, int n_heads, int n_kv, int hd,
-                   cudaStream_t st, float q_scale, void* vt, int t_ld, const KvRef* ref, int layer, void* kws,
+                   cudaStream_t st, float q_scale, const KvRef* ref, int layer, bool k_in_place,
                    const void* tok_loc, long row_stride) {
   B200_REQUIRE(T > 0 && ctx0 >= 0 && (ref || tok_loc || ctx0 + T <= cap), "mrope_kv_write: T=%d ctx0=%d cap=%d", T,
                ctx0, cap);
-  B200_REQUIRE(!vt || t_ld >= T, "mrope_kv_write: V^T pitch %d < T %d", t_ld, T);
   static const bool scalar_only = getenv("B200_MROPE_SCALAR") != nullptr;   // A/B and fallback
-  if (!scalar_only && (hd % 16) == 0 && hd <= 128 && (!vt || (t_ld % 8) == 0)) {
+  if (!scalar_only && (hd % 16) == 0 && hd <= 128) {
     const int slots = n_heads + 2 * n_kv, tiles = (T + 31) / 32;
     int groups = (4 * 148 + tiles - 1) / tiles;          // about four waves of CTAs
     if (groups > slots) groups = slots;
     if (groups < 1) groups = 1;
     const int per = (slots + groups - 1) / groups;
     B200_CUDA(launch_pdl(mrope_kv_write_tiled_kernel, dim3(tiles, (slots + per - 1) / per), dim3(256), 0, st, (bf16*)qkv,
-                         pos3, inv_freq, axis_sel, (bf16*)kc, (bf16*)vc, T, ctx0, cap, n_heads, n_kv, hd, q_scale, (bf16*)vt,
-                         t_ld, ref, layer, (bf16*)kws, (const int2*)tok_loc, row_stride, per));
+                         pos3, inv_freq, axis_sel, (bf16*)kc, (bf16*)vc, T, ctx0, cap, n_heads, n_kv, hd, q_scale, ref,
+                         layer, k_in_place, (const int2*)tok_loc, row_stride, per));
     return B200_OK;
   }
   const long total = (long)T * (n_heads + 2 * n_kv) * (hd / 2);
   B200_CUDA(launch_pdl(mrope_kv_write_kernel, dim3(grid_for(total, 256)), dim3(256), 0, st, (bf16*)qkv, pos3, inv_freq,
-                       axis_sel, (bf16*)kc, (bf16*)vc, T, ctx0, cap, n_heads, n_kv, hd, q_scale, (bf16*)vt, t_ld, ref,
-                       layer, (bf16*)kws, (const int2*)tok_loc, row_stride));
+                       axis_sel, (bf16*)kc, (bf16*)vc, T, ctx0, cap, n_heads, n_kv, hd, q_scale, ref, layer, k_in_place,
+                       (const int2*)tok_loc, row_stride));
   return B200_OK;
 }
 
 // ---------------------------------------------------------------------------
 // Vision tower, after the qkv GEMM: 2-D rotary on q and k in place (same arithmetic as
-// vision_rope_kernel), q pre-scaled for the SDPA (qs = bf16(q * bf16(scale))), and V written
-// TRANSPOSED ([head][dim][token], tokens contiguous) through a shared-memory tile: the
-// pipelined attention kernel loads Q, K and V^T with TMA and touches no operand with a thread.
+// vision_rope_kernel), q pre-scaled for the SDPA (qs = bf16(q * bf16(scale))), and, where vt is given, V written
+// TRANSPOSED ([head][dim][token], tokens contiguous) through a shared-memory tile (the tower itself passes none: its
+// attention reads V from the qkv rows).
 // grid (ceil(T / 32), heads), 256 threads.
 __global__ void vision_rope_table_kernel(const int* __restrict__ pos_hw, const float* __restrict__ inv_freq, int T,
                                         int half, float2* __restrict__ cs) {
@@ -569,6 +530,7 @@ __global__ void vision_qkv_post_kernel(bf16* __restrict__ qkv, const int* __rest
       base[j + half] = f2bf(o2);
     }
   }
+  if (!vt) return;
   const int nv = hd >> 3;
   for (int idx = threadIdx.x; idx < 32 * nv; idx += blockDim.x) {
     const int tl = idx / nv, c = idx % nv;
@@ -601,7 +563,7 @@ int vision_rope_table(const int* pos_hw, const float* inv_freq, int n_tok, int h
 
 int vision_qkv_post(void* qkv, const int* pos_hw, const float* inv_freq, int n_tok, int n_heads, int hd,
                     float scale, void* vt, int t_ld, cudaStream_t st, const void* cs) {
-  B200_REQUIRE(n_tok > 0 && n_heads > 0 && (hd % 8) == 0 && hd <= 128 && (t_ld % 8) == 0 && t_ld >= n_tok,
+  B200_REQUIRE(n_tok > 0 && n_heads > 0 && (hd % 8) == 0 && hd <= 128 && (!vt || ((t_ld % 8) == 0 && t_ld >= n_tok)),
                "vision_qkv_post: bad shape (hd=%d t_ld=%d)", hd, t_ld);
   const float scale_bf = __bfloat162float(__float2bfloat16_rn(scale));
   B200_CUDA(launch_pdl(vision_qkv_post_kernel, dim3(cdiv(n_tok, 32), n_heads), dim3(256), 0, st, (bf16*)qkv, pos_hw,
@@ -658,10 +620,11 @@ int b200_mrope_kv_write(void* qkv, const int* pos3, const float* inv_freq, const
                         void* kc, void* vc, int T, int ctx0, int cap, int n_heads, int n_kv,
                         int hd, void* st) {
   return mrope_kv_write(qkv, pos3, inv_freq, axis_sel, kc, vc, T, ctx0, cap, n_heads, n_kv, hd,
-                        (cudaStream_t)st, 0.f, nullptr, 0, nullptr, 0, nullptr, nullptr, 0);
+                        (cudaStream_t)st, 0.f, nullptr, 0, false, nullptr, 0);
 }
 int b200_vision_qkv_post(void* qkv, const int* pos_hw, const float* inv_freq, int n_tok, int n_heads,
                          int hd, float scale, void* vt, int t_ld, void* st) {
+  B200_REQUIRE(vt, "vision_qkv_post: V^T buffer missing");
   return vision_qkv_post(qkv, pos_hw, inv_freq, n_tok, n_heads, hd, scale, vt, t_ld, (cudaStream_t)st, nullptr);
 }
 int b200_swiglu(const void* gu, void* out, int rows, int inter, void* st) {
