@@ -216,6 +216,24 @@ int finish_rows(const float* P, int S, const void* bias, const void* resid, long
                 long ldh, int norm_kind, const void* nw, const void* nb, float eps, void* xn, long ldx,
                 int T, int N, cudaStream_t st, const void* l2_prefetch = nullptr, long l2_prefetch_bytes = 0);
 void gemm_wt_set_pdl(bool on);
+// fp32 attention of the towers (attention_f32_tc.cu)
+struct AttnF32P {
+  const float *q, *k, *v;
+  long q_ts, q_hs, k_ts, k_hs, v_ts, v_hs;  // element strides: token, head
+  float* out32;
+  long o_ts;
+  bf16* out_split;
+  long os_ts;
+  int n_pad;
+  int n_heads, n_kv, Lq, S, hd;
+  long q_seg, k_seg;   // tokens between consecutive segments (blockIdx.z)
+  const unsigned char* key_mask;  // optional [segments][S]: 0 = key masked out
+  const int* cu;                  // optional [segments + 1]: segment z = tokens [cu[z], cu[z+1]) of q, k and v (self-attention
+                                  // over ragged segments, e.g. Qwen2.5-VL's windows); Lq is then the longest segment
+  float scale;
+  bool out_vec;                   // the outputs may be stored four elements at a time (set by the launch)
+};
+int attention_f32_tc(AttnF32P p, int n_seg, cudaStream_t st);
 int attention(const void* q, long q_ts, long q_hs, const void* k, long k_ts, long k_hs,
               const void* v, long v_ts, long v_hs, void* out, long o_ts, int n_heads, int n_kv,
               int hd, int Lq, int S, int causal, float scale, cudaStream_t st);

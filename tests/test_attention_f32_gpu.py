@@ -1,0 +1,82 @@
+"""fp32 attention of the towers (csrc/attention_f32_tc.cu) against float64 at the edges of its tiles: 128 query rows, 64 keys,
+groups of 16 keys, head sizes padded to 32 / 64 / 80 / 96.
+
+Bound: a score is a sum of at most 96 products with 24 bits each (relative error about 1e-7 of |q||k|, |scores| <= ~6 here, so
+6e-7 in the exponent), the exponential 2^-22, sums and outputs 2^-24 a step: 2e-6 of the output's size."""
+import pytest
+import torch
+
+from _util import rl2
+
+pytestmark = pytest.mark.gpu
+BOUND = 2e-6
+
+
+@pytest.fixture(scope="module")
+def lib():
+    from mlx_vlm_b200 import _native as N
+    return N.lib()
+
+
+def _rand(*shape, seed):
+    return torch.randn(shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda")
+
+
+def _want(q, k, v, nh, nkv, hd, keep=None):
+    q = q.double().view(-1, nh, hd).transpose(0, 1)
+    k, v = (x.double().view(-1, nkv, hd).transpose(0, 1).repeat_interleave(nh // nkv, 0) for x in (k, v))
+    s = q @ k.transpose(1, 2) * hd ** -0.5
+    if keep is not None:
+        s = s.masked_fill(~keep, float("-inf"))
+    return (torch.softmax(s, -1) @ v).transpose(0, 1).reshape(-1, nh * hd)
+
+
+def _split_value(t, n, n_pad):
+    return t[:, :n].double() + t[:, n_pad:n_pad + n].double()
+
+
+@pytest.mark.parametrize("nh,nkv,hd,Lq,S", [
+    (2, 2, 64, 128, 64), (2, 2, 64, 129, 65), (1, 1, 64, 127, 63), (2, 1, 64, 1, 1), (2, 2, 64, 5, 16), (2, 2, 64, 130, 17),
+    (3, 3, 72, 64, 128), (2, 2, 72, 200, 129), (4, 1, 96, 64, 113), (2, 2, 80, 33, 49), (2, 2, 20, 70, 100), (1, 1, 4, 3, 80),
+    (2, 2, 32, 40, 192)])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_tile_edges(lib, nh, nkv, hd, Lq, S, aligned):
+    """two segments, both outputs; unaligned output addresses are stored element by element"""
+    from mlx_vlm_b200 import _native as N
+    q, k, v = _rand(2 * Lq, nh * hd, seed=1), _rand(2 * S, nkv * hd, seed=2), _rand(2 * S, nkv * hd, seed=3)
+    E, n_pad, off = nh * hd, (nh * hd + 63) // 64 * 64, 0 if aligned else 1
+    o32 = torch.full((2 * Lq * E + 2,), 7.0, device="cuda")
+    osp = torch.full((2 * Lq * 2 * n_pad + 2,), 7.0, device="cuda", dtype=torch.bfloat16)
+    N.check(lib.b200_attention_f32(q.data_ptr(), E, hd, k.data_ptr(), nkv * hd, hd, v.data_ptr(), nkv * hd, hd,
+                                   o32[off:].data_ptr(), E, osp[off:].data_ptr(), 2 * n_pad, n_pad, nh, nkv, hd, Lq, S, 2, Lq, S, 0,
+                                   hd ** -0.5, 0), "attention_f32")
+    torch.cuda.synchronize()
+    want = torch.cat([_want(q[s * Lq:(s + 1) * Lq], k[s * S:(s + 1) * S], v[s * S:(s + 1) * S], nh, nkv, hd) for s in (0, 1)])
+    assert rl2(o32[off:off + 2 * Lq * E].view(2 * Lq, E).double(), want) <= BOUND
+    got = _split_value(osp[off:off + 2 * Lq * 2 * n_pad].view(2 * Lq, 2 * n_pad), E, n_pad)
+    assert rl2(got, want) <= BOUND + 2.0 ** -17
+    assert float(o32[-1]) == 7.0 and float(osp[-1]) == 7.0
+
+
+def test_masked_keys_and_ragged_segments(lib):
+    from mlx_vlm_b200 import _native as N
+    nh, hd, S = 2, 64, 200
+    q, k, v = (_rand(2 * S, nh * hd, seed=s) for s in (4, 5, 6))
+    mask = torch.rand(2, S, generator=torch.Generator().manual_seed(7)) > 0.4
+    mask[0, :64], mask[1, 64:130], mask[0, 199] = False, False, True       # whole tiles without a key
+    m = mask.to(device="cuda", dtype=torch.uint8)
+    out = torch.empty(2 * S, nh * hd, device="cuda")
+    args = (q.data_ptr(), nh * hd, hd, k.data_ptr(), nh * hd, hd, v.data_ptr(), nh * hd, hd, out.data_ptr(), nh * hd, 0, 0, 0, nh,
+            nh, hd)
+    N.check(lib.b200_attention_f32(*args, S, S, 2, S, S, m.data_ptr(), hd ** -0.5, 0), "attention_f32")
+    torch.cuda.synchronize()
+    for s in (0, 1):
+        sl = slice(s * S, (s + 1) * S)
+        assert rl2(out[sl].double(), _want(q[sl], k[sl], v[sl], nh, nh, hd, m[s].bool())) <= BOUND
+    cuts = [0, 1, 65, 65, 193, 400]
+    cu = torch.tensor(cuts, dtype=torch.int32, device="cuda")
+    N.check(lib.b200_attention_f32_varlen(*args, cu.data_ptr(), len(cuts) - 1, 207, hd ** -0.5, 0), "attention_f32_varlen")
+    torch.cuda.synchronize()
+    for a, b in zip(cuts, cuts[1:]):
+        if b > a:
+            assert rl2(out[a:b].double(), _want(q[a:b], k[a:b], v[a:b], nh, nh, hd)) <= BOUND
