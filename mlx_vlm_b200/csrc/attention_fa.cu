@@ -22,8 +22,8 @@
 // a segment may start at any token (keys are a TMA coordinate without an alignment rule) and a later portion of a prompt
 // reads the cached keys and values where they are.  (V^T, [head][dim][key], is still taken by b200_attention_fa.)
 // Measured against the kernel without TMA that such calls fell back to (attention_tc.cu): 2048 queries behind 2048 cached
-// keys, 28 heads of 128: 1094 -> 354 us; four pictures and a clip of four frames (6012 patches, 16 heads of 80), which start
-// at odd offsets: 773 us in eight launches -> 236 us in one.
+// keys, 28 heads of 128: 1094 -> 354 us (249 with the pairwise softmax below); four pictures and a clip of four frames (6012
+// patches, 16 heads of 80), which start at odd offsets: 773 us in eight launches -> 236 us in one.
 #include <mutex>
 #include <unordered_map>
 
@@ -112,19 +112,44 @@ __device__ __forceinline__ uint32_t f_desc_lo(uint32_t addr) { return ((addr & 0
 __device__ __forceinline__ uint32_t f_desc_lo_mn(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | ((uint32_t)(FA_BLK >> 4) << 16); }
 constexpr uint32_t F_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 
-__device__ __forceinline__ void f_tmem_ld32(uint32_t taddr, uint32_t* r) {
+// (its values may be used after f_ld_wait)
+__device__ __forceinline__ void f_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
 }
+__device__ __forceinline__ void f_ld_wait(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                 "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
+}
+// 64 scores of a row, rounded to bf16, two to a register; those from column `vis` on are -inf
+__device__ __forceinline__ void f_scores(uint32_t taddr, int vis, uint32_t (&pk)[32]) {
+  uint32_t v[2][16];
+  f_ld16(taddr, v[0]);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t(&x)[16] = v[c & 1];
+    f_ld_wait(x);
+    if (c < 3) f_ld16(taddr + (uint32_t)(c + 1) * 16, v[(c + 1) & 1]);
+    if (__any_sync(0xffffffffu, vis < c * 16 + 16)) {
+#pragma unroll
+      for (int e = 0; e < 16; ++e) x[e] = c * 16 + e < vis ? x[e] : 0xff800000u;
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) pk[c * 8 + e] = pack2(__uint_as_float(x[2 * e]), __uint_as_float(x[2 * e + 1]));
+  }
+}
+__device__ __forceinline__ uint32_t f_max2(uint32_t a, uint32_t b) {   // of bf16 pairs
+  uint32_t r;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f_pair(uint32_t x) { return f2(__uint_as_float(x << 16), __uint_as_float(x & 0xffff0000u)); }
 __device__ __forceinline__ void f_tmem_ld16(uint32_t taddr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -152,7 +177,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   if (p_in.segs) {   // static table (written before the producing kernels ran): safe to read ahead of griddepcontrol.wait
     const int4 sg = __ldg(p_in.segs + blockIdx.z);
     p.q0 = sg.x; p.Lq = sg.y; p.k0 = sg.z; p.S = sg.w;
-    if ((int)blockIdx.x * FA_TQ >= p.Lq) return;   // the grid is sized for the longest segment
+    if ((int)(p.causal ? gridDim.y - 1 - blockIdx.y : blockIdx.y) * FA_TQ >= p.Lq) return;   // sized for the longest segment
   }
   extern __shared__ uint8_t fa_smem_raw[];
   __shared__ FaBars bars;
@@ -165,8 +190,9 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint8_t* Vs = sm + 6 * FA_BLK;             // 2 slots x (VT: 2 key-blocks x [hdp d][64 keys], else 2 dim-blocks x [128 keys][64 d])
   uint8_t* Ps = sm + 10 * FA_BLK;            // [128 q][128 keys]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.y, kvh = h / (p.n_heads / p.n_kv);
-  const int row0 = blockIdx.x * FA_TQ;
+  const int h = blockIdx.x, kvh = h / (p.n_heads / p.n_kv);
+  // causal: the query tiles with the most keys start first, of all heads, so that the short ones fill the last wave
+  const int row0 = (p.causal ? gridDim.y - 1 - blockIdx.y : blockIdx.y) * FA_TQ;
   const int S = p.S;
   const int q_last = min(row0 + FA_TQ, p.Lq) - 1;
   const int vis_tile = p.causal ? min(S, S - p.Lq + q_last + 1) : S;
@@ -283,46 +309,40 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int vis = (qi < p.Lq) ? (p.causal ? min(S, S - p.Lq + qi + 1) : S) : S;
     const uint32_t t_row = tmem + ((uint32_t)(q4 * 32) << 16);
     constexpr float LOG2E = 1.4426950408889634f;
-    // The softmax warps are the instruction-bound part of the kernel (2 warps per scheduler, 288+ score
-    // elements per thread and pass), so the inner loops are kept to ~6 instructions per element: bf16
-    // rounding by cvt + shift, one FMA into the exponent, ex2 on the SFU, multiplication by 1/l.
+    // The softmax warps bound the kernel (two warps per scheduler, 64 scores per thread and pass), so they work on pairs: one
+    // cvt rounds two scores, the maximum is taken of bf16 pairs, exponents and sums are f32x2 operations, 4 instructions per
+    // score; the tensor-memory loads of the next 16 columns are in flight meanwhile, and the score tile is free for the next
+    // product as soon as it is in registers.  What is left is the SFU: 128 x 128 exponentials at 16 a cycle per pass.
+    // Measured (element by element -> pairs, with the long query tiles first): 2048 queries behind 2048 keys, 28 heads of
+    // 128: 354 -> 249 us; 8 prompts of about 608 tokens, 32 heads of 128: 154 -> 130; 576 patches, 16 heads of 80: 24 -> 19.
+    const uint64_t log2e = f2(LOG2E, LOG2E);
+    uint32_t pk[32];
     float m = -INFINITY, l = 0.f;
     for (int i = 0; i < n_tiles; ++i) {  // ---- pass 1: row max and sum of exp over bf16 scores ----
       const int s = i & 1;
       f_wait(&bars.s_full[s], (i >> 1) & 1, dead);
+      __syncwarp();
       f_fence_after();
-      const int jbase = i * FA_TK + half * 64;
-#pragma unroll 1
-      for (int c0 = 0; c0 < 64; c0 += 32) {
-        uint32_t r[32];
-        f_tmem_ld32(t_row + (uint32_t)(s * 128 + half * 64 + c0), r);
-        float sc[32];
-        float cm = -INFINITY;
-        if (jbase + c0 + 32 <= vis) {  // whole chunk visible: no per-element mask
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            sc[e] = rbf(__uint_as_float(r[e]));
-            cm = fmaxf(cm, sc[e]);
-          }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            sc[e] = (jbase + c0 + e < vis) ? rbf(__uint_as_float(r[e])) : -INFINITY;
-            cm = fmaxf(cm, sc[e]);
-          }
-        }
-        if (cm > -INFINITY) {
-          const float mn = fmaxf(m, cm);
-          const float nb = -mn * LOG2E;
-          float add = 0.f;
-#pragma unroll
-          for (int e = 0; e < 32; ++e) add += f_ex2(fmaf(sc[e], LOG2E, nb));
-          l = l * f_ex2((m - mn) * LOG2E) + add;
-          m = mn;
-        }
-      }
+      f_scores(t_row + (uint32_t)(s * 128 + half * 64), vis - (i * FA_TK + half * 64), pk);
       f_fence_before();
       f_arrive(&bars.s_empty[s]);
+      uint32_t mx = pk[0];
+#pragma unroll
+      for (int e = 1; e < 32; ++e) mx = f_max2(mx, pk[e]);
+      const float cm = fmaxf(__uint_as_float(mx << 16), __uint_as_float(mx & 0xffff0000u));
+      if (cm > -INFINITY) {
+        const float mn = fmaxf(m, cm);
+        const uint64_t nb = f2(-mn * LOG2E, -mn * LOG2E);
+        uint64_t add[2] = {0ull, 0ull};
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+          const uint64_t x = fma2(f_pair(pk[e]), log2e, nb);
+          add[e & 1] = add2(add[e & 1], f2(f_ex2(f2_lo(x)), f_ex2(f2_hi(x))));
+        }
+        add[0] = add2(add[0], add[1]);
+        l = l * f_ex2((m - mn) * LOG2E) + (f2_lo(add[0]) + f2_hi(add[0]));
+        m = mn;
+      }
     }
     stat[half][row] = make_float2(m, l);
     f_sbar();
@@ -332,35 +352,26 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       l = (a.y > 0.f ? a.y * f_ex2((a.x - m) * LOG2E) : 0.f) + (b.y > 0.f ? b.y * f_ex2((b.x - m) * LOG2E) : 0.f);
     }
     const float inv_l = 1.0f / l;
-    const float nbm = -m * LOG2E;
+    const uint64_t nbm = f2(-m * LOG2E, -m * LOG2E), inv2 = f2(inv_l, inv_l);
     for (int j = 0; j < n_tiles; ++j) {  // ---- pass 2: p = bf16(exp(s - m) / l) -> shared memory ----
       const int i = n_tiles + j, s = i & 1;
       f_wait(&bars.s_full[s], (i >> 1) & 1, dead);
+      __syncwarp();
       f_fence_after();
-      f_wait(&bars.p_empty, (j & 1) ^ 1, dead);  // the previous P.V has consumed the P tile
-      uint8_t* prow = Ps + half * FA_BLK + row * 128;
-      const int jbase = j * FA_TK + half * 64;
-#pragma unroll 1
-      for (int c0 = 0; c0 < 64; c0 += 32) {
-        uint32_t r[32];
-        f_tmem_ld32(t_row + (uint32_t)(s * 128 + half * 64 + c0), r);
-        const bool full = jbase + c0 + 32 <= vis;
-#pragma unroll
-        for (int e = 0; e < 32; e += 8) {
-          float pv[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const float pe = f_ex2(fmaf(rbf(__uint_as_float(r[e + u])), LOG2E, nbm)) * inv_l;
-            pv[u] = (full || jbase + c0 + e + u < vis) ? pe : 0.f;
-          }
-          uint4 o;
-          o.x = pack2(pv[0], pv[1]); o.y = pack2(pv[2], pv[3]); o.z = pack2(pv[4], pv[5]); o.w = pack2(pv[6], pv[7]);
-          const int chunk = (c0 + e) >> 3;
-          *reinterpret_cast<uint4*>(prow + ((chunk ^ (row & 7)) << 4)) = o;
-        }
-      }
+      f_scores(t_row + (uint32_t)(s * 128 + half * 64), vis - (j * FA_TK + half * 64), pk);
       f_fence_before();
       f_arrive(&bars.s_empty[s]);
+#pragma unroll
+      for (int e = 0; e < 32; ++e) {
+        const uint64_t x = fma2(f_pair(pk[e]), log2e, nbm);
+        const uint64_t w = mul2(f2(f_ex2(f2_lo(x)), f_ex2(f2_hi(x))), inv2);
+        pk[e] = pack2(f2_lo(w), f2_hi(w));
+      }
+      f_wait(&bars.p_empty, (j & 1) ^ 1, dead);  // the previous P.V has consumed the P tile
+      uint8_t* prow = Ps + half * FA_BLK + row * 128;
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        *reinterpret_cast<uint4*>(prow + ((c ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
       if constexpr (!VT) {
         // V rows behind the segment's last key (another segment's, or a cache's unused rows) meet p = 0, but 0 times a NaN
         // or an infinity would still reach O: those of the last group of 16 keys that is multiplied are cleared
@@ -533,7 +544,7 @@ int attention_fa(const void* q, long q_ts, long q_hs, const void* k, long k_ts, 
   p.out = (bf16*)out; p.o_ts = o_ts; p.n_heads = n_heads; p.n_kv = n_kv; p.hd = hd; p.hdp = hdp;
   p.Lq = Lq; p.S = S; p.causal = causal; p.q0 = q0; p.k0 = k0;
   p.segs = (const int4*)segs;
-  B200_CUDA(launch_pdl(kern, dim3(cdiv(Lq, FA_TQ), n_heads, segs ? n_seg : 1), dim3(FA_THREADS), smem, st, tq, tk, tv, p));
+  B200_CUDA(launch_pdl(kern, dim3(n_heads, cdiv(Lq, FA_TQ), segs ? n_seg : 1), dim3(FA_THREADS), smem, st, tq, tk, tv, p));
   return B200_OK;
 }
 
