@@ -214,7 +214,7 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
                   const WtExt* ext = nullptr);
 int finish_rows(const float* P, int S, const void* bias, const void* resid, long ldr, void* h_out,
                 long ldh, int norm_kind, const void* nw, const void* nb, float eps, void* xn, long ldx,
-                int T, int N, cudaStream_t st, const void* l2_prefetch = nullptr, long l2_prefetch_bytes = 0);
+                int T, int N, cudaStream_t st);
 void gemm_wt_set_pdl(bool on);
 // fp32 attention of the towers (attention_f32_tc.cu)
 struct AttnF32P {

@@ -25,8 +25,6 @@ namespace b200 {
 
 namespace {
 
-constexpr int BD_AG_MAX = 4;  // q heads per attention CTA: 4, 2 or 1 — the smallest that keeps the grid within one wave
-
 __device__ __forceinline__ void bd_pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void bd_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -77,7 +75,15 @@ __global__ void __launch_bounds__(256) bd_begin_kernel(const int* __restrict__ t
   bd_embed_norm_row(embed, tok[b], H, lnw, eps, h + (long)b * H, xn + (long)b * H, red);
 }
 
-// ---- attention of one (row, kv head, q-head part): finishes q/k/v from the qkv partials ----------
+// ---- attention of one (row, kv head, part of its q heads): finishes q/k/v from the qkv partials -----------------
+// A cluster of up to 8 CTAs shares the row's keys (contiguous ranges in units of 16).  Each CTA brings its keys, then its
+// values, through a ring of 128-row slots (cp.async: everything of a row of up to 384 keys per CTA is in flight while q is
+// still being finished), multiplies them on mma.sync with keys (scores) or dims (P.V) on the M side and up to 8 q heads on
+// the N side (operands are bf16 by definition here, accumulators fp32), and meets the others twice in distributed shared
+// memory: for the softmax's maximum and sum (p is rounded after the division, so both are needed first) and for the sum of
+// the partial outputs, in rank order.  Bound by its chain of dependent steps, not by bytes.  Measured against one CTA per part
+// of the heads that read the whole row through registers, a layer: 5 rows of 1025 - 3777 keys, 2 kv heads: 71 -> 22 us; 8 rows
+// of 272 - 784, 4 kv heads: 27 -> 17.
 struct BdAttnP {
   const float* P;     // [S][B][QKV] fp32 split-K partials of the qkv GEMM
   int S, B, QKV;
@@ -90,255 +96,302 @@ struct BdAttnP {
   bf16* out;          // [B][n_heads*hd]
   int n_heads, n_kv, cap, hsplit;
   float scale_bf;
-  // weights of the GEMMs that follow (o_proj, gate/up, down): this kernel is a chain of dependent round trips that
-  // leaves HBM idle, so its CTAs ask the L2 for them up front (l2_prefetch_span; weights are static during a step)
-  const void* pf[3];
-  long pf_bytes[3];
 };
 
-template <int HD, int AG>
+constexpr int BA_HEADS = 8;     // q heads of a CTA: the N side of the products
+constexpr int BA_ROWS = 128;    // keys of a ring slot: 16 per warp
+constexpr int BA_SLOTS = 3;
+
+__device__ __forceinline__ uint32_t ba_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void ba_ldm4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ba_ldm4t(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ba_ldm2t(uint32_t addr, uint32_t& a, uint32_t& b) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(a), "=r"(b) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ba_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ba_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ba_peer(const float* p, int rank) {   // *p of the cluster's CTA `rank`
+  uint32_t addr;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(ba_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+// byte offset of (row, 16-byte chunk) in a slot: the eight rows of an ldmatrix hit different banks
+template <int HD>
+__device__ __forceinline__ uint32_t ba_off(int row, int chunk) {
+  return (uint32_t)(row * HD * 2 + ((chunk ^ (row & 7)) << 4));
+}
+static __host__ __device__ __forceinline__ int ba_share(int keys, int ranks) { return (keys + 16 * ranks - 1) / (16 * ranks) * 16; }
+
+template <int HD>
 __global__ void __launch_bounds__(256) bd_attn_kernel(const BdAttnP p) {
   bd_pdl_launch();
-  if (threadIdx.x == 0) {
-    const int n = gridDim.x * gridDim.y, id = blockIdx.y * gridDim.x + blockIdx.x;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-      if (p.pf_bytes[i] > 0) l2_prefetch_span(p.pf[i], p.pf_bytes[i], id, n);
-  }
-  extern __shared__ __align__(16) uint8_t bd_sm[];
-  constexpr int NCH = HD / 8, half = HD / 2;
-  constexpr int SEG = HD / 8;   // dims per lane in the P.V phase (lane = key sub-index x dim segment)
-  constexpr int NV = SEG / 8;   // 16-byte vectors per lane and key
-  constexpr int VU = 8;         // key trips in flight per warp in the P.V phase (32 keys)
-  constexpr int PMAX = 12;      // split-K partials summed with all loads in flight
-  float* qs = reinterpret_cast<float*>(bd_sm);  // [AG][HD] q * scale (rotated)
-  float* kn = qs + AG * HD;                     // [HD] new key (rotated)
-  float* vn = kn + HD;                          // [HD] new value
-  float* sc = vn + HD;                          // [AG][cap]
-  float* red = sc + (long)AG * p.cap;           // [8][AG*HD]
-  __shared__ float s_m[8][AG], s_l[8][AG];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.y;
+  constexpr int SLOT = BA_ROWS * HD * 2, NCH = HD / 8, half = HD / 2, QP = HD + 8;
+  extern __shared__ __align__(128) uint8_t bd_sm[];
+  uint8_t* ring = bd_sm;                                            // [BA_SLOTS][128 keys][HD] bf16
+  bf16* ps = reinterpret_cast<bf16*>(bd_sm + BA_SLOTS * SLOT);      // [keys of this CTA][8]: scores, then p
+  __shared__ float qf[BA_HEADS][HD], kn[HD], vn[HD];
+  __shared__ __align__(16) bf16 qs[BA_HEADS][QP];
+  __shared__ float wstat[8][BA_HEADS], own[2][BA_HEADS], all[2][8][BA_HEADS], part[HD * BA_HEADS];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int C = gridDim.x, rank = blockIdx.x, row = blockIdx.z;     // the cluster is the x extent
   const int Gall = p.n_heads / p.n_kv;
-  const int Gc = (Gall + p.hsplit - 1) / p.hsplit;
-  const int kvh = blockIdx.x / p.hsplit, part = blockIdx.x % p.hsplit;
-  const int G = min(Gc, Gall - part * Gc);
-  const int h0 = kvh * Gall + part * Gc;
+  const int kvh = blockIdx.y / p.hsplit, hp = blockIdx.y % p.hsplit;
+  const int G = min(BA_HEADS, Gall - hp * BA_HEADS), h0 = kvh * Gall + hp * BA_HEADS;
   bf16* kb = p.kv + (long)row * p.row_stride + (long)kvh * p.cap * HD;
   bf16* vb = kb + p.v_off;
   bd_pdl_wait();
   const int ctx = p.ctx[row], pos = p.pos[row];
-  const int nkeys = ctx + 1;
-  // Every dependent global round trip costs ~1 us here, so the requests are issued as early as their
-  // addresses are known: the first block of cached keys (one row per lane) goes out BEFORE the
-  // split-K partials of q/k/v are summed, the first block of values before the softmax.
-  uint4 kfirst[NCH];
-  {
-    const int j = warp * 32 + lane;
-    const uint4* kr = reinterpret_cast<const uint4*>(kb + (long)j * HD);
-#pragma unroll
-    for (int c = 0; c < NCH; ++c) kfirst[c] = (j < ctx) ? __ldcg(kr + c) : make_uint4(0, 0, 0, 0);
-  }
-  // ---- finish q (G heads), k, v of this step: sum of the split-K partials + bias, one rounding ----
-  for (int i = threadIdx.x; i < (G + 2) * HD; i += 256) {
-    const int slot = i / HD, j = i % HD;
-    const int n = (slot < G ? (h0 + slot) : (slot == G ? p.n_heads + kvh : p.n_heads + p.n_kv + kvh)) * HD + j;
-    float a = 0.f;
-    for (int s0 = 0; s0 < p.S; s0 += PMAX) {
-      float v[PMAX];
-#pragma unroll
-      for (int u = 0; u < PMAX; ++u)
-        v[u] = (s0 + u < p.S) ? __ldcg(p.P + ((long)(s0 + u) * p.B + row) * p.QKV + n) : 0.f;
-#pragma unroll
-      for (int u = 0; u < PMAX; ++u) a += v[u];
+  const int nkeys = ctx + 1, share = ba_share(nkeys, C);
+  const int j0 = min(rank * share, nkeys), n_own = min(share, nkeys - j0);   // this CTA's keys
+  const int n = (n_own + BA_ROWS - 1) / BA_ROWS;                             // slots of keys, then as many of values
+  // step i < n: keys of slot i; else values of slot i - n.  One commit group per step, also past the end.
+  auto issue = [&](int i) {
+    if (i < 2 * n) {
+      const int first = (i < n ? i : i - n) * BA_ROWS;
+      const bf16* src = (i < n ? kb : vb) + (long)(j0 + first) * HD;
+      const uint32_t dst = ba_u32(ring + (i % BA_SLOTS) * SLOT);
+      const int rows = min(BA_ROWS, n_own - first);
+      for (int c = tid; c < BA_ROWS * NCH; c += 256) {
+        const int r = c / NCH, ch = c % NCH;
+        if (r >= ((rows + 15) & ~15)) break;
+        const bool ok = r < rows && j0 + first + r < ctx;   // (the new key is not cached yet: zeros, patched below)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + ba_off<HD>(r, ch)),
+                     "l"(src + (ok ? (long)r * HD + ch * 8 : 0)), "r"(ok ? 16 : 0)
+                     : "memory");
+      }
     }
-    a = rbf(a + bf2f(p.bias[n]));
-    (slot < G ? qs + slot * HD : (slot == G ? kn : vn))[j] = a;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int i = 0; i < BA_SLOTS; ++i) issue(i);
+  // ---- finish q (G heads), k, v of this step: sum of the split-K partials in split order + bias, one rounding ----
+  constexpr int ITEMS = (BA_HEADS + 2) * (HD / 4), NI = (ITEMS + 255) / 256;   // 4 elements each, the loads of all in flight
+  float4 a[NI], v[NI][8];
+  int at[NI];
+#pragma unroll
+  for (int u = 0; u < NI; ++u) {
+    const int i = tid + u * 256, slot = i / (HD / 4);
+    const bool use = i < ITEMS && (slot < G || slot >= BA_HEADS);
+    at[u] = !use ? -1 : (slot < G ? h0 + slot : (slot == BA_HEADS ? p.n_heads + kvh : p.n_heads + p.n_kv + kvh)) * HD + i % (HD / 4) * 4;
+    a[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  for (int s0 = 0; s0 < p.S; s0 += 8) {
+#pragma unroll
+    for (int u = 0; u < NI; ++u)
+#pragma unroll
+      for (int w = 0; w < 8; ++w)
+        v[u][w] = s0 + w < p.S && at[u] >= 0
+                      ? __ldcg(reinterpret_cast<const float4*>(p.P + ((long)(s0 + w) * p.B + row) * p.QKV + at[u]))
+                      : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < NI; ++u)
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        a[u].x += v[u][w].x; a[u].y += v[u][w].y; a[u].z += v[u][w].z; a[u].w += v[u][w].w;
+      }
+  }
+  // (the angle of this thread's rotary pairs: 256 is a multiple of HD / 2)
+  const float ang = (float)pos * p.inv_freq[tid % half];
+  const float cs = rbf(cosf(ang)), sn = rbf(sinf(ang));
+#pragma unroll
+  for (int u = 0; u < NI; ++u) {
+    const int i = tid + u * 256, slot = i / (HD / 4), j = i % (HD / 4) * 4;
+    if (i >= ITEMS) continue;
+    if (at[u] >= 0) {
+      float bb[4];
+      unpack4(*reinterpret_cast<const uint2*>(p.bias + at[u]), bb);
+      a[u] = make_float4(rbf(a[u].x + bb[0]), rbf(a[u].y + bb[1]), rbf(a[u].z + bb[2]), rbf(a[u].w + bb[3]));
+    }
+    *reinterpret_cast<float4*>((slot < BA_HEADS ? qf[slot] : (slot == BA_HEADS ? kn : vn)) + j) = a[u];
   }
   __syncthreads();
   // M-RoPE at a decode position: the three axes carry the same position (language.py:476-509)
-  for (int i = threadIdx.x; i < (G + 1) * half; i += 256) {
+  for (int i = tid; i < (BA_HEADS + 1) * half; i += 256) {
     const int slot = i / half, j = i % half;
-    float* v = slot < G ? qs + slot * HD : kn;
+    float* v = slot < BA_HEADS ? qf[slot] : kn;
     const float y1 = v[j], y2 = v[j + half];
-    const float ang = (float)pos * p.inv_freq[j];
-    const float c = rbf(cosf(ang)), sn = rbf(sinf(ang));
-    float o1 = rbf(rbf(y1 * c) + rbf((-y2) * sn));
-    float o2 = rbf(rbf(y2 * c) + rbf(y1 * sn));
-    if (slot < G) {
-      o1 = rbf(o1 * p.scale_bf);
-      o2 = rbf(o2 * p.scale_bf);
+    const float o1 = rbf(rbf(y1 * cs) + rbf((-y2) * sn)), o2 = rbf(rbf(y2 * cs) + rbf(y1 * sn));
+    if (slot < BA_HEADS) {
+      qs[slot][j] = f2bf(o1 * p.scale_bf);
+      qs[slot][j + half] = f2bf(o2 * p.scale_bf);
+    } else {
+      kn[j] = o1;
+      kn[j + half] = o2;
     }
-    v[j] = o1;
-    v[j + half] = o2;
   }
-  for (int i = threadIdx.x + G * HD; i < AG * HD; i += 256) qs[i] = 0.f;
   __syncthreads();
-  if (part == 0) {  // append the new position to the row's cache (one CTA per kv head)
-    for (int i = threadIdx.x; i < HD; i += 256) {
+  if (hp == 0 && rank == 0) {  // append the new position to the row's cache
+    for (int i = tid; i < HD; i += 256) {
       kb[(long)ctx * HD + i] = f2bf(kn[i]);
       vb[(long)ctx * HD + i] = f2bf(vn[i]);
     }
   }
-  // ---- scores: lane <-> key; cached keys from global, the new key from shared memory ----
-  float lm[AG];
+  uint32_t qb[HD / 32][4];   // q as the B operand: heads x 32 dims each
 #pragma unroll
-  for (int g = 0; g < AG; ++g) lm[g] = -INFINITY;
-  for (int j0 = warp * 32; j0 < nkeys; j0 += 256) {
-    const int j = j0 + lane;
-    uint4 kv[NCH];
-    if (j0 == warp * 32) {
-#pragma unroll
-      for (int c = 0; c < NCH; ++c) kv[c] = kfirst[c];
-    } else if (j < ctx) {
-      const uint4* kr = reinterpret_cast<const uint4*>(kb + (long)j * HD);
-#pragma unroll
-      for (int c = 0; c < NCH; ++c) kv[c] = __ldcg(kr + c);
+  for (int k = 0; k < HD / 32; ++k) ba_ldm4(ba_u32(&qs[lane & 7][k * 32 + (lane >> 3) * 8]), qb[k]);
+  // the slot of step i has landed; the new key / value goes in by hand
+  auto arrived = [&](int i) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(BA_SLOTS - 1) : "memory");
+    const int r = ctx - j0 - (i < n ? i : i - n) * BA_ROWS;
+    if (r >= 0 && r < BA_ROWS && ctx - j0 < n_own) {
+      __syncthreads();   // (the row's zeros have landed for every thread)
+      for (int d = tid; d < HD; d += 256)
+        *reinterpret_cast<bf16*>(ring + (i % BA_SLOTS) * SLOT + ba_off<HD>(r, d >> 3) + (d & 7) * 2) = f2bf((i < n ? kn : vn)[d]);
     }
-    if (j < nkeys) {
-      if (j == ctx) {
+    __syncthreads();
+  };
+  for (int i = 0; i < n; ++i) {   // ---- scores: D[16 keys][8 heads] per warp ----
+    arrived(i);
+    const int k0 = i * BA_ROWS + warp * 16;
+    if (k0 < n_own) {
+      const uint32_t slot = ba_u32(ring + (i % BA_SLOTS) * SLOT);
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int c = 0; c < NCH; ++c) {
-          kv[c].x = pack2(kn[c * 8 + 0], kn[c * 8 + 1]); kv[c].y = pack2(kn[c * 8 + 2], kn[c * 8 + 3]);
-          kv[c].z = pack2(kn[c * 8 + 4], kn[c * 8 + 5]); kv[c].w = pack2(kn[c * 8 + 6], kn[c * 8 + 7]);
-        }
+      for (int k = 0; k < HD / 16; ++k) {
+        uint32_t a[4];
+        ba_ldm4(slot + ba_off<HD>(warp * 16 + (lane & 15), k * 2 + (lane >> 4)), a);
+        ba_mma(d, a, qb[k >> 1][(k & 1) * 2], qb[k >> 1][(k & 1) * 2 + 1]);
       }
-      float s[AG][2];
-#pragma unroll
-      for (int g = 0; g < AG; ++g) s[g][0] = s[g][1] = 0.f;
-#pragma unroll
-      for (int c = 0; c < NCH; ++c) {
-        float kf[8];
-        unpack8(kv[c], kf);
-#pragma unroll
-        for (int g = 0; g < AG; ++g) {
-          const float4 a = *reinterpret_cast<const float4*>(qs + g * HD + c * 8);
-          const float4 b = *reinterpret_cast<const float4*>(qs + g * HD + c * 8 + 4);
-          s[g][0] = fmaf(a.x, kf[0], fmaf(a.y, kf[1], fmaf(a.z, kf[2], fmaf(a.w, kf[3], s[g][0]))));
-          s[g][1] = fmaf(b.x, kf[4], fmaf(b.y, kf[5], fmaf(b.z, kf[6], fmaf(b.w, kf[7], s[g][1]))));
-        }
-      }
-#pragma unroll
-      for (int g = 0; g < AG; ++g) {
-        const float r = rbf(s[g][0] + s[g][1]);
-        sc[(long)g * p.cap + j] = r;
-        lm[g] = fmaxf(lm[g], r);
-      }
+      const int r = k0 + (lane >> 2), c = (lane & 3) * 2;
+      *reinterpret_cast<uint32_t*>(ps + r * BA_HEADS + c) = r < n_own ? pack2(d[0], d[1]) : 0xff80ff80u;
+      *reinterpret_cast<uint32_t*>(ps + (r + 8) * BA_HEADS + c) = r + 8 < n_own ? pack2(d[2], d[3]) : 0xff80ff80u;
     }
+    __syncthreads();
+    issue(i + BA_SLOTS);
   }
-  // first block of values: warp w, trip q, key = 32 * w + 4 * q + ksub; lane = (ksub, dim segment)
-  const int seg = lane & 7, ksub = lane >> 3;
-  uint4 vfirst[VU][NV];
+  // ---- maximum and sum of this CTA's keys, then of the row's ----
+  const int n16 = (n_own + 15) & ~15;
+  float m[BA_HEADS], l[BA_HEADS];
 #pragma unroll
-  for (int q = 0; q < VU; ++q) {
-    const int j = warp * 32 + q * 4 + ksub;
+  for (int g = 0; g < BA_HEADS; ++g) m[g] = -INFINITY;
+  for (int j = tid; j < n16; j += 256) {
+    float f[8];
+    unpack8(*reinterpret_cast<const uint4*>(ps + j * BA_HEADS), f);
 #pragma unroll
-    for (int v = 0; v < NV; ++v)
-      vfirst[q][v] = (j < ctx) ? __ldcg(reinterpret_cast<const uint4*>(vb + (long)j * HD + seg * SEG + v * 8))
-                               : make_uint4(0, 0, 0, 0);
+    for (int g = 0; g < BA_HEADS; ++g) m[g] = fmaxf(m[g], f[g]);
   }
 #pragma unroll
-  for (int g = 0; g < AG; ++g) {
-    lm[g] = warp_max(lm[g]);
-    if (lane == 0) s_m[warp][g] = lm[g];
+  for (int g = 0; g < BA_HEADS; ++g) {
+    m[g] = warp_max(m[g]);
+    if (lane == 0) wstat[warp][g] = m[g];
   }
   __syncthreads();
-  float M[AG], ls[AG];
 #pragma unroll
-  for (int g = 0; g < AG; ++g) {
-    float m = -INFINITY;
+  for (int g = 0; g < BA_HEADS; ++g) {
+    m[g] = wstat[0][g];
 #pragma unroll
-    for (int w = 0; w < 8; ++w) m = fmaxf(m, s_m[w][g]);
-    M[g] = m;
-    ls[g] = 0.f;
+    for (int w = 1; w < 8; ++w) m[g] = fmaxf(m[g], wstat[w][g]);
+    l[g] = 0.f;
   }
-  for (int j = threadIdx.x; j < nkeys; j += 256) {
+  for (int j = tid; j < n16; j += 256) {
+    float f[8];
+    unpack8(*reinterpret_cast<const uint4*>(ps + j * BA_HEADS), f);
 #pragma unroll
-    for (int g = 0; g < AG; ++g) {
-      const float e = expf(sc[(long)g * p.cap + j] - M[g]);
-      sc[(long)g * p.cap + j] = e;
-      ls[g] += e;
-    }
-  }
-#pragma unroll
-  for (int g = 0; g < AG; ++g) {
-    ls[g] = warp_sum(ls[g]);
-    if (lane == 0) s_l[warp][g] = ls[g];
+    for (int g = 0; g < BA_HEADS; ++g) l[g] += expf(f[g] - m[g]);
   }
   __syncthreads();
-  float L[AG];
 #pragma unroll
-  for (int g = 0; g < AG; ++g) {
-    float l = 0.f;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) l += s_l[w][g];
-    L[g] = l;
-  }
-  for (int j = threadIdx.x; j < nkeys; j += 256) {
-#pragma unroll
-    for (int g = 0; g < AG; ++g) sc[(long)g * p.cap + j] = rbf(sc[(long)g * p.cap + j] / L[g]);
+  for (int g = 0; g < BA_HEADS; ++g) {
+    l[g] = warp_sum(l[g]);
+    if (lane == 0) wstat[warp][g] = l[g];
   }
   __syncthreads();
-  // ---- P.V: 256 keys per CTA iteration, 8 x NV 16-byte loads in flight per lane ----
-  float acc[AG][SEG];
+  if (tid < BA_HEADS) {
+    float t = 0.f;
 #pragma unroll
-  for (int g = 0; g < AG; ++g)
+    for (int w = 0; w < 8; ++w) t += wstat[w][tid];
+    own[1][tid] = t;
+  }
+  if (tid == 0) {
 #pragma unroll
-    for (int e = 0; e < SEG; ++e) acc[g][e] = 0.f;
-  for (int j0 = 0; j0 < nkeys; j0 += 256) {
-    uint4 vv[VU][NV];
+    for (int g = 0; g < BA_HEADS; ++g) own[0][g] = m[g];
+  }
+  ba_cluster_sync();
+  if (tid < 16 * C) {
+    const int r = tid >> 4, w = (tid >> 3) & 1, g = tid & 7;
+    all[w][r][g] = ba_peer(&own[w][g], r);
+  }
+  __syncthreads();
 #pragma unroll
-    for (int q = 0; q < VU; ++q) {
-      const int j = j0 + warp * 32 + q * 4 + ksub;
+  for (int g = 0; g < BA_HEADS; ++g) {
+    float M = all[0][0][g];
+    for (int r = 1; r < C; ++r) M = fmaxf(M, all[0][r][g]);
+    float L = 0.f;
+    for (int r = 0; r < C; ++r) L += all[0][r][g] > -INFINITY ? all[1][r][g] * expf(all[0][r][g] - M) : 0.f;
+    m[g] = M;
+    l[g] = L;
+  }
+  for (int j = tid; j < n16; j += 256) {
+    uint4* at = reinterpret_cast<uint4*>(ps + j * BA_HEADS);
+    float f[8];
+    unpack8(*at, f);
 #pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        if (j0 == 0) vv[q][v] = vfirst[q][v];
-        else vv[q][v] = (j < ctx) ? __ldcg(reinterpret_cast<const uint4*>(vb + (long)j * HD + seg * SEG + v * 8))
-                                  : make_uint4(0, 0, 0, 0);
+    for (int g = 0; g < BA_HEADS; ++g) f[g] = expf(f[g] - m[g]) / l[g];
+    *at = make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
+  }
+  // ---- P.V: D[16 dims][8 heads] x HD / 16 per warp over its keys ----
+  float acc[HD / 16][4];
+#pragma unroll
+  for (int t = 0; t < HD / 16; ++t)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[t][e] = 0.f;
+  for (int i = n; i < 2 * n; ++i) {
+    arrived(i);
+    const int k0 = (i - n) * BA_ROWS + warp * 16;
+    if (k0 < n_own) {
+      const uint32_t slot = ba_u32(ring + (i % BA_SLOTS) * SLOT);
+      uint32_t b0, b1;
+      ba_ldm2t(ba_u32(ps + (k0 + (lane & 15)) * BA_HEADS), b0, b1);
+      const int r = warp * 16 + ((lane >> 4) << 3) + (lane & 7);
+#pragma unroll
+      for (int t = 0; t < HD / 16; ++t) {
+        uint32_t a[4];
+        ba_ldm4t(slot + ba_off<HD>(r, t * 2 + ((lane >> 3) & 1)), a);
+        ba_mma(acc[t], a, b0, b1);
       }
     }
-#pragma unroll
-    for (int q = 0; q < VU; ++q) {
-      const int j = j0 + warp * 32 + q * 4 + ksub;
-      if (j < nkeys) {
-        float pj[AG];
-#pragma unroll
-        for (int g = 0; g < AG; ++g) pj[g] = sc[(long)g * p.cap + j];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-          float vf[8];
-          if (j == ctx) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) vf[e] = rbf(vn[seg * SEG + v * 8 + e]);
-          } else {
-            unpack8(vv[q][v], vf);
-          }
-#pragma unroll
-          for (int g = 0; g < AG; ++g)
-#pragma unroll
-            for (int e = 0; e < 8; ++e) acc[g][v * 8 + e] = fmaf(pj[g], vf[e], acc[g][v * 8 + e]);
-        }
-      }
-    }
+    __syncthreads();
+    issue(i + BA_SLOTS);
   }
-  // sum over the 4 key sub-indices of the warp, then over the 8 warps through shared memory
-#pragma unroll
-  for (int g = 0; g < AG; ++g)
-#pragma unroll
-    for (int e = 0; e < SEG; ++e) {
-      float a = acc[g][e];
-      a += __shfl_xor_sync(0xffffffffu, a, 8);
-      a += __shfl_xor_sync(0xffffffffu, a, 16);
-      if (ksub == 0) red[((long)warp * AG + g) * HD + seg * SEG + e] = a;
-    }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  bf16* orow = p.out + (long)row * p.n_heads * HD + (long)h0 * HD;
-  for (int i = threadIdx.x; i < G * HD; i += 256) {
-    float s = 0.f;
+  float* red = reinterpret_cast<float*>(ring);   // [8 warps][HD dims][8 heads]
 #pragma unroll
-    for (int w = 0; w < 8; ++w) s += red[(long)w * AG * HD + i];
-    orow[i] = f2bf(s);
+  for (int t = 0; t < HD / 16; ++t) {
+    const int d = t * 16 + (lane >> 2), c = (lane & 3) * 2;
+    *reinterpret_cast<float2*>(red + ((long)warp * HD + d) * BA_HEADS + c) = make_float2(acc[t][0], acc[t][1]);
+    *reinterpret_cast<float2*>(red + ((long)warp * HD + d + 8) * BA_HEADS + c) = make_float2(acc[t][2], acc[t][3]);
   }
+  __syncthreads();
+  for (int i = tid; i < HD * BA_HEADS; i += 256) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += red[w * HD * BA_HEADS + i];
+    part[i] = t;
+  }
+  ba_cluster_sync();
+  // each CTA adds up and stores its share of the dims
+  const int dims = (HD + C - 1) / C, d0 = rank * dims, dn = min(dims, HD - d0);
+  for (int i = tid; i < G * dn; i += 256) {
+    const int g = i / dn, d = d0 + i % dn;
+    float t = 0.f;
+    for (int r = 0; r < C; ++r) t += ba_peer(&part[d * BA_HEADS + g], r);
+    p.out[(long)row * p.n_heads * HD + (long)(h0 + g) * HD + d] = f2bf(t);
+  }
+  ba_cluster_sync();   // nobody leaves while its memory is read
 }
 
 // ---- sampler + state update + next embedding, one CTA per row ------------------------------------
@@ -531,42 +584,40 @@ static int bd_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
   return B200_OK;
 }
 
-static size_t bd_attn_smem(const DecodeDims& d, int ag) {
-  return ((size_t)(ag + 2) * d.hd + (size_t)ag * d.cap + (size_t)8 * ag * d.hd) * 4;
+static size_t bd_attn_smem(const DecodeDims& d, int ranks) {
+  const int slots = cdiv(ba_share(d.cap, ranks), BA_ROWS);
+  return (size_t)BA_SLOTS * BA_ROWS * d.hd * 2 + (size_t)slots * BA_ROWS * BA_HEADS * 2;
 }
 
-// q heads per attention CTA: the latency chain of a CTA (partials -> rope -> keys -> softmax -> values) does not
-// shrink with fewer heads, its arithmetic does; so use as many CTAs as fit one wave of the SMs
-static int bd_attn_heads_per_cta(const DecodeDims& d, int B, int sm_count) {
-  const int Gall = d.n_heads / d.n_kv;
-  for (int ag : {1, 2, 4})
-    if ((long)d.n_kv * ((Gall + ag - 1) / ag) * B <= sm_count) return ag;
-  return BD_AG_MAX;
+// CTAs of a row's cluster: as many as one wave holds at one per SM (two leave no room for the next GEMM, whose weights are on
+// their way while this kernel runs: 8 rows of 272 - 784 keys, 4 kv heads: 20 us a layer instead of 27, and the step no
+// shorter), and no fewer than the scores of the longest row need shared memory for
+static int bd_attn_ranks(const DecodeDims& d, int B, int sm_count) {
+  const long groups = (long)d.n_kv * cdiv(d.n_heads / d.n_kv, BA_HEADS) * B;
+  int ranks = 1;
+  for (int r : {2, 4, 8})
+    if (groups * r <= sm_count) ranks = r;
+  while (ranks < 8 && bd_attn_smem(d, ranks) > 200 * 1024) ranks *= 2;
+  return ranks;
 }
 
 template <int HD>
-static int bd_attn_launch(int ag, dim3 grid, size_t smem, cudaStream_t s, const BdAttnP& ap) {
-  switch (ag) {
-    case 1: return bd_launch(bd_attn_kernel<HD, 1>, grid, dim3(256), smem, s, ap);
-    case 2: return bd_launch(bd_attn_kernel<HD, 2>, grid, dim3(256), smem, s, ap);
-    default: return bd_launch(bd_attn_kernel<HD, 4>, grid, dim3(256), smem, s, ap);
-  }
-}
-
-// L2 prefetch budget of the latency-bound kernels of a step, in bytes (B200_BD_PREFETCH_MB).  DEFAULT 0 = off: measured on
-// C5 (Qwen2-VL-7B, 8 rows) the step got SLOWER with it — 3.672 ms off, 3.745 ms at 60 MB, 3.804 ms at 96 MB
-// (profiles/r2_bd_l2_prefetch_ab.txt): the prefetch traffic lengthens the attention kernel's dependent round trips by
-// more than the L2-resident weights save the GEMMs.  Kept as a tuning knob.
-static long bd_prefetch_budget() {
-  static long v = -1;
-  if (v < 0) {
-    const char* e = getenv("B200_BD_PREFETCH_MB");
-    long mb = e ? atol(e) : 0;
-    if (mb < 0) mb = 0;
-    if (mb > 120) mb = 120;
-    v = mb << 20;
-  }
-  return v;
+static int bd_attn_launch(int ranks, int groups, int B, size_t smem, cudaStream_t s, const BdAttnP& ap) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ranks, groups, B);
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = ranks;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
+  B200_CUDA(cudaLaunchKernelEx(&cfg, bd_attn_kernel<HD>, ap));
+  return B200_OK;
 }
 
 // one lock-step step as plain launches on `s` (also what gets captured)
@@ -575,9 +626,9 @@ static int bd_enqueue_step(BatchDecoder* d, const BdModel& m, cudaStream_t s, lo
   const int B = d->B, H = dd.hidden, I = dd.inter;
   const int QH = dd.n_heads * dd.hd, QKV = (dd.n_heads + 2 * dd.n_kv) * dd.hd;
   int rc;
-  const int Gall = dd.n_heads / dd.n_kv;
-  const int ag_heads = bd_attn_heads_per_cta(dd, B, m.sm_count);
-  const int hs = (Gall + ag_heads - 1) / ag_heads;
+  const int hs = cdiv(dd.n_heads / dd.n_kv, BA_HEADS), ranks = bd_attn_ranks(dd, B, m.sm_count);
+  const size_t att_smem = bd_attn_smem(dd, ranks);
+  B200_REQUIRE(att_smem <= 200 * 1024, "batch decode: cache capacity %d too large for the attention kernel", dd.cap);
   for (int l = 0; l < m.n_layers; ++l) {
     const LayerW& lw = m.layers[l];
     int split = 1;
@@ -589,19 +640,8 @@ static int bd_enqueue_step(BatchDecoder* d, const BdModel& m, cudaStream_t s, lo
     ap.ctx = d->ctx; ap.pos = d->pos; ap.kv = m.kv + (long)l * m.layer_stride; ap.v_off = m.v_off;
     ap.row_stride = m.row_stride; ap.out = d->att; ap.n_heads = dd.n_heads; ap.n_kv = dd.n_kv; ap.cap = dd.cap;
     ap.hsplit = hs; ap.scale_bf = dd.scale_bf;
-    {  // o_proj, then gate/up, then down, as far as the budget goes
-      long left = bd_prefetch_budget();
-      const void* w[3] = {lw.wo, lw.wgu, lw.wd};
-      const long bytes[3] = {(long)H * QH * 2, 2L * I * H * 2, (long)H * I * 2};
-      for (int i = 0; i < 3; ++i) {
-        ap.pf[i] = w[i];
-        ap.pf_bytes[i] = bytes[i] < left ? bytes[i] : left;
-        left -= ap.pf_bytes[i];
-      }
-    }
-    const dim3 ag(dd.n_kv * hs, B);
-    if (dd.hd == 128) rc = bd_attn_launch<128>(ag_heads, ag, bd_attn_smem(dd, ag_heads), s, ap);
-    else rc = bd_attn_launch<64>(ag_heads, ag, bd_attn_smem(dd, ag_heads), s, ap);
+    rc = dd.hd == 128 ? bd_attn_launch<128>(ranks, dd.n_kv * hs, B, att_smem, s, ap)
+                      : bd_attn_launch<64>(ranks, dd.n_kv * hs, B, att_smem, s, ap);
     if (rc) return rc;
     if ((rc = gemm_wt_tuned(d->att, QH, lw.wo, nullptr, nullptr, 0, nullptr, 0, d->partial, d->partial_bytes, B, H, QH,
                             B200_EPI_NONE, B200_WT_PARTIAL, 0, true, m.sm_count, &split, s)))
@@ -616,11 +656,8 @@ static int bd_enqueue_step(BatchDecoder* d, const BdModel& m, cudaStream_t s, lo
                             B200_EPI_NONE, B200_WT_PARTIAL, 0, true, m.sm_count, &split, s)))
       return rc;
     const bf16* nw = (l + 1 == m.n_layers) ? m.final_norm : m.layers[l + 1].ln1;
-    // the finish of `down` is the other HBM-idle spot: it asks for the next layer's qkv weights
-    const void* nq = (l + 1 == m.n_layers) ? nullptr : (const void*)m.layers[l + 1].wqkv;
-    const long nq_bytes = nq ? ((long)QKV * H * 2 < bd_prefetch_budget() ? (long)QKV * H * 2 : bd_prefetch_budget()) : 0;
     if ((rc = finish_rows(d->partial, split, nullptr, d->h, H, d->h, H, B200_NORM_RMS, nw, nullptr, dd.eps, d->xn, H, B,
-                          H, s, nq, nq_bytes)))
+                          H, s)))
       return rc;
     *launches += 7;
   }
@@ -642,7 +679,7 @@ int batch_decoder_begin(void** handle, const BdModel& m, int B, const int* tok, 
   B200_REQUIRE(B >= 1 && B <= 16, "batch decode: B=%d (1..16)", B);
   B200_REQUIRE(m.d.hd == 64 || m.d.hd == 128, "batch decode: head_dim %d (64|128)", m.d.hd);
   B200_REQUIRE(B <= m.kv_batch, "batch decode: B=%d > KV pool rows %d", B, m.kv_batch);
-  B200_REQUIRE(bd_attn_smem(m.d, BD_AG_MAX) <= 200 * 1024, "batch decode: cache capacity %d too large for the attention kernel", m.d.cap);
+  B200_REQUIRE(bd_attn_smem(m.d, 8) <= 200 * 1024, "batch decode: cache capacity %d too large for the attention kernel", m.d.cap);
   BatchDecoder* d = reinterpret_cast<BatchDecoder*>(*handle);
   if (!d) {
     d = new BatchDecoder();
@@ -654,12 +691,8 @@ int batch_decoder_begin(void** handle, const BdModel& m, int B, const int* tok, 
     *handle = d;
     static unsigned long long attr_mask = 0ull;
     if (first_use_on_device(&attr_mask)) {
-      B200_CUDA(cudaFuncSetAttribute(bd_attn_kernel<128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      B200_CUDA(cudaFuncSetAttribute(bd_attn_kernel<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      B200_CUDA(cudaFuncSetAttribute(bd_attn_kernel<128, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      B200_CUDA(cudaFuncSetAttribute(bd_attn_kernel<64, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      B200_CUDA(cudaFuncSetAttribute(bd_attn_kernel<64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      B200_CUDA(cudaFuncSetAttribute(bd_attn_kernel<64, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+      B200_CUDA(cudaFuncSetAttribute(bd_attn_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+      B200_CUDA(cudaFuncSetAttribute(bd_attn_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     }
   }
   d->B = B;

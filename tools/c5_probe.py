@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Run only the lock-step legs of bench.py (C5: Qwen2-VL-7B, 8 rows; the 2B model with 8 rows) and print their numbers —
-an A/B probe for decode_batch.cu changes (e.g. B200_BD_PREFETCH_MB=0 vs the default).
+an A/B probe for decode_batch.cu changes.
 usage: python tools/c5_probe.py [--c5-out 256]"""
 import argparse
 import json
@@ -23,7 +23,7 @@ def main():
     dev = torch.device("cuda", 0)
     torch.cuda.set_device(dev)
     out = bench.c5_leg(1, 0, dev, args)
-    print(json.dumps({"env": os.environ.get("B200_BD_PREFETCH_MB"), "c5": {k: out[k] for k in out if k != "workload"}}))
+    print(json.dumps({"c5": {k: out[k] for k in out if k != "workload"}}))
 
 
 if __name__ == "__main__":
