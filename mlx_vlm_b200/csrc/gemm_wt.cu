@@ -26,6 +26,7 @@
 // Replaces nn.Linear of the reference (models/qwen2_vl/vision.py:83-102,108-119,132-133,168-169;
 // language.py:52-55; mlp.py:9-15; activations.py:8-10).  Rounding points follow
 // oracle/mlx_semantics.py::linear (+ activations, residual add).
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 #include <vector>
@@ -179,6 +180,156 @@ __device__ __forceinline__ void wt_stage_f32(const uint32_t (&a)[32], float bias
   }
 }
 
+// The accumulator tile (128 weight rows x TN tokens, fp32 in TMEM) -> its outputs, by 256 threads (tid; warp tid / 32 reads TMEM
+// lane quarter (tid / 32) mod 4, which must be its own) through a staging tile in shared memory.  dead: a wait of this CTA
+// ended without its data, NaN is stored.
+template <bool TOWER>
+__device__ __forceinline__ void wt_store_tile(const WtParams& p, uint8_t* stg, uint32_t tmem, int n0, int t0, long cg, int split,
+                                              int tid, bool dead) {
+  const int warp = tid >> 5, lane = tid & 31, q = warp & 3, half = warp >> 2;
+  const int row = q * 32 + lane;  // weight row of the tile == TMEM lane
+  float bias_v = 0.f;
+  if ((TOWER || p.mode == B200_WT_BF16) && p.bias && n0 + row < p.N) bias_v = bf2f(p.bias[n0 + row]);
+  for (int c0 = 0; c0 < p.TN; c0 += WT_EPI_TOK) {
+    const int cc = c0 + half * 32;
+    if (cc < p.TN && !(p.flags & 1u)) {
+      uint32_t a[32];
+      w_tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cc, a);
+      if (dead)
+        for (int j = 0; j < 32; ++j) a[j] = 0x7FC00000u;
+      if (!TOWER && p.mode == B200_WT_PARTIAL) {
+        float* sf = reinterpret_cast<float*>(stg);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) sf[(half * 32 + j) * WT_ROWS + row] = __uint_as_float(a[j]);
+      } else if constexpr (TOWER) {
+        float* sf = reinterpret_cast<float*>(stg) + (half * 32) * WT_ROWS + row;
+        if (p.epilogue == B200_EPI_GELU_FAST) wt_stage_f32<B200_EPI_GELU_FAST>(a, bias_v, sf);
+        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_stage_f32<B200_EPI_GELU_EXACT>(a, bias_v, sf);
+        else if (p.epilogue == B200_EPI_GELU_TANH) wt_stage_f32<B200_EPI_GELU_TANH>(a, bias_v, sf);
+        else wt_stage_f32<B200_EPI_NONE>(a, bias_v, sf);
+      } else {
+        // one unrolled loop per epilogue kind, chosen OUTSIDE the loop: left to itself the compiler merged the
+        // three kinds into one predicated body of ~90 instructions per element (6-7 us per launch, A/B measured)
+        bf16* sb = reinterpret_cast<bf16*>(stg) + (half * 32) * WT_ROWS + row;
+        if (p.epilogue == B200_EPI_GELU_FAST) wt_stage_bf16<B200_EPI_GELU_FAST>(a, bias_v, sb);
+        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_stage_bf16<B200_EPI_GELU_EXACT>(a, bias_v, sb);
+        else wt_stage_bf16<B200_EPI_NONE>(a, bias_v, sb);
+      }
+    }
+    w_ebar();
+    if (!(p.flags & 4u)) {
+      if (!TOWER && p.mode == B200_WT_BF16) {
+        const bool vec_all = ((p.ldc & 7) == 0) && (!p.residual || (p.ldr & 7) == 0) &&
+                            ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0) &&
+                            (!p.residual || (reinterpret_cast<uintptr_t>(p.residual) & 15) == 0);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int idx = tid + 256 * u;
+          const int tl = idx >> 4, ch = idx & 15;
+          const int t = t0 + c0 + tl, n = n0 + ch * 8;
+          if (c0 + tl >= p.TN || t >= p.T || n >= p.N) continue;
+          const uint4 sv = *reinterpret_cast<const uint4*>(stg + (tl * WT_ROWS + ch * 8) * 2);
+          const bool vec_ok = vec_all && n + 8 <= p.N;  // only the last chunk of an odd N goes element-wise
+          if (vec_ok) {
+            uint4 o = sv;
+            if (p.residual) {
+              float r[8], v[8];
+              unpack8(*reinterpret_cast<const uint4*>(p.residual + (long)t * p.ldr + n), r);
+              unpack8(sv, v);
+#pragma unroll
+              for (int e = 0; e < 8; ++e) v[e] = rbf(r[e] + v[e]);
+              o.x = pack2(v[0], v[1]); o.y = pack2(v[2], v[3]); o.z = pack2(v[4], v[5]); o.w = pack2(v[6], v[7]);
+            }
+            *reinterpret_cast<uint4*>(p.C + (long)t * p.ldc + n) = o;
+          } else {
+            float v[8];
+            unpack8(sv, v);
+            for (int e = 0; e < 8 && n + e < p.N; ++e) {
+              float o = v[e];
+              if (p.residual) o = rbf(bf2f(p.residual[(long)t * p.ldr + n + e]) + o);
+              p.C[(long)t * p.ldc + n + e] = f2bf(o);
+            }
+          }
+        }
+      } else if (!TOWER && p.mode == B200_WT_SWIGLU) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int idx = tid + 256 * u;
+          const int tl = idx >> 3, ch = idx & 7;
+          const int t = t0 + c0 + tl, i = n0 + ch * 8;
+          if (c0 + tl >= p.TN || t >= p.T || i >= p.inter) continue;
+          float g[8], uu[8], o[8];
+          unpack8(*reinterpret_cast<const uint4*>(stg + (tl * WT_ROWS + ch * 8) * 2), g);
+          unpack8(*reinterpret_cast<const uint4*>(stg + (tl * WT_ROWS + 64 + ch * 8) * 2), uu);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) o[e] = swiglu_bf(g[e], uu[e]);
+          uint4 ov;
+          ov.x = pack2(o[0], o[1]); ov.y = pack2(o[2], o[3]); ov.z = pack2(o[4], o[5]); ov.w = pack2(o[6], o[7]);
+          *reinterpret_cast<uint4*>(p.C + (long)t * p.ldc + i) = ov;
+        }
+      } else if constexpr (TOWER) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int idx = tid + 256 * u;
+          const int tl = idx >> 5, ch = idx & 31;
+          const int t = t0 + c0 + tl, n = n0 + ch * 4;
+          if (c0 + tl >= p.TN || t >= p.T || n >= p.N) continue;
+          float4 v = *reinterpret_cast<const float4*>(stg + (tl * WT_ROWS + ch * 4) * 4);
+          if (p.mode == B200_WT_F32) {
+            float* dst = p.C32 + (long)t * p.ldc32 + cg + n;
+            if (n + 4 <= p.N && (p.ldc32 & 3) == 0 && (cg & 3) == 0) {
+              if (p.res32) {
+                const float4 r = *reinterpret_cast<const float4*>(p.res32 + (long)t * p.ldr32 + n);
+                v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w;
+              }
+              *reinterpret_cast<float4*>(dst) = v;
+            } else {
+              const float vv[4] = {v.x, v.y, v.z, v.w};
+              for (int e = 0; e < 4 && n + e < p.N; ++e)
+                dst[e] = vv[e] + (p.res32 ? p.res32[(long)t * p.ldr32 + n + e] : 0.f);
+            }
+          } else {  // [hi | lo]: hi = bf16(v), lo = bf16(v - hi)
+            const float vv[4] = {v.x, v.y, v.z, v.w};
+            float hi[4], lo[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              hi[e] = rbf(vv[e]);
+              lo[e] = vv[e] - hi[e];
+            }
+            bf16* dh = p.Csplit + (long)t * p.ld_split + n;
+            if (n + 4 <= p.N) {
+              *reinterpret_cast<uint2*>(dh) = make_uint2(pack2(hi[0], hi[1]), pack2(hi[2], hi[3]));
+              *reinterpret_cast<uint2*>(dh + p.n_pad) = make_uint2(pack2(lo[0], lo[1]), pack2(lo[2], lo[3]));
+            } else {
+              for (int e = 0; e < 4 && n + e < p.N; ++e) {
+                dh[e] = f2bf(hi[e]);
+                dh[p.n_pad + e] = f2bf(lo[e]);
+              }
+            }
+          }
+        }
+      } else {  // fp32 partial tile -> P[split][t][n]
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int idx = tid + 256 * u;
+          const int tl = idx >> 5, ch = idx & 31;
+          const int t = t0 + c0 + tl, n = n0 + ch * 4;
+          if (c0 + tl >= p.TN || t >= p.T || n >= p.N) continue;
+          const float4 v = *reinterpret_cast<const float4*>(stg + (tl * WT_ROWS + ch * 4) * 4);
+          float* dst = p.partial + ((long)split * p.T + t) * p.N + n;
+          if (n + 4 <= p.N && (p.N & 3) == 0) {
+            *reinterpret_cast<float4*>(dst) = v;
+          } else {
+            const float vv[4] = {v.x, v.y, v.z, v.w};
+            for (int e = 0; e < 4 && n + e < p.N; ++e) dst[e] = vv[e];
+          }
+        }
+      }
+    }
+    w_ebar();
+  }
+}
+
 // TOWER = false: the bf16 paths (B200_WT_BF16 / PARTIAL / SWIGLU); TOWER = true: the fp32-accurate paths
 // (B200_WT_F32 / SPLIT).  Two instantiations keep each one's code small (tools/wt_ab_probe.py A/B-times builds).
 template <bool TOWER>
@@ -322,148 +473,8 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   // ===== epilogue (all 8 warps): warp w reads TMEM lane quarter w % 4, token half w / 4 =====
   w_mbar_wait(&tmem_full, 0);
   w_fence_after();
-  const int q = warp & 3, half = warp >> 2;
-  const int row = q * 32 + lane;  // weight row of the tile == TMEM lane
-  float bias_v = 0.f;
-  if ((TOWER || p.mode == B200_WT_BF16) && p.bias && n0 + row < p.N) bias_v = bf2f(p.bias[n0 + row]);
-  uint8_t* stg = ring;  // every TMA load has landed and every MMA has retired: the ring is free
-  const int tid = threadIdx.x;
-  for (int c0 = 0; c0 < p.TN; c0 += WT_EPI_TOK) {
-    const int cc = c0 + half * 32;
-    if (cc < p.TN && !(p.flags & 1u)) {
-      uint32_t a[32];
-      w_tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)cc, a);
-      if (!TOWER && p.mode == B200_WT_PARTIAL) {
-        float* sf = reinterpret_cast<float*>(stg);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) sf[(half * 32 + j) * WT_ROWS + row] = __uint_as_float(a[j]);
-      } else if constexpr (TOWER) {
-        float* sf = reinterpret_cast<float*>(stg) + (half * 32) * WT_ROWS + row;
-        if (p.epilogue == B200_EPI_GELU_FAST) wt_stage_f32<B200_EPI_GELU_FAST>(a, bias_v, sf);
-        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_stage_f32<B200_EPI_GELU_EXACT>(a, bias_v, sf);
-        else if (p.epilogue == B200_EPI_GELU_TANH) wt_stage_f32<B200_EPI_GELU_TANH>(a, bias_v, sf);
-        else wt_stage_f32<B200_EPI_NONE>(a, bias_v, sf);
-      } else {
-        // one unrolled loop per epilogue kind, chosen OUTSIDE the loop: left to itself the compiler merged the
-        // three kinds into one predicated body of ~90 instructions per element (6-7 us per launch, A/B measured)
-        bf16* sb = reinterpret_cast<bf16*>(stg) + (half * 32) * WT_ROWS + row;
-        if (p.epilogue == B200_EPI_GELU_FAST) wt_stage_bf16<B200_EPI_GELU_FAST>(a, bias_v, sb);
-        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_stage_bf16<B200_EPI_GELU_EXACT>(a, bias_v, sb);
-        else wt_stage_bf16<B200_EPI_NONE>(a, bias_v, sb);
-      }
-    }
-    w_ebar();
-    if (!(p.flags & 4u)) {
-      if (!TOWER && p.mode == B200_WT_BF16) {
-        const bool vec_all = ((p.ldc & 7) == 0) && (!p.residual || (p.ldr & 7) == 0) &&
-                            ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0) &&
-                            (!p.residual || (reinterpret_cast<uintptr_t>(p.residual) & 15) == 0);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int idx = tid + 256 * u;
-          const int tl = idx >> 4, ch = idx & 15;
-          const int t = t0 + c0 + tl, n = n0 + ch * 8;
-          if (c0 + tl >= p.TN || t >= p.T || n >= p.N) continue;
-          const uint4 sv = *reinterpret_cast<const uint4*>(stg + (tl * WT_ROWS + ch * 8) * 2);
-          const bool vec_ok = vec_all && n + 8 <= p.N;  // only the last chunk of an odd N goes element-wise
-          if (vec_ok) {
-            uint4 o = sv;
-            if (p.residual) {
-              float r[8], v[8];
-              unpack8(*reinterpret_cast<const uint4*>(p.residual + (long)t * p.ldr + n), r);
-              unpack8(sv, v);
-#pragma unroll
-              for (int e = 0; e < 8; ++e) v[e] = rbf(r[e] + v[e]);
-              o.x = pack2(v[0], v[1]); o.y = pack2(v[2], v[3]); o.z = pack2(v[4], v[5]); o.w = pack2(v[6], v[7]);
-            }
-            *reinterpret_cast<uint4*>(p.C + (long)t * p.ldc + n) = o;
-          } else {
-            float v[8];
-            unpack8(sv, v);
-            for (int e = 0; e < 8 && n + e < p.N; ++e) {
-              float o = v[e];
-              if (p.residual) o = rbf(bf2f(p.residual[(long)t * p.ldr + n + e]) + o);
-              p.C[(long)t * p.ldc + n + e] = f2bf(o);
-            }
-          }
-        }
-      } else if (!TOWER && p.mode == B200_WT_SWIGLU) {
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int idx = tid + 256 * u;
-          const int tl = idx >> 3, ch = idx & 7;
-          const int t = t0 + c0 + tl, i = n0 + ch * 8;
-          if (c0 + tl >= p.TN || t >= p.T || i >= p.inter) continue;
-          float g[8], uu[8], o[8];
-          unpack8(*reinterpret_cast<const uint4*>(stg + (tl * WT_ROWS + ch * 8) * 2), g);
-          unpack8(*reinterpret_cast<const uint4*>(stg + (tl * WT_ROWS + 64 + ch * 8) * 2), uu);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) o[e] = swiglu_bf(g[e], uu[e]);
-          uint4 ov;
-          ov.x = pack2(o[0], o[1]); ov.y = pack2(o[2], o[3]); ov.z = pack2(o[4], o[5]); ov.w = pack2(o[6], o[7]);
-          *reinterpret_cast<uint4*>(p.C + (long)t * p.ldc + i) = ov;
-        }
-      } else if constexpr (TOWER) {
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int idx = tid + 256 * u;
-          const int tl = idx >> 5, ch = idx & 31;
-          const int t = t0 + c0 + tl, n = n0 + ch * 4;
-          if (c0 + tl >= p.TN || t >= p.T || n >= p.N) continue;
-          float4 v = *reinterpret_cast<const float4*>(stg + (tl * WT_ROWS + ch * 4) * 4);
-          if (p.mode == B200_WT_F32) {
-            float* dst = p.C32 + (long)t * p.ldc32 + cg + n;
-            if (n + 4 <= p.N && (p.ldc32 & 3) == 0 && (cg & 3) == 0) {
-              if (p.res32) {
-                const float4 r = *reinterpret_cast<const float4*>(p.res32 + (long)t * p.ldr32 + n);
-                v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w;
-              }
-              *reinterpret_cast<float4*>(dst) = v;
-            } else {
-              const float vv[4] = {v.x, v.y, v.z, v.w};
-              for (int e = 0; e < 4 && n + e < p.N; ++e)
-                dst[e] = vv[e] + (p.res32 ? p.res32[(long)t * p.ldr32 + n + e] : 0.f);
-            }
-          } else {  // [hi | lo]: hi = bf16(v), lo = bf16(v - hi)
-            const float vv[4] = {v.x, v.y, v.z, v.w};
-            float hi[4], lo[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              hi[e] = rbf(vv[e]);
-              lo[e] = vv[e] - hi[e];
-            }
-            bf16* dh = p.Csplit + (long)t * p.ld_split + n;
-            if (n + 4 <= p.N) {
-              *reinterpret_cast<uint2*>(dh) = make_uint2(pack2(hi[0], hi[1]), pack2(hi[2], hi[3]));
-              *reinterpret_cast<uint2*>(dh + p.n_pad) = make_uint2(pack2(lo[0], lo[1]), pack2(lo[2], lo[3]));
-            } else {
-              for (int e = 0; e < 4 && n + e < p.N; ++e) {
-                dh[e] = f2bf(hi[e]);
-                dh[p.n_pad + e] = f2bf(lo[e]);
-              }
-            }
-          }
-        }
-      } else {  // fp32 partial tile -> P[split][t][n]
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int idx = tid + 256 * u;
-          const int tl = idx >> 5, ch = idx & 31;
-          const int t = t0 + c0 + tl, n = n0 + ch * 4;
-          if (c0 + tl >= p.TN || t >= p.T || n >= p.N) continue;
-          const float4 v = *reinterpret_cast<const float4*>(stg + (tl * WT_ROWS + ch * 4) * 4);
-          float* dst = p.partial + ((long)split * p.T + t) * p.N + n;
-          if (n + 4 <= p.N && (p.N & 3) == 0) {
-            *reinterpret_cast<float4*>(dst) = v;
-          } else {
-            const float vv[4] = {v.x, v.y, v.z, v.w};
-            for (int e = 0; e < 4 && n + e < p.N; ++e) dst[e] = vv[e];
-          }
-        }
-      }
-    }
-    w_ebar();
-  }
+  // every TMA load has landed and every MMA has retired: the ring is free for the staging tile
+  wt_store_tile<TOWER>(p, ring, tmem_base, n0, t0, cg, split, threadIdx.x, false);
   w_fence_before();
   __syncthreads();
   if (warp == 2) {
@@ -471,6 +482,231 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
                  "r"(tmem_cols)
                  : "memory");
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The same product for many tokens: CTA PAIRS (cta_group::2), persistent.  A pair multiplies 256 weight rows by TN tokens:
+// each CTA keeps 128 weight rows and HALF of the tokens of a k-block in its shared memory and the tensor cores of both read
+// both halves, so a 128 x 256 share of the output costs 32 KB of fill per k-block instead of 48: what bounds the one-CTA
+// kernel at these sizes is the fill (all SMs together take 11.5 - 12 TB/s out of the L2: 1,050 TFLOP/s at 48 KB).  Two
+// accumulators in TMEM: the epilogue warps store a tile while the next one is multiplied, and the ring never drains between
+// tiles.
+// Measured, one CTA -> pairs: 4896 tokens x 22016 rows x 4096 (SwiGLU) 878 -> 629 us (1,404 TFLOP/s), x 12288 x 4096 479 -> 335,
+// x 4096 x 11008 427 -> 332; 2048 x 37888 x 3584 588 -> 418; 6012 x 3840 x 1280 64 -> 52; below a wave of pairs it loses
+// (576 x 3840 x 1280 11.8 -> 14.7), so it is one more candidate of the measured choice.
+//   warp 0  TMA producer of this CTA's operands; the bytes of both CTAs count on the leader's (rank 0) full barrier
+//   warp 1  leader only: MMA issuer; its commits free the slot / hand the accumulator over in both CTAs
+//   warp 2  TMEM
+//   warps 4..11  epilogue of this CTA's 128 weight rows
+// Tiles are dealt out round robin, token tile first, so that the pairs of a wave share weight rows in the L2.
+// ---------------------------------------------------------------------------------------------
+constexpr int WP_THREADS = 384;
+constexpr int WP_MAX_STAGES = 12;
+
+struct WpBars {
+  uint64_t full[WP_MAX_STAGES], empty[WP_MAX_STAGES], acc_full[2], acc_empty[2];
+};
+
+// Bounded: a wait that does not end (about a second) gives up, and so does every later one of the thread; the tiles that it
+// would have stored become NaN.
+__device__ __forceinline__ void wp_wait(uint64_t* bar, uint32_t parity, bool& dead) {
+  uint32_t done = 0;
+  const uint32_t addr = w_smem_u32(bar);
+  for (int i = 0; !done && !dead; ++i) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (i > (1 << 24)) dead = true;
+  }
+}
+__device__ __forceinline__ uint32_t wp_leader(const void* p) {   // shared::cluster address of *p in the pair's rank 0
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(w_smem_u32(p)));
+  return r;
+}
+__device__ __forceinline__ void wp_tma_2d(void* dst, const CUtensorMap* tmap, uint32_t bar, int c0, int c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
+      " [%0], [%1, {%2, %3}], [%4];" ::"r"(w_smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void wp_umma(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(tmem_d),
+      "r"(a_lo), "r"(b_lo), "r"(W_DESC_HI), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void wp_commit(uint64_t* bar) {   // arrives on *bar of both CTAs when the MMAs so far have retired
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(w_smem_u32(bar)),
+      "h"((uint16_t)3)
+      : "memory");
+}
+__device__ __forceinline__ void wp_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <bool TOWER>
+__global__ void __launch_bounds__(WP_THREADS, 1)
+gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const WtParams p) {
+  extern __shared__ uint8_t wt_smem_raw[];
+  __shared__ WpBars bars;
+  __shared__ uint32_t tmem_slot;
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(wt_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+  const bool swiglu = !TOWER && (p.mode == B200_WT_SWIGLU);
+  const int xhalf = p.TN / 2, stage_bytes = WT_WBLK + xhalf * 128, NS = p.n_stages;
+  uint8_t* stg = ring + (long)NS * stage_bytes;
+  const int kb_total = (p.K + WT_BK - 1) / WT_BK;
+  const int row_tiles = ((swiglu ? 2 * p.inter : p.N) + 2 * WT_ROWS - 1) / (2 * WT_ROWS), tok_tiles = (p.T + p.TN - 1) / p.TN;
+  const int splits = (kb_total + p.kb_per_split - 1) / p.kb_per_split;
+  const int n_tiles = row_tiles * tok_tiles * splits;
+  bool dead = false;
+  // tile -> this CTA's first output feature, its first token, its k-blocks
+  auto tile_at = [&](int tile, int& n0, int& t0, int& split, int& kb0, int& kb1) {
+    t0 = tile % tok_tiles * p.TN;
+    tile /= tok_tiles;
+    n0 = (tile % row_tiles * 2 + rank) * (swiglu ? 64 : WT_ROWS);
+    split = tile / row_tiles;
+    kb0 = split * p.kb_per_split;
+    kb1 = min(kb_total, kb0 + p.kb_per_split);
+  };
+
+  w_pdl_launch();
+  if (warp == 0 && lane == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmW)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmX)) : "memory");
+    for (int s = 0; s < NS; ++s) {
+      w_mbar_init(&bars.full[s], 1);
+      w_mbar_init(&bars.empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      w_mbar_init(&bars.acc_full[b], 1);
+      w_mbar_init(&bars.acc_empty[b], 16);   // eight epilogue warps of each CTA
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(w_smem_u32(&tmem_slot)), "r"(512u)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  w_fence_before();
+  __syncthreads();
+  wp_cluster_sync();   // the peer's barriers exist before anything arrives on them
+  w_fence_after();
+  const uint32_t tmem = tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {  // ===== TMA producer =====
+      const uint32_t full0 = wp_leader(&bars.full[0]);
+      auto load_w = [&](int s, int kb, int n0) {
+        if (p.kb_w > 0) kb %= p.kb_w;
+        uint8_t* sW = ring + (long)s * stage_bytes;
+        const uint32_t bar = full0 + s * 8;
+        if (rank == 0) w_mbar_expect_tx(&bars.full[s], 2u * (uint32_t)stage_bytes);
+        if (swiglu) {
+          wp_tma_2d(sW, &tmW, bar, kb * WT_BK, n0);
+          wp_tma_2d(sW + 64 * 128, &tmW, bar, kb * WT_BK, p.inter + n0);
+        } else {
+          wp_tma_2d(sW, &tmW, bar, kb * WT_BK, n0);
+        }
+      };
+      auto load_x = [&](int s, int kb, int t0) {
+        wp_tma_2d(ring + (long)s * stage_bytes + WT_WBLK, &tmX, full0 + s * 8, kb * WT_BK, t0 + rank * xhalf);
+      };
+      int n0, t0, split, kb0, kb1;
+      // weights never depend on the previous kernel: those of the first slots are requested before waiting for it
+      int pre = 0;
+      if (pair < n_tiles) {
+        tile_at(pair, n0, t0, split, kb0, kb1);
+        pre = min(NS, kb1 - kb0);
+        for (int i = 0; i < pre; ++i) load_w(i, kb0 + i, n0);
+      }
+      w_pdl_wait();
+      int s = 0;
+      uint32_t free_parity = 1;
+      for (int tile = pair; tile < n_tiles && !dead; tile += n_pairs) {
+        tile_at(tile, n0, t0, split, kb0, kb1);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (pre > 0) {
+            --pre;
+          } else {
+            wp_wait(&bars.empty[s], free_parity, dead);
+            if (dead) break;   // nothing more is requested
+            load_w(s, kb, n0);
+          }
+          load_x(s, kb, t0);
+          if (++s == NS) s = 0, free_parity ^= 1;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (rank == 0 && lane == 0) {  // ===== MMA issuer =====
+      // D = f32, A = B = bf16, both K-major; M = 256 weight rows, N = TN tokens
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.TN >> 3) << 17) | (16u << 24);
+      // (slot and parity are counted along: a division per k-block would cost more than its four products)
+      const uint32_t w_first = w_desc_lo(w_smem_u32(ring)), x_first = w_desc_lo(w_smem_u32(ring + WT_WBLK));
+      const uint32_t step = (uint32_t)stage_bytes >> 4;
+      int s = 0, j = 0, n0, t0, split, kb0, kb1;
+      uint32_t w_lo = w_first, x_lo = x_first, parity = 0;
+      for (int tile = pair; tile < n_tiles && !dead; tile += n_pairs, ++j) {
+        tile_at(tile, n0, t0, split, kb0, kb1);
+        const uint32_t d = tmem + (uint32_t)(j & 1) * 256u;
+        wp_wait(&bars.acc_empty[j & 1], ((j >> 1) & 1) ^ 1, dead);
+        w_fence_after();
+        uint32_t acc = 0;
+        for (int kb = kb0; kb < kb1; ++kb) {
+          wp_wait(&bars.full[s], parity, dead);
+          if (dead) break;
+          w_fence_after();
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            wp_umma(d, w_lo + k * 2, x_lo + k * 2, idesc, acc);
+            acc = 1;
+          }
+          wp_commit(&bars.empty[s]);
+          w_lo += step;
+          x_lo += step;
+          if (++s == NS) s = 0, w_lo = w_first, x_lo = x_first, parity ^= 1;
+        }
+        wp_commit(&bars.acc_full[j & 1]);
+      }
+    }
+  } else if (warp >= 4) {  // ===== epilogue =====
+    w_pdl_wait();
+    int j = 0, n0, t0, split, kb0, kb1;
+    for (int tile = pair; tile < n_tiles; tile += n_pairs, ++j) {
+      tile_at(tile, n0, t0, split, kb0, kb1);
+      wp_wait(&bars.acc_full[j & 1], (j >> 1) & 1, dead);
+      __syncwarp();
+      w_fence_after();
+      wt_store_tile<TOWER>(p, stg, tmem + (uint32_t)(j & 1) * 256u, n0, t0, 0, split, threadIdx.x - 128, dead);
+      w_fence_before();
+      __syncwarp();
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(wp_leader(&bars.acc_empty[j & 1]))
+                     : "memory");
+    }
+  }
+  __syncwarp();
+  w_fence_before();
+  __syncthreads();
+  wp_cluster_sync();   // nobody's shared memory or TMEM goes while the peer still uses it
+  if (warp == 2) {
+    w_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
 }
 
@@ -685,6 +921,11 @@ void gemm_wt_set_pdl(bool on) { g_wt_pdl = on; }
 
 static int round16(int x) { return (x + 15) & ~15; }
 
+constexpr int WP_PAIRS = 74;   // pairs of SMs
+static size_t wp_staging(int mode) {   // the epilogue's staging tile: WT_EPI_TOK tokens x 128 rows
+  return (size_t)WT_EPI_TOK * WT_ROWS * (mode == B200_WT_BF16 || mode == B200_WT_SWIGLU ? 2 : 4);
+}
+
 // Tile / pipeline configuration for (T, row blocks, K): a small cost model calibrated on the round-2
 // sweep (profiles/r2_gemm_wt_sweep.txt, B200):
 //   * a CTA costs ~4.5 us of fixed latency (launch, barrier/TMEM set-up, first TMA round trip,
@@ -779,8 +1020,9 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
   B200_REQUIRE(T > 0 && N > 0 && K > 0, "gemm_wt: empty problem T=%d N=%d K=%d", T, N, K);
   B200_REQUIRE((ldx % 8) == 0 && (K % 8) == 0, "gemm_wt: ldx (%ld) and K (%d) must be multiples of 8", ldx, K);
   B200_REQUIRE(((uintptr_t)X & 15) == 0 && ((uintptr_t)W & 15) == 0, "gemm_wt: X and W must be 16-byte aligned");
-  B200_REQUIRE(cfg.TN >= 16 && cfg.TN <= 256 && (cfg.TN % 16) == 0, "gemm_wt: TN=%d", cfg.TN);
-  B200_REQUIRE(cfg.KS >= 1 && cfg.stages >= 2 && cfg.stages <= WT_MAX_STAGES && cfg.split >= 1,
+  const bool pair = cfg.KS == 0;   // CTA pairs
+  B200_REQUIRE(cfg.TN >= 16 && cfg.TN <= 256 && (cfg.TN % (pair ? 32 : 16)) == 0, "gemm_wt: TN=%d", cfg.TN);
+  B200_REQUIRE(cfg.KS >= 0 && cfg.stages >= 2 && cfg.stages <= (pair ? WP_MAX_STAGES : WT_MAX_STAGES) && cfg.split >= 1,
                "gemm_wt: bad config KS=%d stages=%d split=%d", cfg.KS, cfg.stages, cfg.split);
   B200_REQUIRE(mode >= B200_WT_BF16 && mode <= B200_WT_SPLIT, "gemm_wt: mode %d", mode);
   B200_REQUIRE((mode != B200_WT_F32 && mode != B200_WT_SPLIT) || ext, "gemm_wt: fp32 / split output needs WtExt");
@@ -801,7 +1043,7 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
   p.kb_per_split = cdiv(kb_total, cfg.split);
   const int splits = cdiv(kb_total, p.kb_per_split);
   B200_REQUIRE(splits == cfg.split, "gemm_wt: split %d leaves empty splits (%d k-blocks)", cfg.split, kb_total);
-  p.epilogue = epilogue; p.mode = mode; p.inter = inter; p.flags = flags;
+  p.epilogue = epilogue; p.mode = mode; p.inter = inter; p.flags = flags & 7u;
   int k_w = K;  // columns of W (the split operand repeats the weight k-blocks)
   if (ext) {
     p.kb_w = ext->kb_w; p.C32 = ext->C32; p.res32 = ext->res32; p.ldc32 = ext->ldc32; p.ldr32 = ext->ldr32;
@@ -821,17 +1063,18 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
   const bool grouped = ext && ext->tile_group;
   B200_REQUIRE(!grouped || (mode == B200_WT_F32 && ext->n_groups > 0 && cfg.split == 1 && !bias),
                "gemm_wt: grouped products are fp32-output, unsplit, without bias");
-  const int stage = cfg.KS * (WT_WBLK + cfg.TN * 128);
-  const size_t smem = (size_t)cfg.stages * stage + 1024;
+  B200_REQUIRE(!pair || (!grouped && !heads), "gemm_wt: pairs take no groups");
+  const int stage = pair ? WT_WBLK + cfg.TN * 64 : cfg.KS * (WT_WBLK + cfg.TN * 128);
+  const size_t smem = (size_t)cfg.stages * stage + 1024 + (pair ? wp_staging(mode) : 0);
   B200_REQUIRE(smem <= 227 * 1024 - 1024, "gemm_wt: %zu B of shared memory", smem);
-  B200_REQUIRE((size_t)cfg.stages * stage >= (size_t)WT_EPI_TOK * WT_ROWS * 4, "gemm_wt: ring smaller than the epilogue staging tile");
+  B200_REQUIRE(pair || (size_t)cfg.stages * stage >= (size_t)WT_EPI_TOK * WT_ROWS * 4, "gemm_wt: ring smaller than the epilogue staging tile");
   CUtensorMap tw, tx;
   int rc = wt_tmap(W, (long)(ext && ext->ldw > 0 ? ext->ldw : k_w),
                    grouped ? ext->n_groups * N : (heads && !w_cols ? ext->col_groups * N : N),
                    w_cols ? (ext->col_groups - 1) * ext->w_group_cols + k_w : k_w,
                    mode == B200_WT_SWIGLU ? 64 : WT_ROWS, &tw);
   if (rc) return rc;
-  if ((rc = wt_tmap(X, ldx, T, heads ? ext->x_cols : K, cfg.TN, &tx))) return rc;
+  if ((rc = wt_tmap(X, ldx, T, heads ? ext->x_cols : K, pair ? cfg.TN / 2 : cfg.TN, &tx))) return rc;
   static unsigned long long set_mask = 0ull;
   int dev = 0;
   B200_CUDA(cudaGetDevice(&dev));
@@ -842,6 +1085,8 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
     B200_CUDA(cudaFuncSetAttribute(gemm_wt_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024));
     B200_CUDA(cudaFuncSetAttribute(gemm_wt_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                    cudaSharedmemCarveoutMaxShared));
+    B200_CUDA(cudaFuncSetAttribute(gemm_wt_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024));
+    B200_CUDA(cudaFuncSetAttribute(gemm_wt_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024));
     set_mask |= 1ull << (dev & 63);
   }
   const int row_blocks = mode == B200_WT_SWIGLU ? cdiv(inter, 64) : cdiv(N, WT_ROWS);
@@ -855,6 +1100,21 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
   at[0].val.programmaticStreamSerializationAllowed = 1;
   lc.attrs = at;
   lc.numAttrs = (g_wt_pdl && !grouped) ? 1 : 0;
+  if (pair) {
+    const int tiles = cdiv(mode == B200_WT_SWIGLU ? 2 * inter : N, 2 * WT_ROWS) * cdiv(T, cfg.TN) * splits;
+    lc.gridDim = dim3(2 * (tiles < WP_PAIRS ? tiles : WP_PAIRS));
+    lc.blockDim = dim3(WP_THREADS);
+    cudaLaunchAttribute pa[2];
+    pa[0].id = cudaLaunchAttributeClusterDimension;
+    pa[0].val.clusterDim.x = 2;
+    pa[0].val.clusterDim.y = pa[0].val.clusterDim.z = 1;
+    pa[1] = at[0];
+    lc.attrs = pa;
+    lc.numAttrs = g_wt_pdl ? 2 : 1;
+    if (mode == B200_WT_F32 || mode == B200_WT_SPLIT) B200_CUDA(cudaLaunchKernelEx(&lc, gemm_wt_pair_kernel<true>, tw, tx, p));
+    else B200_CUDA(cudaLaunchKernelEx(&lc, gemm_wt_pair_kernel<false>, tw, tx, p));
+    return B200_OK;
+  }
   if (mode == B200_WT_F32 || mode == B200_WT_SPLIT) {
     B200_CUDA(cudaLaunchKernelEx(&lc, gemm_wt_kernel<true>, tw, tx, p));
   } else {
@@ -926,7 +1186,7 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
         if (FILE* fp = fopen(path, "r")) {
           int tb, n, k, md, so, tn, ks, stg, sp;
           while (fscanf(fp, "%d %d %d %d %d %d %d %d %d", &tb, &n, &k, &md, &so, &tn, &ks, &stg, &sp) == 9)
-            if (tn >= 16 && tn <= 256 && tn % 16 == 0 && ks >= 1 && stg >= 2 && stg <= WT_MAX_STAGES && sp >= 1)
+            if (tn >= 16 && tn <= 256 && tn % (ks ? 16 : 32) == 0 && ks >= 0 && stg >= 2 && stg <= WT_MAX_STAGES && sp >= 1)
               cache[TuneKey{tb, n, k, md, so, dev}] = WtConfig{tn, ks, stg, sp};
           fclose(fp);
         }
@@ -990,6 +1250,29 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
       for (int sp : sps) {
         add(tn, 2, 208 * 1024, sp);  // one CTA per SM, 256-byte weight-row bursts
         add(tn, 1, 110 * 1024, sp);  // two CTAs per SM
+      }
+    }
+    // CTA pairs (KS = 0) from about a wave of them on: the token tile whose last wave is fullest, the next best, and 256
+    if (T >= 192 && !(ext && (ext->tile_group || ext->col_groups > 0))) {
+      const int pair_rows = cdiv(mode == B200_WT_SWIGLU ? 2 * inter : N, 2 * WT_ROWS);
+      auto add_pair = [&](int tn, int split) {
+        const int stage = WT_WBLK + tn * 64;
+        int stg = (int)((226 * 1024 - 1024 - wp_staging(mode)) / stage);
+        if (stg > WP_MAX_STAGES) stg = WP_MAX_STAGES;
+        split = cdiv(kb_total, cdiv(kb_total, split < 1 ? 1 : split));
+        const WtConfig c{tn, 0, stg, split};
+        if (!fits(c)) return;
+        for (const auto& o : cand)
+          if (o.TN == c.TN && o.KS == 0 && o.split == c.split) return;
+        cand.push_back(c);
+      };
+      int order[5] = {256, 224, 192, 160, 128};
+      auto waves_cost = [&](int tn) { return cdiv((long)pair_rows * cdiv(T, tn), WP_PAIRS) * (long)(128 + tn / 2); };
+      std::stable_sort(order, order + 5, [&](int a, int b) { return waves_cost(a) < waves_cost(b); });
+      for (int tn : {order[0], order[1], 256}) {
+        const int base = pair_rows * cdiv(T, tn);
+        add_pair(tn, 1);
+        if (allow_split && base < WP_PAIRS) add_pair(tn, WP_PAIRS / base);
       }
     }
     if (cand.empty()) {
@@ -1059,6 +1342,11 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
       set_error("gemm_wt: configuration measurement failed (T=%d N=%d K=%d mode=%d)", T, N, K, mode);
       return rc;
     }
+    // Back to back a pair does not show what it costs in a sequence: all of an SM's shared memory, so the next kernel's set-up
+    // and weight loads wait for it, and code of its own to fetch.  It has to win by 8 % (a 2048 x 2048 x 2048 product measured 3 %
+    // faster alone and was 4 us of 26 slower between row kernels).
+    for (size_t i = 0; i < cand.size(); ++i)
+      if (cand[i].KS == 0) ms[i] *= 1.08f;
     float best = 1e30f;
     for (float t : ms) best = t < best ? t : best;
     size_t pick = 0;
@@ -1082,7 +1370,7 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
     }
   }
   // a cached configuration was tuned for a token count in the same 64-bucket: re-check the bounds
-  if (cfg.TN > round16(T)) cfg.TN = round16(T);
+  if (cfg.TN > round16(T) && cfg.KS > 0) cfg.TN = round16(T);
   while (cfg.split > 1 && !fits(cfg)) cfg.split = cdiv(kb_total, cdiv(kb_total, cfg.split - 1));
   B200_REQUIRE(fits(cfg), "gemm_wt: the partial-tile buffer (%ld B) is too small for T=%d N=%d", partial_bytes, T, N);
   if (split_out) *split_out = cfg.split;
@@ -1133,6 +1421,8 @@ int b200_gemm_wt(const void* X, long ldx, const void* W, const void* bias, const
   WtConfig c;
   if (cfg4 && cfg4[0] > 0) {
     c.TN = cfg4[0]; c.KS = cfg4[1]; c.stages = cfg4[2]; c.split = cfg4[3];
+    B200_REQUIRE(c.KS >= 1, "gemm_wt: bad config KS=%d", c.KS);
+    if (flags & B200_WT_FLAG_PAIR) c.KS = 0;
   } else {
     const int rbs = mode == B200_WT_SWIGLU ? cdiv(inter, 64) : cdiv(N, 128);
     gemm_wt_auto(T, rbs, K, mode == B200_WT_PARTIAL, &c, 148);

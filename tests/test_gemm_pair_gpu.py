@@ -1,0 +1,116 @@
+"""The GEMM of CTA pairs (csrc/gemm_wt.cu: gemm_wt_pair_kernel) at the edges of its tiles: 256 weight rows (128 / SwiGLU: 64 channels
+per CTA of the pair), token tiles of 128 .. 256, k-blocks of 64, one and several tiles per pair, split-K.
+
+Bound: bf16 products are exact in fp32, sums of K of them err by less than 2^-20 here, outputs are rounded to bf16 (2^-9): the
+relative L2 distance from the rounded float64 result stays below 1e-3 (single roundings that fall the other way)."""
+import os
+import subprocess
+import sys
+
+import pytest
+import torch
+
+from _util import rl2
+
+pytestmark = pytest.mark.gpu
+PAIR = 8          # B200_WT_FLAG_PAIR
+
+
+@pytest.fixture(scope="module")
+def lib():
+    from mlx_vlm_b200 import _native as N
+    return N.lib()
+
+
+def _rand(*shape, seed, std=1.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(shape, generator=g, device="cuda") * std).to(torch.bfloat16)
+
+
+def _call(lib, x, w, bias, res, out, part, N, epi, mode, inter, cfg):
+    import ctypes
+    from mlx_vlm_b200 import _native as Nn
+    T, K = x.shape
+    c = (ctypes.c_int * 4)(*cfg)
+    Nn.check(lib.b200_gemm_wt(x.data_ptr(), K, w.data_ptr(), Nn.ptr(bias), Nn.ptr(res), 0 if res is None else res.shape[1],
+                              Nn.ptr(out), 0 if out is None else out.shape[1], Nn.ptr(part), T, N, K, epi, mode, inter, c, PAIR, 0),
+             "gemm_wt")
+    torch.cuda.synchronize()
+
+
+# (T, N, K, TN, stages): one tile and less | ragged tokens, rows and k | more tiles than pairs | an odd row count
+@pytest.mark.parametrize("T,N,K,TN,stages", [(1, 8, 64, 64, 2), (128, 256, 64, 128, 4), (129, 257, 72, 128, 3), (300, 520, 1000, 224, 6),
+                                             (1000, 3000, 256, 256, 6), (2100, 2600, 192, 160, 5), (513, 131, 4096, 192, 2)])
+def test_bf16_with_bias_and_residual(lib, T, N, K, TN, stages):
+    x, w, b, r = _rand(T, K, seed=1), _rand(N, K, seed=2, std=K ** -0.5), _rand(N, seed=3), _rand(T, N, seed=4)
+    y = x.double() @ w.double().T
+    ldn = (N + 7) // 8 * 8
+    plain = torch.full((T, ldn), 9.0, dtype=torch.bfloat16, device="cuda")
+    _call(lib, x, w, None, None, plain, None, N, 0, 0, 0, (TN, 1, stages, 1))
+    assert rl2(plain[:, :N], y.to(torch.bfloat16)) <= 1e-3 and bool((plain[:, N:] == 9.0).all())
+    got = torch.empty(T, N, dtype=torch.bfloat16, device="cuda")
+    _call(lib, x, w, b, r, got, None, N, 0, 0, 0, (TN, 1, stages, 1))
+    want = ((y + b.double()).to(torch.bfloat16).double() + r.double()).to(torch.bfloat16)
+    assert rl2(got, want) <= 1e-3
+
+
+@pytest.mark.parametrize("T,inter,K,TN", [(128, 64, 64, 128), (257, 200, 320, 256), (700, 1032, 128, 192), (64, 4096, 64, 64)])
+def test_swiglu(lib, T, inter, K, TN):
+    x, w = _rand(T, K, seed=5), _rand(2 * inter, K, seed=6, std=K ** -0.5)
+    got = torch.full((T, inter), 9.0, dtype=torch.bfloat16, device="cuda")
+    _call(lib, x, w, None, None, got, None, 2 * inter, 0, 2, inter, (TN, 1, 4, 1))
+    g, u = ((x.double() @ w.double().T).to(torch.bfloat16).double()).split(inter, 1)
+    # three roundings of the unit, one of each product: 4 x 2^-9, most of them shared with the reference's
+    assert rl2(got, torch.nn.functional.silu(g) * u) <= 2.0 ** -8
+
+
+@pytest.mark.parametrize("T,N,K,TN,split", [(200, 300, 512, 128, 2), (600, 1280, 5120, 192, 4), (33, 64, 192, 64, 3), (900, 640, 64, 256, 1)])
+def test_split_k_partials(lib, T, N, K, TN, split):
+    x, w = _rand(T, K, seed=7), _rand(N, K, seed=8, std=K ** -0.5)
+    part = torch.full((split, T, N), float("nan"), device="cuda")
+    _call(lib, x, w, None, None, None, part, N, 0, 1, 0, (TN, 1, 4, split))
+    assert rl2(part.double().sum(0), x.double() @ w.double().T) <= 1e-5
+
+
+_CHILD = """
+import sys, torch
+sys.path.insert(0, {root!r})
+from mlx_vlm_b200 import _native as N
+lib = N.lib()
+g = torch.Generator(device="cuda").manual_seed(9)
+for T, n, K, mode, epi in {cases!r}:
+    kp = (K + 63) // 64 * 64
+    x = torch.randn(T, K, generator=g, device="cuda")
+    xs = torch.zeros(T, 2 * kp, dtype=torch.bfloat16, device="cuda")
+    xs[:, :K] = x.to(torch.bfloat16); xs[:, kp:kp + K] = (x - xs[:, :K].float()).to(torch.bfloat16)
+    w = (torch.randn(n, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    b = torch.randn(n, generator=g, device="cuda").to(torch.bfloat16)
+    r = torch.randn(T, n, generator=g, device="cuda")
+    y = (xs[:, :K].double() + xs[:, kp:kp + K].double()) @ w.double().T + b.double()
+    if epi == 2: y = torch.nn.functional.gelu(y)
+    npad = (n + 63) // 64 * 64
+    o32, osp = torch.zeros(T, n, device="cuda"), torch.zeros(T, 2 * npad, dtype=torch.bfloat16, device="cuda")
+    for _ in range(2):
+        N.check(lib.b200_gemm_wt_f32(xs.data_ptr(), 2 * kp, w.data_ptr(), K, b.data_ptr(), r.data_ptr() if mode == 3 else 0, n,
+                                     o32.data_ptr(), n, osp.data_ptr(), 2 * npad, npad, T, n, K, 2, epi, mode, 0), "f32")
+    torch.cuda.synchronize()
+    got = o32.double() - r.double() if mode == 3 else osp[:, :n].double() + osp[:, npad:npad + n].double()
+    e = float((got - y).norm() / y.norm())
+    print(T, n, K, mode, e)
+    assert e <= (2e-6 if mode == 3 else 2.0 ** -17), e
+"""
+
+
+def test_fp32_outputs_of_split_operands(tmp_path):
+    """the fp32-accurate modes, with the configuration given by a file of measured choices (k-blocks per stage 0: pairs)"""
+    cases = [(300, 264, 128, 3, 0), (577, 1152, 584, 3, 2), (640, 520, 72, 4, 2), (200, 256, 1152, 4, 0)]
+    lines = []
+    for T, n, K, mode, _ in cases:
+        lines.append(f"{(T + 63) // 64} {n} {2 * ((K + 63) // 64 * 64)} {mode} 0 160 0 4 1")
+    path = tmp_path / "choices.txt"
+    path.write_text("\n".join(lines) + "\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _CHILD.format(root=root, cases=cases)], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, B200_WT_TUNE_FILE=str(path)))
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert path.read_text() == "\n".join(lines) + "\n"        # nothing was measured: the file's choices ran
