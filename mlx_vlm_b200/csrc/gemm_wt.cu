@@ -433,11 +433,13 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   if (warp == 0) {
     if (lane == 0) {  // ===== TMA producer =====
       for (int it = 0; it < pre; ++it) issue_x(it, it);
+      int s = 0;   // (slot and parity are counted along: no division per stage)
+      uint32_t parity = 0;
       for (int it = pre; it < n_it; ++it) {
-        const int s = it % NS;
-        w_mbar_wait(&empty_bar[s], ((it / NS) & 1) ^ 1);
+        w_mbar_wait(&empty_bar[s], parity);
         issue_w(it, s);
         issue_x(it, s);
+        if (++s == NS) s = 0, parity ^= 1;
       }
     }
   } else if (warp == 1) {
@@ -445,10 +447,10 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       // D = f32, A = B = bf16, both K-major; M = 128 weight rows, N = TN tokens
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.TN >> 3) << 17) |
                              ((uint32_t)(WT_ROWS >> 4) << 24);
-      uint32_t acc = 0;
+      uint32_t acc = 0, parity = 0;
+      int s = 0;
       for (int it = 0; it < n_it; ++it) {
-        const int s = it % NS;
-        w_mbar_wait(&full_bar[s], (it / NS) & 1);
+        w_mbar_wait(&full_bar[s], parity);
         w_fence_after();
         if (!(p.flags & 1u)) {
           const uint32_t w_lo = w_desc_lo(w_smem_u32(ring + (long)s * stage_bytes));
@@ -464,6 +466,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
           }
         }
         w_commit(&empty_bar[s]);  // frees the ring slot when these MMAs retire
+        if (++s == NS) s = 0, parity ^= 1;
       }
       w_commit(&tmem_full);
     }
