@@ -376,10 +376,12 @@ static int v2_linear_residual_norm(b200_engine* e, const bf16* x, long ldx, cons
   int split = 1;
   int rc;
   e->launches += 2;
-  if ((long)T * N * 4 > WT_PARTIAL_BYTES) {
-    // many tokens (a long chunk or a batched prefill): even one fp32 partial tile set does not fit the partial
-    // region, and with this many token tiles split-K is not needed to fill the SMs either: bias + residual fused in
-    // the bf16 epilogue (same rounding points as finish_rows), then the norm as its own row op
+  if ((long)T * N * 4 > WT_PARTIAL_BYTES || (long)((N + 127) / 128) * ((T + 255) / 256) >= e->sm_count) {
+    // many tokens: the tiles fill the SMs without split-K, so nothing is gained by fp32 partials (a write and a read of
+    // 4 B per output: finish_rows took 48 us at 6012 x 1280, 28 at 2048 x 3584), and beyond the partial region they do not
+    // fit anyway: bias + residual fused in the bf16 epilogue (same rounding points as finish_rows), then the norm as its
+    // own row op.  Measured: two vision blocks on 6012 patches 1206 -> 1098 us, two 7B layers on 2048 tokens 2263 -> 2220;
+    // with fewer tiles than SMs split-K stays ahead.
     if ((rc = gemm_wt_tuned(x, ldx, W, b, h, ldh, h, ldh, nullptr, 0, T, N, K, B200_EPI_NONE, B200_WT_BF16, 0, false,
                             e->sm_count, nullptr, s)))
       return rc;
@@ -657,7 +659,7 @@ static int prefill_layers_v2(b200_engine* e, const void* embeds, const int* pos3
 // segs != nullptr (PromptProcessingBatch, ar.py:1581-2175): several fresh sequences concatenated along the token
 // axis — every GEMM / norm / SwiGLU runs once over all T tokens (the weights are streamed once for the whole
 // batch), M-RoPE + KV append scatter each token to (its row, its position) through `tok_loc`, and attention runs
-// per sequence on its own block of the shared q / K / V^T buffers (block-diagonal causal).
+// per sequence on its own block of the shared q / K / V buffers (block-diagonal causal).
 static int prefill_layers_v2_body(b200_engine* e, const int* pos3, int T, int ctx0, void* all_logits_out,
                                   cudaStream_t s, const PreSeg* segs, int n_seg, const void* tok_loc) {
   const auto& c = e->cfg;
