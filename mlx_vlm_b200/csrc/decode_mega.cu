@@ -7,12 +7,13 @@
 //   * warp 8 of every CTA is a PRODUCER that walks the static tile schedule of the
 //     whole step and streams weight tiles (cp.async.bulk -> shared-memory ring,
 //     mbarrier complete_tx) without ever waiting for a phase boundary: the ring
-//     (up to 4 x 48 KB per SM, ~28 MB chip-wide) runs ahead across phases and layers;
+//     (up to 4 x 48 or 3 x 64 KB per SM, ~28 MB chip-wide) runs ahead across phases and layers;
 //   * warps 0..7 are CONSUMERS that execute the phases in order, separated by a
 //     software grid barrier (one atomic + acquire spin, ~1 us) instead of a kernel
 //     boundary; activations cross CTAs through L2 (ld.global.cg).
 // Rounding points follow oracle/qwen2vl.py::lm_layers_forward (same device
 // functions as the multi-kernel path in decode.cu).
+#include <climits>
 #include "mega_common.cuh"
 
 namespace b200 {
@@ -37,7 +38,7 @@ template <int MODE>
 __device__ __forceinline__ void produce_phase(const MegaPhase& g, const bf16* W, const bf16* W2,
                                               int hd, uint8_t* ring, MegaShared* sh, Ring& rg,
                                               uint64_t pol, Ring& lag, int& issued, int max_inflight,
-                                              long long* tdbg = nullptr) {
+                                              int stage_bytes, long long* tdbg = nullptr) {
   using T = PhTraits<MODE>;
   const int rows_unit = g.K * 2;
   int tn = 0;
@@ -56,7 +57,7 @@ __device__ __forceinline__ void produce_phase(const MegaPhase& g, const bf16* W,
     if (MODE != PH_QKV) rows = min(g.R, g.N - t * g.R);
     const uint32_t bytes = (uint32_t)rows * rows_unit;
     mb_expect_tx(&sh->full_bar[s], bytes * T::NRW);
-    uint8_t* dst = ring + (long)s * MEGA_STAGE;
+    uint8_t* dst = ring + (long)s * stage_bytes;
     bulk_g2s(dst, mega_tile_src<MODE>(g, W, W2, hd, t, 0), bytes, &sh->full_bar[s], pol);
     if (T::PAIR)
       bulk_g2s(dst + (long)g.R * rows_unit, mega_tile_src<MODE>(g, W, W2, hd, t, 1), bytes,
@@ -275,7 +276,7 @@ __device__ __forceinline__ void consume_phase(const MegaP& p, const MegaPhase& g
     mb_wait(&sh->full_bar[s], rg.parity(), &sh->err);
     if (tdbg && threadIdx.x == 0 && tn < 30) tdbg[tn++] = gtimer();
     rg.advance();
-    const uint8_t* base = ring + (long)s * MEGA_STAGE + (long)rloc * rows_unit;
+    const uint8_t* base = ring + (long)s * p.stage_bytes + (long)rloc * rows_unit;
     float acc[T::NRW];
     {
       float a8[T::NRW][8];
@@ -372,7 +373,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_mega(const MegaP p) {
   extern __shared__ __align__(128) uint8_t sm[];
   __shared__ MegaShared sh;
   uint8_t* ring = sm;
-  uint8_t* xs = sm + (long)p.n_stages * MEGA_STAGE;  // activation vector (GEMV phases) /
+  uint8_t* xs = sm + (long)p.n_stages * p.stage_bytes;  // activation vector (GEMV phases) /
   float* scratch = reinterpret_cast<float*>(xs);     // attention scratch (attention phase)
   uint16_t* hraw = reinterpret_cast<uint16_t*>(xs + p.scratch_bytes);  // FLOW: raw residual stream
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -413,14 +414,14 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_mega(const MegaP p) {
           l2_prefetch_phase<PH_GATEUP>(p.ph[PH_GATEUP], lw.wgu, lw.wgu + (long)d.inter * d.hidden);
           l2_prefetch_phase<PH_DRES>(p.ph[PH_DRES], lw.wd, nullptr);
         }
-        produce_phase<PH_QKV>(p.ph[PH_QKV], lw.wqkv, nullptr, d.hd, ring, &sh, rg, pol, lag, issued, mif);
-        produce_phase<PH_ORES>(p.ph[PH_ORES], lw.wo, nullptr, d.hd, ring, &sh, rg, pol, lag, issued, mif);
+        produce_phase<PH_QKV>(p.ph[PH_QKV], lw.wqkv, nullptr, d.hd, ring, &sh, rg, pol, lag, issued, mif, p.stage_bytes);
+        produce_phase<PH_ORES>(p.ph[PH_ORES], lw.wo, nullptr, d.hd, ring, &sh, rg, pol, lag, issued, mif, p.stage_bytes);
         produce_phase<PH_GATEUP>(p.ph[PH_GATEUP], lw.wgu, lw.wgu + (long)d.inter * d.hidden, d.hd,
-                                 ring, &sh, rg, pol, lag, issued, mif,
+                                 ring, &sh, rg, pol, lag, issued, mif, p.stage_bytes,
                                  (p.dbg && l == 5 && blockIdx.x == 0) ? p.dbg + 4096 + 96 : nullptr);
-        produce_phase<PH_DRES>(p.ph[PH_DRES], lw.wd, nullptr, d.hd, ring, &sh, rg, pol, lag, issued, mif);
+        produce_phase<PH_DRES>(p.ph[PH_DRES], lw.wd, nullptr, d.hd, ring, &sh, rg, pol, lag, issued, mif, p.stage_bytes);
       }
-      produce_phase<PH_HEAD>(p.ph[PH_HEAD], p.head, nullptr, d.hd, ring, &sh, rg, pol, lag, issued, mif);
+      produce_phase<PH_HEAD>(p.ph[PH_HEAD], p.head, nullptr, d.hd, ring, &sh, rg, pol, lag, issued, mif, p.stage_bytes);
     }
     return;
   }
@@ -493,13 +494,15 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_mega(const MegaP p) {
 // ---------------------------------------------------------------------------
 // host
 // ---------------------------------------------------------------------------
-static int mega_geometry(MegaPhase& g, int K, int N, bool pair, int units) {
+// R rows of K per tile (pair: of both matrices), each row shared by 8 / R warps: as many as the stage and the registers of a
+// lane (max_chx 16-byte pieces of a row) hold
+static int mega_geometry(MegaPhase& g, int K, int N, bool pair, int units, int stage, int max_chx) {
   g.K = K;
   g.N = N;
   const long unit = (long)K * 2 * (pair ? 2 : 1);
   int R = 8;
-  while (R > 1 && (R * unit > MEGA_STAGE || R > units)) R >>= 1;
-  B200_REQUIRE(R * unit <= MEGA_STAGE, "mega: K=%d does not fit a %d-byte ring stage", K, MEGA_STAGE);
+  while (R > 1 && (R * unit > stage || R > units || cdiv(cdiv(K >> 3, 8 / R), 32) > max_chx)) R >>= 1;
+  B200_REQUIRE(R * unit <= stage, "mega: K=%d does not fit a %d-byte ring stage", K, stage);
   g.R = R;
   g.S = 8 / R;
   return B200_OK;
@@ -513,21 +516,45 @@ static size_t mega_attn_scratch(const DecodeDims& d) {
   return ((att > xs ? att : xs) + 127) & ~(size_t)127;
 }
 
-int mega_fill(MegaP& p, int sm_count) {
+// Geometry of the phases and of the ring for one stage size; returns the number of stages (< 2: it does not fit)
+static int mega_ring(MegaP& p, int stage, int chh, int chi, int* ns) {
   const DecodeDims& d = p.d;
   int rc;
   const int half = d.hd / 2;
-  if ((rc = mega_geometry(p.ph[PH_QKV], d.hidden, 0, true, half))) return rc;
+  if ((rc = mega_geometry(p.ph[PH_QKV], d.hidden, 0, true, half, stage, chh))) return rc;
   B200_REQUIRE(half % p.ph[PH_QKV].R == 0, "mega: head_dim/2 %% tile rows != 0");
   p.ph[PH_QKV].tiles = (d.n_heads + 2 * d.n_kv) * (half / p.ph[PH_QKV].R);
-  if ((rc = mega_geometry(p.ph[PH_ORES], d.n_heads * d.hd, d.hidden, false, d.hidden))) return rc;
+  if ((rc = mega_geometry(p.ph[PH_ORES], d.n_heads * d.hd, d.hidden, false, d.hidden, stage, chh))) return rc;
   p.ph[PH_ORES].tiles = cdiv(d.hidden, p.ph[PH_ORES].R);
-  if ((rc = mega_geometry(p.ph[PH_GATEUP], d.hidden, d.inter, true, d.inter))) return rc;
+  if ((rc = mega_geometry(p.ph[PH_GATEUP], d.hidden, d.inter, true, d.inter, stage, chh))) return rc;
   p.ph[PH_GATEUP].tiles = cdiv(d.inter, p.ph[PH_GATEUP].R);
-  if ((rc = mega_geometry(p.ph[PH_DRES], d.inter, d.hidden, false, d.hidden))) return rc;
+  if ((rc = mega_geometry(p.ph[PH_DRES], d.inter, d.hidden, false, d.hidden, stage, chi))) return rc;
   p.ph[PH_DRES].tiles = cdiv(d.hidden, p.ph[PH_DRES].R);
-  if ((rc = mega_geometry(p.ph[PH_HEAD], d.hidden, d.vocab, false, d.vocab))) return rc;
+  if ((rc = mega_geometry(p.ph[PH_HEAD], d.hidden, d.vocab, false, d.vocab, stage, chh))) return rc;
   p.ph[PH_HEAD].tiles = cdiv(d.vocab, p.ph[PH_HEAD].R);
+  const bool hraw_in = p.flow || stage == MEGA_STAGE;   // dataflow mode: raw residual stream
+  const long hraw = hraw_in ? ((long)d.hidden * 2 + 127) & ~127L : 0;
+  *ns = (int)((227 * 1024 - 2048 - (long)p.scratch_bytes - hraw) / stage);
+  p.stage_bytes = stage;
+  p.n_stages = *ns > 8 ? 8 : *ns;
+  return B200_OK;
+}
+
+int mega_fill(MegaP& p, int sm_count) {
+  const DecodeDims& d = p.d;
+  int rc, ns = 0;
+  p.scratch_bytes = (int)mega_attn_scratch(d);
+  // Widths of 3,584 and 4,096: four rows of gate and up make a tile of 56 / 64 KB.  In 48 KB only two fit: four warps share a
+  // row, and the block barrier of their sum comes once per 28 / 32 KB, 1.07 us, which is less than the memory delivers
+  // (4.5 TB/s).  Measured at 4,096 x 14,336: gate and up 51.6 -> 35.9 us a layer (6.5 TB/s), down 23.2 -> 18.1; a step of
+  // four layers and a head of 8,192 rows behind 6000 keys: 599 -> 515 us.  Wider stages need at least three of them beside the
+  // attention's scores.  (At 1,536 four rows fit as it is, and 48 KB holds eight of them.)
+  const int wide = 4 * d.hidden * 4;
+  if (wide > MEGA_STAGE && wide <= 64 * 1024 && (rc = mega_ring(p, wide, 8, 14, &ns)) != B200_OK) return rc;
+  if (ns < 3) {
+    if ((rc = mega_ring(p, MEGA_STAGE, INT_MAX, INT_MAX, &ns))) return rc;
+    B200_REQUIRE(ns >= 2, "mega: cache capacity %d leaves no room for the weight ring", d.cap);
+  }
   const int G = d.n_heads / d.n_kv;
   int hs = (G + MEGA_ATT_G - 1) / MEGA_ATT_G;  // <= MEGA_ATT_G q heads per CTA, uneven split allowed
   if (hs == 1 && G % 2 == 0 && G >= 4) hs = 2;
@@ -535,14 +562,6 @@ int mega_fill(MegaP& p, int sm_count) {
   p.attn_ctas = d.n_kv * hs * ATT_UN;
   B200_REQUIRE(p.attn_ctas <= sm_count, "mega: %d attention CTAs > %d SMs", p.attn_ctas, sm_count);
   B200_REQUIRE(d.hd == 64 || d.hd == 128, "mega: head_dim %d (64|128)", d.hd);
-  const size_t scratch = mega_attn_scratch(d);
-  p.scratch_bytes = (int)scratch;
-  const size_t hraw = ((size_t)d.hidden * 2 + 127) & ~(size_t)127;  // dataflow mode: raw residual stream
-  const long budget = 227 * 1024 - 2048 - (long)scratch - (long)hraw;
-  int ns = (int)(budget / MEGA_STAGE);
-  B200_REQUIRE(ns >= 2, "mega: cache capacity %d leaves no room for the weight ring", d.cap);
-  p.n_stages = ns > 8 ? 8 : ns;
-  p.stage_bytes = MEGA_STAGE;
   return B200_OK;
 }
 
@@ -585,8 +604,8 @@ static int mega_launch_t(const MegaP& p, int grid, size_t smem, cudaStream_t s) 
 }
 
 int mega_launch(const MegaP& p, int sm_count, cudaStream_t s) {
-  const size_t smem = (size_t)p.n_stages * MEGA_STAGE + mega_attn_scratch(p.d) +
-                      (((size_t)p.d.hidden * 2 + 127) & ~(size_t)127);
+  const size_t smem = (size_t)p.n_stages * p.stage_bytes + mega_attn_scratch(p.d) +
+                      (p.flow || p.stage_bytes == MEGA_STAGE ? ((size_t)p.d.hidden * 2 + 127) & ~(size_t)127 : 0);
   int chh = mega_chx(p.ph[PH_QKV]);
   chh = max(chh, mega_chx(p.ph[PH_ORES]));
   chh = max(chh, mega_chx(p.ph[PH_GATEUP]));
@@ -597,6 +616,7 @@ int mega_launch(const MegaP& p, int sm_count, cudaStream_t s) {
   if (chh <= 2 && chi <= 2) return mega_launch_t<2, 2>(p, grid, smem, s);
   if (chh <= 6 && chi <= 10) return mega_launch_t<6, 10>(p, grid, smem, s);
   if (chh <= 8 && chi <= 10) return mega_launch_t<8, 10>(p, grid, smem, s);  // Qwen2-VL-7B widths
+  if (chh <= 8 && chi <= 14) return mega_launch_t<8, 14>(p, grid, smem, s);   // 4,096 wide, 14,336 in the middle
   if (chh <= 10 && chi <= 10) return mega_launch_t<10, 10>(p, grid, smem, s);
   set_error("mega: unsupported widths (hidden chunks %d, inter chunks %d per lane)", chh, chi);
   return B200_ERR_INVALID;
