@@ -9,13 +9,14 @@
 // attention_tc.cu (round 1) staged every tile with the compute threads and ran
 // load -> sync -> MMA -> wait -> softmax strictly in sequence (61 us per ViT layer, 2 % of the
 // tensor peak).  Here, per CTA = 128 query rows of one head:
-//   warp 0      TMA producer: Q once, K tiles for both passes, V^T tiles for pass 2 (3-D tensor
+//   warp 0      TMA producer: Q once, K tiles for both passes, V tiles for pass 2 (3-D tensor
 //               maps over the packed qkv buffer / the KV cache, 128B swizzle, zero-filled tails)
 //   warp 1      MMA issuer:  S[i % 2] = Qs . K^T  (M128 x N128, TMEM cols 0..255)
 //                            O += P . V           (M128 x N=hd, TMEM cols 256..)
-//               the P.V of tile j is issued AFTER the Q.K^T of tile j+1, so the tensor core
+//               the P.V of tile j is issued AFTER the Q.K^T of tile j+2, so the tensor core
 //               computes the next scores while the softmax warps work on the current ones
-//   warps 2..9  softmax: two threads per query row (64 score columns each), TMEM -> registers,
+//   warps 2..17 softmax: two groups of eight warps that take the key tiles in turn, each with a score tile and a P tile
+//               of its own; two threads per query row (64 score columns each), TMEM -> registers,
 //               pass 1: running max / sum of exp;  pass 2: p -> shared memory (the A operand)
 // V is read as it lies in the qkv buffer or the KV cache ([key][dim]): the B operand of P.V is then MN-major (dims
 // contiguous), which tcgen05 takes from the same 128-byte-swizzled 64-dim blocks that K uses.  So nothing transposes V:
@@ -36,7 +37,7 @@ namespace {
 
 constexpr int FA_TQ = 128, FA_TK = 128;
 constexpr int FA_BLK = 16 * 1024;       // one 128-row x 64-column bf16 operand block
-constexpr int FA_THREADS = 320;         // producer warp, MMA warp, 8 softmax warps
+constexpr int FA_THREADS = 576;         // producer warp, MMA warp, 2 groups of 8 softmax warps
 
 struct FaParams {
   bf16* out;
@@ -48,7 +49,7 @@ struct FaParams {
 };
 
 struct FaBars {
-  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], s_empty[2], p_full, p_empty,
+  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], s_empty[2], p_full[2], p_empty[2],
       o_full;
 };
 
@@ -160,7 +161,7 @@ __device__ __forceinline__ void f_tmem_ld16(uint32_t taddr, uint32_t* r) {
       : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void f_sbar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void f_sbar() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 // 2^x on the SFU (one MUFU instruction, rel. error 2^-22: far below the bf16 rounding of p that follows)
 __device__ __forceinline__ float f_ex2(float x) {
   float y;
@@ -182,13 +183,13 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   extern __shared__ uint8_t fa_smem_raw[];
   __shared__ FaBars bars;
   __shared__ uint32_t tmem_slot;
-  __shared__ float2 stat[2][FA_TQ];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(fa_smem_raw) + 1023) &
                                            ~static_cast<uintptr_t>(1023));
   uint8_t* Qs = sm;                          // [128 q][128 d]            2 k-blocks
   uint8_t* Ks = sm + 2 * FA_BLK;             // 2 slots x [128 keys][128 d]
   uint8_t* Vs = sm + 6 * FA_BLK;             // 2 slots x (VT: 2 key-blocks x [hdp d][64 keys], else 2 dim-blocks x [128 keys][64 d])
-  uint8_t* Ps = sm + 10 * FA_BLK;            // [128 q][128 keys]
+  uint8_t* Ps = sm + 10 * FA_BLK;            // 2 slots x [128 q][128 keys]
+  float2* stat = reinterpret_cast<float2*>(Ps);   // [2 groups x 2 halves][128 q], between the passes
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = blockIdx.x, kvh = h / (p.n_heads / p.n_kv);
   // causal: the query tiles with the most keys start first, of all heads, so that the short ones fill the last wave
@@ -213,9 +214,9 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       f_init(&bars.v_empty[i], 1);
       f_init(&bars.s_full[i], 1);
       f_init(&bars.s_empty[i], 256);
+      f_init(&bars.p_full[i], 256);
+      f_init(&bars.p_empty[i], 1);
     }
-    f_init(&bars.p_full, 256);
-    f_init(&bars.p_empty, 1);
     f_init(&bars.o_full, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -237,26 +238,30 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (lane == 0) {  // ===== TMA producer =====
       f_expect_tx(&bars.q_full, (uint32_t)kbq * FA_BLK);
       for (int c = 0; c < kbq; ++c) f_tma_3d(Qs + c * FA_BLK, &tmQ, &bars.q_full, c * 64, h, p.q0 + row0);
+      auto load_v = [&](int j) {
+        const int sv = j & 1;
+        f_wait(&bars.v_empty[sv], ((j >> 1) & 1) ^ 1, dead);
+        if constexpr (VT) {
+          f_expect_tx(&bars.v_full[sv], 2u * (uint32_t)vblk);
+          for (int c = 0; c < 2; ++c)
+            f_tma_3d(Vs + sv * 2 * FA_BLK + c * vblk, &tmV, &bars.v_full[sv], p.k0 + j * FA_TK + c * 64, 0, kvh);
+        } else {
+          f_expect_tx(&bars.v_full[sv], (uint32_t)kbq * FA_BLK);
+          for (int c = 0; c < kbq; ++c)
+            f_tma_3d(Vs + sv * 2 * FA_BLK + c * FA_BLK, &tmV, &bars.v_full[sv], c * 64, kvh, p.k0 + j * FA_TK);
+        }
+      };
+      int jk = 0;   // key tile of step i
       for (int i = 0; i < 2 * n_tiles; ++i) {
-        const int j = i % n_tiles, s = i & 1;
+        const int s = i & 1;
         f_wait(&bars.k_empty[s], ((i >> 1) & 1) ^ 1, dead);
         f_expect_tx(&bars.k_full[s], (uint32_t)kbq * FA_BLK);
         for (int c = 0; c < kbq; ++c)
-          f_tma_3d(Ks + s * 2 * FA_BLK + c * FA_BLK, &tmK, &bars.k_full[s], c * 64, kvh, p.k0 + j * FA_TK);
-        if (i >= n_tiles) {
-          const int sv = j & 1;
-          f_wait(&bars.v_empty[sv], ((j >> 1) & 1) ^ 1, dead);
-          if constexpr (VT) {
-            f_expect_tx(&bars.v_full[sv], 2u * (uint32_t)vblk);
-            for (int c = 0; c < 2; ++c)
-              f_tma_3d(Vs + sv * 2 * FA_BLK + c * vblk, &tmV, &bars.v_full[sv], p.k0 + j * FA_TK + c * 64, 0, kvh);
-          } else {
-            f_expect_tx(&bars.v_full[sv], (uint32_t)kbq * FA_BLK);
-            for (int c = 0; c < kbq; ++c)
-              f_tma_3d(Vs + sv * 2 * FA_BLK + c * FA_BLK, &tmV, &bars.v_full[sv], c * 64, kvh, p.k0 + j * FA_TK);
-          }
-        }
+          f_tma_3d(Ks + s * 2 * FA_BLK + c * FA_BLK, &tmK, &bars.k_full[s], c * 64, kvh, p.k0 + jk * FA_TK);
+        if (++jk == n_tiles) jk = 0;
+        if (i >= n_tiles + 2) load_v(i - n_tiles - 2);   // (in the order of the products: a wait for V holds up no K before it)
       }
+      for (int j = max(0, n_tiles - 2); j < n_tiles; ++j) load_v(j);
     }
   } else if (warp == 1) {
     if (lane == 0) {  // ===== MMA issuer =====
@@ -264,23 +269,26 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       // (bit 16: the B operand is MN-major)
       const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (VT ? 0u : 1u << 16) | ((uint32_t)(p.hdp >> 3) << 17) |
                                (8u << 24);
-      const uint32_t q_lo = f_desc_lo(f_u32(Qs)), p_lo = f_desc_lo(f_u32(Ps));
+      const uint32_t q_lo = f_desc_lo(f_u32(Qs));
       const int ksteps = p.hdp >> 4;
       auto do_pv = [&](int j) {
-        const int sv = j & 1;
-        f_wait(&bars.p_full, j & 1, dead);
+        const int sv = j & 1, sp = (n_tiles + j) & 1;
+        const uint32_t p_lo = f_desc_lo(f_u32(Ps + sp * 2 * FA_BLK));
+        f_wait(&bars.p_full[sp], (j >> 1) & 1, dead);
         f_wait(&bars.v_full[sv], (j >> 1) & 1, dead);
         f_fence_after();
         const uint32_t v_lo = VT ? f_desc_lo(f_u32(Vs + sv * 2 * FA_BLK)) : f_desc_lo_mn(f_u32(Vs + sv * 2 * FA_BLK));
         // (groups of 16 keys that lie wholly behind the segment's last key are left out)
         const int ks_n = VT ? FA_TK / 16 : min(FA_TK / 16, (S - j * FA_TK + 15) >> 4);
-        for (int ks = 0; ks < ks_n; ++ks) {
+#pragma unroll
+        for (int ks = 0; ks < FA_TK / 16; ++ks) {
+          if (ks >= ks_n) break;
           const uint32_t a = p_lo + (uint32_t)((ks >> 2) * (FA_BLK >> 4) + (ks & 3) * 2);
           // VT: 32 bytes along a 64-key row; else 16 rows of 128 bytes
           const uint32_t b = VT ? v_lo + (uint32_t)((ks >> 2) * (vblk >> 4) + (ks & 3) * 2) : v_lo + (uint32_t)(ks * (2048 >> 4));
           f_umma(tmem + 256, a, b, F_DESC_HI, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
         }
-        f_commit(&bars.p_empty);
+        f_commit(&bars.p_empty[sp]);
         f_commit(&bars.v_empty[sv]);
       };
       f_wait(&bars.q_full, 0, dead);
@@ -290,20 +298,22 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         f_wait(&bars.s_empty[s], ((i >> 1) & 1) ^ 1, dead);
         f_fence_after();
         const uint32_t k_lo = f_desc_lo(f_u32(Ks + s * 2 * FA_BLK));
-        for (int ks = 0; ks < ksteps; ++ks) {
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) {
+          if (ks >= ksteps) break;
           const uint32_t off = (uint32_t)((ks >> 2) * (FA_BLK >> 4) + (ks & 3) * 2);
           f_umma(tmem + (uint32_t)s * 128u, q_lo + off, k_lo + off, F_DESC_HI, idesc_s, ks > 0 ? 1u : 0u);
         }
         f_commit(&bars.k_empty[s]);
         f_commit(&bars.s_full[s]);
-        if (i > n_tiles) do_pv(i - n_tiles - 1);  // P.V of the previous pass-2 tile, under this Q.K^T
+        if (i >= n_tiles + 2) do_pv(i - n_tiles - 2);  // P.V of the group's previous pass-2 tile, under this Q.K^T
       }
-      do_pv(n_tiles - 1);
+      for (int j = max(0, n_tiles - 2); j < n_tiles; ++j) do_pv(j);
       f_commit(&bars.o_full);
     }
   } else {
-    // ===== softmax warps: thread = (query row, score-column half) =====
-    const int q4 = warp & 3, half = (warp - 2) >> 2;
+    // ===== softmax warps: thread = (group, query row, score-column half) =====
+    const int q4 = warp & 3, half = ((warp - 2) >> 2) & 1, grp = (warp - 2) >> 3;
     const int row = q4 * 32 + lane;
     const int qi = row0 + row;
     const int vis = (qi < p.Lq) ? (p.causal ? min(S, S - p.Lq + qi + 1) : S) : S;
@@ -315,11 +325,13 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     // product as soon as it is in registers.  What is left is the SFU: 128 x 128 exponentials at 16 a cycle per pass.
     // Measured (element by element -> pairs, with the long query tiles first): 2048 queries behind 2048 keys, 28 heads of
     // 128: 354 -> 249 us; 8 prompts of about 608 tokens, 32 heads of 128: 154 -> 130; 576 patches, 16 heads of 80: 24 -> 19.
+    // Two groups of warps, one exponentiating while the other waits, loads and rounds: two layers of the first 2220 -> 2175 us,
+    // two vision blocks on 6012 patches (16 heads of 80) 1098 -> 1082.
     const uint64_t log2e = f2(LOG2E, LOG2E);
     uint32_t pk[32];
     float m = -INFINITY, l = 0.f;
-    for (int i = 0; i < n_tiles; ++i) {  // ---- pass 1: row max and sum of exp over bf16 scores ----
-      const int s = i & 1;
+    for (int i = grp; i < n_tiles; i += 2) {  // ---- pass 1: row max and sum of exp over bf16 scores ----
+      const int s = grp;
       f_wait(&bars.s_full[s], (i >> 1) & 1, dead);
       __syncwarp();
       f_fence_after();
@@ -344,17 +356,22 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         m = mn;
       }
     }
-    stat[half][row] = make_float2(m, l);
+    stat[(2 * grp + half) * FA_TQ + row] = make_float2(m, l);
     f_sbar();
     {
-      const float2 a = stat[0][row], b = stat[1][row];
-      m = fmaxf(a.x, b.x);
-      l = (a.y > 0.f ? a.y * f_ex2((a.x - m) * LOG2E) : 0.f) + (b.y > 0.f ? b.y * f_ex2((b.x - m) * LOG2E) : 0.f);
+      float2 a[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[e] = stat[e * FA_TQ + row];
+      m = fmaxf(fmaxf(a[0].x, a[1].x), fmaxf(a[2].x, a[3].x));
+      l = 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) l += a[e].y > 0.f ? a[e].y * f_ex2((a[e].x - m) * LOG2E) : 0.f;
     }
+    f_sbar();   // (the first P tile goes where the statistics were)
     const float inv_l = 1.0f / l;
     const uint64_t nbm = f2(-m * LOG2E, -m * LOG2E), inv2 = f2(inv_l, inv_l);
-    for (int j = 0; j < n_tiles; ++j) {  // ---- pass 2: p = bf16(exp(s - m) / l) -> shared memory ----
-      const int i = n_tiles + j, s = i & 1;
+    for (int j = (n_tiles ^ grp) & 1; j < n_tiles; j += 2) {  // ---- pass 2: p = bf16(exp(s - m) / l) -> shared memory ----
+      const int i = n_tiles + j, s = grp;
       f_wait(&bars.s_full[s], (i >> 1) & 1, dead);
       __syncwarp();
       f_fence_after();
@@ -367,8 +384,8 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const uint64_t w = mul2(f2(f_ex2(f2_lo(x)), f_ex2(f2_hi(x))), inv2);
         pk[e] = pack2(f2_lo(w), f2_hi(w));
       }
-      f_wait(&bars.p_empty, (j & 1) ^ 1, dead);  // the previous P.V has consumed the P tile
-      uint8_t* prow = Ps + half * FA_BLK + row * 128;
+      f_wait(&bars.p_empty[s], ((j >> 1) & 1) ^ 1, dead);  // the group's previous P.V has consumed the P tile
+      uint8_t* prow = Ps + (2 * s + half) * FA_BLK + row * 128;
 #pragma unroll
       for (int c = 0; c < 8; ++c)
         *reinterpret_cast<uint4*>(prow + ((c ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
@@ -379,7 +396,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (first < FA_TK && first != end) {
           f_wait(&bars.v_full[j & 1], (j >> 1) & 1, dead);
           const int per = kbq * 8;
-          for (int idx = threadIdx.x - 64; idx < (end - first) * per; idx += 256) {
+          for (int idx = (threadIdx.x - 64) & 255; idx < (end - first) * per; idx += 256) {
             const int r = first + idx / per, ch = idx % per;
             *reinterpret_cast<uint4*>(Vs + (j & 1) * 2 * FA_BLK + (ch >> 3) * FA_BLK + r * 128 + (ch & 7) * 16) =
                 make_uint4(0, 0, 0, 0);
@@ -387,13 +404,13 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
       }
       f_fence_async();  // generic-proxy writes of P -> visible to the tensor core (async proxy)
-      f_arrive(&bars.p_full);
+      f_arrive(&bars.p_full[s]);
     }
-    // ---- epilogue: O row -> bf16 -> global (16-column chunks alternate between the row's two threads) ----
+    // ---- epilogue: O row -> bf16 -> global (16-column chunks go round the row's four threads) ----
     f_wait(&bars.o_full, 0, dead);
     f_fence_after();
     bf16* orow = p.out + (long)(p.q0 + qi) * p.o_ts + (long)h * p.hd;
-    for (int c0 = 16 * half; c0 < p.hd; c0 += 32) {
+    for (int c0 = 16 * (2 * grp + half); c0 < p.hd; c0 += 64) {
       uint32_t r[16];
       f_tmem_ld16(t_row + 256u + (uint32_t)c0, r);
       if (dead)
@@ -537,7 +554,7 @@ int attention_fa(const void* q, long q_ts, long q_hs, const void* k, long k_ts, 
   if (rc) return rc;
   const auto kern = v_transposed ? attention_fa_kernel<true> : attention_fa_kernel<false>;
   static unsigned long long set_mask[2] = {0ull, 0ull};
-  const size_t smem = 12 * FA_BLK + 1024;
+  const size_t smem = 14 * FA_BLK + 1024;
   if (first_use_on_device(&set_mask[v_transposed]))
     B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   FaParams p;
