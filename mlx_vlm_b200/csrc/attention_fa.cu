@@ -11,10 +11,9 @@
 // tensor peak).  Here, per CTA = 128 query rows of one head:
 //   warp 0      TMA producer: Q once, K tiles for both passes, V tiles for pass 2 (3-D tensor
 //               maps over the packed qkv buffer / the KV cache, 128B swizzle, zero-filled tails)
-//   warp 1      MMA issuer:  S[i % 2] = Qs . K^T  (M128 x N128, TMEM cols 0..255)
-//                            O += P . V           (M128 x N=hd, TMEM cols 256..)
-//               the P.V of tile j is issued AFTER the Q.K^T of tile j+2, so the tensor core
-//               computes the next scores while the softmax warps work on the current ones
+//   warps 1, 18 issue S[i % 2] = Qs . K^T of the even / odd steps (M128 x N128, TMEM cols 0..255)
+//   warp 19     issues O += P . V (M128 x N=hd, TMEM cols 256..).  Three threads, because a thread that waits does not issue:
+//               the waits of one product (0.2 us of 0.5, ready or not) pass while another thread's keeps the tensor core busy
 //   warps 2..17 softmax: two groups of eight warps that take the key tiles in turn, each with a score tile and a P tile
 //               of its own; two threads per query row (64 score columns each), TMEM -> registers,
 //               pass 1: running max / sum of exp;  pass 2: p -> shared memory (the A operand)
@@ -37,7 +36,7 @@ namespace {
 
 constexpr int FA_TQ = 128, FA_TK = 128;
 constexpr int FA_BLK = 16 * 1024;       // one 128-row x 64-column bf16 operand block
-constexpr int FA_THREADS = 576;         // producer warp, MMA warp, 2 groups of 8 softmax warps
+constexpr int FA_THREADS = 640;         // producer warp, 3 MMA warps, 2 groups of 8 softmax warps
 
 struct FaParams {
   bf16* out;
@@ -263,21 +262,38 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       for (int j = max(0, n_tiles - 2); j < n_tiles; ++j) load_v(j);
     }
-  } else if (warp == 1) {
-    if (lane == 0) {  // ===== MMA issuer =====
+  } else if (warp == 1 || warp == 18) {
+    if (lane == 0) {  // ===== issuer of Q.K^T, of every other step =====
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(FA_TK >> 3) << 17) | (8u << 24);
+      const int ksteps = p.hdp >> 4, s = warp == 1 ? 0 : 1;
+      const uint32_t q_lo = f_desc_lo(f_u32(Qs)), k_lo = f_desc_lo(f_u32(Ks + s * 2 * FA_BLK)), d = tmem + (uint32_t)s * 128u;
+      f_wait(&bars.q_full, 0, dead);
+      for (int i = s; i < 2 * n_tiles; i += 2) {
+        f_wait(&bars.k_full[s], (i >> 1) & 1, dead);
+        f_wait(&bars.s_empty[s], ((i >> 1) & 1) ^ 1, dead);
+        f_fence_after();
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) {
+          if (ks >= ksteps) break;
+          const uint32_t off = (uint32_t)((ks >> 2) * (FA_BLK >> 4) + (ks & 3) * 2);
+          f_umma(d, q_lo + off, k_lo + off, F_DESC_HI, idesc_s, ks > 0 ? 1u : 0u);
+        }
+        f_commit(&bars.k_empty[s]);
+        f_commit(&bars.s_full[s]);
+      }
+    }
+  } else if (warp == 19) {
+    if (lane == 0) {  // ===== issuer of P.V =====
       // (bit 16: the B operand is MN-major)
       const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (VT ? 0u : 1u << 16) | ((uint32_t)(p.hdp >> 3) << 17) |
                                (8u << 24);
-      const uint32_t q_lo = f_desc_lo(f_u32(Qs));
-      const int ksteps = p.hdp >> 4;
-      auto do_pv = [&](int j) {
+      for (int j = 0; j < n_tiles; ++j) {
         const int sv = j & 1, sp = (n_tiles + j) & 1;
         const uint32_t p_lo = f_desc_lo(f_u32(Ps + sp * 2 * FA_BLK));
-        f_wait(&bars.p_full[sp], (j >> 1) & 1, dead);
-        f_wait(&bars.v_full[sv], (j >> 1) & 1, dead);
-        f_fence_after();
         const uint32_t v_lo = VT ? f_desc_lo(f_u32(Vs + sv * 2 * FA_BLK)) : f_desc_lo_mn(f_u32(Vs + sv * 2 * FA_BLK));
+        f_wait(&bars.v_full[sv], (j >> 1) & 1, dead);
+        f_wait(&bars.p_full[sp], (j >> 1) & 1, dead);
+        f_fence_after();
         // (groups of 16 keys that lie wholly behind the segment's last key are left out)
         const int ks_n = VT ? FA_TK / 16 : min(FA_TK / 16, (S - j * FA_TK + 15) >> 4);
 #pragma unroll
@@ -290,25 +306,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
         f_commit(&bars.p_empty[sp]);
         f_commit(&bars.v_empty[sv]);
-      };
-      f_wait(&bars.q_full, 0, dead);
-      for (int i = 0; i < 2 * n_tiles; ++i) {
-        const int s = i & 1;
-        f_wait(&bars.k_full[s], (i >> 1) & 1, dead);
-        f_wait(&bars.s_empty[s], ((i >> 1) & 1) ^ 1, dead);
-        f_fence_after();
-        const uint32_t k_lo = f_desc_lo(f_u32(Ks + s * 2 * FA_BLK));
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          if (ks >= ksteps) break;
-          const uint32_t off = (uint32_t)((ks >> 2) * (FA_BLK >> 4) + (ks & 3) * 2);
-          f_umma(tmem + (uint32_t)s * 128u, q_lo + off, k_lo + off, F_DESC_HI, idesc_s, ks > 0 ? 1u : 0u);
-        }
-        f_commit(&bars.k_empty[s]);
-        f_commit(&bars.s_full[s]);
-        if (i >= n_tiles + 2) do_pv(i - n_tiles - 2);  // P.V of the group's previous pass-2 tile, under this Q.K^T
       }
-      for (int j = max(0, n_tiles - 2); j < n_tiles; ++j) do_pv(j);
       f_commit(&bars.o_full);
     }
   } else {
@@ -326,7 +324,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     // Measured (element by element -> pairs, with the long query tiles first): 2048 queries behind 2048 keys, 28 heads of
     // 128: 354 -> 249 us; 8 prompts of about 608 tokens, 32 heads of 128: 154 -> 130; 576 patches, 16 heads of 80: 24 -> 19.
     // Two groups of warps, one exponentiating while the other waits, loads and rounds: two layers of the first 2220 -> 2175 us,
-    // two vision blocks on 6012 patches (16 heads of 80) 1098 -> 1082.
+    // two vision blocks on 6012 patches (16 heads of 80) 1098 -> 1082; with an issuer for each product 2111 and 1053.
     const uint64_t log2e = f2(LOG2E, LOG2E);
     uint32_t pk[32];
     float m = -INFINITY, l = 0.f;
