@@ -355,7 +355,7 @@ def c3_leg(dev, args):
     prefill only: pinned-host pixel_values -> CLIP tower (23 of 24 blocks: feature layer -2) -> projector
     -> merge -> LM prefill of the 8 requests (576 image + 32 text tokens each) incl. the first token.
     The tower is fp32-accurate like the reference's (split-operand tcgen05 GEMMs: every Linear runs as
-    W.x_hi + W.x_lo, i.e. 2x the algorithmic MMA flops; attention / LayerNorm in fp32 on the CUDA cores)."""
+    W.x_hi + W.x_lo, i.e. 2x the algorithmic MMA flops; the attention on three bf16 parts per operand, LayerNorm in fp32)."""
     import numpy as np
     import torch
     from mlx_vlm_b200.models.cache import make_prompt_cache
