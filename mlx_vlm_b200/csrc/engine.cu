@@ -105,7 +105,7 @@ struct b200_engine {
   int tc_alias = 1;
   int tc_inflight = 2;
   int fma_inflight = 0, l2_prefetch = 0, l2_skip = 2;
-  int flow = 0;  // k_mega dataflow mode (set_mega(4) / B200_MEGA_FLOW=1): measured slower, see DESIGN.md
+  int flow = 0;  // k_mega dataflow mode (set_mega(4) / B200_MEGA_FLOW=1): measured slower
   unsigned long long* flow_words = nullptr;
   float* att_part = nullptr;
   float* att_stats = nullptr;
