@@ -1136,23 +1136,26 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
 // the first candidate within 3 % of the best wins, so the choice is stable run to run.
 // B200_WT_TUNE=0 uses the cost model (gemm_wt_auto) instead.
 // ---------------------------------------------------------------------------------------------
+// groups: column groups of the product (0: a plain Linear).  They multiply the tiles and take no CTA pairs, so the choice
+// of a plain product of the same T, N and K is not one for them.
 struct TuneKey {
-  int tb, N, K, mode, split_ok, dev;
+  int tb, N, K, mode, split_ok, groups, dev;
   bool operator==(const TuneKey& o) const {
-    return tb == o.tb && N == o.N && K == o.K && mode == o.mode && split_ok == o.split_ok && dev == o.dev;
+    return tb == o.tb && N == o.N && K == o.K && mode == o.mode && split_ok == o.split_ok && groups == o.groups && dev == o.dev;
   }
 };
 struct TuneHash {
   size_t operator()(const TuneKey& k) const {
     size_t h = (size_t)k.tb;
-    for (int v : {k.N, k.K, k.mode, k.split_ok, k.dev}) h = h * 1000003u ^ (size_t)v;
+    for (int v : {k.N, k.K, k.mode, k.split_ok, k.groups, k.dev}) h = h * 1000003u ^ (size_t)v;
     return h;
   }
 };
 
 // B200_WT_TUNE_FILE=<path>: measured choices are appended to the file and read back at the first call of a
 // later process, so a service does not re-measure at every start and a profiler run (whose serialised
-// replays distort the measurement) uses exactly the production configurations.
+// replays distort the measurement) uses exactly the production configurations.  A line: token bucket, N, K, mode, split
+// allowed, TN, KS, stages, split, column groups (a line without the last is a plain product's).
 static const char* tune_file() {
   static const char* f = getenv("B200_WT_TUNE_FILE");
   return (f && *f) ? f : nullptr;
@@ -1177,7 +1180,8 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
   const int kb_total = cdiv(K, WT_BK);
   int dev = 0;
   B200_CUDA(cudaGetDevice(&dev));
-  const TuneKey key{(T + 63) / 64, N, K, mode, allow_split ? 1 : 0, dev};
+  const int groups = ext ? ext->col_groups : 0;
+  const TuneKey key{(T + 63) / 64, N, K, mode, allow_split ? 1 : 0, groups, dev};
   WtConfig cfg;
   bool have = false;
   {
@@ -1187,10 +1191,14 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
       file_read = true;
       if (const char* path = tune_file()) {
         if (FILE* fp = fopen(path, "r")) {
-          int tb, n, k, md, so, tn, ks, stg, sp;
-          while (fscanf(fp, "%d %d %d %d %d %d %d %d %d", &tb, &n, &k, &md, &so, &tn, &ks, &stg, &sp) == 9)
-            if (tn >= 16 && tn <= 256 && tn % (ks ? 16 : 32) == 0 && ks >= 0 && stg >= 2 && stg <= WT_MAX_STAGES && sp >= 1)
-              cache[TuneKey{tb, n, k, md, so, dev}] = WtConfig{tn, ks, stg, sp};
+          char line[256];
+          while (fgets(line, sizeof line, fp)) {
+            int tb, n, k, md, so, tn, ks, stg, sp, g = 0;
+            if (sscanf(line, "%d %d %d %d %d %d %d %d %d %d", &tb, &n, &k, &md, &so, &tn, &ks, &stg, &sp, &g) < 9) continue;
+            if (tn >= 16 && tn <= 256 && tn % (ks ? 16 : 32) == 0 && ks >= (g > 0 ? 1 : 0) && stg >= 2 &&
+                stg <= (ks ? WT_MAX_STAGES : WP_MAX_STAGES) && sp >= 1)
+              cache[TuneKey{tb, n, k, md, so, g, dev}] = WtConfig{tn, ks, stg, sp};
+          }
           fclose(fp);
         }
       }
@@ -1372,8 +1380,8 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
     cache[key] = cfg;
     if (const char* path = tune_file()) {
       if (FILE* fp = fopen(path, "a")) {
-        fprintf(fp, "%d %d %d %d %d %d %d %d %d\n", key.tb, key.N, key.K, key.mode, key.split_ok, cfg.TN, cfg.KS,
-                cfg.stages, cfg.split);
+        fprintf(fp, "%d %d %d %d %d %d %d %d %d %d\n", key.tb, key.N, key.K, key.mode, key.split_ok, cfg.TN, cfg.KS,
+                cfg.stages, cfg.split, key.groups);
         fclose(fp);
       }
     }

@@ -114,3 +114,40 @@ def test_fp32_outputs_of_split_operands(tmp_path):
                        env=dict(os.environ, B200_WT_TUNE_FILE=str(path)))
     assert r.returncode == 0, r.stdout + r.stderr
     assert path.read_text() == "\n".join(lines) + "\n"        # nothing was measured: the file's choices ran
+
+
+_CHILD_HEADS = """
+import sys, torch
+sys.path.insert(0, {root!r})
+from mlx_vlm_b200 import _native as N
+lib = N.lib()
+T, n, K, heads = 300, 256, 64, 3
+g = torch.Generator(device="cuda").manual_seed(10)
+x = torch.randn(T, heads * K, generator=g, device="cuda").to(torch.bfloat16)
+w = (torch.randn(heads, n, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+one, out = torch.zeros(T, n, device="cuda"), torch.zeros(T, heads * n, device="cuda")
+for _ in range(2):
+    N.check(lib.b200_gemm_wt_f32(x.data_ptr(), heads * K, w.data_ptr(), K, 0, 0, 0, one.data_ptr(), n, 0, 0, 0, T, n, K, 1, 0, 3, 0), "f32")
+    N.check(lib.b200_gemm_wt_f32_heads(x.data_ptr(), heads * K, heads * K, K, w.data_ptr(), K, out.data_ptr(), heads * n, n, T, heads,
+                                       n, K, 1, 0, 0), "heads")
+torch.cuda.synchronize()
+want = torch.einsum("thk,hnk->thn", x.double().view(T, heads, K), w.double())
+for got, ref in ((one, want[:, 0]), (out.view(T, heads, n), want)):
+    e = float((got.double() - ref).norm() / ref.norm())
+    print(e)
+    assert e <= 2e-6, e
+"""
+
+
+@pytest.mark.parametrize("line", ["5 256 64 3 0 160 0 4 1", "5 256 64 3 0 160 0 4 1\n5 256 64 3 0 160 0 4 1 3"])
+def test_column_groups_beside_a_plain_product_of_pairs(tmp_path, line):
+    """a per-head product of the tokens, rows and k of a plain one that runs on pairs keeps a choice of its own; a file's line that
+    gives pairs to column groups is passed over"""
+    path = tmp_path / "choices.txt"
+    path.write_text(line + "\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _CHILD_HEADS.format(root=root)], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, B200_WT_TUNE_FILE=str(path)))
+    assert r.returncode == 0, r.stdout + r.stderr
+    added = path.read_text()[len(line) + 1:].split()
+    assert added[:5] == ["5", "256", "64", "3", "0"] and int(added[6]) >= 1 and added[9] == "3" and len(added) == 10
