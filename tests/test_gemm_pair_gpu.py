@@ -126,10 +126,13 @@ g = torch.Generator(device="cuda").manual_seed(10)
 x = torch.randn(T, heads * K, generator=g, device="cuda").to(torch.bfloat16)
 w = (torch.randn(heads, n, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
 one, out = torch.zeros(T, n, device="cuda"), torch.zeros(T, heads * n, device="cuda")
+torch.cuda.synchronize()
+stream = torch.cuda.Stream()       # (choices are measured under capture, which the default stream does not take)
 for _ in range(2):
-    N.check(lib.b200_gemm_wt_f32(x.data_ptr(), heads * K, w.data_ptr(), K, 0, 0, 0, one.data_ptr(), n, 0, 0, 0, T, n, K, 1, 0, 3, 0), "f32")
+    N.check(lib.b200_gemm_wt_f32(x.data_ptr(), heads * K, w.data_ptr(), K, 0, 0, 0, one.data_ptr(), n, 0, 0, 0, T, n, K, 1, 0, 3,
+                                 stream.cuda_stream), "f32")
     N.check(lib.b200_gemm_wt_f32_heads(x.data_ptr(), heads * K, heads * K, K, w.data_ptr(), K, out.data_ptr(), heads * n, n, T, heads,
-                                       n, K, 1, 0, 0), "heads")
+                                       n, K, 1, 0, stream.cuda_stream), "heads")
 torch.cuda.synchronize()
 want = torch.einsum("thk,hnk->thn", x.double().view(T, heads, K), w.double())
 for got, ref in ((one, want[:, 0]), (out.view(T, heads, n), want)):
