@@ -3,7 +3,7 @@
 // Every fp32 operand is carried as THREE bf16 parts, x = h + m + l (h = bf16(x), m = bf16(x - h), l = bf16(x - h - m): 24
 // mantissa bits, the exponent range of fp32), and a product of two operands as the six products of parts that are not below
 // fp32's own rounding: l.h + h.l + m.m + m.h + h.m + h.h, added smallest first so that the small ones meet an accumulator
-// of their size.  tcgen05 truncates its fp32 accumulator at every step, so no sum runs over more than one tile: the scores of
+// of their size.  Rows with a result that is not finite are computed again without parts (plain_row).  tcgen05 truncates its fp32 accumulator at every step, so no sum runs over more than one tile: the scores of
 // a tile (one head dimension) and its P.V (64 keys) each start from zero in tensor memory, and the softmax threads add the
 // tile's P.V to their fp32 registers with rounding.  Error against 64 bits, relative: 2.2e-7 at 577 keys of 64 dims, 2.5e-7 at
 // 1024 of 72 (a register-tiled FMA kernel: 5.2e-7, 6.5e-7).
@@ -111,7 +111,7 @@ __device__ __forceinline__ void t_st8(uint32_t taddr, const uint32_t* r) {
                : "memory");
 }
 
-// 2^x on the SFU, as in __expf (without its care for results below 2^-126, which are 0 beside the row's largest weight, 1)
+// 2^x on the SFU; results below 2^-126 are 0, beside a row's largest weight of 1
 __device__ __forceinline__ float t_ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -201,6 +201,43 @@ __device__ __forceinline__ void store_values(uint8_t* dst, int part_bytes, const
   }
 }
 
+// One query row by one warp in plain fp32 arithmetic: p.hd floats to out.  The parts of a number that is no finite bf16 (an
+// infinity, a NaN, a magnitude above 3.39e38) are infinities and NaN that the row's other products would spread, so a row
+// with such a result is computed again: a key that scores -inf has weight 0, an infinite value stays in its own dimension.
+__device__ __noinline__ void plain_row(const AttnF32P& p, const float* q, const float* kb, const float* vb, int S,
+                                       const unsigned char* mask, float* out, int lane) {
+  auto score = [&](int j) {
+    if (j >= S || (mask && !mask[j])) return -INFINITY;
+    float s = 0.f;
+    for (int d = 0; d < p.hd; d += 4) {
+      const float4 a = *reinterpret_cast<const float4*>(q + d), b = *reinterpret_cast<const float4*>(kb + (long)j * p.k_ts + d);
+      s = fmaf(a.x * p.scale, b.x, s);
+      s = fmaf(a.y * p.scale, b.y, s);
+      s = fmaf(a.z * p.scale, b.z, s);
+      s = fmaf(a.w * p.scale, b.w, s);
+    }
+    return s;
+  };
+  float m = -INFINITY, l = 0.f, o[3] = {0.f, 0.f, 0.f};
+  for (int j = lane; j < S; j += 32) m = fmaxf(m, score(j));
+  m = warp_max(m);
+  for (int j0 = 0; j0 < S; j0 += 32) {
+    const int j = j0 + lane;
+    const float w = j < S && (!mask || mask[j]) ? expf(score(j) - m) : 0.f;
+    l += w;
+    for (int i = 0; i < min(32, S - j0); ++i) {
+      const float wi = __shfl_sync(0xffffffffu, w, i);
+#pragma unroll
+      for (int e = 0; e < 3; ++e)
+        if (lane + 32 * e < p.hd) o[e] = fmaf(wi, vb[(long)(j0 + i) * p.v_ts + lane + 32 * e], o[e]);
+    }
+  }
+  const float inv = 1.0f / warp_sum(l);
+#pragma unroll
+  for (int e = 0; e < 3; ++e)
+    if (lane + 32 * e < p.hd) out[lane + 32 * e] = o[e] * inv;
+}
+
 template <int HDP>
 constexpr int tc_q_part() { return HDP / 8 * TC_QB; }
 template <int HDP>
@@ -211,11 +248,12 @@ template <int HDP>
 constexpr int tc_smem() { return 3 * tc_q_part<HDP>() + 6 * tc_k_part<HDP>() + 6 * tc_v_part<HDP>() + 128; }
 
 template <int HDP>
-__global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const AttnF32P p) {
+__global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const __grid_constant__ AttnF32P p) {
   extern __shared__ uint8_t tc_raw[];
   __shared__ TcBars bars;
   __shared__ uint32_t tmem_slot;
   __shared__ float2 stat[2][TC_ROWS];
+  __shared__ uint32_t odd[8];   // rows with a result that is not finite, one bit each: [half of the dims][row / 32]
   constexpr int QP = tc_q_part<HDP>(), KP = tc_k_part<HDP>(), VP = tc_v_part<HDP>();
   uint8_t* Qs = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_raw) + 127) & ~static_cast<uintptr_t>(127));
   uint8_t* Ks = Qs + 3 * QP;      // 2 slots x 3 parts
@@ -442,6 +480,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
     }
     // ---- merge: each group stores half of the dims and gets the other group's share of them through the tiles' memory,
     //      which no MMA reads any more ----
+    const int rows = min(TC_ROWS, Lq - q0);
     uint64_t* ox = reinterpret_cast<uint64_t*>(Ks);   // [HDP / 2 pairs][128 rows]
     asm volatile("bar.sync 1, 256;" ::: "memory");
     const float l = dead ? NAN : f2_lo(l2) + f2_hi(l2);
@@ -462,6 +501,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
       const float mt = fmaxf(m, b.x);
       const float fa = m == mt ? 1.f : t_ex2((m - mt) * T_LOG2E), fb = b.x == mt ? 1.f : t_ex2((b.x - mt) * T_LOG2E);
       const float inv = 1.0f / (l * fa + b.y * fb);
+      float zero = 0.f;
 #pragma unroll
       for (int e = 0; e < HDP / 4; e += 2) {
         float a[4];
@@ -472,13 +512,29 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
           a[2 * u + 1] = (f2_hi(x) * fa + f2_hi(y) * fb) * inv;
         }
         *reinterpret_cast<float4*>(of + row * PITCH + (first.value + e) * 2) = make_float4(a[0], a[1], a[2], a[3]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) zero = fmaf(a[u], 0.f, zero);   // (NaN from the first that is not finite on)
       }
+      const uint32_t bits = __ballot_sync(0xffffffffu, !(zero == 0.f) && row < rows && !dead);
+      if (lane == 0) odd[warp] = bits;
     };
     if (g == 0) take(low);
     else take(high);
     asm volatile("bar.sync 1, 256;" ::: "memory");
+    uint32_t any = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) any |= odd[w];
+    if (any) {   // (the same in all 256 threads)
+      for (uint32_t todo = (odd[warp & 3] | odd[4 + (warp & 3)]) & (g == 0 ? 0xffffu : 0xffff0000u); todo; todo &= todo - 1) {
+        const int r = (warp & 3) * 32 + __ffs(todo) - 1;
+        plain_row(p, p.q + (q_first + q0 + r) * p.q_ts + (long)h * p.q_hs, p.k + k_first * p.k_ts + (long)kvh * p.k_hs,
+                  p.v + k_first * p.v_ts + (long)kvh * p.v_hs, S, p.key_mask ? p.key_mask + (long)seg * S : nullptr, of + r * PITCH,
+                  lane);
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+    }
     // stored row by row (a thread's own row in pieces would be 32 sectors per store, most of this kernel's tail)
-    const int nc = p.hd >> 2, rows = min(TC_ROWS, Lq - q0);
+    const int nc = p.hd >> 2;
     for (int i = tid; i < rows * nc; i += 256) {
       const int r = i / nc, d = (i - r * nc) * 4;
       const float4 a = *reinterpret_cast<const float4*>(of + r * PITCH + d);

@@ -80,3 +80,42 @@ def test_masked_keys_and_ragged_segments(lib):
     for a, b in zip(cuts, cuts[1:]):
         if b > a:
             assert rl2(out[a:b].double(), _want(q[a:b], k[a:b], v[a:b], nh, nh, hd)) <= BOUND
+
+
+def _inf_case(kind, q, k, v, hd):
+    if kind == "value":              # stays in its own dimension
+        v[70, 3], v[5, hd + 1] = float("inf"), float("-inf")
+    elif kind == "key":              # every query of head 0 scores -inf: weight 0; head 1 half +inf (NaN), half -inf
+        q[:, 2] = q[:, 2].abs() + 0.1
+        k[66, 2], k[100, hd] = float("-inf"), float("inf")
+    elif kind == "first_tile":       # the whole first tile scores -inf
+        q[:, 2] = q[:, 2].abs() + 0.1
+        k[:64, 2] = float("-inf")
+    elif kind == "query":
+        q[3, 1] = float("inf")
+    elif kind == "large":            # finite in fp32, not in bf16
+        v[7, 0], v[100, hd + 4] = 3.4e38, -3.4e38
+    elif kind == "nan":
+        v[9, 9] = float("nan")
+
+
+@pytest.mark.parametrize("kind", ["value", "key", "first_tile", "query", "large", "nan"])
+@pytest.mark.parametrize("hd,Lq,S", [(64, 130, 200), (72, 40, 129), (96, 128, 131)])
+def test_numbers_that_bf16_parts_do_not_hold(lib, kind, hd, Lq, S):
+    """infinities, NaN and magnitudes above the largest bf16 reach the results that the formula gives them and no others"""
+    from mlx_vlm_b200 import _native as N
+    nh = 2
+    q, k, v = _rand(Lq, nh * hd, seed=11), _rand(S, nh * hd, seed=12), _rand(S, nh * hd, seed=13)
+    _inf_case(kind, q, k, v, hd)
+    out = torch.empty(Lq, nh * hd, device="cuda")
+    N.check(lib.b200_attention_f32(q.data_ptr(), nh * hd, hd, k.data_ptr(), nh * hd, hd, v.data_ptr(), nh * hd, hd, out.data_ptr(),
+                                   nh * hd, 0, 0, 0, nh, nh, hd, Lq, S, 1, Lq, S, 0, hd ** -0.5, 0), "attention_f32")
+    torch.cuda.synchronize()
+    want, got = _want(q, k, v, nh, nh, hd), out.double()
+    assert bool(torch.isfinite(want).any()) and (kind in ("first_tile", "large") or not bool(torch.isfinite(want).all()))
+    odd = ~torch.isfinite(want)
+    assert torch.equal(torch.nan_to_num(got[odd], 1.0, 2.0, 3.0), torch.nan_to_num(want[odd], 1.0, 2.0, 3.0))
+    # column by column: a large value's dimension does not hide the others
+    err = ((got - want).masked_fill(odd, 0.0).norm(dim=0) / want.masked_fill(odd, 0.0).norm(dim=0).clamp_min(1e-300)).max().item()
+    print(kind, hd, err)
+    assert bool(torch.isfinite(got[~odd]).all()) and err <= 2 * BOUND
