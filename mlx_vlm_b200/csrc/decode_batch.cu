@@ -77,8 +77,9 @@ __global__ void __launch_bounds__(256) bd_begin_kernel(const int* __restrict__ t
 
 // ---- attention of one (row, kv head, part of its q heads): finishes q/k/v from the qkv partials -----------------
 // A cluster of up to 8 CTAs shares the row's keys (contiguous ranges in units of 16).  Each CTA brings its keys, then its
-// values, through a ring of 128-row slots (cp.async: everything of a row of up to 384 keys per CTA is in flight while q is
-// still being finished), multiplies them on mma.sync with keys (scores) or dims (P.V) on the M side and up to 8 q heads on
+// values, through a ring of 128-row slots (cp.async: the keys and values of up to 128 keys per CTA, or the keys alone of up to
+// 384, are in flight while q is still being finished), multiplies them on mma.sync with keys (scores) or dims (P.V) on the M
+// side and up to 8 q heads on
 // the N side (operands are bf16 by definition here, accumulators fp32), and meets the others twice in distributed shared
 // memory: for the softmax's maximum and sum (p is rounded after the division, so both are needed first) and for the sum of
 // the partial outputs, in rank order.  Bound by its chain of dependent steps, not by bytes.  Measured against one CTA per part
@@ -394,6 +395,254 @@ __global__ void __launch_bounds__(256) bd_attn_kernel(const BdAttnP p) {
   ba_cluster_sync();   // nobody leaves while its memory is read
 }
 
+// ---- the same for short rows: one CTA per (row, kv head, one or two of its q heads) that reads the row's keys and values
+// through registers.  A cluster's meetings and its slots, which leave the next GEMM no room on the SM for its weights,
+// cost 5 - 10 us a layer whatever the rows hold; until a row has so many keys, this kernel is ahead.  Measured, a layer
+// (attention and GEMMs), this one | clusters: 12 heads on 2 kv heads of 128, 4 rows of 100 keys 39.6 | 46.4 us, 180: 41.5 | 46.8, from
+// 250 on (more keys than its 256 threads): 46.1 | 44.4, 1000: 65.6 | 48.0; 32 on 8 of 128, 4 rows of 180: 66.8 | 73.4; 14 on 2 of 64, 4
+// rows of 250: 34.4 | 39.4, 500: 37.7 | 39.6, 1000: 43.4 | 40.1.  With more than two q heads to a CTA (more rows and heads than
+// SMs) clusters are ahead from the start (32 on 8 of 128, 16 rows of 20: 74.0 | 72.8, of 180: 78.7 | 73.5).
+constexpr int bs_keys(int hd) { return hd == 128 ? 256 : 768; }   // the longest row that it takes
+
+template <int HD, int AG>
+__global__ void __launch_bounds__(256) bd_attn_short_kernel(const BdAttnP p) {
+  bd_pdl_launch();
+  extern __shared__ __align__(128) uint8_t bd_sm[];
+  constexpr int NCH = HD / 8, half = HD / 2, KEYS = bs_keys(HD);
+  constexpr int SEG = HD / 8;   // dims per lane in the P.V phase (lane = key sub-index x dim segment)
+  constexpr int NV = SEG / 8;   // 16-byte vectors per lane and key
+  constexpr int VU = 8;         // key trips in flight per warp in the P.V phase (32 keys)
+  constexpr int PMAX = 12;      // split-K partials summed with all loads in flight
+  float* qs = reinterpret_cast<float*>(bd_sm);  // [AG][HD] q * scale (rotated)
+  float* kn = qs + AG * HD;                     // [HD] new key (rotated)
+  float* vn = kn + HD;                          // [HD] new value
+  float* sc = vn + HD;                          // [AG][KEYS]
+  float* red = sc + AG * KEYS;                  // [8][AG*HD]
+  __shared__ float s_m[8][AG], s_l[8][AG];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row = blockIdx.y;
+  const int Gall = p.n_heads / p.n_kv;
+  const int Gc = (Gall + p.hsplit - 1) / p.hsplit;
+  const int kvh = blockIdx.x / p.hsplit, part = blockIdx.x % p.hsplit;
+  const int G = min(Gc, Gall - part * Gc);
+  const int h0 = kvh * Gall + part * Gc;
+  bf16* kb = p.kv + (long)row * p.row_stride + (long)kvh * p.cap * HD;
+  bf16* vb = kb + p.v_off;
+  bd_pdl_wait();
+  const int ctx = p.ctx[row], pos = p.pos[row];
+  const int nkeys = ctx + 1;
+  // Every dependent global round trip costs ~1 us here, so the requests are issued as early as their
+  // addresses are known: the first block of cached keys (one row per lane) goes out BEFORE the
+  // split-K partials of q/k/v are summed, the first block of values before the softmax.
+  uint4 kfirst[NCH];
+  {
+    const int j = warp * 32 + lane;
+    const uint4* kr = reinterpret_cast<const uint4*>(kb + (long)j * HD);
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) kfirst[c] = (j < ctx) ? __ldcg(kr + c) : make_uint4(0, 0, 0, 0);
+  }
+  // ---- finish q (G heads), k, v of this step: sum of the split-K partials + bias, one rounding ----
+  for (int i = threadIdx.x; i < (G + 2) * HD; i += 256) {
+    const int slot = i / HD, j = i % HD;
+    const int n = (slot < G ? (h0 + slot) : (slot == G ? p.n_heads + kvh : p.n_heads + p.n_kv + kvh)) * HD + j;
+    float a = 0.f;
+    for (int s0 = 0; s0 < p.S; s0 += PMAX) {
+      float v[PMAX];
+#pragma unroll
+      for (int u = 0; u < PMAX; ++u)
+        v[u] = (s0 + u < p.S) ? __ldcg(p.P + ((long)(s0 + u) * p.B + row) * p.QKV + n) : 0.f;
+#pragma unroll
+      for (int u = 0; u < PMAX; ++u) a += v[u];
+    }
+    a = rbf(a + bf2f(p.bias[n]));
+    (slot < G ? qs + slot * HD : (slot == G ? kn : vn))[j] = a;
+  }
+  __syncthreads();
+  // M-RoPE at a decode position: the three axes carry the same position (language.py:476-509)
+  for (int i = threadIdx.x; i < (G + 1) * half; i += 256) {
+    const int slot = i / half, j = i % half;
+    float* v = slot < G ? qs + slot * HD : kn;
+    const float y1 = v[j], y2 = v[j + half];
+    const float ang = (float)pos * p.inv_freq[j];
+    const float c = rbf(cosf(ang)), sn = rbf(sinf(ang));
+    float o1 = rbf(rbf(y1 * c) + rbf((-y2) * sn));
+    float o2 = rbf(rbf(y2 * c) + rbf(y1 * sn));
+    if (slot < G) {
+      o1 = rbf(o1 * p.scale_bf);
+      o2 = rbf(o2 * p.scale_bf);
+    }
+    v[j] = o1;
+    v[j + half] = o2;
+  }
+  for (int i = threadIdx.x + G * HD; i < AG * HD; i += 256) qs[i] = 0.f;
+  __syncthreads();
+  if (part == 0) {  // append the new position to the row's cache (one CTA per kv head)
+    for (int i = threadIdx.x; i < HD; i += 256) {
+      kb[(long)ctx * HD + i] = f2bf(kn[i]);
+      vb[(long)ctx * HD + i] = f2bf(vn[i]);
+    }
+  }
+  // ---- scores: lane <-> key; cached keys from global, the new key from shared memory ----
+  float lm[AG];
+#pragma unroll
+  for (int g = 0; g < AG; ++g) lm[g] = -INFINITY;
+  for (int j0 = warp * 32; j0 < nkeys; j0 += 256) {
+    const int j = j0 + lane;
+    uint4 kv[NCH];
+    if (j0 == warp * 32) {
+#pragma unroll
+      for (int c = 0; c < NCH; ++c) kv[c] = kfirst[c];
+    } else if (j < ctx) {
+      const uint4* kr = reinterpret_cast<const uint4*>(kb + (long)j * HD);
+#pragma unroll
+      for (int c = 0; c < NCH; ++c) kv[c] = __ldcg(kr + c);
+    }
+    if (j < nkeys) {
+      if (j == ctx) {
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) {
+          kv[c].x = pack2(kn[c * 8 + 0], kn[c * 8 + 1]); kv[c].y = pack2(kn[c * 8 + 2], kn[c * 8 + 3]);
+          kv[c].z = pack2(kn[c * 8 + 4], kn[c * 8 + 5]); kv[c].w = pack2(kn[c * 8 + 6], kn[c * 8 + 7]);
+        }
+      }
+      float s[AG][2];
+#pragma unroll
+      for (int g = 0; g < AG; ++g) s[g][0] = s[g][1] = 0.f;
+#pragma unroll
+      for (int c = 0; c < NCH; ++c) {
+        float kf[8];
+        unpack8(kv[c], kf);
+#pragma unroll
+        for (int g = 0; g < AG; ++g) {
+          const float4 a = *reinterpret_cast<const float4*>(qs + g * HD + c * 8);
+          const float4 b = *reinterpret_cast<const float4*>(qs + g * HD + c * 8 + 4);
+          s[g][0] = fmaf(a.x, kf[0], fmaf(a.y, kf[1], fmaf(a.z, kf[2], fmaf(a.w, kf[3], s[g][0]))));
+          s[g][1] = fmaf(b.x, kf[4], fmaf(b.y, kf[5], fmaf(b.z, kf[6], fmaf(b.w, kf[7], s[g][1]))));
+        }
+      }
+#pragma unroll
+      for (int g = 0; g < AG; ++g) {
+        const float r = rbf(s[g][0] + s[g][1]);
+        sc[g * KEYS + j] = r;
+        lm[g] = fmaxf(lm[g], r);
+      }
+    }
+  }
+  // first block of values: warp w, trip q, key = 32 * w + 4 * q + ksub; lane = (ksub, dim segment)
+  const int seg = lane & 7, ksub = lane >> 3;
+  uint4 vfirst[VU][NV];
+#pragma unroll
+  for (int q = 0; q < VU; ++q) {
+    const int j = warp * 32 + q * 4 + ksub;
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+      vfirst[q][v] = (j < ctx) ? __ldcg(reinterpret_cast<const uint4*>(vb + (long)j * HD + seg * SEG + v * 8))
+                               : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int g = 0; g < AG; ++g) {
+    lm[g] = warp_max(lm[g]);
+    if (lane == 0) s_m[warp][g] = lm[g];
+  }
+  __syncthreads();
+  float M[AG], ls[AG];
+#pragma unroll
+  for (int g = 0; g < AG; ++g) {
+    float m = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) m = fmaxf(m, s_m[w][g]);
+    M[g] = m;
+    ls[g] = 0.f;
+  }
+  for (int j = threadIdx.x; j < nkeys; j += 256) {
+#pragma unroll
+    for (int g = 0; g < AG; ++g) {
+      const float e = expf(sc[g * KEYS + j] - M[g]);
+      sc[g * KEYS + j] = e;
+      ls[g] += e;
+    }
+  }
+#pragma unroll
+  for (int g = 0; g < AG; ++g) {
+    ls[g] = warp_sum(ls[g]);
+    if (lane == 0) s_l[warp][g] = ls[g];
+  }
+  __syncthreads();
+  float L[AG];
+#pragma unroll
+  for (int g = 0; g < AG; ++g) {
+    float l = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) l += s_l[w][g];
+    L[g] = l;
+  }
+  for (int j = threadIdx.x; j < nkeys; j += 256) {
+#pragma unroll
+    for (int g = 0; g < AG; ++g) sc[g * KEYS + j] = rbf(sc[g * KEYS + j] / L[g]);
+  }
+  __syncthreads();
+  // ---- P.V: 256 keys per CTA iteration, 8 x NV 16-byte loads in flight per lane ----
+  float acc[AG][SEG];
+#pragma unroll
+  for (int g = 0; g < AG; ++g)
+#pragma unroll
+    for (int e = 0; e < SEG; ++e) acc[g][e] = 0.f;
+  for (int j0 = 0; j0 < nkeys; j0 += 256) {
+    uint4 vv[VU][NV];
+#pragma unroll
+    for (int q = 0; q < VU; ++q) {
+      const int j = j0 + warp * 32 + q * 4 + ksub;
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        if (j0 == 0) vv[q][v] = vfirst[q][v];
+        else vv[q][v] = (j < ctx) ? __ldcg(reinterpret_cast<const uint4*>(vb + (long)j * HD + seg * SEG + v * 8))
+                                  : make_uint4(0, 0, 0, 0);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < VU; ++q) {
+      const int j = j0 + warp * 32 + q * 4 + ksub;
+      if (j < nkeys) {
+        float pj[AG];
+#pragma unroll
+        for (int g = 0; g < AG; ++g) pj[g] = sc[g * KEYS + j];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          float vf[8];
+          if (j == ctx) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) vf[e] = rbf(vn[seg * SEG + v * 8 + e]);
+          } else {
+            unpack8(vv[q][v], vf);
+          }
+#pragma unroll
+          for (int g = 0; g < AG; ++g)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[g][v * 8 + e] = fmaf(pj[g], vf[e], acc[g][v * 8 + e]);
+        }
+      }
+    }
+  }
+  // sum over the 4 key sub-indices of the warp, then over the 8 warps through shared memory
+#pragma unroll
+  for (int g = 0; g < AG; ++g)
+#pragma unroll
+    for (int e = 0; e < SEG; ++e) {
+      float a = acc[g][e];
+      a += __shfl_xor_sync(0xffffffffu, a, 8);
+      a += __shfl_xor_sync(0xffffffffu, a, 16);
+      if (ksub == 0) red[((long)warp * AG + g) * HD + seg * SEG + e] = a;
+    }
+  __syncthreads();
+  bf16* orow = p.out + (long)row * p.n_heads * HD + (long)h0 * HD;
+  for (int i = threadIdx.x; i < G * HD; i += 256) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) s += red[(long)w * AG * HD + i];
+    orow[i] = f2bf(s);
+  }
+}
+
 // ---- sampler + state update + next embedding, one CTA per row ------------------------------------
 __device__ __forceinline__ uint32_t bd_orderable(float f) {
   const uint32_t u = __float_as_uint(f);
@@ -521,16 +770,25 @@ struct BatchDecoder {
   float* partial = nullptr;
   long partial_bytes = 0;
   int* stage_host = nullptr;  // pinned [4][max_b]
-  cudaGraphExec_t gexec = nullptr;
+  cudaGraphExec_t gexec[5] = {};   // short rows; clusters of 1, 2, 4, 8
   const void* graph_kv = nullptr;
   int graph_B = 0, graph_cap = 0, graph_lp = 0;
   long steps_done = 0;
+  int longest = 0;   // cached tokens of the longest row at begin()
+  int fit[4] = {}, fit_cap = -1;   // clusters of 1, 2, 4, 8 CTAs that the chip holds at once, for rows of fit_cap keys
   bool want_logprobs = false;
 };
 
+static void bd_drop_graphs(BatchDecoder* d) {
+  for (cudaGraphExec_t& g : d->gexec) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
+}
+
 static void bd_free(BatchDecoder* d) {
   if (!d) return;
-  if (d->gexec) cudaGraphExecDestroy(d->gexec);
+  bd_drop_graphs(d);
   for (void* p : {(void*)d->tok, (void*)d->ctx, (void*)d->pos, (void*)d->active, (void*)d->n_out, (void*)d->token_log,
                   (void*)d->lp_log, (void*)d->h, (void*)d->xn, (void*)d->att, (void*)d->act, (void*)d->logits,
                   (void*)d->logprobs, (void*)d->partial})
@@ -589,45 +847,88 @@ static size_t bd_attn_smem(const DecodeDims& d, int ranks) {
   return (size_t)BA_SLOTS * BA_ROWS * d.hd * 2 + (size_t)slots * BA_ROWS * BA_HEADS * 2;
 }
 
-// CTAs of a row's cluster: as many as one wave holds at one per SM (two leave no room for the next GEMM, whose weights are on
-// their way while this kernel runs: 8 rows of 272 - 784 keys, 4 kv heads: 20 us a layer instead of 27, and the step no
-// shorter), and no fewer than the scores of the longest row need shared memory for
-static int bd_attn_ranks(const DecodeDims& d, int B, int sm_count) {
+struct BdAttnLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[2];
+  BdAttnLaunch(int ranks, int groups, int B, size_t smem, cudaStream_t s) {
+    cfg.gridDim = dim3(ranks, groups, B);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = ranks;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+  }
+  BdAttnLaunch(const BdAttnLaunch&) = delete;   // cfg points into the object
+};
+
+// The attention of a step: -1: the kernel for short rows, its CTAs (one or two q heads each) in one wave; else the CTAs of a
+// row's cluster (1, 2, 4, 8).
+//  * as many as one wave holds at one per SM (two leave no room for the next GEMM, whose weights are on their way while this
+//    kernel runs: 8 rows of 272 - 784 keys, 4 kv heads: 20 us a layer instead of 27, and the step no shorter), the clusters
+//    counted as the chip's groups of SMs hold them: 16 clusters of 8 that take an SM per CTA (from about 1500 keys of capacity on)
+//    ran in two waves, 8 rows of 2000 keys, 2 kv heads: 66.0 us a layer instead of 53.0 in clusters of 4
+//  * 8 from 1024 keys on (a layer, 4 | 8: 8 rows on 2 kv heads of 250 keys 46.8 | 47.1, 500: 47.6 | 47.5, 1000: 48.5 | 48.6; 2 rows
+//    on 4 of 500: 65.4 | 66.6, 1000: 66.9 | 67.8)
+//  * and no fewer than the scores of the longest row need shared memory for
+static int bd_short_heads(const DecodeDims& d, int B, int sm_count) {   // q heads per CTA; 0: more than a wave
+  const int G = d.n_heads / d.n_kv;
+  for (int ag : {1, 2})
+    if ((long)d.n_kv * cdiv(G, ag) * B <= sm_count) return ag;
+  return 0;
+}
+
+static int bd_attn_variant(BatchDecoder* bd, const DecodeDims& d, int B, int keys, int sm_count, int* ranks) {
+  if (keys <= bs_keys(d.hd) && bd_short_heads(d, B, sm_count)) {
+    *ranks = -1;
+    return B200_OK;
+  }
   const long groups = (long)d.n_kv * cdiv(d.n_heads / d.n_kv, BA_HEADS) * B;
-  int ranks = 1;
-  for (int r : {2, 4, 8})
-    if (groups * r <= sm_count) ranks = r;
-  while (ranks < 8 && bd_attn_smem(d, ranks) > 200 * 1024) ranks *= 2;
-  return ranks;
+  if (bd->fit_cap != d.cap) {
+    for (int i = 0; i < 4; ++i) {
+      bd->fit[i] = 0;
+      if (bd_attn_smem(d, 1 << i) > 200 * 1024) continue;
+      const BdAttnLaunch l(1 << i, 1, 1, bd_attn_smem(d, 1 << i), nullptr);
+      B200_CUDA(d.hd == 128 ? cudaOccupancyMaxActiveClusters(&bd->fit[i], bd_attn_kernel<128>, &l.cfg)
+                            : cudaOccupancyMaxActiveClusters(&bd->fit[i], bd_attn_kernel<64>, &l.cfg));
+    }
+    bd->fit_cap = d.cap;
+  }
+  int i = 0;
+  for (int j = 1; j < 4; ++j)
+    if ((groups << j) <= sm_count && groups <= bd->fit[j] && (j < 3 || keys >= 1024)) i = j;
+  while (i < 3 && bd_attn_smem(d, 1 << i) > 200 * 1024) ++i;
+  *ranks = 1 << i;
+  return B200_OK;
 }
 
 template <int HD>
 static int bd_attn_launch(int ranks, int groups, int B, size_t smem, cudaStream_t s, const BdAttnP& ap) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ranks, groups, B);
-  cfg.blockDim = dim3(256);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = ranks;
-  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 2;
-  B200_CUDA(cudaLaunchKernelEx(&cfg, bd_attn_kernel<HD>, ap));
+  const BdAttnLaunch l(ranks, groups, B, smem, s);
+  B200_CUDA(cudaLaunchKernelEx(&l.cfg, bd_attn_kernel<HD>, ap));
   return B200_OK;
+}
+template <int HD>
+static int bd_attn_short(int ag, int B, cudaStream_t s, const BdAttnP& ap) {
+  const dim3 grid(ap.n_kv * ap.hsplit, B);
+  const size_t smem = ((size_t)(ag + 2) * HD + (size_t)ag * bs_keys(HD) + (size_t)8 * ag * HD) * 4;
+  return ag == 1 ? bd_launch(bd_attn_short_kernel<HD, 1>, grid, dim3(256), smem, s, ap)
+                 : bd_launch(bd_attn_short_kernel<HD, 2>, grid, dim3(256), smem, s, ap);
 }
 
 // one lock-step step as plain launches on `s` (also what gets captured)
-static int bd_enqueue_step(BatchDecoder* d, const BdModel& m, cudaStream_t s, long* launches) {
+static int bd_enqueue_step(BatchDecoder* d, const BdModel& m, int ranks, cudaStream_t s, long* launches) {
   const DecodeDims& dd = m.d;
   const int B = d->B, H = dd.hidden, I = dd.inter;
   const int QH = dd.n_heads * dd.hd, QKV = (dd.n_heads + 2 * dd.n_kv) * dd.hd;
   int rc;
-  const int hs = cdiv(dd.n_heads / dd.n_kv, BA_HEADS), ranks = bd_attn_ranks(dd, B, m.sm_count);
-  const size_t att_smem = bd_attn_smem(dd, ranks);
+  const bool rows_short = ranks < 0;
+  const int ag = rows_short ? bd_short_heads(dd, B, m.sm_count) : BA_HEADS, hs = cdiv(dd.n_heads / dd.n_kv, ag);
+  const size_t att_smem = rows_short ? 0 : bd_attn_smem(dd, ranks);
   B200_REQUIRE(att_smem <= 200 * 1024, "batch decode: cache capacity %d too large for the attention kernel", dd.cap);
   for (int l = 0; l < m.n_layers; ++l) {
     const LayerW& lw = m.layers[l];
@@ -640,8 +941,9 @@ static int bd_enqueue_step(BatchDecoder* d, const BdModel& m, cudaStream_t s, lo
     ap.ctx = d->ctx; ap.pos = d->pos; ap.kv = m.kv + (long)l * m.layer_stride; ap.v_off = m.v_off;
     ap.row_stride = m.row_stride; ap.out = d->att; ap.n_heads = dd.n_heads; ap.n_kv = dd.n_kv; ap.cap = dd.cap;
     ap.hsplit = hs; ap.scale_bf = dd.scale_bf;
-    rc = dd.hd == 128 ? bd_attn_launch<128>(ranks, dd.n_kv * hs, B, att_smem, s, ap)
-                      : bd_attn_launch<64>(ranks, dd.n_kv * hs, B, att_smem, s, ap);
+    if (rows_short) rc = dd.hd == 128 ? bd_attn_short<128>(ag, B, s, ap) : bd_attn_short<64>(ag, B, s, ap);
+    else rc = dd.hd == 128 ? bd_attn_launch<128>(ranks, dd.n_kv * hs, B, att_smem, s, ap)
+                           : bd_attn_launch<64>(ranks, dd.n_kv * hs, B, att_smem, s, ap);
     if (rc) return rc;
     if ((rc = gemm_wt_tuned(d->att, QH, lw.wo, nullptr, nullptr, 0, nullptr, 0, d->partial, d->partial_bytes, B, H, QH,
                             B200_EPI_NONE, B200_WT_PARTIAL, 0, true, m.sm_count, &split, s)))
@@ -696,7 +998,9 @@ int batch_decoder_begin(void** handle, const BdModel& m, int B, const int* tok, 
     }
   }
   d->B = B;
+  d->longest = 0;
   for (int b = 0; b < B; ++b) {
+    d->longest = ctx[b] > d->longest ? ctx[b] : d->longest;
     B200_REQUIRE(ctx[b] >= 0 && ctx[b] < m.d.cap, "batch decode: row %d holds %d tokens, capacity %d", b, ctx[b], m.d.cap);
     d->stage_host[b] = tok[b];
     d->stage_host[d->max_b + b] = ctx[b];
@@ -723,34 +1027,32 @@ int batch_decoder_step(void* handle, const BdModel& m, int n_steps, bool want_lo
   d->want_logprobs = want_logprobs;
   int rc;
   int done = 0;
-  const bool stale = !d->gexec || d->graph_kv != m.kv || d->graph_B != d->B || d->graph_cap != m.d.cap ||
-                     d->graph_lp != (int)want_logprobs;
-  if (stale) {
-    if (d->gexec) {
-      cudaGraphExecDestroy(d->gexec);
-      d->gexec = nullptr;
-    }
+  int ranks = 1;
+  if ((rc = bd_attn_variant(d, m.d, d->B, (int)(d->longest + d->steps_done + n_steps), m.sm_count, &ranks))) return rc;
+  cudaGraphExec_t& gexec = d->gexec[ranks < 0 ? 0 : ranks == 8 ? 4 : ranks == 4 ? 3 : ranks];
+  if (d->graph_kv != m.kv || d->graph_B != d->B || d->graph_cap != m.d.cap || d->graph_lp != (int)want_logprobs) bd_drop_graphs(d);
+  if (!gexec) {
     // first step eagerly: the GEMM configurations are measured on first use (not under capture)
-    if ((rc = bd_enqueue_step(d, m, s, launches))) return rc;
+    if ((rc = bd_enqueue_step(d, m, ranks, s, launches))) return rc;
     done = 1;
     if (n_steps > 1) {
       cudaGraph_t graph = nullptr;
       long dummy = 0;
       B200_CUDA(cudaStreamBeginCapture(cap_stream, cudaStreamCaptureModeThreadLocal));
-      rc = bd_enqueue_step(d, m, cap_stream, &dummy);
+      rc = bd_enqueue_step(d, m, ranks, cap_stream, &dummy);
       cudaError_t ce = cudaStreamEndCapture(cap_stream, &graph);
       if (rc) {
         if (graph) cudaGraphDestroy(graph);
         return rc;
       }
       if (ce != cudaSuccess) return cuda_fail(ce, "cudaStreamEndCapture(batch step)", __FILE__, __LINE__);
-      ce = cudaGraphInstantiate(&d->gexec, graph, 0);
+      ce = cudaGraphInstantiate(&gexec, graph, 0);
       cudaGraphDestroy(graph);
       if (ce != cudaSuccess) return cuda_fail(ce, "cudaGraphInstantiate(batch step)", __FILE__, __LINE__);
       d->graph_kv = m.kv; d->graph_B = d->B; d->graph_cap = m.d.cap; d->graph_lp = (int)want_logprobs;
     }
   }
-  for (int i = done; i < n_steps; ++i) B200_CUDA(cudaGraphLaunch(d->gexec, s));
+  for (int i = done; i < n_steps; ++i) B200_CUDA(cudaGraphLaunch(gexec, s));
   *launches += (long)(n_steps - done) * (m.n_layers * 7 + 2);
   d->steps_done += n_steps;
   return B200_OK;

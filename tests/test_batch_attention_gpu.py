@@ -65,8 +65,9 @@ def test_rows_of_any_length(hd, nh, nkv, lens):
         pool[:, :, b, :, n:] = float("nan")        # rows that are not cached yet are never part of a result
     before = pool.clone()
     ids = np.random.default_rng(3).integers(0, 512, size=(len(lens), 1))
-    got = lm(ids, cache=caches).logits[:, 0].double()
-    model.engine.stream.synchronize()
+    got = lm(ids, cache=caches).logits
+    model.engine.stream.synchronize()       # (the logits are the engine stream's: nothing else waits for it)
+    got = got[:, 0].double()
     want = _want(model, ids, before, lens)
     # two layers of bf16 roundings (2^-9 each at about ten places a layer): measured 0.008 - 0.02
     err = ((got - want).norm(dim=1) / want.norm(dim=1)).max().item()
@@ -76,3 +77,76 @@ def test_rows_of_any_length(hd, nh, nkv, lens):
         assert torch.equal(pool[:, :, b, :, :n], before[:, :, b, :, :n])
         assert not bool(torch.isnan(pool[:, :, b, :, n].float()).any())
         assert bool(torch.isnan(pool[:, :, b, :, n + 1:].float()).all())
+
+
+def _boundaries(n):
+    """keys of a row of n cached ones at the edges of every split: first and last key of each CTA of 1, 2, 4 and 8, the ends of
+    their 128-key slots, the last key"""
+    at = {0, n - 1}
+    for ranks in (1, 2, 4, 8):
+        share = -(-(n + 1) // (16 * ranks)) * 16
+        for r in range(ranks):
+            at |= {j for j in (r * share, r * share + 127, r * share + 128, (r + 1) * share - 1)}
+    return sorted(j for j in at if 0 <= j < n)
+
+
+# rows for the kernel of short rows (up to 256 keys of 128 dims, 768 of 64) and for clusters; one more key than it takes
+@pytest.mark.parametrize("hd,nh,nkv", [(128, 14, 2), (64, 4, 4), (64, 18, 2), (128, 40, 8)])
+@pytest.mark.parametrize("lens", [(2, 17, 255), (256, 5), (127, 767), (768, 33, 130), (1023, 1024, 1025), (40,) * 16])
+@pytest.mark.parametrize("what", ["cached", "new"])
+def test_every_key_counts(hd, nh, nkv, lens, what):
+    """cached: nearly equal weights and values of n times the size at the edges of the splits, so that one of these keys left out
+    or counted twice moves the result by more than a tenth; new: the step's own key takes nearly all of the weight"""
+    model = _model(hd * nh, nh, nkv)
+    model.engine.stream.synchronize()
+    lm = model.language_model
+    rows, caches = lm.make_batch_cache(len(lens), max(lens) + 8)
+    rows.lengths = list(lens)
+    g = torch.Generator(device="cuda").manual_seed(len(lens) + hd)
+    pool = rows.pool.buf
+    pool.copy_(torch.randn(pool.shape, generator=g, device="cuda"))
+    pool[:, 0] *= 0.02 if what == "cached" else 0.0
+    H = hd * nh
+    for i in range(2):
+        b = model.engine.weights[f"lm.{i}.bqkv"]
+        b.copy_(torch.randn(b.shape, generator=g, device="cuda"))
+        b[:H + nkv * hd] = 0.0 if what == "cached" else 1.0     # (q . k = hd at the same position: weight e^(sqrt hd))
+    for b, n in enumerate(lens):
+        if what == "cached":
+            pool[:, 1, b, :, _boundaries(n)] *= n
+        pool[:, :, b, :, n:] = float("nan")
+    before = pool.clone()
+    torch.cuda.synchronize()
+    ids = np.random.default_rng(5).integers(0, 512, size=(len(lens), 1))
+    got = lm(ids, cache=caches).logits
+    model.engine.stream.synchronize()       # (the logits are the engine stream's: nothing else waits for it)
+    got = got[:, 0].double()
+    want = _want(model, ids, before, lens)
+    err = ((got - want).norm(dim=1) / want.norm(dim=1)).max().item()
+    print(f"{what} {lens} hd={hd}: {err:.4f}")
+    assert err <= 0.05        # the roundings of test_rows_of_any_length
+
+
+def test_rows_grow_from_one_kernel_to_the_other():
+    """a generation whose rows pass the longest that the kernel of short rows takes, in chunks: the graphs of both kernels give the
+    tokens of single steps"""
+    model = _model(128 * 4, 4, 2)
+    eng, lm = model.engine, model.language_model
+    ids = np.random.default_rng(6).integers(0, 512, size=(2, 1))
+
+    def run(chunks):
+        rows, caches = lm.make_batch_cache(2, 512)
+        rows.lengths = [210, 230]
+        rows.pool.buf.copy_(torch.randn(rows.pool.buf.shape, generator=torch.Generator(device="cuda").manual_seed(7), device="cuda"))
+        torch.cuda.synchronize()
+        lm(ids, cache=caches)
+        for n in chunks:
+            eng.batch_decode(n)
+        eng.stream.synchronize()
+        return eng.batch_token_log_view()[:1 + sum(chunks), :2].clone(), rows.pool.buf.clone()
+    ones, pool1 = run([1] * 48)
+    many, pool2 = run([12, 4, 8, 8, 16])
+    again, _ = run([48])
+    assert torch.equal(ones, many)
+    assert torch.equal(pool1[:, :, :, :, 210:220], pool2[:, :, :, :, 210:220])
+    assert torch.equal(ones[:1], again[:1])
