@@ -38,6 +38,9 @@ const char* b200_last_error(void);
 int b200_abi_version(void);
 /* Fails with B200_ERR_UNSUPPORTED unless `device` is compute capability 10.x. */
 int b200_device_check(int device, int* sm_count);
+/* Synchronous: which kernel gave up on a wait inside it (it then stores NaN) on the current device, 0 = none.  Stays set. */
+#define B200_WAIT_PAIR 5       /* gemm_wt_pair_kernel */
+int b200_wait_error(int* out);
 
 /* ------------------------------------------------------------------------- */
 /* Op level (each is one kernel launch; used directly by the kernel tests)    */
@@ -79,7 +82,8 @@ int b200_gemm_bf16_tn(const void* A, long lda, const void* W, const void* bias,
  * B200_WT_PARTIAL: fp32 tiles partial[split][T][N] (bias / residual applied by
  * b200_finish_rows); B200_WT_SWIGLU: W = [gate; up] (N == 2*inter), C[T][inter] =
  * swiglu (mlp.py:9-15, activations.py:8-10).  cfg4 = {TN, k-blocks per stage, stages,
- * splits} or NULL / {0} for the automatic choice.  flags: debugging aids, pass 0. */
+ * splits} or NULL / {0} for the automatic choice.  flags: debugging aids, pass 0 (2: nothing is loaded; with CTA pairs the
+ * waits for it then run out: NaN, b200_wait_error). */
 int b200_gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void* residual,
                  long ldr, void* C, long ldc, float* partial, int T, int N, int K, int epilogue,
                  int mode, int inter, const int* cfg4, unsigned flags, void* stream);
@@ -249,7 +253,7 @@ int b200_engine_set_mega(b200_engine* e, int enabled);
 /* debugging / test aid: device pointer and size of an internal buffer.  names: "h", "act",
  * "tc_acc" (k_mega_tc fixed-point split-K accumulators, 3 x rows int64). */
 int b200_engine_debug_buffer(b200_engine* e, const char* name, void** ptr, long* bytes);
-/* synchronous: reads the device-side error flag (0 = none; a bounded wait gave up) */
+/* synchronous: the engine's device-side error flag, else b200_wait_error's (0 = none; a bounded wait gave up) */
 int b200_engine_device_error(b200_engine* e, int* out);
 /* debugging aid (k_mega): first call enables per-barrier globaltimer stamps, later
  * calls copy them out: out_host[2][1024][2] int64 = (arrive, release) per grid barrier

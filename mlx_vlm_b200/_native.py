@@ -38,6 +38,7 @@ SIGNATURES = {
     "b200_last_error": (C.c_char_p, []),
     "b200_abi_version": (_I, []),
     "b200_device_check": (_I, [_I, C.POINTER(_I)]),
+    "b200_wait_error": (_I, [C.POINTER(_I)]),
     "b200_cast_f32_bf16": (_I, [_P, _P, _L, _P]),
     "b200_gemm_bf16_tn": (_I, [_P, _L, _P, _P, _P, _L, _P, _L, _I, _I, _I, _I, _P]),
     "b200_gemm_wt": (_I, [_P, _L, _P, _P, _P, _L, _P, _L, _P, _I, _I, _I, _I, _I, _I, _P, C.c_uint, _P]),
@@ -111,6 +112,7 @@ LM_SIGNATURES = {
     "b200_last_error": (C.c_char_p, []),
     "b200_abi_version": (_I, []),
     "b200_device_check": (_I, [_I, C.POINTER(_I)]),
+    "b200_wait_error": (_I, [C.POINTER(_I)]),
     "b200_lm_embed": (_I, [_P, _P, _F, _P, _I, _I, _I, _P]),
     "b200_lm_embed_bigram": (_I, [_P, _P, _F, _P, _I, _L, _L, _P, _L, _P, _P, _P, _P, _I, _I, _P, _P, _P, _F, _P, _P, _L, _I, _I,
                                   _I, _P]),

@@ -126,6 +126,13 @@ __device__ __forceinline__ float gelu_exact_bf(float x) {
 
 inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 
+// A unit's device word that its kernels raise when a wait ran out (0: never did); wait_error: the first one raised on the
+// current device.  A word stays raised: the results of that launch were NaN, and something that should not happen did.
+struct WaitWord {
+  explicit WaitWord(int (*read)(int*));
+};
+int wait_error(int* out);
+
 // per-DEVICE one-time setup (cudaFuncSetAttribute is per device): true the first time the current device asks
 inline bool first_use_on_device(unsigned long long* mask) {
   int dev = 0;
@@ -134,6 +141,36 @@ inline bool first_use_on_device(unsigned long long* mask) {
   if (*mask & bit) return false;
   *mask |= bit;
   return true;
+}
+
+// ---- waits that end ----------------------------------------------------------------
+// Waits for a phase of an mbarrier of this CTA; false, and *failed (shared memory, zeroed before the first wait) set, after
+// WAIT_TRIES tries.  Whoever gets a false multiplies, signals and requests nothing more, and waits for no later phase (a
+// barrier of which a phase was passed over answers for another one); so the waits of others for it run out too, its own copies
+// and products end (mbar_drain), and NaN is stored.  The kernel raises its unit's word (WaitWord), which b200_wait_error reads.
+constexpr int WAIT_TRIES = 1 << 18;   // 4 us each: a second
+__device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(addr), "r"(parity)
+      : "memory");
+  return done;
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* failed) {
+  const uint32_t addr = static_cast<uint32_t>(__cvta_generic_to_shared(bar));
+#pragma unroll 1
+  for (int i = 0; i < WAIT_TRIES; ++i)
+    if (mbar_try(addr, parity)) return true;
+  *static_cast<volatile int*>(failed) = 1;
+  return false;
+}
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {   // the same after a failure
+  int mine = 0;
+  mbar_wait(bar, parity, &mine);
 }
 
 // ---- programmatic dependent launch -------------------------------------------------

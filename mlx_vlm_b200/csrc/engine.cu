@@ -1269,7 +1269,7 @@ int b200_engine_device_error(b200_engine* e, int* out) {
   DecState st;
   B200_CUDA(cudaMemcpy(&st, e->st, sizeof(st), cudaMemcpyDeviceToHost));
   *out = st.error;
-  return B200_OK;
+  return st.error ? B200_OK : wait_error(out);
 }
 /* debugging aid: per-barrier globaltimer stamps of CTA 0 and the last CTA for the most
  * recent step; out_host must hold 2*1024*2 int64.  Enables stamping on first call. */

@@ -18,6 +18,18 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
   return B200_ERR_CUDA;
 }
 
+static int (*g_wait_words[8])(int*) = {};
+static int g_n_wait_words = 0;
+WaitWord::WaitWord(int (*read)(int*)) {
+  if (g_n_wait_words < 8) g_wait_words[g_n_wait_words++] = read;
+}
+int wait_error(int* out) {
+  *out = 0;
+  for (int i = 0; i < g_n_wait_words && *out == 0; ++i)
+    if (int rc = g_wait_words[i](out)) return rc;
+  return B200_OK;
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -26,6 +38,14 @@ extern "C" {
 
 const char* b200_last_error(void) { return g_err; }
 int b200_abi_version(void) { return B200_ABI_VERSION; }
+
+int b200_wait_error(int* out) {
+  if (!out) {
+    set_error("wait_error: null argument");
+    return B200_ERR_INVALID;
+  }
+  return wait_error(out);
+}
 
 int b200_device_check(int device, int* sm_count) {
   cudaDeviceProp prop;

@@ -508,25 +508,11 @@ constexpr int WP_THREADS = 384;
 constexpr int WP_MAX_STAGES = 12;
 
 struct WpBars {
-  uint64_t full[WP_MAX_STAGES], empty[WP_MAX_STAGES], acc_full[2], acc_empty[2];
+  uint64_t full[WP_MAX_STAGES], empty[WP_MAX_STAGES], acc_full[2], acc_empty[2], drained;
 };
 
-// Bounded: a wait that does not end (about a second) gives up, and so does every later one of the thread; the tiles that it
-// would have stored become NaN.
-__device__ __forceinline__ void wp_wait(uint64_t* bar, uint32_t parity, bool& dead) {
-  uint32_t done = 0;
-  const uint32_t addr = w_smem_u32(bar);
-  for (int i = 0; !done && !dead; ++i) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (i > (1 << 24)) dead = true;
-  }
-}
+__device__ int g_pair_wait_failed;   // a wait of gemm_wt_pair_kernel ran out: B200_WAIT_PAIR
+
 __device__ __forceinline__ uint32_t wp_leader(const void* p) {   // shared::cluster address of *p in the pair's rank 0
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(w_smem_u32(p)));
@@ -564,6 +550,7 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   extern __shared__ uint8_t wt_smem_raw[];
   __shared__ WpBars bars;
   __shared__ uint32_t tmem_slot;
+  __shared__ int failed;
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(wt_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
@@ -574,7 +561,7 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   const int row_tiles = ((swiglu ? 2 * p.inter : p.N) + 2 * WT_ROWS - 1) / (2 * WT_ROWS), tok_tiles = (p.T + p.TN - 1) / p.TN;
   const int splits = (kb_total + p.kb_per_split - 1) / p.kb_per_split;
   const int n_tiles = row_tiles * tok_tiles * splits;
-  bool dead = false;
+  int loads = 0;   // of this CTA's producer
   // tile -> this CTA's first output feature, its first token, its k-blocks
   auto tile_at = [&](int tile, int& n0, int& t0, int& split, int& kb0, int& kb1) {
     t0 = tile % tok_tiles * p.TN;
@@ -597,6 +584,8 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       w_mbar_init(&bars.acc_full[b], 1);
       w_mbar_init(&bars.acc_empty[b], 16);   // eight epilogue warps of each CTA
     }
+    w_mbar_init(&bars.drained, 1);
+    failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -615,6 +604,8 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     if (lane == 0) {  // ===== TMA producer =====
       const uint32_t full0 = wp_leader(&bars.full[0]);
       auto load_w = [&](int s, int kb, int n0) {
+        if (p.flags & 2u) return;   // (no loads: every wait for them runs out)
+        ++loads;
         if (p.kb_w > 0) kb %= p.kb_w;
         uint8_t* sW = ring + (long)s * stage_bytes;
         const uint32_t bar = full0 + s * 8;
@@ -627,6 +618,7 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
         }
       };
       auto load_x = [&](int s, int kb, int t0) {
+        if (p.flags & 2u) return;
         wp_tma_2d(ring + (long)s * stage_bytes + WT_WBLK, &tmX, full0 + s * 8, kb * WT_BK, t0 + rank * xhalf);
       };
       int n0, t0, split, kb0, kb1;
@@ -640,14 +632,15 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       w_pdl_wait();
       int s = 0;
       uint32_t free_parity = 1;
-      for (int tile = pair; tile < n_tiles && !dead; tile += n_pairs) {
+      bool ok = true;
+      for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
         tile_at(tile, n0, t0, split, kb0, kb1);
         for (int kb = kb0; kb < kb1; ++kb) {
           if (pre > 0) {
             --pre;
           } else {
-            wp_wait(&bars.empty[s], free_parity, dead);
-            if (dead) break;   // nothing more is requested
+            ok = mbar_wait(&bars.empty[s], free_parity, &failed);
+            if (!ok) break;
             load_w(s, kb, n0);
           }
           load_x(s, kb, t0);
@@ -664,15 +657,16 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       const uint32_t step = (uint32_t)stage_bytes >> 4;
       int s = 0, j = 0, n0, t0, split, kb0, kb1;
       uint32_t w_lo = w_first, x_lo = x_first, parity = 0;
-      for (int tile = pair; tile < n_tiles && !dead; tile += n_pairs, ++j) {
+      bool ok = true;
+      w_pdl_wait();   // (the time of a wait starts when the tokens can be on their way)
+      for (int tile = pair; tile < n_tiles; tile += n_pairs, ++j) {
         tile_at(tile, n0, t0, split, kb0, kb1);
         const uint32_t d = tmem + (uint32_t)(j & 1) * 256u;
-        wp_wait(&bars.acc_empty[j & 1], ((j >> 1) & 1) ^ 1, dead);
+        if (!(ok = mbar_wait(&bars.acc_empty[j & 1], ((j >> 1) & 1) ^ 1, &failed))) break;
         w_fence_after();
         uint32_t acc = 0;
         for (int kb = kb0; kb < kb1; ++kb) {
-          wp_wait(&bars.full[s], parity, dead);
-          if (dead) break;
+          if (!(ok = mbar_wait(&bars.full[s], parity, &failed))) break;
           w_fence_after();
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
@@ -684,18 +678,19 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
           x_lo += step;
           if (++s == NS) s = 0, w_lo = w_first, x_lo = x_first, parity ^= 1;
         }
+        if (!ok) break;   // (an accumulator that is not whole is not handed over)
         wp_commit(&bars.acc_full[j & 1]);
       }
     }
   } else if (warp >= 4) {  // ===== epilogue =====
     w_pdl_wait();
     int j = 0, n0, t0, split, kb0, kb1;
+    bool ok = true;   // (the same in a warp)
     for (int tile = pair; tile < n_tiles; tile += n_pairs, ++j) {
       tile_at(tile, n0, t0, split, kb0, kb1);
-      wp_wait(&bars.acc_full[j & 1], (j >> 1) & 1, dead);
-      __syncwarp();
+      ok = ok && __all_sync(0xffffffffu, mbar_wait(&bars.acc_full[j & 1], (j >> 1) & 1, &failed));
       w_fence_after();
-      wt_store_tile<TOWER>(p, stg, tmem + (uint32_t)(j & 1) * 256u, n0, t0, 0, split, threadIdx.x - 128, dead);
+      wt_store_tile<TOWER>(p, stg, tmem + (uint32_t)(j & 1) * 256u, n0, t0, 0, split, threadIdx.x - 128, !ok);
       w_fence_before();
       __syncwarp();
       if (lane == 0)
@@ -706,7 +701,28 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   __syncwarp();
   w_fence_before();
   __syncthreads();
+  if (failed && threadIdx.x == 0)
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.b32 [a], %2;\n\t}" ::"r"(w_smem_u32(&failed)),
+                   "r"(r), "r"(1)
+                   : "memory");
   wp_cluster_sync();   // nobody's shared memory or TMEM goes while the peer still uses it
+  // (in both CTAs) nothing is left in flight: the last load of every slot that the leader counts, the products; loads that only
+  // the other CTA requested have had the time of a wait that ran out
+  if (*static_cast<volatile int*>(&failed)) {
+    if (rank == 0 && lane == 0) {
+      if (warp == 0) {
+        g_pair_wait_failed = B200_WAIT_PAIR;
+        for (int i = max(0, loads - NS); i < loads; ++i) mbar_drain(&bars.full[i % NS], (i / NS) & 1);
+      } else if (warp == 1) {
+        wp_commit(&bars.drained);
+        mbar_drain(&bars.drained, 0);
+      }
+    }
+    __syncwarp();
+    wp_cluster_sync();
+  }
   if (warp == 2) {
     w_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
@@ -919,6 +935,11 @@ int wt_tmap(const void* ptr, long ld, int rows, int k, int box_rows, CUtensorMap
 static bool g_wt_pdl = true;
 
 }  // namespace
+
+static WaitWord g_pair_wait_word([](int* v) -> int {
+  B200_CUDA(cudaMemcpyFromSymbol(v, g_pair_wait_failed, sizeof(int)));
+  return B200_OK;
+});
 
 void gemm_wt_set_pdl(bool on) { g_wt_pdl = on; }
 

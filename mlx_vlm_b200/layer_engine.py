@@ -254,4 +254,6 @@ class LayerEngine:
         return self._blog
 
     def device_error(self) -> int:
-        return 0
+        v = N.C.c_int(0)
+        N.check(self.lib.b200_wait_error(N.C.byref(v)), "wait_error", self.lib)
+        return int(v.value)

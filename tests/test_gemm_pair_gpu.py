@@ -154,3 +154,42 @@ def test_column_groups_beside_a_plain_product_of_pairs(tmp_path, line):
     assert r.returncode == 0, r.stdout + r.stderr
     added = path.read_text()[len(line) + 1:].split()
     assert added[:5] == ["5", "256", "64", "3", "0"] and int(added[6]) >= 1 and added[9] == "3" and len(added) == 10
+
+
+_CHILD_WAIT = """
+import sys, ctypes as C, torch
+sys.path.insert(0, {root!r})
+from mlx_vlm_b200 import _native as N
+lib = N.lib()
+def state():
+    v = C.c_int(-1)
+    N.check(lib.b200_wait_error(C.byref(v)))
+    return v.value
+T, n, K = {T}, {n}, {K}
+x = torch.randn(T, K, device="cuda").to(torch.bfloat16)
+w = torch.randn(n, K, device="cuda").to(torch.bfloat16)
+cfg = (C.c_int * 4)(128, 1, 4, 1)
+out = torch.zeros(T, n, device="cuda", dtype=torch.bfloat16)
+def run(flags):
+    out.zero_()
+    torch.cuda.synchronize()
+    N.check(lib.b200_gemm_wt(x.data_ptr(), K, w.data_ptr(), 0, 0, 0, out.data_ptr(), n, 0, T, n, K, 0, 0, 0, cfg, 8 | flags, 0))
+    torch.cuda.synchronize()
+want = (x.double() @ w.double().T).to(torch.bfloat16)
+run(0)
+assert torch.allclose(out.float(), want.float(), atol=0.5) and state() == 0
+run(2)                                # nothing is loaded: the waits run out after a second
+assert bool(torch.isnan(out.float()).all()) and state() == 5, (out, state())
+run(0)
+assert torch.allclose(out.float(), want.float(), atol=0.5) and state() == 5
+"""
+
+
+# fewer k-blocks than the ring has stages; several tiles of a pair and several rounds of the ring
+@pytest.mark.parametrize("T,n,K", [(128, 256, 64), (1300, 4096, 640)])
+def test_a_wait_that_runs_out_is_told(T, n, K):
+    """in a process of its own: NaN instead of an accumulator that is not whole, the word that the host reads, and the next launch
+    as if nothing had been"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _CHILD_WAIT.format(root=root, T=T, n=n, K=K)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
