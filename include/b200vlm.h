@@ -40,6 +40,7 @@ int b200_abi_version(void);
 int b200_device_check(int device, int* sm_count);
 /* Synchronous: which kernel gave up on a wait inside it (it then stores NaN) on the current device, 0 = none.  Stays set. */
 #define B200_WAIT_PAIR 5       /* gemm_wt_pair_kernel */
+#define B200_WAIT_ATTENTION 6  /* attention_fa_kernel */
 int b200_wait_error(int* out);
 
 /* ------------------------------------------------------------------------- */
@@ -137,6 +138,12 @@ int b200_attention(const void* q, long q_tok_stride, long q_head_stride,
 int b200_attention_fa(const void* q, long q_ts, long q_hs, const void* k, long k_ts, long k_hs,
                       const void* vt, long vt_hs, long vt_ds, void* out, long o_ts, int n_heads,
                       int n_kv, int hd, int Lq, int S, int causal, void* stream);
+/* the form that the engine runs: V rows, element (key, kv head, dim) at v + key*v_ts + kvh*v_hs + dim.  The tensors hold q_tot
+ * queries and k_tot keys; segs: optional device table of n_seg (first query, queries, first key, keys), Lq / S then the longest.
+ * flags: pass 0 (1, a debugging aid: nothing is loaded, the waits run out: NaN, b200_wait_error) */
+int b200_attention_fa_rows(const void* q, long q_ts, long q_hs, const void* k, long k_ts, long k_hs, const void* v, long v_ts,
+                           long v_hs, void* out, long o_ts, int n_heads, int n_kv, int hd, int Lq, int S, int causal, int q_tot,
+                           int k_tot, const int* segs, int n_seg, int flags, void* stream);
 /* vision tower after the qkv GEMM: 2-D rotary on q,k in place (vision.py:35-50), q pre-scaled
  * by bf16(scale), V^T written to vt[head][dim][t_ld] (t_ld % 8 == 0, >= n_tok) */
 int b200_vision_qkv_post(void* qkv, const int* pos_hw, const float* inv_freq, int n_tok, int n_heads,

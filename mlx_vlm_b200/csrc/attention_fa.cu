@@ -45,11 +45,12 @@ struct FaParams {
   int q0, k0;  // token offsets of this segment inside the tensors the maps describe
   const int4* segs;  // optional [gridDim.z]: (q0, Lq, k0, S) of segment blockIdx.z — several independent sequences of one
                      // concatenated batch in ONE launch (the tail wave of a 160-CTA launch per sequence idles half the SMs)
+  int flags;
 };
 
 struct FaBars {
   uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], s_empty[2], p_full[2], p_empty[2],
-      o_full;
+      o_full, drained[3];
 };
 
 __device__ __forceinline__ uint32_t f_u32(const void* p) {
@@ -65,22 +66,8 @@ __device__ __forceinline__ void f_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void f_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(f_u32(bar)) : "memory");
 }
-// Bounded: a wait that does not end (about a second) gives up, and so does every later one of the thread; the rows that it
-// would have stored become NaN.
-__device__ __forceinline__ void f_wait(uint64_t* bar, uint32_t parity, bool& dead) {
-  uint32_t done = 0;
-  const uint32_t addr = f_u32(bar);
-  for (int i = 0; !done && !dead; ++i) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (i > (1 << 24)) dead = true;
-  }
-}
+__device__ int g_fa_wait_failed;   // a wait of attention_fa_kernel ran out: B200_WAIT_ATTENTION
+
 __device__ __forceinline__ void f_tma_3d(void* dst, const CUtensorMap* tmap, uint64_t* bar, int c0, int c1,
                                          int c2) {
   asm volatile(
@@ -182,6 +169,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   extern __shared__ uint8_t fa_smem_raw[];
   __shared__ FaBars bars;
   __shared__ uint32_t tmem_slot;
+  __shared__ int failed;
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(fa_smem_raw) + 1023) &
                                            ~static_cast<uintptr_t>(1023));
   uint8_t* Qs = sm;                          // [128 q][128 d]            2 k-blocks
@@ -217,6 +205,8 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       f_init(&bars.p_empty[i], 1);
     }
     f_init(&bars.o_full, 1);
+    for (int i = 0; i < 3; ++i) f_init(&bars.drained[i], 1);
+    failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -231,15 +221,16 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   f_fence_after();
   const uint32_t tmem = tmem_slot;
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  bool dead = false;
+  int k_loads = 0, v_loads = 0;   // of the producer
 
   if (warp == 0) {
-    if (lane == 0) {  // ===== TMA producer =====
+    if (lane == 0 && !(p.flags & 1)) {  // ===== TMA producer (flags 1: no loads, every wait for them runs out) =====
       f_expect_tx(&bars.q_full, (uint32_t)kbq * FA_BLK);
       for (int c = 0; c < kbq; ++c) f_tma_3d(Qs + c * FA_BLK, &tmQ, &bars.q_full, c * 64, h, p.q0 + row0);
       auto load_v = [&](int j) {
         const int sv = j & 1;
-        f_wait(&bars.v_empty[sv], ((j >> 1) & 1) ^ 1, dead);
+        if (!mbar_wait(&bars.v_empty[sv], ((j >> 1) & 1) ^ 1, &failed)) return false;
+        ++v_loads;
         if constexpr (VT) {
           f_expect_tx(&bars.v_full[sv], 2u * (uint32_t)vblk);
           for (int c = 0; c < 2; ++c)
@@ -249,28 +240,31 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           for (int c = 0; c < kbq; ++c)
             f_tma_3d(Vs + sv * 2 * FA_BLK + c * FA_BLK, &tmV, &bars.v_full[sv], c * 64, kvh, p.k0 + j * FA_TK);
         }
+        return true;
       };
       int jk = 0;   // key tile of step i
-      for (int i = 0; i < 2 * n_tiles; ++i) {
+      bool ok = true;
+      for (int i = 0; i < 2 * n_tiles && ok; ++i) {
         const int s = i & 1;
-        f_wait(&bars.k_empty[s], ((i >> 1) & 1) ^ 1, dead);
+        if (!(ok = mbar_wait(&bars.k_empty[s], ((i >> 1) & 1) ^ 1, &failed))) break;
+        ++k_loads;
         f_expect_tx(&bars.k_full[s], (uint32_t)kbq * FA_BLK);
         for (int c = 0; c < kbq; ++c)
           f_tma_3d(Ks + s * 2 * FA_BLK + c * FA_BLK, &tmK, &bars.k_full[s], c * 64, kvh, p.k0 + jk * FA_TK);
         if (++jk == n_tiles) jk = 0;
-        if (i >= n_tiles + 2) load_v(i - n_tiles - 2);   // (in the order of the products: a wait for V holds up no K before it)
+        if (i >= n_tiles + 2) ok = load_v(i - n_tiles - 2);   // (in the order of the products: a wait for V holds up no K before it)
       }
-      for (int j = max(0, n_tiles - 2); j < n_tiles; ++j) load_v(j);
+      for (int j = max(0, n_tiles - 2); j < n_tiles && ok; ++j) ok = load_v(j);
     }
   } else if (warp == 1 || warp == 18) {
     if (lane == 0) {  // ===== issuer of Q.K^T, of every other step =====
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(FA_TK >> 3) << 17) | (8u << 24);
       const int ksteps = p.hdp >> 4, s = warp == 1 ? 0 : 1;
       const uint32_t q_lo = f_desc_lo(f_u32(Qs)), k_lo = f_desc_lo(f_u32(Ks + s * 2 * FA_BLK)), d = tmem + (uint32_t)s * 128u;
-      f_wait(&bars.q_full, 0, dead);
-      for (int i = s; i < 2 * n_tiles; i += 2) {
-        f_wait(&bars.k_full[s], (i >> 1) & 1, dead);
-        f_wait(&bars.s_empty[s], ((i >> 1) & 1) ^ 1, dead);
+      bool ok = mbar_wait(&bars.q_full, 0, &failed);
+      for (int i = s; i < 2 * n_tiles && ok; i += 2) {
+        ok = mbar_wait(&bars.k_full[s], (i >> 1) & 1, &failed) && mbar_wait(&bars.s_empty[s], ((i >> 1) & 1) ^ 1, &failed);
+        if (!ok) break;
         f_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
@@ -287,12 +281,13 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       // (bit 16: the B operand is MN-major)
       const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (VT ? 0u : 1u << 16) | ((uint32_t)(p.hdp >> 3) << 17) |
                                (8u << 24);
+      bool ok = true;
       for (int j = 0; j < n_tiles; ++j) {
         const int sv = j & 1, sp = (n_tiles + j) & 1;
         const uint32_t p_lo = f_desc_lo(f_u32(Ps + sp * 2 * FA_BLK));
         const uint32_t v_lo = VT ? f_desc_lo(f_u32(Vs + sv * 2 * FA_BLK)) : f_desc_lo_mn(f_u32(Vs + sv * 2 * FA_BLK));
-        f_wait(&bars.v_full[sv], (j >> 1) & 1, dead);
-        f_wait(&bars.p_full[sp], (j >> 1) & 1, dead);
+        ok = mbar_wait(&bars.v_full[sv], (j >> 1) & 1, &failed) && mbar_wait(&bars.p_full[sp], (j >> 1) & 1, &failed);
+        if (!ok) break;
         f_fence_after();
         // (groups of 16 keys that lie wholly behind the segment's last key are left out)
         const int ks_n = VT ? FA_TK / 16 : min(FA_TK / 16, (S - j * FA_TK + 15) >> 4);
@@ -307,7 +302,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         f_commit(&bars.p_empty[sp]);
         f_commit(&bars.v_empty[sv]);
       }
-      f_commit(&bars.o_full);
+      if (ok) f_commit(&bars.o_full);   // (an output that is not whole is not handed over)
     }
   } else {
     // ===== softmax warps: thread = (group, query row, score-column half) =====
@@ -328,10 +323,11 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const uint64_t log2e = f2(LOG2E, LOG2E);
     uint32_t pk[32];
     float m = -INFINITY, l = 0.f;
+    bool ok = true;   // (the same in a warp)
     for (int i = grp; i < n_tiles; i += 2) {  // ---- pass 1: row max and sum of exp over bf16 scores ----
       const int s = grp;
-      f_wait(&bars.s_full[s], (i >> 1) & 1, dead);
-      __syncwarp();
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars.s_full[s], (i >> 1) & 1, &failed));
+      if (!ok) break;
       f_fence_after();
       f_scores(t_row + (uint32_t)(s * 128 + half * 64), vis - (i * FA_TK + half * 64), pk);
       f_fence_before();
@@ -368,10 +364,10 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     f_sbar();   // (the first P tile goes where the statistics were)
     const float inv_l = 1.0f / l;
     const uint64_t nbm = f2(-m * LOG2E, -m * LOG2E), inv2 = f2(inv_l, inv_l);
-    for (int j = (n_tiles ^ grp) & 1; j < n_tiles; j += 2) {  // ---- pass 2: p = bf16(exp(s - m) / l) -> shared memory ----
+    for (int j = (n_tiles ^ grp) & 1; j < n_tiles && ok; j += 2) {  // ---- pass 2: p = bf16(exp(s - m) / l) -> shared memory ----
       const int i = n_tiles + j, s = grp;
-      f_wait(&bars.s_full[s], (i >> 1) & 1, dead);
-      __syncwarp();
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars.s_full[s], (i >> 1) & 1, &failed));
+      if (!ok) break;
       f_fence_after();
       f_scores(t_row + (uint32_t)(s * 128 + half * 64), vis - (j * FA_TK + half * 64), pk);
       f_fence_before();
@@ -382,7 +378,8 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const uint64_t w = mul2(f2(f_ex2(f2_lo(x)), f_ex2(f2_hi(x))), inv2);
         pk[e] = pack2(f2_lo(w), f2_hi(w));
       }
-      f_wait(&bars.p_empty[s], ((j >> 1) & 1) ^ 1, dead);  // the group's previous P.V has consumed the P tile
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars.p_empty[s], ((j >> 1) & 1) ^ 1, &failed));  // the group's previous P.V has consumed the P tile
+      if (!ok) break;
       uint8_t* prow = Ps + (2 * s + half) * FA_BLK + row * 128;
 #pragma unroll
       for (int c = 0; c < 8; ++c)
@@ -392,7 +389,8 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         // or an infinity would still reach O: those of the last group of 16 keys that is multiplied are cleared
         const int first = S - j * FA_TK, end = (first + 15) & ~15;
         if (first < FA_TK && first != end) {
-          f_wait(&bars.v_full[j & 1], (j >> 1) & 1, dead);
+          ok = __all_sync(0xffffffffu, mbar_wait(&bars.v_full[j & 1], (j >> 1) & 1, &failed));
+          if (!ok) break;
           const int per = kbq * 8;
           for (int idx = (threadIdx.x - 64) & 255; idx < (end - first) * per; idx += 256) {
             const int r = first + idx / per, ch = idx % per;
@@ -405,13 +403,13 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       f_arrive(&bars.p_full[s]);
     }
     // ---- epilogue: O row -> bf16 -> global (16-column chunks go round the row's four threads) ----
-    f_wait(&bars.o_full, 0, dead);
+    ok = ok && __all_sync(0xffffffffu, mbar_wait(&bars.o_full, 0, &failed));
     f_fence_after();
     bf16* orow = p.out + (long)(p.q0 + qi) * p.o_ts + (long)h * p.hd;
     for (int c0 = 16 * (2 * grp + half); c0 < p.hd; c0 += 64) {
       uint32_t r[16];
       f_tmem_ld16(t_row + 256u + (uint32_t)c0, r);
-      if (dead)
+      if (!ok)
         for (int e = 0; e < 16; ++e) r[e] = 0x7FC00000u;
       if (qi < p.Lq) {
         if (c0 + 16 <= p.hd) {
@@ -434,6 +432,21 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   }
   f_fence_before();
   __syncthreads();
+  if (failed) {   // nothing is left in flight: the last loads of every slot, the products of each issuer
+    if (lane == 0 && (warp < 2 || warp >= 18)) {
+      if (warp == 0) {
+        g_fa_wait_failed = B200_WAIT_ATTENTION;
+        if (!(p.flags & 1)) mbar_drain(&bars.q_full, 0);
+        for (int i = max(0, k_loads - 2); i < k_loads; ++i) mbar_drain(&bars.k_full[i & 1], (i >> 1) & 1);
+        for (int i = max(0, v_loads - 2); i < v_loads; ++i) mbar_drain(&bars.v_full[i & 1], (i >> 1) & 1);
+      } else {
+        uint64_t* mine = &bars.drained[warp == 1 ? 0 : warp - 17];
+        f_commit(mine);
+        mbar_drain(mine, 0);
+      }
+    }
+    __syncthreads();
+  }
   if (warp == 1) {
     f_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
@@ -516,6 +529,11 @@ int fa_tmap3(const void* ptr, int d0, int d1, long s1, int d2, long s2, int b0, 
 
 }  // namespace
 
+static WaitWord g_fa_wait_word([](int* v) -> int {
+  B200_CUDA(cudaMemcpyFromSymbol(v, g_fa_wait_failed, sizeof(int)));
+  return B200_OK;
+});
+
 // v: V^T (strides head, dim) or V rows (strides token, head): the same alignment rules
 bool attention_fa_supported(const void* q, long q_ts, long q_hs, const void* k, long k_ts, long k_hs,
                             const void* vt, long vt_hs, long vt_ds, const void* out, long o_ts, int hd) {
@@ -535,7 +553,7 @@ bool attention_fa_supported(const void* q, long q_ts, long q_hs, const void* k, 
 int attention_fa(const void* q, long q_ts, long q_hs, const void* k, long k_ts, long k_hs, const void* v,
                  long v_s0, long v_s1, void* out, long o_ts, int n_heads, int n_kv, int hd, int Lq, int S,
                  int causal, cudaStream_t st, int q0, int q_tot, int k0, int k_tot, const void* segs, int n_seg,
-                 bool v_transposed) {
+                 bool v_transposed, int flags) {
   if (q_tot <= 0) q_tot = q0 + Lq;
   if (k_tot <= 0) k_tot = k0 + S;
   B200_REQUIRE(!segs || n_seg > 0, "attention_fa: segment table without segments");
@@ -559,6 +577,7 @@ int attention_fa(const void* q, long q_ts, long q_hs, const void* k, long k_ts, 
   p.out = (bf16*)out; p.o_ts = o_ts; p.n_heads = n_heads; p.n_kv = n_kv; p.hd = hd; p.hdp = hdp;
   p.Lq = Lq; p.S = S; p.causal = causal; p.q0 = q0; p.k0 = k0;
   p.segs = (const int4*)segs;
+  p.flags = flags;
   B200_CUDA(launch_pdl(kern, dim3(n_heads, cdiv(Lq, FA_TQ), segs ? n_seg : 1), dim3(FA_THREADS), smem, st, tq, tk, tv, p));
   return B200_OK;
 }
@@ -570,4 +589,10 @@ extern "C" int b200_attention_fa(const void* q, long q_ts, long q_hs, const void
                                  int n_kv, int hd, int Lq, int S, int causal, void* stream) {
   return b200::attention_fa(q, q_ts, q_hs, k, k_ts, k_hs, vt, vt_hs, vt_ds, out, o_ts, n_heads, n_kv, hd, Lq, S,
                             causal, (cudaStream_t)stream, 0, Lq, 0, S, nullptr, 0, true);
+}
+extern "C" int b200_attention_fa_rows(const void* q, long q_ts, long q_hs, const void* k, long k_ts, long k_hs, const void* v,
+                                      long v_ts, long v_hs, void* out, long o_ts, int n_heads, int n_kv, int hd, int Lq, int S,
+                                      int causal, int q_tot, int k_tot, const int* segs, int n_seg, int flags, void* stream) {
+  return b200::attention_fa(q, q_ts, q_hs, k, k_ts, k_hs, v, v_ts, v_hs, out, o_ts, n_heads, n_kv, hd, Lq, S, causal,
+                            (cudaStream_t)stream, 0, q_tot, 0, k_tot, segs, n_seg, false, flags);
 }

@@ -169,7 +169,8 @@ int attention_fa(const void* q, long q_ts, long q_hs, const void* k, long k_ts, 
                  long v_s0, long v_s1, void* out, long o_ts, int n_heads, int n_kv, int hd, int Lq, int S,
                  int causal, cudaStream_t st, int q0 = 0, int q_tot = 0, int k0 = 0, int k_tot = 0,
                  const void* segs = nullptr, int n_seg = 0,    // segs: device int4 (q0, Lq, k0, S) per segment; Lq / S = the longest
-                 bool v_transposed = false);                   // V rows (token, head strides) or V^T (head, dim strides)
+                 bool v_transposed = false,                    // V rows (token, head strides) or V^T (head, dim strides)
+                 int flags = 0);                               // 1: nothing is loaded (the waits run out)
 int swiglu(const void* gu, void* out, int rows, int inter, cudaStream_t st);
 int embed_merge(const int* ids, int B, int T, const void* table, int hidden, const void* feats,
                 int n_feats, int image_token, int video_token, void* out, int* src_out,
