@@ -50,7 +50,7 @@ struct FaParams {
 
 struct FaBars {
   uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], s_empty[2], p_full[2], p_empty[2],
-      o_full, drained[3];
+      o_full, dropped, drained[3];
 };
 
 __device__ __forceinline__ uint32_t f_u32(const void* p) {
@@ -205,6 +205,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       f_init(&bars.p_empty[i], 1);
     }
     f_init(&bars.o_full, 1);
+    f_init(&bars.dropped, 1);
     for (int i = 0; i < 3; ++i) f_init(&bars.drained[i], 1);
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -261,10 +262,11 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(FA_TK >> 3) << 17) | (8u << 24);
       const int ksteps = p.hdp >> 4, s = warp == 1 ? 0 : 1;
       const uint32_t q_lo = f_desc_lo(f_u32(Qs)), k_lo = f_desc_lo(f_u32(Ks + s * 2 * FA_BLK)), d = tmem + (uint32_t)s * 128u;
-      bool ok = mbar_wait(&bars.q_full, 0, &failed);
-      for (int i = s; i < 2 * n_tiles && ok; i += 2) {
-        ok = mbar_wait(&bars.k_full[s], (i >> 1) & 1, &failed) && mbar_wait(&bars.s_empty[s], ((i >> 1) & 1) ^ 1, &failed);
-        if (!ok) break;
+      bool dead = false;
+      mbar_wait_issuer(&bars.q_full, 0, dead);
+      for (int i = s; i < 2 * n_tiles; i += 2) {
+        mbar_wait_issuer(&bars.k_full[s], (i >> 1) & 1, dead);
+        mbar_wait_issuer(&bars.s_empty[s], ((i >> 1) & 1) ^ 1, dead);
         f_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
@@ -272,22 +274,23 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           const uint32_t off = (uint32_t)((ks >> 2) * (FA_BLK >> 4) + (ks & 3) * 2);
           f_umma(d, q_lo + off, k_lo + off, F_DESC_HI, idesc_s, ks > 0 ? 1u : 0u);
         }
-        f_commit(&bars.k_empty[s]);
-        f_commit(&bars.s_full[s]);
+        f_commit(dead ? &bars.dropped : &bars.k_empty[s]);
+        f_commit(dead ? &bars.dropped : &bars.s_full[s]);
       }
+      if (dead) *static_cast<volatile int*>(&failed) = 1;
     }
   } else if (warp == 19) {
     if (lane == 0) {  // ===== issuer of P.V =====
       // (bit 16: the B operand is MN-major)
       const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (VT ? 0u : 1u << 16) | ((uint32_t)(p.hdp >> 3) << 17) |
                                (8u << 24);
-      bool ok = true;
+      bool dead = false;
       for (int j = 0; j < n_tiles; ++j) {
         const int sv = j & 1, sp = (n_tiles + j) & 1;
         const uint32_t p_lo = f_desc_lo(f_u32(Ps + sp * 2 * FA_BLK));
         const uint32_t v_lo = VT ? f_desc_lo(f_u32(Vs + sv * 2 * FA_BLK)) : f_desc_lo_mn(f_u32(Vs + sv * 2 * FA_BLK));
-        ok = mbar_wait(&bars.v_full[sv], (j >> 1) & 1, &failed) && mbar_wait(&bars.p_full[sp], (j >> 1) & 1, &failed);
-        if (!ok) break;
+        mbar_wait_issuer(&bars.v_full[sv], (j >> 1) & 1, dead);
+        mbar_wait_issuer(&bars.p_full[sp], (j >> 1) & 1, dead);
         f_fence_after();
         // (groups of 16 keys that lie wholly behind the segment's last key are left out)
         const int ks_n = VT ? FA_TK / 16 : min(FA_TK / 16, (S - j * FA_TK + 15) >> 4);
@@ -299,10 +302,11 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           const uint32_t b = VT ? v_lo + (uint32_t)((ks >> 2) * (vblk >> 4) + (ks & 3) * 2) : v_lo + (uint32_t)(ks * (2048 >> 4));
           f_umma(tmem + 256, a, b, F_DESC_HI, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
         }
-        f_commit(&bars.p_empty[sp]);
-        f_commit(&bars.v_empty[sv]);
+        f_commit(dead ? &bars.dropped : &bars.p_empty[sp]);
+        f_commit(dead ? &bars.dropped : &bars.v_empty[sv]);
       }
-      if (ok) f_commit(&bars.o_full);   // (an output that is not whole is not handed over)
+      f_commit(dead ? &bars.dropped : &bars.o_full);   // (an output that is not whole is not handed over)
+      if (dead) *static_cast<volatile int*>(&failed) = 1;
     }
   } else {
     // ===== softmax warps: thread = (group, query row, score-column half) =====

@@ -508,7 +508,7 @@ constexpr int WP_THREADS = 384;
 constexpr int WP_MAX_STAGES = 12;
 
 struct WpBars {
-  uint64_t full[WP_MAX_STAGES], empty[WP_MAX_STAGES], acc_full[2], acc_empty[2], drained;
+  uint64_t full[WP_MAX_STAGES], empty[WP_MAX_STAGES], acc_full[2], acc_empty[2], dropped, drained;
 };
 
 __device__ int g_pair_wait_failed;   // a wait of gemm_wt_pair_kernel ran out: B200_WAIT_PAIR
@@ -561,7 +561,8 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   const int row_tiles = ((swiglu ? 2 * p.inter : p.N) + 2 * WT_ROWS - 1) / (2 * WT_ROWS), tok_tiles = (p.T + p.TN - 1) / p.TN;
   const int splits = (kb_total + p.kb_per_split - 1) / p.kb_per_split;
   const int n_tiles = row_tiles * tok_tiles * splits;
-  int loads = 0;   // of this CTA's producer
+  int s_next = 0;             // the producer's next slot
+  uint32_t free_parity = 1;   // and the phase in which it is free
   // tile -> this CTA's first output feature, its first token, its k-blocks
   auto tile_at = [&](int tile, int& n0, int& t0, int& split, int& kb0, int& kb1) {
     t0 = tile % tok_tiles * p.TN;
@@ -584,6 +585,7 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       w_mbar_init(&bars.acc_full[b], 1);
       w_mbar_init(&bars.acc_empty[b], 16);   // eight epilogue warps of each CTA
     }
+    w_mbar_init(&bars.dropped, 1);
     w_mbar_init(&bars.drained, 1);
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -601,11 +603,9 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   const uint32_t tmem = tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {  // ===== TMA producer =====
+    if (lane == 0 && !(p.flags & 2u)) {  // ===== TMA producer (flags 2: nothing is loaded; a test in its loop cost 2 %) =====
       const uint32_t full0 = wp_leader(&bars.full[0]);
       auto load_w = [&](int s, int kb, int n0) {
-        if (p.flags & 2u) return;   // (no loads: every wait for them runs out)
-        ++loads;
         if (p.kb_w > 0) kb %= p.kb_w;
         uint8_t* sW = ring + (long)s * stage_bytes;
         const uint32_t bar = full0 + s * 8;
@@ -618,7 +618,6 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
         }
       };
       auto load_x = [&](int s, int kb, int t0) {
-        if (p.flags & 2u) return;
         wp_tma_2d(ring + (long)s * stage_bytes + WT_WBLK, &tmX, full0 + s * 8, kb * WT_BK, t0 + rank * xhalf);
       };
       int n0, t0, split, kb0, kb1;
@@ -631,7 +630,6 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       }
       w_pdl_wait();
       int s = 0;
-      uint32_t free_parity = 1;
       bool ok = true;
       for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
         tile_at(tile, n0, t0, split, kb0, kb1);
@@ -647,6 +645,7 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
           if (++s == NS) s = 0, free_parity ^= 1;
         }
       }
+      s_next = s;
     }
   } else if (warp == 1) {
     if (rank == 0 && lane == 0) {  // ===== MMA issuer =====
@@ -657,30 +656,30 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       const uint32_t step = (uint32_t)stage_bytes >> 4;
       int s = 0, j = 0, n0, t0, split, kb0, kb1;
       uint32_t w_lo = w_first, x_lo = x_first, parity = 0;
-      bool ok = true;
+      bool dead = false;
       w_pdl_wait();   // (the time of a wait starts when the tokens can be on their way)
       for (int tile = pair; tile < n_tiles; tile += n_pairs, ++j) {
         tile_at(tile, n0, t0, split, kb0, kb1);
         const uint32_t d = tmem + (uint32_t)(j & 1) * 256u;
-        if (!(ok = mbar_wait(&bars.acc_empty[j & 1], ((j >> 1) & 1) ^ 1, &failed))) break;
+        mbar_wait_issuer(&bars.acc_empty[j & 1], ((j >> 1) & 1) ^ 1, dead);
         w_fence_after();
         uint32_t acc = 0;
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!(ok = mbar_wait(&bars.full[s], parity, &failed))) break;
+          mbar_wait_issuer(&bars.full[s], parity, dead);
           w_fence_after();
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             wp_umma(d, w_lo + k * 2, x_lo + k * 2, idesc, acc);
             acc = 1;
           }
-          wp_commit(&bars.empty[s]);
+          wp_commit(dead ? &bars.dropped : &bars.empty[s]);
           w_lo += step;
           x_lo += step;
           if (++s == NS) s = 0, w_lo = w_first, x_lo = x_first, parity ^= 1;
         }
-        if (!ok) break;   // (an accumulator that is not whole is not handed over)
-        wp_commit(&bars.acc_full[j & 1]);
+        wp_commit(dead ? &bars.dropped : &bars.acc_full[j & 1]);   // (an accumulator that is not whole is not handed over)
       }
+      if (dead) *static_cast<volatile int*>(&failed) = 1;
     }
   } else if (warp >= 4) {  // ===== epilogue =====
     w_pdl_wait();
@@ -714,7 +713,7 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     if (rank == 0 && lane == 0) {
       if (warp == 0) {
         g_pair_wait_failed = B200_WAIT_PAIR;
-        for (int i = max(0, loads - NS); i < loads; ++i) mbar_drain(&bars.full[i % NS], (i / NS) & 1);
+        for (int i = 0; i < NS; ++i) mbar_drain(&bars.full[i], i < s_next ? free_parity ^ 1 : free_parity);   // (never loaded: ends at once)
       } else if (warp == 1) {
         wp_commit(&bars.drained);
         mbar_drain(&bars.drained, 0);
