@@ -41,6 +41,7 @@ int b200_device_check(int device, int* sm_count);
 /* Synchronous: which kernel gave up on a wait inside it (it then stores NaN) on the current device, 0 = none.  Stays set. */
 #define B200_WAIT_PAIR 5       /* gemm_wt_pair_kernel */
 #define B200_WAIT_ATTENTION 6  /* attention_fa_kernel */
+#define B200_WAIT_TOWER 7      /* attention_f32_tc_kernel */
 int b200_wait_error(int* out);
 
 /* ------------------------------------------------------------------------- */
@@ -312,6 +313,10 @@ int b200_attention_f32(const float* q, long q_ts, long q_hs, const float* k, lon
                        long v_ts, long v_hs, float* out32, long o_ts, void* out_split, long os_ts, int n_pad,
                        int n_heads, int n_kv, int hd, int Lq, int S, int n_seg, long q_seg, long k_seg,
                        const unsigned char* key_mask, float scale, void* stream);
+/* the same on one segment without a mask, flags a debugging aid (1: nothing is loaded, the waits run out: NaN, b200_wait_error) */
+int b200_attention_f32_debug(const float* q, long q_ts, long q_hs, const float* k, long k_ts, long k_hs, const float* v,
+                             long v_ts, long v_hs, float* out32, long o_ts, int n_heads, int n_kv, int hd, int Lq, int S,
+                             float scale, int flags, void* stream);
 /* the same attention over RAGGED self-attention segments: segment z = tokens [cu_seqlens[z], cu_seqlens[z+1]) of q, k and
  * v (device int array of n_seg + 1 entries); max_len = the longest segment.  Qwen2.5-VL's windowed blocks
  * (qwen2_5_vl/vision.py:147-160: one SDPA per split of cu_seqlens). */

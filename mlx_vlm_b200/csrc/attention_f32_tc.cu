@@ -39,7 +39,7 @@ constexpr int TC_QB = TC_ROWS * 16 + 16, TC_KB = TC_KEYS * 16 + 16;   // bytes o
 constexpr int TC_P0 = 128, TC_O0 = 320, TC_GB = 96;   // TMEM columns: S 2 x 64 | P 2 x (3 x 32) | O 2 x 96
 
 struct TcBars {
-  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], o_full[2];
+  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], o_full[2], drained, dropped;
 };
 
 __device__ __forceinline__ uint32_t t_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -49,22 +49,7 @@ __device__ __forceinline__ void t_init(uint64_t* bar, uint32_t n) {
 __device__ __forceinline__ void t_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(t_u32(bar)) : "memory");
 }
-// Bounded: a wait that does not end (about a second) gives up, and so does every later one of the thread; the rows that it
-// would have stored become NaN.
-__device__ __forceinline__ void t_wait(uint64_t* bar, uint32_t parity, bool& dead) {
-  uint32_t done = 0;
-  const uint32_t addr = t_u32(bar);
-  for (int i = 0; !done && !dead; ++i) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (i > (1 << 24)) dead = true;
-  }
-}
+__device__ int g_f32_wait_failed;   // a wait of attention_f32_tc_kernel ran out: B200_WAIT_TOWER
 __device__ __forceinline__ void t_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void t_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void t_fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -253,6 +238,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
   __shared__ TcBars bars;
   __shared__ uint32_t tmem_slot;
   __shared__ float2 stat[2][TC_ROWS];
+  __shared__ int failed;
   __shared__ uint32_t odd[8];   // rows with a result that is not finite, one bit each: [half of the dims][row / 32]
   constexpr int QP = tc_q_part<HDP>(), KP = tc_k_part<HDP>(), VP = tc_v_part<HDP>();
   uint8_t* Qs = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_raw) + 127) & ~static_cast<uintptr_t>(127));
@@ -269,10 +255,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
     if (q0 >= Lq) return;   // uniform per CTA, nothing is allocated yet
   }
   const int n_tiles = (S + TC_KEYS - 1) / TC_KEYS;
-  bool dead = false;
-
   if (tid == 0) {
+    failed = 0;
     t_init(&bars.q_full, 256);
+    t_init(&bars.drained, 1);
+    t_init(&bars.dropped, 1);
     for (int i = 0; i < 2; ++i) {
       t_init(&bars.k_full[i], TC_LOADERS);
       t_init(&bars.v_full[i], TC_LOADERS);
@@ -303,10 +290,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
       constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
       constexpr int KS = HDP / 16, VL = HDP * 16 + 16;
       const uint32_t q_lo = t_desc(t_u32(Qs), TC_QB), k_lo = t_desc(t_u32(Ks), TC_KB), v_lo = t_desc(t_u32(Vs), VL);
+      bool dead = false;
       auto keys16 = [&](int j) { return min(TC_KEYS, (S - j * TC_KEYS + 15) & ~15); };
       auto issue_s = [&](int j) {
         const int s = j & 1;
-        t_wait(&bars.k_full[s], (j >> 1) & 1, dead);
+        mbar_wait_issuer(&bars.k_full[s], (j >> 1) & 1, dead);
         t_fence_after();
         const uint32_t idesc = ID | ((uint32_t)(keys16(j) >> 3) << 17), d = tmem + (uint32_t)s * TC_KEYS;
         const uint32_t ka = k_lo + s * (3 * KP >> 4);
@@ -316,16 +304,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
           const int t = i / KS, ks = i % KS;
           t_mma_ss<true>(d, q_lo + ((PA[t] * QP + ks * 2 * TC_QB) >> 4), ka + ((PB[t] * KP + ks * 2 * TC_KB) >> 4), idesc);
         }
-        t_commit(&bars.k_empty[s]);
-        t_commit(&bars.s_full[s]);
+        t_commit(dead ? &bars.dropped : &bars.k_empty[s]);
+        t_commit(dead ? &bars.dropped : &bars.s_full[s]);
       };
-      t_wait(&bars.q_full, 0, dead);
+      mbar_wait_issuer(&bars.q_full, 0, dead);
       issue_s(0);
       if (n_tiles > 1) issue_s(1);
       for (int j = 0; j < n_tiles; ++j) {
         const int s = j & 1;
-        t_wait(&bars.p_full[s], (j >> 1) & 1, dead);
-        t_wait(&bars.v_full[s], (j >> 1) & 1, dead);
+        mbar_wait_issuer(&bars.p_full[s], (j >> 1) & 1, dead);
+        mbar_wait_issuer(&bars.v_full[s], (j >> 1) & 1, dead);
         t_fence_after();
         const uint32_t d = tmem + TC_O0 + s * TC_GB, pa = tmem + TC_P0 + s * TC_GB, va = v_lo + s * (3 * VP >> 4);
         t_mma_ts<false>(d, pa + PA[0] * 32, va + (PB[0] * VP >> 4), ID_O);
@@ -342,9 +330,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
             for (int ks = t == 0 ? 1 : 0; ks < steps; ++ks)
               t_mma_ts<true>(d, pa + PA[t] * 32 + ks * 8, va + ((PB[t] * VP) >> 4) + ks * (2 * VL >> 4), ID_O);
         }
-        t_commit(&bars.v_empty[s]);
-        t_commit(&bars.o_full[s]);
+        t_commit(dead ? &bars.dropped : &bars.v_empty[s]);
+        t_commit(dead ? &bars.dropped : &bars.o_full[s]);
         if (j + 2 < n_tiles) issue_s(j + 2);   // (the group has read S of tile j: it has stored its P)
+      }
+      if (dead) {   // no product is left in flight; the threads that wait for what was dropped give up as well
+        *static_cast<volatile int*>(&failed) = 1;
+        t_commit(&bars.drained);
+        mbar_drain(&bars.drained, 0);
       }
     }
   } else if (warp >= 8) {  // ===== keys and values of a tile =====
@@ -362,14 +355,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
 #pragma unroll
       for (int u = 0; u < VU; ++u)
         if ((wv + u * (TC_LOADERS / 32)) * 16 < HDP) load_values(x[u], vb + (long)j * TC_KEYS * p.v_ts, p.v_ts, rows, p.hd, (wv + u * (TC_LOADERS / 32)) * 16, lane);
-      t_wait(&bars.k_empty[s], free_parity, dead);
+      if (p.flags & 1) break;   // (nothing is loaded: every wait for it runs out)
+      if (!mbar_wait(&bars.k_empty[s], free_parity, &failed)) break;
       store_items<HDP, TC_KEYS, U, TC_LOADERS>(Ks + s * 3 * KP, KP, ka, kc, t, 1.f);
       t_fence_async();
       t_arrive(&bars.k_full[s]);
       if (j + 1 < n_tiles)
         load_items<HDP, TC_KEYS, U, TC_LOADERS, false>(ka, kc, t, kb + (long)(j + 1) * TC_KEYS * p.k_ts, p.k_ts,
                                                 min(TC_KEYS, S - (j + 1) * TC_KEYS), p.hd);
-      t_wait(&bars.v_empty[s], free_parity, dead);
+      if (!mbar_wait(&bars.v_empty[s], free_parity, &failed)) break;
 #pragma unroll
       for (int u = 0; u < VU; ++u) {
         const int dim = (wv + u * (TC_LOADERS / 32)) * 16;
@@ -408,6 +402,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
       }
     };
     int t = 0;
+    bool ok = true;   // (the same in a warp)
     for (int j = g; j < n_tiles; j += 2, ++t) {
       // keys of this tile that take part, one bit each
       uint32_t on[2];
@@ -416,8 +411,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
         const int key = j * TC_KEYS + w * 32 + lane;
         on[w] = __ballot_sync(0xffffffffu, key < S && (!p.key_mask || p.key_mask[(long)seg * S + key]));
       }
-      t_wait(&bars.s_full[g], t & 1, dead);
-      __syncwarp();
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars.s_full[g], t & 1, &failed));
+      if (!ok) break;
       t_fence_after();
       uint32_t v[2][16];
       const bool all = (on[0] & on[1]) == 0xffffffffu;
@@ -444,8 +439,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
       m = mn;
       l2 = mul2(l2, f2(f, f));
       if (t > 0) {   // (the last P.V has also read P: it may be written again)
-        t_wait(&bars.o_full[g], (t - 1) & 1, dead);
-        __syncwarp();
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars.o_full[g], (t - 1) & 1, &failed));
+        if (!ok) break;
         t_fence_after();
         add_tile(f);
       }
@@ -472,18 +467,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
       t_fence_before();
       t_arrive(&bars.p_full[g]);
     }
-    if (t > 0) {
-      t_wait(&bars.o_full[g], (t - 1) & 1, dead);
-      __syncwarp();
-      t_fence_after();
-      add_tile(1.f);
+    if (ok && t > 0) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars.o_full[g], (t - 1) & 1, &failed));
+      if (ok) {
+        t_fence_after();
+        add_tile(1.f);
+      }
     }
     // ---- merge: each group stores half of the dims and gets the other group's share of them through the tiles' memory,
     //      which no MMA reads any more ----
     const int rows = min(TC_ROWS, Lq - q0);
     uint64_t* ox = reinterpret_cast<uint64_t*>(Ks);   // [HDP / 2 pairs][128 rows]
     asm volatile("bar.sync 1, 256;" ::: "memory");
-    const float l = dead ? NAN : f2_lo(l2) + f2_hi(l2);
+    const bool whole = !*static_cast<volatile int*>(&failed);   // (else all rows of the CTA are NaN)
+    const float l = whole ? f2_lo(l2) + f2_hi(l2) : NAN;
     stat[g][row] = make_float2(m, l);
     auto give = [&](auto first) {
 #pragma unroll
@@ -512,10 +509,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
           a[2 * u + 1] = (f2_hi(x) * fa + f2_hi(y) * fb) * inv;
         }
         *reinterpret_cast<float4*>(of + row * PITCH + (first.value + e) * 2) = make_float4(a[0], a[1], a[2], a[3]);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) zero = fmaf(a[u], 0.f, zero);   // (NaN from the first that is not finite on)
+        zero = fmaf((a[0] + a[1]) + (a[2] + a[3]), 0.f, zero);   // (NaN from the first that is not finite on)
       }
-      const uint32_t bits = __ballot_sync(0xffffffffu, !(zero == 0.f) && row < rows && !dead);
+      const uint32_t bits = __ballot_sync(0xffffffffu, !(zero == 0.f) && row < rows && whole);
       if (lane == 0) odd[warp] = bits;
     };
     if (g == 0) take(low);
@@ -566,6 +562,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
   }
   t_fence_before();
   __syncthreads();
+  if (tid == 0 && failed) g_f32_wait_failed = B200_WAIT_TOWER;
   if (warp == 11) {
     t_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
@@ -583,6 +580,11 @@ int tc_launch(const AttnF32P& p, dim3 grid, cudaStream_t st) {
 }
 
 }  // namespace
+
+static WaitWord g_f32_wait_word([](int* v) -> int {
+  B200_CUDA(cudaMemcpyFromSymbol(v, g_f32_wait_failed, sizeof(int)));
+  return B200_OK;
+});
 
 int attention_f32_tc(AttnF32P p, int n_seg, cudaStream_t st) {
   p.out_vec = ((uintptr_t)p.out32 & 15) == 0 && ((uintptr_t)p.out_split & 7) == 0;

@@ -233,6 +233,7 @@ struct AttnF32P {
                                   // over ragged segments, e.g. Qwen2.5-VL's windows); Lq is then the longest segment
   float scale;
   bool out_vec;                   // the outputs may be stored four elements at a time (set by the launch)
+  int flags;                      // 1: nothing is loaded (the waits run out)
 };
 int attention_f32_tc(AttnF32P p, int n_seg, cudaStream_t st);
 int attention(const void* q, long q_ts, long q_hs, const void* k, long k_ts, long k_hs,

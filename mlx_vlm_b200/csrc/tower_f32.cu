@@ -362,7 +362,7 @@ int f32_gather_rows(const float* in, long ld_in, const int* idx, int n_idx, int 
 int attention_f32(const float* q, long q_ts, long q_hs, const float* k, long k_ts, long k_hs, const float* v,
                   long v_ts, long v_hs, float* out32, long o_ts, void* out_split, long os_ts, int n_pad,
                   int n_heads, int n_kv, int hd, int Lq, int S, int n_seg, long q_seg, long k_seg,
-                  const unsigned char* key_mask, float scale, cudaStream_t st, const int* cu = nullptr) {
+                  const unsigned char* key_mask, float scale, cudaStream_t st, const int* cu = nullptr, int flags = 0) {
   B200_REQUIRE(q && k && v && (out32 || out_split) && Lq > 0 && S > 0 && n_seg > 0 && n_heads % n_kv == 0,
                "attention_f32: bad arguments");
   B200_REQUIRE(!cu || !key_mask, "attention_f32: ragged segments take no key mask");
@@ -375,6 +375,7 @@ int attention_f32(const float* q, long q_ts, long q_hs, const float* k, long k_t
   p.n_heads = n_heads; p.n_kv = n_kv; p.Lq = Lq; p.S = S; p.q_seg = q_seg; p.k_seg = k_seg; p.key_mask = key_mask;
   p.scale = scale;
   p.cu = cu;
+  p.flags = flags;
   p.hd = hd;
   B200_REQUIRE((hd % 4) == 0 && hd <= 96, "attention_f32: head_dim %d (multiple of 4, <= 96)", hd);
   return attention_f32_tc(p, n_seg, st);
@@ -416,6 +417,12 @@ int b200_attention_f32(const float* q, long q_ts, long q_hs, const float* k, lon
                        const unsigned char* key_mask, float scale, void* st) {
   return attention_f32(q, q_ts, q_hs, k, k_ts, k_hs, v, v_ts, v_hs, out32, o_ts, out_split, os_ts, n_pad, n_heads,
                        n_kv, hd, Lq, S, n_seg, q_seg, k_seg, key_mask, scale, (cudaStream_t)st);
+}
+int b200_attention_f32_debug(const float* q, long q_ts, long q_hs, const float* k, long k_ts, long k_hs, const float* v,
+                             long v_ts, long v_hs, float* out32, long o_ts, int n_heads, int n_kv, int hd, int Lq, int S,
+                             float scale, int flags, void* st) {
+  return attention_f32(q, q_ts, q_hs, k, k_ts, k_hs, v, v_ts, v_hs, out32, o_ts, nullptr, 0, 0, n_heads, n_kv, hd, Lq, S, 1, 0,
+                       0, nullptr, scale, (cudaStream_t)st, nullptr, flags);
 }
 int b200_attention_f32_varlen(const float* q, long q_ts, long q_hs, const float* k, long k_ts, long k_hs, const float* v,
                               long v_ts, long v_hs, float* out32, long o_ts, void* out_split, long os_ts, int n_pad,

@@ -3,6 +3,10 @@ groups of 16 keys, head sizes padded to 32 / 64 / 80 / 96.
 
 Bound: a score is a sum of at most 96 products with 24 bits each (relative error about 1e-7 of |q||k|, |scores| <= ~6 here, so
 6e-7 in the exponent), the exponential 2^-22, sums and outputs 2^-24 a step: 2e-6 of the output's size."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -119,3 +123,40 @@ def test_numbers_that_bf16_parts_do_not_hold(lib, kind, hd, Lq, S):
     err = ((got - want).masked_fill(odd, 0.0).norm(dim=0) / want.masked_fill(odd, 0.0).norm(dim=0).clamp_min(1e-300)).max().item()
     print(kind, hd, err)
     assert bool(torch.isfinite(got[~odd]).all()) and err <= 2 * BOUND
+
+
+_CHILD = """
+import sys, ctypes as C, torch
+sys.path.insert(0, {root!r})
+from mlx_vlm_b200 import _native as N
+lib = N.lib()
+def state():
+    v = C.c_int(-1)
+    N.check(lib.b200_wait_error(C.byref(v)))
+    return v.value
+T, S, hd = {T}, {S}, 64
+g = torch.Generator(device="cuda").manual_seed(1)
+q, k, v = (torch.randn(n, hd, device="cuda", generator=g) for n in (T, S, S))
+out = torch.zeros(T, hd, device="cuda")
+def run(flags):
+    out.zero_()
+    torch.cuda.synchronize()
+    N.check(lib.b200_attention_f32_debug(q.data_ptr(), hd, hd, k.data_ptr(), hd, hd, v.data_ptr(), hd, hd, out.data_ptr(), hd, 1, 1, hd,
+                                         T, S, 1.0, flags, 0))
+    torch.cuda.synchronize()
+    return out.clone()
+want = torch.softmax(q.double() @ k.double().T, -1) @ v.double()
+a = run(0)
+assert float((a - want).norm() / want.norm()) < 1e-5 and state() == 0
+b = run(1)                            # nothing is loaded: the waits run out after a second
+assert bool(torch.isnan(b).all()) and state() == 7, (b, state())
+assert torch.equal(run(0), a) and state() == 7
+"""
+
+
+@pytest.mark.parametrize("T,S", [(5, 7), (300, 700)])
+def test_a_wait_that_runs_out_is_told(T, S):
+    """in a process of its own: NaN, the word that the host reads, and the next launch as if nothing had been"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _CHILD.format(root=root, T=T, S=S)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
