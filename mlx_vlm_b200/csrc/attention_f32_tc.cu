@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
 template <int HDP>
 int tc_launch(const AttnF32P& p, dim3 grid, cudaStream_t st) {
   static unsigned long long attr_mask = 0ull;
-  if (first_use_on_device(&attr_mask))
+  if (FirstUse first{&attr_mask})
     B200_CUDA(cudaFuncSetAttribute(attention_f32_tc_kernel<HDP>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem<HDP>()));
   attention_f32_tc_kernel<HDP><<<grid, TC_THREADS, tc_smem<HDP>(), st>>>(p);
   B200_CHECK_LAUNCH();

@@ -575,7 +575,7 @@ int attention_fa(const void* q, long q_ts, long q_hs, const void* k, long k_ts, 
   const auto kern = v_transposed ? attention_fa_kernel<true> : attention_fa_kernel<false>;
   static unsigned long long set_mask[2] = {0ull, 0ull};
   const size_t smem = 14 * FA_BLK + 1024;
-  if (first_use_on_device(&set_mask[v_transposed]))
+  if (FirstUse first{&set_mask[v_transposed]})
     B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   FaParams p;
   p.out = (bf16*)out; p.o_ts = o_ts; p.n_heads = n_heads; p.n_kv = n_kv; p.hd = hd; p.hdp = hdp;

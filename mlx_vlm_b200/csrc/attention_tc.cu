@@ -383,7 +383,7 @@ int attention_tc(const void* q, long q_ts, long q_hs, const void* k, long k_ts, 
                  int hd, int Lq, int S, int causal, float scale, cudaStream_t st) {
   static unsigned long long set_mask = 0ull;
   const size_t smem = 8 * KBLK + 1024;
-  if (first_use_on_device(&set_mask)) {
+  if (FirstUse first{&set_mask}) {
     B200_CUDA(cudaFuncSetAttribute(attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)smem));
   }

@@ -133,15 +133,22 @@ struct WaitWord {
 };
 int wait_error(int* out);
 
-// per-DEVICE one-time setup (cudaFuncSetAttribute is per device): true the first time the current device asks
-inline bool first_use_on_device(unsigned long long* mask) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return true;
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (*mask & bit) return false;
-  *mask |= bit;
-  return true;
-}
+// per-DEVICE one-time setup (cudaFuncSetAttribute is per device): `if (FirstUse first{&mask}) B200_CUDA(...)` runs until it has
+// succeeded once on the current device.  The device is marked when the setup is done, not before: a second thread that comes
+// meanwhile does it again instead of launching without it.
+struct FirstUse {
+  unsigned long long *mask, bit = 0ull;
+  explicit FirstUse(unsigned long long* m) : mask(m) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
+    if (!(__atomic_load_n(mask, __ATOMIC_ACQUIRE) >> (dev & 63) & 1ull)) bit = 1ull << (dev & 63);
+  }
+  ~FirstUse() {
+    if (bit && cudaPeekAtLastError() == cudaSuccess) __atomic_fetch_or(mask, bit, __ATOMIC_RELEASE);
+  }
+  FirstUse(const FirstUse&) = delete;
+  explicit operator bool() const { return bit != 0ull; }
+};
 
 // ---- waits that end ----------------------------------------------------------------
 // Waits for a phase of an mbarrier of this CTA; false, and *failed (shared memory, zeroed before the first wait) set, after

@@ -992,7 +992,7 @@ int batch_decoder_begin(void** handle, const BdModel& m, int B, const int* tok, 
     }
     *handle = d;
     static unsigned long long attr_mask = 0ull;
-    if (first_use_on_device(&attr_mask)) {
+    if (FirstUse first{&attr_mask}) {
       B200_CUDA(cudaFuncSetAttribute(bd_attn_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
       B200_CUDA(cudaFuncSetAttribute(bd_attn_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     }

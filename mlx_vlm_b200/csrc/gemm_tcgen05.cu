@@ -363,7 +363,7 @@ template <int BN>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
                        cudaStream_t st) {
   static unsigned long long attr_mask = 0ull;
-  if (first_use_on_device(&attr_mask)) {
+  if (FirstUse first{&attr_mask}) {
     B200_CUDA(cudaFuncSetAttribute(gemm_tn_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    GemmSmem<BN>::TOTAL));
   }

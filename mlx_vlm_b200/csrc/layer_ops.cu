@@ -1425,12 +1425,12 @@ int b200_lm_latent_attention(const float* qa, long ldqa, const void* cache, int 
   B200_REQUIRE(smem <= 200 * 1024, "lm_latent_attention: rows of %d numbers do not fit shared memory", Dl);
   dim3 grid(T, cdiv(H, nw), n_split);
   if (cache_bf16) {
-    if (first_use_on_device(&g_attn_attr_bf16))
+    if (FirstUse first{&g_attn_attr_bf16})
       B200_CUDA(cudaFuncSetAttribute(latent_attention_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     LatAttnP<bf16> p{qa, ldqa, (const bf16*)cache, slot_stride, tok_stride, slot, pos, out, ldo, H, Dl, kv_rank, scale, round_q, part, n_split, vec8, window};
     latent_attention_kernel<bf16><<<grid, nw * 32, smem, (cudaStream_t)st>>>(p);
   } else {
-    if (first_use_on_device(&g_attn_attr_f32))
+    if (FirstUse first{&g_attn_attr_f32})
       B200_CUDA(cudaFuncSetAttribute(latent_attention_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     LatAttnP<float> p{qa, ldqa, (const float*)cache, slot_stride, tok_stride, slot, pos, out, ldo, H, Dl, kv_rank, scale, round_q, part, n_split, 0, window};
     latent_attention_kernel<float><<<grid, nw * 32, smem, (cudaStream_t)st>>>(p);

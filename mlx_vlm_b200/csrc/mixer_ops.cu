@@ -1507,7 +1507,7 @@ int delta_chunks(const DeltaChunkP& p, int n_seq, int max_rows, cudaStream_t cs)
   static unsigned long long attr = 0;
   constexpr int TILE = (3 * DC_C + 1) * P * LS_R + 2 * DC_C * DC_C, cols = DC_THREADS / P;
   auto smem = [](int nc) { return (size_t)(2 * TILE + cols * nc * 4 * DC_C) * sizeof(float); };
-  if (first_use_on_device(&attr)) {
+  if (FirstUse first{&attr}) {
     B200_CUDA(cudaFuncSetAttribute(delta_chunk_kernel<P, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem(1)));
     B200_CUDA(cudaFuncSetAttribute(delta_chunk_kernel<P, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem(2)));
     B200_CUDA(cudaFuncSetAttribute(delta_chunk_kernel<P, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem(4)));
@@ -1620,13 +1620,13 @@ int b200_lm_sink_attention(const float* q, long ldq, const void* cache, int cach
   B200_REQUIRE(smem <= 200 * 1024, "lm_sink_attention: rows of %d + %d numbers do not fit shared memory", dim, vdim);
   dim3 grid(T, G * cdiv(rep, nw), n_split);
   if (cache_bf16) {
-    if (first_use_on_device(&g_sink_attr_bf16))
+    if (FirstUse first{&g_sink_attr_bf16})
       B200_CUDA(cudaFuncSetAttribute(sink_attention_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     const int vec = dim % 8 == 0 && vdim % 8 == 0 && tok_stride % 8 == 0 && slot_stride % 8 == 0 && ((uintptr_t)cache & 15) == 0;
     SinkAttnP<bf16> p{q, ldq, (const bf16*)cache, slot_stride, tok_stride, slot, pos, out, ldo, (const bf16*)sink, H, G, dim, vdim, scale, chunk, window, part, n_split, vec, bias_exp, unit_sink, softcap};
     sink_attention_kernel<bf16><<<grid, nw * 32, smem, (cudaStream_t)st>>>(p);
   } else {
-    if (first_use_on_device(&g_sink_attr_f32))
+    if (FirstUse first{&g_sink_attr_f32})
       B200_CUDA(cudaFuncSetAttribute(sink_attention_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     const int vec = dim % 4 == 0 && vdim % 4 == 0 && tok_stride % 4 == 0 && slot_stride % 4 == 0 && ((uintptr_t)cache & 15) == 0;
     SinkAttnP<float> p{q, ldq, (const float*)cache, slot_stride, tok_stride, slot, pos, out, ldo, (const bf16*)sink, H, G, dim, vdim, scale, chunk, window, part, n_split, vec, bias_exp, unit_sink, softcap};

@@ -622,7 +622,7 @@ int b200_lm_matrix_memory(const float* q, long ldq, const float* k, long ldk, co
   if (!scratch) {                    // few rows
     const size_t smem = (size_t)(2 * dim + 4 + (MW_THREADS / 32 + 1) * ((vdim + 3) / 4 * 4)) * sizeof(float);
     B200_REQUIRE(smem <= 200 * 1024, "lm_matrix_memory: heads of %d x %d do not fit shared memory", dim, vdim);
-    if (first_use_on_device(&g_walk_attr)) {
+    if (FirstUse first{&g_walk_attr}) {
       B200_CUDA(cudaFuncSetAttribute(memory_walk_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
       B200_CUDA(cudaFuncSetAttribute(memory_walk_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     }
@@ -645,7 +645,7 @@ int b200_lm_matrix_memory(const float* q, long ldq, const float* k, long ldk, co
   p.mstart = p.m0 + chunks * H;
   const size_t smem = sizeof(MemTile) + (size_t)MC * MC_LD * 4 + (size_t)MC * vdim * 4;
   B200_REQUIRE(smem <= 200 * 1024, "lm_matrix_memory: values of %d numbers do not fit shared memory", vdim);
-  if (first_use_on_device(&g_mem_attr)) {
+  if (FirstUse first{&g_mem_attr}) {
     B200_CUDA(cudaFuncSetAttribute(memory_out_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     B200_CUDA(cudaFuncSetAttribute(memory_out_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   }

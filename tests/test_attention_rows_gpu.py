@@ -111,3 +111,40 @@ def test_a_wait_that_runs_out_is_told(T, S):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", _CHILD.format(root=root, T=T, S=S)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+_CHILD_THREADS = """
+import sys, threading, torch
+sys.path.insert(0, {root!r})
+from mlx_vlm_b200 import _native as N
+lib = N.lib()
+n, hd = 200, 64
+x = torch.randn(3, n, hd, device="cuda").to(torch.bfloat16)
+f = torch.randn(3, n, hd, device="cuda")
+streams = [torch.cuda.Stream() for _ in range(16)]
+outs = [(torch.zeros(n, hd, device="cuda", dtype=torch.bfloat16), torch.zeros(n, hd, device="cuda")) for _ in streams]
+torch.cuda.synchronize()
+gate, bad = threading.Barrier(len(streams)), []
+def go(s, o):
+    with torch.cuda.stream(s): torch.zeros(1, device="cuda")      # (the thread has a context)
+    s.synchronize()
+    gate.wait()
+    a = lib.b200_attention_fa_rows(x[0].data_ptr(), hd, hd, x[1].data_ptr(), hd, hd, x[2].data_ptr(), hd, hd, o[0].data_ptr(), hd, 1, 1, hd,
+                                   n, n, 0, n, n, 0, 0, 0, s.cuda_stream)
+    b = lib.b200_attention_f32(f[0].data_ptr(), hd, hd, f[1].data_ptr(), hd, hd, f[2].data_ptr(), hd, hd, o[1].data_ptr(), hd, 0, 0, 0, 1,
+                               1, hd, n, n, 1, n, n, 0, 0.1, s.cuda_stream)
+    if a or b: bad.append((a, b, lib.b200_last_error()))
+ts = [threading.Thread(target=go, args=a) for a in zip(streams, outs)]
+[t.start() for t in ts]
+[t.join() for t in ts]
+torch.cuda.synchronize()
+assert not bad, bad
+assert all(torch.equal(o[i], outs[0][i]) and bool(o[i].any()) for o in outs for i in (0, 1))
+"""
+
+
+def test_first_calls_of_many_threads():
+    """none of the threads launches before the kernel's shared memory is allowed for"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _CHILD_THREADS.format(root=root)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
