@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """bench.py — headline benchmark of the B200-native generate path.
 
-Workload ("C2"): Qwen2-VL-2B bf16, 1 synthetic image
+Workload "C2": Qwen2-VL-2B bf16, 1 synthetic image
 336x336 (144 merged image tokens), 128 text-side prompt tokens (T = 272),
 512 generated tokens, batch 1, greedy, EOS ignored; seeded random-init weights
 (no checkpoints offline).  One "step" = one whole request: ViT -> merge ->
@@ -29,11 +29,11 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 N_TEXT, N_OUT, IMG_HW = 128, 512, (336, 336)
-W_BYTES_2B = 3_087_428_608      # SURVEY §8(d): decode weight bytes / token (bf16, tied head)
+W_BYTES_2B = 3_087_428_608      # decode weight bytes / token (bf16, tied head)
 KV_BYTES_PER_POS = 28_672       # 2 (k,v) * 2 kv heads * 128 * 2 B * 28 layers
 
 
-# ViT + merge + LM prefill FLOPs of one C2 request (SURVEY §8d: 2*M*N*K per GEMM, 4*N^2*D attention)
+# ViT + merge + LM prefill FLOPs of one C2 request (2*M*N*K per GEMM, 4*N^2*D attention)
 VIT_GFLOP, PREFILL_GFLOP_T272 = 790.7, 720.0
 
 
@@ -58,7 +58,7 @@ def _tensor_peak():
 
 def _ncu_traffic():
     """dram bytes (read + write) of ONE decode-kernel launch from the committed ncu capture
-    (profiles/decode_traffic.json: written by tools/ncu_traffic.py from an `ncu --set full` run)."""
+    (profiles/decode_traffic.json, if there is one)."""
     p = os.path.join(ROOT, "profiles", "decode_traffic.json")
     if os.path.exists(p):
         with open(p) as f:
@@ -217,7 +217,7 @@ def cpu_reference_run(W, n_decode, threads=None):
             "cores": torch.get_num_threads()}
 
 
-W_BYTES_7B = 2 * 7_070_619_136          # SURVEY §8(d): Qwen2-VL-7B LM weights (untied head), bf16
+W_BYTES_7B = 2 * 7_070_619_136          # Qwen2-VL-7B LM weights (untied head), bf16
 KV_BYTES_PER_POS_7B = 57_344            # 2 * 4 kv heads * 128 * 2 B * 28 layers
 
 
@@ -267,7 +267,7 @@ def lockstep_2b(world, rank, dev, args, model, processor, ids, pvd, grid):
 
 
 def c5_leg(world, rank, dev, args):
-    """Qwen2-VL-7B, `rows` concurrent image+prompt requests PER GPU (64 over 8 GPUs),
+    """"C5": Qwen2-VL-7B, `rows` concurrent image+prompt requests PER GPU (64 over 8 GPUs),
     routed by parallel.generate_sharded (request i -> rank i mod N), each replica running its own
     lock-step BatchGenerator; 336x336 image, 128 text tokens in, 512 out, greedy, EOS ignored.
     Timed: max over ranks of (insert -> last token), CUDA-synchronised wall clock (host admission and
@@ -351,7 +351,7 @@ def c5_leg(world, rank, dev, args):
 
 
 def c3_leg(dev, args):
-    """LLaVA-1.5-7B (CLIP-ViT-L/14-336 + Llama-7B geometry) bf16, batch = 8 images,
+    """"C3": LLaVA-1.5-7B (CLIP-ViT-L/14-336 + Llama-7B geometry) bf16, batch = 8 images,
     prefill only: pinned-host pixel_values -> CLIP tower (23 of 24 blocks: feature layer -2) -> projector
     -> merge -> LM prefill of the 8 requests (576 image + 32 text tokens each) incl. the first token.
     The tower is fp32-accurate like the reference's (split-operand tcgen05 GEMMs: every Linear runs as
@@ -438,7 +438,7 @@ def c3_leg(dev, args):
 
 
 def c4_leg(dev, args):
-    """Idefics2-8B (SigLIP-SO400M + perceiver + Mistral-7B geometry) bf16, one request with
+    """"C4": Idefics2-8B (SigLIP-SO400M + perceiver + Mistral-7B geometry) bf16, one request with
     4 images of 448x448 (4 x 1024 patches -> 4 x 64 latents = 256 image tokens) interleaved with 256 text
     tokens (T = 512), 256 greedy tokens out."""
     import numpy as np

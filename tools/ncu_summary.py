@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """One-screen summary of an `ncu -i X.ncu-rep --page raw --csv` export (first profiled kernel):
 duration, DRAM bytes / throughput, tensor-pipe and TMEM activity, occupancy, launch geometry.
-usage: python tools/ncu_summary.py gpurun_out/prof/*.raw.csv > profiles/r2_ncu_full_summary.txt"""
+usage: python tools/ncu_summary.py *.raw.csv"""
 import csv
 import sys
 

@@ -1,4 +1,4 @@
-"""CPU study for the round-2 LLaVA / Idefics2 vision tower (DESIGN.md round-2 plan, item 4).
+"""CPU study for the LLaVA / Idefics2 vision tower.
 
 The reference computes the CLIP tower in fp32 (float32 pixel_values x bf16-valued weights) and rounds
 the projected features to bf16 only at the merge.  Which tensor-core formulation reproduces THOSE
