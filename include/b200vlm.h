@@ -4,7 +4,7 @@
  * The reference (Blaizzy/mlx-vlm) has NO FFI: its hot path is Python calling the
  * third-party `mlx` array library.  This header is the boundary a maintainer
  * would bind instead of `mlx`: every entry point names the reference call site
- * (file:line under /root/reference/mlx_vlm) whose arithmetic it replaces.
+ * (file:line of its mlx_vlm package) whose arithmetic it replaces.
  *
  * Conventions
  *   - plain pointers + sizes only; all data pointers are DEVICE pointers unless
@@ -182,7 +182,7 @@ typedef struct {
 int b200_engine_create(const b200_qwen2vl_config* cfg, int device, b200_engine** out);
 int b200_engine_destroy(b200_engine* e);
 
-/* Weight registration by name (packed names, see DESIGN.md §layout):
+/* Weight registration by name (packed names):
  *   v.patch_embed.w | v.blk.<i>.{ln1.w,ln1.b,ln2.w,ln2.b,qkv.w,qkv.b,proj.w,proj.b,
  *   fc1.w,fc1.b,fc2.w,fc2.b} | v.merger.{ln.w,ln.b,fc1.w,fc1.b,fc2.w,fc2.b} |
  *   lm.embed | lm.head (untied only) | lm.norm | lm.<i>.{ln1,ln2,wqkv,bqkv,wo,wgu,wd} */

@@ -6,7 +6,7 @@
 // p is rounded AFTER normalisation with the final row max / sum, so the kernel is two-pass over
 // the keys and the second pass recomputes the score tile on the tensor cores.
 //
-// attention_tc.cu (round 1) staged every tile with the compute threads and ran
+// attention_tc.cu stages every tile with the compute threads and runs
 // load -> sync -> MMA -> wait -> softmax strictly in sequence (61 us per ViT layer, 2 % of the
 // tensor peak).  Here, per CTA = 128 query rows of one head:
 //   warp 0      TMA producer: Q once, K tiles for both passes, V tiles for pass 2 (3-D tensor

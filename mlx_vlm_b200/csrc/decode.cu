@@ -802,7 +802,7 @@ __global__ void k_set_state(DecState* st, int tok, int ctx, int pos, int use_for
 // host-side launchers
 // ---------------------------------------------------------------------------
 static int g_sm_count = 148;
-static bool g_pdl = false;  // measured on B200: no gain for this kernel mix (DESIGN.md)
+static bool g_pdl = false;  // measured on B200: no gain for this kernel mix
 void decode_set_sm_count(int n) { g_sm_count = n > 0 ? n : 148; }
 void decode_set_pdl(bool on) { g_pdl = on; }
 

@@ -1,4 +1,4 @@
-// Lock-step batched decode (continuous batching, SURVEY §8 a15 / config C5): B <= 16 independent
+// Lock-step batched decode (continuous batching): B <= 16 independent
 // requests advance one token per step and share ONE stream of the weights.
 //
 // The reference batches rows by left-padding them to a common length inside a BatchKVCache

@@ -116,7 +116,7 @@ __device__ __forceinline__ void consume_phase(const MegaP& p, const MegaPhase& g
   // ---- prologue: the 256 consumer threads load / RMS-normalise the activation vector ONCE
   // per CTA into shared memory (one global round trip, two block barriers); each warp then
   // takes its register slice from there.  (Per-warp redundant normalisation cost 2.4 us of
-  // every NORM phase in the round-1 timeline; this costs 0.8-1.0 us.)
+  // every NORM phase in an earlier timeline; this costs 0.8-1.0 us.)
   uint4* xs = reinterpret_cast<uint4*>(xs_raw);
   {
     float ss = 0.f;
@@ -408,8 +408,8 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_mega(const MegaP p) {
         // the qkv/attention/o_proj chain is latency-bound (~20 us with ~11 MB of weights):
         // use it to pull this CTA's share of the layer's MLP weights (82 MB chip-wide,
         // fits the 126 MB L2) into L2, so the ring later refills at L2 speed.
-        // (measured, round 1: no gain — gate/up is consumer-bound at 8 warps — and a
-        // straggler CTA in the down phase; kept behind a switch for round 2)
+        // (measured: no gain — gate/up is consumer-bound at 8 warps — and a
+        // straggler CTA in the down phase; kept behind a switch)
         if (p.l2_prefetch == 1) {
           l2_prefetch_phase<PH_GATEUP>(p.ph[PH_GATEUP], lw.wgu, lw.wgu + (long)d.inter * d.hidden);
           l2_prefetch_phase<PH_DRES>(p.ph[PH_DRES], lw.wd, nullptr);
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_mega(const MegaP p) {
     // B200_L2_PREFETCH >= 2: the CONSUMER side, entering the latency-bound qkv -> attention -> o_proj chain of this
     // layer (~16 us during which HBM is idle once the ring is full), asks the L2 for this CTA's share of the layer's
     // MLP weights; the first `l2_skip` gate/up tiles are already on their way into the ring.  (The producer-issued
-    // variant of round 1 fired while the PREVIOUS layer's MLP was still streaming: no gain.)
+    // earlier variant fired while the PREVIOUS layer's MLP was still streaming: no gain.)
     if (p.l2_prefetch >= 2 && threadIdx.x == 0) {
       l2_prefetch_phase<PH_GATEUP>(p.ph[PH_GATEUP], lw.wgu, lw.wgu + (long)d.inter * d.hidden, p.l2_skip);
       if (p.l2_prefetch >= 3) l2_prefetch_phase<PH_DRES>(p.ph[PH_DRES], lw.wd, nullptr);
@@ -548,7 +548,8 @@ int mega_fill(MegaP& p, int sm_count) {
   // row, and the block barrier of their sum comes once per 28 / 32 KB, 1.07 us, which is less than the memory delivers
   // (4.5 TB/s).  Measured at 4,096 x 14,336: gate and up 51.6 -> 35.9 us a layer (6.5 TB/s), down 23.2 -> 18.1; a step of
   // four layers and a head of 8,192 rows behind 6000 keys: 599 -> 515 us.  Wider stages need at least three of them beside the
-  // attention's scores.  (At 1,536 four rows fit as it is, and 48 KB holds eight of them.)
+  // attention's scores, which they have up to a cache of 7,168 positions at 4,096 wide and 19,456 at 3,584 (heads of 128); beyond, the
+  // phases take the 48 KB times again.  (At 1,536 four rows fit as it is, and 48 KB holds eight of them.)
   const int wide = 4 * d.hidden * 4;
   if (wide > MEGA_STAGE && wide <= 64 * 1024 && (rc = mega_ring(p, wide, 8, 14, &ns)) != B200_OK) return rc;
   if (ns < 3) {

@@ -78,7 +78,7 @@ struct b200_engine {
   KvRef* kvref = nullptr;       // device: where the bound pool row lives (read by the captured prefill)
   KvRef* kvref_host = nullptr;  // pinned staging
   cudaEvent_t kvref_ev = nullptr;
-  bool v2 = true;               // weight-major GEMMs + pipelined attention (B200_PREFILL_V1=1: round-1 path)
+  bool v2 = true;               // weight-major GEMMs + pipelined attention (B200_PREFILL_V1=1: the earlier path)
   int log_cap = 1 << 16;
   // host mirrors of the decode state
   int ctx_host = 0, pos_host = 0;
@@ -344,7 +344,7 @@ static int kernels_per_step(const b200_engine* e) {
 
 
 // ---------------------------------------------------------------------------------------------
-// round-2 prefill / vision path: weight-major GEMMs (gemm_wt.cu), split-K partials finished by
+// prefill / vision path: weight-major GEMMs (gemm_wt.cu), split-K partials finished by
 // finish_rows (bias + residual + the NEXT norm fused), pipelined attention (attention_fa.cu)
 // ---------------------------------------------------------------------------------------------
 static long align256(long x) { return (x + 255) & ~255L; }
@@ -434,7 +434,6 @@ static int upload_loc(b200_engine* e, const std::vector<int>& loc, cudaStream_t 
   return B200_OK;
 }
 
-// rot_pos_emb ids (vision.py:219-249), host side, merge-group-major order
 // the attention segments behind the ids: (first token, tokens, first key, keys) of every frame (vision.py:270-281)
 static void append_frames(const int* grid, int n_img, std::vector<int>* out, int* n_frames, int* longest) {
   int off = 0;
@@ -449,6 +448,7 @@ static void append_frames(const int* grid, int n_img, std::vector<int>* out, int
   }
 }
 
+// rot_pos_emb ids (vision.py:219-249), host side, merge-group-major order
 static void build_pos_hw(const int* grid, int n_img, int ms, std::vector<int>* out) {
   out->clear();
   for (int i = 0; i < n_img; ++i) {
@@ -671,7 +671,7 @@ static int prefill_layers_v2_body(b200_engine* e, const int* pos3, int T, int ct
   bf16* xn = (bf16*)p; p += align256((long)T * H * 2);
   bf16* qkv = (bf16*)p; p += align256((long)T * QKV * 2);
   bf16* att = (bf16*)p; p += align256((long)T * QH * 2);
-  p += align256((long)T * 2 * I * 2);  // (gate/up buffer of the round-1 path)
+  p += align256((long)T * 2 * I * 2);  // (gate/up buffer of the earlier path)
   bf16* act = (bf16*)p; p += align256((long)T * I * 2);
   int rc;
   if ((rc = rms_norm(h, e->layers[0].ln1, xn, T, (int)H, c.rms_eps, s))) return rc;
@@ -759,7 +759,7 @@ int b200_engine_create(const b200_qwen2vl_config* cfg, int device, b200_engine**
   e->sm_count = sm;
   decode_set_sm_count(sm);
   if (const char* v = getenv("B200_MEGA_FLOW")) e->flow = atoi(v) != 0;  // tuning aid (A/B)
-  if (const char* v = getenv("B200_PREFILL_V1")) e->v2 = atoi(v) == 0;    // A/B: round-1 prefill kernels
+  if (const char* v = getenv("B200_PREFILL_V1")) e->v2 = atoi(v) == 0;    // A/B: the earlier prefill kernels
   if (const char* v = getenv("B200_SEQ_GRAPH")) e->seq_graphs = atoi(v) != 0;
   const auto& c = e->cfg;
   B200_CUDA(cudaMalloc(&e->st, sizeof(DecState)));

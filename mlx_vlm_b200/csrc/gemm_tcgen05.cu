@@ -206,7 +206,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     // ALL 8 warps take part once their main-loop role is done (the producer / MMA threads have
     // issued everything by now): warp w reads TMEM lane quarter w % 4 and column half w / 4, so
     // the non-overlapped tail of a CTA (bias, GELU, residual, 16-byte stores) is half as long
-    // (ncu, round 1: a 128x128 tile's epilogue is 3-5 us of a 13-24 us CTA).
+    // (ncu: a 128x128 tile's epilogue is 3-5 us of a 13-24 us CTA).
     const int q = warp & 3;  // TMEM lane quarter == warp % 4
     const int chalf = warp >> 2;
     mbar_wait(tmem_full, 0);

@@ -331,7 +331,7 @@ __device__ __forceinline__ void wt_store_tile(const WtParams& p, uint8_t* stg, u
 }
 
 // TOWER = false: the bf16 paths (B200_WT_BF16 / PARTIAL / SWIGLU); TOWER = true: the fp32-accurate paths
-// (B200_WT_F32 / SPLIT).  Two instantiations keep each one's code small (tools/wt_ab_probe.py A/B-times builds).
+// (B200_WT_F32 / SPLIT).  Two instantiations keep each one's code small.
 template <bool TOWER>
 __global__ void __launch_bounds__(256, 2)
 gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
@@ -949,7 +949,7 @@ static size_t wp_staging(int mode) {   // the epilogue's staging tile: WT_EPI_TO
   return (size_t)WT_EPI_TOK * WT_ROWS * (mode == B200_WT_BF16 || mode == B200_WT_SWIGLU ? 2 : 4);
 }
 
-// Tile / pipeline configuration for (T, row blocks, K): a small cost model calibrated on the round-2
+// Tile / pipeline configuration for (T, row blocks, K): a small cost model calibrated on a
 // sweep (profiles/r2_gemm_wt_sweep.txt, B200):
 //   * a CTA costs ~4.5 us of fixed latency (launch, barrier/TMEM set-up, first TMA round trip,
 //     epilogue) + per k-block max(MMA time, shared-memory fill time at ~130 GB/s per SM);
@@ -1150,8 +1150,8 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
 // Measured configuration choice ("measure, don't guess"): the first call for a problem class
 // (tokens rounded up to 64, N, K, mode) times a short list of candidate configurations on the
 // caller's stream with the call's own operands (CUDA events, one warm-up + two timed launches
-// each) and caches the winner; later calls cost one hash lookup.  Candidates follow what the
-// round-2 sweep showed matters: token tile {96,128,144,192,256}, one CTA per SM with 2 k-blocks
+// each) and caches the winner; later calls cost one hash lookup.  Candidates follow what that
+// sweep showed matters: token tile {96,128,144,192,256}, one CTA per SM with 2 k-blocks
 // per stage vs two CTAs per SM with 1, and split-K to one or two waves.  The list is ordered and
 // the first candidate within 3 % of the best wins, so the choice is stable run to run.
 // B200_WT_TUNE=0 uses the cost model (gemm_wt_auto) instead.

@@ -478,7 +478,7 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
   // (8-byte accesses are single-copy atomic; the epoch changes every attention phase), and
   // ONE warp (lane = u*AG + g) polls the 32 pairs directly.  This replaces
   // store + atomic arrive + counter poll + stats load (3 dependent L2 round trips) by
-  // store + poll (round 1: 750 -> 897 tok/s came from shortening this chain).
+  // store + poll (750 -> 897 tok/s came from shortening this chain).
   {
     static_assert(ATT_UN * MEGA_ATT_G == 32, "one lane per (unit, head)");
     unsigned long long* gw = reinterpret_cast<unsigned long long*>(p.att_stats) + (long)grp * ATT_UN * AG * 2;

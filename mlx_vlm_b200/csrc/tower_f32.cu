@@ -24,12 +24,6 @@ __device__ __forceinline__ void split_store4(bf16* dst, int n_pad, float a, floa
   *reinterpret_cast<uint2*>(dst + n_pad) = make_uint2(pack2(a - h0, b - h1), pack2(c - h2, d - h3));
 }
 
-__device__ __forceinline__ void split_store2(bf16* dst, int n_pad, float a, float b) {
-  const float h0 = rbf(a), h1 = rbf(b);
-  *reinterpret_cast<uint32_t*>(dst) = pack2(h0, h1);
-  *reinterpret_cast<uint32_t*>(dst + n_pad) = pack2(a - h0, b - h1);
-}
-
 __device__ __forceinline__ float t_block_sum(float v, float* red) {
   v = warp_sum(v);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -381,7 +381,7 @@ class RunCache(_BaseCache):
 def make_prompt_cache(model: Any, max_kv_size: Optional[int] = None) -> List[Any]:
     """cache.py:45-70: defer to model.make_cache() when present."""
     if max_kv_size is not None:
-        raise NotImplementedError("RotatingKVCache (max_kv_size) is out of scope (SURVEY §2.1 #6)")
+        raise NotImplementedError("RotatingKVCache (max_kv_size) is out of scope")
     if hasattr(model, "make_cache"):
         return model.make_cache()
     return [KVCache() for _ in range(len(model.layers))]

@@ -1,4 +1,4 @@
-"""LLaVA-Next (LLaVA-1.6) `Model` — a sibling of LLaVA-1.5 that shares its kernels (SURVEY §8 f4; reference
+"""LLaVA-Next (LLaVA-1.6) `Model` — a sibling of LLaVA-1.5 that shares its kernels (reference
 mlx_vlm/models/llava_next/llava_next.py:32-144).  What differs from LLaVA-1.5, all of it host logic around the same
 device ops:
   * `pixel_values` is (1, N, C, H, W): the N crops of ONE image (base view + any-resolution tiles); the tower and the

@@ -1,4 +1,4 @@
-"""Multi-GPU plumbing of the generate path (SURVEY §8e): requests are independent
+"""Multi-GPU plumbing of the generate path: requests are independent
 units, so the design is one full model replica per GPU (one process per GPU,
 `torch.distributed`), a single weight broadcast from rank 0 at start-up (NCCL over
 NVLink / NVSwitch on the GPU box, gloo in the CPU tests), a host-side request router,

@@ -4,8 +4,8 @@ and hand over a request; the loop admits waiting requests between decode steps (
 runs the vision tower for a new request on the GPU thread (`_gpu_embed`, generation.py:1636-1675),
 streams every generated token back through the request's own queue, honours cancellation and a
 `max_num_seqs` admission cap (back-pressure: the rest stay queued), and reports an engine error to every
-request it affects.  The HTTP / OpenAI front end is outside the hot-path scope (the
-loop is the part that touches the path); `ResponseGenerator.generate()` is what such a front end calls.
+request it affects.  The HTTP / OpenAI front end is outside the hot-path scope (the loop is the part
+that touches the path); `ResponseGenerator.generate()` is what such a front end calls.
 
 Differences from the reference, by design: no speculative / diffusion / APC branches (out of scope), the
 sampler is the engine's fused greedy sampler unless a request asks for temperature > 0 (then the batch
