@@ -689,7 +689,11 @@ static int prefill_layers_v2_body(b200_engine* e, const int* pos3, int T, int ct
     const bool fresh = ctx0 == 0;
     const bf16 *ka = fresh ? qkv + QH : kc, *va = fresh ? qkv + QH + (long)c.n_kv_heads * hd : vc;
     const long kv_ts = fresh ? QKV : hd, kv_hs = fresh ? hd : (long)e->kv_cap * hd;
-    const bool fa = attention_fa_supported(qkv, QKV, hd, ka, kv_ts, kv_hs, va, kv_ts, kv_hs, att, QH, hd);
+    // A portion whose keys, the cached ones included, are one tile of 128 has nothing to pipeline: the kernel without TMA is ahead by
+    // what the other's launch costs.  Two 7B layers, that one | the pipelined: 2 tokens behind 13 217 | 228 us, 16 behind 100
+    // 224 | 228, 100 behind 13 260 | 262; two tiles: 100 behind 100 267 | 264, 2 behind 300 230 | 229.
+    const bool fa = (fresh || S > 128) &&
+                    attention_fa_supported(qkv, QKV, hd, ka, kv_ts, kv_hs, va, kv_ts, kv_hs, att, QH, hd);
     e->launches += 2;
     if (segs) {
       B200_REQUIRE(fa, "prefill_batch: the pipelined attention kernel does not support this geometry");

@@ -55,7 +55,7 @@ struct WtParams {
   int kb_per_split;
   int epilogue, mode;
   int inter;
-  unsigned flags;  // debug: 1 = no MMA (loads only), 2 = no loads (MMA on stale smem), 4 = no epilogue stores
+  unsigned flags;  // debug: 1 = no MMA (loads only), 2 = no loads (MMA on stale smem; CTA pairs: the waits run out), 4 = no epilogue stores
   // fp32-accurate towers (LLaVA / Idefics2: the reference runs them in fp32 with bf16-valued weights):
   // X is a SPLIT operand [x_hi | x_lo] (n parts of K_w columns, each padded to 64) multiplied by the SAME
   // weight k-blocks (kb_w of them): D = W.x_hi + W.x_lo in fp32 — exact to ~2^-17 relative.

@@ -49,7 +49,7 @@ def test_a_picture_of_nans_stays_alone():
     assert torch.equal(a[:9], b[:9]) and bool(torch.isnan(b[9:].float()).all())
 
 
-@pytest.mark.parametrize("first,total", [(1, 130), (127, 128), (128, 257), (129, 160), (200, 201)])
+@pytest.mark.parametrize("first,total", [(1, 130), (127, 128), (128, 257), (129, 160), (200, 201), (20, 51), (13, 15), (100, 129)])
 def test_a_later_portion_reads_the_cache(first, total):
     """two portions == one, at the real head size: same kernel, same keys and values, same order of sums"""
     from mlx_vlm_b200.models.cache import make_prompt_cache
