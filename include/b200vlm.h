@@ -42,6 +42,7 @@ int b200_device_check(int device, int* sm_count);
 #define B200_WAIT_PAIR 5       /* gemm_wt_pair_kernel */
 #define B200_WAIT_ATTENTION 6  /* attention_fa_kernel */
 #define B200_WAIT_TOWER 7      /* attention_f32_tc_kernel */
+#define B200_WAIT_LATENT 8     /* attention_latent_kernel */
 int b200_wait_error(int* out);
 
 /* ------------------------------------------------------------------------- */
@@ -489,6 +490,18 @@ int b200_lm_moe_tiles(const int* list, long list_stride, const int* count, int E
 int b200_lm_masked_softmax_bf16(const float* S, long lds, const int* pos, int H, float scale, void* P, long ldp,
                                 int rows, int Sp, void* stream);
 int b200_lm_cache_transpose(const void* cache_rows, long tok_stride, int S, int Sp, int kv_rank, void* out, void* stream);
+/* rows of query heads (dim | rot_dim fp32 each, heads side by side), their last rot_dim turned by cs, as bf16 rows */
+int b200_lm_latent_queries(const float* q, long ldq, void* out, long ldo, const void* cs, int H, int dim, int rot_dim, int rot_dims,
+                           int pairs, int T, void* stream);
+/* causal attention of a prompt portion over keys and values expanded from latent rows (attention_latent.cu): q bf16
+ * [n_q][H][dn + dr] (pitch q_ts), k [S][H][dn], kr [S][dr] (shared by the heads), v [S][H][dv]; query i sees the keys
+ * 0 .. S - n_q + i; out [n_q][H dv], fp32 (out32) or bf16.  Head dims multiples of 8, ceil(dn / 64) + (dr > 0) <= 3, dr <= 64,
+ * dv <= 128; 16-byte rows; scale > 0.  flags: 1: nothing is loaded (the waits run out: NaN, b200_wait_error) */
+int b200_lm_latent_expanded_attention(const void* q, long q_ts, const void* k, long k_ts, const void* kr, long kr_ts, const void* v,
+                                      long v_ts, void* out, long o_ts, int out32, int H, int dn, int dr, int dv, int n_q, int S,
+                                      float scale, int flags, void* stream);
+/* C [T, N] (bf16) = X [T, K] . W [N, K]^T (bf16 operands, row pitches in elements, multiples of 8) on the tensor cores */
+int b200_gemm_wt_rows(const void* X, long ldx, const void* W, void* C, long ldc, int T, int N, int K, void* stream);
 /* greedy: lowest index of the largest logit per row and its log-probability */
 int b200_lm_argmax_rows(const float* z, long ldz, int V, int* tok, float* logprob, int B, void* stream);
 /* device-side token feedback of a decode loop (one block): tok = sampled, pos += 1 for active rows;

@@ -419,6 +419,31 @@ __global__ void rope_q_kernel(const float* __restrict__ q, long ldq, int qh_stri
   }
 }
 
+// the query operand of the expanded form: bf16 rows, the last rot_dim of every head turned.  A thread takes four columns
+// (VEC: dim, rot_dim and the pitches are multiples of 4).
+template <bool VEC>
+__global__ void latent_queries_kernel(const float* __restrict__ q, long ldq, bf16* __restrict__ out, long ldo,
+                                      const float2* __restrict__ cs, int n_cols, int dim, int rot_dim, int rot_dims, int pairs) {
+  const int t = blockIdx.x, hd = dim + rot_dim;
+  const float* x = q + (long)t * ldq;
+  const float2* a = cs + (long)t * (rot_dims >> 1);
+  bf16* o = out + (long)t * ldo;
+  constexpr int W = VEC ? 4 : 1;
+  for (int e = threadIdx.x * W; e < n_cols; e += blockDim.x * W) {
+    const int i = e % hd;
+    float v[W];
+    if (i < dim) {
+      if constexpr (VEC) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(x + e);
+      else v[0] = x[e];
+    } else {
+#pragma unroll
+      for (int u = 0; u < W; ++u) v[u] = rope_elem(x + e - i + dim, i - dim + u, rot_dims, a, pairs);
+    }
+    if constexpr (VEC) *reinterpret_cast<uint2*>(o + e) = make_uint2(pack2(v[0], v[1]), pack2(v[2], v[3]));
+    else o[e] = f2bf(v[0]);
+  }
+}
+
 // ---------------------------------------------------------------------------------------------------------
 // absorbed latent attention.  Block = (query token, group of up to 8 heads); a warp per head.  Keys are the cache
 // rows 0..pos[t] of slot[t], staged 32 at a time in shared memory (fp32); lane j scores key j, then the lanes
@@ -1566,6 +1591,17 @@ int b200_lm_masked_softmax_bf16(const float* S, long lds, const int* pos, int H,
   return B200_OK;
 }
 
+int b200_lm_latent_queries(const float* q, long ldq, void* out, long ldo, const void* cs, int H, int dim, int rot_dim, int rot_dims,
+                           int pairs, int T, void* st) {
+  B200_REQUIRE(q && out && H > 0 && dim > 0 && rot_dim >= 0 && rot_dims >= 0 && rot_dims <= rot_dim && rot_dims % 2 == 0 && T > 0 &&
+                   (cs || !rot_dims) && ldq >= (long)H * (dim + rot_dim) && ldo >= (long)H * (dim + rot_dim),
+               "lm_latent_queries: bad argument");
+  const bool vec = dim % 4 == 0 && rot_dim % 4 == 0 && ldq % 4 == 0 && ldo % 4 == 0 && ((uintptr_t)q & 15) == 0 && ((uintptr_t)out & 7) == 0;
+  if (vec) latent_queries_kernel<true><<<T, 256, 0, (cudaStream_t)st>>>(q, ldq, (bf16*)out, ldo, (const float2*)cs, H * (dim + rot_dim), dim, rot_dim, rot_dims, pairs);
+  else latent_queries_kernel<false><<<T, 256, 0, (cudaStream_t)st>>>(q, ldq, (bf16*)out, ldo, (const float2*)cs, H * (dim + rot_dim), dim, rot_dim, rot_dims, pairs);
+  B200_CHECK_LAUNCH();
+  return B200_OK;
+}
 int b200_lm_cache_transpose(const void* cache_rows, long tok_stride, int S, int Sp, int kv_rank, void* out, void* st) {
   B200_REQUIRE(cache_rows && out && S > 0 && Sp >= S && kv_rank > 0, "lm_cache_transpose: bad argument");
   cache_transpose_kernel<<<dim3(cdiv(Sp, 32), cdiv(kv_rank, 32)), 256, 0, (cudaStream_t)st>>>(

@@ -446,6 +446,11 @@ int b200_gemm_wt_f32(const void* X, long ldx, const void* W, long ldw, const voi
   return gemm_wt_tuned(X, ldx, W, bias, nullptr, 0, nullptr, 0, nullptr, 0, T, N, n_parts * kbw * 64, epilogue, mode, 0,
                        false, 148, nullptr, (cudaStream_t)stream, &ext);
 }
+int b200_gemm_wt_rows(const void* X, long ldx, const void* W, void* C, long ldc, int T, int N, int K, void* stream) {
+  B200_REQUIRE(X && W && C && ldc >= N, "gemm_wt_rows: bad argument");
+  return gemm_wt_tuned(X, ldx, W, nullptr, nullptr, 0, C, ldc, nullptr, 0, T, N, K, B200_EPI_NONE, B200_WT_BF16, 0, false, 148,
+                       nullptr, (cudaStream_t)stream);
+}
 /* Grouped Linear on the tensor cores, ONE launch: token tile y (128 rows of X, C32) multiplies the weight rows of group
  * tile_group[y] (device array of n_tiles entries; < 0: an empty tile).  X [n_tiles * 128, ceil64(K_w)] bf16 holds every
  * group's rows in a segment padded to whole tiles, W [n_groups][N][K_w] bf16, C32 [n_tiles * 128, N] fp32.  No host

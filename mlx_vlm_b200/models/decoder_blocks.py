@@ -79,6 +79,8 @@ from .._native import B200Error as _B200Error
 from .layer_ops import (ACT_GELU, ACT_TANH, EPI_GELU, EPI_RELU2, EPI_SOFTCAP, EPI_TABLE_GATE, GELU_TANH_ALPHA, GELU_TANH_CUBIC,
                         WAVELENGTH, LayerOps)
 
+EXPANDED_MAX = 1 << 29      # numbers of a slot's expanded keys and values (one GiB); a longer context keeps the absorbed form
+
 
 @dataclass
 class StepCtx:
@@ -145,6 +147,10 @@ class LatentAttention:
         if not self.q_rank and self.kv_from is not None:
             raise ValueError(f"layer {index}: a layer that borrows its latent needs a query latent")
         self.n_q = self.H * (self.dim + self.rot_dim)
+        # head dims that a long portion's keys and values may be expanded for (csrc/attention_latent.cu)
+        self.expands = (not self.window and not self.split_weights and self.scale > 0 and self.dim % 8 == 0 and self.kv_rank % 8 == 0
+                        and self.rot_dim % 8 == 0 and self.rot_dim <= 64 and self.vdim % 8 == 0 and self.vdim <= 128
+                        and (self.dim + 63) // 64 + (self.rot_dim > 0) <= 3)
         self.cache_index = -1     # set by the model: which caching layer of the pool this mixer reads (and writes)
         self.kv_dim, self.state_floats, self.state_off = self.kv_rank + self.rot_dim, 0, 0
         self.w: Dict[str, torch.Tensor] = {}
@@ -164,8 +170,10 @@ class LatentAttention:
         out = [(p + "down", (n_down, self.W))]
         if self.q_rank:
             out += [(p + "dq.norm", (self.q_rank,)), (p + "uq", (self.n_q, self.q_rank))]
-        out += [(p + "ukT", (self.H, self.kv_rank, self.dim)), (p + "uv", (self.H * self.vdim, self.kv_rank)),
-                (p + "o", (self.W, self.H * self.vdim))]
+        # `ukv`: [uk; uv], both up-projections of a latent row as ONE product; uv is its second part
+        out += [(p + "ukT", (self.H, self.kv_rank, self.dim)),
+                (p + "ukv", (self.H * (self.dim + self.vdim), self.kv_rank)) if self.expands else
+                (p + "uv", (self.H * self.vdim, self.kv_rank)), (p + "o", (self.W, self.H * self.vdim))]
         if self.own_kv:
             out.append((p + "dkv.norm", (self.kv_rank,)))
         return out
@@ -196,14 +204,45 @@ class LatentAttention:
             at += self.row_dim
         if self.gated:
             down[at:].copy_(ck[p + "g"])
-        for n in (("dq.norm", "uq") if self.q_rank else ()) + ("uv", "o"):
+        for n in (("dq.norm", "uq") if self.q_rank else ()) + (() if self.expands else ("uv",)) + ("o",):
             view(p + n).copy_(ck[p + n])
+        if self.expands:
+            ukv = view(p + "ukv")
+            ukv[:self.H * self.dim].copy_(ck[p + "uk"])
+            ukv[self.H * self.dim:].copy_(ck[p + "uv"])
         # the key up-projection per head, transposed: it is applied to the QUERY (absorbed form)
         view(p + "ukT").copy_(ck[p + "uk"].view(self.H, self.dim, self.kv_rank).transpose(1, 2))
         self.bind(p, view)
 
     def bind(self, p: str, view):
         self.w = {n[len(p):]: view(n) for n, _ in self.manifest(p)}
+        if self.expands:
+            self.w["uv"] = self.w["ukv"][self.H * self.dim:]
+
+    def _expand_portions(self, ops: LayerOps, segs, cache_layer) -> bool:
+        """Whether a step's portions take the expanded form: from 128 tokens on, where the tensor cores take a step at all, it
+        was the faster at every context tried (128 tokens behind 4000: 239 -> 177 us a layer, 16 heads; 512 behind 8000: 583 ->
+        282; 2048 behind 6000: 2086 -> 385), and its distance from 64 bits is the smaller (0.0037 against 0.0041 there)."""
+        if not self.expands or not segs or cache_layer.dtype != torch.bfloat16:
+            return False
+        H, r, Dl, per = self.H, self.kv_rank, self.row_dim, self.H * (self.dim + self.vdim)
+        return ops.tc_ok(min(n for _, n, _, _ in segs), r, Dl, cache_layer.stride(1)) and cache_layer.data_ptr() % 16 == 0 and \
+            max((p0 + n) * per for _, n, _, p0 in segs) <= EXPANDED_MAX
+
+    def _expanded(self, ctx: StepCtx, q, cs, segs, cache_layer) -> torch.Tensor:
+        """Portions of prompts with the keys and values of their slots expanded from the cached rows: one product for both
+        ([W_uk; W_uv] on the latent part), attention heads of dim + rot_dim and vdim numbers.  -> the heads' outputs, bf16
+        operand rows where nothing but W_o reads them"""
+        ops, H, dn, dr, r, dv = ctx.ops, self.H, self.dim, self.rot_dim, self.kv_rank, self.vdim
+        qb = ops.latent_queries(q, cs, H, dn, dr, self.rot_dims if dr else 0, pairs=self.pairs)
+        operand = not self.gated and H * dv % 64 == 0 and ops.takes_operand(q.shape[0], self.w["o"])
+        att = ops.empty((q.shape[0], H * dv), torch.bfloat16 if operand else torch.float32)
+        for start, n, slot, p0 in segs:
+            rows = cache_layer[slot][:p0 + n]
+            kv = ops.rows_gemm(rows, self.w["ukv"], r)
+            ops.expanded_attention(qb[start:start + n], kv[:, :H * dn], rows[:, r:] if dr else None, kv[:, H * dn:],
+                                   att[start:start + n], H, dn, dr, dv, self.scale)
+        return att
 
     def forward(self, ctx: StepCtx, x: torch.Tensor) -> torch.Tensor:
         ops, w, T = ctx.ops, self.w, x.shape[0]
@@ -223,6 +262,17 @@ class LatentAttention:
                             dr, self.rot_dims, pairs=self.pairs)
             q = D[:, :self.n_q]
             n_read = self.n_q + Dl
+        segs = ctx.segments or []
+        if self._expand_portions(ops, segs, cache_layer):
+            try:
+                att = self._expanded(ctx, q, cs, segs, cache_layer)
+                if att.dtype == torch.bfloat16:
+                    return ops.operand_linear(att, w["o"])
+                if self.gated:
+                    ops.head_post(att, att, dv=dv, gate=D[:, n_read:], gate_per_head=self.gate_per_head)
+                return ops.linear(att, w["o"])
+            except _B200Error as e:
+                ops.tc_refused(e)
         qa = ops.empty((T, H * Dl))
         heads_tc = ops.tc_ok(T, dn, dn + dr, r) and dn % 64 == 0 and r % 64 == 0 and Dl % 4 == 0 and dv % 4 == 0
         if heads_tc:     # a prompt: the heads' products as ONE tcgen05 launch (inner sizes are whole k-blocks)
@@ -238,7 +288,6 @@ class LatentAttention:
         if dr:
             ops.rope_q(q, qa, cs, H, dn, dr, self.rot_dims, r, pairs=self.pairs)
         ol = ops.empty((T, H * r))
-        segs = ctx.segments or []
         done = False
         if any(ops.tc_ok(n, Dl, r, cache_layer.stride(1)) for _, n, _, _ in segs) and cache_layer.dtype == torch.bfloat16:
             try:

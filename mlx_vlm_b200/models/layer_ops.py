@@ -445,6 +445,31 @@ class LayerOps:
                  "lm_cache_transpose")
         return out
 
+    def latent_queries(self, q: torch.Tensor, cs: torch.Tensor, H: int, dim: int, rot_dim: int, rot_dims: int,
+                       pairs: bool = False) -> torch.Tensor:
+        """fp32 rows of query heads -> bf16 rows with their rotated part turned"""
+        T, out = q.shape[0], self.empty((q.shape[0], H * (dim + rot_dim)), torch.bfloat16)
+        self._ok(self.lib.b200_lm_latent_queries(q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0), cs.data_ptr(), H, dim,
+                                                 rot_dim, rot_dims, int(pairs), T, self.s), "lm_latent_queries")
+        return out
+
+    def rows_gemm(self, Xb: torch.Tensor, W: torch.Tensor, K: int) -> torch.Tensor:
+        """bf16 rows (T, >= K) -> Xb[:, :K] . W^T as bf16 rows, on the tensor cores"""
+        T, n = Xb.shape[0], W.shape[0]
+        out = self.empty((T, n), torch.bfloat16)
+        self._ok(self.lib.b200_gemm_wt_rows(Xb.data_ptr(), Xb.stride(0), W.data_ptr(), out.data_ptr(), n, T, n, K, self.s),
+                 "gemm_wt_rows")
+        return out
+
+    def expanded_attention(self, q: torch.Tensor, k: torch.Tensor, kr: Optional[torch.Tensor], v: torch.Tensor, out: torch.Tensor,
+                           H: int, dim: int, rot_dim: int, vdim: int, scale: float):
+        """q (n, H (dim + rot_dim)) bf16 against k (S, H dim), kr (S, rot_dim) and v (S, H vdim), all bf16 rows with pitches of
+        their own; the queries are the last n of the S positions; out (n, H vdim) fp32 or bf16"""
+        self._ok(self.lib.b200_lm_latent_expanded_attention(
+            q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), N.ptr(kr), kr.stride(0) if kr is not None else 0, v.data_ptr(),
+            v.stride(0), out.data_ptr(), out.stride(0), int(out.dtype == torch.float32), H, dim, rot_dim, vdim, q.shape[0],
+            k.shape[0], float(scale), 0, self.s), "lm_latent_expanded_attention")
+
     def linear(self, X: torch.Tensor, W: torch.Tensor, bias=None, epi=EPI_NONE, epi_param=0.0,
                out: Optional[torch.Tensor] = None, add: bool = False, exact_x: bool = False,
                operand: Optional[torch.Tensor] = None) -> torch.Tensor:
