@@ -288,6 +288,9 @@ int b200_engine_fetch_tokens(b200_engine* e, long start, int n, int* host_out, v
 int b200_f32_layer_norm(const float* x, long ldx, const void* w, const void* b, float eps, float* out32,
                         long ld32, void* out_split, long ld_split, int n_pad, int T, int N, void* stream);
 int b200_f32_split(const float* x, long ldx, void* out_split, long ld_split, int n_pad, int T, int N, void* stream);
+/* b200_f32_split of rows seg_off .. seg_off + seg_out - 1 of every seg_in input rows (T output rows in all) */
+int b200_f32_split_segments(const float* x, long ldx, int seg_in, int seg_off, int seg_out, void* out, long ld_split, int n_pad,
+                            int T, int N, void* stream);
 /* nn.RMSNorm on fp32 rows (idefics2.py:60-90,118-143); input row t goes to output row
  * (t / seg_in) * seg_out + seg_off + t % seg_in (seg_in == 0: row t) */
 int b200_f32_rms_norm(const float* x, long ldx, const void* w, float eps, float* out32, long ld32, void* out_split,
@@ -304,6 +307,9 @@ int b200_pixel_shuffle_split(const float* x, int n_img, int side, int E, int s, 
  * [B*gh*gw, Kp | Kp] (llava/vision.py:108-127, idefics2/vision.py:123-148) */
 int b200_clip_patchify(const float* pixels_nhwc, int B, int H, int W, int C, int patch, void* out_split, int Kp,
                        void* stream);
+/* the same for pixels in any order: element (b, y, x, c) at b sb + y sy + x sx + c sc */
+int b200_clip_patchify_strided(const float* pix, long sb, long sy, long sx, long sc, int B, int H, int W, int C, int ps, void* out,
+                               int Kp, void* stream);
 /* class token + learned positions (CLIP), or positions gathered by pos_ids (SigLIP, idefics2/vision.py:150-173;
  * negative ids index from the end like numpy) */
 int b200_tower_embed(const float* patch, const void* cls, const void* pos, const int* pos_ids, float* emb, int B,
@@ -338,6 +344,9 @@ int b200_f32_gather_rows(const float* in, long ld_in, const int* idx, int n_idx,
 int b200_gemm_wt_f32(const void* X, long ldx, const void* W, long ldw, const void* bias, const float* res32,
                      long ldr32, float* C32, long ldc32, void* Csplit, long ld_split, int n_pad, int T, int N,
                      int K_w, int n_parts, int epilogue, int mode, void* stream);
+/* the same sums (+ bias), rounded once to bf16 rows */
+int b200_gemm_wt_f32_bf16(const void* X, long ldx, const void* W, long ldw, const void* bias, void* C, long ldc, int T, int N,
+                          int K_w, int n_parts, void* stream);
 /* grouped Linear in ONE launch: token tile y (128 rows) of X [n_tiles * 128, ceil64(K_w)] bf16 multiplies the weight
  * rows of group tile_group[y] (device; < 0: empty tile) of W [n_groups][N][K_w]; C32 [n_tiles * 128, N] fp32.  The groups'
  * rows lie in segments padded to whole tiles (b200_lm_moe_tiles builds the table on the device) */

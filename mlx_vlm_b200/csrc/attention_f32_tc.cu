@@ -250,11 +250,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
   long q_first = (long)seg * p.q_seg, k_first = (long)seg * p.k_seg;
   int Lq = p.Lq, S = p.S;
   if (p.cu) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // (the table may come from the kernel before)
     q_first = k_first = p.cu[seg];
     Lq = S = p.cu[seg + 1] - p.cu[seg];
     if (q0 >= Lq) return;   // uniform per CTA, nothing is allocated yet
   }
   const int n_tiles = (S + TC_KEYS - 1) / TC_KEYS;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (tid == 0) {
     failed = 0;
     t_init(&bars.q_full, 256);
@@ -280,6 +282,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
   __syncthreads();
   t_fence_after();
   const uint32_t tmem = tmem_slot;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 
   if (warp == 11) {
     if (lane == 0) {  // ===== MMA issuer =====
@@ -574,8 +577,7 @@ int tc_launch(const AttnF32P& p, dim3 grid, cudaStream_t st) {
   static unsigned long long attr_mask = 0ull;
   if (FirstUse first{&attr_mask})
     B200_CUDA(cudaFuncSetAttribute(attention_f32_tc_kernel<HDP>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem<HDP>()));
-  attention_f32_tc_kernel<HDP><<<grid, TC_THREADS, tc_smem<HDP>(), st>>>(p);
-  B200_CHECK_LAUNCH();
+  B200_CUDA(launch_pdl(attention_f32_tc_kernel<HDP>, grid, dim3(TC_THREADS), tc_smem<HDP>(), st, p));
   return B200_OK;
 }
 

@@ -45,6 +45,7 @@ __global__ void __launch_bounds__(256) f32_layer_norm_kernel(const float* __rest
                                                              bf16* __restrict__ out_split, long ld_split,
                                                              int n_pad, int N) {
   __shared__ float red[8];
+  pdl_prologue();
   const int t = blockIdx.x;
   const int nv = N >> 2;
   float4 h[8];
@@ -84,6 +85,51 @@ __global__ void __launch_bounds__(256) f32_layer_norm_kernel(const float* __rest
   }
 }
 
+// The same with a warp per row (rows of up to 128 V numbers, V float4 a lane): no block-wide sums, eight rows of loads in
+// flight per CTA.  Bound by its bytes (2 fp32 numbers a column in and out).  Measured, 4616 rows of 1024 (38 MB, out of the
+// L2): a CTA per row 14.7 us, this 5.4; 4096 of 1152: 14.1, 5.9.
+template <int V>
+__global__ void __launch_bounds__(256) f32_layer_norm_warp_kernel(const float* __restrict__ x, long ldx, const bf16* __restrict__ w,
+                                                                  const bf16* __restrict__ b, float eps, float* __restrict__ out32,
+                                                                  long ld32, bf16* __restrict__ out_split, long ld_split, int n_pad,
+                                                                  int T, int N) {
+  pdl_prologue();
+  const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= T) return;
+  const int nv = N >> 2;
+  float4 h[V];
+  float s1 = 0.f;
+#pragma unroll
+  for (int u = 0; u < V; ++u) {
+    const int c = lane + 32 * u;
+    h[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < nv) h[u] = *reinterpret_cast<const float4*>(x + (long)t * ldx + c * 4);
+  }
+#pragma unroll
+  for (int u = 0; u < V; ++u) s1 += (h[u].x + h[u].y) + (h[u].z + h[u].w);
+  const float mu = warp_sum(s1) / (float)N;
+  float v = 0.f;
+#pragma unroll
+  for (int u = 0; u < V; ++u) {
+    if (lane + 32 * u >= nv) continue;
+    const float d0 = h[u].x - mu, d1 = h[u].y - mu, d2 = h[u].z - mu, d3 = h[u].w - mu;
+    v += (d0 * d0 + d1 * d1) + (d2 * d2 + d3 * d3);
+  }
+  const float rstd = rsqrtf(warp_sum(v) / (float)N + eps);
+#pragma unroll
+  for (int u = 0; u < V; ++u) {
+    const int c = lane + 32 * u;
+    if (c >= nv) continue;
+    float wf[4] = {1.f, 1.f, 1.f, 1.f}, bb[4] = {0.f, 0.f, 0.f, 0.f};
+    if (w) unpack4(*reinterpret_cast<const uint2*>(w + c * 4), wf);
+    if (b) unpack4(*reinterpret_cast<const uint2*>(b + c * 4), bb);
+    const float o0 = (h[u].x - mu) * rstd * wf[0] + bb[0], o1 = (h[u].y - mu) * rstd * wf[1] + bb[1];
+    const float o2 = (h[u].z - mu) * rstd * wf[2] + bb[2], o3 = (h[u].w - mu) * rstd * wf[3] + bb[3];
+    if (out32) *reinterpret_cast<float4*>(out32 + (long)t * ld32 + c * 4) = make_float4(o0, o1, o2, o3);
+    if (out_split) split_store4(out_split + (long)t * ld_split + c * 4, n_pad, o0, o1, o2, o3);
+  }
+}
+
 // RMSNorm in fp32 (nn.RMSNorm on fp32 rows, bf16-valued weight) -> fp32 and / or split output.  Input row
 // t is written to output row (t / seg_in) * seg_out + seg_off + t % seg_in: the Idefics2 perceiver
 // normalises the context and the latents separately and attends over their concatenation
@@ -94,6 +140,7 @@ __global__ void __launch_bounds__(256) f32_rms_norm_kernel(const float* __restri
                                                            bf16* __restrict__ out_split, long ld_split, int n_pad,
                                                            int N, int seg_in, int seg_out, int seg_off) {
   __shared__ float red[8];
+  pdl_prologue();
   const int t = blockIdx.x;
   const long ot = seg_in > 0 ? (long)(t / seg_in) * seg_out + seg_off + t % seg_in : t;
   const int nv = N >> 2;
@@ -125,6 +172,7 @@ __global__ void __launch_bounds__(256) f32_rms_norm_kernel(const float* __restri
 // SwiGLU in fp32: gu [T, 2I] = [gate | up] -> split operand of silu(gate) * up (idefics2.py:146-171, mlp)
 __global__ void f32_swiglu_split_kernel(const float* __restrict__ gu, long ldg, bf16* __restrict__ out, long ld_split,
                                         int n_pad, int T, int I) {
+  pdl_prologue();
   const int nv = I >> 2;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < (long)T * nv; i += (long)gridDim.x * blockDim.x) {
     const int t = (int)(i / nv), c = (int)(i % nv);
@@ -135,13 +183,16 @@ __global__ void f32_swiglu_split_kernel(const float* __restrict__ gu, long ldg, 
   }
 }
 
-// fp32 [T, N] -> split operand [T, hi | lo] (zero padding columns are the caller's: buffers are zeroed once)
+// fp32 [T, N] -> split operand [T, hi | lo] (zero padding columns are the caller's).  seg_out > 0: output row t is input row
+// (t / seg_out) * seg_in + seg_off + t mod seg_out (an image's rows without its class token)
 __global__ void f32_split_kernel(const float* __restrict__ x, long ldx, bf16* __restrict__ out, long ld_split,
-                                 int n_pad, int T, int N) {
+                                 int n_pad, int T, int N, int seg_in, int seg_off, int seg_out) {
+  pdl_prologue();
   const int nv = N >> 2;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < (long)T * nv; i += (long)gridDim.x * blockDim.x) {
     const int t = (int)(i / nv), c = (int)(i % nv);
-    const float4 v = *reinterpret_cast<const float4*>(x + (long)t * ldx + c * 4);
+    const long r = seg_out > 0 ? (long)(t / seg_out) * seg_in + seg_off + t % seg_out : t;
+    const float4 v = *reinterpret_cast<const float4*>(x + r * ldx + c * 4);
     split_store4(out + (long)t * ld_split + c * 4, n_pad, v.x, v.y, v.z, v.w);
   }
 }
@@ -205,24 +256,36 @@ __global__ void f32_gather_rows_kernel(const float* __restrict__ in, long ld_in,
   }
 }
 
-// Conv2d(kernel == stride) as a Linear: NHWC fp32 pixels -> rows of (kh, kw, c)-ordered patches, written
-// as a split operand [B * gh * gw, Kp | Kp] (K = ps * ps * C, zero padded to Kp).  (llava/vision.py:108-127)
-__global__ void clip_patchify_kernel(const float* __restrict__ pix, int B, int H, int W, int C, int ps,
-                                     bf16* __restrict__ out, int Kp) {
-  const int gh = H / ps, gw = W / ps, K = ps * ps * C;
-  const long total = (long)B * gh * gw * Kp;
-  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const int k = (int)(i % Kp);
-    const long r = i / Kp;
-    float v = 0.f;
-    if (k < K) {
-      const int c = k % C, kw = (k / C) % ps, kh = k / (C * ps);
-      const int gx = (int)(r % gw), gy = (int)((r / gw) % gh), b = (int)(r / ((long)gw * gh));
-      v = pix[(((long)b * H + gy * ps + kh) * W + gx * ps + kw) * C + c];
+// Conv2d(kernel == stride) as a Linear: fp32 pixels, element (b, y, x, c) at b sb + y sy + x sx + c sc, -> rows of
+// (kh, kw, c)-ordered patches, written as a split operand [B * gh * gw, Kp | Kp] (K = ps * ps * C, zero padded to Kp).
+// (llava/vision.py:108-127)  A CTA takes `per` patches of a row of patches (blockIdx.y) and 256 of their columns: a thread
+// keeps two columns (Kp is even) and walks the patches, so the divisions are made once, the pixels are read where they lie
+// (any channel order) and the stores are whole words.  Measured, 8 pictures of 336 x 336: an element at a time from NHWC
+// 30 us and the permutation before it 12, this 6.6; one picture 6.6, 2.4.
+__global__ void __launch_bounds__(128) clip_patchify_kernel(const float* __restrict__ pix, long sb, long sy, long sx, long sc, int gh,
+                                                            int gw, int per, int C, int ps, bf16* __restrict__ out, int Kp) {
+  pdl_prologue();
+  const int b = blockIdx.y / gh, gy = blockIdx.y % gh, K = ps * ps * C;
+  const float* row = pix + b * sb + (long)gy * ps * sy;
+  bf16* o = out + (long)blockIdx.y * gw * 2 * Kp;
+  for (int k = 2 * (blockIdx.x * blockDim.x + threadIdx.x); k < Kp; k += 2 * blockDim.x * gridDim.x) {
+    long at[2];
+    bool in[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int kk = k + e, c = kk % C, r = kk / C;
+      in[e] = kk < K;
+      at[e] = (r / ps) * sy + (r % ps) * sx + c * sc;
     }
-    const float hi = rbf(v);
-    out[r * 2 * Kp + k] = f2bf(hi);
-    out[r * 2 * Kp + Kp + k] = f2bf(v - hi);
+#pragma unroll 8
+    for (int gx = blockIdx.z * per; gx < min(gw, (int)(blockIdx.z + 1) * per); ++gx) {
+      const float* p = row + (long)gx * ps * sx;
+      const float v0 = in[0] ? __ldg(p + at[0]) : 0.f, v1 = in[1] ? __ldg(p + at[1]) : 0.f;
+      const float h0 = rbf(v0), h1 = rbf(v1);
+      uint32_t* d = reinterpret_cast<uint32_t*>(o + (long)gx * 2 * Kp + k);
+      d[0] = pack2(h0, h1);
+      d[Kp >> 1] = pack2(v0 - h0, v1 - h1);
+    }
   }
 }
 
@@ -231,6 +294,7 @@ __global__ void clip_patchify_kernel(const float* __restrict__ pix, int B, int H
 __global__ void tower_embed_kernel(const float* __restrict__ patch, const bf16* __restrict__ cls,
                                    const bf16* __restrict__ pos, const int* __restrict__ pos_ids,
                                    float* __restrict__ emb, int B, int P, int E, int n_pos) {
+  pdl_prologue();
   const int L = P + (cls ? 1 : 0);
   const long total = (long)B * L * (E >> 2);
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
@@ -273,9 +337,16 @@ int f32_layer_norm(const float* x, long ldx, const void* w, const void* b, float
   B200_REQUIRE(x && T > 0 && N > 0 && (N % 4) == 0 && N <= 8192 && (ldx % 4) == 0, "f32_layer_norm: T=%d N=%d", T, N);
   B200_REQUIRE(out32 || out_split, "f32_layer_norm: no output");
   B200_REQUIRE(!out_split || ((ld_split % 4) == 0 && (n_pad % 4) == 0), "f32_layer_norm: split pitch");
-  f32_layer_norm_kernel<<<T, 256, 0, st>>>(x, ldx, (const bf16*)w, (const bf16*)b, eps, out32, ld32,
-                                           (bf16*)out_split, ld_split, n_pad, N);
-  B200_CHECK_LAUNCH();
+  // up to 2048 columns a warp holds a row in registers; rows of less than eight warps an SM are a chain of latencies that a
+  // CTA per row makes shorter (577 x 1024: 2.8 us, a warp per row 4.2; 1024 x 1152: 5.1 both)
+  if (N <= 2048 && T >= 8 * 148) {
+    const auto k = N <= 1024 ? f32_layer_norm_warp_kernel<8> : N <= 1280 ? f32_layer_norm_warp_kernel<10> : f32_layer_norm_warp_kernel<16>;
+    B200_CUDA(launch_pdl(k, dim3(cdiv(T, 8)), dim3(256), 0, st, x, ldx, (const bf16*)w, (const bf16*)b, eps, out32, ld32,
+                         (bf16*)out_split, ld_split, n_pad, T, N));
+    return B200_OK;
+  }
+  B200_CUDA(launch_pdl(f32_layer_norm_kernel, dim3(T), dim3(256), 0, st, x, ldx, (const bf16*)w, (const bf16*)b, eps, out32, ld32,
+                       (bf16*)out_split, ld_split, n_pad, N));
   return B200_OK;
 }
 
@@ -283,24 +354,25 @@ int f32_rms_norm(const float* x, long ldx, const void* w, float eps, float* out3
                  long ld_split, int n_pad, int T, int N, int seg_in, int seg_out, int seg_off, cudaStream_t st) {
   B200_REQUIRE(x && w && T > 0 && N > 0 && (N % 4) == 0 && N <= 8192 && (ldx % 4) == 0 && (out32 || out_split),
                "f32_rms_norm: T=%d N=%d", T, N);
-  f32_rms_norm_kernel<<<T, 256, 0, st>>>(x, ldx, (const bf16*)w, eps, out32, ld32, (bf16*)out_split, ld_split, n_pad, N,
-                                         seg_in, seg_out, seg_off);
-  B200_CHECK_LAUNCH();
+  B200_CUDA(launch_pdl(f32_rms_norm_kernel, dim3(T), dim3(256), 0, st, x, ldx, (const bf16*)w, eps, out32, ld32, (bf16*)out_split,
+                       ld_split, n_pad, N, seg_in, seg_out, seg_off));
   return B200_OK;
 }
 
 int f32_swiglu_split(const float* gu, long ldg, void* out, long ld_split, int n_pad, int T, int I, cudaStream_t st) {
   B200_REQUIRE(gu && out && T > 0 && I > 0 && (I % 4) == 0 && (ldg % 4) == 0 && (ld_split % 4) == 0, "f32_swiglu: bad shape");
-  f32_swiglu_split_kernel<<<t_grid((long)T * (I / 4), 256), 256, 0, st>>>(gu, ldg, (bf16*)out, ld_split, n_pad, T, I);
-  B200_CHECK_LAUNCH();
+  B200_CUDA(launch_pdl(f32_swiglu_split_kernel, dim3(t_grid((long)T * (I / 4), 256)), dim3(256), 0, st, gu, ldg, (bf16*)out, ld_split,
+                       n_pad, T, I));
   return B200_OK;
 }
 
-int f32_split(const float* x, long ldx, void* out, long ld_split, int n_pad, int T, int N, cudaStream_t st) {
+int f32_split(const float* x, long ldx, void* out, long ld_split, int n_pad, int T, int N, cudaStream_t st, int seg_in = 0,
+              int seg_off = 0, int seg_out = 0) {
   B200_REQUIRE(x && out && T > 0 && N > 0 && (N % 4) == 0 && (ldx % 4) == 0 && (ld_split % 4) == 0 && (n_pad % 4) == 0,
                "f32_split: bad shape");
-  f32_split_kernel<<<t_grid((long)T * (N / 4), 256), 256, 0, st>>>(x, ldx, (bf16*)out, ld_split, n_pad, T, N);
-  B200_CHECK_LAUNCH();
+  B200_REQUIRE(seg_out >= 0 && seg_off >= 0 && (seg_out == 0 || (seg_off + seg_out <= seg_in && T % seg_out == 0)), "f32_split: segments");
+  B200_CUDA(launch_pdl(f32_split_kernel, dim3(t_grid((long)T * (N / 4), 256)), dim3(256), 0, st, x, ldx, (bf16*)out, ld_split, n_pad,
+                       T, N, seg_in, seg_off, seg_out));
   return B200_OK;
 }
 
@@ -315,12 +387,17 @@ int pixel_shuffle_split(const float* x, int n_img, int side, int E, int s, int r
   return B200_OK;
 }
 
-int clip_patchify(const float* pix, int B, int H, int W, int C, int ps, void* out, int Kp, cudaStream_t st) {
-  B200_REQUIRE(pix && out && B > 0 && H % ps == 0 && W % ps == 0 && Kp >= ps * ps * C && (Kp % 8) == 0,
+int clip_patchify(const float* pix, long sb, long sy, long sx, long sc, int B, int H, int W, int C, int ps, void* out, int Kp,
+                  cudaStream_t st) {
+  B200_REQUIRE(pix && out && B > 0 && ps > 0 && C > 0 && H >= ps && W >= ps && H % ps == 0 && W % ps == 0 && Kp >= ps * ps * C &&
+                   (Kp % 8) == 0 && ((uintptr_t)out & 3) == 0,
                "clip_patchify: bad shape");
-  const long total = (long)B * (H / ps) * (W / ps) * Kp;
-  clip_patchify_kernel<<<t_grid(total, 256), 256, 0, st>>>(pix, B, H, W, C, ps, (bf16*)out, Kp);
-  B200_CHECK_LAUNCH();
+  // eight patches a thread: as many loads in flight as it keeps, and CTAs enough for one picture to fill the chip
+  const int gh = H / ps, gw = W / ps, per = 8, most = 65535 / gh;
+  B200_REQUIRE(gh <= 65535, "clip_patchify: %d rows of patches", gh);
+  for (int b = 0; b < B; b += most)      // (the grid's second axis ends at 65535)
+    B200_CUDA(launch_pdl(clip_patchify_kernel, dim3(cdiv(Kp, 256), min(most, B - b) * gh, cdiv(gw, per)), dim3(128), 0, st, pix + b * sb,
+                         sb, sy, sx, sc, gh, gw, per, C, ps, (bf16*)out + (long)b * gh * gw * 2 * Kp, Kp));
   return B200_OK;
 }
 
@@ -328,9 +405,8 @@ int tower_embed(const float* patch, const void* cls, const void* pos, const int*
                 int E, int n_pos, cudaStream_t st) {
   B200_REQUIRE(patch && pos && emb && B > 0 && P > 0 && (E % 4) == 0, "tower_embed: bad shape");
   const long total = (long)B * (P + (cls ? 1 : 0)) * (E / 4);
-  tower_embed_kernel<<<t_grid(total, 256), 256, 0, st>>>(patch, (const bf16*)cls, (const bf16*)pos, pos_ids, emb, B, P,
-                                                         E, n_pos);
-  B200_CHECK_LAUNCH();
+  B200_CUDA(launch_pdl(tower_embed_kernel, dim3(t_grid(total, 256)), dim3(256), 0, st, patch, (const bf16*)cls, (const bf16*)pos, pos_ids,
+                       emb, B, P, E, n_pos));
   return B200_OK;
 }
 
@@ -399,7 +475,16 @@ int b200_pixel_shuffle_split(const float* x, int n_img, int side, int E, int s, 
   return pixel_shuffle_split(x, n_img, side, E, s, round_in, out_split, ld_split, n_pad, (cudaStream_t)st);
 }
 int b200_clip_patchify(const float* pix, int B, int H, int W, int C, int ps, void* out, int Kp, void* st) {
-  return clip_patchify(pix, B, H, W, C, ps, out, Kp, (cudaStream_t)st);
+  return clip_patchify(pix, (long)H * W * C, (long)W * C, C, 1, B, H, W, C, ps, out, Kp, (cudaStream_t)st);
+}
+int b200_clip_patchify_strided(const float* pix, long sb, long sy, long sx, long sc, int B, int H, int W, int C, int ps, void* out,
+                               int Kp, void* st) {
+  return clip_patchify(pix, sb, sy, sx, sc, B, H, W, C, ps, out, Kp, (cudaStream_t)st);
+}
+int b200_f32_split_segments(const float* x, long ldx, int seg_in, int seg_off, int seg_out, void* out, long ld_split, int n_pad,
+                            int T, int N, void* st) {
+  B200_REQUIRE(seg_out > 0, "f32_split_segments: empty segments");
+  return f32_split(x, ldx, out, ld_split, n_pad, T, N, (cudaStream_t)st, seg_in, seg_off, seg_out);
 }
 int b200_tower_embed(const float* patch, const void* cls, const void* pos, const int* pos_ids, float* emb, int B,
                      int P, int E, int n_pos, void* st) {
@@ -445,6 +530,17 @@ int b200_gemm_wt_f32(const void* X, long ldx, const void* W, long ldw, const voi
   ext.ldr32 = ldr32; ext.Csplit = (bf16*)Csplit; ext.ld_split = ld_split; ext.n_pad = n_pad;
   return gemm_wt_tuned(X, ldx, W, bias, nullptr, 0, nullptr, 0, nullptr, 0, T, N, n_parts * kbw * 64, epilogue, mode, 0,
                        false, 148, nullptr, (cudaStream_t)stream, &ext);
+}
+/* the same product as b200_gemm_wt_f32 (fp32 sums of n_parts parts, + bias), rounded once to bf16 rows */
+int b200_gemm_wt_f32_bf16(const void* X, long ldx, const void* W, long ldw, const void* bias, void* C, long ldc, int T, int N, int K_w,
+                          int n_parts, void* stream) {
+  B200_REQUIRE(X && W && C && ldc >= N && n_parts >= 1, "gemm_wt_f32_bf16: bad argument");
+  const int kbw = cdiv(K_w, 64);
+  WtExt ext;
+  memset(static_cast<void*>(&ext), 0, sizeof(ext));
+  ext.kb_w = kbw; ext.k_w = K_w; ext.ldw = ldw;
+  return gemm_wt_tuned(X, ldx, W, bias, nullptr, 0, C, ldc, nullptr, 0, T, N, n_parts * kbw * 64, B200_EPI_NONE, B200_WT_BF16, 0, false,
+                       148, nullptr, (cudaStream_t)stream, &ext);
 }
 int b200_gemm_wt_rows(const void* X, long ldx, const void* W, void* C, long ldc, int T, int N, int K, void* stream) {
   B200_REQUIRE(X && W && C && ldc >= N, "gemm_wt_rows: bad argument");

@@ -97,8 +97,7 @@ class VisionModel:
         pos_dev = torch.from_numpy(np.ascontiguousarray(pos_ids))
         with torch.cuda.stream(eng.stream):
             pos_dev = pos_dev.to(eng.device)
-        x = x.contiguous()
-        pat = SplitBuf(eng, T, K)
+        pat = SplitBuf(eng, T, K, padded=True)
         ops.patchify(x, ps, pat)
         patch = ops.f32(T, E)
         ops.linear(pat, w["patch"], w["patch.b"], out32=patch, k_w=K)

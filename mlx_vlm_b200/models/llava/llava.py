@@ -126,7 +126,7 @@ class Model:
         ops = TowerOps(eng)
         v = self.config.vision_config
         with torch.cuda.stream(eng.stream):
-            x = pixel_values.to(torch.float32).permute(0, 2, 3, 1).contiguous()   # NHWC, like llava.py:62
+            x = pixel_values.to(torch.float32).permute(0, 2, 3, 1)   # NHWC, like llava.py:62 (a view: patchify takes any strides)
         B = x.shape[0]
         _, _, states = self.vision_tower(x, output_hidden_states=True, feature_layer=self.vision_feature_layer)
         if not isinstance(self.vision_feature_layer, int):
@@ -138,15 +138,11 @@ class Model:
         rows = L - skip
         E, H = v.hidden_size, self.config.text_config.hidden_size
         xs = SplitBuf(eng, B * rows, E)
-        for b in range(B):   # drop the class token of every image (llava.py:66-68)
-            N.check(eng.lib.b200_f32_split(sel[b * L + skip:].data_ptr(), E, xs.t[b * rows:].data_ptr(), xs.ld, xs.n_pad,
-                                           rows, E, eng.s), "f32_split")
+        ops.split_segments(sel, L, skip, xs)     # without the class token of every image (llava.py:66-68)
         mid = SplitBuf(eng, B * rows, H)
         ops.linear(xs, self.proj["linear_1.w"], self.proj["linear_1.b"], out_split=mid, epi=EPI_GELU_EXACT)
-        feats32 = ops.f32(B * rows, H)
-        ops.linear(mid, self.proj["linear_2.w"], self.proj["linear_2.b"], out32=feats32)
         feats = eng.empty((B, rows, H))
-        N.check(eng.lib.b200_cast_f32_bf16(feats32.data_ptr(), feats.data_ptr(), B * rows * H, eng.s), "cast")
+        ops.linear_bf16(mid, self.proj["linear_2.w"], self.proj["linear_2.b"], feats.view(B * rows, H))
         return feats   # astype(inputs_embeds.dtype): the ONE rounding of the vision path (llava.py:101-104)
 
     def get_input_embeddings(self, input_ids=None, pixel_values=None, **kwargs):

@@ -82,8 +82,7 @@ class VisionModel:
         hd = E // nh
         K = ps * ps * C
         w = self.w
-        x = x.contiguous()
-        pat = SplitBuf(eng, B * P, K)
+        pat = SplitBuf(eng, B * P, K, padded=True)
         ops.patchify(x, ps, pat)
         patch = ops.f32(B * P, E)
         ops.linear(pat, w["patch"], None, out32=patch, k_w=K)

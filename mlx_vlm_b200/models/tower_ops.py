@@ -22,12 +22,15 @@ def pad64(n: int) -> int:
 
 
 class SplitBuf:
-    """[T, 2 * n_pad] bf16: hi half at columns [0, n), lo half at [n_pad, n_pad + n); padding is zero."""
+    """[T, 2 * n_pad] bf16: hi half at columns [0, n), lo half at [n_pad, n_pad + n); padding is zero.  Whoever fills the buffer
+    writes all its rows; `padded`: and the padding as well."""
 
-    def __init__(self, eng, T: int, n: int):
+    def __init__(self, eng, T: int, n: int, padded: bool = False):
         self.T, self.n, self.n_pad = T, n, pad64(n)
         with torch.cuda.stream(eng.stream):
-            self.t = torch.zeros((T, 2 * self.n_pad), dtype=torch.bfloat16, device=eng.device)
+            self.t = torch.empty((T, 2 * self.n_pad), dtype=torch.bfloat16, device=eng.device)
+            if n < self.n_pad and not padded:
+                self.t.view(T, 2, self.n_pad)[:, :, n:].zero_()
 
     @property
     def ld(self) -> int:
@@ -70,6 +73,11 @@ class TowerOps:
         N.check(self.lib.b200_f32_split(x.data_ptr(), x.stride(0), out.t.data_ptr(), out.ld, out.n_pad, T, n,
                                         self.eng.s), "f32_split")
 
+    def split_segments(self, x: torch.Tensor, seg_in: int, skip: int, out: SplitBuf):
+        """rows skip .. seg_in - 1 of every seg_in rows of x"""
+        N.check(self.lib.b200_f32_split_segments(x.data_ptr(), x.stride(0), seg_in, skip, seg_in - skip, out.t.data_ptr(), out.ld,
+                                                 out.n_pad, out.T, x.shape[1], self.eng.s), "f32_split_segments")
+
     def linear(self, x: SplitBuf, w: torch.Tensor, bias, *, out32: Optional[torch.Tensor] = None,
                res32: Optional[torch.Tensor] = None, out_split: Optional[SplitBuf] = None, epi: int = EPI_NONE,
                k_w: Optional[int] = None, n_parts: int = 2):
@@ -84,6 +92,11 @@ class TowerOps:
             res32.stride(0) if res32 is not None else 0, N.ptr(out32), out32.stride(0) if out32 is not None else 0,
             N.ptr(out_split.t) if out_split else 0, out_split.ld if out_split else 0,
             out_split.n_pad if out_split else 0, x.T, n_out, k_w, n_parts, epi, mode, self.eng.s), "gemm_wt_f32")
+
+    def linear_bf16(self, x: SplitBuf, w: torch.Tensor, bias, out: torch.Tensor):
+        """y = W . x + bias, rounded once to the bf16 rows of `out`"""
+        N.check(self.lib.b200_gemm_wt_f32_bf16(x.t.data_ptr(), x.ld, w.data_ptr(), w.stride(0), N.ptr(bias), out.data_ptr(),
+                                               out.stride(0), x.T, w.shape[0], x.n, 2, self.eng.s), "gemm_wt_f32_bf16")
 
     def attention(self, q, k, v, *, n_heads: int, n_kv: int, hd: int, Lq: int, S: int, n_seg: int, q_seg: int,
                   k_seg: int, scale: float, out32: Optional[torch.Tensor] = None, out_split: Optional[SplitBuf] = None,
@@ -120,9 +133,10 @@ class TowerOps:
                                                   out.n_pad, self.eng.s), "pixel_shuffle_split")
 
     def patchify(self, pix_nhwc: torch.Tensor, ps: int, out: SplitBuf):
+        """pix_nhwc: fp32 (B, H, W, C), any strides (a view of channel-first pixels is read as it lies); writes `out` with its padding"""
         B, H, W, C = pix_nhwc.shape
-        N.check(self.lib.b200_clip_patchify(pix_nhwc.data_ptr(), B, H, W, C, ps, out.t.data_ptr(), out.n_pad,
-                                            self.eng.s), "clip_patchify")
+        N.check(self.lib.b200_clip_patchify_strided(pix_nhwc.data_ptr(), *pix_nhwc.stride(), B, H, W, C, ps, out.t.data_ptr(), out.n_pad,
+                                                    self.eng.s), "clip_patchify")
 
     def embed(self, patch: torch.Tensor, cls, pos: torch.Tensor, pos_ids, emb: torch.Tensor, B: int, P: int):
         E = patch.shape[1]
