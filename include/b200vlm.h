@@ -59,6 +59,7 @@ int b200_cast_f32_bf16(const float* src, void* dst, long n, void* stream);
 #define B200_WT_SWIGLU 2  /* W = [gate rows; up rows]: C[t][i] = silu(gate) * up, bf16     */
 #define B200_WT_F32 3     /* fp32 output (bias, fp32 activation, fp32 residual): fp32 towers  */
 #define B200_WT_SPLIT 4   /* fp32 result written as [hi | lo] bf16 halves (next GEMM's operand) */
+#define B200_WT_SWIGLU_SPLIT 5 /* W = [gate rows; up rows]: silu(gate) * up in fp32 as [hi | lo] halves */
 #define B200_NORM_NONE 0
 #define B200_NORM_RMS 1   /* mx.fast.rms_norm   (language.py:139-140)                      */
 #define B200_NORM_LN 2    /* mx.fast.layer_norm (vision.py:180-181)                        */
@@ -344,6 +345,9 @@ int b200_f32_gather_rows(const float* in, long ld_in, const int* idx, int n_idx,
 int b200_gemm_wt_f32(const void* X, long ldx, const void* W, long ldw, const void* bias, const float* res32,
                      long ldr32, float* C32, long ldc32, void* Csplit, long ld_split, int n_pad, int T, int N,
                      int K_w, int n_parts, int epilogue, int mode, void* stream);
+/* the same sums (+ bias) of W = [gate; up] ([2 inter, K_w]), Csplit [T, hi | lo] = silu(gate) * up in fp32 (inter % 4 == 0) */
+int b200_gemm_wt_f32_swiglu(const void* X, long ldx, const void* W, long ldw, const void* bias, void* Csplit, long ld_split, int n_pad,
+                            int T, int inter, int K_w, int n_parts, void* stream);
 /* the same sums (+ bias), rounded once to bf16 rows */
 int b200_gemm_wt_f32_bf16(const void* X, long ldx, const void* W, long ldw, const void* bias, void* C, long ldc, int T, int N,
                           int K_w, int n_parts, void* stream);

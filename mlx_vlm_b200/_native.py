@@ -89,6 +89,7 @@ SIGNATURES = {
     "b200_clip_patchify": (_I, [_P, _I, _I, _I, _I, _I, _P, _I, _P]),
     "b200_clip_patchify_strided": (_I, [_P, _L, _L, _L, _L, _I, _I, _I, _I, _I, _P, _I, _P]),
     "b200_f32_split_segments": (_I, [_P, _L, _I, _I, _I, _P, _L, _I, _I, _I, _P]),
+    "b200_gemm_wt_f32_swiglu": (_I, [_P, _L, _P, _L, _P, _P, _L, _I, _I, _I, _I, _I, _P]),
     "b200_gemm_wt_f32_bf16": (_I, [_P, _L, _P, _L, _P, _P, _L, _I, _I, _I, _I, _P]),
     "b200_tower_embed": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _P]),
     "b200_attention_f32": (_I, [_P, _L, _L, _P, _L, _L, _P, _L, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _I, _L, _L,

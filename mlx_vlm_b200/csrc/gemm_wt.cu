@@ -189,7 +189,15 @@ __device__ __forceinline__ void wt_store_tile(const WtParams& p, uint8_t* stg, u
   const int warp = tid >> 5, lane = tid & 31, q = warp & 3, half = warp >> 2;
   const int row = q * 32 + lane;  // weight row of the tile == TMEM lane
   float bias_v = 0.f;
-  if ((TOWER || p.mode == B200_WT_BF16) && p.bias && n0 + row < p.N) bias_v = bf2f(p.bias[n0 + row]);
+  if constexpr (TOWER) {
+    if (p.bias && p.mode == B200_WT_SWIGLU_SPLIT) {   // rows 0..63: gate channels, 64..127: up channels
+      if (n0 + (row & 63) < p.inter) bias_v = bf2f(p.bias[(row >> 6) * p.inter + n0 + (row & 63)]);
+    } else if (p.bias && n0 + row < p.N) {
+      bias_v = bf2f(p.bias[n0 + row]);
+    }
+  } else if (p.mode == B200_WT_BF16 && p.bias && n0 + row < p.N) {
+    bias_v = bf2f(p.bias[n0 + row]);
+  }
   for (int c0 = 0; c0 < p.TN; c0 += WT_EPI_TOK) {
     const int cc = c0 + half * 32;
     if (cc < p.TN && !(p.flags & 1u)) {
@@ -267,6 +275,26 @@ __device__ __forceinline__ void wt_store_tile(const WtParams& p, uint8_t* stg, u
           ov.x = pack2(o[0], o[1]); ov.y = pack2(o[2], o[3]); ov.z = pack2(o[4], o[5]); ov.w = pack2(o[6], o[7]);
           *reinterpret_cast<uint4*>(p.C + (long)t * p.ldc + i) = ov;
         }
+      } else if (TOWER && p.mode == B200_WT_SWIGLU_SPLIT) {
+        // silu(gate) * up in fp32, as the next product's operand: the [T, 2 inter] fp32 rows between the two never reach memory.
+        // 4096 tokens x 28672 rows x 1152 (two parts) with a kernel of its own behind it 399 + 115 us (and 60 to clear its rows), this 396.
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int idx = tid + 256 * u;
+          const int tl = idx >> 4, ch = idx & 15;
+          const int t = t0 + c0 + tl, i = n0 + ch * 4;
+          if (c0 + tl >= p.TN || t >= p.T || i >= p.inter) continue;
+          const float4 g = *reinterpret_cast<const float4*>(stg + (tl * WT_ROWS + ch * 4) * 4);
+          const float4 x = *reinterpret_cast<const float4*>(stg + (tl * WT_ROWS + 64 + ch * 4) * 4);
+          const float v[4] = {g.x * sigmoid_f(g.x) * x.x, g.y * sigmoid_f(g.y) * x.y, g.z * sigmoid_f(g.z) * x.z,
+                              g.w * sigmoid_f(g.w) * x.w};
+          float hi[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) hi[e] = rbf(v[e]);
+          bf16* dh = p.Csplit + (long)t * p.ld_split + i;
+          *reinterpret_cast<uint2*>(dh) = make_uint2(pack2(hi[0], hi[1]), pack2(hi[2], hi[3]));
+          *reinterpret_cast<uint2*>(dh + p.n_pad) = make_uint2(pack2(v[0] - hi[0], v[1] - hi[1]), pack2(v[2] - hi[2], v[3] - hi[3]));
+        }
       } else if constexpr (TOWER) {
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
@@ -331,7 +359,7 @@ __device__ __forceinline__ void wt_store_tile(const WtParams& p, uint8_t* stg, u
 }
 
 // TOWER = false: the bf16 paths (B200_WT_BF16 / PARTIAL / SWIGLU); TOWER = true: the fp32-accurate paths
-// (B200_WT_F32 / SPLIT).  Two instantiations keep each one's code small.
+// (B200_WT_F32 / SPLIT / SWIGLU_SPLIT).  Two instantiations keep each one's code small.
 template <bool TOWER>
 __global__ void __launch_bounds__(256, 2)
 gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
@@ -343,7 +371,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(wt_smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool swiglu = !TOWER && (p.mode == B200_WT_SWIGLU);
+  const bool swiglu = p.mode == (TOWER ? B200_WT_SWIGLU_SPLIT : B200_WT_SWIGLU);
   const int rb = blockIdx.x;
   const int n0 = rb * (swiglu ? 64 : WT_ROWS);  // first output feature (SwiGLU: channel) of the tile
   int n0w = n0;                                 // first weight row of the tile (grouped: inside the tile's group)
@@ -554,7 +582,7 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(wt_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-  const bool swiglu = !TOWER && (p.mode == B200_WT_SWIGLU);
+  const bool swiglu = p.mode == (TOWER ? B200_WT_SWIGLU_SPLIT : B200_WT_SWIGLU);
   const int xhalf = p.TN / 2, stage_bytes = WT_WBLK + xhalf * 128, NS = p.n_stages;
   uint8_t* stg = ring + (long)NS * stage_bytes;
   const int kb_total = (p.K + WT_BK - 1) / WT_BK;
@@ -945,6 +973,7 @@ void gemm_wt_set_pdl(bool on) { g_wt_pdl = on; }
 static int round16(int x) { return (x + 15) & ~15; }
 
 constexpr int WP_PAIRS = 74;   // pairs of SMs
+static bool wt_swiglu(int mode) { return mode == B200_WT_SWIGLU || mode == B200_WT_SWIGLU_SPLIT; }
 static size_t wp_staging(int mode) {   // the epilogue's staging tile: WT_EPI_TOK tokens x 128 rows
   return (size_t)WT_EPI_TOK * WT_ROWS * (mode == B200_WT_BF16 || mode == B200_WT_SWIGLU ? 2 : 4);
 }
@@ -1047,16 +1076,17 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
   B200_REQUIRE(cfg.TN >= 16 && cfg.TN <= 256 && (cfg.TN % (pair ? 32 : 16)) == 0, "gemm_wt: TN=%d", cfg.TN);
   B200_REQUIRE(cfg.KS >= 0 && cfg.stages >= 2 && cfg.stages <= (pair ? WP_MAX_STAGES : WT_MAX_STAGES) && cfg.split >= 1,
                "gemm_wt: bad config KS=%d stages=%d split=%d", cfg.KS, cfg.stages, cfg.split);
-  B200_REQUIRE(mode >= B200_WT_BF16 && mode <= B200_WT_SPLIT, "gemm_wt: mode %d", mode);
-  B200_REQUIRE((mode != B200_WT_F32 && mode != B200_WT_SPLIT) || ext, "gemm_wt: fp32 / split output needs WtExt");
+  B200_REQUIRE(mode >= B200_WT_BF16 && mode <= B200_WT_SWIGLU_SPLIT, "gemm_wt: mode %d", mode);
+  const bool tower = mode == B200_WT_F32 || mode == B200_WT_SPLIT || mode == B200_WT_SWIGLU_SPLIT, swiglu = wt_swiglu(mode);
+  B200_REQUIRE(!tower || ext, "gemm_wt: fp32 / split output needs WtExt");
   B200_REQUIRE(mode != B200_WT_F32 || (ext->C32 && ((uintptr_t)ext->C32 & 15) == 0), "gemm_wt: fp32 output missing / misaligned");
-  B200_REQUIRE(mode != B200_WT_SPLIT || (ext->Csplit && (ext->n_pad % 8) == 0 && (ext->ld_split % 8) == 0 &&
+  B200_REQUIRE((mode != B200_WT_SPLIT && mode != B200_WT_SWIGLU_SPLIT) || (ext->Csplit && (ext->n_pad % 8) == 0 && (ext->ld_split % 8) == 0 &&
                                          ((uintptr_t)ext->Csplit & 15) == 0),
                "gemm_wt: split output missing / misaligned");
   B200_REQUIRE(mode != B200_WT_PARTIAL || partial, "gemm_wt: partial buffer missing");
   B200_REQUIRE(mode == B200_WT_PARTIAL || cfg.split == 1, "gemm_wt: split-K needs the partial mode");
-  B200_REQUIRE(mode != B200_WT_SWIGLU || (inter > 0 && (inter % 8) == 0 && N == 2 * inter),
-               "gemm_wt: SwiGLU needs N == 2 * inter (inter %% 8 == 0)");
+  B200_REQUIRE(!swiglu || (inter > 0 && inter % (tower ? 4 : 8) == 0 && N == 2 * inter),
+               "gemm_wt: SwiGLU needs N == 2 * inter, inter a multiple of 8 (fp32: 4)");
   const int kb_total = cdiv(K, WT_BK);
   WtParams p;
   memset(&p, 0, sizeof(p));
@@ -1095,7 +1125,7 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
   int rc = wt_tmap(W, (long)(ext && ext->ldw > 0 ? ext->ldw : k_w),
                    grouped ? ext->n_groups * N : (heads && !w_cols ? ext->col_groups * N : N),
                    w_cols ? (ext->col_groups - 1) * ext->w_group_cols + k_w : k_w,
-                   mode == B200_WT_SWIGLU ? 64 : WT_ROWS, &tw);
+                   swiglu ? 64 : WT_ROWS, &tw);
   if (rc) return rc;
   if ((rc = wt_tmap(X, ldx, T, heads ? ext->x_cols : K, pair ? cfg.TN / 2 : cfg.TN, &tx))) return rc;
   static unsigned long long set_mask = 0ull;
@@ -1112,7 +1142,7 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
     B200_CUDA(cudaFuncSetAttribute(gemm_wt_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024));
     set_mask |= 1ull << (dev & 63);
   }
-  const int row_blocks = mode == B200_WT_SWIGLU ? cdiv(inter, 64) : cdiv(N, WT_ROWS);
+  const int row_blocks = swiglu ? cdiv(inter, 64) : cdiv(N, WT_ROWS);
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(row_blocks, cdiv(T, cfg.TN) * (heads ? ext->col_groups : 1), splits);
   lc.blockDim = dim3(256);
@@ -1124,7 +1154,7 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
   lc.attrs = at;
   lc.numAttrs = (g_wt_pdl && !grouped) ? 1 : 0;
   if (pair) {
-    const int tiles = cdiv(mode == B200_WT_SWIGLU ? 2 * inter : N, 2 * WT_ROWS) * cdiv(T, cfg.TN) * splits;
+    const int tiles = cdiv(swiglu ? 2 * inter : N, 2 * WT_ROWS) * cdiv(T, cfg.TN) * splits;
     lc.gridDim = dim3(2 * (tiles < WP_PAIRS ? tiles : WP_PAIRS));
     lc.blockDim = dim3(WP_THREADS);
     cudaLaunchAttribute pa[2];
@@ -1134,11 +1164,11 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
     pa[1] = at[0];
     lc.attrs = pa;
     lc.numAttrs = g_wt_pdl ? 2 : 1;
-    if (mode == B200_WT_F32 || mode == B200_WT_SPLIT) B200_CUDA(cudaLaunchKernelEx(&lc, gemm_wt_pair_kernel<true>, tw, tx, p));
+    if (tower) B200_CUDA(cudaLaunchKernelEx(&lc, gemm_wt_pair_kernel<true>, tw, tx, p));
     else B200_CUDA(cudaLaunchKernelEx(&lc, gemm_wt_pair_kernel<false>, tw, tx, p));
     return B200_OK;
   }
-  if (mode == B200_WT_F32 || mode == B200_WT_SPLIT) {
+  if (tower) {
     B200_CUDA(cudaLaunchKernelEx(&lc, gemm_wt_kernel<true>, tw, tx, p));
   } else {
     B200_CUDA(cudaLaunchKernelEx(&lc, gemm_wt_kernel<false>, tw, tx, p));
@@ -1196,7 +1226,7 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
                   const WtExt* ext) {
   static std::unordered_map<TuneKey, WtConfig, TuneHash> cache;
   static std::mutex mu;
-  const int row_blocks = mode == B200_WT_SWIGLU ? cdiv(inter, 64) : cdiv(N, WT_ROWS);
+  const int row_blocks = wt_swiglu(mode) ? cdiv(inter, 64) : cdiv(N, WT_ROWS);
   const int kb_total = cdiv(K, WT_BK);
   int dev = 0;
   B200_CUDA(cudaGetDevice(&dev));
@@ -1285,7 +1315,7 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
     }
     // CTA pairs (KS = 0) from about a wave of them on: the token tile whose last wave is fullest, the next best, and 256
     if (T >= 192 && !(ext && (ext->tile_group || ext->col_groups > 0))) {
-      const int pair_rows = cdiv(mode == B200_WT_SWIGLU ? 2 * inter : N, 2 * WT_ROWS);
+      const int pair_rows = cdiv(wt_swiglu(mode) ? 2 * inter : N, 2 * WT_ROWS);
       auto add_pair = [&](int tn, int split) {
         const int stage = WT_WBLK + tn * 64;
         int stg = (int)((226 * 1024 - 1024 - wp_staging(mode)) / stage);

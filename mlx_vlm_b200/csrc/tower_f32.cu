@@ -531,6 +531,16 @@ int b200_gemm_wt_f32(const void* X, long ldx, const void* W, long ldw, const voi
   return gemm_wt_tuned(X, ldx, W, bias, nullptr, 0, nullptr, 0, nullptr, 0, T, N, n_parts * kbw * 64, epilogue, mode, 0,
                        false, 148, nullptr, (cudaStream_t)stream, &ext);
 }
+int b200_gemm_wt_f32_swiglu(const void* X, long ldx, const void* W, long ldw, const void* bias, void* Csplit, long ld_split, int n_pad,
+                            int T, int inter, int K_w, int n_parts, void* stream) {
+  B200_REQUIRE(X && W && Csplit && n_parts >= 1, "gemm_wt_f32_swiglu: bad argument");
+  const int kbw = cdiv(K_w, 64);
+  WtExt ext;
+  memset(static_cast<void*>(&ext), 0, sizeof(ext));
+  ext.kb_w = kbw; ext.k_w = K_w; ext.ldw = ldw; ext.Csplit = (bf16*)Csplit; ext.ld_split = ld_split; ext.n_pad = n_pad;
+  return gemm_wt_tuned(X, ldx, W, bias, nullptr, 0, nullptr, 0, nullptr, 0, T, 2 * inter, n_parts * kbw * 64, B200_EPI_NONE,
+                       B200_WT_SWIGLU_SPLIT, inter, false, 148, nullptr, (cudaStream_t)stream, &ext);
+}
 /* the same product as b200_gemm_wt_f32 (fp32 sums of n_parts parts, + bias), rounded once to bf16 rows */
 int b200_gemm_wt_f32_bf16(const void* X, long ldx, const void* W, long ldw, const void* bias, void* C, long ldc, int T, int N, int K_w,
                           int n_parts, void* stream) {

@@ -85,10 +85,8 @@ class Connector:
         # ---- modality projection: x = down(silu(gate f) * up f)
         fs = SplitBuf(eng, n_img * P, E)
         ops.split(feats, fs)
-        gu = ops.f32(n_img * P, 2 * I)
-        ops.linear(fs, w["mp.gu"], None, out32=gu)
         act = SplitBuf(eng, n_img * P, I)
-        ops.swiglu(gu, act)
+        ops.linear_swiglu(fs, w["mp.gu"], None, act)
         x = ops.f32(n_img * P, H)
         ops.linear(act, w["mp.down"], None, out32=x)
         # ---- perceiver resampler: latents attend to [context; latents]
@@ -103,7 +101,6 @@ class Connector:
         kv32 = ops.f32(n_img * S, 2 * nkv * hd)
         o = SplitBuf(eng, n_img * nl, nh * hd)
         y = SplitBuf(eng, n_img * nl, H)
-        gu2 = ops.f32(n_img * nl, 8 * H)
         act2 = SplitBuf(eng, n_img * nl, 4 * H)
         for i in range(pc.resampler_depth):
             ops.rms_norm(h, w[f"{i}.ln_lat"], eps, out_split=lat)
@@ -116,8 +113,7 @@ class Connector:
                           out_split=o)
             ops.linear(o, w[f"{i}.o"], None, out32=h, res32=h)
             ops.rms_norm(h, w[f"{i}.ln_post"], eps, out_split=y)
-            ops.linear(y, w[f"{i}.gu"], None, out32=gu2)
-            ops.swiglu(gu2, act2)
+            ops.linear_swiglu(y, w[f"{i}.gu"], None, act2)
             ops.linear(act2, w[f"{i}.down"], None, out32=h, res32=h)
         out = ops.f32(n_img * nl, H)
         ops.rms_norm(h, w["norm"], eps, out32=out)

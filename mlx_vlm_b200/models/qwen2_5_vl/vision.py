@@ -150,7 +150,7 @@ class VisionModel:
         h = ops.f32(T, E)
         ops.linear(pat, w["patch"], None, out32=h, k_w=K, n_parts=1)   # pixels rounded to bf16 (qwen2_5_vl.py: astype)
         y, o, act = SplitBuf(eng, T, E), SplitBuf(eng, T, E), SplitBuf(eng, T, I)
-        qkv, gu = ops.f32(T, 3 * E), ops.f32(T, 2 * I)
+        qkv = ops.f32(T, 3 * E)
         win_max, frm_max = int(np.diff(windows).max()), int(np.diff(frames).max())
         for i in range(c.depth):
             full = i in c.fullatt_block_indexes
@@ -163,8 +163,7 @@ class VisionModel:
                                  max_len=frm_max if full else win_max, scale=hd ** -0.5, out_split=o)
             ops.linear(o, w[f"{i}.proj.w"], w[f"{i}.proj.b"], out32=h, res32=h)
             ops.rms_norm(h, w[f"{i}.n2"], 1e-6, out_split=y)
-            ops.linear(y, w[f"{i}.gu.w"], w[f"{i}.gu.b"], out32=gu)
-            ops.swiglu(gu, act)
+            ops.linear_swiglu(y, w[f"{i}.gu.w"], w[f"{i}.gu.b"], act)
             ops.linear(act, w[f"{i}.down.w"], w[f"{i}.down.b"], out32=h, res32=h)
         Tm, Em = T // unit, E * unit
         n32 = ops.f32(T, E)

@@ -63,11 +63,6 @@ class TowerOps:
                                            out_split.n_pad if out_split else 0, T, n, seg_in, seg_out, seg_off,
                                            self.eng.s), "f32_rms_norm")
 
-    def swiglu(self, gu: torch.Tensor, out: SplitBuf):
-        T = gu.shape[0]
-        N.check(self.lib.b200_f32_swiglu_split(gu.data_ptr(), gu.stride(0), out.t.data_ptr(), out.ld, out.n_pad, T,
-                                               out.n, self.eng.s), "f32_swiglu")
-
     def split(self, x: torch.Tensor, out: SplitBuf):
         T, n = x.shape
         N.check(self.lib.b200_f32_split(x.data_ptr(), x.stride(0), out.t.data_ptr(), out.ld, out.n_pad, T, n,
@@ -92,6 +87,11 @@ class TowerOps:
             res32.stride(0) if res32 is not None else 0, N.ptr(out32), out32.stride(0) if out32 is not None else 0,
             N.ptr(out_split.t) if out_split else 0, out_split.ld if out_split else 0,
             out_split.n_pad if out_split else 0, x.T, n_out, k_w, n_parts, epi, mode, self.eng.s), "gemm_wt_f32")
+
+    def linear_swiglu(self, x: SplitBuf, w: torch.Tensor, bias, out: SplitBuf):
+        """silu(gate) * up in fp32 as a split operand, [gate | up] = W . x + bias"""
+        N.check(self.lib.b200_gemm_wt_f32_swiglu(x.t.data_ptr(), x.ld, w.data_ptr(), w.stride(0), N.ptr(bias), out.t.data_ptr(), out.ld,
+                                                 out.n_pad, x.T, out.n, x.n, 2, self.eng.s), "gemm_wt_f32_swiglu")
 
     def linear_bf16(self, x: SplitBuf, w: torch.Tensor, bias, out: torch.Tensor):
         """y = W . x + bias, rounded once to the bf16 rows of `out`"""

@@ -89,3 +89,28 @@ def test_sums_rounded_once(eng, T, n, K):
     torch.cuda.synchronize()
     assert ((o16.float() - o32).abs() <= 2.0 ** -8 * o32.abs() + 1e-5).all()
     assert (o16 != o32.to(torch.bfloat16)).float().mean() < 0.01
+
+
+@pytest.mark.parametrize("T", [1, 63, 130, 600, 2500])
+@pytest.mark.parametrize("inter,K,bias", [(64, 64, False), (132, 200, True), (4, 128, True), (3420, 1280, True), (1000, 320, False)])
+def test_swiglu_in_the_product(eng, T, inter, K, bias):
+    """against float64 on the same operands.  x keeps 16 mantissa bits (2^-17 of each term), the sums are fp32 (truncated: 2^-23
+    a step), the logistic function is good to a few fp32 ulps, the result keeps 16 mantissa bits"""
+    from mlx_vlm_b200.models.tower_ops import SplitBuf, TowerOps
+    g = torch.Generator(device="cuda").manual_seed(T + inter)
+    ops, x = TowerOps(eng), torch.randn(T, K, device="cuda", generator=g)
+    w = (torch.randn(2 * inter, K, device="cuda", generator=g) * K ** -0.5).to(torch.bfloat16)
+    b = torch.randn(2 * inter, device="cuda", generator=g).to(torch.bfloat16) if bias else None
+    sp, out = SplitBuf(eng, T, K), SplitBuf(eng, T, inter)
+    ops.split(x, sp)
+    ops.linear_swiglu(sp, w, b, out)
+    torch.cuda.synchronize()
+    wd, bd = w.double(), b.double() if bias else torch.zeros(2 * inter, device="cuda", dtype=torch.float64)
+    y, size = x.double() @ wd.T + bd, x.double().abs() @ wd.abs().T + bd.abs()
+    gate, up = y[:, :inter], y[:, inter:]
+    want = torch.nn.functional.silu(gate) * up
+    err = (2.0 ** -17 + (K / 16 + 8) * 2.0 ** -23) * size          # of the two sums
+    bound = 1.1 * err[:, :inter] * (up.abs() + err[:, inter:]) + gate.abs() * err[:, inter:] + 2.0 ** -16 * want.abs() + 1e-30
+    both, raw = _parts(out)
+    assert bool(((both - want).abs() <= bound).all())
+    assert not raw[:, inter:out.n_pad].any() and not raw[:, out.n_pad + inter:].any()
