@@ -106,6 +106,32 @@ __device__ __forceinline__ float warp_max(float v) {
 // bf16 caller applies next and below the 2^-17 of the split-operand GEMMs on the fp32 paths (the libm expf + IEEE
 // division version has a slow-path branch per element and cost ~9 us per GEMM epilogue)
 __device__ __forceinline__ float sigmoid_f(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
+// The same of a pair: one packed multiplication and addition, an exponential and a reciprocal each (results below 2^-126 are 0)
+__device__ __forceinline__ uint64_t sigmoid2(uint64_t x) {
+  const uint64_t t = mul2(x, f2(-1.4426950408889634f, -1.4426950408889634f));
+  float a, b;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(f2_lo(t)));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(b) : "f"(f2_hi(t)));
+  const uint64_t d = add2(f2(a, b), f2(1.f, 1.f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(f2_lo(d)));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(b) : "f"(f2_hi(d)));
+  return f2(a, b);
+}
+// of bf16 pairs: a product of two bf16 is exact in fp32, so the packed multiplication rounds where rbf(a * b) does
+__device__ __forceinline__ uint32_t mul_bf2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t unpack_bf2(uint32_t x) { return f2(__uint_as_float(x << 16), __uint_as_float(x & 0xffff0000u)); }
+__device__ __forceinline__ uint32_t pack_bf2(uint64_t x) { return pack2(f2_lo(x), f2_hi(x)); }
+// swiglu_bf and gelu_fast_bf of bf16 pairs, the same roundings
+__device__ __forceinline__ uint32_t swiglu_bf2(uint32_t g, uint32_t u) {
+  return mul_bf2(mul_bf2(g, pack_bf2(sigmoid2(unpack_bf2(g)))), u);
+}
+__device__ __forceinline__ uint32_t gelu_fast_bf2(uint32_t x) {
+  return mul_bf2(x, pack_bf2(sigmoid2(unpack_bf2(mul_bf2(x, 0x3FDA3FDAu)))));   // 1.703125
+}
 // nn.silu(g) * u : three roundings
 __device__ __forceinline__ float swiglu_bf(float g, float u) {
   float s = rbf(g * rbf(sigmoid_f(g)));
