@@ -134,6 +134,10 @@ int launch_res(const bf16* W, const bf16* x, bf16* h, int N, int K, cudaStream_t
 int launch_gateup(const DecodeDims& d, const LayerW& lw, const bf16* h, bf16* act, cudaStream_t s);
 int launch_head(const DecodeDims& d, const bf16* norm_w, const bf16* E, const bf16* h,
                 bf16* logits, float2* partials, cudaStream_t s);
+// the first tokens of `rows` prompts from their logits [rows][ldv] (bf16), appended to the token log in order; tail: the last of
+// them is what the engine goes on from (logits, logprobs, next token and its embedding, as launch_sample leaves them)
+int launch_rows_sample(const DecodeDims& d, const bf16* rows_logits, long ldv, int rows, bool tail, bf16* logits, bf16* logprobs,
+                       const bf16* E, bf16* h, DecState* st, int* token_log, int log_cap, cudaStream_t s);
 int launch_sample(const DecodeDims& d, const bf16* logits, const float2* partials, bf16* logprobs,
                   const bf16* E, bf16* h, DecState* st, int* token_log, int log_cap,
                   const int* force_tokens, int advance, cudaStream_t s);
@@ -152,7 +156,8 @@ struct KvRef {
 int cast_f32_bf16(const float* src, void* dst, long n, cudaStream_t st);
 int layer_norm(const void* x, const void* w, const void* b, void* y, int rows, int dim, float eps,
                cudaStream_t st);
-int rms_norm(const void* x, const void* w, void* y, int rows, int dim, float eps, cudaStream_t st);
+int rms_norm(const void* x, const void* w, void* y, int rows, int dim, float eps, cudaStream_t st,
+             const int* map = nullptr);   // map: row i of y is row map[i] of x
 int vision_rope(void* qkv, const int* pos_hw, const float* inv_freq, int n_tok, int n_heads,
                 int hd, cudaStream_t st);
 int mrope_kv_write(void* qkv, const int* pos3, const float* inv_freq, const int* axis_sel,

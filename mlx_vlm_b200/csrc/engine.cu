@@ -1086,8 +1086,8 @@ int b200_engine_prefill(b200_engine* e, const void* embeds, const int* pos3, int
 // PromptProcessingBatch (ar.py:1581-2175): n_seq FRESH prompts prefilled in one pass.  embeds = the sequences'
 // embeddings concatenated along the token axis, EACH SEQUENCE PADDED TO A MULTIPLE OF 8 TOKENS (any finite values in
 // the padding rows): [sum round8(T_g), hidden]; pos3 = (3, sum round8(T_g)) int32 device, laid out the same way;
-// sequence g has seq_len[g] real tokens and fills KV pool row rows[g] from position 0.  The first token of every sequence goes through
-// the fused head + sampler in order: token_log receives n_seq entries (tokens_launched += n_seq).
+// sequence g has seq_len[g] real tokens and fills KV pool row rows[g] from position 0.  The first tokens of the sequences come
+// from one product with the head: token_log receives n_seq entries in their order (tokens_launched += n_seq).
 int b200_engine_prefill_batch(b200_engine* e, const void* embeds, const int* pos3, int n_seq, const int* seq_len,
                               const int* rows, void* stream) {
   B200_REQUIRE(e && embeds && pos3 && n_seq > 0 && seq_len && rows, "engine_prefill_batch: bad arguments");
@@ -1125,8 +1125,14 @@ int b200_engine_prefill_batch(b200_engine* e, const void* embeds, const int* pos
     }
   for (int g = 0; g < n_seq; ++g)   // attention segments (q0, Lq, k0, S), 16-byte aligned behind the table (T % 8 == 0)
     for (int v : {segs[g].off, segs[g].T, segs[g].off, segs[g].T}) loc.push_back(v);
+  const size_t last_at = loc.size();   // and the last row of every sequence
+  for (int g = 0; g < n_seq; ++g) loc.push_back(segs[g].off + segs[g].T - 1);
   if ((rc = upload_loc(e, loc, s))) return rc;
   rc = prefill_layers_v2_body(e, pos_stage, (int)T, 0, nullptr, s, segs.data(), n_seq, e->loc_dev);
+  // first token of every sequence: the final norm of its last row (into the normed rows' buffer, which nothing reads any more), ONE
+  // product with the head for as many rows as the partial region takes logits of, and a sampler with a CTA per row
+  bf16* last_rows = (bf16*)(e->ws + align256(T * H * 2));
+  if (!rc) rc = rms_norm(h, e->norm, last_rows, n_seq, (int)H, c.rms_eps, s, e->loc_dev + last_at);
   B200_CUDA(cudaEventRecord(e->loc_ev, s));   // the table (and its staging copy) may be rewritten after this point
   if (rc) return rc;
   const DecodeDims d = e->dims();
@@ -1135,16 +1141,21 @@ int b200_engine_prefill_batch(b200_engine* e, const void* embeds, const int* pos
     e->prepared_cap = e->kv_cap;
     e->prepared_cluster = e->attn_cluster;
   }
-  for (int g = 0; g < n_seq; ++g) {   // first token of every sequence: fused head + sampler on its last row
-    if ((rc = launch_set_state(e->st, 0, segs[g].T, segs[g].T, 0, 0, e->embed, e->h, c.hidden, s))) return rc;
-    if ((rc = launch_head(d, e->norm, e->head, h + (long)(segs[g].off + segs[g].T - 1) * H, e->logits, e->partials, s)))
+  if ((rc = launch_set_state(e->st, 0, segs[n_seq - 1].T, segs[n_seq - 1].T, 0, 0, e->embed, e->h, c.hidden, s))) return rc;
+  const long ldv = round8(c.vocab);
+  bf16* rows_logits = (bf16*)ws_partial(e);
+  const int most = (int)std::min<long>(n_seq, WT_PARTIAL_BYTES / (ldv * 2));
+  B200_REQUIRE(most > 0, "engine_prefill_batch: a vocabulary of %d", c.vocab);
+  for (int g = 0; g < n_seq; g += most) {
+    const int n = std::min(most, n_seq - g);
+    if ((rc = v2_linear(e, last_rows + (long)g * H, H, e->head, nullptr, rows_logits, ldv, n, c.vocab, (int)H, B200_EPI_NONE, s))) return rc;
+    if ((rc = launch_rows_sample(d, rows_logits, ldv, n, g + n == n_seq, e->logits, e->logprobs, e->embed, e->h, e->st, e->token_log,
+                                 e->log_cap, s)))
       return rc;
-    if ((rc = launch_sample(d, e->logits, e->partials, e->logprobs, e->embed, e->h, e->st, e->token_log, e->log_cap,
-                            e->force, 0, s)))
-      return rc;
-    e->launches += 3;
-    e->tokens_launched += 1;
+    e->launches += 1;
   }
+  e->launches += 2;
+  e->tokens_launched += n_seq;
   e->ctx_host = segs[n_seq - 1].T;
   e->pos_host = segs[n_seq - 1].T;
   return B200_OK;

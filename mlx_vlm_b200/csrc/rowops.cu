@@ -79,13 +79,14 @@ __global__ void layer_norm_kernel(const bf16* __restrict__ x, const bf16* __rest
 }
 
 // mx.fast.rms_norm CPU fallback: bf16(x * rsqrt(mean(x^2)+eps)) then * w (round).
+// map (optional): row i of y is row map[i] of x
 __global__ void rms_norm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
-                                bf16* __restrict__ y, int rows, int dim, float eps) {
+                                bf16* __restrict__ y, int rows, int dim, float eps, const int* __restrict__ map) {
   pdl_prologue();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= rows) return;
-  const bf16* xr = x + (long)warp * dim;
+  const bf16* xr = x + (long)(map ? map[warp] : warp) * dim;
   bf16* yr = y + (long)warp * dim;
   const int nvec = dim >> 3;
   float s = 0.f;
@@ -402,10 +403,10 @@ int layer_norm(const void* x, const void* w, const void* b, void* y, int rows, i
 }
 
 int rms_norm(const void* x, const void* w, void* y, int rows, int dim, float eps,
-             cudaStream_t st) {
+             cudaStream_t st, const int* map) {
   B200_REQUIRE(rows > 0 && dim > 0 && (dim % 8) == 0 && w, "rms_norm: rows=%d dim=%d", rows, dim);
   B200_CUDA(launch_pdl(rms_norm_kernel, dim3(cdiv(rows, 8)), dim3(256), 0, st, (const bf16*)x, (const bf16*)w,
-                       (bf16*)y, rows, dim, eps));
+                       (bf16*)y, rows, dim, eps, map));
   return B200_OK;
 }
 

@@ -277,3 +277,38 @@ def test_batched_prefill_equals_single_prefills():
             assert rl2(k2, k1) <= 1e-3 and rl2(v2, v1) <= 1e-3, (b, layer, rl2(k2, k1), rl2(v2, v1))
         assert _token_ok(toks[b], singles[b][2]), (b, toks[b], firsts[b])
     print("batched prefill first tokens", toks, "single", firsts)
+
+
+@pytest.mark.parametrize("n", [1, 2, 5])
+def test_first_tokens_of_a_batched_prefill(n):
+    """what the engine goes on from after a batched prefill is its last prompt: logits, log-probabilities, next token and its
+    embedding as after that prompt alone; every prompt's token is the one that its own logits give; the log grows by n"""
+    c, W, model, req = _build("wide2", 10, (56, 56))
+    lm, eng = model.language_model, model.engine
+    reqs = (_requests(c, req, 4) + _requests(c, req, 2))[:n]
+    embs, lps, lgs = [], [], []
+    for ids, kw, _ in reqs:
+        emb = model.get_input_embeddings(ids, kw.get("pixel_values"), image_grid_thw=kw.get("image_grid_thw"))
+        cache = lm.make_cache()
+        lm._rope_deltas, lm._position_ids = None, None
+        lm(ids, inputs_embeds=emb.inputs_embeds, cache=cache, position_ids=emb.position_ids, rope_deltas=emb.rope_deltas, logits_to_keep=1)
+        eng.stream.synchronize()
+        embs.append(emb)
+        lps.append(eng.logprobs_view().float().cpu().clone())
+        lgs.append(eng.snapshot("logits").float().cpu().reshape(-1).clone())
+    rows, _ = lm.make_batch_cache(n, 256)
+    start = eng.tokens_launched
+    toks = lm.prefill_rows([r[0] for r in reqs], [e.inputs_embeds for e in embs], [lm.make_cache_row(rows.pool, b) for b in range(n)],
+                           [e.position_ids for e in embs], [e.rope_deltas for e in embs], reserve_tokens=256)
+    eng.stream.synchronize()
+    assert eng.tokens_launched == start + n
+    log = eng.token_log_view()
+    assert [int(log[(start + i) % eng.token_log_capacity]) for i in range(n)] == toks
+    for b in range(n):
+        assert _token_ok(toks[b], lps[b]), (b, toks[b])
+    lg, lp = eng.snapshot("logits").float().cpu().reshape(-1), eng.logprobs_view().float().cpu()
+    assert rl2(lg, lgs[-1]) <= 5e-3 and float((lp - lps[-1]).abs().max()) <= 0.07     # a bf16 unit of a number below 16
+    assert toks[-1] == int(torch.argmax(lp.reshape(-1)[:lg.numel()]))
+    want = lg - torch.logsumexp(lg.double(), 0).float()
+    assert float((lp.reshape(-1)[:lg.numel()] - want).abs().max()) <= 0.13             # lse and the difference are rounded to bf16
+    assert eng.device_error() == 0

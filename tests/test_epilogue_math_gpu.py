@@ -29,11 +29,13 @@ def _sigmoid(x):
 
 
 def _close(got, want):
-    """the exponential and the reciprocal err by some 2^-22: where the logistic function lies that close to the middle of two bf16
-    numbers it may round the other way, one unit; numbers below 2^-120 are left to the flushed range"""
+    """The exponential and the reciprocal err by some 2^-22 (more where the exponent is large: 2^-24 of it): where the logistic function
+    lies that close to the middle of two bf16 numbers it may round the other way, one unit (2^-7 at most), which the one or two
+    products behind it hand on and may round once more each: below 2^-6.  A logistic function below 2^-126 counts as 0: it
+    belongs to arguments between 87 and 89, so 3 x 89 x 2^-126 < 2^-117 of the result."""
     g, w = got.double(), want.double()
-    assert bool(((g - w).abs() <= 2.0 ** -7 * w.abs() + 2.0 ** -120).all())
-    assert float((g != w).double().mean()) < 2e-3
+    assert bool(((g - w).abs() <= 2.0 ** -6 * w.abs() + 2.0 ** -117).all())
+    assert float((g != w).double().mean()) < 5e-3
 
 
 @pytest.mark.parametrize("pair", [False, True])
