@@ -16,11 +16,17 @@
 //               the waits of one product (0.2 us of 0.5, ready or not) pass while another thread's keeps the tensor core busy
 //   warps 2..17 softmax: two groups of eight warps that take the key tiles in turn, each with a score tile and a P tile
 //               of its own; two threads per query row (64 score columns each), TMEM -> registers,
-//               pass 1: running max / sum of exp;  pass 2: p -> shared memory (the A operand)
+//               pass 1: running max / sum of exp;  pass 2: p -> tensor memory (the A operand)
 // V is read as it lies in the qkv buffer or the KV cache ([key][dim]): the B operand of P.V is then MN-major (dims
 // contiguous), which tcgen05 takes from the same 128-byte-swizzled 64-dim blocks that K uses.  So nothing transposes V:
 // a segment may start at any token (keys are a TMA coordinate without an alignment rule) and a later portion of a prompt
 // reads the cached keys and values where they are.  (V^T, [head][dim][key], is still taken by b200_attention_fa.)
+// A tile's time, from clock stamps (28 heads of 128): 1330 cycles in pass 1, of which the exponentials' 1024 are one part and
+// the two groups' loads and waits, which fall together, the other; 1450 in pass 2, where the thread that issues P.V is the
+// chain: 8 products of 64 cycles beside Q.K^T's, a wait for P and one for V.  With P in tensor memory instead of shared
+// memory, three key slots in the room that this gives, one commit for the value slot and the P tile, and half tiles that a
+// warp's rows do not see left out: 2048 queries behind 2048 keys, 28 heads, 168.5 -> 164 us; 8 prompts of 608, 32 heads, 120 ->
+// 117.6; four pictures and a clip (6012 patches, 16 heads of 80) 131.5 -> 130.
 // Measured against the kernel without TMA that such calls fell back to (attention_tc.cu): 2048 queries behind 2048 cached
 // keys, 28 heads of 128: 1094 -> 354 us (249 with the pairwise softmax below); four pictures and a clip of four frames (6012
 // patches, 16 heads of 80), which start at odd offsets: 773 us in eight launches -> 236 us in one.
@@ -37,6 +43,8 @@ namespace {
 constexpr int FA_TQ = 128, FA_TK = 128;
 constexpr int FA_BLK = 16 * 1024;       // one 128-row x 64-column bf16 operand block
 constexpr int FA_THREADS = 640;         // producer warp, 3 MMA warps, 2 groups of 8 softmax warps
+constexpr int FA_NK = 3, FA_NV = 2;     // ring slots of key and of value tiles (a value slot and a P tile are free at the same time)
+constexpr uint32_t FA_O0 = 256, FA_P0 = 384;   // TMEM columns: scores 2 x 128 | O 128 | P 2 x 64 (two bf16 a column)
 
 struct FaParams {
   bf16* out;
@@ -49,8 +57,7 @@ struct FaParams {
 };
 
 struct FaBars {
-  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], s_empty[2], p_full[2], p_empty[2],
-      o_full, dropped, drained[3];
+  uint64_t q_full, k_full[FA_NK], k_empty[FA_NK], v_full[FA_NV], s_full[2], s_empty[2], p_full[2], pv_done[2], o_full, dropped, drained[3];
 };
 
 __device__ __forceinline__ uint32_t f_u32(const void* p) {
@@ -87,6 +94,24 @@ __device__ __forceinline__ void f_umma(uint32_t tmem_d, uint32_t a_lo, uint32_t 
       "setp.ne.b32 p, %5, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(tmem_d),
       "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// A (here P) in tensor memory
+__device__ __forceinline__ void f_umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void f_st16(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"r"(r[0]),
+      "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
       : "memory");
 }
 __device__ __forceinline__ void f_commit(uint64_t* bar) {
@@ -173,10 +198,9 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(fa_smem_raw) + 1023) &
                                            ~static_cast<uintptr_t>(1023));
   uint8_t* Qs = sm;                          // [128 q][128 d]            2 k-blocks
-  uint8_t* Ks = sm + 2 * FA_BLK;             // 2 slots x [128 keys][128 d]
-  uint8_t* Vs = sm + 6 * FA_BLK;             // 2 slots x (VT: 2 key-blocks x [hdp d][64 keys], else 2 dim-blocks x [128 keys][64 d])
-  uint8_t* Ps = sm + 10 * FA_BLK;            // 2 slots x [128 q][128 keys]
-  float2* stat = reinterpret_cast<float2*>(Ps);   // [2 groups x 2 halves][128 q], between the passes
+  uint8_t* Ks = sm + 2 * FA_BLK;             // FA_NK slots x [128 keys][128 d]
+  uint8_t* Vs = Ks + 2 * FA_NK * FA_BLK;     // FA_NV slots x (VT: 2 key-blocks x [hdp d][64 keys], else 2 dim-blocks x [128 keys][64 d])
+  float2* stat = reinterpret_cast<float2*>(Vs + 2 * FA_NV * FA_BLK);   // [2 groups x 2 halves][128 q], between the passes
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = blockIdx.x, kvh = h / (p.n_heads / p.n_kv);
   // causal: the query tiles with the most keys start first, of all heads, so that the short ones fill the last wave
@@ -194,15 +218,16 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmK)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmV)) : "memory");
     f_init(&bars.q_full, 1);
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < FA_NK; ++i) {
       f_init(&bars.k_full[i], 1);
       f_init(&bars.k_empty[i], 1);
-      f_init(&bars.v_full[i], 1);
-      f_init(&bars.v_empty[i], 1);
+    }
+    for (int i = 0; i < FA_NV; ++i) f_init(&bars.v_full[i], 1);
+    for (int i = 0; i < 2; ++i) {
       f_init(&bars.s_full[i], 1);
       f_init(&bars.s_empty[i], 256);
       f_init(&bars.p_full[i], 256);
-      f_init(&bars.p_empty[i], 1);
+      f_init(&bars.pv_done[i], 1);
     }
     f_init(&bars.o_full, 1);
     f_init(&bars.dropped, 1);
@@ -230,7 +255,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       for (int c = 0; c < kbq; ++c) f_tma_3d(Qs + c * FA_BLK, &tmQ, &bars.q_full, c * 64, h, p.q0 + row0);
       auto load_v = [&](int j) {
         const int sv = j & 1;
-        if (!mbar_wait(&bars.v_empty[sv], ((j >> 1) & 1) ^ 1, &failed)) return false;
+        if (!mbar_wait(&bars.pv_done[sv], ((j >> 1) & 1) ^ 1, &failed)) return false;
         ++v_loads;
         if constexpr (VT) {
           f_expect_tx(&bars.v_full[sv], 2u * (uint32_t)vblk);
@@ -245,14 +270,16 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       };
       int jk = 0;   // key tile of step i
       bool ok = true;
+      int s = 0;
+      uint32_t free_par = 1;
       for (int i = 0; i < 2 * n_tiles && ok; ++i) {
-        const int s = i & 1;
-        if (!(ok = mbar_wait(&bars.k_empty[s], ((i >> 1) & 1) ^ 1, &failed))) break;
+        if (!(ok = mbar_wait(&bars.k_empty[s], free_par, &failed))) break;
         ++k_loads;
         f_expect_tx(&bars.k_full[s], (uint32_t)kbq * FA_BLK);
         for (int c = 0; c < kbq; ++c)
           f_tma_3d(Ks + s * 2 * FA_BLK + c * FA_BLK, &tmK, &bars.k_full[s], c * 64, kvh, p.k0 + jk * FA_TK);
         if (++jk == n_tiles) jk = 0;
+        if (++s == FA_NK) s = 0, free_par ^= 1;
         if (i >= n_tiles + 2) ok = load_v(i - n_tiles - 2);   // (in the order of the products: a wait for V holds up no K before it)
       }
       for (int j = max(0, n_tiles - 2); j < n_tiles && ok; ++j) ok = load_v(j);
@@ -261,11 +288,14 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (lane == 0) {  // ===== issuer of Q.K^T, of every other step =====
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(FA_TK >> 3) << 17) | (8u << 24);
       const int ksteps = p.hdp >> 4, s = warp == 1 ? 0 : 1;
-      const uint32_t q_lo = f_desc_lo(f_u32(Qs)), k_lo = f_desc_lo(f_u32(Ks + s * 2 * FA_BLK)), d = tmem + (uint32_t)s * 128u;
+      const uint32_t q_lo = f_desc_lo(f_u32(Qs)), k_first = f_desc_lo(f_u32(Ks)), d = tmem + (uint32_t)s * 128u;
       bool dead = false;
+      int sk = s;           // ring slot of step i and the parity of its round
+      uint32_t k_par = 0;
       mbar_wait_issuer(&bars.q_full, 0, dead);
       for (int i = s; i < 2 * n_tiles; i += 2) {
-        mbar_wait_issuer(&bars.k_full[s], (i >> 1) & 1, dead);
+        const uint32_t k_lo = k_first + (uint32_t)(sk * 2 * (FA_BLK >> 4));
+        mbar_wait_issuer(&bars.k_full[sk], k_par, dead);
         mbar_wait_issuer(&bars.s_empty[s], ((i >> 1) & 1) ^ 1, dead);
         f_fence_after();
 #pragma unroll
@@ -274,8 +304,9 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           const uint32_t off = (uint32_t)((ks >> 2) * (FA_BLK >> 4) + (ks & 3) * 2);
           f_umma(d, q_lo + off, k_lo + off, F_DESC_HI, idesc_s, ks > 0 ? 1u : 0u);
         }
-        f_commit(dead ? &bars.dropped : &bars.k_empty[s]);
+        f_commit(dead ? &bars.dropped : &bars.k_empty[sk]);
         f_commit(dead ? &bars.dropped : &bars.s_full[s]);
+        if ((sk += 2) >= FA_NK) sk -= FA_NK, k_par ^= 1;
       }
       if (dead) *static_cast<volatile int*>(&failed) = 1;
     }
@@ -287,7 +318,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       bool dead = false;
       for (int j = 0; j < n_tiles; ++j) {
         const int sv = j & 1, sp = (n_tiles + j) & 1;
-        const uint32_t p_lo = f_desc_lo(f_u32(Ps + sp * 2 * FA_BLK));
+        const uint32_t p_at = tmem + FA_P0 + (uint32_t)sp * 64u;
         const uint32_t v_lo = VT ? f_desc_lo(f_u32(Vs + sv * 2 * FA_BLK)) : f_desc_lo_mn(f_u32(Vs + sv * 2 * FA_BLK));
         mbar_wait_issuer(&bars.v_full[sv], (j >> 1) & 1, dead);
         mbar_wait_issuer(&bars.p_full[sp], (j >> 1) & 1, dead);
@@ -297,13 +328,11 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
         for (int ks = 0; ks < FA_TK / 16; ++ks) {
           if (ks >= ks_n) break;
-          const uint32_t a = p_lo + (uint32_t)((ks >> 2) * (FA_BLK >> 4) + (ks & 3) * 2);
           // VT: 32 bytes along a 64-key row; else 16 rows of 128 bytes
           const uint32_t b = VT ? v_lo + (uint32_t)((ks >> 2) * (vblk >> 4) + (ks & 3) * 2) : v_lo + (uint32_t)(ks * (2048 >> 4));
-          f_umma(tmem + 256, a, b, F_DESC_HI, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+          f_umma_ts(tmem + FA_O0, p_at + (uint32_t)(ks * 8), b, F_DESC_HI, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
         }
-        f_commit(dead ? &bars.dropped : &bars.p_empty[sp]);
-        f_commit(dead ? &bars.dropped : &bars.v_empty[sv]);
+        f_commit(dead ? &bars.dropped : &bars.pv_done[sv]);   // frees the value slot and the P tile
       }
       f_commit(dead ? &bars.dropped : &bars.o_full);   // (an output that is not whole is not handed over)
       if (dead) *static_cast<volatile int*>(&failed) = 1;
@@ -313,7 +342,8 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int q4 = warp & 3, half = ((warp - 2) >> 2) & 1, grp = (warp - 2) >> 3;
     const int row = q4 * 32 + lane;
     const int qi = row0 + row;
-    const int vis = (qi < p.Lq) ? (p.causal ? min(S, S - p.Lq + qi + 1) : S) : S;
+    const int vis = p.causal ? min(S, S - p.Lq + min(qi, p.Lq - 1) + 1) : S;   // (rows behind the last query repeat it)
+    const int vis_most = __shfl_sync(0xffffffffu, vis, 31);                     // of the warp's rows
     const uint32_t t_row = tmem + ((uint32_t)(q4 * 32) << 16);
     constexpr float LOG2E = 1.4426950408889634f;
     // The softmax warps bound the kernel (two warps per scheduler, 64 scores per thread and pass), so they work on pairs: one
@@ -333,9 +363,12 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       ok = __all_sync(0xffffffffu, mbar_wait(&bars.s_full[s], (i >> 1) & 1, &failed));
       if (!ok) break;
       f_fence_after();
-      f_scores(t_row + (uint32_t)(s * 128 + half * 64), vis - (i * FA_TK + half * 64), pk);
+      // (half tiles that no row of the warp sees, a third of a diagonal tile: nothing to add)
+      const bool any = vis_most > i * FA_TK + half * 64;
+      if (any) f_scores(t_row + (uint32_t)(s * 128 + half * 64), vis - (i * FA_TK + half * 64), pk);
       f_fence_before();
       f_arrive(&bars.s_empty[s]);
+      if (!any) continue;
       uint32_t mx = pk[0];
 #pragma unroll
       for (int e = 1; e < 32; ++e) mx = f_max2(mx, pk[e]);
@@ -365,7 +398,6 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
       for (int e = 0; e < 4; ++e) l += a[e].y > 0.f ? a[e].y * f_ex2((a[e].x - m) * LOG2E) : 0.f;
     }
-    f_sbar();   // (the first P tile goes where the statistics were)
     const float inv_l = 1.0f / l;
     const uint64_t nbm = f2(-m * LOG2E, -m * LOG2E), inv2 = f2(inv_l, inv_l);
     for (int j = (n_tiles ^ grp) & 1; j < n_tiles && ok; j += 2) {  // ---- pass 2: p = bf16(exp(s - m) / l) -> shared memory ----
@@ -373,21 +405,25 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       ok = __all_sync(0xffffffffu, mbar_wait(&bars.s_full[s], (i >> 1) & 1, &failed));
       if (!ok) break;
       f_fence_after();
-      f_scores(t_row + (uint32_t)(s * 128 + half * 64), vis - (j * FA_TK + half * 64), pk);
+      const bool any = vis_most > j * FA_TK + half * 64;
+      if (any) f_scores(t_row + (uint32_t)(s * 128 + half * 64), vis - (j * FA_TK + half * 64), pk);
       f_fence_before();
       f_arrive(&bars.s_empty[s]);
+      if (any) {
 #pragma unroll
-      for (int e = 0; e < 32; ++e) {
-        const uint64_t x = fma2(f_pair(pk[e]), log2e, nbm);
-        const uint64_t w = mul2(f2(f_ex2(f2_lo(x)), f_ex2(f2_hi(x))), inv2);
-        pk[e] = pack2(f2_lo(w), f2_hi(w));
+        for (int e = 0; e < 32; ++e) {
+          const uint64_t x = fma2(f_pair(pk[e]), log2e, nbm);
+          const uint64_t w = mul2(f2(f_ex2(f2_lo(x)), f_ex2(f2_hi(x))), inv2);
+          pk[e] = pack2(f2_lo(w), f2_hi(w));
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 32; ++e) pk[e] = 0u;
       }
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars.p_empty[s], ((j >> 1) & 1) ^ 1, &failed));  // the group's previous P.V has consumed the P tile
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars.pv_done[j & 1], ((j >> 1) & 1) ^ 1, &failed));  // the group's previous P.V has consumed the P tile
       if (!ok) break;
-      uint8_t* prow = Ps + (2 * s + half) * FA_BLK + row * 128;
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        *reinterpret_cast<uint4*>(prow + ((c ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+      f_st16(t_row + FA_P0 + (uint32_t)(s * 64 + half * 32), pk);
+      f_st16(t_row + FA_P0 + (uint32_t)(s * 64 + half * 32 + 16), pk + 16);
       if constexpr (!VT) {
         // V rows behind the segment's last key (another segment's, or a cache's unused rows) meet p = 0, but 0 times a NaN
         // or an infinity would still reach O: those of the last group of 16 keys that is multiplied are cleared
@@ -401,9 +437,11 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             *reinterpret_cast<uint4*>(Vs + (j & 1) * 2 * FA_BLK + (ch >> 3) * FA_BLK + r * 128 + (ch & 7) * 16) =
                 make_uint4(0, 0, 0, 0);
           }
+          f_fence_async();  // generic-proxy writes -> visible to the tensor core (async proxy)
         }
       }
-      f_fence_async();  // generic-proxy writes of P -> visible to the tensor core (async proxy)
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      f_fence_before();
       f_arrive(&bars.p_full[s]);
     }
     // ---- epilogue: O row -> bf16 -> global (16-column chunks go round the row's four threads) ----
@@ -412,7 +450,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     bf16* orow = p.out + (long)(p.q0 + qi) * p.o_ts + (long)h * p.hd;
     for (int c0 = 16 * (2 * grp + half); c0 < p.hd; c0 += 64) {
       uint32_t r[16];
-      f_tmem_ld16(t_row + 256u + (uint32_t)c0, r);
+      f_tmem_ld16(t_row + FA_O0 + (uint32_t)c0, r);
       if (!ok)
         for (int e = 0; e < 16; ++e) r[e] = 0x7FC00000u;
       if (qi < p.Lq) {
@@ -441,8 +479,8 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (warp == 0) {
         g_fa_wait_failed = B200_WAIT_ATTENTION;
         if (!(p.flags & 1)) mbar_drain(&bars.q_full, 0);
-        for (int i = max(0, k_loads - 2); i < k_loads; ++i) mbar_drain(&bars.k_full[i & 1], (i >> 1) & 1);
-        for (int i = max(0, v_loads - 2); i < v_loads; ++i) mbar_drain(&bars.v_full[i & 1], (i >> 1) & 1);
+        for (int i = max(0, k_loads - FA_NK); i < k_loads; ++i) mbar_drain(&bars.k_full[i % FA_NK], (i / FA_NK) & 1);
+        for (int i = max(0, v_loads - FA_NV); i < v_loads; ++i) mbar_drain(&bars.v_full[i % FA_NV], (i / FA_NV) & 1);
       } else {
         uint64_t* mine = &bars.drained[warp == 1 ? 0 : warp - 17];
         f_commit(mine);
@@ -574,7 +612,7 @@ int attention_fa(const void* q, long q_ts, long q_hs, const void* k, long k_ts, 
   if (rc) return rc;
   const auto kern = v_transposed ? attention_fa_kernel<true> : attention_fa_kernel<false>;
   static unsigned long long set_mask[2] = {0ull, 0ull};
-  const size_t smem = 14 * FA_BLK + 1024;
+  const size_t smem = (2 + 2 * FA_NK + 2 * FA_NV) * FA_BLK + 4 * FA_TQ * sizeof(float2) + 1024;
   if (FirstUse first{&set_mask[v_transposed]})
     B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   FaParams p;

@@ -193,8 +193,21 @@ __device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
       : "memory");
   return done;
 }
+// (a try_wait takes some 200 cycles even where the phase is over, a test_wait 80: every wait asks once that way first)
+__device__ __forceinline__ bool mbar_test(uint32_t addr, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(addr), "r"(parity)
+      : "memory");
+  return done;
+}
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* failed) {
   const uint32_t addr = static_cast<uint32_t>(__cvta_generic_to_shared(bar));
+  if (mbar_test(addr, parity)) return true;
 #pragma unroll 1
   for (int i = 0; i < WAIT_TRIES; ++i)
     if (mbar_try(addr, parity)) return true;
@@ -206,7 +219,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* f
 // tower attention, which is bound by its issuing thread, slower: three CLIP blocks of 8 pictures 1400 -> 1440 us.
 __device__ __forceinline__ void mbar_wait_issuer(uint64_t* bar, uint32_t parity, bool& dead) {
   const uint32_t addr = static_cast<uint32_t>(__cvta_generic_to_shared(bar));
-  uint32_t done = 0;
+  uint32_t done = mbar_test(addr, parity);
   for (int i = 0; !done && !dead; ++i) {
     done = mbar_try(addr, parity);
     if (i > WAIT_TRIES) dead = true;

@@ -87,9 +87,9 @@ __device__ __forceinline__ void w_mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(w_smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void w_mbar_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t done;
   const uint32_t addr = w_smem_u32(bar);
-  do {
+  uint32_t done = mbar_test(addr, parity);
+  while (!done) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -97,7 +97,7 @@ __device__ __forceinline__ void w_mbar_wait(uint64_t* bar, uint32_t parity) {
         : "=r"(done)
         : "r"(addr), "r"(parity)
         : "memory");
-  } while (!done);
+  }
 }
 __device__ __forceinline__ void w_tma_2d(void* dst, const CUtensorMap* tmap, uint64_t* bar, int c0,
                                          int c1) {
