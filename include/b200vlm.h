@@ -513,6 +513,16 @@ int b200_lm_latent_queries(const float* q, long ldq, void* out, long ldo, const 
 int b200_lm_latent_expanded_attention(const void* q, long q_ts, const void* k, long k_ts, const void* kr, long kr_ts, const void* v,
                                       long v_ts, void* out, long o_ts, int out32, int H, int dn, int dr, int dv, int n_q, int S,
                                       float scale, int flags, void* stream);
+/* a step of prompt portions through a latent attention layer (bf16 cache, no window, no gate) in the expanded form: y [T][W] =
+ * W_o attention(..) of x [T][W] (fp32; or xb: its bf16 rows, ceil64(W) wide); weights as LatentAttention packs them: down
+ * [q latent or queries | kv latent, rotated part], ukv [H dim + H vdim][kv_rank]; segs (host): (first row, rows, slot, first
+ * position) per portion; ws: 256-byte aligned, b200_lm_latent_portions_ws bytes (longest: keys of the longest portion) */
+long b200_lm_latent_portions_ws(int T, int W, int n_down, int q_rank, int H, int dim, int rot_dim, int vdim, int longest);
+int b200_lm_latent_portions(const float* x, long ldx, const void* xb, int W, const void* down, int n_down, const void* dq_norm, const void* uq,
+                            const void* dkv_norm, const void* ukv, const void* o, float eps, void* cache, long slot_stride,
+                            long tok_stride, const int* slot, const int* pos, const float* cs, int q_rank, int kv_rank, int H, int dim,
+                            int rot_dim, int rot_dims, int vdim, int own_kv, int pairs, float scale, const int* segs, int n_seg, float* y,
+                            long ldy, void* ws, long ws_bytes, int T, void* stream);
 /* C [T, N] (bf16) = X [T, K] . W [N, K]^T (bf16 operands, row pitches in elements, multiples of 8) on the tensor cores */
 int b200_gemm_wt_rows(const void* X, long ldx, const void* W, void* C, long ldc, int T, int N, int K, void* stream);
 /* greedy: lowest index of the largest logit per row and its log-probability */

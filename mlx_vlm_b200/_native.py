@@ -149,6 +149,9 @@ LM_SIGNATURES = {
     "b200_lm_cache_transpose": (_I, [_P, _L, _I, _I, _I, _P, _P]),
     "b200_lm_latent_queries": (_I, [_P, _L, _P, _L, _P, _I, _I, _I, _I, _I, _I, _P]),
     "b200_lm_latent_expanded_attention": (_I, [_P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _I, _F, _I, _P]),
+    "b200_lm_latent_portions_ws": (_L, [_I] * 9),
+    "b200_lm_latent_portions": (_I, [_P, _L, _P, _I, _P, _I, _P, _P, _P, _P, _P, _F, _P, _L, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I,
+                                     _I, _F, _P, _I, _P, _L, _P, _L, _I, _P]),
     "b200_gemm_wt_rows": (_I, [_P, _L, _P, _P, _L, _I, _I, _I, _P]),
     "b200_gemm_wt_f32": (_I, [_P, _L, _P, _L, _P, _P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _I, _P]),
     "b200_f32_split": (_I, [_P, _L, _P, _L, _I, _I, _I, _P]),

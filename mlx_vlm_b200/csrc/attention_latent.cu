@@ -21,7 +21,7 @@
 //   warp 11      allocates the tensor memory
 // Bound by the exponentials (16 a cycle and SM: 1024 cycles a tile of 128 x 128) and the L2 (80 KB a tile).  2048 tokens, 16
 // heads of 128 + 64 / 128: the absorbed form's products over the whole square, its softmax and conversions took 390 us, the
-// expansion (a product of 4096 rows) and this kernel 48; the layer 526 -> 164 us (the host's launches from there on).
+// expansion (a product of 4096 rows) and this kernel 48; the layer 526 -> 164 us (149 with its launches in one call).
 #include <mutex>
 
 #include "common.cuh"

@@ -370,6 +370,8 @@ struct LatentPostP {
   const float2* cs;                          // [T][rot_dims/2]
   int q_rank, kv_rank, rot_dim, rot_dims, own_kv;
   int pairs;                                 // the rotation pairs (2i, 2i + 1) instead of (i, i + rot_dims / 2)
+  bf16* cqb = nullptr;                       // instead of cq: bf16 operand rows, ldq numbers each, zero behind q_rank
+  int pdl = 0;                               // launched as a dependent of the kernel before (b200_lm_latent_portions)
 };
 // element i of a vector r whose first `dims` numbers turn by the table row a[0 .. dims/2)
 __device__ __forceinline__ float rope_elem(const float* r, int i, int dims, const float2* a, int pairs) {
@@ -386,13 +388,17 @@ __device__ __forceinline__ float rope_elem(const float* r, int i, int dims, cons
 template <typename CT>
 __global__ void latent_post_kernel(LatentPostP<CT> p) {
   __shared__ float red[32];
+  if (p.pdl) pdl_prologue();
   const int t = blockIdx.x;
   const float* d = p.D + (long)t * p.ldd;
   float ss = 0.f, inv = 0.f;
   if (p.q_rank > 0) {                 // a design without a query latent has q_rank 0: the row starts with the kv latent
     for (int i = threadIdx.x; i < p.q_rank; i += blockDim.x) ss += d[i] * d[i];
     inv = 1.0f / sqrtf(block_sum(ss, red) / (float)p.q_rank + p.eps);
-    for (int i = threadIdx.x; i < p.q_rank; i += blockDim.x) p.cq[(long)t * p.ldq + i] = d[i] * inv * bf2f(p.wq[i]);
+    if (p.cqb)
+      for (int i = threadIdx.x; i < p.ldq; i += blockDim.x) p.cqb[(long)t * p.ldq + i] = f2bf(i < p.q_rank ? d[i] * inv * bf2f(p.wq[i]) : 0.f);
+    else
+      for (int i = threadIdx.x; i < p.q_rank; i += blockDim.x) p.cq[(long)t * p.ldq + i] = d[i] * inv * bf2f(p.wq[i]);
   }
   if (!p.own_kv) return;
   const float* k = d + p.q_rank;
@@ -423,7 +429,9 @@ __global__ void rope_q_kernel(const float* __restrict__ q, long ldq, int qh_stri
 // (VEC: dim, rot_dim and the pitches are multiples of 4).
 template <bool VEC>
 __global__ void latent_queries_kernel(const float* __restrict__ q, long ldq, bf16* __restrict__ out, long ldo,
-                                      const float2* __restrict__ cs, int n_cols, int dim, int rot_dim, int rot_dims, int pairs) {
+                                      const float2* __restrict__ cs, int n_cols, int dim, int rot_dim, int rot_dims, int pairs,
+                                      int pdl) {
+  if (pdl) pdl_prologue();
   const int t = blockIdx.x, hd = dim + rot_dim;
   const float* x = q + (long)t * ldq;
   const float2* a = cs + (long)t * (rot_dims >> 1);
@@ -1058,7 +1066,8 @@ __global__ void rows_to_bf16_kernel(const float* __restrict__ X, long ldx, const
 }
 // the same with four columns per thread (rows of whole, aligned 16-byte vectors; K, Kp multiples of 4)
 __global__ void rows_to_bf16x4_kernel(const float* __restrict__ X, long ldx, const int* __restrict__ map, int div,
-                                      bf16* __restrict__ out, long ldo, int K, int Kp, int relu2) {
+                                      bf16* __restrict__ out, long ldo, int K, int Kp, int relu2, int pdl) {
+  if (pdl) pdl_prologue();
   const int i = blockIdx.x;
   const int src = map ? map[i] : i;
   const float* x = X + (long)(src < 0 ? 0 : (map ? src / div : src)) * ldx;
@@ -1553,7 +1562,7 @@ int b200_lm_rows_to_bf16(const float* X, long ldx, const int* map, int div, void
                          int relu2, void* st) {
   B200_REQUIRE(X && out && T > 0 && K > 0 && Kp >= K, "lm_rows_to_bf16: bad argument");
   const bool v4 = K % 4 == 0 && Kp % 4 == 0 && ldx % 4 == 0 && ldo % 4 == 0 && ((uintptr_t)X & 15) == 0 && ((uintptr_t)out & 7) == 0;
-  if (v4) rows_to_bf16x4_kernel<<<T, Kp >= 1024 ? 256 : 128, 0, (cudaStream_t)st>>>(X, ldx, map, div > 0 ? div : 1, (bf16*)out, ldo, K, Kp, relu2);
+  if (v4) rows_to_bf16x4_kernel<<<T, Kp >= 1024 ? 256 : 128, 0, (cudaStream_t)st>>>(X, ldx, map, div > 0 ? div : 1, (bf16*)out, ldo, K, Kp, relu2, 0);
   else rows_to_bf16_kernel<<<T, 256, 0, (cudaStream_t)st>>>(X, ldx, map, div > 0 ? div : 1, (bf16*)out, ldo, K, Kp, relu2);
   B200_CHECK_LAUNCH();
   return B200_OK;
@@ -1597,10 +1606,77 @@ int b200_lm_latent_queries(const float* q, long ldq, void* out, long ldo, const 
                    (cs || !rot_dims) && ldq >= (long)H * (dim + rot_dim) && ldo >= (long)H * (dim + rot_dim),
                "lm_latent_queries: bad argument");
   const bool vec = dim % 4 == 0 && rot_dim % 4 == 0 && ldq % 4 == 0 && ldo % 4 == 0 && ((uintptr_t)q & 15) == 0 && ((uintptr_t)out & 7) == 0;
-  if (vec) latent_queries_kernel<true><<<T, 256, 0, (cudaStream_t)st>>>(q, ldq, (bf16*)out, ldo, (const float2*)cs, H * (dim + rot_dim), dim, rot_dim, rot_dims, pairs);
-  else latent_queries_kernel<false><<<T, 256, 0, (cudaStream_t)st>>>(q, ldq, (bf16*)out, ldo, (const float2*)cs, H * (dim + rot_dim), dim, rot_dim, rot_dims, pairs);
+  if (vec) latent_queries_kernel<true><<<T, 256, 0, (cudaStream_t)st>>>(q, ldq, (bf16*)out, ldo, (const float2*)cs, H * (dim + rot_dim), dim, rot_dim, rot_dims, pairs, 0);
+  else latent_queries_kernel<false><<<T, 256, 0, (cudaStream_t)st>>>(q, ldq, (bf16*)out, ldo, (const float2*)cs, H * (dim + rot_dim), dim, rot_dim, rot_dims, pairs, 0);
   B200_CHECK_LAUNCH();
   return B200_OK;
+}
+static long lp_bytes(long n) { return (n + 255) & ~255L; }
+static long lp_pad64(long n) { return (n + 63) / 64 * 64; }
+long b200_lm_latent_portions_ws(int T, int W, int n_down, int q_rank, int H, int dim, int rot_dim, int vdim, int longest) {
+  const long nq = (long)H * (dim + rot_dim);
+  return lp_bytes(T * lp_pad64(W) * 2) + lp_bytes((long)T * n_down * 4) + (q_rank ? lp_bytes(T * lp_pad64(q_rank) * 2) + lp_bytes(T * nq * 4) : 0) +
+         lp_bytes(T * nq * 2) + lp_bytes((long)longest * H * (dim + vdim) * 2) + lp_bytes((long)T * H * vdim * 2);
+}
+// The launches of a step of prompt portions in the expanded form, one after the other.  Every kernel between the products is a
+// programmatic dependent launch (all weights are fixed, so that a product may ask for its own before the kernel ahead has ended),
+// the query latent is written as the operand of its product.  One by one from Python they took the host 197 us a layer, in this call 104; 2048 tokens, 16 heads: 164 -> 149 us.
+int b200_lm_latent_portions(const float* x, long ldx, const void* xb, int W, const void* down, int n_down, const void* dq_norm, const void* uq,
+                            const void* dkv_norm, const void* ukv, const void* o, float eps, void* cache, long slot_stride,
+                            long tok_stride, const int* slot, const int* pos, const float* cs, int q_rank, int kv_rank, int H, int dim,
+                            int rot_dim, int rot_dims, int vdim, int own_kv, int pairs, float scale, const int* segs, int n_seg, float* y,
+                            long ldy, void* ws, long ws_bytes, int T, void* stream) {
+  cudaStream_t st = (cudaStream_t)stream;
+  B200_REQUIRE((x || xb) && down && ukv && o && cache && segs && n_seg > 0 && y && ws && T > 0 && W > 0 && H > 0, "lm_latent_portions: bad argument");
+  B200_REQUIRE((q_rank == 0 || (dq_norm && uq)) && (!own_kv || (dkv_norm && slot && pos)) && (cs || !rot_dims) && rot_dims % 2 == 0 && rot_dims <= rot_dim,
+               "lm_latent_portions: bad argument");
+  const long nq = (long)H * (dim + rot_dim), Wp = lp_pad64(W), qp = lp_pad64(q_rank), per = (long)H * (dim + vdim);
+  const bool vec_x = xb || (W % 4 == 0 && ldx % 4 == 0 && ((uintptr_t)x & 15) == 0);
+  B200_REQUIRE(vec_x && dim % 4 == 0 && rot_dim % 4 == 0 && (H * vdim) % 64 == 0 && nq % 4 == 0 && n_down % 4 == 0,
+               "lm_latent_portions: rows of %d, heads of %d + %d and %d", W, dim, rot_dim, vdim);
+  int longest = 0;
+  for (int g = 0; g < n_seg; ++g) {
+    const int* s = segs + 4 * g;
+    B200_REQUIRE(s[0] >= 0 && s[1] > 0 && s[0] + s[1] <= T && s[3] >= 0, "lm_latent_portions: segment %d", g);
+    longest = max(longest, s[1] + s[3]);
+  }
+  B200_REQUIRE(b200_lm_latent_portions_ws(T, W, n_down, q_rank, H, dim, rot_dim, vdim, longest) <= ws_bytes && ((uintptr_t)ws & 255) == 0,
+               "lm_latent_portions: workspace of %ld B", ws_bytes);
+  uint8_t* w = (uint8_t*)ws;
+  auto take = [&](long bytes) { uint8_t* p = w; w += lp_bytes(bytes); return p; };
+  bf16* xo = (bf16*)take(T * Wp * 2);
+  float* D = (float*)take((long)T * n_down * 4);
+  bf16* cq = q_rank ? (bf16*)take(T * qp * 2) : nullptr;
+  float* q = q_rank ? (float*)take(T * nq * 4) : D;
+  bf16* qb = (bf16*)take(T * nq * 2);
+  bf16* kv = (bf16*)take((long)longest * per * 2);
+  bf16* att = (bf16*)take((long)T * H * vdim * 2);
+  int rc;
+  if (!xb) B200_CUDA(launch_pdl(rows_to_bf16x4_kernel, dim3(T), dim3(Wp >= 1024 ? 256 : 128), 0, st, x, ldx, nullptr, 1, xo, Wp, W, (int)Wp, 0, 1));
+  if ((rc = b200_gemm_wt_f32(xb ? xb : xo, Wp, down, W, nullptr, nullptr, 0, D, n_down, nullptr, 0, 0, T, n_down, W, 1, 0, B200_WT_F32, stream)))
+    return rc;
+  if (q_rank || own_kv) {
+    LatentPostP<bf16> p{q_rank ? D : D + nq, n_down, (const bf16*)dq_norm, (const bf16*)dkv_norm, eps, nullptr, qp, (bf16*)cache, slot_stride,
+                        tok_stride, slot, pos, (const float2*)cs, q_rank, kv_rank, rot_dim, rot_dims, own_kv, pairs};
+    p.cqb = cq;
+    p.pdl = 1;
+    B200_CUDA(launch_pdl(latent_post_kernel<bf16>, dim3(T), dim3(256), 0, st, p));
+  }
+  if (q_rank && (rc = b200_gemm_wt_f32(cq, qp, uq, q_rank, nullptr, nullptr, 0, q, nq, nullptr, 0, 0, T, (int)nq, q_rank, 1, 0, B200_WT_F32, stream)))
+    return rc;
+  const long ldq = q_rank ? nq : n_down;
+  B200_CUDA(launch_pdl(latent_queries_kernel<true>, dim3(T), dim3(256), 0, st, (const float*)q, ldq, qb, nq, (const float2*)cs, (int)nq, dim, rot_dim,
+                       rot_dims, pairs, 1));
+  for (int g = 0; g < n_seg; ++g) {
+    const int *s = segs + 4 * g, S = s[3] + s[1];
+    const bf16* rows = (const bf16*)cache + (long)s[2] * slot_stride;
+    if ((rc = b200_gemm_wt_rows(rows, tok_stride, ukv, kv, per, S, (int)per, kv_rank, stream))) return rc;
+    if ((rc = b200_lm_latent_expanded_attention(qb + s[0] * nq, nq, kv, per, rot_dim ? rows + kv_rank : nullptr, tok_stride, kv + (long)H * dim, per,
+                                                att + (long)s[0] * H * vdim, (long)H * vdim, 0, H, dim, rot_dim, vdim, s[1], S, scale, 0, stream)))
+      return rc;
+  }
+  return b200_gemm_wt_f32(att, (long)H * vdim, o, (long)H * vdim, nullptr, nullptr, 0, y, ldy, nullptr, 0, 0, T, W, H * vdim, 1, 0, B200_WT_F32,
+                          stream);
 }
 int b200_lm_cache_transpose(const void* cache_rows, long tok_stride, int S, int Sp, int kv_rank, void* out, void* st) {
   B200_REQUIRE(cache_rows && out && S > 0 && Sp >= S && kv_rank > 0, "lm_cache_transpose: bad argument");

@@ -229,6 +229,13 @@ class LatentAttention:
         return ops.tc_ok(min(n for _, n, _, _ in segs), r, Dl, cache_layer.stride(1)) and cache_layer.data_ptr() % 16 == 0 and \
             max((p0 + n) * per for _, n, _, p0 in segs) <= EXPANDED_MAX
 
+    def _one_call(self, ops: LayerOps, x, T: int, xb) -> bool:
+        """whether all launches of the expanded form go out in one call (ops.latent_portions)"""
+        w = self.w
+        return (xb is None or (xb.stride(0) == (self.W + 63) // 64 * 64 and xb.data_ptr() % 16 == 0)) and not self.gated and (self.H * self.vdim) % 64 == 0 and x.dtype == torch.float32 and x.stride(0) % 4 == 0 and x.stride(1) == 1 and \
+            x.data_ptr() % 16 == 0 and self.W % 8 == 0 and w["down"].shape[0] % 4 == 0 and self.rot_dims % 2 == 0 and \
+            ops.tc_ok(T, self.W, self.q_rank) and all(w[n].data_ptr() % 16 == 0 for n in ("down", "ukv", "o"))
+
     def _expanded(self, ctx: StepCtx, q, cs, segs, cache_layer) -> torch.Tensor:
         """Portions of prompts with the keys and values of their slots expanded from the cached rows: one product for both
         ([W_uk; W_uv] on the latent part), attention heads of dim + rot_dim and vdim numbers.  -> the heads' outputs, bf16
@@ -248,9 +255,17 @@ class LatentAttention:
         ops, w, T = ctx.ops, self.w, x.shape[0]
         H, dn, dr, r, dv = self.H, self.dim, self.rot_dim, self.kv_rank, self.vdim
         Dl = r + dr
-        D = ops.linear(x, w["down"], operand=ctx.x_operand)
         cache_layer = ctx.pool.buf[self.cache_index][..., :Dl]    # a pool row may be wider than this layer's
         cs = ctx.rope(self.rot_base, self.rot_dims, self.rot_scaling)
+        segs = ctx.segments or []
+        expand = self._expand_portions(ops, segs, cache_layer)
+        if expand and self._one_call(ops, x, T, ctx.x_operand):
+            try:
+                return ops.latent_portions(self, x, ctx, cs, segs, cache_layer)
+            except _B200Error as e:
+                ops.tc_refused(e)
+                expand = False
+        D = ops.linear(x, w["down"], operand=ctx.x_operand)
         if self.q_rank:
             cq = ops.empty((T, self.q_rank))
             ops.latent_post(D, w["dq.norm"], w.get("dkv.norm"), ctx.eps, cq, cache_layer if self.own_kv else None,
@@ -262,8 +277,7 @@ class LatentAttention:
                             dr, self.rot_dims, pairs=self.pairs)
             q = D[:, :self.n_q]
             n_read = self.n_q + Dl
-        segs = ctx.segments or []
-        if self._expand_portions(ops, segs, cache_layer):
+        if expand:
             try:
                 att = self._expanded(ctx, q, cs, segs, cache_layer)
                 if att.dtype == torch.bfloat16:

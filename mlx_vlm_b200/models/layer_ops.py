@@ -8,6 +8,7 @@ are bf16 and the operands of the matrix products are rounded to bf16 on load (fp
 """
 from __future__ import annotations
 
+import ctypes as C
 from typing import Optional
 
 import numpy as np
@@ -452,6 +453,24 @@ class LayerOps:
         self._ok(self.lib.b200_lm_latent_queries(q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0), cs.data_ptr(), H, dim,
                                                  rot_dim, rot_dims, int(pairs), T, self.s), "lm_latent_queries")
         return out
+
+    def latent_portions(self, m, x: torch.Tensor, ctx, cs: torch.Tensor, segs, cache_layer: torch.Tensor) -> torch.Tensor:
+        """a step of prompt portions through latent attention layer `m` in its expanded form: all launches in one call"""
+        T, W = x.shape
+        w = m.w
+        flat = [v for s in segs for v in s]
+        dims = (T, W, w["down"].shape[0], m.q_rank, m.H, m.dim, m.rot_dim, m.vdim, max(s[1] + s[3] for s in segs))
+        nbytes = self.lib.b200_lm_latent_portions_ws(*dims)
+        ws, y = self.empty((nbytes,), torch.uint8), self.empty((T, W))
+        xb = ctx.x_operand
+        self._ok(self.lib.b200_lm_latent_portions(
+            x.data_ptr(), x.stride(0), N.ptr(xb), W, w["down"].data_ptr(), dims[2], N.ptr(w.get("dq.norm")), N.ptr(w.get("uq")),
+            N.ptr(w.get("dkv.norm")), w["ukv"].data_ptr(), w["o"].data_ptr(), float(ctx.eps), cache_layer.data_ptr(), cache_layer.stride(0),
+            cache_layer.stride(1), ctx.slot.data_ptr(), ctx.pos.data_ptr(), cs.data_ptr(), m.q_rank, m.kv_rank, m.H, m.dim, m.rot_dim,
+            m.rot_dims if m.rot_dim else 0, m.vdim, int(m.own_kv), int(m.pairs), m.scale, (C.c_int * len(flat))(*flat), len(segs),
+            y.data_ptr(), W, ws.data_ptr(), nbytes, T, self.s), "lm_latent_portions")
+        self.launches += 4 + 2 * len(segs) + (1 if m.q_rank else 0)
+        return y
 
     def rows_gemm(self, Xb: torch.Tensor, W: torch.Tensor, K: int) -> torch.Tensor:
         """bf16 rows (T, >= K) -> Xb[:, :K] . W^T as bf16 rows, on the tensor cores"""
