@@ -24,8 +24,7 @@
 // A tile's time, from clock stamps (28 heads of 128): 1330 cycles in pass 1, of which the exponentials' 1024 are one part and
 // the two groups' loads and waits, which fall together, the other; 1450 in pass 2, where the thread that issues P.V is the
 // chain: 8 products of 64 cycles beside Q.K^T's, a wait for P and one for V.  With P in tensor memory instead of shared
-// memory, three key slots in the room that this gives, one commit for the value slot and the P tile, and half tiles that a
-// warp's rows do not see left out: 2048 queries behind 2048 keys, 28 heads, 168.5 -> 164 us; 8 prompts of 608, 32 heads, 120 ->
+// memory, one commit for the value slot and the P tile, and half tiles that a warp's rows do not see left out: 2048 queries behind 2048 keys, 28 heads, 168.5 -> 164 us; 8 prompts of 608, 32 heads, 120 ->
 // 117.6; four pictures and a clip (6012 patches, 16 heads of 80) 131.5 -> 130.
 // Measured against the kernel without TMA that such calls fell back to (attention_tc.cu): 2048 queries behind 2048 cached
 // keys, 28 heads of 128: 1094 -> 354 us (249 with the pairwise softmax below); four pictures and a clip of four frames (6012
@@ -43,7 +42,10 @@ namespace {
 constexpr int FA_TQ = 128, FA_TK = 128;
 constexpr int FA_BLK = 16 * 1024;       // one 128-row x 64-column bf16 operand block
 constexpr int FA_THREADS = 640;         // producer warp, 3 MMA warps, 2 groups of 8 softmax warps
-constexpr int FA_NK = 3, FA_NV = 2;     // ring slots of key and of value tiles (a value slot and a P tile are free at the same time)
+constexpr int FA_NK = 2, FA_NV = 2;     // ring slots of key and of value tiles (a value slot and a P tile are free at the same time)
+// A key slot belongs to one of the two threads that issue Q.K^T.  With an odd number of slots both would use each in turn, and a
+// thread that waits for the round after next would take the parity of a round long past for it: it has to see every round.
+static_assert(FA_NK % 2 == 0, "a slot's waiter sees every round of it");
 constexpr uint32_t FA_O0 = 256, FA_P0 = 384;   // TMEM columns: scores 2 x 128 | O 128 | P 2 x 64 (two bf16 a column)
 
 struct FaParams {

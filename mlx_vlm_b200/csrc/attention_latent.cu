@@ -517,8 +517,10 @@ static int attention_latent(const void* q, long q_ts, const void* k, long k_ts, 
   p.dn = dn; p.dr = dr; p.dv = dv; p.dvp = dvp; p.n_q = n_q; p.S = S;
   p.c = scale * 1.4426950408889634f;
   p.flags = flags;
-  // as many ring slots as fit beside Q (192 + 128 wide: 2, 128 + 128: 3)
-  p.stages = min(LP_MAX_STAGES, (LP_MAX_SMEM - 1024 - kb * LP_BLK) / ((kb + vb) * LP_BLK));
+  // As many ring slots as fit beside Q, an even number: a slot belongs to one of the two issuing threads, which then sees every
+  // round of it (with an odd number it would meet each second round, and the parity of the one before the last passes for it)
+  p.stages = min(LP_MAX_STAGES, (LP_MAX_SMEM - 1024 - kb * LP_BLK) / ((kb + vb) * LP_BLK)) & ~1;
+  B200_REQUIRE(p.stages >= 2, "attention_latent: %d key and %d value blocks", kb, vb);
   static unsigned long long set_mask = 0ull;
   if (FirstUse first{&set_mask})
     B200_CUDA(cudaFuncSetAttribute(attention_latent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LP_MAX_SMEM));
