@@ -402,7 +402,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     const float inv_l = 1.0f / l;
     const uint64_t nbm = f2(-m * LOG2E, -m * LOG2E), inv2 = f2(inv_l, inv_l);
-    for (int j = (n_tiles ^ grp) & 1; j < n_tiles && ok; j += 2) {  // ---- pass 2: p = bf16(exp(s - m) / l) -> shared memory ----
+    for (int j = (n_tiles ^ grp) & 1; j < n_tiles && ok; j += 2) {  // ---- pass 2: p = bf16(exp(s - m) / l) -> tensor memory ----
       const int i = n_tiles + j, s = grp;
       ok = __all_sync(0xffffffffu, mbar_wait(&bars.s_full[s], (i >> 1) & 1, &failed));
       if (!ok) break;
@@ -424,6 +424,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       ok = __all_sync(0xffffffffu, mbar_wait(&bars.pv_done[j & 1], ((j >> 1) & 1) ^ 1, &failed));  // the group's previous P.V has consumed the P tile
       if (!ok) break;
+      f_fence_after();
       f_st16(t_row + FA_P0 + (uint32_t)(s * 64 + half * 32), pk);
       f_st16(t_row + FA_P0 + (uint32_t)(s * 64 + half * 32 + 16), pk + 16);
       if constexpr (!VT) {
