@@ -381,10 +381,13 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       ok = __all_sync(0xffffffffu, mbar_wait(&bars.o_full[g], (t - 1) & 1, &failed));
       l_fence_after();
     }
-    // ---- merge: out = (O0 2^(m0 - m) + O1 2^(m1 - m)) / l, 16 columns at a time, the groups in turn ----
+    // ---- merge: out = (O0 2^(m0 - m) + O1 2^(m1 - m)) / l, 16 columns at a time, the groups in turn; a thread reads the other
+    //      group's accumulator too, for whose products only that group has waited ----
+    l_fence_before();
     l_bar256();     // (no product reads Q any more)
     stat[g * LP_TQ + row] = make_float2(m, l);
     l_bar256();
+    l_fence_after();
     const bool whole = !*static_cast<volatile int*>(&failed);
     const float2 a = stat[row], b = stat[LP_TQ + row];
     const float mm = fmaxf(a.x, b.x);

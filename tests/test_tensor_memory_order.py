@@ -9,7 +9,8 @@ import re
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mlx_vlm_b200", "csrc")
-KERNELS = [("attention_fa.cu", "attention_fa_kernel"), ("attention_f32_tc.cu", "attention_f32_tc_kernel")]
+KERNELS = [("attention_fa.cu", "attention_fa_kernel"), ("attention_f32_tc.cu", "attention_f32_tc_kernel"),
+           ("attention_latent.cu", "attention_latent_kernel")]
 
 
 def _body(name, kernel):
