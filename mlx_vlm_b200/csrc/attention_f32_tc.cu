@@ -256,7 +256,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
     if (q0 >= Lq) return;   // uniform per CTA, nothing is allocated yet
   }
   const int n_tiles = (S + TC_KEYS - 1) / TC_KEYS;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (tid == 0) {
     failed = 0;
     t_init(&bars.q_full, 256);
@@ -282,6 +281,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
   __syncthreads();
   t_fence_after();
   const uint32_t tmem = tmem_slot;
+  // (the next kernel may start from here on, not before: it may ask for tensor memory too, and would hold what this one still needs)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   if (warp == 11) {

@@ -214,7 +214,6 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int kbq = (p.hdp + 63) >> 6;         // 64-column blocks of the head dimension
   const int vblk = p.hdp * 128;              // bytes of one 64-key block of a V^T tile
 
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmQ)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmK)) : "memory");
@@ -248,6 +247,8 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   f_fence_after();
   const uint32_t tmem = tmem_slot;
+  // (the next kernel may start from here on, not before: it may ask for tensor memory too, and would hold what this one still needs)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   int k_loads = 0, v_loads = 0;   // of the producer
 

@@ -162,7 +162,6 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   const int end = S - p.n_q + q_last + 1;           // keys that the tile's last query sees
   const int n_tiles = (end + LP_TK - 1) / LP_TK;
 
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
     l_init(&bars.q_full, 1);
     for (int i = 0; i < LP_MAX_STAGES; ++i) {
@@ -191,6 +190,8 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   __syncthreads();
   l_fence_after();
   const uint32_t tmem = tmem_slot;
+  // (the next kernel may start from here on, not before: it may ask for tensor memory too, and would hold what this one still needs)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   int k_loads = 0, v_loads = 0;   // of the loading thread
 

@@ -615,7 +615,6 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     kb1 = min(kb_total, kb0 + p.kb_per_split);
   };
 
-  w_pdl_launch();
   if (warp == 0 && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmW)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmX)) : "memory");
@@ -643,6 +642,7 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   wp_cluster_sync();   // the peer's barriers exist before anything arrives on them
   w_fence_after();
   const uint32_t tmem = tmem_slot;
+  w_pdl_launch();   // (not before all columns are this pair's: the next kernel may ask for some)
 
   if (warp == 0) {
     if (lane == 0 && !(p.flags & 2u)) {  // ===== TMA producer (flags 2: nothing is loaded; a test in its loop cost 2 %) =====

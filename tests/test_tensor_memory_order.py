@@ -57,3 +57,13 @@ def test_an_access_behind_a_wait_is_fenced(name, kernel):
             fenced_before = False
             seen += 1
     assert seen >= 6
+
+
+@pytest.mark.parametrize("name,kernel", KERNELS + [("gemm_wt.cu", "gemm_wt_pair_kernel")])
+def test_columns_are_allocated_before_the_next_kernel_may_start(name, kernel):
+    """A kernel that asks for all 512 columns and lets its dependent start first could find columns taken by a CTA that waits for it"""
+    body = _body(name, kernel)
+    alloc = body.index("tcgen05.alloc")
+    assert "512u" in body[alloc:alloc + 200]
+    signals = [m.start() for m in re.finditer(r"griddepcontrol\.launch_dependents|w_pdl_launch\(\)", body)]
+    assert len(signals) == 1 and signals[0] > body.index("__syncthreads()", alloc), name
