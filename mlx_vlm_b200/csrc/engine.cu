@@ -1130,9 +1130,15 @@ int b200_engine_prefill_batch(b200_engine* e, const void* embeds, const int* pos
   if ((rc = upload_loc(e, loc, s))) return rc;
   rc = prefill_layers_v2_body(e, pos_stage, (int)T, 0, nullptr, s, segs.data(), n_seq, e->loc_dev);
   // first token of every sequence: the final norm of its last row (into the normed rows' buffer, which nothing reads any more), ONE
-  // product with the head for as many rows as the partial region takes logits of, and a sampler with a CTA per row
+  // product with the head for as many rows as the partial region takes logits of, and a sampler with a CTA per row.  One sequence
+  // of a model up to 1536 wide keeps the head and the sampler of a decode step: the head alone is as fast there (vocabulary of
+  // 151936: 77 us, the product 75; 3584 wide 321, 165), and its sampler's CTAs share the vocabulary (7 us, one CTA 34): the
+  // whole call with one layer 353 us, by the product 398 (3584 wide: 674, 555; two sequences of the 1536-wide model: 515, 465).
+  const long ldv = round8(c.vocab);
+  const int most = (int)std::min<long>(n_seq, WT_PARTIAL_BYTES / (ldv * 2));
+  const bool by_rows = most > 0 && (n_seq > 1 || H > 1536);
   bf16* last_rows = (bf16*)(e->ws + align256(T * H * 2));
-  if (!rc) rc = rms_norm(h, e->norm, last_rows, n_seq, (int)H, c.rms_eps, s, e->loc_dev + last_at);
+  if (!rc && by_rows) rc = rms_norm(h, e->norm, last_rows, n_seq, (int)H, c.rms_eps, s, e->loc_dev + last_at);
   B200_CUDA(cudaEventRecord(e->loc_ev, s));   // the table (and its staging copy) may be rewritten after this point
   if (rc) return rc;
   const DecodeDims d = e->dims();
@@ -1142,11 +1148,14 @@ int b200_engine_prefill_batch(b200_engine* e, const void* embeds, const int* pos
     e->prepared_cluster = e->attn_cluster;
   }
   if ((rc = launch_set_state(e->st, 0, segs[n_seq - 1].T, segs[n_seq - 1].T, 0, 0, e->embed, e->h, c.hidden, s))) return rc;
-  const long ldv = round8(c.vocab);
+  for (int g = 0; g < n_seq && !by_rows; ++g) {
+    if ((rc = launch_head(d, e->norm, e->head, h + (long)(segs[g].off + segs[g].T - 1) * H, e->logits, e->partials, s)) ||
+        (rc = launch_sample(d, e->logits, e->partials, e->logprobs, e->embed, e->h, e->st, e->token_log, e->log_cap, e->force, 0, s)))
+      return rc;
+    e->launches += 2;
+  }
   bf16* rows_logits = (bf16*)ws_partial(e);
-  const int most = (int)std::min<long>(n_seq, WT_PARTIAL_BYTES / (ldv * 2));
-  B200_REQUIRE(most > 0, "engine_prefill_batch: a vocabulary of %d", c.vocab);
-  for (int g = 0; g < n_seq; g += most) {
+  for (int g = 0; g < n_seq && by_rows; g += most) {
     const int n = std::min(most, n_seq - g);
     if ((rc = v2_linear(e, last_rows + (long)g * H, H, e->head, nullptr, rows_logits, ldv, n, c.vocab, (int)H, B200_EPI_NONE, s))) return rc;
     if ((rc = launch_rows_sample(d, rows_logits, ldv, n, g + n == n_seq, e->logits, e->logprobs, e->embed, e->h, e->st, e->token_log,
@@ -1154,7 +1163,7 @@ int b200_engine_prefill_batch(b200_engine* e, const void* embeds, const int* pos
       return rc;
     e->launches += 1;
   }
-  e->launches += 2;
+  e->launches += by_rows ? 2 : 1;
   e->tokens_launched += n_seq;
   e->ctx_host = segs[n_seq - 1].T;
   e->pos_host = segs[n_seq - 1].T;

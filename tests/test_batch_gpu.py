@@ -312,3 +312,76 @@ def test_first_tokens_of_a_batched_prefill(n):
     want = lg - torch.logsumexp(lg.double(), 0).float()
     assert float((lp.reshape(-1)[:lg.numel()] - want).abs().max()) <= 0.13             # lse and the difference are rounded to bf16
     assert eng.device_error() == 0
+
+
+def _left(eng):
+    """(logits, log-probabilities) that the engine goes on from, on the host"""
+    lg, lp = eng.snapshot("logits"), eng.logprobs_view()
+    eng.stream.synchronize()
+    return tuple(x.float().cpu().reshape(-1).clone() for x in (lg, lp))
+
+
+@pytest.mark.parametrize("kind", ["wide2", "oddvocab"])
+@pytest.mark.parametrize("n", [1, 2, 4])
+def test_decoding_goes_on_from_the_last_prompt_of_a_batch(kind, n):
+    """the state that a batched prefill leaves (token, its embedding, context, position): a decode step on the last prompt's pool
+    row gives what it gives after that prompt alone with the same token"""
+    c, W, model, req = _build(kind, 10, (56, 56))
+    lm, eng = model.language_model, model.engine
+    reqs = _requests(c, req, 4)[:n]
+    embs = [model.get_input_embeddings(ids, kw.get("pixel_values"), image_grid_thw=kw.get("image_grid_thw")) for ids, kw, _ in reqs]
+    rows, _ = lm.make_batch_cache(n, 256)
+    toks = lm.prefill_rows([r[0] for r in reqs], [e.inputs_embeds for e in embs], [lm.make_cache_row(rows.pool, b) for b in range(n)],
+                           [e.position_ids for e in embs], [e.rope_deltas for e in embs], reserve_tokens=256)
+    lg0 = _left(eng)[0]
+    eng.set_kv_row(n - 1)
+    eng.decode(1)
+    got = _left(eng)[0]
+    eng.set_kv_row(0)
+    ids, emb = reqs[-1][0], embs[-1]
+    lm._rope_deltas, lm._position_ids = None, None
+    lm(ids, inputs_embeds=emb.inputs_embeds, cache=lm.make_cache(), position_ids=emb.position_ids, rope_deltas=emb.rope_deltas,
+       logits_to_keep=1, reserve_tokens=256)
+    assert rl2(lg0, _left(eng)[0]) <= 5e-3
+    eng.set_next(toks[-1], ids.shape[1], ids.shape[1])
+    eng.decode(1)
+    assert rl2(got, _left(eng)[0]) <= 5e-3 and eng.device_error() == 0     # two layers of bf16 roundings apart, as the first logits above
+
+
+def test_first_tokens_of_many_prompts():
+    """more prompts than one product with the head takes (48 MB of logits), an odd vocabulary, enough last rows for the register
+    form of RMSNorm with its row map"""
+    from mlx_vlm_b200.models.qwen2_vl import Model
+    from oracle import qwen2vl as O
+    c = O.tiny_cfg()
+    c.text.vocab_size = 50003
+    W = O.init_weights(c, 0, norm_jitter=0.05)
+    model = Model(_to_model_config(c), device="cuda:0")
+    model.load_weights(W)
+    lm, eng, n = model.language_model, model.engine, 600
+    assert (48 << 20) // (2 * 50008) < n
+    rng = np.random.default_rng(11)
+    ids = [rng.integers(0, 50000, size=(1, 1 + i % 5)) for i in range(n)]
+    embs = [model.get_input_embeddings(x).inputs_embeds for x in ids]
+    rows, _ = lm.make_batch_cache(n, 16)
+    start = eng.tokens_launched
+    toks = lm.prefill_rows(ids, embs, [lm.make_cache_row(rows.pool, b) for b in range(n)])
+    lg, lp = _left(eng)
+    assert eng.tokens_launched == start + n
+    log = eng.token_log_view()
+    assert [int(log[(start + i) % eng.token_log_capacity]) for i in range(n)] == toks
+    assert toks[-1] == int(torch.argmax(lp[:lg.numel()]))
+    for b in [0, 1, 500, 501, 502, 503, n - 2, n - 1] + rng.integers(2, n - 2, size=16).tolist():
+        lm._rope_deltas, lm._position_ids = None, None
+        lm(ids[b], inputs_embeds=embs[b], cache=lm.make_cache(), logits_to_keep=1)
+        assert _token_ok(toks[b], _left(eng)[1]), (b, toks[b])
+    lm._rope_deltas, lm._position_ids = None, None
+    lm(ids[-1], inputs_embeds=embs[-1], cache=lm.make_cache(), logits_to_keep=1)
+    want_lg, want_lp = _left(eng)
+    assert rl2(lg, want_lg) <= 5e-3
+    few = [3, 77, n - 1]                        # few prompts share a row's columns among the CTAs of a cluster
+    toks3 = lm.prefill_rows([ids[b] for b in few], [embs[b] for b in few], [lm.make_cache_row(rows.pool, b) for b in range(3)])
+    lg3, lp3 = _left(eng)
+    assert rl2(lg3, want_lg) <= 5e-3 and float((lp3[:50003] - want_lp[:50003]).abs().max()) <= 0.13    # as above: two bf16 units below 16
+    assert toks3[-1] == int(torch.argmax(lp3[:50003])) and bool((lp3[50003:] == float("-inf")).all())
+    assert _token_ok(toks3[-1], want_lp) and eng.device_error() == 0
