@@ -106,6 +106,25 @@ def test_norms(lib, rows, dim):
     cmp_bf16(y, S.rms_norm(r, x, w, 1e-6), "rms_norm")
 
 
+@pytest.mark.parametrize("rows", [592, 593, 1201])
+@pytest.mark.parametrize("dim", [8, 256, 1288, 1536, 1544, 3584, 3592, 4096, 4104])
+def test_rms_norm_of_many_rows(lib, rows, dim):
+    """from 592 rows of up to 4096 columns the row is held in registers, in three sizes: bit for bit what fewer rows give"""
+    from mlx_vlm_b200 import _native as Nn
+    from oracle import mlx_semantics as S
+    r = R()
+    x, w = rnd(rows, dim, scale=2.0, seed=rows + dim), r.r(1.0 + 0.1 * torch.randn(dim, generator=torch.Generator().manual_seed(dim)))
+    dx, dw = to_dev(x), to_dev(w)
+    y, few = torch.full((rows + 1, dim), 7.0, dtype=torch.bfloat16, device="cuda"), torch.empty_like(dx)
+    Nn.check(lib.b200_rms_norm(dx.data_ptr(), dw.data_ptr(), y.data_ptr(), rows, dim, 1e-6, 0), "rms")
+    for a in range(0, rows, 500):
+        n = min(500, rows - a)
+        Nn.check(lib.b200_rms_norm(dx[a:].data_ptr(), dw.data_ptr(), few[a:].data_ptr(), n, dim, 1e-6, 0), "rms")
+    torch.cuda.synchronize()
+    assert torch.equal(y[:rows], few) and bool((y[rows] == 7.0).all())
+    cmp_bf16(y[:rows], S.rms_norm(r, x, w, 1e-6), f"rms_norm {rows} x {dim}")
+
+
 def test_cast(lib):
     from mlx_vlm_b200 import _native as Nn
     x = torch.randn(576 * 1176 + 3, generator=torch.Generator().manual_seed(11))

@@ -51,14 +51,47 @@ def test_kernel(n, S, H, dn, dr, dv, out_type):
     assert bool((out[n:] == 9.0).all())
 
 
-def _layer(H, dn, dr, dv, r, q_rank, pairs, gated, pool_extra, seed):
+@pytest.mark.parametrize("n,S", [(140, 140), (130, 400)])
+def test_scores_that_are_not_finite(n, S):
+    """infinities and NaN in a query or a key: NaN exactly where float64's softmax gives it (a row whose scores hold +inf or NaN, or
+    nothing but -inf), the other rows untouched; a key behind a query's last visible one does not reach it"""
+    from mlx_vlm_b200 import _native as N
+    lib = N.lm_lib()
+    H, dn, dr, dv = 2, 64, 0, 64
+    g = torch.Generator(device="cuda").manual_seed(n)
+    mk = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+    q, k, v = mk(n, H, dn), mk(S, H, dn), mk(S, H, dv)
+    q[:, :, 0] = q[:, :, 0].abs() + 0.1
+    q[n // 3, 0, 5] = float("nan")
+    q[n // 2, 1, 7] = float("inf")
+    k[S - 60, 0, 0] = float("-inf")            # weight 0 for every query that sees it
+    k[S - 20, 0, 0] = float("inf")
+    k[S - 2, 1, 3] = float("nan")
+    if n == S:
+        k[0, 1, 0] = float("-inf")             # the first query's only key
+    out = torch.empty(n, H * dv, device="cuda")
+    N.check(lib.b200_lm_latent_expanded_attention(q.data_ptr(), H * dn, k.data_ptr(), H * dn, 0, 0, v.data_ptr(), H * dv, out.data_ptr(),
+                                                  H * dv, 1, H, dn, dr, dv, n, S, 0.11, 0, 0), "attention", lib)
+    torch.cuda.synchronize()
+    s = torch.einsum("thd,shd->hts", q.double(), k.double()) * 0.11
+    seen = torch.arange(S, device="cuda")[None, :] <= torch.arange(S - n, S, device="cuda")[:, None]
+    p = torch.softmax(s.masked_fill(~seen, float("-inf")), -1)
+    want = torch.einsum("hts,shd->thd", p, v.double()).reshape(n, -1)
+    bound = 2.0 ** -8 * torch.einsum("hts,shd->thd", p, v.double().abs()).reshape(n, -1) + 1e-6     # as in test_kernel
+    bad = torch.isnan(want)
+    # two queries; the 20 that see key S - 20 and the 2 that see S - 2, each in its head; the first query where all it sees is -inf
+    assert torch.equal(torch.isnan(out), bad) and int(bad.sum()) == (24 + (n == S)) * dv
+    assert bool(((out.double() - want).abs() <= bound)[~bad].all())
+
+
+def _layer(H, dn, dr, dv, r, q_rank, pairs, gated, pool_extra, seed, kv_from=None):
     from mlx_vlm_b200.models.cache import LatentPool
     from mlx_vlm_b200.models.decoder_blocks import LatentAttention
     W = 256
     g = torch.Generator(device="cuda").manual_seed(seed)
     mk = lambda *s: (0.06 * torch.randn(*s, device="cuda", generator=g)).to(torch.bfloat16)
     m = LatentAttention(0, {"heads": H, "dim": dn, "rot_dim": dr, "vdim": dv, "kv_rank": r, "q_rank": q_rank, "scale": (dn + dr) ** -0.5,
-                            "rot": {"base": 10000.0, "dims": dr}}, W, rotation="pairs" if pairs else "half", gated=gated)
+                            "rot": {"base": 10000.0, "dims": dr}, "kv_from": kv_from}, W, rotation="pairs" if pairs else "half", gated=gated)
     m.cache_index = 0
     w = {n: 1 + mk(*s) if n.endswith("norm") else mk(*s) for n, s in m.checkpoint_tensors("").items()}
     arena = {n: torch.empty(s, device="cuda", dtype=torch.bfloat16) for n, s in m.manifest("")}
@@ -97,6 +130,32 @@ def test_layer_against_its_absorbed_form(H, dn, dr, dv, r, q_rank, pairs, gated,
         got[form] = (y.double(), pool.buf.clone())
     assert torch.equal(got["expanded"][1], got["absorbed"][1])
     err = lambda f: float((got[f][0] - got["rows"][0]).norm() / got["rows"][0].norm())
+    assert err("expanded") < max(1.1 * err("absorbed"), 2.0 ** -8), (err("expanded"), err("absorbed"))
+
+
+@pytest.mark.parametrize("segs", [[(0, 128, 1, 0)], [(0, 130, 2, 0), (130, 256, 0, 1030)]])
+def test_a_layer_that_borrows_its_latent(segs):
+    """own rows are neither normed nor written: the slots stay as they are, the launches go out in one call"""
+    from mlx_vlm_b200.models.decoder_blocks import StepCtx
+    from mlx_vlm_b200.models.layer_ops import LayerOps
+    m, pool, x = _layer(4, 128, 64, 128, 512, 96, False, False, 0, 3, kv_from=0)
+    assert m.expands and not m.own_kv
+    T = sum(n for _, n, _, _ in segs)
+    slot = torch.cat([torch.full((n,), s, dtype=torch.int32) for _, n, s, _ in segs]).cuda()
+    pos = torch.cat([torch.arange(p, p + n, dtype=torch.int32) for _, n, _, p in segs]).cuda()
+    cached = pool.buf.clone()
+    got = {}
+    for form in ("expanded", "absorbed", "rows"):
+        ops = LayerOps("cuda:0", torch.cuda.Stream())
+        ops.tc_enabled = form != "rows"
+        m.expands = form == "expanded"
+        torch.cuda.synchronize()
+        with ops.on_stream():
+            y = m.forward(StepCtx(ops, slot, pos, pool, 1e-5, segments=segs), x[:T].contiguous())
+        torch.cuda.synchronize()
+        assert ops.tc_enabled == (form != "rows") and torch.equal(pool.buf, cached)
+        got[form] = y.double()
+    err = lambda f: float((got[f] - got["rows"]).norm() / got["rows"].norm())
     assert err("expanded") < max(1.1 * err("absorbed"), 2.0 ** -8), (err("expanded"), err("absorbed"))
 
 
