@@ -80,6 +80,7 @@ from .layer_ops import (ACT_GELU, ACT_TANH, EPI_GELU, EPI_RELU2, EPI_SOFTCAP, EP
                         WAVELENGTH, LayerOps)
 
 EXPANDED_MAX = 1 << 29      # numbers of a slot's expanded keys and values (one GiB); a longer context keeps the absorbed form
+EXPANDED_PAIRS, EXPANDED_KEYS = 2048, 8192      # heads x tokens of a portion from which any context, keys up to which any portion is expanded
 
 
 @dataclass
@@ -220,14 +221,17 @@ class LatentAttention:
             self.w["uv"] = self.w["ukv"][self.H * self.dim:]
 
     def _expand_portions(self, ops: LayerOps, segs, cache_layer) -> bool:
-        """Whether a step's portions take the expanded form: from 128 tokens on, where the tensor cores take a step at all, it
-        was the faster at every context tried (128 tokens behind 4000: 239 -> 177 us a layer, 16 heads; 512 behind 8000: 583 ->
-        282; 2048 behind 6000: 2086 -> 385), and its distance from 64 bits is the smaller (0.0037 against 0.0041 there)."""
+        """Whether a step's portions take the expanded form: from 128 tokens on, where the tensor cores take a step at all.  Its
+        attention is a chain along the keys (1.8 us a tile of 128 in each of heads x tokens / 128 blocks), so few heads and tokens
+        behind a long context stay absorbed.  Absorbed against expanded, us a layer, 128 tokens behind 8000 / 16000 keys: 2 heads 258,
+        246 / 317, 363; 4 heads 268, 253 / 359, 388; 8 heads 297, 273 / 387, 416; 16 heads 342, 305 / 500, 467; 64 heads 671, 480 /
+        1183, 777; 1024 tokens, 4 heads 466, 283 / 705, 411.  Head dims from 64 + 32 / 64 to 192 / 128 and ranks from 64 to 512 moved the
+        line little.  The step is decided as a whole: one portion that has to stay absorbed keeps the others absorbed."""
         if not self.expands or not segs or cache_layer.dtype != torch.bfloat16:
             return False
         H, r, Dl, per = self.H, self.kv_rank, self.row_dim, self.H * (self.dim + self.vdim)
         return ops.tc_ok(min(n for _, n, _, _ in segs), r, Dl, cache_layer.stride(1)) and cache_layer.data_ptr() % 16 == 0 and \
-            max((p0 + n) * per for _, n, _, p0 in segs) <= EXPANDED_MAX
+            all((p0 + n) * per <= EXPANDED_MAX and (H * n >= EXPANDED_PAIRS or p0 + n <= EXPANDED_KEYS) for _, n, _, p0 in segs)
 
     def _one_call(self, ops: LayerOps, x, T: int, xb) -> bool:
         """whether all launches of the expanded form go out in one call (ops.latent_portions)"""

@@ -174,6 +174,9 @@ def test_what_keeps_the_absorbed_form():
     assert m._expand_portions(ops, [(0, 200, 0, 0)], rows)
     assert not m._expand_portions(ops, [(0, 200, 0, 0), (200, 100, 1, 0)], rows)             # a short portion
     assert not m._expand_portions(ops, [(0, 200, 0, EXPANDED_MAX // per)], rows)             # too long a context
+    assert m._expand_portions(ops, [(0, 200, 0, 8192 - 200)], rows) and m._expand_portions(ops, [(0, 512, 0, 100000)], rows)
+    assert not m._expand_portions(ops, [(0, 200, 0, 8193 - 200)], rows)                      # few heads and tokens, many keys
+    assert not m._expand_portions(ops, [(0, 512, 0, 100000), (512, 511, 1, 8192)], rows)
     assert not m._expand_portions(ops, None, rows) and not m._expand_portions(ops, [(0, 200, 0, 0)], rows.float())
     assert not m._expand_portions(ops, [(0, 200, 0, 0)], rows[..., 4:])                       # rows that do not start on 16 bytes
 
