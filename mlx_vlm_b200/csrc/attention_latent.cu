@@ -1,6 +1,6 @@
 // Causal attention of a prompt portion over keys and values expanded from latent cache rows: one pass over the keys, running
-// maximum and sum (rescaled only when the maximum grows by more than 2^8), probabilities rounded to bf16 before the division
-// by the row sum, fp32 sums.  The layer's prompt form without a window (models/decoder_blocks.py, LatentAttention).
+// maximum and sum (rescaled only when a weight would exceed 2^8, the conditional rescaling that FlashAttention 4 describes),
+// probabilities rounded to bf16 before the division by the row sum, fp32 sums.  The layer's prompt form without a window (models/decoder_blocks.py, LatentAttention).
 //
 //   q    bf16 [token][head][dn + dr]   the last dr rotated
 //   k    bf16 [key][head][dn]          expanded from the latent; the rotated part of a key is shared by the heads and read
@@ -203,7 +203,7 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         if (p.dr) l_tma_3d(Qs + kbn * LP_BLK, &tmQr, &bars.q_full, 0, h, row0);
         LpSlot sk{0, 1u}, sv{0, 1u};
         bool ok = true;
-        for (int j = 0; j < n_tiles + 2 && ok; ++j) {   // in the order of the products: K of tile j, then V of j - 2
+        for (int j = 0; j < n_tiles + 1 && ok; ++j) {   // K of tile j, then V of j - 1 (a tile ahead of its product)
           if (j < n_tiles) {
             if (!(ok = mbar_wait(&bars.k_empty[sk.i], sk.par, &failed))) break;
             ++k_loads;
@@ -213,7 +213,7 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
             if (p.dr) l_tma_3d(d + kbn * LP_BLK, &tmKr, &bars.k_full[sk.i], 0, 0, j * LP_TK);
             sk.step(1, nst);
           }
-          if (j >= 1 && j - 1 < n_tiles) {
+          if (j >= 1) {
             if (!(ok = mbar_wait(&bars.v_empty[sv.i], sv.par, &failed))) break;
             ++v_loads;
             l_expect_tx(&bars.v_full[sv.i], (uint32_t)vb * LP_BLK);
@@ -263,7 +263,8 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
           mbar_wait_issuer(&bars.p_full[g], par, dead);
           l_fence_after();
           const uint32_t va = v_lo + (uint32_t)(sv.i * vb * (LP_BLK >> 4));
-          const int n = keys16(j) >> 4;   // (groups of 16 keys that no query of the tile sees are left out)
+          const int n = keys16(j) >> 4;   // (groups of 16 keys that no query of the tile sees are left out; rows behind the last key
+                                          //  are zeros: the tensor maps end there)
 #pragma unroll
           for (int i = 0; i < LP_TK / 16; ++i) {
             if (i >= n) break;
@@ -362,18 +363,6 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       }
       sum[0] = add2(sum[0], sum[1]);
       l += f2_lo(sum[0]) + f2_hi(sum[0]);
-      // value rows behind the last key (a cache's unused rows) meet P = 0, but 0 times a NaN would still reach O
-      const int first = S - j * LP_TK, stop = (first + 15) & ~15;
-      if (first < LP_TK && first != stop) {
-        const int s = j % nst;
-        ok = __all_sync(0xffffffffu, mbar_wait(&bars.v_full[s], (j / nst) & 1, &failed));
-        if (!ok) break;
-        for (int i = threadIdx.x & 127; i < (stop - first) * vb * 8; i += 128) {
-          const int r = first + i / (vb * 8), ch = i % (vb * 8);
-          *reinterpret_cast<uint4*>(Vs + (s * vb + (ch >> 3)) * LP_BLK + r * 128 + (ch & 7) * 16) = make_uint4(0, 0, 0, 0);
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      }
       l_st_wait();
       l_fence_before();
       l_arrive(&bars.p_full[g]);
