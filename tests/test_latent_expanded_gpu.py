@@ -159,6 +159,24 @@ def test_a_layer_that_borrows_its_latent(segs):
     assert err("expanded") < max(1.1 * err("absorbed"), 2.0 ** -8), (err("expanded"), err("absorbed"))
 
 
+@pytest.mark.parametrize("gated", [False, "head"])
+def test_operand_rows_written_by_the_norm_before(gated):
+    """where the norm ahead left the step's bf16 operand rows (StepCtx.x_operand) they are read instead of x: the same sums"""
+    from mlx_vlm_b200.models.decoder_blocks import StepCtx
+    from mlx_vlm_b200.models.layer_ops import LayerOps
+    m, pool, x = _layer(4, 128, 64, 128, 512, 96, False, gated, 0, 5)
+    T, x = 300, x[:300].contiguous()
+    slot, pos = torch.zeros(T, dtype=torch.int32).cuda(), torch.arange(T, dtype=torch.int32).cuda()
+    ops, got = LayerOps("cuda:0", torch.cuda.Stream()), []
+    torch.cuda.synchronize()
+    with ops.on_stream():
+        for xb in (None, ops.to_bf16(x, x.shape[1])):
+            got.append(m.forward(StepCtx(ops, slot, pos, pool, 1e-5, segments=[(0, T, 0, 0)], x_operand=xb),
+                                 x if xb is None else torch.full_like(x, float("nan"))))
+    torch.cuda.synchronize()
+    assert ops.tc_enabled and torch.equal(*got)
+
+
 def test_what_keeps_the_absorbed_form():
     from mlx_vlm_b200.models.decoder_blocks import EXPANDED_MAX, LatentAttention
     base = {"heads": 4, "dim": 64, "rot_dim": 32, "vdim": 64, "kv_rank": 64, "scale": 0.1}

@@ -114,3 +114,30 @@ def test_swiglu_in_the_product(eng, T, inter, K, bias):
     both, raw = _parts(out)
     assert bool(((both - want).abs() <= bound).all())
     assert not raw[:, inter:out.n_pad].any() and not raw[:, out.n_pad + inter:].any()
+
+
+@pytest.mark.parametrize("T,inter", [(1, 4), (577, 1028), (130, 4304)])
+def test_swiglu_of_rows(eng, T, inter):
+    """the C entry for gate and up rows that lie in memory: fp32 arithmetic (a few ulps), the result keeps 16 mantissa bits"""
+    from mlx_vlm_b200 import _native as N
+    from mlx_vlm_b200.models.tower_ops import SplitBuf
+    gu = 3 * torch.randn(T, 2 * inter + 4, device="cuda")
+    out = SplitBuf(eng, T, inter)
+    N.check(eng.lib.b200_f32_swiglu_split(gu.data_ptr(), gu.stride(0), out.t.data_ptr(), out.ld, out.n_pad, T, inter, eng.s), "swiglu")
+    torch.cuda.synchronize()
+    want = torch.nn.functional.silu(gu[:, :inter].double()) * gu[:, inter:2 * inter].double()
+    both, raw = _parts(out)
+    assert bool(((both - want).abs() <= (2.0 ** -16 + 2.0 ** -20) * want.abs() + 1e-30).all())
+    assert not raw[:, inter:out.n_pad].any() and not raw[:, out.n_pad + inter:].any()
+
+
+def test_patches_of_channel_last_pixels(eng):
+    """the C entry without strides reads (B, H, W, C) as it lies"""
+    from mlx_vlm_b200 import _native as N
+    from mlx_vlm_b200.models.tower_ops import SplitBuf, TowerOps
+    pix = torch.randn(2, 28, 42, 3, device="cuda")
+    a, b = (SplitBuf(eng, 2 * 2 * 3, 588, padded=True) for _ in range(2))
+    TowerOps(eng).patchify(pix, 14, a)
+    N.check(eng.lib.b200_clip_patchify(pix.data_ptr(), 2, 28, 42, 3, 14, b.t.data_ptr(), b.n_pad, eng.s), "clip_patchify")
+    torch.cuda.synchronize()
+    assert torch.equal(a.t, b.t)
