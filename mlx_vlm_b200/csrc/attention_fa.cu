@@ -21,11 +21,12 @@
 // contiguous), which tcgen05 takes from the same 128-byte-swizzled 64-dim blocks that K uses.  So nothing transposes V:
 // a segment may start at any token (keys are a TMA coordinate without an alignment rule) and a later portion of a prompt
 // reads the cached keys and values where they are.  (V^T, [head][dim][key], is still taken by b200_attention_fa.)
-// A tile's time, from clock stamps (28 heads of 128): 1330 cycles in pass 1, of which the exponentials' 1024 are one part and
-// the two groups' loads and waits, which fall together, the other; 1450 in pass 2, where the thread that issues P.V is the
-// chain: 8 products of 64 cycles beside Q.K^T's, a wait for P and one for V.  With P in tensor memory instead of shared
-// memory, one commit for the value slot and the P tile, and half tiles that a warp's rows do not see left out: 2048 queries behind 2048 keys, 28 heads, 168.5 -> 164 us; 8 prompts of 608, 32 heads, 120 ->
-// 117.6; four pictures and a clip (6012 patches, 16 heads of 80) 131.5 -> 130.
+// A tile's time, from clock stamps (28 heads of 128): 1280 cycles in pass 1, of which the exponentials' 1024 are one part and
+// the two groups' loads and waits, which fall together, the other; 1350 in pass 2, where the thread that issues P.V is the
+// chain: 8 products of 64 cycles beside Q.K^T's, a wait for P and one for V.  P in tensor memory instead of shared memory, one
+// commit for the value slot and the P tile, half tiles that a warp's rows do not see left out, and waits that ask once before
+// they suspend, together (the kernel alone, cold L2): 2048 queries behind 2048 keys, 28 heads, 190.5 -> 186.4 us; 8 prompts of
+// 608, 32 heads, 129.0 -> 127.0; four pictures and a clip (6012 patches, 16 heads of 80) 146.2 -> 143.4.
 // Measured against the kernel without TMA that such calls fell back to (attention_tc.cu): 2048 queries behind 2048 cached
 // keys, 28 heads of 128: 1094 -> 354 us (249 with the pairwise softmax below); four pictures and a clip of four frames (6012
 // patches, 16 heads of 80), which start at odd offsets: 773 us in eight launches -> 236 us in one.

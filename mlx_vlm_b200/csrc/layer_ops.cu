@@ -1606,8 +1606,8 @@ int b200_lm_latent_queries(const float* q, long ldq, void* out, long ldo, const 
                    (cs || !rot_dims) && ldq >= (long)H * (dim + rot_dim) && ldo >= (long)H * (dim + rot_dim),
                "lm_latent_queries: bad argument");
   const bool vec = dim % 4 == 0 && rot_dim % 4 == 0 && ldq % 4 == 0 && ldo % 4 == 0 && ((uintptr_t)q & 15) == 0 && ((uintptr_t)out & 7) == 0;
-  if (vec) latent_queries_kernel<true><<<T, 256, 0, (cudaStream_t)st>>>(q, ldq, (bf16*)out, ldo, (const float2*)cs, H * (dim + rot_dim), dim, rot_dim, rot_dims, pairs, 0);
-  else latent_queries_kernel<false><<<T, 256, 0, (cudaStream_t)st>>>(q, ldq, (bf16*)out, ldo, (const float2*)cs, H * (dim + rot_dim), dim, rot_dim, rot_dims, pairs, 0);
+  const auto k = vec ? latent_queries_kernel<true> : latent_queries_kernel<false>;
+  k<<<T, 256, 0, (cudaStream_t)st>>>(q, ldq, (bf16*)out, ldo, (const float2*)cs, H * (dim + rot_dim), dim, rot_dim, rot_dims, pairs, 0);
   B200_CHECK_LAUNCH();
   return B200_OK;
 }
@@ -1615,20 +1615,23 @@ static long lp_bytes(long n) { return (n + 255) & ~255L; }
 static long lp_pad64(long n) { return (n + 63) / 64 * 64; }
 long b200_lm_latent_portions_ws(int T, int W, int n_down, int q_rank, int H, int dim, int rot_dim, int vdim, int longest) {
   const long nq = (long)H * (dim + rot_dim);
-  return lp_bytes(T * lp_pad64(W) * 2) + lp_bytes((long)T * n_down * 4) + (q_rank ? lp_bytes(T * lp_pad64(q_rank) * 2) + lp_bytes(T * nq * 4) : 0) +
-         lp_bytes(T * nq * 2) + lp_bytes((long)longest * H * (dim + vdim) * 2) + lp_bytes((long)T * H * vdim * 2);
+  return lp_bytes(T * lp_pad64(W) * 2) + lp_bytes((long)T * n_down * 4) +
+         (q_rank ? lp_bytes(T * lp_pad64(q_rank) * 2) + lp_bytes(T * nq * 4) : 0) + lp_bytes(T * nq * 2) +
+         lp_bytes((long)longest * H * (dim + vdim) * 2) + lp_bytes((long)T * H * vdim * 2);
 }
 // The launches of a step of prompt portions in the expanded form, one after the other.  Every kernel between the products is a
 // programmatic dependent launch (all weights are fixed, so that a product may ask for its own before the kernel ahead has ended),
-// the query latent is written as the operand of its product.  One by one from Python they took the host 197 us a layer, in this call 104; 2048 tokens, 16 heads: 164 -> 149 us.
-int b200_lm_latent_portions(const float* x, long ldx, const void* xb, int W, const void* down, int n_down, const void* dq_norm, const void* uq,
-                            const void* dkv_norm, const void* ukv, const void* o, float eps, void* cache, long slot_stride,
+// the query latent is written as the operand of its product.  One by one from Python they took the host 197 us a layer, in this
+// call 104; 2048 tokens, 16 heads: 164 -> 149 us.
+int b200_lm_latent_portions(const float* x, long ldx, const void* xb, int W, const void* down, int n_down, const void* dq_norm,
+                            const void* uq, const void* dkv_norm, const void* ukv, const void* o, float eps, void* cache, long slot_stride,
                             long tok_stride, const int* slot, const int* pos, const float* cs, int q_rank, int kv_rank, int H, int dim,
                             int rot_dim, int rot_dims, int vdim, int own_kv, int pairs, float scale, const int* segs, int n_seg, float* y,
                             long ldy, void* ws, long ws_bytes, int T, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
-  B200_REQUIRE((x || xb) && down && ukv && o && cache && segs && n_seg > 0 && y && ws && T > 0 && W > 0 && H > 0, "lm_latent_portions: bad argument");
-  B200_REQUIRE((q_rank == 0 || (dq_norm && uq)) && (!own_kv || (dkv_norm && slot && pos)) && (cs || !rot_dims) && rot_dims % 2 == 0 && rot_dims <= rot_dim,
+  B200_REQUIRE((x || xb) && down && ukv && o && cache && segs && n_seg > 0 && y && ws && T > 0 && W > 0 && H > 0 &&
+                   (q_rank == 0 || (dq_norm && uq)) && (!own_kv || (dkv_norm && slot && pos)) && (cs || !rot_dims) &&
+                   rot_dims % 2 == 0 && rot_dims <= rot_dim,
                "lm_latent_portions: bad argument");
   const long nq = (long)H * (dim + rot_dim), Wp = lp_pad64(W), qp = lp_pad64(q_rank), per = (long)H * (dim + vdim);
   const bool vec_x = xb || (W % 4 == 0 && ldx % 4 == 0 && ((uintptr_t)x & 15) == 0);

@@ -337,7 +337,8 @@ int f32_layer_norm(const float* x, long ldx, const void* w, const void* b, float
   B200_REQUIRE(x && T > 0 && N > 0 && (N % 4) == 0 && N <= 8192 && (ldx % 4) == 0, "f32_layer_norm: T=%d N=%d", T, N);
   B200_REQUIRE(out32 || out_split, "f32_layer_norm: no output");
   B200_REQUIRE(!out_split || ((ld_split % 4) == 0 && (n_pad % 4) == 0), "f32_layer_norm: split pitch");
-  // up to 2048 columns a warp holds a row in registers; rows of less than eight warps an SM are a chain of latencies that a
+  // up to 2048 columns a warp holds a row in registers (the towers' rows are 1024 to 1280 wide; wider ones were not tried); rows
+  // of less than eight warps an SM are a chain of latencies that a
   // CTA per row makes shorter (577 x 1024: 2.8 us, a warp per row 4.2; 1024 x 1152: 5.1 both)
   if (N <= 2048 && T >= 8 * 148) {
     const auto k = N <= 1024 ? f32_layer_norm_warp_kernel<8> : N <= 1280 ? f32_layer_norm_warp_kernel<10> : f32_layer_norm_warp_kernel<16>;

@@ -236,9 +236,12 @@ class LatentAttention:
     def _one_call(self, ops: LayerOps, x, T: int, xb) -> bool:
         """whether all launches of the expanded form go out in one call (ops.latent_portions)"""
         w = self.w
-        return (xb is None or (xb.stride(0) == (self.W + 63) // 64 * 64 and xb.data_ptr() % 16 == 0)) and not self.gated and (self.H * self.vdim) % 64 == 0 and x.dtype == torch.float32 and x.stride(0) % 4 == 0 and x.stride(1) == 1 and \
-            x.data_ptr() % 16 == 0 and self.W % 8 == 0 and w["down"].shape[0] % 4 == 0 and self.rot_dims % 2 == 0 and \
-            ops.tc_ok(T, self.W, self.q_rank) and all(w[n].data_ptr() % 16 == 0 for n in ("down", "ukv", "o"))
+        if self.gated or (self.H * self.vdim) % 64 or self.W % 8 or w["down"].shape[0] % 4 or self.rot_dims % 2:
+            return False
+        if xb is not None and (xb.stride(0) != (self.W + 63) // 64 * 64 or xb.data_ptr() % 16):
+            return False
+        rows = x.dtype == torch.float32 and x.stride(0) % 4 == 0 and x.stride(1) == 1 and x.data_ptr() % 16 == 0
+        return rows and ops.tc_ok(T, self.W, self.q_rank) and all(w[n].data_ptr() % 16 == 0 for n in ("down", "ukv", "o"))
 
     def _expanded(self, ctx: StepCtx, q, cs, segs, cache_layer) -> torch.Tensor:
         """Portions of prompts with the keys and values of their slots expanded from the cached rows: one product for both
