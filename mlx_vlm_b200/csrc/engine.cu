@@ -1055,7 +1055,7 @@ int b200_engine_prefill(b200_engine* e, const void* embeds, const int* pos3, int
   }
   if (all_logits_out) {  // the reference computes the head on every row (ar.py:358)
     if ((rc = rms_norm(h, e->norm, xn, T, (int)H, c.rms_eps, s))) return rc;
-    B200_REQUIRE(c.vocab % 8 == 0, "prefill (round-1 kernels): all-row logits need vocab %% 8 == 0");
+    B200_REQUIRE(c.vocab % 8 == 0, "prefill (kernels without TMA): all-row logits need vocab %% 8 == 0");
     if ((rc = gemm_bf16_tn(xn, H, e->head, nullptr, nullptr, 0, all_logits_out, c.vocab, T,
                            c.vocab, (int)H, B200_EPI_NONE, s)))
       return rc;
@@ -1093,7 +1093,7 @@ int b200_engine_prefill_batch(b200_engine* e, const void* embeds, const int* pos
   B200_REQUIRE(e && embeds && pos3 && n_seq > 0 && seq_len && rows, "engine_prefill_batch: bad arguments");
   int rc = resolve(e);
   if (rc) return rc;
-  B200_REQUIRE(e->kv && e->v2, "engine_prefill_batch: KV pool not bound / round-1 prefill kernels selected");
+  B200_REQUIRE(e->kv && e->v2, "engine_prefill_batch: KV pool not bound / prefill kernels without TMA selected");
   long T = 0;
   std::vector<PreSeg> segs(n_seq);
   for (int g = 0; g < n_seq; ++g) {

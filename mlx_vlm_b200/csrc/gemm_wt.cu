@@ -1321,7 +1321,7 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
         sps[2] = b < 1 ? 1 : (b > cap_k ? cap_k : b);
       }
       // (measured and discarded: restricting the list to <= 110 KB configurations so that the NEXT kernel's prologue
-      // can always co-reside under PDL made the C2 prefill 2-5 % slower)
+      // can always co-reside under PDL made the prefill of 272 tokens 2-5 % slower)
       for (int sp : sps) {
         add(tn, 2, 208 * 1024, sp);  // one CTA per SM, 256-byte weight-row bursts
         add(tn, 1, 110 * 1024, sp);  // two CTAs per SM

@@ -24,7 +24,7 @@ from ..tower_ops import EPI_GELU_TANH, SplitBuf, TowerOps
 def _arange_f32(start: float, stop: float, step: float) -> np.ndarray:
     """`mx.arange` on python floats: float32, element i = start + i * step with the product rounded to float32 (the Metal
     kernel of the device the reference runs on).  The buckets below are decided by `>=` between float32 values and an image
-    that fills the grid makes every comparison a tie, so this rounding is part of the reference's behaviour (DESIGN §7)."""
+    that fills the grid makes every comparison a tie, so this rounding is part of the reference's behaviour."""
     n = max(int(np.ceil((stop - start) / step)), 0)
     first = np.float32(start)
     inc = np.float32(np.float32(start + step) - first)

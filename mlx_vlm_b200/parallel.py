@@ -53,7 +53,7 @@ def max_over_ranks(values: Sequence[float], device=None, group=None) -> List[flo
 
 def generate_sharded(make_generator: Callable[[], Any], prompts: Sequence[Sequence[int]],
                      max_tokens, prompt_kwargs: Optional[List[dict]] = None, group=None) -> List[List[int]]:
-    """Config C5 on N replicas: request i runs on rank i % world (round-robin router), every rank drives
+    """Continuous batching on N replicas: request i runs on rank i % world (round-robin router), every rank drives
     its own `BatchGenerator` (`make_generator()` builds it around the rank's replica) to completion,
     and the generated token ids come back on EVERY rank in request order.  The only communication is
     the final gather of python lists — nothing per step."""

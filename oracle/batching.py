@@ -1,6 +1,6 @@
 """ORACLE — TEST INFRASTRUCTURE ONLY. Not imported by the product path.
 
-CPU restatement of the reference's LOCK-STEP batched generation (SURVEY §8 row a15, config C5): what a
+CPU restatement of the reference's LOCK-STEP batched generation: what a
 batched decode kernel has to reproduce.
   generate/ar.py:675-722   `_merge_prefill_prompt_kwargs`: per-row `inputs_embeds` (each row embedded on
                            its own, vision included) LEFT-padded with zeros to the longest prompt;
@@ -11,10 +11,10 @@ batched decode kernel has to reproduce.
   models/cache.py:24-42    mask: key j visible to query i of row b iff j <= i and j >= left_padding[b]
   models/qwen2_vl/language.py:404-518 decode positions: offset[b] + rope_delta[b] on all three axes
 
-The round-1 product time-multiplexes rows over the batch-1 engine, which is equivalent BY CONSTRUCTION
+Taking turns on the batch-1 engine is equivalent BY CONSTRUCTION
 to running every row alone; this module states the lock-step formulation and
 tests/test_oracle_batching.py shows it gives the same tokens / logits as the rows alone, i.e. it is the
-acceptance oracle for the round-2 batched kernel (padding positions are dead weight, not semantics).
+acceptance oracle for the batched kernels (padding positions are dead weight, not semantics).
 """
 from __future__ import annotations
 

@@ -1,6 +1,6 @@
 """ORACLE — TEST INFRASTRUCTURE ONLY. Not imported by the product path.
 
-CPU restatement of the reference's Idefics2 generate path (SURVEY §8 row a17, config C4):
+CPU restatement of the reference's Idefics2 generate path:
   models/idefics2/vision.py:123-173  patch embedding (Conv2d 14x14 + bias) and the BUCKETED
                                      fractional position ids (`np.digitize`; integer, bit-exact)
   models/idefics2/vision.py:20-120   SigLIP encoder: N x {LN, MHA with bias, LN, fast-GELU MLP}
@@ -11,7 +11,6 @@ CPU restatement of the reference's Idefics2 generate path (c
                                      patch mask, vision -> connector -> masked_scatter merge
   models/idefics2/language.py:16-150 Mistral decoder (nn.RoPE, no biases, untied head)
 
-PARITY STATUS: oracle only — the product kernels for this row are not built yet (round 2).
 Pinned (tests/test_oracle_idefics2.py): position ids / patch mask / padding-image removal /
 merge against the reference's own source (tests/golden/), the whole wiring in fp32 against
 HuggingFace transformers' Idefics2ForConditionalGeneration with the same weights.

@@ -1,6 +1,6 @@
 """ORACLE — TEST INFRASTRUCTURE ONLY. Not imported by the product path.
 
-CPU restatement of the reference's Idefics3 / SmolVLM generate path (SURVEY §8 f4; SmolVLM is an alias,
+CPU restatement of the reference's Idefics3 / SmolVLM generate path (SmolVLM is an alias,
 models/smolvlm/smolvlm.py):
   models/idefics3/vision.py:67-150   VisionEmbeddings: Conv2d 14x14 + bias on fp32 pixels, position ids = buckets of the
                                      fractional coordinates of the VALID block (sum(frac >= boundaries): the correct

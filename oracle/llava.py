@@ -1,6 +1,6 @@
 """ORACLE — TEST INFRASTRUCTURE ONLY. Not imported by the product path.
 
-CPU restatement of the reference's LLaVA-1.5 generate path:
+CPU restatement of the reference's LLaVA-1.5 generate path :
   models/llava/vision.py:108-185   CLIP ViT-L/14 tower (Conv2d patch embedding without bias,
                                    class token, learned positions, pre-LayerNorm, N x {LN, MHA
                                    with bias, LN, fast-GELU MLP}, all hidden states returned)
@@ -79,7 +79,7 @@ class LlavaCfg:
 
 
 def llava_15_7b() -> LlavaCfg:
-    """config C3 shapes."""
+    """LLaVA-1.5-7B shapes."""
     return LlavaCfg()
 
 

@@ -1,7 +1,7 @@
 """ORACLE — TEST INFRASTRUCTURE ONLY. Not imported by the product path.
 
 CPU restatement of the reference's LLaVA-Next (LLaVA-1.6) generate path, a sibling of LLaVA-1.5 that shares its
-tower, projector and language model (SURVEY §8 f4):
+tower, projector and language model:
   models/llava_next/llava_next.py:47-96    get_input_embeddings: `pixel_values[0]` = the crops of ONE image
                                            (N, C, H, W) -> NHWC -> CLIP tower on the N crops -> hidden state
                                            `vision_feature_layer` -> class token dropped ("default") -> projector ->

@@ -1,6 +1,6 @@
 """ORACLE — TEST INFRASTRUCTURE ONLY. Not imported by the product path.
 
-CPU restatement of the reference's Qwen2.5-VL generate path (SURVEY §8 f4).  The language model, the M-RoPE index, the
+CPU restatement of the reference's Qwen2.5-VL generate path.  The language model, the M-RoPE index, the
 merge and the generation loop are Qwen2-VL's (models/qwen2_5_vl/language.py and qwen2_5_vl.py differ from qwen2_vl's
 only in comments and in the tiling of text-only position ids) and are taken from oracle/qwen2vl.py; the vision tower is
 restated here:

@@ -110,7 +110,7 @@ def weight_shapes(cfg: Cfg) -> Dict[str, Tuple[int, ...]]:
     shapes: Dict[str, Tuple[int, ...]] = {}
     # HF layout [out, C, T, ps, ps]; the reference stores [out,T,ps,ps,C] after
     # vision.sanitize — both describe the same (out, C*T*ps*ps) GEMM when the
-    # pixel row is ordered (C,T,ps,ps)  (vision.py:92-98, SURVEY App. C).
+    # pixel row is ordered (C,T,ps,ps)  (vision.py:92-98).
     shapes["vision_tower.patch_embed.proj.weight"] = (
         E, v.in_channels, v.temporal_patch_size, v.patch_size, v.patch_size)
     for i in range(v.depth):
@@ -157,7 +157,7 @@ def weight_shapes(cfg: Cfg) -> Dict[str, Tuple[int, ...]]:
 
 def init_weights(cfg: Cfg, seed: int = 0, dtype: str = "bf16", std: float = 0.02,
                  norm_jitter: float = 0.0) -> Dict[str, torch.Tensor]:
-    """Seeded random-init weights (SURVEY §8d: N(0, 0.02), norm weights 1).
+    """Seeded random-init weights (N(0, 0.02), norm weights 1).
 
     One generator stream per tensor (seed, index) so that the SAME values can be
     regenerated tensor by tensor anywhere (CPU here, and uploaded to the GPU by
@@ -663,7 +663,7 @@ def greedy_generate(cfg: Cfg, W, input_ids, pixel_values, grid_thw, max_tokens: 
 
 
 # ---------------------------------------------------------------------------
-# synthetic request (SURVEY §8d C1/C2)
+# synthetic request
 # ---------------------------------------------------------------------------
 def synthetic_request(cfg: Cfg, n_text: int, image_hw=(336, 336), seed: int = 0,
                       text_vocab: Optional[int] = None):

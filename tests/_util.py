@@ -10,7 +10,7 @@ def to_dev(x, dtype=torch.bfloat16):
 def cmp_bf16(got: torch.Tensor, want: torch.Tensor, name="", rel_l2=1e-3, max_mismatch=0.02,
              ulps=2):
     """got: bf16 device tensor; want: fp32 CPU tensor of bf16-representable values.
-    Bar: relative L2 error <= rel_l2 (the north star's 1e-3), at most `max_mismatch`
+    Bar: relative L2 error <= rel_l2 (1e-3), at most `max_mismatch`
     of the elements differ at all, and no element differs by more than `ulps` bf16 ulps
     of max(|want|, tiny)."""
     g = got.detach().float().cpu().reshape(-1)

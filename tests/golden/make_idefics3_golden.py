@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Golden vectors for Idefics3 / SmolVLM (SURVEY §8 f4): the reference's own `Idefics3Connector.pixel_shuffle`
+"""Golden vectors for Idefics3 / SmolVLM: the reference's own `Idefics3Connector.pixel_shuffle`
 (mlx_vlm/models/idefics3/idefics3.py) and `VisionEmbeddings.__call__` (idefics3/vision.py: bucketed position ids —
 NOT Idefics2's digitize quirk —, ids written to the first `valid` positions, position embeddings zeroed on padding
 patches) are extracted with `ast` and EXECUTED over the numpy stand-in for mlx.core of make_golden.py.

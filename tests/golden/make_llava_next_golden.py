@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Golden vectors for LLaVA-Next (SURVEY §8 f4: a sibling of LLaVA-1.5 that shares its kernels): the reference's own
+"""Golden vectors for LLaVA-Next (a sibling of LLaVA-1.5 that shares its kernels): the reference's own
 `Model.get_input_embeddings` and `_merge_input_ids_with_image_features` (mlx_vlm/models/llava_next/llava_next.py:47-127)
 are extracted with `ast` from /root/reference and EXECUTED over the numpy stand-in for mlx.core of make_golden.py, with
 stub sub-modules (tower: deterministic hidden states per crop, projector: x -> 2x + 1, embedding table: row lookup),

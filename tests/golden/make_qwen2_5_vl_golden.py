@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Golden vectors for Qwen2.5-VL (SURVEY §8 f4): the reference's own `VisionModel.get_window_index`, `rot_pos_emb` and the
+"""Golden vectors for Qwen2.5-VL: the reference's own `VisionModel.get_window_index`, `rot_pos_emb` and the
 integer bookkeeping of `VisionModel.__call__` (mlx_vlm/models/qwen2_5_vl/vision.py: window permutation of the merge
 units, de-duplicated window boundaries, per-frame boundaries, which blocks see which, the reverse permutation after the
 merger) are extracted with `ast` and EXECUTED over the numpy stand-in for mlx.core of make_golden.py; the blocks and the

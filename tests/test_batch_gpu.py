@@ -1,4 +1,4 @@
-"""Lock-step batched decode on the GPU (csrc/decode_batch.cu; SURVEY §8 a15, config C5): rows that
+"""Lock-step batched decode on the GPU (csrc/decode_batch.cu): rows that
 share one weight stream must produce what each request produces alone.
 
 The batch-1 path (persistent k_mega) and the batched path (weight-major tcgen05 GEMMs + bd_attn)

@@ -1,4 +1,4 @@
-"""CPU: continuous-batching host logic (SURVEY §8 a15) and sampler / cache bookkeeping against
+"""CPU: continuous-batching host logic and sampler / cache bookkeeping against
 the reference's own function source (tests/golden/reference_golden.json, generated by
 tests/golden/make_golden.py).  The scheduling tests drive `BatchGenerator` with a deterministic
 stand-in for the engine (same call surface as mlx_vlm_b200.engine.Engine), so that

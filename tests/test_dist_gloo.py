@@ -39,7 +39,7 @@ def _worker(rank, world, port, ret):
     ok = ok and flat == list(range(11))
     mx = max_over_ranks([1.0 + rank, 5.0 - rank])
     ok = ok and mx == [float(world), 5.0]
-    # C5 host logic: 5 requests over 2 replicas, each rank drives its own BatchGenerator; the tokens
+    # host logic of the replicas: 5 requests over 2 replicas, each rank drives its own BatchGenerator; the tokens
     # every rank sees must equal the requests run alone (deterministic stand-in engine)
     import sys
     sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))

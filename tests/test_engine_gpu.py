@@ -8,7 +8,7 @@ Bars
     bit-exact;
   * stages whose INPUTS are identical to the oracle's (one decoder layer fed the
     oracle's hidden state, the fused head fed the oracle's final hidden state):
-    relative L2 <= 1e-3 (the north star's bar);
+    relative L2 <= 1e-3;
   * deep end-to-end outputs (ViT features after 32 blocks, logits after 28
     layers): `_util.cmp_noise` — a bf16 pipeline is chaotic (see its docstring), so
     the CUDA path must be no further from the oracle's bf16 result than that
@@ -273,7 +273,7 @@ def test_tensor_core_megakernel_parity(kind, mode):
 
 
 def test_batch_generator_rows_equal_single_requests():
-    """Continuous batching (SURVEY §8 a15) on the real engine: three requests (two with an
+    """Continuous batching on the real engine: three requests (two with an
     image, different lengths / max_tokens) time-multiplexed through BatchGenerator produce
     exactly the tokens each produces alone through generate_step."""
     import types
@@ -425,7 +425,7 @@ def test_merge_count_mismatch_raises():
 
 
 def test_full_size_c1():
-    """BASELINE config C1: Qwen2-VL-2B shapes, 1 image 336x336, 32 text tokens (+144
+    """Qwen2-VL-2B shapes, 1 image 336x336, 32 text tokens (+144
     image tokens), 64 greedy tokens — oracle (CPU) vs CUDA path."""
     from mlx_vlm_b200.generate import generate_step
     from oracle import qwen2vl as O
@@ -446,8 +446,8 @@ def test_full_size_c1():
         if got[n] != toks[n]:
             break
         if n < 4:
-            cmp_noise(lps[n], ref["logprobs"][n][0], ex["logprobs"][n][0], f"C1 logprobs step {n}")
+            cmp_noise(lps[n], ref["logprobs"][n][0], ex["logprobs"][n][0], f"logprobs step {n}")
         else:
             d = rl2(lps[n], ref["logprobs"][n][0])
-            assert d <= 2e-2, f"C1 step {n}: logprobs rel-L2 {d:.3e}"
-    print(f"C1: tokens equal to the oracle's: {got == toks}; first 8 {got[:8]} vs {toks[:8]}")
+            assert d <= 2e-2, f"step {n}: logprobs rel-L2 {d:.3e}"
+    print(f"tokens equal to the oracle's: {got == toks}; first 8 {got[:8]} vs {toks[:8]}")

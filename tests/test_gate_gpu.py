@@ -1,7 +1,6 @@
-"""Round-2 gate tests: the configurations that were benchmarked or
-claimed but had no parity test.
+"""Parity of the configurations that are benchmarked or claimed as a whole.
 
-  * C2 exactly as benched: Qwen2-VL-2B shapes, T = 128 + 144 = 272 prompt rows, 511 teacher-forced
+  * the headline benchmark's request: Qwen2-VL-2B shapes, T = 128 + 144 = 272 prompt rows, 511 teacher-forced
     decode steps (context up to 783): logits at steps {1, 128, 256, 511} against the oracle, K/V rows
     of layer 0 (identical inputs -> the 1e-3 bar) and of the last layer (deep -> noise bar);
   * Qwen2-VL-7B decoder GEOMETRY (28 q / 4 kv heads, hidden 3584, inter 18944; 2 layers) through the
@@ -61,7 +60,7 @@ def test_c2_as_benched_teacher_forced():
                          rope_deltas=np.asarray(deltas), logits_to_keep=1, reserve_tokens=T + n_out + 1)
     eng.stream.synchronize()
     cmp_noise(eng.logits_view(), O.lm_head(c, W, hid_b[:, T - 1], Rb)[0],
-              O.lm_head(c, W, hid_f[:, T - 1], R32)[0], "C2 prefill logits (step 0)")
+              O.lm_head(c, W, hid_f[:, T - 1], R32)[0], "prefill logits (step 0)")
     eng.set_next(int(forced[0]), T, T + delta)
     done = 0
     launches0 = eng.launch_count
@@ -75,18 +74,18 @@ def test_c2_as_benched_teacher_forced():
         done = step
         row = T + step - 1
         cmp_noise(eng.logits_view(), O.lm_head(c, W, hid_b[:, row], Rb)[0],
-                  O.lm_head(c, W, hid_f[:, row], R32)[0], f"C2 decode step {step} (ctx {row + 1}) logits")
+                  O.lm_head(c, W, hid_f[:, row], R32)[0], f"decode step {step} (ctx {row + 1}) logits")
     assert eng.device_error() == 0
     assert (eng.launch_count - launches0 - 4) == 511, "one launch per decode step (+1 state launch per call)"
     L = c.text.num_hidden_layers
-    cmp_bf16(cache[0].keys[0, :, :S_], cache_b[0].keys[0, :, :S_], "C2 K rows layer 0, ctx 783",
+    cmp_bf16(cache[0].keys[0, :, :S_], cache_b[0].keys[0, :, :S_], "K rows layer 0, ctx 783",
              rel_l2=1e-3, max_mismatch=0.02)
-    cmp_bf16(cache[0].values[0, :, :S_], cache_b[0].values[0, :, :S_], "C2 V rows layer 0, ctx 783",
+    cmp_bf16(cache[0].values[0, :, :S_], cache_b[0].values[0, :, :S_], "V rows layer 0, ctx 783",
              rel_l2=1e-3, max_mismatch=0.02)
     cmp_noise(cache[L - 1].keys[0, :, :S_], cache_b[L - 1].keys[0, :, :S_], cache_f[L - 1].keys[0, :, :S_],
-              "C2 K rows last layer, ctx 783")
+              "K rows last layer, ctx 783")
     cmp_noise(cache[L - 1].values[0, :, :S_], cache_b[L - 1].values[0, :, :S_],
-              cache_f[L - 1].values[0, :, :S_], "C2 V rows last layer, ctx 783")
+              cache_f[L - 1].values[0, :, :S_], "V rows last layer, ctx 783")
 
 
 def _cfg_7b_geometry():
@@ -259,7 +258,7 @@ def test_fused_greedy_decode_hook_has_the_reference_contract():
 
 
 def test_samplers_on_the_device():
-    """SURVEY §8 a13 on the GPU: (i) the sampler masks (top-k / top-p / min-p / top-n-sigma / p-less / typical-p) on
+    """On the GPU: (i) the sampler masks (top-k / top-p / min-p / top-n-sigma / p-less / typical-p) on
     DEVICE tensors against the goldens produced by the reference's own functions (tests/golden); (ii) the sampled
     generate path (temperature + top-p + top-k, seeded): every sampled token lies inside the oracle's nucleus for
     its step (teacher-forced on the tokens actually sampled), the yielded logprobs are the engine's, the run is

@@ -1,4 +1,4 @@
-"""Idefics2 product path on the GPU (SURVEY §8 a17, config C4) against oracle/idefics2.py: SigLIP tower with
+"""Idefics2 product path on the GPU against oracle/idefics2.py: SigLIP tower with
 bucketed position ids + modality projection + Perceiver resampler in fp32 with bf16-valued weights (the
 reference never casts float32 pixel_values), ONE rounding at the merge, Mistral LM in bf16."""
 import numpy as np

@@ -1,4 +1,4 @@
-"""Idefics3 / SmolVLM product path on the GPU (SURVEY §8 f4) against oracle/idefics3.py.  The reference runs this
+"""Idefics3 / SmolVLM product path on the GPU against oracle/idefics3.py.  The reference runs this
 tower in bf16; the product computes it at fp32 accuracy and rounds where the reference hands the pooled output over, so
 the end-to-end bar is the noise-relative one (tests/_util.cmp_noise): no further from the oracle's bf16 result than the
 oracle's bf16 result is from the exact evaluation.  The pixel shuffle is a permutation: bit-exact."""

@@ -1,4 +1,4 @@
-"""CPU: Idefics3 / SmolVLM (SURVEY §8 f4) — the oracle's and the product's integer logic against goldens produced by
+"""CPU: Idefics3 / SmolVLM — the oracle's and the product's integer logic against goldens produced by
 EXECUTING the reference's own source (tests/golden/make_idefics3_golden.py): pixel shuffle, position ids (correct
 buckets, ids written to the first n_valid positions, position embedding zeroed on padding patches); config rules."""
 import json

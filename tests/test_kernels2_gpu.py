@@ -1,4 +1,4 @@
-"""GPU parity of the round-2 ops (weight-major GEMM, finish_rows, pipelined attention, qkv post
+"""GPU parity of the prompt ops (weight-major GEMM, finish_rows, pipelined attention, qkv post
 kernel) against the oracle's restatement, through the C ABI.  Same bar as test_kernels_gpu.py:
 relative L2 <= 1e-3 with the oracle's rounding points mirrored."""
 import ctypes as C

@@ -1,4 +1,4 @@
-"""LLaVA-1.5 product path on the GPU (SURVEY §8 a16, config C3) against oracle/llava.py — the reference's
+"""LLaVA-1.5 product path on the GPU against oracle/llava.py — the reference's
 semantics: CLIP tower + projector in fp32 with bf16-valued weights, ONE rounding at the merge, Llama LM in
 bf16.  The tower ops are checked on their own against fp32 torch first (identical inputs: 1e-5), then the
 features at tiny and at CLIP-L widths, the merge (bit-exact copies) and the generate path."""
@@ -170,7 +170,7 @@ def test_llava_features_merge_and_generate(kind):
 
 
 def test_vision_feature_cache_through_the_server_loop():
-    """SURVEY §8 f1/f2: the GPU thread fills `VisionFeatureCache` on a miss (models with `encode_image`) and hands a
+    """the GPU thread fills `VisionFeatureCache` on a miss (models with `encode_image`) and hands a
     hit to the model as `cached_image_features` (server/generation.py:1636-1675, dispatch.py:800-809): the repeat of
     a request produces the same tokens without running the tower again."""
     import types

@@ -1,4 +1,4 @@
-"""LLaVA-Next product path on the GPU (SURVEY §8 f4, a sibling of LLaVA-1.5 on the same kernels) against
+"""LLaVA-Next product path on the GPU (a sibling of LLaVA-1.5 on the same kernels) against
 oracle/llava_next.py: the crops of one image through the fp32-accurate CLIP tower + projector, newline blocks, the
 growing merge (image rows pure copies in block order, text rows exact embeddings), greedy generation."""
 import numpy as np

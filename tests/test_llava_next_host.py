@@ -1,4 +1,4 @@
-"""CPU: LLaVA-Next (SURVEY §8 f4) — the oracle (oracle/llava_next.py) and the product's host logic
+"""CPU: LLaVA-Next — the oracle (oracle/llava_next.py) and the product's host logic
 (models/llava_next/llava_next.py::merge_plan) against the goldens produced by EXECUTING the reference's own
 `get_input_embeddings` / `_merge_input_ids_with_image_features` (tests/golden/make_llava_next_golden.py):
 crop selection, class-token drop, newline blocks along the crop axis, the growing merge and its zip() truncation."""

@@ -1,6 +1,6 @@
 """CPU: the lock-step batched formulation of the reference (left-padded rows, BatchKVCache write index,
-per-row rope deltas; oracle/batching.py) gives the same result as every row alone — the statement the
-round-1 time-multiplexed BatchGenerator relies on, and the acceptance oracle of a batched kernel."""
+per-row rope deltas; oracle/batching.py) gives the same result as every row alone — the statement that
+taking turns relies on, and the acceptance oracle of a batched kernel."""
 import numpy as np
 import torch
 

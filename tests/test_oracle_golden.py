@@ -195,7 +195,7 @@ def test_greedy_sampler_semantics():
 
 
 def test_load_path_key_renames_and_conv_layout_match_reference_source():
-    """SURVEY §8 a1: `Model.sanitize` (qwen2_vl.py:179-190) and the patch-embed layout rule
+    """`Model.sanitize` (qwen2_vl.py:179-190) and the patch-embed layout rule
     (vision.py:9-25, 292-310).  The reference normalises the conv weight to MLX [O,T,H,W,C]; the
     engine wants HF [O,C,T,H,W] (same linear map on (C,T,H,W)-ordered pixel rows): both layouts
     must come out as the HF tensor."""
@@ -219,7 +219,7 @@ def test_load_path_key_renames_and_conv_layout_match_reference_source():
 
 
 def test_image_processor_matches_reference_source_bit_exactly():
-    """SURVEY §8 a2: `Qwen3VLImageProcessor._process_one` (processing_qwen3_vl.py:302-354) executed
+    """`Qwen3VLImageProcessor._process_one` (processing_qwen3_vl.py:302-354) executed
     from the reference's source: smart_resize, PIL bicubic, rescale/normalise, temporal duplication,
     merge-group-major patch order.  Oracle and product must give the same bytes."""
     import hashlib
@@ -237,7 +237,7 @@ def test_image_processor_matches_reference_source_bit_exactly():
 
 
 def test_language_model_position_bookkeeping():
-    """SURVEY §8 a7 (language.py:404-518): prefill uses get_rope_index, chunks slice the stored ids,
+    """language.py:404-518: prefill uses get_rope_index, chunks slice the stored ids,
     decode steps use cache_offset + rope_delta on all three axes (== oracle.decode_position_ids),
     explicit position ids longer than the chunk are sliced at the cache offset."""
     lm = _product_lm()

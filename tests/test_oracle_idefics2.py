@@ -1,4 +1,4 @@
-"""CPU: the Idefics2 oracle (oracle/idefics2.py, SURVEY §8 row a17) pinned before any kernel is
+"""CPU: the Idefics2 oracle (oracle/idefics2.py) pinned before any kernel is
 written for it: the integer logic (bucketed position ids incl. the reference's negative buckets,
 pixel mask -> patch mask, padding-image removal, masked_scatter merge) against the reference's own
 source (tests/golden/make_golden.py), the wiring in fp32 against HuggingFace transformers."""

@@ -1,4 +1,4 @@
-"""CPU: the LLaVA-1.5 oracle (oracle/llava.py, SURVEY §8 row a16) is pinned before any kernel is
+"""CPU: the LLaVA-1.5 oracle (oracle/llava.py) is pinned before any kernel is
 written for it:
   * merge indexing against the reference's own function source (tests/golden/make_golden.py);
   * the whole wiring (CLIP tower incl. class token / positions / pre-LN / feature layer -2 / CLS
@@ -117,7 +117,7 @@ def test_llava_oracle_f32_matches_hf_transformers():
 def test_llava_vision_tower_is_fp32_in_the_reference():
     """The reference feeds float32 pixel_values to bf16 weights (llava.py:61-63, utils.py:2091): the
     tower runs in fp32.  A bf16 tower is a different (measurably noisier) function — quantified here
-    so that the round-2 kernel choice is explicit."""
+    so that the choice of fp32 kernels is explicit."""
     c = L.tiny_cfg()
     W = L.init_weights(c, seed=1)
     pv = L.synthetic_request(c, seed=2)["pixel_values"]

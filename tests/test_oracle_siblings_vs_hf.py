@@ -1,4 +1,4 @@
-"""Independent cross-check of the sibling oracles' WIRING (SURVEY §8c "HF-torch as tie-breaker"): HuggingFace transformers'
+"""Independent cross-check of the sibling oracles' WIRING (HF-torch as tie-breaker): HuggingFace transformers'
 torch implementations of Qwen2.5-VL and Idefics3 with the same random weights, in fp32, must give the same vision
 features and last-token logits as oracle/qwen2_5vl.py and oracle/idefics3.py in their un-rounded ("f32") mode.  This pins
 structure (window permutation and its inverse, windowed vs full attention blocks, RMSNorm / SwiGLU-with-bias blocks, 2-D

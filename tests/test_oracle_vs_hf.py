@@ -1,4 +1,4 @@
-"""Independent cross-check of the oracle's WIRING (SURVEY §8c "HF-torch as tie-breaker"):
+"""Independent cross-check of the oracle's WIRING (HF-torch as tie-breaker):
 HuggingFace transformers' torch Qwen2VLForConditionalGeneration with the same random
 weights, fp32, must give the same logits / vision features / M-RoPE position ids as the
 oracle in its un-rounded ("f32") mode.  This pins structure (layer order, QKV split,

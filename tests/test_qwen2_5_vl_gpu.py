@@ -1,4 +1,4 @@
-"""Qwen2.5-VL product path on the GPU (SURVEY §8 f4) against oracle/qwen2_5vl.py: the new device ops (2-D rotary on fp32
+"""Qwen2.5-VL product path on the GPU against oracle/qwen2_5vl.py: the new device ops (2-D rotary on fp32
 q / k, attention inside ragged segments, row gather) op by op against plain fp32 references, then the tower
 (window-ordered RMSNorm / SwiGLU blocks, windowed + full attention, merger, reverse order), the merge and greedy tokens.
 The reference runs this tower in bf16; the product computes it at fp32 accuracy from the bf16-rounded pixels and rounds the

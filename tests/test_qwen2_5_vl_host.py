@@ -1,4 +1,4 @@
-"""CPU: Qwen2.5-VL (SURVEY §8 f4) — the oracle's and the product's integer logic (window permutation of the merge units,
+"""CPU: Qwen2.5-VL — the oracle's and the product's integer logic (window permutation of the merge units,
 window / frame boundaries, rotary ids, reverse permutation) against goldens produced by EXECUTING the reference's own
 `VisionModel.get_window_index` / `rot_pos_emb` / `__call__` (tests/golden/make_qwen2_5_vl_golden.py); config rules."""
 import json

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""One warm batched prefill of the C3 request (8 x T=608 on the Llama-7B geometry) inside a cudaProfilerStart/Stop range,
+"""One warm batched prefill of eight LLaVA-1.5 prompts (8 x T=608 on the Llama-7B geometry) inside a cudaProfilerStart/Stop range,
 for `ncu --profile-from-start off --metrics gpu__time_duration.sum` (launch list of the final code).
 Prints the per-kernel totals itself when given an ncu csv:  python tools/c3_launch_list.py --summarise launches.csv"""
 import collections
@@ -26,7 +26,7 @@ def summarise(path):
         a[1] += float(x["Metric Value"].replace(",", "")) / 1e3
         n += 1
     tot = sum(a[1] for a in agg.values())
-    print(f"C3 batched LM prefill (8 x T=608, Llama-7B geometry), one call: {n} launches, {tot / 1e3:.2f} ms serialised under ncu")
+    print(f"batched LM prefill (8 x T=608, Llama-7B geometry), one call: {n} launches, {tot / 1e3:.2f} ms serialised under ncu")
     for (name, grid), (c, t) in sorted(agg.items(), key=lambda kv: -kv[1][1]):
         print(f"   {name:34s} grid {grid:18s} x{c:4d} {t:10.1f} us  avg {t / c:8.2f}  {100 * t / tot:5.1f} %")
 

@@ -1,4 +1,4 @@
-"""attention_fa vs attention_tc timing at the C2 shapes (CUDA-graph replay, CUDA events)."""
+"""attention_fa vs attention_tc timing at the shapes of the headline request (CUDA-graph replay, CUDA events)."""
 import os, sys
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 import torch

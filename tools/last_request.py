@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Per-kernel totals of the LAST request / step in an ncu launch list (gpu__time_duration.sum, csv):
-   python tools/last_request.py launches.csv c2     -> vision tower, LM prefill, decode steps of the last C2 request
+   python tools/last_request.py launches.csv c2     -> vision tower, LM prefill, decode steps of the last 2B request
    python tools/last_request.py launches.csv batch  -> the last lock-step decode step, launch by launch"""
 import collections
 import csv

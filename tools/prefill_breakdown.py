@@ -1,4 +1,4 @@
-"""GPU time of the C2 vision tower and LM prefill in isolation (CUDA events around N back-to-back
+"""GPU time of the headline request's vision tower and LM prefill in isolation (CUDA events around N back-to-back
 calls with no Python work in between), with the captured sequence graphs on / off.
 usage: [B200_SEQ_GRAPH=0] python tools/prefill_breakdown.py"""
 import os, sys, time

@@ -1,4 +1,4 @@
-"""Profiling target: C2 request, prefill once + a few decode steps as plain launches
+"""Profiling target: the headline request (2B, one picture), prefill once + a few decode steps as plain launches
 (no graph) so that ncu lists every kernel.  usage: profile_decode.py [n_steps] [graph]"""
 import sys, os
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))

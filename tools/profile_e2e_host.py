@@ -1,5 +1,5 @@
 """Where does the host time of generate(model, processor, prompt, image=<host array>) go?  cProfile of one warm call
-(C2 shapes) + wall-clock split: preprocessing / embeddings+prefill enqueue / decode loop / tail."""
+(the headline request's shapes) + wall-clock split: preprocessing / embeddings+prefill enqueue / decode loop / tail."""
 import cProfile, io, os, pstats, sys, time
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 import numpy as np, torch

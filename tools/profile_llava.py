@@ -1,4 +1,4 @@
-"""Profiling target for the fp32-accurate CLIP tower of LLaVA-1.5 (C3): CLIP-L/14-336 widths, n layers, B images,
+"""Profiling target for the fp32-accurate CLIP tower of LLaVA-1.5: CLIP-L/14-336 widths, n layers, B images,
 a few calls of encode_image so that ncu lists every kernel.  usage: profile_llava.py [layers] [B] [calls]"""
 import os, sys
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
