@@ -927,6 +927,9 @@ static int stream_geometry(StreamP& p, bool pair, int units /*rows or pairs avai
   const long unit = (long)p.K * 2 * (pair ? 2 : 1);
   int R = 8;
   while (R > 1 && (R * unit > 50 * 1024 || R > units)) R >>= 1;
+  // a warp holds its share of the activations in registers, at most ten vectors a lane (K of 2561 - 3200, 5121 - 6400 and 10241 -
+  // 12800, a 7B model's 11008 among them, would be more): fewer rows a tile, more warps to share a row
+  while (R > 1 && cdiv(cdiv(p.K >> 3, 8 / R), 32) > 10) R >>= 1;
   B200_REQUIRE(R * unit <= STREAM_SMEM_BUDGET / 2, "decode: K=%d too large for the weight ring", p.K);
   p.R = R;
   p.S = 8 / R;

@@ -380,6 +380,32 @@ def test_geometry_that_does_not_fit_the_persistent_kernel_falls_back_per_phase()
     assert per_step > 2, f"expected the per-phase path (several launches per step), got {per_step}"
 
 
+@pytest.mark.parametrize("inter", [2816, 5504, 10240, 11008, 12800])
+def test_per_phase_decode_of_any_mlp_width(inter):
+    """the widths at which a tile of the weight ring has to hold fewer rows for the activations to fit a warp's registers"""
+    from mlx_vlm_b200.models.cache import make_prompt_cache
+    from mlx_vlm_b200.models.qwen2_vl import Model
+    from oracle import qwen2vl as O
+    c = _mk_cfg("mha32")
+    c.text.intermediate_size = inter
+    W = O.init_weights(c, 0, norm_jitter=0.05)
+    model = Model(_to_model_config(c), device="cuda:0")
+    model.load_weights(W)
+    eng, ids = model.engine, np.arange(5, 16)[None]
+    ref = O.greedy_generate(c, W, ids, None, None, 2)
+    toks = ref["tokens"][0].tolist()
+    ex = O.greedy_generate(c, W, ids, None, None, 2, dtype="f32", force_tokens=toks[:])
+    emb = model.get_input_embeddings(ids, None)
+    model.language_model(ids, inputs_embeds=emb.inputs_embeds, cache=make_prompt_cache(model.language_model), position_ids=emb.position_ids)
+    T = ids.shape[1]
+    eng.set_next(toks[0], T, T)
+    launches = eng.launch_count
+    eng.decode(1, force_tokens=np.asarray([toks[1]], dtype=np.int32))
+    eng.stream.synchronize()
+    assert eng.launch_count - launches > 2 and eng.device_error() == 0
+    cmp_noise(eng.logits_view(), ref["logits"][1][0], ex["logits"][1][0], f"decode step, mlp of {inter}")
+
+
 def test_text_only_and_cache_reuse():
     """text-only request (qwen2_vl.py:34-42) + chunked prefill == one-shot prefill
     (reference tests/cache_invariants.py:47-115)."""
