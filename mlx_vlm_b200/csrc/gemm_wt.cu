@@ -412,7 +412,11 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   uint32_t tmem_cols = 32;
   while ((int)tmem_cols < p.TN) tmem_cols <<= 1;
 
-  w_pdl_launch();  // the next kernel may start its prologue / weight prefetch as SM resources free up
+  // The next kernel may start its prologue / weight prefetch as SM resources free up.  It may do so before this block has its columns:
+  // up to 256 of them, and what fits beside a block of 256 threads x 128 registers is one more like it; the kernels that ask for all
+  // 512 take more than the other half of the registers.  (Signalled behind the allocation: eight lock-step rows 383 -> 386 us, the
+  // latent prompt 152 -> 156, one picture 289 -> 286.)
+  w_pdl_launch();
 
   auto issue_w = [&](int it, int s) {
     uint8_t* sW = ring + (long)s * stage_bytes;
