@@ -81,6 +81,7 @@ int b200_gemm_bf16_tn(const void* A, long lda, const void* W, const void* bias,
                       int M, int N, int K, int epilogue, void* stream);
 
 #define B200_WT_FLAG_PAIR 8u /* b200_gemm_wt flags, with an explicit cfg4: CTA pairs (k-blocks per stage: 1) */
+#define B200_WT_FLAG_WIDE 16u /* the same with 512 instead of 256 weight rows a pair (not for B200_WT_PARTIAL) */
 /* The same Linear, weight-major (gemm_wt.cu): weight rows on the UMMA M side, TN tokens
  * (16..256) on the N side, optional split-K.  mode B200_WT_BF16 as b200_gemm_bf16_tn;
  * B200_WT_PARTIAL: fp32 tiles partial[split][T][N] (bias / residual applied by

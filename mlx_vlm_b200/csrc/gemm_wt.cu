@@ -148,17 +148,27 @@ __device__ __forceinline__ void w_tmem_ld32(uint32_t taddr, uint32_t* r) {
       : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void w_tmem_ld16(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void w_pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void w_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void w_ebar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void w_ebar(int id) { asm volatile("bar.sync %0, 256;" ::"r"(id) : "memory"); }
 
 // TMEM registers of one lane (weight row) -> bf16 staging tile [token][row]: + bias, one rounding, activation
-template <int EPI>
-__device__ __forceinline__ void wt_stage_bf16(const uint32_t (&a)[32], float bias_v, bf16* sb) {
+template <int EPI, int PER>
+__device__ __forceinline__ void wt_stage_bf16(const uint32_t (&a)[PER], float bias_v, bf16* sb) {
   const uint64_t bias2 = f2(bias_v, bias_v);
   unsigned short* s = reinterpret_cast<unsigned short*>(sb);
 #pragma unroll
-  for (int j = 0; j < 32; j += 2) {   // on pairs of tokens: this arithmetic is what bounds short products (gemm_wt_pair_kernel)
+  for (int j = 0; j < PER; j += 2) {   // on pairs of tokens: this arithmetic is what bounds short products (gemm_wt_pair_kernel)
     uint32_t v = pack_bf2(add2(f2(__uint_as_float(a[j]), __uint_as_float(a[j + 1])), bias2));
     if constexpr (EPI == B200_EPI_GELU_FAST) v = gelu_fast_bf2(v);
     if constexpr (EPI == B200_EPI_GELU_EXACT)
@@ -169,12 +179,12 @@ __device__ __forceinline__ void wt_stage_bf16(const uint32_t (&a)[32], float bia
 }
 
 // the fp32-accurate paths: no rounding anywhere
-template <int EPI>
-__device__ __forceinline__ void wt_stage_f32(const uint32_t (&a)[32], float bias_v, float* sf) {
+template <int EPI, int PER>
+__device__ __forceinline__ void wt_stage_f32(const uint32_t (&a)[PER], float bias_v, float* sf) {
   if constexpr (EPI == B200_EPI_GELU_FAST) {
     const uint64_t bias2 = f2(bias_v, bias_v), k = f2(1.702f, 1.702f);
 #pragma unroll
-    for (int j = 0; j < 32; j += 2) {
+    for (int j = 0; j < PER; j += 2) {
       uint64_t v = add2(f2(__uint_as_float(a[j]), __uint_as_float(a[j + 1])), bias2);
       v = mul2(v, sigmoid2(mul2(v, k)));
       sf[j * WT_ROWS] = f2_lo(v);
@@ -183,7 +193,7 @@ __device__ __forceinline__ void wt_stage_f32(const uint32_t (&a)[32], float bias
     return;
   }
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
+  for (int j = 0; j < PER; ++j) {
     float v = __uint_as_float(a[j]) + bias_v;
     if constexpr (EPI == B200_EPI_GELU_EXACT) v = v * (1.0f + erff(v / 1.41421356237309515f)) * 0.5f;
     if constexpr (EPI == B200_EPI_GELU_TANH) {
@@ -196,10 +206,11 @@ __device__ __forceinline__ void wt_stage_f32(const uint32_t (&a)[32], float bias
 
 // The accumulator tile (128 weight rows x TN tokens, fp32 in TMEM) -> its outputs, by 256 threads (tid; warp tid / 32 reads TMEM
 // lane quarter (tid / 32) mod 4, which must be its own) through a staging tile in shared memory.  dead: a wait of this CTA
-// ended without its data, NaN is stored.
-template <bool TOWER>
+// ended without its data, NaN is stored.  TOK: tokens staged at a time; bar: the named barrier of these threads.
+template <bool TOWER, int TOK = WT_EPI_TOK>
 __device__ __forceinline__ void wt_store_tile(const WtParams& p, uint8_t* stg, uint32_t tmem, int n0, int t0, long cg, int split,
-                                              int tid, bool dead) {
+                                              int tid, bool dead, int bar = 1) {
+  constexpr int PER = TOK / 2;
   const int warp = tid >> 5, lane = tid & 31, q = warp & 3, half = warp >> 2;
   const int row = q * 32 + lane;  // weight row of the tile == TMEM lane
   float bias_v = 0.f;
@@ -212,40 +223,41 @@ __device__ __forceinline__ void wt_store_tile(const WtParams& p, uint8_t* stg, u
   } else if (p.mode == B200_WT_BF16 && p.bias && n0 + row < p.N) {
     bias_v = bf2f(p.bias[n0 + row]);
   }
-  for (int c0 = 0; c0 < p.TN; c0 += WT_EPI_TOK) {
-    const int cc = c0 + half * 32;
+  for (int c0 = 0; c0 < p.TN; c0 += TOK) {
+    const int cc = c0 + half * PER;
     if (cc < p.TN && !(p.flags & 1u)) {
-      uint32_t a[32];
-      w_tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cc, a);
+      uint32_t a[PER];
+      if constexpr (PER == 32) w_tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cc, a);
+      else w_tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cc, a);
       if (dead)
-        for (int j = 0; j < 32; ++j) a[j] = 0x7FC00000u;
+        for (int j = 0; j < PER; ++j) a[j] = 0x7FC00000u;
       if (!TOWER && p.mode == B200_WT_PARTIAL) {
         float* sf = reinterpret_cast<float*>(stg);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) sf[(half * 32 + j) * WT_ROWS + row] = __uint_as_float(a[j]);
+        for (int j = 0; j < PER; ++j) sf[(half * PER + j) * WT_ROWS + row] = __uint_as_float(a[j]);
       } else if constexpr (TOWER) {
-        float* sf = reinterpret_cast<float*>(stg) + (half * 32) * WT_ROWS + row;
-        if (p.epilogue == B200_EPI_GELU_FAST) wt_stage_f32<B200_EPI_GELU_FAST>(a, bias_v, sf);
-        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_stage_f32<B200_EPI_GELU_EXACT>(a, bias_v, sf);
-        else if (p.epilogue == B200_EPI_GELU_TANH) wt_stage_f32<B200_EPI_GELU_TANH>(a, bias_v, sf);
-        else wt_stage_f32<B200_EPI_NONE>(a, bias_v, sf);
+        float* sf = reinterpret_cast<float*>(stg) + (half * PER) * WT_ROWS + row;
+        if (p.epilogue == B200_EPI_GELU_FAST) wt_stage_f32<B200_EPI_GELU_FAST, PER>(a, bias_v, sf);
+        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_stage_f32<B200_EPI_GELU_EXACT, PER>(a, bias_v, sf);
+        else if (p.epilogue == B200_EPI_GELU_TANH) wt_stage_f32<B200_EPI_GELU_TANH, PER>(a, bias_v, sf);
+        else wt_stage_f32<B200_EPI_NONE, PER>(a, bias_v, sf);
       } else {
         // one unrolled loop per epilogue kind, chosen OUTSIDE the loop: left to itself the compiler merged the
         // three kinds into one predicated body of ~90 instructions per element (6-7 us per launch, A/B measured)
-        bf16* sb = reinterpret_cast<bf16*>(stg) + (half * 32) * WT_ROWS + row;
-        if (p.epilogue == B200_EPI_GELU_FAST) wt_stage_bf16<B200_EPI_GELU_FAST>(a, bias_v, sb);
-        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_stage_bf16<B200_EPI_GELU_EXACT>(a, bias_v, sb);
-        else wt_stage_bf16<B200_EPI_NONE>(a, bias_v, sb);
+        bf16* sb = reinterpret_cast<bf16*>(stg) + (half * PER) * WT_ROWS + row;
+        if (p.epilogue == B200_EPI_GELU_FAST) wt_stage_bf16<B200_EPI_GELU_FAST, PER>(a, bias_v, sb);
+        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_stage_bf16<B200_EPI_GELU_EXACT, PER>(a, bias_v, sb);
+        else wt_stage_bf16<B200_EPI_NONE, PER>(a, bias_v, sb);
       }
     }
-    w_ebar();
+    w_ebar(bar);
     if (!(p.flags & 4u)) {
       if (!TOWER && p.mode == B200_WT_BF16) {
         const bool vec_all = ((p.ldc & 7) == 0) && (!p.residual || (p.ldr & 7) == 0) &&
                             ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0) &&
                             (!p.residual || (reinterpret_cast<uintptr_t>(p.residual) & 15) == 0);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < TOK / 16; ++u) {
           const int idx = tid + 256 * u;
           const int tl = idx >> 4, ch = idx & 15;
           const int t = t0 + c0 + tl, n = n0 + ch * 8;
@@ -275,7 +287,7 @@ __device__ __forceinline__ void wt_store_tile(const WtParams& p, uint8_t* stg, u
         }
       } else if (!TOWER && p.mode == B200_WT_SWIGLU) {
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < TOK / 32; ++u) {
           const int idx = tid + 256 * u;
           const int tl = idx >> 3, ch = idx & 7;
           const int t = t0 + c0 + tl, i = n0 + ch * 8;
@@ -289,7 +301,7 @@ __device__ __forceinline__ void wt_store_tile(const WtParams& p, uint8_t* stg, u
         // silu(gate) * up in fp32, as the next product's operand: the [T, 2 inter] fp32 rows between the two never reach memory.
         // 4096 tokens x 28672 rows x 1152 (two parts) with a kernel of its own behind it 399 + 115 us (and 60 to clear its rows), this 396.
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < TOK / 16; ++u) {
           const int idx = tid + 256 * u;
           const int tl = idx >> 4, ch = idx & 15;
           const int t = t0 + c0 + tl, i = n0 + ch * 4;
@@ -308,7 +320,7 @@ __device__ __forceinline__ void wt_store_tile(const WtParams& p, uint8_t* stg, u
         }
       } else if constexpr (TOWER) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = 0; u < TOK / 8; ++u) {
           const int idx = tid + 256 * u;
           const int tl = idx >> 5, ch = idx & 31;
           const int t = t0 + c0 + tl, n = n0 + ch * 4;
@@ -349,7 +361,7 @@ __device__ __forceinline__ void wt_store_tile(const WtParams& p, uint8_t* stg, u
         }
       } else {  // fp32 partial tile -> P[split][t][n]
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = 0; u < TOK / 8; ++u) {
           const int idx = tid + 256 * u;
           const int tl = idx >> 5, ch = idx & 31;
           const int t = t0 + c0 + tl, n = n0 + ch * 4;
@@ -365,7 +377,7 @@ __device__ __forceinline__ void wt_store_tile(const WtParams& p, uint8_t* stg, u
         }
       }
     }
-    w_ebar();
+    w_ebar(bar);
   }
 }
 
@@ -544,13 +556,24 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
 //   warp 0  TMA producer of this CTA's operands; the bytes of both CTAs count on the leader's (rank 0) full barrier
 //   warp 1  leader only: MMA issuer; its commits free the slot / hand the accumulator over in both CTAs
 //   warp 2  TMEM
-//   warps 4..11  epilogue of this CTA's 128 weight rows
+//   warps 4..11  epilogue of this CTA's 128 weight rows (wide: of the first 128, warps 12..19 of the others)
 // Tiles are dealt out round robin, token tile first, so that the pairs of a wave share weight rows in the L2.
 // Up to about 3600 columns of k the epilogue's arithmetic shows: its eight warps have as long as the products of a tile take.  In
 // pairs of tokens (packed additions and bf16 products, ex2 and rcp without their slow ranges: about 9 instructions an element for
 // the fast GELU instead of some 45): 6012 x 5120 x 1280 with GELU 91 -> 66 us (65 without GELU, 54 without any epilogue).
+// HALVES = 2, "wide": 512 weight rows a pair, 256 of each CTA as two accumulators of 128 x TN that share the token operand.  What
+// bounds the pairs of 256 rows with long k is their fill, 32 KB of each CTA for 512 cycles of products (64 bytes a cycle, where
+// all SMs together got 42 - 53 out of the L2); here 48 KB serve 1024 cycles.  All of the tensor memory is taken, so
+// a tile's accumulators are read while the tensor core works on the other half: the second half's products run WP_LAG k-blocks
+// behind the first's where a tile begins and ends, and eight epilogue warps belong to each half.  256 -> 512 rows, back to back:
+// 2048 tokens x 3584 rows x 18944 207 -> 188 us, 4864 x 4096 x 11008 324 -> 300, 4096 x 4096 x 28672 675 -> 623 (under the
+// power limit 243 -> 222, 376 -> 353, 776 -> 728; one-CTA tiles 273, 465, 861).  With k below some 3000 the ends of a tile cost
+// more than the fill saves (6012 x 3840 x 1280 45 -> 56, 4096 x 28672 x 2304 367 -> 390).  WP_LAG 0 / 1 / 2 / 3 / 4:
+// 2048 x 37888 x 3584 371 / 375 / 365 / 363 / 363, 6012 x 5120 x 1280 93 / 92 / 88 / 84 / 83.
 // ---------------------------------------------------------------------------------------------
-constexpr int WP_THREADS = 384;
+constexpr int WP_THREADS = 384, WP_WIDE_THREADS = 640;
+constexpr int WP_LAG = 3;                                   // (at most the ring's stages, which are held meanwhile)
+constexpr int WP_WIDE_STAGING = WT_EPI_TOK * WT_ROWS * 2;   // bytes for each half's warps: 64 tokens in bf16, 32 in fp32
 constexpr int WP_MAX_STAGES = 12;
 
 struct WpBars {
@@ -590,8 +613,8 @@ __device__ __forceinline__ void wp_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <bool TOWER>
-__global__ void __launch_bounds__(WP_THREADS, 1)
+template <bool TOWER, int HALVES>
+__global__ void __launch_bounds__(HALVES == 2 ? WP_WIDE_THREADS : WP_THREADS, 1)
 gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const WtParams p) {
   extern __shared__ uint8_t wt_smem_raw[];
   __shared__ WpBars bars;
@@ -601,10 +624,11 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const bool swiglu = p.mode == (TOWER ? B200_WT_SWIGLU_SPLIT : B200_WT_SWIGLU);
-  const int xhalf = p.TN / 2, stage_bytes = WT_WBLK + xhalf * 128, NS = p.n_stages;
+  const int xhalf = p.TN / 2, stage_bytes = HALVES * WT_WBLK + xhalf * 128, NS = p.n_stages;
   uint8_t* stg = ring + (long)NS * stage_bytes;
   const int kb_total = (p.K + WT_BK - 1) / WT_BK;
-  const int row_tiles = ((swiglu ? 2 * p.inter : p.N) + 2 * WT_ROWS - 1) / (2 * WT_ROWS), tok_tiles = (p.T + p.TN - 1) / p.TN;
+  const int unit = swiglu ? 64 : WT_ROWS;   // output features of 128 weight rows
+  const int row_tiles = ((swiglu ? 2 * p.inter : p.N) + 2 * HALVES * WT_ROWS - 1) / (2 * HALVES * WT_ROWS), tok_tiles = (p.T + p.TN - 1) / p.TN;
   const int splits = (kb_total + p.kb_per_split - 1) / p.kb_per_split;
   const int n_tiles = row_tiles * tok_tiles * splits;
   int s_next = 0;             // the producer's next slot
@@ -613,7 +637,7 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   auto tile_at = [&](int tile, int& n0, int& t0, int& split, int& kb0, int& kb1) {
     t0 = tile % tok_tiles * p.TN;
     tile /= tok_tiles;
-    n0 = (tile % row_tiles * 2 + rank) * (swiglu ? 64 : WT_ROWS);
+    n0 = (tile % row_tiles * 2 * HALVES + rank) * unit;   // (the second half's: 2 units on)
     split = tile / row_tiles;
     kb0 = split * p.kb_per_split;
     kb1 = min(kb_total, kb0 + p.kb_per_split);
@@ -656,15 +680,15 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
         uint8_t* sW = ring + (long)s * stage_bytes;
         const uint32_t bar = full0 + s * 8;
         if (rank == 0) w_mbar_expect_tx(&bars.full[s], 2u * (uint32_t)stage_bytes);
-        if (swiglu) {
-          wp_tma_2d(sW, &tmW, bar, kb * WT_BK, n0);
-          wp_tma_2d(sW + 64 * 128, &tmW, bar, kb * WT_BK, p.inter + n0);
-        } else {
-          wp_tma_2d(sW, &tmW, bar, kb * WT_BK, n0);
+#pragma unroll
+        for (int h = 0; h < HALVES; ++h) {
+          const int n = n0 + h * 2 * unit;
+          wp_tma_2d(sW + h * WT_WBLK, &tmW, bar, kb * WT_BK, n);
+          if (swiglu) wp_tma_2d(sW + h * WT_WBLK + 64 * 128, &tmW, bar, kb * WT_BK, p.inter + n);
         }
       };
       auto load_x = [&](int s, int kb, int t0) {
-        wp_tma_2d(ring + (long)s * stage_bytes + WT_WBLK, &tmX, full0 + s * 8, kb * WT_BK, t0 + rank * xhalf);
+        wp_tma_2d(ring + (long)s * stage_bytes + HALVES * WT_WBLK, &tmX, full0 + s * 8, kb * WT_BK, t0 + rank * xhalf);
       };
       int n0, t0, split, kb0, kb1;
       // weights never depend on the previous kernel: those of the first slots are requested before waiting for it
@@ -698,32 +722,89 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       // D = f32, A = B = bf16, both K-major; M = 256 weight rows, N = TN tokens
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.TN >> 3) << 17) | (16u << 24);
       // (slot and parity are counted along: a division per k-block would cost more than its four products)
-      const uint32_t w_first = w_desc_lo(w_smem_u32(ring)), x_first = w_desc_lo(w_smem_u32(ring + WT_WBLK));
+      const uint32_t w_first = w_desc_lo(w_smem_u32(ring)), x_first = w_desc_lo(w_smem_u32(ring + HALVES * WT_WBLK));
       const uint32_t step = (uint32_t)stage_bytes >> 4;
       int s = 0, j = 0, n0, t0, split, kb0, kb1;
       uint32_t w_lo = w_first, x_lo = x_first, parity = 0;
       bool dead = false;
       w_pdl_wait();   // (the time of a wait starts when the tokens can be on their way)
-      for (int tile = pair; tile < n_tiles; tile += n_pairs, ++j) {
-        tile_at(tile, n0, t0, split, kb0, kb1);
-        const uint32_t d = tmem + (uint32_t)(j & 1) * 256u;
-        mbar_wait_issuer(&bars.acc_empty[j & 1], ((j >> 1) & 1) ^ 1, dead);
-        w_fence_after();
-        uint32_t acc = 0;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          mbar_wait_issuer(&bars.full[s], parity, dead);
-          w_fence_after();
+      if constexpr (HALVES == 2) {
+        // the products of k-block s with one half of the weight rows
+        auto half = [&](int h, uint32_t acc) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            wp_umma(d, w_lo + k * 2, x_lo + k * 2, idesc, acc);
-            acc = 1;
-          }
-          wp_commit(dead ? &bars.dropped : &bars.empty[s]);
+          for (int k = 0; k < 4; ++k) wp_umma(tmem + h * 256u, w_lo + h * (WT_WBLK >> 4) + k * 2, x_lo + k * 2, idesc, k > 0 ? 1u : acc);
+        };
+        auto next = [&] {
           w_lo += step;
           x_lo += step;
           if (++s == NS) s = 0, w_lo = w_first, x_lo = x_first, parity ^= 1;
+        };
+        auto arrived = [&] {
+          mbar_wait_issuer(&bars.full[s], parity, dead);
+          w_fence_after();
+        };
+        for (int tile = pair; tile < n_tiles; tile += n_pairs, ++j) {
+          tile_at(tile, n0, t0, split, kb0, kb1);
+          const int nk = kb1 - kb0, lag = min(min(WP_LAG, NS), nk >> 1);
+          const uint32_t free_par = (j & 1) ^ 1;
+          mbar_wait_issuer(&bars.acc_empty[0], free_par, dead);
+          w_fence_after();
+          // the first k-blocks: the second half lags behind, its accumulator is still being read (their slots are full: no waits)
+          int s0 = s;
+          uint32_t w0 = w_lo, x0 = x_lo, p0 = parity;
+          for (int i = 0; i < lag; ++i, next()) {
+            arrived();
+            half(0, i > 0);
+          }
+          mbar_wait_issuer(&bars.acc_empty[1], free_par, dead);
+          w_fence_after();
+          if (lag > 0) s = s0, w_lo = w0, x_lo = x0, parity = p0;
+          for (int i = 0; i < lag; ++i, next()) {
+            half(1, i > 0);
+            wp_commit(dead ? &bars.dropped : &bars.empty[s]);
+          }
+          for (int i = lag; i < nk - lag; ++i, next()) {
+            arrived();
+            half(0, i > 0);
+            half(1, i > 0);
+            wp_commit(dead ? &bars.dropped : &bars.empty[s]);
+          }
+          // the last ones: the first half is whole before the second's products begin
+          s0 = s, w0 = w_lo, x0 = x_lo, p0 = parity;
+          for (int i = 0; i < lag; ++i, next()) {
+            arrived();
+            half(0, 1u);
+          }
+          wp_commit(dead ? &bars.dropped : &bars.acc_full[0]);
+          if (lag > 0) s = s0, w_lo = w0, x_lo = x0, parity = p0;
+          for (int i = 0; i < lag; ++i, next()) {
+            half(1, 1u);
+            wp_commit(dead ? &bars.dropped : &bars.empty[s]);
+          }
+          wp_commit(dead ? &bars.dropped : &bars.acc_full[1]);
         }
-        wp_commit(dead ? &bars.dropped : &bars.acc_full[j & 1]);   // (an accumulator that is not whole is not handed over)
+      } else {
+        for (int tile = pair; tile < n_tiles; tile += n_pairs, ++j) {
+          tile_at(tile, n0, t0, split, kb0, kb1);
+          const uint32_t d = tmem + (uint32_t)(j & 1) * 256u;
+          mbar_wait_issuer(&bars.acc_empty[j & 1], ((j >> 1) & 1) ^ 1, dead);
+          w_fence_after();
+          uint32_t acc = 0;
+          for (int kb = kb0; kb < kb1; ++kb) {
+            mbar_wait_issuer(&bars.full[s], parity, dead);
+            w_fence_after();
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              wp_umma(d, w_lo + k * 2, x_lo + k * 2, idesc, acc);
+              acc = 1;
+            }
+            wp_commit(dead ? &bars.dropped : &bars.empty[s]);
+            w_lo += step;
+            x_lo += step;
+            if (++s == NS) s = 0, w_lo = w_first, x_lo = x_first, parity ^= 1;
+          }
+          wp_commit(dead ? &bars.dropped : &bars.acc_full[j & 1]);   // (an accumulator that is not whole is not handed over)
+        }
       }
       if (dead) *static_cast<volatile int*>(&failed) = 1;
     }
@@ -731,15 +812,18 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     w_pdl_wait();
     int j = 0, n0, t0, split, kb0, kb1;
     bool ok = true;   // (the same in a warp)
+    const int half = HALVES == 2 ? (warp - 4) >> 3 : 0;   // eight warps to a half
     for (int tile = pair; tile < n_tiles; tile += n_pairs, ++j) {
       tile_at(tile, n0, t0, split, kb0, kb1);
-      ok = ok && __all_sync(0xffffffffu, mbar_wait(&bars.acc_full[j & 1], (j >> 1) & 1, &failed));
+      const int a = HALVES == 2 ? half : j & 1;   // accumulator
+      ok = ok && __all_sync(0xffffffffu, mbar_wait(&bars.acc_full[a], (HALVES == 2 ? j : j >> 1) & 1, &failed));
       w_fence_after();
-      wt_store_tile<TOWER>(p, stg, tmem + (uint32_t)(j & 1) * 256u, n0, t0, 0, split, threadIdx.x - 128, !ok);
+      wt_store_tile<TOWER, HALVES == 2 && TOWER ? 32 : WT_EPI_TOK>(p, stg + half * WP_WIDE_STAGING, tmem + (uint32_t)a * 256u, n0 + half * 2 * unit, t0, 0,
+                                                                   split, (int)(threadIdx.x - 128) & 255, !ok, 1 + half);
       w_fence_before();
       __syncwarp();
       if (lane == 0)
-        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(wp_leader(&bars.acc_empty[j & 1]))
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(wp_leader(&bars.acc_empty[a]))
                      : "memory");
     }
   }
@@ -991,8 +1075,10 @@ void gemm_wt_set_pdl(bool on) { g_wt_pdl = on; }
 static int round16(int x) { return (x + 15) & ~15; }
 
 constexpr int WP_PAIRS = 74;   // pairs of SMs
+constexpr int WT_KS_WIDE = -1; // WtConfig::KS of a pair with 512 weight rows (0: 256)
 static bool wt_swiglu(int mode) { return mode == B200_WT_SWIGLU || mode == B200_WT_SWIGLU_SPLIT; }
-static size_t wp_staging(int mode) {   // the epilogue's staging tile: WT_EPI_TOK tokens x 128 rows
+static size_t wp_staging(int mode, bool wide) {   // the epilogue's staging tile: WT_EPI_TOK tokens x 128 rows
+  if (wide) return 2 * WP_WIDE_STAGING;
   return (size_t)WT_EPI_TOK * WT_ROWS * (mode == B200_WT_BF16 || mode == B200_WT_SWIGLU ? 2 : 4);
 }
 
@@ -1090,9 +1176,9 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
   B200_REQUIRE(T > 0 && N > 0 && K > 0, "gemm_wt: empty problem T=%d N=%d K=%d", T, N, K);
   B200_REQUIRE((ldx % 8) == 0 && (K % 8) == 0, "gemm_wt: ldx (%ld) and K (%d) must be multiples of 8", ldx, K);
   B200_REQUIRE(((uintptr_t)X & 15) == 0 && ((uintptr_t)W & 15) == 0, "gemm_wt: X and W must be 16-byte aligned");
-  const bool pair = cfg.KS == 0;   // CTA pairs
+  const bool pair = cfg.KS <= 0, wide = cfg.KS == WT_KS_WIDE;   // CTA pairs
   B200_REQUIRE(cfg.TN >= 16 && cfg.TN <= 256 && (cfg.TN % (pair ? 32 : 16)) == 0, "gemm_wt: TN=%d", cfg.TN);
-  B200_REQUIRE(cfg.KS >= 0 && cfg.stages >= 2 && cfg.stages <= (pair ? WP_MAX_STAGES : WT_MAX_STAGES) && cfg.split >= 1,
+  B200_REQUIRE(cfg.KS >= WT_KS_WIDE && cfg.stages >= 2 && cfg.stages <= (pair ? WP_MAX_STAGES : WT_MAX_STAGES) && cfg.split >= 1,
                "gemm_wt: bad config KS=%d stages=%d split=%d", cfg.KS, cfg.stages, cfg.split);
   B200_REQUIRE(mode >= B200_WT_BF16 && mode <= B200_WT_SWIGLU_SPLIT, "gemm_wt: mode %d", mode);
   const bool tower = mode == B200_WT_F32 || mode == B200_WT_SPLIT || mode == B200_WT_SWIGLU_SPLIT, swiglu = wt_swiglu(mode);
@@ -1103,6 +1189,7 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
                "gemm_wt: split output missing / misaligned");
   B200_REQUIRE(mode != B200_WT_PARTIAL || partial, "gemm_wt: partial buffer missing");
   B200_REQUIRE(mode == B200_WT_PARTIAL || cfg.split == 1, "gemm_wt: split-K needs the partial mode");
+  B200_REQUIRE(!wide || mode != B200_WT_PARTIAL, "gemm_wt: wide pairs write no partial tiles");
   B200_REQUIRE(!swiglu || (inter > 0 && inter % (tower ? 4 : 8) == 0 && N == 2 * inter),
                "gemm_wt: SwiGLU needs N == 2 * inter, inter a multiple of 8 (fp32: 4)");
   const int kb_total = cdiv(K, WT_BK);
@@ -1135,8 +1222,8 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
   B200_REQUIRE(!grouped || (mode == B200_WT_F32 && ext->n_groups > 0 && cfg.split == 1 && !bias),
                "gemm_wt: grouped products are fp32-output, unsplit, without bias");
   B200_REQUIRE(!pair || (!grouped && !heads), "gemm_wt: pairs take no groups");
-  const int stage = pair ? WT_WBLK + cfg.TN * 64 : cfg.KS * (WT_WBLK + cfg.TN * 128);
-  const size_t smem = (size_t)cfg.stages * stage + 1024 + (pair ? wp_staging(mode) : 0);
+  const int stage = pair ? (wide ? 2 : 1) * WT_WBLK + cfg.TN * 64 : cfg.KS * (WT_WBLK + cfg.TN * 128);
+  const size_t smem = (size_t)cfg.stages * stage + 1024 + (pair ? wp_staging(mode, wide) : 0);
   B200_REQUIRE(smem <= 227 * 1024 - 1024, "gemm_wt: %zu B of shared memory", smem);
   B200_REQUIRE(pair || (size_t)cfg.stages * stage >= (size_t)WT_EPI_TOK * WT_ROWS * 4, "gemm_wt: ring smaller than the epilogue staging tile");
   CUtensorMap tw, tx;
@@ -1156,8 +1243,8 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
     B200_CUDA(cudaFuncSetAttribute(gemm_wt_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024));
     B200_CUDA(cudaFuncSetAttribute(gemm_wt_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                    cudaSharedmemCarveoutMaxShared));
-    B200_CUDA(cudaFuncSetAttribute(gemm_wt_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024));
-    B200_CUDA(cudaFuncSetAttribute(gemm_wt_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024));
+    for (auto kern : {gemm_wt_pair_kernel<false, 1>, gemm_wt_pair_kernel<true, 1>, gemm_wt_pair_kernel<false, 2>, gemm_wt_pair_kernel<true, 2>})
+      B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024));
     set_mask |= 1ull << (dev & 63);
   }
   const int row_blocks = swiglu ? cdiv(inter, 64) : cdiv(N, WT_ROWS);
@@ -1172,9 +1259,9 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
   lc.attrs = at;
   lc.numAttrs = (g_wt_pdl && !grouped) ? 1 : 0;
   if (pair) {
-    const int tiles = cdiv(swiglu ? 2 * inter : N, 2 * WT_ROWS) * cdiv(T, cfg.TN) * splits;
+    const int tiles = cdiv(swiglu ? 2 * inter : N, (wide ? 4 : 2) * WT_ROWS) * cdiv(T, cfg.TN) * splits;
     lc.gridDim = dim3(2 * (tiles < WP_PAIRS ? tiles : WP_PAIRS));
-    lc.blockDim = dim3(WP_THREADS);
+    lc.blockDim = dim3(wide ? WP_WIDE_THREADS : WP_THREADS);
     cudaLaunchAttribute pa[2];
     pa[0].id = cudaLaunchAttributeClusterDimension;
     pa[0].val.clusterDim.x = 2;
@@ -1182,8 +1269,9 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
     pa[1] = at[0];
     lc.attrs = pa;
     lc.numAttrs = g_wt_pdl ? 2 : 1;
-    if (tower) B200_CUDA(cudaLaunchKernelEx(&lc, gemm_wt_pair_kernel<true>, tw, tx, p));
-    else B200_CUDA(cudaLaunchKernelEx(&lc, gemm_wt_pair_kernel<false>, tw, tx, p));
+    const auto kern = wide ? (tower ? gemm_wt_pair_kernel<true, 2> : gemm_wt_pair_kernel<false, 2>)
+                           : (tower ? gemm_wt_pair_kernel<true, 1> : gemm_wt_pair_kernel<false, 1>);
+    B200_CUDA(cudaLaunchKernelEx(&lc, kern, tw, tx, p));
     return B200_OK;
   }
   if (tower) {
@@ -1200,7 +1288,7 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
 // caller's stream with the call's own operands (CUDA events, one warm-up + two timed launches
 // each) and caches the winner; later calls cost one hash lookup.  Candidates follow what that
 // sweep showed matters: token tile {96,128,144,192,256}, one CTA per SM with 2 k-blocks
-// per stage vs two CTAs per SM with 1, and split-K to one or two waves.  The list is ordered and
+// per stage vs two CTAs per SM with 1, split-K to one or two waves, and CTA pairs.  The list is ordered and
 // the first candidate within 3 % of the best wins, so the choice is stable run to run.
 // B200_WT_TUNE=0 uses the cost model (gemm_wt_auto) instead.
 // ---------------------------------------------------------------------------------------------
@@ -1223,7 +1311,7 @@ struct TuneHash {
 // B200_WT_TUNE_FILE=<path>: measured choices are appended to the file and read back at the first call of a
 // later process, so a service does not re-measure at every start and a profiler run (whose serialised
 // replays distort the measurement) uses exactly the production configurations.  A line: token bucket, N, K, mode, split
-// allowed, TN, KS, stages, split, column groups (a line without the last is a plain product's).
+// allowed, TN, KS (0: CTA pairs, -1: wide ones), stages, split, column groups (a line without the last is a plain product's).
 static const char* tune_file() {
   static const char* f = getenv("B200_WT_TUNE_FILE");
   return (f && *f) ? f : nullptr;
@@ -1263,8 +1351,8 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
           while (fgets(line, sizeof line, fp)) {
             int tb, n, k, md, so, tn, ks, stg, sp, g = 0;
             if (sscanf(line, "%d %d %d %d %d %d %d %d %d %d", &tb, &n, &k, &md, &so, &tn, &ks, &stg, &sp, &g) < 9) continue;
-            if (tn >= 16 && tn <= 256 && tn % (ks ? 16 : 32) == 0 && ks >= (g > 0 ? 1 : 0) && stg >= 2 &&
-                stg <= (ks ? WT_MAX_STAGES : WP_MAX_STAGES) && sp >= 1)
+            if (tn >= 16 && tn <= 256 && tn % (ks > 0 ? 16 : 32) == 0 && ks >= (g > 0 ? 1 : WT_KS_WIDE) && stg >= 2 &&
+                stg <= (ks > 0 ? WT_MAX_STAGES : WP_MAX_STAGES) && sp >= 1)
               cache[TuneKey{tb, n, k, md, so, g, dev}] = WtConfig{tn, ks, stg, sp};
           }
           fclose(fp);
@@ -1333,16 +1421,16 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
     }
     // CTA pairs (KS = 0) from about a wave of them on: the token tile whose last wave is fullest, the next best, and 256
     if (T >= 192 && !(ext && (ext->tile_group || ext->col_groups > 0))) {
-      const int pair_rows = cdiv(wt_swiglu(mode) ? 2 * inter : N, 2 * WT_ROWS);
-      auto add_pair = [&](int tn, int split) {
-        const int stage = WT_WBLK + tn * 64;
-        int stg = (int)((226 * 1024 - 1024 - wp_staging(mode)) / stage);
+      const int w_rows = wt_swiglu(mode) ? 2 * inter : N, pair_rows = cdiv(w_rows, 2 * WT_ROWS), wide_rows = cdiv(w_rows, 4 * WT_ROWS);
+      auto add_pair = [&](int tn, int split, bool wide = false) {
+        const int stage = (wide ? 2 : 1) * WT_WBLK + tn * 64;
+        int stg = (int)((226 * 1024 - 1024 - wp_staging(mode, wide)) / stage);
         if (stg > WP_MAX_STAGES) stg = WP_MAX_STAGES;
         split = cdiv(kb_total, cdiv(kb_total, split < 1 ? 1 : split));
-        const WtConfig c{tn, 0, stg, split};
+        const WtConfig c{tn, wide ? WT_KS_WIDE : 0, stg, split};
         if (!fits(c)) return;
         for (const auto& o : cand)
-          if (o.TN == c.TN && o.KS == 0 && o.split == c.split) return;
+          if (o.TN == c.TN && o.KS == c.KS && o.split == c.split) return;
         cand.push_back(c);
       };
       int order[5] = {256, 224, 192, 160, 128};
@@ -1352,6 +1440,15 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
         const int base = pair_rows * cdiv(T, tn);
         add_pair(tn, 1);
         if (allow_split && base < WP_PAIRS) add_pair(tn, WP_PAIRS / base);
+      }
+      // 512 weight rows a pair: for long k (gemm_wt_pair_kernel), from half a wave of them on (fewer leave more than half of the
+      // chip idle, and halves of them are there among the candidates above)
+      if (mode != B200_WT_PARTIAL && K >= 3072) {
+        int worder[3] = {256, 224, 192};
+        auto wide_cost = [&](int tn) { return cdiv((long)wide_rows * cdiv(T, tn), WP_PAIRS) * (long)(256 + tn / 2); };
+        std::stable_sort(worder, worder + 3, [&](int a, int b) { return wide_cost(a) < wide_cost(b); });
+        for (int tn : {worder[0], worder[1]})
+          if (2 * wide_rows * cdiv(T, tn) >= WP_PAIRS) add_pair(tn, 1, true);
       }
     }
     if (cand.empty()) {
@@ -1429,9 +1526,10 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
     }
     // Back to back a pair does not show what it costs in a sequence: all of an SM's shared memory, so the next kernel's set-up
     // and weight loads wait for it, and code of its own to fetch.  It has to win by 8 % (a 2048 x 2048 x 2048 product measured 3 %
-    // faster alone and was 4 us of 26 slower between row kernels).
+    // faster alone and was 4 us of 26 slower between row kernels), or 4 us: the cost does not grow with the product (with 8 % of
+    // everything one-CTA tiles took 4096 x 4096 x 28672 in fp32 at 827 us, where wide pairs take 685).
     for (size_t i = 0; i < cand.size(); ++i)
-      if (cand[i].KS == 0) ms[i] *= 1.08f;
+      if (cand[i].KS <= 0) ms[i] += std::min(0.08f * ms[i], 0.004f);
     float best = 1e30f;
     for (float t : ms) best = t < best ? t : best;
     size_t pick = 0;
@@ -1508,6 +1606,7 @@ int b200_gemm_wt(const void* X, long ldx, const void* W, const void* bias, const
     c.TN = cfg4[0]; c.KS = cfg4[1]; c.stages = cfg4[2]; c.split = cfg4[3];
     B200_REQUIRE(c.KS >= 1, "gemm_wt: bad config KS=%d", c.KS);
     if (flags & B200_WT_FLAG_PAIR) c.KS = 0;
+    if (flags & B200_WT_FLAG_WIDE) c.KS = WT_KS_WIDE;
   } else {
     const int rbs = mode == B200_WT_SWIGLU ? cdiv(inter, 64) : cdiv(N, 128);
     gemm_wt_auto(T, rbs, K, mode == B200_WT_PARTIAL, &c, 148);

@@ -193,3 +193,61 @@ def test_a_wait_that_runs_out_is_told(T, n, K):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", _CHILD_WAIT.format(root=root, T=T, n=n, K=K)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+# ---- wide pairs: 512 weight rows (SwiGLU: 256 channels) a pair, the second half's products a few k-blocks behind the first's
+WIDE = 16         # B200_WT_FLAG_WIDE
+
+
+# one k-block and fewer of them than twice the lag | one row more or less than a half, a tile | more tiles than pairs, several
+# rounds of the ring
+@pytest.mark.parametrize("T,N,K,TN,stages", [(1, 8, 64, 64, 3), (129, 256, 128, 128, 4), (130, 257, 200, 256, 4), (256, 520, 320, 224, 3),
+                                             (300, 1030, 392, 192, 2), (2100, 10000, 576, 256, 4), (513, 131, 4096, 192, 4)])
+def test_wide_pairs_give_what_pairs_give(lib, T, N, K, TN, stages):
+    """the same sums in the same order: bit for bit the output of the pairs of 256 rows, which the tests above hold to float64"""
+    import ctypes
+    from mlx_vlm_b200 import _native as Nn
+    x, w, b, r = _rand(T, K, seed=11), _rand(N, K, seed=12, std=K ** -0.5), _rand(N, seed=13), _rand(T, N, seed=14)
+    ld = (N + 7) // 8 * 8
+    for epi, mode, inter, bias, res in ((0, 0, 0, b, r), (1, 0, 0, b, None), (2, 0, 0, None, None), (0, 2, N // 16 * 8, None, None)):
+        n = 2 * inter if mode == 2 else N
+        if n == 0:
+            continue
+        outs = []
+        for flag in (PAIR, WIDE):
+            out = torch.full((T, ld), 9.0, dtype=torch.bfloat16, device="cuda")
+            Nn.check(lib.b200_gemm_wt(x.data_ptr(), K, w.data_ptr(), Nn.ptr(bias), Nn.ptr(res), N if res is not None else 0, out.data_ptr(),
+                                      ld, 0, T, n, K, epi, mode, inter, (ctypes.c_int * 4)(TN, 1, stages, 1), flag, 0), "gemm_wt")
+            outs.append(out)
+        torch.cuda.synchronize()
+        assert torch.equal(*outs), (epi, mode)
+        assert bool((outs[1][:, inter or N:] == 9.0).all()) and not bool((outs[1][:, :inter or N] == 9.0).all())
+
+
+def test_wide_pairs_take_no_partials(lib):
+    import ctypes
+    x, w = _rand(64, 128, seed=15), _rand(64, 128, seed=16)
+    part = torch.empty(2, 64, 64, device="cuda")
+    assert lib.b200_gemm_wt(x.data_ptr(), 128, w.data_ptr(), 0, 0, 0, 0, 0, part.data_ptr(), 64, 64, 128, 0, 1, 0,
+                            (ctypes.c_int * 4)(64, 1, 4, 2), WIDE, 0) != 0
+
+
+def test_fp32_outputs_of_wide_pairs(tmp_path):
+    """as test_fp32_outputs_of_split_operands, with a file that gives wide pairs (k-blocks per stage -1)"""
+    cases = [(300, 264, 128, 3, 0), (577, 1152, 584, 3, 2), (640, 520, 72, 4, 2), (200, 1000, 1152, 4, 0)]
+    lines = [f"{(T + 63) // 64} {n} {2 * ((K + 63) // 64 * 64)} {mode} 0 {tn} -1 4 1" for (T, n, K, mode, _), tn in zip(cases, (160, 256, 224, 96))]
+    path = tmp_path / "choices.txt"
+    path.write_text("\n".join(lines) + "\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _CHILD.format(root=root, cases=cases)], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, B200_WT_TUNE_FILE=str(path)))
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert path.read_text() == "\n".join(lines) + "\n"
+
+
+@pytest.mark.parametrize("T,n,K", [(128, 512, 64), (1300, 8192, 640)])
+def test_a_wait_of_wide_pairs_that_runs_out_is_told(T, n, K):
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    child = _CHILD_WAIT.replace("cfg, 8 | flags", "cfg, 16 | flags")
+    r = subprocess.run([sys.executable, "-c", child.format(root=root, T=T, n=n, K=K)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
