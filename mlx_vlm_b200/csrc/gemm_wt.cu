@@ -19,9 +19,8 @@
 //   * split-K over gridDim.z for the GEMMs with few weight rows and long K (o_proj, down, fc2):
 //     fp32 partial tiles, summed in a FIXED order by the row-op kernel that follows
 //     (finish_rows: bias + residual + RMSNorm / LayerNorm of the next block, fused);
-//   * epilogue: TMEM -> registers (lane = weight row) -> transposed through shared memory ->
-//     coalesced 16-byte rows of C (bias / GELU / residual), or SwiGLU of interleaved gate/up
-//     row blocks (64 + 64 rows per tile, two TMA boxes), or fp32 partial tiles.
+//   * epilogue: TMEM -> registers (lane = weight row) -> rows of C (bias / GELU / residual) or fp32 partial tiles; SwiGLU of
+//     interleaved gate/up row blocks (64 + 64 rows per tile, two TMA boxes) through a staging tile.
 //
 // Replaces nn.Linear of the reference (models/qwen2_vl/vision.py:83-102,108-119,132-133,168-169;
 // language.py:52-55; mlp.py:9-15; activations.py:8-10).  Rounding points follow
@@ -162,149 +161,224 @@ __device__ __forceinline__ void w_pdl_launch() { asm volatile("griddepcontrol.la
 __device__ __forceinline__ void w_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void w_ebar(int id) { asm volatile("bar.sync %0, 256;" ::"r"(id) : "memory"); }
 
-// TMEM registers of one lane (weight row) -> bf16 staging tile [token][row]: + bias, one rounding, activation
-template <int EPI, int PER>
-__device__ __forceinline__ void wt_stage_bf16(const uint32_t (&a)[PER], float bias_v, bf16* sb) {
+// ---- the accumulator tile (128 weight rows x TN tokens, fp32 in TMEM) -> its outputs, by 256 threads (tid; warp tid / 32 reads
+// TMEM lane quarter (tid / 32) mod 4, which must be its own, and every other group of 32 tokens).  dead: a wait of this CTA ended
+// without its data, NaN is stored.
+struct WtTile {
+  uint32_t tmem;
+  int n0, t0;     // first output feature and token
+  long cg;        // first C32 column (column groups)
+  int split, tid;
+  bool dead;
+};
+
+// bias + activation of 32 tokens of one weight row, rounded to bf16 once before and once after the activation: pairs of tokens
+template <int EPI>
+__device__ __forceinline__ void wt_act_bf16(uint32_t (&a)[32], float bias_v, uint32_t (&v)[16]) {
   const uint64_t bias2 = f2(bias_v, bias_v);
-  unsigned short* s = reinterpret_cast<unsigned short*>(sb);
 #pragma unroll
-  for (int j = 0; j < PER; j += 2) {   // on pairs of tokens: this arithmetic is what bounds short products (gemm_wt_pair_kernel)
-    uint32_t v = pack_bf2(add2(f2(__uint_as_float(a[j]), __uint_as_float(a[j + 1])), bias2));
-    if constexpr (EPI == B200_EPI_GELU_FAST) v = gelu_fast_bf2(v);
+  for (int i = 0; i < 16; ++i) {   // (this arithmetic is what bounds short products of pairs: gemm_wt_pair_kernel)
+    v[i] = pack_bf2(add2(f2(__uint_as_float(a[2 * i]), __uint_as_float(a[2 * i + 1])), bias2));
+    if constexpr (EPI == B200_EPI_GELU_FAST) v[i] = gelu_fast_bf2(v[i]);
     if constexpr (EPI == B200_EPI_GELU_EXACT)
-      v = pack2(gelu_exact_bf(__uint_as_float(v << 16)), gelu_exact_bf(__uint_as_float(v & 0xffff0000u)));
-    s[j * WT_ROWS] = (unsigned short)v;
-    s[(j + 1) * WT_ROWS] = (unsigned short)(v >> 16);
+      v[i] = pack2(gelu_exact_bf(__uint_as_float(v[i] << 16)), gelu_exact_bf(__uint_as_float(v[i] & 0xffff0000u)));
   }
 }
-
 // the fp32-accurate paths: no rounding anywhere
-template <int EPI, int PER>
-__device__ __forceinline__ void wt_stage_f32(const uint32_t (&a)[PER], float bias_v, float* sf) {
-  if constexpr (EPI == B200_EPI_GELU_FAST) {
-    const uint64_t bias2 = f2(bias_v, bias_v), k = f2(1.702f, 1.702f);
+template <int EPI>
+__device__ __forceinline__ void wt_act_f32(uint32_t (&a)[32], float bias_v) {
+  const uint64_t bias2 = f2(bias_v, bias_v);
 #pragma unroll
-    for (int j = 0; j < PER; j += 2) {
-      uint64_t v = add2(f2(__uint_as_float(a[j]), __uint_as_float(a[j + 1])), bias2);
-      v = mul2(v, sigmoid2(mul2(v, k)));
-      sf[j * WT_ROWS] = f2_lo(v);
-      sf[(j + 1) * WT_ROWS] = f2_hi(v);
+  for (int i = 0; i < 32; i += 2) {
+    uint64_t v = add2(f2(__uint_as_float(a[i]), __uint_as_float(a[i + 1])), bias2);
+    if constexpr (EPI == B200_EPI_GELU_FAST) v = mul2(v, sigmoid2(mul2(v, f2(1.702f, 1.702f))));
+    float x[2] = {f2_lo(v), f2_hi(v)};
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      if constexpr (EPI == B200_EPI_GELU_EXACT) x[e] = x[e] * (1.0f + erff(x[e] / 1.41421356237309515f)) * 0.5f;
+      if constexpr (EPI == B200_EPI_GELU_TANH) {
+        const float u = 0.7978845608028654f * (x[e] + 0.044715f * x[e] * x[e] * x[e]);
+        x[e] = 0.5f * x[e] * (1.0f + tanhf(u));
+      }
+      a[i + e] = __float_as_uint(x[e]);
     }
-    return;
   }
+}
+// A lane holds two tokens (low, high half) of its row; the even lane of a pair gets both rows of the first token, the odd one
+// those of the second.
+__device__ __forceinline__ uint32_t wt_transpose2(uint32_t v, uint32_t sel) {
+  return __byte_perm(v, __shfl_xor_sync(0xffffffffu, v, 1), sel);
+}
+
+// All outputs but SwiGLU's go from the registers to memory as they are: a lane has a weight row, so a warp's store of a token is
+// 32 consecutive features: 128 bytes of fp32, and of bf16, two tokens at a time, 64 bytes of each.  Through a staging tile in
+// shared memory, as 16-byte rows, the warps waited for one another twice per 64 tokens, which every product pays at its end and
+// those of short k of pairs all along.  Staged -> direct, calls of several products and what lies between them: one picture
+// through four vision blocks 287 -> 269 us, 6012 patches through two 1001 -> 981, eight pictures through three CLIP blocks (fp32)
+// 1234 -> 1199, 2048 tokens through a latent attention block (fp32) 149 -> 140, 272 through four 2B layers 249 -> 243.
+template <bool TOWER>
+__device__ __forceinline__ void wt_store_rows(const WtParams& p, const WtTile& c) {
+  const int warp = c.tid >> 5, lane = c.tid & 31, q = warp & 3, half = warp >> 2;
+  if (c.n0 + q * 32 >= p.N || (p.flags & 1u)) return;
+  const int n = c.n0 + q * 32 + lane, odd = lane & 1;
+  const bool in = n < p.N;
+  const uint32_t sel = odd ? 0x3276u : 0x5410u;
+  const float bias_v = p.bias && in && p.mode != B200_WT_PARTIAL ? bf2f(p.bias[n]) : 0.f;
+  const int tokens = min(p.TN, p.T - c.t0);
+  const bool store = in && !(p.flags & 4u);
+  bool pairs = (p.N & 1) == 0;   // two features of a token as one word
+  if constexpr (!TOWER)
+    pairs = pairs && ((p.ldc | (p.residual ? p.ldr : 0)) & 1) == 0 &&
+            ((reinterpret_cast<uintptr_t>(p.C) | (p.residual ? reinterpret_cast<uintptr_t>(p.residual) : 0)) & 3) == 0;
+  for (int cc = half * 32; cc < tokens; cc += 64) {
+    uint32_t a[32];
+    w_tmem_ld32(c.tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cc, a);
+    if (c.dead)
 #pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    float v = __uint_as_float(a[j]) + bias_v;
-    if constexpr (EPI == B200_EPI_GELU_EXACT) v = v * (1.0f + erff(v / 1.41421356237309515f)) * 0.5f;
-    if constexpr (EPI == B200_EPI_GELU_TANH) {
-      const float u = 0.7978845608028654f * (v + 0.044715f * v * v * v);
-      v = 0.5f * v * (1.0f + tanhf(u));
+      for (int j = 0; j < 32; ++j) a[j] = 0x7FC00000u;
+    const int nv = store ? tokens - cc : 0;   // tokens that this lane stores
+    const long t = c.t0 + cc;
+    if (!TOWER && p.mode == B200_WT_PARTIAL) {   // fp32 partial tile -> P[split][t][n]
+      float* d = p.partial + ((long)c.split * p.T + t) * p.N + n;
+#pragma unroll
+      for (int j = 0; j < 32; ++j, d += p.N)
+        if (j < nv) *d = __uint_as_float(a[j]);
+    } else if constexpr (!TOWER) {
+      // one unrolled loop per epilogue kind, chosen OUTSIDE the loop: left to itself the compiler merged the
+      // three kinds into one predicated body of ~90 instructions per element (6-7 us per launch, A/B measured)
+      uint32_t v[16], r[16];
+      if (pairs) {
+        if (p.residual) {   // (in flight before the activation)
+          const bf16* s = p.residual + (t + odd) * p.ldr + (n & ~1);
+#pragma unroll
+          for (int i = 0; i < 16; ++i, s += 2 * p.ldr) r[i] = 2 * i + odd < nv ? *reinterpret_cast<const uint32_t*>(s) : 0u;
+        }
+        if (p.epilogue == B200_EPI_GELU_FAST) wt_act_bf16<B200_EPI_GELU_FAST>(a, bias_v, v);
+        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_act_bf16<B200_EPI_GELU_EXACT>(a, bias_v, v);
+        else wt_act_bf16<B200_EPI_NONE>(a, bias_v, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = wt_transpose2(v[i], sel);
+        if (p.residual)
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = pack_bf2(add2(unpack_bf2(r[i]), unpack_bf2(v[i])));
+        bf16* d = p.C + (t + odd) * p.ldc + (n & ~1);
+#pragma unroll
+        for (int i = 0; i < 16; ++i, d += 2 * p.ldc)
+          if (2 * i + odd < nv) *reinterpret_cast<uint32_t*>(d) = v[i];
+      } else {
+        if (p.epilogue == B200_EPI_GELU_FAST) wt_act_bf16<B200_EPI_GELU_FAST>(a, bias_v, v);
+        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_act_bf16<B200_EPI_GELU_EXACT>(a, bias_v, v);
+        else wt_act_bf16<B200_EPI_NONE>(a, bias_v, v);
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (j < nv) {
+            float x = __uint_as_float(j & 1 ? v[j >> 1] & 0xffff0000u : v[j >> 1] << 16);
+            if (p.residual) x = rbf(bf2f(p.residual[(t + j) * p.ldr + n]) + x);
+            p.C[(t + j) * p.ldc + n] = f2bf(x);
+          }
+      }
+    } else {
+      if (p.epilogue == B200_EPI_GELU_FAST) wt_act_f32<B200_EPI_GELU_FAST>(a, bias_v);
+      else if (p.epilogue == B200_EPI_GELU_EXACT) wt_act_f32<B200_EPI_GELU_EXACT>(a, bias_v);
+      else if (p.epilogue == B200_EPI_GELU_TANH) wt_act_f32<B200_EPI_GELU_TANH>(a, bias_v);
+      else wt_act_f32<B200_EPI_NONE>(a, bias_v);
+      if (p.mode == B200_WT_F32) {
+        float* d = p.C32 + t * p.ldc32 + c.cg + n;
+        if (p.res32) {
+          const float* s = p.res32 + t * p.ldr32 + n;
+#pragma unroll
+          for (int b = 0; b < 32; b += 8) {
+            float r[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j, s += p.ldr32) r[j] = b + j < nv ? *s : 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) a[b + j] = __float_as_uint(__uint_as_float(a[b + j]) + r[j]);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 32; ++j, d += p.ldc32)
+          if (j < nv) *d = __uint_as_float(a[j]);
+      } else {   // [hi | lo]: hi = bf16(v), lo = bf16(v - hi)
+        bf16* d = p.Csplit + (t + (pairs ? odd : 0)) * p.ld_split + (pairs ? n & ~1 : n);
+#pragma unroll
+        for (int i = 0; i < 16; ++i, d += 2 * p.ld_split) {
+          const float x0 = __uint_as_float(a[2 * i]), x1 = __uint_as_float(a[2 * i + 1]);
+          uint32_t hi = pack2(x0, x1);
+          uint32_t lo = pack2(x0 - __uint_as_float(hi << 16), x1 - __uint_as_float(hi & 0xffff0000u));
+          if (pairs) {
+            hi = wt_transpose2(hi, sel);
+            lo = wt_transpose2(lo, sel);
+            if (2 * i + odd < nv) {
+              *reinterpret_cast<uint32_t*>(d) = hi;
+              *reinterpret_cast<uint32_t*>(d + p.n_pad) = lo;
+            }
+          } else {
+            unsigned short* w = reinterpret_cast<unsigned short*>(d);
+            if (2 * i < nv) w[0] = (unsigned short)hi, w[p.n_pad] = (unsigned short)lo;
+            if (2 * i + 1 < nv) w[p.ld_split] = (unsigned short)(hi >> 16), w[p.ld_split + p.n_pad] = (unsigned short)(lo >> 16);
+          }
+        }
+      }
     }
-    sf[j * WT_ROWS] = v;
   }
 }
 
-// The accumulator tile (128 weight rows x TN tokens, fp32 in TMEM) -> its outputs, by 256 threads (tid; warp tid / 32 reads TMEM
-// lane quarter (tid / 32) mod 4, which must be its own) through a staging tile in shared memory.  dead: a wait of this CTA
-// ended without its data, NaN is stored.  TOK: tokens staged at a time; bar: the named barrier of these threads.
-template <bool TOWER, int TOK = WT_EPI_TOK>
-__device__ __forceinline__ void wt_store_tile(const WtParams& p, uint8_t* stg, uint32_t tmem, int n0, int t0, long cg, int split,
-                                              int tid, bool dead, int bar = 1) {
+// SwiGLU: a channel's gate and up rows (0..63 and 64..127 of the tile) are in different warps, so the tile goes through shared
+// memory, TOK tokens at a time; bar: the named barrier of these threads.
+template <bool TOWER, int TOK>
+__device__ __forceinline__ void wt_store_swiglu(const WtParams& p, const WtTile& c, uint8_t* stg, int bar) {
   constexpr int PER = TOK / 2;
-  const int warp = tid >> 5, lane = tid & 31, q = warp & 3, half = warp >> 2;
+  const int tid = c.tid, warp = tid >> 5, lane = tid & 31, q = warp & 3, half = warp >> 2;
   const int row = q * 32 + lane;  // weight row of the tile == TMEM lane
   float bias_v = 0.f;
-  if constexpr (TOWER) {
-    if (p.bias && p.mode == B200_WT_SWIGLU_SPLIT) {   // rows 0..63: gate channels, 64..127: up channels
-      if (n0 + (row & 63) < p.inter) bias_v = bf2f(p.bias[(row >> 6) * p.inter + n0 + (row & 63)]);
-    } else if (p.bias && n0 + row < p.N) {
-      bias_v = bf2f(p.bias[n0 + row]);
-    }
-  } else if (p.mode == B200_WT_BF16 && p.bias && n0 + row < p.N) {
-    bias_v = bf2f(p.bias[n0 + row]);
-  }
+  if (TOWER && p.bias && c.n0 + (row & 63) < p.inter) bias_v = bf2f(p.bias[(row >> 6) * p.inter + c.n0 + (row & 63)]);
   for (int c0 = 0; c0 < p.TN; c0 += TOK) {
     const int cc = c0 + half * PER;
     if (cc < p.TN && !(p.flags & 1u)) {
       uint32_t a[PER];
-      if constexpr (PER == 32) w_tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cc, a);
-      else w_tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cc, a);
-      if (dead)
+      if constexpr (PER == 32) w_tmem_ld32(c.tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cc, a);
+      else w_tmem_ld16(c.tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cc, a);
+      if (c.dead)
         for (int j = 0; j < PER; ++j) a[j] = 0x7FC00000u;
-      if (!TOWER && p.mode == B200_WT_PARTIAL) {
-        float* sf = reinterpret_cast<float*>(stg);
+      if constexpr (TOWER) {
+        float* s = reinterpret_cast<float*>(stg) + half * PER * WT_ROWS + row;
 #pragma unroll
-        for (int j = 0; j < PER; ++j) sf[(half * PER + j) * WT_ROWS + row] = __uint_as_float(a[j]);
-      } else if constexpr (TOWER) {
-        float* sf = reinterpret_cast<float*>(stg) + (half * PER) * WT_ROWS + row;
-        if (p.epilogue == B200_EPI_GELU_FAST) wt_stage_f32<B200_EPI_GELU_FAST, PER>(a, bias_v, sf);
-        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_stage_f32<B200_EPI_GELU_EXACT, PER>(a, bias_v, sf);
-        else if (p.epilogue == B200_EPI_GELU_TANH) wt_stage_f32<B200_EPI_GELU_TANH, PER>(a, bias_v, sf);
-        else wt_stage_f32<B200_EPI_NONE, PER>(a, bias_v, sf);
+        for (int j = 0; j < PER; ++j) s[j * WT_ROWS] = __uint_as_float(a[j]) + bias_v;
       } else {
-        // one unrolled loop per epilogue kind, chosen OUTSIDE the loop: left to itself the compiler merged the
-        // three kinds into one predicated body of ~90 instructions per element (6-7 us per launch, A/B measured)
-        bf16* sb = reinterpret_cast<bf16*>(stg) + (half * PER) * WT_ROWS + row;
-        if (p.epilogue == B200_EPI_GELU_FAST) wt_stage_bf16<B200_EPI_GELU_FAST, PER>(a, bias_v, sb);
-        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_stage_bf16<B200_EPI_GELU_EXACT, PER>(a, bias_v, sb);
-        else wt_stage_bf16<B200_EPI_NONE, PER>(a, bias_v, sb);
+        uint32_t v[16];
+        if (p.epilogue == B200_EPI_GELU_FAST) wt_act_bf16<B200_EPI_GELU_FAST>(a, 0.f, v);
+        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_act_bf16<B200_EPI_GELU_EXACT>(a, 0.f, v);
+        else wt_act_bf16<B200_EPI_NONE>(a, 0.f, v);
+        unsigned short* s = reinterpret_cast<unsigned short*>(stg) + half * PER * WT_ROWS + row;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          s[2 * i * WT_ROWS] = (unsigned short)v[i];
+          s[(2 * i + 1) * WT_ROWS] = (unsigned short)(v[i] >> 16);
+        }
       }
     }
     w_ebar(bar);
     if (!(p.flags & 4u)) {
-      if (!TOWER && p.mode == B200_WT_BF16) {
-        const bool vec_all = ((p.ldc & 7) == 0) && (!p.residual || (p.ldr & 7) == 0) &&
-                            ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0) &&
-                            (!p.residual || (reinterpret_cast<uintptr_t>(p.residual) & 15) == 0);
-#pragma unroll
-        for (int u = 0; u < TOK / 16; ++u) {
-          const int idx = tid + 256 * u;
-          const int tl = idx >> 4, ch = idx & 15;
-          const int t = t0 + c0 + tl, n = n0 + ch * 8;
-          if (c0 + tl >= p.TN || t >= p.T || n >= p.N) continue;
-          const uint4 sv = *reinterpret_cast<const uint4*>(stg + (tl * WT_ROWS + ch * 8) * 2);
-          const bool vec_ok = vec_all && n + 8 <= p.N;  // only the last chunk of an odd N goes element-wise
-          if (vec_ok) {
-            uint4 o = sv;
-            if (p.residual) {
-              float r[8], v[8];
-              unpack8(*reinterpret_cast<const uint4*>(p.residual + (long)t * p.ldr + n), r);
-              unpack8(sv, v);
-#pragma unroll
-              for (int e = 0; e < 8; ++e) v[e] = rbf(r[e] + v[e]);
-              o.x = pack2(v[0], v[1]); o.y = pack2(v[2], v[3]); o.z = pack2(v[4], v[5]); o.w = pack2(v[6], v[7]);
-            }
-            *reinterpret_cast<uint4*>(p.C + (long)t * p.ldc + n) = o;
-          } else {
-            float v[8];
-            unpack8(sv, v);
-            for (int e = 0; e < 8 && n + e < p.N; ++e) {
-              float o = v[e];
-              if (p.residual) o = rbf(bf2f(p.residual[(long)t * p.ldr + n + e]) + o);
-              p.C[(long)t * p.ldc + n + e] = f2bf(o);
-            }
-          }
-        }
-      } else if (!TOWER && p.mode == B200_WT_SWIGLU) {
+      if constexpr (!TOWER) {
 #pragma unroll
         for (int u = 0; u < TOK / 32; ++u) {
           const int idx = tid + 256 * u;
           const int tl = idx >> 3, ch = idx & 7;
-          const int t = t0 + c0 + tl, i = n0 + ch * 8;
+          const int t = c.t0 + c0 + tl, i = c.n0 + ch * 8;
           if (c0 + tl >= p.TN || t >= p.T || i >= p.inter) continue;
           const uint4 g = *reinterpret_cast<const uint4*>(stg + (tl * WT_ROWS + ch * 8) * 2);
           const uint4 x = *reinterpret_cast<const uint4*>(stg + (tl * WT_ROWS + 64 + ch * 8) * 2);
           *reinterpret_cast<uint4*>(p.C + (long)t * p.ldc + i) =
               make_uint4(swiglu_bf2(g.x, x.x), swiglu_bf2(g.y, x.y), swiglu_bf2(g.z, x.z), swiglu_bf2(g.w, x.w));
         }
-      } else if (TOWER && p.mode == B200_WT_SWIGLU_SPLIT) {
+      } else {
         // silu(gate) * up in fp32, as the next product's operand: the [T, 2 inter] fp32 rows between the two never reach memory.
         // 4096 tokens x 28672 rows x 1152 (two parts) with a kernel of its own behind it 399 + 115 us (and 60 to clear its rows), this 396.
 #pragma unroll
         for (int u = 0; u < TOK / 16; ++u) {
           const int idx = tid + 256 * u;
           const int tl = idx >> 4, ch = idx & 15;
-          const int t = t0 + c0 + tl, i = n0 + ch * 4;
+          const int t = c.t0 + c0 + tl, i = c.n0 + ch * 4;
           if (c0 + tl >= p.TN || t >= p.T || i >= p.inter) continue;
           const float4 g = *reinterpret_cast<const float4*>(stg + (tl * WT_ROWS + ch * 4) * 4);
           const float4 x = *reinterpret_cast<const float4*>(stg + (tl * WT_ROWS + 64 + ch * 4) * 4);
@@ -318,67 +392,15 @@ __device__ __forceinline__ void wt_store_tile(const WtParams& p, uint8_t* stg, u
           *reinterpret_cast<uint2*>(dh) = make_uint2(pack2(hi[0], hi[1]), pack2(hi[2], hi[3]));
           *reinterpret_cast<uint2*>(dh + p.n_pad) = make_uint2(pack2(v[0] - hi[0], v[1] - hi[1]), pack2(v[2] - hi[2], v[3] - hi[3]));
         }
-      } else if constexpr (TOWER) {
-#pragma unroll
-        for (int u = 0; u < TOK / 8; ++u) {
-          const int idx = tid + 256 * u;
-          const int tl = idx >> 5, ch = idx & 31;
-          const int t = t0 + c0 + tl, n = n0 + ch * 4;
-          if (c0 + tl >= p.TN || t >= p.T || n >= p.N) continue;
-          float4 v = *reinterpret_cast<const float4*>(stg + (tl * WT_ROWS + ch * 4) * 4);
-          if (p.mode == B200_WT_F32) {
-            float* dst = p.C32 + (long)t * p.ldc32 + cg + n;
-            if (n + 4 <= p.N && (p.ldc32 & 3) == 0 && (cg & 3) == 0) {
-              if (p.res32) {
-                const float4 r = *reinterpret_cast<const float4*>(p.res32 + (long)t * p.ldr32 + n);
-                v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w;
-              }
-              *reinterpret_cast<float4*>(dst) = v;
-            } else {
-              const float vv[4] = {v.x, v.y, v.z, v.w};
-              for (int e = 0; e < 4 && n + e < p.N; ++e)
-                dst[e] = vv[e] + (p.res32 ? p.res32[(long)t * p.ldr32 + n + e] : 0.f);
-            }
-          } else {  // [hi | lo]: hi = bf16(v), lo = bf16(v - hi)
-            const float vv[4] = {v.x, v.y, v.z, v.w};
-            float hi[4], lo[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              hi[e] = rbf(vv[e]);
-              lo[e] = vv[e] - hi[e];
-            }
-            bf16* dh = p.Csplit + (long)t * p.ld_split + n;
-            if (n + 4 <= p.N) {
-              *reinterpret_cast<uint2*>(dh) = make_uint2(pack2(hi[0], hi[1]), pack2(hi[2], hi[3]));
-              *reinterpret_cast<uint2*>(dh + p.n_pad) = make_uint2(pack2(lo[0], lo[1]), pack2(lo[2], lo[3]));
-            } else {
-              for (int e = 0; e < 4 && n + e < p.N; ++e) {
-                dh[e] = f2bf(hi[e]);
-                dh[p.n_pad + e] = f2bf(lo[e]);
-              }
-            }
-          }
-        }
-      } else {  // fp32 partial tile -> P[split][t][n]
-#pragma unroll
-        for (int u = 0; u < TOK / 8; ++u) {
-          const int idx = tid + 256 * u;
-          const int tl = idx >> 5, ch = idx & 31;
-          const int t = t0 + c0 + tl, n = n0 + ch * 4;
-          if (c0 + tl >= p.TN || t >= p.T || n >= p.N) continue;
-          const float4 v = *reinterpret_cast<const float4*>(stg + (tl * WT_ROWS + ch * 4) * 4);
-          float* dst = p.partial + ((long)split * p.T + t) * p.N + n;
-          if (n + 4 <= p.N && (p.N & 3) == 0) {
-            *reinterpret_cast<float4*>(dst) = v;
-          } else {
-            const float vv[4] = {v.x, v.y, v.z, v.w};
-            for (int e = 0; e < 4 && n + e < p.N; ++e) dst[e] = vv[e];
-          }
-        }
       }
     }
     w_ebar(bar);
   }
+}
+template <bool TOWER, int TOK = WT_EPI_TOK>
+__device__ __forceinline__ void wt_store_tile(const WtParams& p, const WtTile& c, uint8_t* stg, int bar = 1) {
+  if (p.mode == (TOWER ? B200_WT_SWIGLU_SPLIT : B200_WT_SWIGLU)) wt_store_swiglu<TOWER, TOK>(p, c, stg, bar);
+  else wt_store_rows<TOWER>(p, c);
 }
 
 // TOWER = false: the bf16 paths (B200_WT_BF16 / PARTIAL / SWIGLU); TOWER = true: the fp32-accurate paths
@@ -532,7 +554,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   w_mbar_wait(&tmem_full, 0);
   w_fence_after();
   // every TMA load has landed and every MMA has retired: the ring is free for the staging tile
-  wt_store_tile<TOWER>(p, ring, tmem_base, n0, t0, cg, split, threadIdx.x, false);
+  wt_store_tile<TOWER>(p, WtTile{tmem_base, n0, t0, cg, split, (int)threadIdx.x, false}, ring);
   w_fence_before();
   __syncthreads();
   if (warp == 2) {
@@ -818,8 +840,8 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       const int a = HALVES == 2 ? half : j & 1;   // accumulator
       ok = ok && __all_sync(0xffffffffu, mbar_wait(&bars.acc_full[a], (HALVES == 2 ? j : j >> 1) & 1, &failed));
       w_fence_after();
-      wt_store_tile<TOWER, HALVES == 2 && TOWER ? 32 : WT_EPI_TOK>(p, stg + half * WP_WIDE_STAGING, tmem + (uint32_t)a * 256u, n0 + half * 2 * unit, t0, 0,
-                                                                   split, (int)(threadIdx.x - 128) & 255, !ok, 1 + half);
+      wt_store_tile<TOWER, HALVES == 2 && TOWER ? 32 : WT_EPI_TOK>(
+          p, WtTile{tmem + (uint32_t)a * 256u, n0 + half * 2 * unit, t0, 0, split, (int)(threadIdx.x - 128) & 255, !ok}, stg + half * WP_WIDE_STAGING, 1 + half);
       w_fence_before();
       __syncwarp();
       if (lane == 0)
