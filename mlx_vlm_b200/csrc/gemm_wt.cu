@@ -19,8 +19,8 @@
 //   * split-K over gridDim.z for the GEMMs with few weight rows and long K (o_proj, down, fc2):
 //     fp32 partial tiles, summed in a FIXED order by the row-op kernel that follows
 //     (finish_rows: bias + residual + RMSNorm / LayerNorm of the next block, fused);
-//   * epilogue: TMEM -> registers (lane = weight row) -> rows of C (bias / GELU / residual) or fp32 partial tiles; SwiGLU of
-//     interleaved gate/up row blocks (64 + 64 rows per tile, two TMA boxes) through a staging tile.
+//   * epilogue: TMEM -> registers (lane = weight row) -> rows of C (bias / GELU / residual, or SwiGLU of gate and up rows that
+//     the TMA box interleaves: 64 channels per tile) or fp32 partial tiles; nothing goes through shared memory.
 //
 // Replaces nn.Linear of the reference (models/qwen2_vl/vision.py:83-102,108-119,132-133,168-169;
 // language.py:52-55; mlp.py:9-15; activations.py:8-10).  Rounding points follow
@@ -41,7 +41,6 @@ constexpr int WT_ROWS = 128;        // weight rows per CTA (UMMA M)
 constexpr int WT_BK = 64;           // one k-block: 64 bf16 = 128 B = one swizzle row
 constexpr int WT_WBLK = WT_ROWS * 128;  // bytes of one weight k-block tile
 constexpr int WT_MAX_STAGES = 16;
-constexpr int WT_EPI_TOK = 64;      // tokens staged per epilogue pass
 
 struct WtParams {
   const bf16* bias;
@@ -106,6 +105,14 @@ __device__ __forceinline__ void w_tma_2d(void* dst, const CUtensorMap* tmap, uin
       "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(w_smem_u32(bar))
       : "memory");
 }
+// SwiGLU's weights as [channel][gate, up][k]: 64 channels are 128 rows of the tile
+__device__ __forceinline__ void w_tma_3d(void* dst, const CUtensorMap* tmap, uint64_t* bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(w_smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(c2), "r"(w_smem_u32(bar))
+      : "memory");
+}
 __device__ __forceinline__ void w_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
@@ -147,19 +154,8 @@ __device__ __forceinline__ void w_tmem_ld32(uint32_t taddr, uint32_t* r) {
       : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void w_tmem_ld16(uint32_t taddr, uint32_t* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void w_pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void w_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void w_ebar(int id) { asm volatile("bar.sync %0, 256;" ::"r"(id) : "memory"); }
 
 // ---- the accumulator tile (128 weight rows x TN tokens, fp32 in TMEM) -> its outputs, by 256 threads (tid; warp tid / 32 reads
 // TMEM lane quarter (tid / 32) mod 4, which must be its own, and every other group of 32 tokens).  dead: a wait of this CTA ended
@@ -204,13 +200,13 @@ __device__ __forceinline__ void wt_act_f32(uint32_t (&a)[32], float bias_v) {
     }
   }
 }
-// A lane holds two tokens (low, high half) of its row; the even lane of a pair gets both rows of the first token, the odd one
-// those of the second.
-__device__ __forceinline__ uint32_t wt_transpose2(uint32_t v, uint32_t sel) {
-  return __byte_perm(v, __shfl_xor_sync(0xffffffffu, v, 1), sel);
+// Lanes of a pair (by apart) hold two tokens (low, high half) each of their row; the first gets both rows of the low token, the
+// second those of the high one.
+__device__ __forceinline__ uint32_t wt_swap(uint32_t v, int by, uint32_t sel) {
+  return __byte_perm(v, __shfl_xor_sync(0xffffffffu, v, by), sel);
 }
 
-// All outputs but SwiGLU's go from the registers to memory as they are: a lane has a weight row, so a warp's store of a token is
+// Outputs go from the registers to memory as they are: a lane has a weight row, so a warp's store of a token is
 // 32 consecutive features: 128 bytes of fp32, and of bf16, two tokens at a time, 64 bytes of each.  Through a staging tile in
 // shared memory, as 16-byte rows, the warps waited for one another twice per 64 tokens, which every product pays at its end and
 // those of short k of pairs all along.  Staged -> direct, calls of several products and what lies between them: one picture
@@ -257,7 +253,7 @@ __device__ __forceinline__ void wt_store_rows(const WtParams& p, const WtTile& c
         else if (p.epilogue == B200_EPI_GELU_EXACT) wt_act_bf16<B200_EPI_GELU_EXACT>(a, bias_v, v);
         else wt_act_bf16<B200_EPI_NONE>(a, bias_v, v);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = wt_transpose2(v[i], sel);
+        for (int i = 0; i < 16; ++i) v[i] = wt_swap(v[i], 1, sel);
         if (p.residual)
 #pragma unroll
           for (int i = 0; i < 16; ++i) v[i] = pack_bf2(add2(unpack_bf2(r[i]), unpack_bf2(v[i])));
@@ -306,8 +302,8 @@ __device__ __forceinline__ void wt_store_rows(const WtParams& p, const WtTile& c
           uint32_t hi = pack2(x0, x1);
           uint32_t lo = pack2(x0 - __uint_as_float(hi << 16), x1 - __uint_as_float(hi & 0xffff0000u));
           if (pairs) {
-            hi = wt_transpose2(hi, sel);
-            lo = wt_transpose2(lo, sel);
+            hi = wt_swap(hi, 1, sel);
+            lo = wt_swap(lo, 1, sel);
             if (2 * i + odd < nv) {
               *reinterpret_cast<uint32_t*>(d) = hi;
               *reinterpret_cast<uint32_t*>(d + p.n_pad) = lo;
@@ -323,83 +319,70 @@ __device__ __forceinline__ void wt_store_rows(const WtParams& p, const WtTile& c
   }
 }
 
-// SwiGLU: a channel's gate and up rows (0..63 and 64..127 of the tile) are in different warps, so the tile goes through shared
-// memory, TOK tokens at a time; bar: the named barrier of these threads.
-template <bool TOWER, int TOK>
-__device__ __forceinline__ void wt_store_swiglu(const WtParams& p, const WtTile& c, uint8_t* stg, int bar) {
-  constexpr int PER = TOK / 2;
-  const int tid = c.tid, warp = tid >> 5, lane = tid & 31, q = warp & 3, half = warp >> 2;
-  const int row = q * 32 + lane;  // weight row of the tile == TMEM lane
-  float bias_v = 0.f;
-  if (TOWER && p.bias && c.n0 + (row & 63) < p.inter) bias_v = bf2f(p.bias[(row >> 6) * p.inter + c.n0 + (row & 63)]);
-  for (int c0 = 0; c0 < p.TN; c0 += TOK) {
-    const int cc = c0 + half * PER;
-    if (cc < p.TN && !(p.flags & 1u)) {
-      uint32_t a[PER];
-      if constexpr (PER == 32) w_tmem_ld32(c.tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cc, a);
-      else w_tmem_ld16(c.tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cc, a);
-      if (c.dead)
-        for (int j = 0; j < PER; ++j) a[j] = 0x7FC00000u;
-      if constexpr (TOWER) {
-        float* s = reinterpret_cast<float*>(stg) + half * PER * WT_ROWS + row;
+// SwiGLU: the tile's rows are gate and up of its channels in turn (w_tma_3d), so neighbouring lanes hold a channel: one swap gives
+// each both of them for one token, another one, of two tokens between channels, two channels to a word.  Gate and up as blocks of
+// 64 rows each, which met in shared memory: eight prompts of 608 tokens through two Llama-7B layers 4120 us, so 4080; 272 tokens
+// through four 2B layers 243 and 241; five lock-step rows 172 and 160; four pictures through the SigLIP projection 2734 and 2702.
+template <bool TOWER>
+__device__ __forceinline__ void wt_store_swiglu(const WtParams& p, const WtTile& c) {
+  const int warp = c.tid >> 5, lane = c.tid & 31, q = warp & 3, half = warp >> 2;
+  if (c.n0 + q * 16 >= p.inter || (p.flags & 1u)) return;
+  const int i0 = c.n0 + q * 16 + (lane >> 1), odd = lane & 1, later = lane & 2;   // channel; which tokens it gets and stores
+  const bool in = i0 < p.inter;
+  const uint32_t sel = odd ? 0x3276u : 0x5410u, sel2 = later ? 0x3276u : 0x5410u;
+  const float bias_v = TOWER && p.bias && in ? bf2f(p.bias[odd * p.inter + i0]) : 0.f;
+  const int tokens = min(p.TN, p.T - c.t0);
+  const bool store = in && !(p.flags & 4u);
+  for (int cc = half * 32; cc < tokens; cc += 64) {
+    uint32_t a[32];
+    w_tmem_ld32(c.tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cc, a);
+    if (c.dead)
 #pragma unroll
-        for (int j = 0; j < PER; ++j) s[j * WT_ROWS] = __uint_as_float(a[j]) + bias_v;
-      } else {
-        uint32_t v[16];
-        if (p.epilogue == B200_EPI_GELU_FAST) wt_act_bf16<B200_EPI_GELU_FAST>(a, 0.f, v);
-        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_act_bf16<B200_EPI_GELU_EXACT>(a, 0.f, v);
-        else wt_act_bf16<B200_EPI_NONE>(a, 0.f, v);
-        unsigned short* s = reinterpret_cast<unsigned short*>(stg) + half * PER * WT_ROWS + row;
+      for (int j = 0; j < 32; ++j) a[j] = 0x7FC00000u;
+    const int first = odd + later, nv = store ? tokens - cc - first : 0;
+    const long t = c.t0 + cc + first;
+    if constexpr (!TOWER) {
+      uint32_t v[16];
+      if (p.epilogue == B200_EPI_GELU_FAST) wt_act_bf16<B200_EPI_GELU_FAST>(a, 0.f, v);
+      else if (p.epilogue == B200_EPI_GELU_EXACT) wt_act_bf16<B200_EPI_GELU_EXACT>(a, 0.f, v);
+      else wt_act_bf16<B200_EPI_NONE>(a, 0.f, v);
+      bf16* d = p.C + t * p.ldc + (i0 & ~1);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          s[2 * i * WT_ROWS] = (unsigned short)v[i];
-          s[(2 * i + 1) * WT_ROWS] = (unsigned short)(v[i] >> 16);
+      for (int i = 0; i < 16; i += 2, d += 4 * p.ldc) {   // tokens 2 i + odd and two on
+        const uint32_t x = wt_swap(v[i], 1, sel), y = wt_swap(v[i + 1], 1, sel);
+        const uint32_t r = wt_swap(swiglu_bf2(__byte_perm(x, y, 0x5410), __byte_perm(x, y, 0x7632)), 2, sel2);
+        if (2 * i < nv) *reinterpret_cast<uint32_t*>(d) = r;
+      }
+    } else {
+      // silu(gate) * up in fp32, as the next product's operand: the [T, 2 inter] fp32 rows between the two never reach memory.
+      // 4096 tokens x 28672 rows x 1152 (two parts) with a kernel of its own behind it 399 + 115 us (and 60 to clear its rows), this 396.
+      wt_act_f32<B200_EPI_NONE>(a, bias_v);
+      bf16* d = p.Csplit + t * p.ld_split + (i0 & ~1);
+#pragma unroll
+      for (int i = 0; i < 32; i += 4, d += 4 * p.ld_split) {
+        float g[2], u[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const uint32_t mine = odd ? a[i + 2 * e + 1] : a[i + 2 * e];
+          const uint32_t its = __shfl_xor_sync(0xffffffffu, odd ? a[i + 2 * e] : a[i + 2 * e + 1], 1);
+          g[e] = __uint_as_float(odd ? its : mine);
+          u[e] = __uint_as_float(odd ? mine : its);
+        }
+        const uint64_t g2 = f2(g[0], g[1]), v = mul2(mul2(g2, sigmoid2(g2)), f2(u[0], u[1]));
+        const uint32_t h = pack_bf2(v);
+        const uint32_t l = pack2(f2_lo(v) - __uint_as_float(h << 16), f2_hi(v) - __uint_as_float(h & 0xffff0000u));
+        const uint32_t hi = wt_swap(h, 2, sel2), lo = wt_swap(l, 2, sel2);
+        if (i < nv) {
+          *reinterpret_cast<uint32_t*>(d) = hi;
+          *reinterpret_cast<uint32_t*>(d + p.n_pad) = lo;
         }
       }
     }
-    w_ebar(bar);
-    if (!(p.flags & 4u)) {
-      if constexpr (!TOWER) {
-#pragma unroll
-        for (int u = 0; u < TOK / 32; ++u) {
-          const int idx = tid + 256 * u;
-          const int tl = idx >> 3, ch = idx & 7;
-          const int t = c.t0 + c0 + tl, i = c.n0 + ch * 8;
-          if (c0 + tl >= p.TN || t >= p.T || i >= p.inter) continue;
-          const uint4 g = *reinterpret_cast<const uint4*>(stg + (tl * WT_ROWS + ch * 8) * 2);
-          const uint4 x = *reinterpret_cast<const uint4*>(stg + (tl * WT_ROWS + 64 + ch * 8) * 2);
-          *reinterpret_cast<uint4*>(p.C + (long)t * p.ldc + i) =
-              make_uint4(swiglu_bf2(g.x, x.x), swiglu_bf2(g.y, x.y), swiglu_bf2(g.z, x.z), swiglu_bf2(g.w, x.w));
-        }
-      } else {
-        // silu(gate) * up in fp32, as the next product's operand: the [T, 2 inter] fp32 rows between the two never reach memory.
-        // 4096 tokens x 28672 rows x 1152 (two parts) with a kernel of its own behind it 399 + 115 us (and 60 to clear its rows), this 396.
-#pragma unroll
-        for (int u = 0; u < TOK / 16; ++u) {
-          const int idx = tid + 256 * u;
-          const int tl = idx >> 4, ch = idx & 15;
-          const int t = c.t0 + c0 + tl, i = c.n0 + ch * 4;
-          if (c0 + tl >= p.TN || t >= p.T || i >= p.inter) continue;
-          const float4 g = *reinterpret_cast<const float4*>(stg + (tl * WT_ROWS + ch * 4) * 4);
-          const float4 x = *reinterpret_cast<const float4*>(stg + (tl * WT_ROWS + 64 + ch * 4) * 4);
-          const uint64_t ga = f2(g.x, g.y), gb = f2(g.z, g.w);
-          const uint64_t va = mul2(mul2(ga, sigmoid2(ga)), f2(x.x, x.y)), vb = mul2(mul2(gb, sigmoid2(gb)), f2(x.z, x.w));
-          const float v[4] = {f2_lo(va), f2_hi(va), f2_lo(vb), f2_hi(vb)};
-          float hi[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) hi[e] = rbf(v[e]);
-          bf16* dh = p.Csplit + (long)t * p.ld_split + i;
-          *reinterpret_cast<uint2*>(dh) = make_uint2(pack2(hi[0], hi[1]), pack2(hi[2], hi[3]));
-          *reinterpret_cast<uint2*>(dh + p.n_pad) = make_uint2(pack2(v[0] - hi[0], v[1] - hi[1]), pack2(v[2] - hi[2], v[3] - hi[3]));
-        }
-      }
-    }
-    w_ebar(bar);
   }
 }
-template <bool TOWER, int TOK = WT_EPI_TOK>
-__device__ __forceinline__ void wt_store_tile(const WtParams& p, const WtTile& c, uint8_t* stg, int bar = 1) {
-  if (p.mode == (TOWER ? B200_WT_SWIGLU_SPLIT : B200_WT_SWIGLU)) wt_store_swiglu<TOWER, TOK>(p, c, stg, bar);
+template <bool TOWER>
+__device__ __forceinline__ void wt_store_tile(const WtParams& p, const WtTile& c) {
+  if (p.mode == (TOWER ? B200_WT_SWIGLU_SPLIT : B200_WT_SWIGLU)) wt_store_swiglu<TOWER>(p, c);
   else wt_store_rows<TOWER>(p, c);
 }
 
@@ -464,12 +447,8 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       int kbw = kb0 + it * p.KS + j;
       if (p.kb_w > 0) kbw %= p.kb_w;
       const int kc = kbw * WT_BK + wk0;
-      if (swiglu) {
-        w_tma_2d(sW + j * WT_WBLK, &tmW, &full_bar[s], kc, n0);
-        w_tma_2d(sW + j * WT_WBLK + 64 * 128, &tmW, &full_bar[s], kc, p.inter + n0);
-      } else {
-        w_tma_2d(sW + j * WT_WBLK, &tmW, &full_bar[s], kc, n0w);
-      }
+      if (swiglu) w_tma_3d(sW + j * WT_WBLK, &tmW, &full_bar[s], kc, 0, n0);
+      else w_tma_2d(sW + j * WT_WBLK, &tmW, &full_bar[s], kc, n0w);
     }
   };
   auto issue_x = [&](int it, int s) {
@@ -553,8 +532,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   // ===== epilogue (all 8 warps): warp w reads TMEM lane quarter w % 4, token half w / 4 =====
   w_mbar_wait(&tmem_full, 0);
   w_fence_after();
-  // every TMA load has landed and every MMA has retired: the ring is free for the staging tile
-  wt_store_tile<TOWER>(p, WtTile{tmem_base, n0, t0, cg, split, (int)threadIdx.x, false}, ring);
+  wt_store_tile<TOWER>(p, WtTile{tmem_base, n0, t0, cg, split, (int)threadIdx.x, false});
   w_fence_before();
   __syncthreads();
   if (warp == 2) {
@@ -595,7 +573,6 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
 // ---------------------------------------------------------------------------------------------
 constexpr int WP_THREADS = 384, WP_WIDE_THREADS = 640;
 constexpr int WP_LAG = 3;                                   // (at most the ring's stages, which are held meanwhile)
-constexpr int WP_WIDE_STAGING = WT_EPI_TOK * WT_ROWS * 2;   // bytes for each half's warps: 64 tokens in bf16, 32 in fp32
 constexpr int WP_MAX_STAGES = 12;
 
 struct WpBars {
@@ -614,6 +591,13 @@ __device__ __forceinline__ void wp_tma_2d(void* dst, const CUtensorMap* tmap, ui
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
       " [%0], [%1, {%2, %3}], [%4];" ::"r"(w_smem_u32(dst)),
       "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void wp_tma_3d(void* dst, const CUtensorMap* tmap, uint32_t bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
+      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(w_smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
       : "memory");
 }
 __device__ __forceinline__ void wp_umma(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
@@ -647,7 +631,6 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const bool swiglu = p.mode == (TOWER ? B200_WT_SWIGLU_SPLIT : B200_WT_SWIGLU);
   const int xhalf = p.TN / 2, stage_bytes = HALVES * WT_WBLK + xhalf * 128, NS = p.n_stages;
-  uint8_t* stg = ring + (long)NS * stage_bytes;
   const int kb_total = (p.K + WT_BK - 1) / WT_BK;
   const int unit = swiglu ? 64 : WT_ROWS;   // output features of 128 weight rows
   const int row_tiles = ((swiglu ? 2 * p.inter : p.N) + 2 * HALVES * WT_ROWS - 1) / (2 * HALVES * WT_ROWS), tok_tiles = (p.T + p.TN - 1) / p.TN;
@@ -705,8 +688,8 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
 #pragma unroll
         for (int h = 0; h < HALVES; ++h) {
           const int n = n0 + h * 2 * unit;
-          wp_tma_2d(sW + h * WT_WBLK, &tmW, bar, kb * WT_BK, n);
-          if (swiglu) wp_tma_2d(sW + h * WT_WBLK + 64 * 128, &tmW, bar, kb * WT_BK, p.inter + n);
+          if (swiglu) wp_tma_3d(sW + h * WT_WBLK, &tmW, bar, kb * WT_BK, 0, n);
+          else wp_tma_2d(sW + h * WT_WBLK, &tmW, bar, kb * WT_BK, n);
         }
       };
       auto load_x = [&](int s, int kb, int t0) {
@@ -840,8 +823,7 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       const int a = HALVES == 2 ? half : j & 1;   // accumulator
       ok = ok && __all_sync(0xffffffffu, mbar_wait(&bars.acc_full[a], (HALVES == 2 ? j : j >> 1) & 1, &failed));
       w_fence_after();
-      wt_store_tile<TOWER, HALVES == 2 && TOWER ? 32 : WT_EPI_TOK>(
-          p, WtTile{tmem + (uint32_t)a * 256u, n0 + half * 2 * unit, t0, 0, split, (int)(threadIdx.x - 128) & 255, !ok}, stg + half * WP_WIDE_STAGING, 1 + half);
+      wt_store_tile<TOWER>(p, WtTile{tmem + (uint32_t)a * 256u, n0 + half * 2 * unit, t0, 0, split, (int)(threadIdx.x - 128) & 255, !ok});
       w_fence_before();
       __syncwarp();
       if (lane == 0)
@@ -1029,8 +1011,9 @@ struct WtKey {
   const void* ptr;
   long ld;
   int rows, k, box_rows;
+  bool gate_up;
   bool operator==(const WtKey& o) const {
-    return ptr == o.ptr && ld == o.ld && rows == o.rows && k == o.k && box_rows == o.box_rows;
+    return ptr == o.ptr && ld == o.ld && rows == o.rows && k == o.k && box_rows == o.box_rows && gate_up == o.gate_up;
   }
 };
 struct WtHash {
@@ -1039,15 +1022,16 @@ struct WtHash {
     h = h * 1000003u ^ std::hash<long>()(k.ld);
     h = h * 1000003u ^ (size_t)k.rows;
     h = h * 1000003u ^ (size_t)k.k;
-    h = h * 1000003u ^ (size_t)k.box_rows;
+    h = h * 1000003u ^ (size_t)(2 * k.box_rows + k.gate_up);
     return h;
   }
 };
-// 2-D K-major bf16 operand (rows x K, row pitch ld elements), box = box_rows x 64
-int wt_tmap(const void* ptr, long ld, int rows, int k, int box_rows, CUtensorMap* out) {
+// 2-D K-major bf16 operand (rows x K, row pitch ld elements), box = box_rows x 64; gate_up: [gate rows; up rows], `rows` of each,
+// as a 3-D one (rows x 2 x K), so that a box has box_rows / 2 of both in turn
+int wt_tmap(const void* ptr, long ld, int rows, int k, int box_rows, CUtensorMap* out, bool gate_up = false) {
   static std::unordered_map<WtKey, CUtensorMap, WtHash> cache;
   static std::mutex mu;
-  WtKey key{ptr, ld, rows, k, box_rows};
+  WtKey key{ptr, ld, rows, k, box_rows, gate_up};
   {
     std::lock_guard<std::mutex> g(mu);
     auto it = cache.find(key);
@@ -1061,12 +1045,16 @@ int wt_tmap(const void* ptr, long ld, int rows, int k, int box_rows, CUtensorMap
     set_error("cuTensorMapEncodeTiled unavailable (no CUDA driver?)");
     return B200_ERR_CUDA;
   }
-  cuuint64_t gdim[2] = {(cuuint64_t)k, (cuuint64_t)rows};
-  cuuint64_t gstr[1] = {(cuuint64_t)ld * 2};
-  cuuint32_t box[2] = {(cuuint32_t)WT_BK, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
+  const int last = gate_up ? 2 : 1;   // the dimension of the rows
+  cuuint64_t gdim[3] = {(cuuint64_t)k, 2, 0};
+  cuuint64_t gstr[2] = {(cuuint64_t)rows * ld * 2, 0};
+  cuuint32_t box[3] = {(cuuint32_t)WT_BK, 2, 0};
+  cuuint32_t estr[3] = {1, 1, 1};
+  gdim[last] = (cuuint64_t)rows;
+  gstr[last - 1] = (cuuint64_t)ld * 2;
+  box[last] = (cuuint32_t)(gate_up ? box_rows / 2 : box_rows);
   CUtensorMap tm;
-  CUresult r = enc(&tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), gdim, gstr,
+  CUresult r = enc(&tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, last + 1, const_cast<void*>(ptr), gdim, gstr,
                    box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
@@ -1099,10 +1087,6 @@ static int round16(int x) { return (x + 15) & ~15; }
 constexpr int WP_PAIRS = 74;   // pairs of SMs
 constexpr int WT_KS_WIDE = -1; // WtConfig::KS of a pair with 512 weight rows (0: 256)
 static bool wt_swiglu(int mode) { return mode == B200_WT_SWIGLU || mode == B200_WT_SWIGLU_SPLIT; }
-static size_t wp_staging(int mode, bool wide) {   // the epilogue's staging tile: WT_EPI_TOK tokens x 128 rows
-  if (wide) return 2 * WP_WIDE_STAGING;
-  return (size_t)WT_EPI_TOK * WT_ROWS * (mode == B200_WT_BF16 || mode == B200_WT_SWIGLU ? 2 : 4);
-}
 
 // Tile / pipeline configuration for (T, row blocks, K): a small cost model calibrated on a
 // sweep (profiles/r2_gemm_wt_sweep.txt, B200):
@@ -1144,7 +1128,7 @@ void gemm_wt_auto(int T, int row_blocks, int K, bool allow_split, WtConfig* best
         const int budget = occ == 2 ? 110 * 1024 : 208 * 1024;
         int st = budget / stage;
         if (st > 8) st = 8;
-        if (st < 2 || st * KS < 3 || (long)st * stage < (long)WT_EPI_TOK * WT_ROWS * 4) continue;
+        if (st < 2 || st * KS < 3) continue;
         if (occ == 1 && (long)st * stage + 2048 <= 110 * 1024) continue;  // same as the occ == 2 case
         int cand[6] = {1, 0, 0, 0, 0, 0};
         int n_sp = 1;
@@ -1245,14 +1229,13 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
                "gemm_wt: grouped products are fp32-output, unsplit, without bias");
   B200_REQUIRE(!pair || (!grouped && !heads), "gemm_wt: pairs take no groups");
   const int stage = pair ? (wide ? 2 : 1) * WT_WBLK + cfg.TN * 64 : cfg.KS * (WT_WBLK + cfg.TN * 128);
-  const size_t smem = (size_t)cfg.stages * stage + 1024 + (pair ? wp_staging(mode, wide) : 0);
+  const size_t smem = (size_t)cfg.stages * stage + 1024;
   B200_REQUIRE(smem <= 227 * 1024 - 1024, "gemm_wt: %zu B of shared memory", smem);
-  B200_REQUIRE(pair || (size_t)cfg.stages * stage >= (size_t)WT_EPI_TOK * WT_ROWS * 4, "gemm_wt: ring smaller than the epilogue staging tile");
   CUtensorMap tw, tx;
   int rc = wt_tmap(W, (long)(ext && ext->ldw > 0 ? ext->ldw : k_w),
-                   grouped ? ext->n_groups * N : (heads && !w_cols ? ext->col_groups * N : N),
+                   grouped ? ext->n_groups * N : (heads && !w_cols ? ext->col_groups * N : (swiglu ? inter : N)),
                    w_cols ? (ext->col_groups - 1) * ext->w_group_cols + k_w : k_w,
-                   swiglu ? 64 : WT_ROWS, &tw);
+                   WT_ROWS, &tw, swiglu);
   if (rc) return rc;
   if ((rc = wt_tmap(X, ldx, T, heads ? ext->x_cols : K, pair ? cfg.TN / 2 : cfg.TN, &tx))) return rc;
   static unsigned long long set_mask = 0ull;
@@ -1405,7 +1388,7 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
       const int stage = ks * (WT_WBLK + tn * 128);
       int stg = budget / stage;
       if (stg > 6) stg = 6;
-      if (stg < 2 || (long)stg * stage < (long)WT_EPI_TOK * WT_ROWS * 4) return;
+      if (stg < 2) return;
       split = cdiv(kb_total, cdiv(kb_total, split < 1 ? 1 : split));
       WtConfig c{tn, ks, stg, split};
       if (!fits(c)) return;
@@ -1446,7 +1429,7 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
       const int w_rows = wt_swiglu(mode) ? 2 * inter : N, pair_rows = cdiv(w_rows, 2 * WT_ROWS), wide_rows = cdiv(w_rows, 4 * WT_ROWS);
       auto add_pair = [&](int tn, int split, bool wide = false) {
         const int stage = (wide ? 2 : 1) * WT_WBLK + tn * 64;
-        int stg = (int)((226 * 1024 - 1024 - wp_staging(mode, wide)) / stage);
+        int stg = (int)((226 * 1024 - 1024) / stage);
         if (stg > WP_MAX_STAGES) stg = WP_MAX_STAGES;
         split = cdiv(kb_total, cdiv(kb_total, split < 1 ? 1 : split));
         const WtConfig c{tn, wide ? WT_KS_WIDE : 0, stg, split};
