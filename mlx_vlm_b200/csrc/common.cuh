@@ -141,9 +141,10 @@ __device__ __forceinline__ float swiglu_bf(float g, float u) {
 __device__ __forceinline__ float gelu_fast_bf(float x) {
   return rbf(x * rbf(sigmoid_f(rbf(1.703125f * x))));
 }
-// nn.GELU(): x * (1 + erf(x / sqrt2)) / 2; sqrt2 weak-typed to bf16 = 1.4140625
+// nn.GELU(): x * (1 + erf(x / sqrt2)) / 2; sqrt2 weak-typed to bf16 = 1.4140625 (for every bf16 x the product with its reciprocal
+// rounds to the same bf16 as the quotient)
 __device__ __forceinline__ float gelu_exact_bf(float x) {
-  float a = rbf(x / 1.4140625f);
+  float a = rbf(x * (1.0f / 1.4140625f));
   float b = rbf(erff(a));
   float c = rbf(1.0f + b);
   float d = rbf(x * c);

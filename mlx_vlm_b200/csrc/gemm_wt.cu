@@ -27,6 +27,7 @@
 // oracle/mlx_semantics.py::linear (+ activations, residual add).
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 #include <vector>
 
@@ -141,64 +142,72 @@ __device__ __forceinline__ uint32_t w_desc_lo(uint32_t addr) {
 }
 constexpr uint32_t W_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 
-__device__ __forceinline__ void w_tmem_ld32(uint32_t taddr, uint32_t* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+// (its values may be used after w_ld_wait)
+__device__ __forceinline__ void w_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void w_ld_wait(uint32_t (&r)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])::"memory");
 }
 __device__ __forceinline__ void w_pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void w_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- the accumulator tile (128 weight rows x TN tokens, fp32 in TMEM) -> its outputs, by 256 threads (tid; warp tid / 32 reads
-// TMEM lane quarter (tid / 32) mod 4, which must be its own, and every other group of 32 tokens).  dead: a wait of this CTA ended
-// without its data, NaN is stored.
+// TMEM lane quarter (tid / 32) mod 4, which must be its own, and every other group of 8 tokens).
+// Outputs go from the registers to memory as they are: a lane has a weight row, so a warp's store of a token is 32 consecutive
+// features: 128 bytes of fp32, and of bf16, two tokens at a time, 64 bytes of each.  Through a staging tile in shared memory, as
+// 16-byte rows, the warps waited for one another twice per 64 tokens, which every product pays at its end and those of short k
+// of pairs all along.  Staged -> direct, calls of several products and what lies between them: one picture through four vision
+// blocks 287 -> 269 us, 6012 patches through two 1001 -> 981, eight pictures through three CLIP blocks (fp32) 1234 -> 1199, 2048
+// tokens through a latent attention block (fp32) 149 -> 140, 272 through four 2B layers 249 -> 243.
+// The loops are small on purpose: a launch fetches its code anew, and 32 tokens unrolled were 1 - 2 us of fetching at the end of
+// every product (stamps of one CTA, 576 x 5120 x 1280 with GELU: 2.1 us for the first 32 tokens, 1.0 for the next; the exact GELU
+// 15 and 4.2).
 struct WtTile {
   uint32_t tmem;
   int n0, t0;     // first output feature and token
   long cg;        // first C32 column (column groups)
   int split, tid;
-  bool dead;
+  float bias;     // of the thread's weight row: loaded before the products are waited for
+  bool dead;      // a wait of this CTA ended without its data: NaN is stored
 };
 
-// bias + activation of 32 tokens of one weight row, rounded to bf16 once before and once after the activation: pairs of tokens
+// the bias of a thread's weight row (SwiGLU: rows are gate and up of the channels in turn)
+template <bool TOWER>
+__device__ __forceinline__ float wt_bias(const WtParams& p, int n0, int tid) {
+  const int row = (tid >> 5 & 3) * 32 + (tid & 31);
+  if (TOWER && p.mode == B200_WT_SWIGLU_SPLIT) return p.bias && n0 + (row >> 1) < p.inter ? bf2f(p.bias[(row & 1) * p.inter + n0 + (row >> 1)]) : 0.f;
+  return p.bias && (TOWER || p.mode == B200_WT_BF16) && n0 + row < p.N ? bf2f(p.bias[n0 + row]) : 0.f;
+}
+
+// bias + activation of two tokens of one weight row, rounded to bf16 before and after the activation
 template <int EPI>
-__device__ __forceinline__ void wt_act_bf16(uint32_t (&a)[32], float bias_v, uint32_t (&v)[16]) {
-  const uint64_t bias2 = f2(bias_v, bias_v);
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {   // (this arithmetic is what bounds short products of pairs: gemm_wt_pair_kernel)
-    v[i] = pack_bf2(add2(f2(__uint_as_float(a[2 * i]), __uint_as_float(a[2 * i + 1])), bias2));
-    if constexpr (EPI == B200_EPI_GELU_FAST) v[i] = gelu_fast_bf2(v[i]);
-    if constexpr (EPI == B200_EPI_GELU_EXACT)
-      v[i] = pack2(gelu_exact_bf(__uint_as_float(v[i] << 16)), gelu_exact_bf(__uint_as_float(v[i] & 0xffff0000u)));
-  }
+__device__ __forceinline__ uint32_t wt_act_bf16(uint32_t a0, uint32_t a1, float bias) {
+  const uint32_t v = pack_bf2(add2(f2(__uint_as_float(a0), __uint_as_float(a1)), f2(bias, bias)));
+  if constexpr (EPI == B200_EPI_GELU_FAST) return gelu_fast_bf2(v);
+  if constexpr (EPI == B200_EPI_GELU_EXACT) return pack2(gelu_exact_bf(__uint_as_float(v << 16)), gelu_exact_bf(__uint_as_float(v & 0xffff0000u)));
+  return v;
 }
 // the fp32-accurate paths: no rounding anywhere
 template <int EPI>
-__device__ __forceinline__ void wt_act_f32(uint32_t (&a)[32], float bias_v) {
-  const uint64_t bias2 = f2(bias_v, bias_v);
+__device__ __forceinline__ void wt_act_f32(uint32_t& a0, uint32_t& a1, float bias) {
+  uint64_t v = add2(f2(__uint_as_float(a0), __uint_as_float(a1)), f2(bias, bias));
+  if constexpr (EPI == B200_EPI_GELU_FAST) v = mul2(v, sigmoid2(mul2(v, f2(1.702f, 1.702f))));
+  float x[2] = {f2_lo(v), f2_hi(v)};
 #pragma unroll
-  for (int i = 0; i < 32; i += 2) {
-    uint64_t v = add2(f2(__uint_as_float(a[i]), __uint_as_float(a[i + 1])), bias2);
-    if constexpr (EPI == B200_EPI_GELU_FAST) v = mul2(v, sigmoid2(mul2(v, f2(1.702f, 1.702f))));
-    float x[2] = {f2_lo(v), f2_hi(v)};
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      if constexpr (EPI == B200_EPI_GELU_EXACT) x[e] = x[e] * (1.0f + erff(x[e] / 1.41421356237309515f)) * 0.5f;
-      if constexpr (EPI == B200_EPI_GELU_TANH) {
-        const float u = 0.7978845608028654f * (x[e] + 0.044715f * x[e] * x[e] * x[e]);
-        x[e] = 0.5f * x[e] * (1.0f + tanhf(u));
-      }
-      a[i + e] = __float_as_uint(x[e]);
+  for (int e = 0; e < 2; ++e) {
+    if constexpr (EPI == B200_EPI_GELU_EXACT) x[e] = x[e] * (1.0f + erff(x[e] / 1.41421356237309515f)) * 0.5f;
+    if constexpr (EPI == B200_EPI_GELU_TANH) {
+      const float u = 0.7978845608028654f * (x[e] + 0.044715f * x[e] * x[e] * x[e]);
+      x[e] = 0.5f * x[e] * (1.0f + tanhf(u));
     }
   }
+  a0 = __float_as_uint(x[0]);
+  a1 = __float_as_uint(x[1]);
 }
 // Lanes of a pair (by apart) hold two tokens (low, high half) each of their row; the first gets both rows of the low token, the
 // second those of the high one.
@@ -206,165 +215,171 @@ __device__ __forceinline__ uint32_t wt_swap(uint32_t v, int by, uint32_t sel) {
   return __byte_perm(v, __shfl_xor_sync(0xffffffffu, v, by), sel);
 }
 
-// Outputs go from the registers to memory as they are: a lane has a weight row, so a warp's store of a token is
-// 32 consecutive features: 128 bytes of fp32, and of bf16, two tokens at a time, 64 bytes of each.  Through a staging tile in
-// shared memory, as 16-byte rows, the warps waited for one another twice per 64 tokens, which every product pays at its end and
-// those of short k of pairs all along.  Staged -> direct, calls of several products and what lies between them: one picture
-// through four vision blocks 287 -> 269 us, 6012 patches through two 1001 -> 981, eight pictures through three CLIP blocks (fp32)
-// 1234 -> 1199, 2048 tokens through a latent attention block (fp32) 149 -> 140, 272 through four 2B layers 249 -> 243.
-template <bool TOWER>
-__device__ __forceinline__ void wt_store_rows(const WtParams& p, const WtTile& c) {
-  const int warp = c.tid >> 5, lane = c.tid & 31, q = warp & 3, half = warp >> 2;
-  if (c.n0 + q * 32 >= p.N || (p.flags & 1u)) return;
-  const int n = c.n0 + q * 32 + lane, odd = lane & 1;
-  const bool in = n < p.N;
+// The warp's groups of 8 tokens in turn: body(first token, accumulators, residuals); the accumulators of the next group, and what
+// its residual(first token, words) asks for, are on their way meanwhile.
+template <class Residual, class Body>
+__device__ __forceinline__ void wt_groups(const WtTile& c, int tokens, Residual residual, Body body) {
+  const int warp = c.tid >> 5;
+  const uint32_t taddr = c.tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  uint32_t next[8], a[8], r_next[8], r[8];
+  int cc = (warp >> 2) * 8;
+  if (cc >= tokens) return;
+  w_ld8(taddr + (uint32_t)cc, next);
+  residual(cc, r_next);
+#pragma unroll 1
+  for (; cc < tokens; cc += 16) {
+    w_ld_wait(next);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] = c.dead ? 0x7FC00000u : next[j], r[j] = r_next[j];
+    if (cc + 16 < tokens) {
+      w_ld8(taddr + (uint32_t)cc + 16, next);
+      residual(cc + 16, r_next);
+    }
+    body(cc, a, r);
+  }
+}
+
+// bf16 rows
+template <int EPI>
+__device__ __forceinline__ void wt_store_bf16(const WtParams& p, const WtTile& c, int tokens) {
+  const int lane = c.tid & 31, n = c.n0 + (c.tid >> 5 & 3) * 32 + lane, odd = lane & 1;
   const uint32_t sel = odd ? 0x3276u : 0x5410u;
-  const float bias_v = p.bias && in && p.mode != B200_WT_PARTIAL ? bf2f(p.bias[n]) : 0.f;
-  const int tokens = min(p.TN, p.T - c.t0);
-  const bool store = in && !(p.flags & 4u);
-  bool pairs = (p.N & 1) == 0;   // two features of a token as one word
-  if constexpr (!TOWER)
-    pairs = pairs && ((p.ldc | (p.residual ? p.ldr : 0)) & 1) == 0 &&
-            ((reinterpret_cast<uintptr_t>(p.C) | (p.residual ? reinterpret_cast<uintptr_t>(p.residual) : 0)) & 3) == 0;
-  for (int cc = half * 32; cc < tokens; cc += 64) {
-    uint32_t a[32];
-    w_tmem_ld32(c.tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cc, a);
-    if (c.dead)
+  const bool store = n < p.N && !(p.flags & 4u);
+  const bool res = p.residual != nullptr;
+  auto none = [](int, uint32_t (&)[8]) {};
+  // two features of a token as one word
+  if ((p.N & 1) == 0 && ((p.ldc | (res ? p.ldr : 0)) & 1) == 0 &&
+      ((reinterpret_cast<uintptr_t>(p.C) | (res ? reinterpret_cast<uintptr_t>(p.residual) : 0)) & 3) == 0) {
+    bf16* const d0 = p.C + (long)(c.t0 + odd) * p.ldc + (n & ~1);
+    const bf16* const s0 = p.residual + (long)(c.t0 + odd) * p.ldr + (n & ~1);
+    auto body = [&](int cc, uint32_t (&a)[8], uint32_t (&r)[8], auto with_res) {
+      const int nv = store ? tokens - cc - odd : 0;
+      bf16* d = d0 + (long)cc * p.ldc;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) a[j] = 0x7FC00000u;
-    const int nv = store ? tokens - cc : 0;   // tokens that this lane stores
-    const long t = c.t0 + cc;
-    if (!TOWER && p.mode == B200_WT_PARTIAL) {   // fp32 partial tile -> P[split][t][n]
-      float* d = p.partial + ((long)c.split * p.T + t) * p.N + n;
-#pragma unroll
-      for (int j = 0; j < 32; ++j, d += p.N)
-        if (j < nv) *d = __uint_as_float(a[j]);
-    } else if constexpr (!TOWER) {
-      // one unrolled loop per epilogue kind, chosen OUTSIDE the loop: left to itself the compiler merged the
-      // three kinds into one predicated body of ~90 instructions per element (6-7 us per launch, A/B measured)
-      uint32_t v[16], r[16];
-      if (pairs) {
-        if (p.residual) {   // (in flight before the activation)
-          const bf16* s = p.residual + (t + odd) * p.ldr + (n & ~1);
-#pragma unroll
-          for (int i = 0; i < 16; ++i, s += 2 * p.ldr) r[i] = 2 * i + odd < nv ? *reinterpret_cast<const uint32_t*>(s) : 0u;
-        }
-        if (p.epilogue == B200_EPI_GELU_FAST) wt_act_bf16<B200_EPI_GELU_FAST>(a, bias_v, v);
-        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_act_bf16<B200_EPI_GELU_EXACT>(a, bias_v, v);
-        else wt_act_bf16<B200_EPI_NONE>(a, bias_v, v);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = wt_swap(v[i], 1, sel);
-        if (p.residual)
-#pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = pack_bf2(add2(unpack_bf2(r[i]), unpack_bf2(v[i])));
-        bf16* d = p.C + (t + odd) * p.ldc + (n & ~1);
-#pragma unroll
-        for (int i = 0; i < 16; ++i, d += 2 * p.ldc)
-          if (2 * i + odd < nv) *reinterpret_cast<uint32_t*>(d) = v[i];
-      } else {
-        if (p.epilogue == B200_EPI_GELU_FAST) wt_act_bf16<B200_EPI_GELU_FAST>(a, bias_v, v);
-        else if (p.epilogue == B200_EPI_GELU_EXACT) wt_act_bf16<B200_EPI_GELU_EXACT>(a, bias_v, v);
-        else wt_act_bf16<B200_EPI_NONE>(a, bias_v, v);
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (j < nv) {
-            float x = __uint_as_float(j & 1 ? v[j >> 1] & 0xffff0000u : v[j >> 1] << 16);
-            if (p.residual) x = rbf(bf2f(p.residual[(t + j) * p.ldr + n]) + x);
-            p.C[(t + j) * p.ldc + n] = f2bf(x);
-          }
+      for (int i = 0; i < 4; ++i, d += 2 * p.ldc) {
+        uint32_t v = wt_swap(wt_act_bf16<EPI>(a[2 * i], a[2 * i + 1], c.bias), 1, sel);
+        if constexpr (decltype(with_res)::value) v = pack_bf2(add2(unpack_bf2(r[i]), unpack_bf2(v)));
+        if (2 * i < nv) *reinterpret_cast<uint32_t*>(d) = v;
       }
+    };
+    if (res) {
+      wt_groups(c, tokens, [&](int cc, uint32_t (&r)[8]) {
+        const int nv = store ? tokens - cc - odd : 0;
+        const bf16* s = s0 + (long)cc * p.ldr;
+#pragma unroll
+        for (int i = 0; i < 4; ++i, s += 2 * p.ldr) r[i] = 2 * i < nv ? *reinterpret_cast<const uint32_t*>(s) : 0u;
+      }, [&](int cc, uint32_t (&a)[8], uint32_t (&r)[8]) { body(cc, a, r, std::true_type{}); });
     } else {
-      if (p.epilogue == B200_EPI_GELU_FAST) wt_act_f32<B200_EPI_GELU_FAST>(a, bias_v);
-      else if (p.epilogue == B200_EPI_GELU_EXACT) wt_act_f32<B200_EPI_GELU_EXACT>(a, bias_v);
-      else if (p.epilogue == B200_EPI_GELU_TANH) wt_act_f32<B200_EPI_GELU_TANH>(a, bias_v);
-      else wt_act_f32<B200_EPI_NONE>(a, bias_v);
-      if (p.mode == B200_WT_F32) {
-        float* d = p.C32 + t * p.ldc32 + c.cg + n;
-        if (p.res32) {
-          const float* s = p.res32 + t * p.ldr32 + n;
+      wt_groups(c, tokens, none, [&](int cc, uint32_t (&a)[8], uint32_t (&r)[8]) { body(cc, a, r, std::false_type{}); });
+    }
+    return;
+  }
+  wt_groups(c, tokens, none, [&](int cc, uint32_t (&a)[8], uint32_t (&)[8]) {
+    const int nv = store ? tokens - cc : 0;
 #pragma unroll
-          for (int b = 0; b < 32; b += 8) {
-            float r[8];
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t v = wt_act_bf16<EPI>(a[j], a[j], c.bias);
+      if (j >= nv) continue;
+      const long t = c.t0 + cc + j;
+      float x = __uint_as_float(v << 16);
+      if (res) x = rbf(bf2f(p.residual[t * p.ldr + n]) + x);
+      p.C[t * p.ldc + n] = f2bf(x);
+    }
+  });
+}
+
+// fp32 rows, or [hi | lo]: hi = bf16(v), lo = bf16(v - hi)
+template <int EPI>
+__device__ __forceinline__ void wt_store_f32(const WtParams& p, const WtTile& c, int tokens) {
+  const int lane = c.tid & 31, n = c.n0 + (c.tid >> 5 & 3) * 32 + lane, odd = lane & 1;
+  const bool store = n < p.N && !(p.flags & 4u);
+  auto none = [](int, uint32_t (&)[8]) {};
+  if (p.mode == B200_WT_F32) {
+    float* const d0 = p.C32 + (long)c.t0 * p.ldc32 + c.cg + n;
+    auto body = [&](int cc, uint32_t (&a)[8], uint32_t (&r)[8], auto with_res) {
+      const int nv = store ? tokens - cc : 0;
+      float* d = d0 + (long)cc * p.ldc32;
 #pragma unroll
-            for (int j = 0; j < 8; ++j, s += p.ldr32) r[j] = b + j < nv ? *s : 0.f;
+      for (int j = 0; j < 8; j += 2) wt_act_f32<EPI>(a[j], a[j + 1], c.bias);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) a[b + j] = __float_as_uint(__uint_as_float(a[b + j]) + r[j]);
-          }
+      for (int j = 0; j < 8; ++j, d += p.ldc32) {
+        float v = __uint_as_float(a[j]);
+        if constexpr (decltype(with_res)::value) v += __uint_as_float(r[j]);
+        if (j < nv) *d = v;
+      }
+    };
+    if (p.res32) {
+      const float* const s0 = p.res32 + (long)c.t0 * p.ldr32 + n;
+      wt_groups(c, tokens, [&](int cc, uint32_t (&r)[8]) {
+        const int nv = store ? tokens - cc : 0;
+        const float* s = s0 + (long)cc * p.ldr32;
+#pragma unroll
+        for (int j = 0; j < 8; ++j, s += p.ldr32) r[j] = j < nv ? __float_as_uint(*s) : 0u;
+      }, [&](int cc, uint32_t (&a)[8], uint32_t (&r)[8]) { body(cc, a, r, std::true_type{}); });
+    } else {
+      wt_groups(c, tokens, none, [&](int cc, uint32_t (&a)[8], uint32_t (&r)[8]) { body(cc, a, r, std::false_type{}); });
+    }
+    return;
+  }
+  const uint32_t sel = odd ? 0x3276u : 0x5410u;
+  const bool pairs = (p.N & 1) == 0;   // two features of a token as one word
+  bf16* const d0 = p.Csplit + (long)(c.t0 + (pairs ? odd : 0)) * p.ld_split + (pairs ? n & ~1 : n);
+  wt_groups(c, tokens, none, [&](int cc, uint32_t (&a)[8], uint32_t (&)[8]) {
+    const int nv = store ? tokens - cc - (pairs ? odd : 0) : 0;
+    bf16* d = d0 + (long)cc * p.ld_split;
+#pragma unroll
+    for (int i = 0; i < 4; ++i, d += 2 * p.ld_split) {
+      wt_act_f32<EPI>(a[2 * i], a[2 * i + 1], c.bias);
+      const float x0 = __uint_as_float(a[2 * i]), x1 = __uint_as_float(a[2 * i + 1]);
+      uint32_t hi = pack2(x0, x1);
+      uint32_t lo = pack2(x0 - __uint_as_float(hi << 16), x1 - __uint_as_float(hi & 0xffff0000u));
+      if (pairs) {
+        hi = wt_swap(hi, 1, sel);
+        lo = wt_swap(lo, 1, sel);
+        if (2 * i < nv) {
+          *reinterpret_cast<uint32_t*>(d) = hi;
+          *reinterpret_cast<uint32_t*>(d + p.n_pad) = lo;
         }
-#pragma unroll
-        for (int j = 0; j < 32; ++j, d += p.ldc32)
-          if (j < nv) *d = __uint_as_float(a[j]);
-      } else {   // [hi | lo]: hi = bf16(v), lo = bf16(v - hi)
-        bf16* d = p.Csplit + (t + (pairs ? odd : 0)) * p.ld_split + (pairs ? n & ~1 : n);
-#pragma unroll
-        for (int i = 0; i < 16; ++i, d += 2 * p.ld_split) {
-          const float x0 = __uint_as_float(a[2 * i]), x1 = __uint_as_float(a[2 * i + 1]);
-          uint32_t hi = pack2(x0, x1);
-          uint32_t lo = pack2(x0 - __uint_as_float(hi << 16), x1 - __uint_as_float(hi & 0xffff0000u));
-          if (pairs) {
-            hi = wt_swap(hi, 1, sel);
-            lo = wt_swap(lo, 1, sel);
-            if (2 * i + odd < nv) {
-              *reinterpret_cast<uint32_t*>(d) = hi;
-              *reinterpret_cast<uint32_t*>(d + p.n_pad) = lo;
-            }
-          } else {
-            unsigned short* w = reinterpret_cast<unsigned short*>(d);
-            if (2 * i < nv) w[0] = (unsigned short)hi, w[p.n_pad] = (unsigned short)lo;
-            if (2 * i + 1 < nv) w[p.ld_split] = (unsigned short)(hi >> 16), w[p.ld_split + p.n_pad] = (unsigned short)(lo >> 16);
-          }
-        }
+      } else {
+        unsigned short* w = reinterpret_cast<unsigned short*>(d);
+        if (2 * i < nv) w[0] = (unsigned short)hi, w[p.n_pad] = (unsigned short)lo;
+        if (2 * i + 1 < nv) w[p.ld_split] = (unsigned short)(hi >> 16), w[p.ld_split + p.n_pad] = (unsigned short)(lo >> 16);
       }
     }
-  }
+  });
 }
 
 // SwiGLU: the tile's rows are gate and up of its channels in turn (w_tma_3d), so neighbouring lanes hold a channel: one swap gives
 // each both of them for one token, another one, of two tokens between channels, two channels to a word.  Gate and up as blocks of
 // 64 rows each, which met in shared memory: eight prompts of 608 tokens through two Llama-7B layers 4120 us, so 4080; 272 tokens
 // through four 2B layers 243 and 241; five lock-step rows 172 and 160; four pictures through the SigLIP projection 2734 and 2702.
-template <bool TOWER>
-__device__ __forceinline__ void wt_store_swiglu(const WtParams& p, const WtTile& c) {
-  const int warp = c.tid >> 5, lane = c.tid & 31, q = warp & 3, half = warp >> 2;
-  if (c.n0 + q * 16 >= p.inter || (p.flags & 1u)) return;
-  const int i0 = c.n0 + q * 16 + (lane >> 1), odd = lane & 1, later = lane & 2;   // channel; which tokens it gets and stores
-  const bool in = i0 < p.inter;
+template <bool TOWER, int EPI>
+__device__ __forceinline__ void wt_store_swiglu(const WtParams& p, const WtTile& c, int tokens) {
+  const int lane = c.tid & 31, i0 = c.n0 + (c.tid >> 5 & 3) * 16 + (lane >> 1);   // channel
+  const int odd = lane & 1, later = lane & 2;                                      // which tokens it gets and stores
   const uint32_t sel = odd ? 0x3276u : 0x5410u, sel2 = later ? 0x3276u : 0x5410u;
-  const float bias_v = TOWER && p.bias && in ? bf2f(p.bias[odd * p.inter + i0]) : 0.f;
-  const int tokens = min(p.TN, p.T - c.t0);
-  const bool store = in && !(p.flags & 4u);
-  for (int cc = half * 32; cc < tokens; cc += 64) {
-    uint32_t a[32];
-    w_tmem_ld32(c.tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cc, a);
-    if (c.dead)
+  const bool store = i0 < p.inter && !(p.flags & 4u);
+  auto none = [](int, uint32_t (&)[8]) {};
+  const long ld = TOWER ? p.ld_split : p.ldc;
+  bf16* const d0 = (TOWER ? p.Csplit : p.C) + (long)(c.t0 + odd + later) * ld + (i0 & ~1);
+  wt_groups(c, tokens, none, [&](int cc, uint32_t (&a)[8], uint32_t (&)[8]) {
+    const int nv = store ? tokens - cc - odd - later : 0;
+    bf16* d = d0 + cc * ld;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) a[j] = 0x7FC00000u;
-    const int first = odd + later, nv = store ? tokens - cc - first : 0;
-    const long t = c.t0 + cc + first;
-    if constexpr (!TOWER) {
-      uint32_t v[16];
-      if (p.epilogue == B200_EPI_GELU_FAST) wt_act_bf16<B200_EPI_GELU_FAST>(a, 0.f, v);
-      else if (p.epilogue == B200_EPI_GELU_EXACT) wt_act_bf16<B200_EPI_GELU_EXACT>(a, 0.f, v);
-      else wt_act_bf16<B200_EPI_NONE>(a, 0.f, v);
-      bf16* d = p.C + t * p.ldc + (i0 & ~1);
-#pragma unroll
-      for (int i = 0; i < 16; i += 2, d += 4 * p.ldc) {   // tokens 2 i + odd and two on
-        const uint32_t x = wt_swap(v[i], 1, sel), y = wt_swap(v[i + 1], 1, sel);
+    for (int i = 0; i < 8; i += 4, d += 4 * ld) {   // tokens i + odd and two on
+      if constexpr (!TOWER) {
+        const uint32_t x = wt_swap(wt_act_bf16<EPI>(a[i], a[i + 1], 0.f), 1, sel), y = wt_swap(wt_act_bf16<EPI>(a[i + 2], a[i + 3], 0.f), 1, sel);
         const uint32_t r = wt_swap(swiglu_bf2(__byte_perm(x, y, 0x5410), __byte_perm(x, y, 0x7632)), 2, sel2);
-        if (2 * i < nv) *reinterpret_cast<uint32_t*>(d) = r;
-      }
-    } else {
-      // silu(gate) * up in fp32, as the next product's operand: the [T, 2 inter] fp32 rows between the two never reach memory.
-      // 4096 tokens x 28672 rows x 1152 (two parts) with a kernel of its own behind it 399 + 115 us (and 60 to clear its rows), this 396.
-      wt_act_f32<B200_EPI_NONE>(a, bias_v);
-      bf16* d = p.Csplit + t * p.ld_split + (i0 & ~1);
-#pragma unroll
-      for (int i = 0; i < 32; i += 4, d += 4 * p.ld_split) {
+        if (i < nv) *reinterpret_cast<uint32_t*>(d) = r;
+      } else {
+        // silu(gate) * up in fp32, as the next product's operand: the [T, 2 inter] fp32 rows between the two never reach memory.
+        // 4096 tokens x 28672 rows x 1152 (two parts) with a kernel of its own behind it 399 + 115 us (and 60 to clear its rows), this 396.
         float g[2], u[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const uint32_t mine = odd ? a[i + 2 * e + 1] : a[i + 2 * e];
-          const uint32_t its = __shfl_xor_sync(0xffffffffu, odd ? a[i + 2 * e] : a[i + 2 * e + 1], 1);
+          uint32_t &a0 = a[i + 2 * e], &a1 = a[i + 2 * e + 1];
+          wt_act_f32<EPI>(a0, a1, c.bias);
+          const uint32_t mine = odd ? a1 : a0, its = __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 1);
           g[e] = __uint_as_float(odd ? its : mine);
           u[e] = __uint_as_float(odd ? mine : its);
         }
@@ -378,12 +393,48 @@ __device__ __forceinline__ void wt_store_swiglu(const WtParams& p, const WtTile&
         }
       }
     }
-  }
+  });
 }
+
 template <bool TOWER>
 __device__ __forceinline__ void wt_store_tile(const WtParams& p, const WtTile& c) {
-  if (p.mode == (TOWER ? B200_WT_SWIGLU_SPLIT : B200_WT_SWIGLU)) wt_store_swiglu<TOWER>(p, c);
-  else wt_store_rows<TOWER>(p, c);
+  if (p.flags & 1u) return;
+  const int tokens = min(p.TN, p.T - c.t0), q = c.tid >> 5 & 3;
+  // one loop per epilogue kind, chosen OUTSIDE the loop: left to itself the compiler merged the
+  // three kinds into one predicated body of ~90 instructions per element (6-7 us per launch, A/B measured)
+  if (p.mode == (TOWER ? B200_WT_SWIGLU_SPLIT : B200_WT_SWIGLU)) {
+    if (c.n0 + q * 16 >= p.inter) return;
+    if constexpr (TOWER) {
+      wt_store_swiglu<true, B200_EPI_NONE>(p, c, tokens);
+    } else {
+      if (p.epilogue == B200_EPI_GELU_FAST) wt_store_swiglu<false, B200_EPI_GELU_FAST>(p, c, tokens);
+      else if (p.epilogue == B200_EPI_GELU_EXACT) wt_store_swiglu<false, B200_EPI_GELU_EXACT>(p, c, tokens);
+      else wt_store_swiglu<false, B200_EPI_NONE>(p, c, tokens);
+    }
+    return;
+  }
+  if (c.n0 + q * 32 >= p.N) return;
+  if constexpr (TOWER) {
+    if (p.epilogue == B200_EPI_GELU_FAST) wt_store_f32<B200_EPI_GELU_FAST>(p, c, tokens);
+    else if (p.epilogue == B200_EPI_GELU_EXACT) wt_store_f32<B200_EPI_GELU_EXACT>(p, c, tokens);
+    else if (p.epilogue == B200_EPI_GELU_TANH) wt_store_f32<B200_EPI_GELU_TANH>(p, c, tokens);
+    else wt_store_f32<B200_EPI_NONE>(p, c, tokens);
+  } else if (p.mode == B200_WT_PARTIAL) {   // fp32 partial tile -> P[split][t][n]
+    const int n = c.n0 + q * 32 + (c.tid & 31);
+    const bool store = n < p.N && !(p.flags & 4u);
+    float* const d0 = p.partial + ((long)c.split * p.T + c.t0) * p.N + n;
+    wt_groups(c, tokens, [](int, uint32_t (&)[8]) {}, [&](int cc, uint32_t (&a)[8], uint32_t (&)[8]) {
+      const int nv = store ? tokens - cc : 0;
+      float* d = d0 + (long)cc * p.N;
+#pragma unroll
+      for (int j = 0; j < 8; ++j, d += p.N)
+        if (j < nv) *d = __uint_as_float(a[j]);
+    });
+  } else {
+    if (p.epilogue == B200_EPI_GELU_FAST) wt_store_bf16<B200_EPI_GELU_FAST>(p, c, tokens);
+    else if (p.epilogue == B200_EPI_GELU_EXACT) wt_store_bf16<B200_EPI_GELU_EXACT>(p, c, tokens);
+    else wt_store_bf16<B200_EPI_NONE>(p, c, tokens);
+  }
 }
 
 // TOWER = false: the bf16 paths (B200_WT_BF16 / PARTIAL / SWIGLU); TOWER = true: the fp32-accurate paths
@@ -430,9 +481,9 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   while ((int)tmem_cols < p.TN) tmem_cols <<= 1;
 
   // The next kernel may start its prologue / weight prefetch as SM resources free up.  It may do so before this block has its columns:
-  // up to 256 of them, and what fits beside a block of 256 threads x 128 registers is one more like it; the kernels that ask for all
-  // 512 take more than the other half of the registers.  (Signalled behind the allocation: eight lock-step rows 383 -> 386 us, the
-  // latent prompt 152 -> 156, one picture 289 -> 286.)
+  // up to 256 of them, and what asks for some and fits beside a block of 256 threads x 96 registers is one more like it; the kernels
+  // that ask for all 512 take more registers and shared memory than it leaves.  (Signalled behind the allocation: eight lock-step
+  // rows 383 -> 386 us, the latent prompt 152 -> 156, one picture 289 -> 286.)
   w_pdl_launch();
 
   auto issue_w = [&](int it, int s) {
@@ -484,6 +535,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   __syncthreads();
   w_fence_after();
   const uint32_t tmem_base = tmem_slot;
+  const float bias = wt_bias<TOWER>(p, n0, threadIdx.x);
   w_pdl_wait();  // everything the previous kernels wrote (X, residual) is visible from here on
 
   if (warp == 0) {
@@ -532,7 +584,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   // ===== epilogue (all 8 warps): warp w reads TMEM lane quarter w % 4, token half w / 4 =====
   w_mbar_wait(&tmem_full, 0);
   w_fence_after();
-  wt_store_tile<TOWER>(p, WtTile{tmem_base, n0, t0, cg, split, (int)threadIdx.x, false});
+  wt_store_tile<TOWER>(p, WtTile{tmem_base, n0, t0, cg, split, (int)threadIdx.x, bias, false});
   w_fence_before();
   __syncthreads();
   if (warp == 2) {
@@ -821,9 +873,11 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     for (int tile = pair; tile < n_tiles; tile += n_pairs, ++j) {
       tile_at(tile, n0, t0, split, kb0, kb1);
       const int a = HALVES == 2 ? half : j & 1;   // accumulator
+      const int row0 = n0 + half * 2 * unit, tid = (int)(threadIdx.x - 128) & 255;
+      const float bias = wt_bias<TOWER>(p, row0, tid);
       ok = ok && __all_sync(0xffffffffu, mbar_wait(&bars.acc_full[a], (HALVES == 2 ? j : j >> 1) & 1, &failed));
       w_fence_after();
-      wt_store_tile<TOWER>(p, WtTile{tmem + (uint32_t)a * 256u, n0 + half * 2 * unit, t0, 0, split, (int)(threadIdx.x - 128) & 255, !ok});
+      wt_store_tile<TOWER>(p, WtTile{tmem + (uint32_t)a * 256u, row0, t0, 0, split, tid, bias, !ok});
       w_fence_before();
       __syncwarp();
       if (lane == 0)
