@@ -480,12 +480,6 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   uint32_t tmem_cols = 32;
   while ((int)tmem_cols < p.TN) tmem_cols <<= 1;
 
-  // The next kernel may start its prologue / weight prefetch as SM resources free up.  It may do so before this block has its columns:
-  // up to 256 of them, and what asks for some and fits beside a block of 256 threads x 96 registers is one more like it; the kernels
-  // that ask for all 512 take more registers and shared memory than it leaves.  (Signalled behind the allocation: eight lock-step
-  // rows 383 -> 386 us, the latent prompt 152 -> 156, one picture 289 -> 286.)
-  w_pdl_launch();
-
   auto issue_w = [&](int it, int s) {
     uint8_t* sW = ring + (long)s * stage_bytes;
     const int cnt = min(p.KS, kb1 - kb0 - it * p.KS);
@@ -577,6 +571,11 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
         if (++s == NS) s = 0, parity ^= 1;
       }
       w_commit(&tmem_full);
+      // The next kernel may start its set-up and weight loads as SM resources free up: not before this tile's products are issued,
+      // for its blocks hold shared memory and registers while they wait, which other streams' kernels could use.  Signalled when
+      // the block starts instead: 272 tokens through four 2B layers, three such sequences in flight, 241 us a call, so 231;
+      // one at a time 439, 432; eight lock-step rows 377 and 375, one picture 259 and 261.
+      w_pdl_launch();
     }
   }
   __syncwarp();
