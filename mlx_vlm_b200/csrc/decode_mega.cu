@@ -11,6 +11,10 @@
 //   * warps 0..7 are CONSUMERS that execute the phases in order, separated by a
 //     software grid barrier (one atomic + acquire spin, ~1 us) instead of a kernel
 //     boundary; activations cross CTAs through L2 (ld.global.cg).
+// A layer runs through some 90 KB of code once, in the 33 us that it takes, and what of it is not in the instruction cache any more
+// is a wait in the middle of a phase.  So the loops here are rolled, and a phase calls its epilogue in one place (it is inlined): the
+// kernel for 1,536 wide models 233 -> 189 KB, its step at a context of 700 1079 -> 1005 us, four layers of 4,096 behind 6000 keys 514
+// -> 472, with the products of mega_common.cuh (fma_bf2) and batched warp sums; with the tile loop unrolled eight times 1284.
 // Rounding points follow oracle/qwen2vl.py::lm_layers_forward (same device
 // functions as the multi-kernel path in decode.cu).
 #include <climits>
@@ -25,8 +29,8 @@ __device__ __forceinline__ const bf16* mega_tile_src(const MegaPhase& g, const b
                                                      const bf16* W2, int hd, int t, int m) {
   if (MODE == PH_QKV) {
     const int half = hd >> 1;
-    const int per_slot = half / g.R;
-    const int slot = t / per_slot, jb = t % per_slot;
+    const int ps = __ffs(half) - __ffs(g.R);   // log2 of the tiles per slot
+    const int slot = t >> ps, jb = t & ((1 << ps) - 1);
     return W + ((long)slot * hd + (long)m * half + (long)jb * g.R) * g.K;
   }
   if (MODE == PH_GATEUP) return (m == 0 ? W : W2) + (long)t * g.R * g.K;
@@ -109,9 +113,10 @@ __device__ __forceinline__ void consume_phase(const MegaP& p, const MegaPhase& g
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int tn = 0;
   if (tdbg && threadIdx.x == 0) tdbg[tn++] = gtimer();
-  const int rloc = warp % g.R, sub = warp / g.R;
+  const int rsh = __ffs(g.R) - 1;   // (R and S = 8 / R are powers of two, half a head as well)
+  const int rloc = warp & (g.R - 1), sub = warp >> rsh;
   const int nvec = g.K >> 3;
-  const int cb = (int)((long)nvec * sub / g.S), ce = (int)((long)nvec * (sub + 1) / g.S);
+  const int cb = nvec * sub >> (3 - rsh), ce = nvec * (sub + 1) >> (3 - rsh);
   const int rows_unit = g.K * 2;
   // ---- prologue: the 256 consumer threads load / RMS-normalise the activation vector ONCE
   // per CTA into shared memory (one global round trip, two block barriers); each warp then
@@ -120,6 +125,7 @@ __device__ __forceinline__ void consume_phase(const MegaP& p, const MegaPhase& g
   uint4* xs = reinterpret_cast<uint4*>(xs_raw);
   {
     float ss = 0.f;
+#pragma unroll(MODE == PH_DRES ? 4 : 1)
     for (int c = threadIdx.x; c < nvec; c += 256) {
       uint4 v;
       if ((MODE == PH_ORES || MODE == PH_DRES) && io.xpart) {
@@ -152,10 +158,10 @@ __device__ __forceinline__ void consume_phase(const MegaP& p, const MegaPhase& g
       xs[c] = v;
       if (FLOW && T::NORM && MODE != PH_HEAD) reinterpret_cast<uint4*>(io.hraw)[c] = v;
       if (T::NORM) {
-        float f[8];
-        unpack8(v, f);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
+        dot_bf2(ss, v.x, v.x);
+        dot_bf2(ss, v.y, v.y);
+        dot_bf2(ss, v.z, v.z);
+        dot_bf2(ss, v.w, v.w);
       }
     }
     if (T::NORM) {
@@ -166,6 +172,7 @@ __device__ __forceinline__ void consume_phase(const MegaP& p, const MegaPhase& g
 #pragma unroll
       for (int w = 0; w < 8; ++w) tot += sh->s_l[w][0];
       const float rs = 1.0f / sqrtf(tot / (float)g.K + p.d.eps);
+#pragma unroll 1
       for (int c = threadIdx.x; c < nvec; c += 256) {
         float f[8], lf[8];
         unpack8(xs[c], f);
@@ -200,8 +207,8 @@ __device__ __forceinline__ void consume_phase(const MegaP& p, const MegaPhase& g
   float pb1 = 0.f, pb2 = 0.f, pc = 1.f;  // QKV, first tile: bias + inverse frequency
   if (MODE == PH_QKV && (int)blockIdx.x < g.tiles) {
     const int hd = p.d.hd, half = hd >> 1;
-    const int per_slot = half / g.R;
-    const int slot = blockIdx.x / per_slot, j = (blockIdx.x % per_slot) * g.R + rloc;
+    const int ps = __ffs(half) - 1 - rsh;
+    const int slot = blockIdx.x >> ps, j = ((blockIdx.x & ((1 << ps) - 1)) << rsh) + rloc;
     pb1 = bf2f(io.bias[slot * hd + j]);
     pb2 = bf2f(io.bias[slot * hd + j + half]);
     pc = p.inv_freq[j];  // raw inverse frequency; cos/sin are taken in the epilogue so that
@@ -217,8 +224,8 @@ __device__ __forceinline__ void consume_phase(const MegaP& p, const MegaPhase& g
     if (MODE == PH_QKV) {
       if (mine) {
         const int hd = p.d.hd, half = hd >> 1;
-        const int per_slot = half / g.R;
-        const int slot = t / per_slot, j = (t % per_slot) * g.R + rloc;
+        const int ps = __ffs(half) - 1 - rsh;
+        const int slot = t >> ps, j = ((t & ((1 << ps) - 1)) << rsh) + rloc;
         const int r1 = slot * hd + j, r2 = r1 + half;
         const float y1 = rbf(keep0 + (ti == 0 ? pb1 : bf2f(io.bias[r1])));
         const float y2 = rbf(keep1 + (ti == 0 ? pb2 : bf2f(io.bias[r2])));
@@ -268,84 +275,87 @@ __device__ __forceinline__ void consume_phase(const MegaP& p, const MegaPhase& g
       }
     }
   };
-  int it = 0;
-  for (int t = blockIdx.x; t < g.tiles; t += gridDim.x, ++it) {
-    const int s = rg.slot();
-    int rows = g.R;
-    if (MODE != PH_QKV) rows = min(g.R, g.N - t * g.R);
-    mb_wait(&sh->full_bar[s], rg.parity(), &sh->err);
-    if (tdbg && threadIdx.x == 0 && tn < 30) tdbg[tn++] = gtimer();
-    rg.advance();
-    const uint8_t* base = ring + (long)s * p.stage_bytes + (long)rloc * rows_unit;
-    float acc[T::NRW];
-    {
-      float a8[T::NRW][8];
+  // ---- the tiles, TB at a time: 8 sums per lane are reduced over the warp together (9 shuffles instead of 40), and where warps share
+  // a row (S > 1) they meet once per batch.  The products are mixed-precision FMAs (bf16 x bf16 + fp32, the roundings of an fp32 FMA
+  // on the unpacked values), so a tile costs little more than its way out of shared memory: 48 KB in 592 cycles with both operands
+  // unpacked for packed fp32 FMAs, 487 with x unpacked beforehand, 399 so (of 384).
+  constexpr int TB = 8 / T::NRW;
+  const int n_it = ((int)blockIdx.x < g.tiles) ? (g.tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+#pragma unroll 1
+  for (int it0 = 0; it0 < n_it; it0 += TB) {
+    float sums[8];
 #pragma unroll
-      for (int m = 0; m < T::NRW; ++m)
+    for (int k = 0; k < 8; ++k) sums[k] = 0.f;
+    const int n_b = min(TB, n_it - it0);
+#pragma unroll 1
+    for (int i = 0; i < n_b; ++i) {   // (rolled: a layer's code has to stay in the instruction cache from one layer to the next)
+      const int t = blockIdx.x + (it0 + i) * gridDim.x;
+      const int s = rg.slot();
+      int rows = g.R;
+      if (MODE != PH_QKV) rows = min(g.R, g.N - t * g.R);
+      mb_wait(&sh->full_bar[s], rg.parity(), &sh->err);
+      if (tdbg && threadIdx.x == 0 && tn < 30) tdbg[tn++] = gtimer();
+      rg.advance();
+      const uint8_t* base = ring + (long)s * p.stage_bytes + (long)rloc * rows_unit;
+      // the whole tile slice of this warp -> registers first (one LDS latency per tile); the slot is free then
+      uint4 w4[T::NRW][CHX];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) a8[m][j] = 0.f;
-      if (rloc < rows) {
-        // the whole tile slice of this warp -> registers first (one LDS latency per tile),
-        // then NRW*8 independent FMA chains
-        uint4 w4[T::NRW][CHX];
+      for (int u = 0; u < CHX; ++u) {
+        const int c = cb + lane + 32 * u;
+#pragma unroll
+        for (int m = 0; m < T::NRW; ++m)
+          w4[m][u] = (c < ce && rloc < rows) ? *reinterpret_cast<const uint4*>(base + (long)m * g.R * rows_unit + (long)c * 16)
+                                             : make_uint4(0, 0, 0, 0);
+      }
+      __syncwarp();
+      if (lane == 0) mb_arrive(&sh->empty_bar[s]);
+#pragma unroll
+      for (int m = 0; m < T::NRW; ++m) {
+        float a8[8];   // independent chains
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a8[j] = 0.f;
 #pragma unroll
         for (int u = 0; u < CHX; ++u) {
-          const int c = cb + lane + 32 * u;
-#pragma unroll
-          for (int m = 0; m < T::NRW; ++m)
-            w4[m][u] = (c < ce) ? *reinterpret_cast<const uint4*>(base + (long)m * g.R * rows_unit +
-                                                                  (long)c * 16)
-                                : make_uint4(0, 0, 0, 0);
+          fma_bf2(a8[0], a8[1], w4[m][u].x, xv[u].x);
+          fma_bf2(a8[2], a8[3], w4[m][u].y, xv[u].y);
+          fma_bf2(a8[4], a8[5], w4[m][u].z, xv[u].z);
+          fma_bf2(a8[6], a8[7], w4[m][u].w, xv[u].w);
         }
+        const float a = ((a8[0] + a8[1]) + (a8[2] + a8[3])) + ((a8[4] + a8[5]) + (a8[6] + a8[7]));
 #pragma unroll
-        for (int u = 0; u < CHX; ++u) {
-          float xf[8];
-          unpack8(xv[u], xf);
-#pragma unroll
-          for (int m = 0; m < T::NRW; ++m) {
-            float wf[8];
-            unpack8(w4[m][u], wf);
-#pragma unroll
-            for (int j = 0; j < 8; j += 2)
-              ffma2(a8[m][j], a8[m][j + 1], wf[j], wf[j + 1], xf[j], xf[j + 1]);
-          }
-        }
+        for (int k = m; k < 8; k += T::NRW) sums[k] = k == i * T::NRW + m ? a : sums[k];
       }
-#pragma unroll
-      for (int m = 0; m < T::NRW; ++m)
-        acc[m] = ((a8[m][0] + a8[m][1]) + (a8[m][2] + a8[m][3])) +
-                 ((a8[m][4] + a8[m][5]) + (a8[m][6] + a8[m][7]));
+      if (tdbg && threadIdx.x == 0 && tn < 30) tdbg[tn++] = gtimer();
     }
-#pragma unroll
-    for (int m = 0; m < T::NRW; ++m) acc[m] = warp_sum(acc[m]);
-    __syncwarp();
-    if (lane == 0) mb_arrive(&sh->empty_bar[s]);
-    if (tdbg && threadIdx.x == 0 && tn < 30) tdbg[tn++] = gtimer();
-    if (g.S > 1) {
-      if (lane == 0) {
-#pragma unroll
-        for (int m = 0; m < T::NRW; ++m) sh->red[it & 1][warp][m] = acc[m];
-      }
-      cbar();
-      if (sub == 0) {
-#pragma unroll
-        for (int m = 0; m < T::NRW; ++m) {
-          float a = 0.f;
-          for (int q = 0; q < g.S; ++q) a += sh->red[it & 1][rloc + q * g.R][m];
-          acc[m] = a;
-        }
-      }
-    }
-    // ---- deferred epilogue: lane (it % 32) keeps this tile's sums; the per-row math
+    const float sum = warp_sum8(sums, lane);   // value lane / 4 of the batch
+    // ---- deferred epilogue: lane (tile % 32) keeps a tile's sums; the per-row math
     // (SwiGLU / rotary / residual / logsumexp) runs once per 32 tiles, one tile per lane,
     // instead of once per tile on lane 0 (measured: 0.38 us of a 1.02 us tile period)
-    if (lane == (it & 31)) {
-      keep0 = acc[0];
-      keep1 = acc[T::NRW - 1];
+    const int v = (lane & (TB - 1)) * T::NRW;   // the lane's tile of the batch, its first value
+    float k0, k1;
+    if (g.S > 1) {
+      float (*red)[8] = sh->red[(it0 / TB) & 1];
+      if ((lane & 3) == 0) red[warp][lane >> 2] = sum;
+      cbar();
+      k0 = k1 = 0.f;
+      if (sub == 0) {
+#pragma unroll 1
+        for (int q = 0; q < g.S; ++q) {
+          k0 += red[rloc + q * g.R][v];
+          k1 += red[rloc + q * g.R][v + T::NRW - 1];
+        }
+      }
+    } else {
+      k0 = __shfl_sync(0xffffffffu, sum, v * 4);
+      k1 = __shfl_sync(0xffffffffu, sum, (v + T::NRW - 1) * 4);
     }
-    if ((it & 31) == 31) flush(it - 31, 32);
+    if ((lane & ~(TB - 1)) == (it0 & 31)) {
+      keep0 = k0;
+      keep1 = k1;
+    }
+    const int done = min(it0 + TB, n_it);
+    if ((done & 31) == 0 || done == n_it) flush((done - 1) & ~31, ((done - 1) & 31) + 1);   // (one call: it is inlined)
   }
-  if (it & 31) flush(it & ~31, it & 31);
   if (MODE == PH_HEAD) {
     if (lane == 0) sh->wstat[warp] = make_float2(run_m, run_l);
     cbar();

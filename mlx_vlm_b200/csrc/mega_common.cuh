@@ -25,10 +25,10 @@ __device__ __forceinline__ void mb_arrive(uint64_t* bar) {
 }
 // bounded wait: a scheduling bug must not hang the GPU (sets *err and falls through)
 __device__ __forceinline__ void mb_wait(uint64_t* bar, uint32_t parity, int* err) {
-  uint32_t done;
   const uint32_t addr = s_u32(bar);
+  uint32_t done = mbar_test(addr, parity);   // (a try_wait takes some 200 cycles even where the phase is over)
   unsigned spins = 0;
-  do {
+  while (!done) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -40,7 +40,7 @@ __device__ __forceinline__ void mb_wait(uint64_t* bar, uint32_t parity, int* err
       *err = 2;
       break;
     }
-  } while (!done);
+  }
 }
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar,
                                          uint64_t policy) {
@@ -112,6 +112,48 @@ __device__ __forceinline__ void ffma2(float& d0, float& d1, float a0, float a1, 
       : "+f"(d0), "+f"(d1)
       : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
 }
+// the same of two bf16 pairs as they are: d0 += lo * lo, d1 += hi * hi, each rounded once like an fp32 FMA of the unpacked values
+__device__ __forceinline__ void fma_bf2(float& d0, float& d1, uint32_t a, uint32_t b) {
+  asm("{\n\t.reg .b16 al, ah, bl, bh;\n\t"
+      "mov.b32 {al, ah}, %2;\n\tmov.b32 {bl, bh}, %3;\n\t"
+      "fma.rn.f32.bf16 %0, al, bl, %0;\n\tfma.rn.f32.bf16 %1, ah, bh, %1;\n\t}"
+      : "+f"(d0), "+f"(d1)
+      : "r"(a), "r"(b));
+}
+// both onto one sum, lo first
+__device__ __forceinline__ void dot_bf2(float& s, uint32_t a, uint32_t b) {
+  asm("{\n\t.reg .b16 al, ah, bl, bh;\n\t"
+      "mov.b32 {al, ah}, %1;\n\tmov.b32 {bl, bh}, %2;\n\t"
+      "fma.rn.f32.bf16 %0, al, bl, %0;\n\tfma.rn.f32.bf16 %0, ah, bh, %0;\n\t}"
+      : "+f"(s)
+      : "r"(a), "r"(b));
+}
+// a pair times one number: p is a bf16 value in fp32
+__device__ __forceinline__ void axpy_bf2(float& d0, float& d1, float p, uint32_t v) {
+  asm("{\n\t.reg .b16 pl, ph, vl, vh;\n\t"
+      "mov.b32 {pl, ph}, %2;\n\tmov.b32 {vl, vh}, %3;\n\t"
+      "fma.rn.f32.bf16 %0, ph, vl, %0;\n\tfma.rn.f32.bf16 %1, ph, vh, %1;\n\t}"
+      : "+f"(d0), "+f"(d1)
+      : "r"(__float_as_uint(p)), "r"(v));
+}
+// warp_sum of 8 values at once, by the same tree: lane L gets the sum of value L / 4
+__device__ __forceinline__ float warp_sum8(const float (&x)[8], int lane) {
+  float a[4], b[2];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const bool up = lane & 16;
+    a[k] = (up ? x[k + 4] : x[k]) + __shfl_xor_sync(0xffffffffu, up ? x[k] : x[k + 4], 16);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const bool up = lane & 8;
+    b[k] = (up ? a[k + 2] : a[k]) + __shfl_xor_sync(0xffffffffu, up ? a[k] : a[k + 2], 8);
+  }
+  const bool up = lane & 4;
+  float s = (up ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, up ? b[0] : b[1], 4);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  return s + __shfl_xor_sync(0xffffffffu, s, 1);
+}
 __device__ __forceinline__ void cbar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
@@ -157,7 +199,7 @@ __device__ __forceinline__ float fix_get(const long long* acc) {
 
 struct MegaShared {
   uint64_t full_bar[8], empty_bar[8];
-  float red[2][8][2];
+  float red[2][8][8];   // [batch][warp][sum of the batch]
   float2 wstat[8];
   float s_m[8][MEGA_ATT_G], s_l[8][MEGA_ATT_G];
   unsigned long long bar_base;
@@ -283,7 +325,7 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
       else vraw[q].x = __ldcg(reinterpret_cast<const uint32_t*>(vr));
     }
   }
-  float qr[AG][SEG];
+  uint32_t qp[AG][SEG / 2];   // q * scale, rounded to bf16: pairs, as the keys lie
   if (AMODE == ATT_FLOW) {
     // poll the finished q (x scale) / new k / new v pairs published by the qkv phase
     const int half = HD / 2;
@@ -318,7 +360,8 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
 #pragma unroll
     for (int g = 0; g < AG; ++g)
 #pragma unroll
-      for (int i = 0; i < SEG; ++i) qr[g][i] = (g < G) ? qs[(long)g * HD + seg * SEG + i] : 0.f;
+      for (int i = 0; i < SEG / 2; ++i)
+        qp[g][i] = (g < G) ? pack2(qs[(long)g * HD + seg * SEG + 2 * i], qs[(long)g * HD + seg * SEG + 2 * i + 1]) : 0u;
   } else if (PARTS) {
     const int half = HD / 2;
     const int nslot = G + (owner ? 2 : 0);
@@ -358,16 +401,16 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
 #pragma unroll
     for (int g = 0; g < AG; ++g)
 #pragma unroll
-      for (int i = 0; i < SEG; ++i) qr[g][i] = (g < G) ? qs[(long)g * HD + seg * SEG + i] : 0.f;
+      for (int i = 0; i < SEG / 2; ++i)
+        qp[g][i] = (g < G) ? pack2(qs[(long)g * HD + seg * SEG + 2 * i], qs[(long)g * HD + seg * SEG + 2 * i + 1]) : 0u;
   } else {
 #pragma unroll
     for (int g = 0; g < AG; ++g)
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
-        float f[8];
-        unpack8(qraw[g][v], f);
+        const uint32_t w[4] = {qraw[g][v].x, qraw[g][v].y, qraw[g][v].z, qraw[g][v].w};
 #pragma unroll
-        for (int i = 0; i < 8; ++i) qr[g][v * 8 + i] = rbf(f[i] * d.scale_bf);
+        for (int i = 0; i < 4; ++i) qp[g][v * 4 + i] = pack_bf2(mul2(unpack_bf2(w[i]), f2(d.scale_bf, d.scale_bf)));
       }
   }
   ATT_STAMP();  // q loaded
@@ -375,6 +418,7 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
   float lm[AG];
 #pragma unroll
   for (int g = 0; g < AG; ++g) lm[g] = -INFINITY;
+#pragma unroll 1
   for (int j0 = u0 + warp * 4; j0 < u1g; j0 += 32 * UNR) {
     uint4 kv[UNR][NV];
 #pragma unroll
@@ -399,12 +443,13 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
       for (int g = 0; g < AG; ++g) s[g] = 0.f;
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
-        float kf[8];
-        unpack8(kv[q][v], kf);
 #pragma unroll
-        for (int g = 0; g < AG; ++g)
-#pragma unroll
-          for (int i = 0; i < 8; ++i) s[g] = fmaf(qr[g][v * 8 + i], kf[i], s[g]);
+        for (int g = 0; g < AG; ++g) {
+          dot_bf2(s[g], qp[g][v * 4], kv[q][v].x);
+          dot_bf2(s[g], qp[g][v * 4 + 1], kv[q][v].y);
+          dot_bf2(s[g], qp[g][v * 4 + 2], kv[q][v].z);
+          dot_bf2(s[g], qp[g][v * 4 + 3], kv[q][v].w);
+        }
       }
 #pragma unroll
       for (int o = 1; o < 8; o <<= 1)
@@ -434,19 +479,6 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
     }
   }
   ATT_STAMP();  // scores done
-  float vpre[VPRE][EPL];
-#pragma unroll
-  for (int q = 0; q < VPRE; ++q) {
-    if (EPL == 4) {
-      float t4[4];
-      unpack4(vraw[q], t4);
-#pragma unroll
-      for (int e = 0; e < EPL; ++e) vpre[q][e] = t4[e];
-    } else {
-      vpre[q][0] = __uint_as_float(vraw[q].x << 16);
-      vpre[q][EPL - 1] = __uint_as_float(vraw[q].x & 0xffff0000u);
-    }
-  }
 #pragma unroll
   for (int g = 0; g < AG; ++g) {
     lm[g] = warp_max(lm[g]);
@@ -462,6 +494,7 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
     ml[g] = m;
     ls[g] = 0.f;
   }
+#pragma unroll 1
   for (int j = threadIdx.x; j < u1 - u0; j += 256) {
 #pragma unroll
     for (int g = 0; g < AG; ++g) ls[g] += expf(sc[(long)g * ucap + j] - ml[g]);
@@ -527,6 +560,7 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
     L[g] = sh->s_l[0][g];
   }
   // p = bf16(exp(s - M) / L) for the own keys, one key per thread, in place
+#pragma unroll 1
   for (int j = threadIdx.x; j < u1 - u0; j += 256) {
 #pragma unroll
     for (int g = 0; g < AG; ++g)
@@ -546,8 +580,8 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
 #pragma unroll
       for (int g = 0; g < AG; ++g) {
         const float pj = sc[(long)g * ucap + (j - u0)];
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) acc[g][e] = fmaf(pj, vpre[q][e], acc[g][e]);
+        axpy_bf2(acc[g][0], acc[g][1], pj, vraw[q].x);
+        if (EPL == 4) axpy_bf2(acc[g][EPL - 2], acc[g][EPL - 1], pj, vraw[q].y);
       }
     }
   }
@@ -559,25 +593,17 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
       for (int e = 0; e < EPL; ++e) acc[g][e] = fmaf(pj, vn[lane * EPL + e], acc[g][e]);
     }
   }
+#pragma unroll 1
   for (int j0 = u0 + warp + 8 * VPRE; j0 < u1g; j0 += 32) {  // 4 keys per trip, loads first
-    float vf[4][EPL];
+    uint2 vw[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int j = j0 + 8 * q;
-#pragma unroll
-      for (int e = 0; e < EPL; ++e) vf[q][e] = 0.f;
+      vw[q] = make_uint2(0, 0);
       if (j < u1g) {
         const bf16* vr = vb + (long)j * HD + lane * EPL;
-        if (EPL == 4) {
-          float t4[4];
-          unpack4(__ldcg(reinterpret_cast<const uint2*>(vr)), t4);
-#pragma unroll
-          for (int e = 0; e < EPL; ++e) vf[q][e] = t4[e];
-        } else {
-          const uint32_t w = __ldcg(reinterpret_cast<const uint32_t*>(vr));
-          vf[q][0] = __uint_as_float(w << 16);
-          vf[q][EPL - 1] = __uint_as_float(w & 0xffff0000u);
-        }
+        if (EPL == 4) vw[q] = __ldcg(reinterpret_cast<const uint2*>(vr));
+        else vw[q].x = __ldcg(reinterpret_cast<const uint32_t*>(vr));
       }
     }
 #pragma unroll
@@ -587,8 +613,8 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
 #pragma unroll
         for (int g = 0; g < AG; ++g) {
           const float pj = sc[(long)g * ucap + (j - u0)];
-#pragma unroll
-          for (int e = 0; e < EPL; ++e) acc[g][e] = fmaf(pj, vf[q][e], acc[g][e]);
+          axpy_bf2(acc[g][0], acc[g][1], pj, vw[q].x);
+          if (EPL == 4) axpy_bf2(acc[g][EPL - 2], acc[g][EPL - 1], pj, vw[q].y);
         }
       }
     }
@@ -600,6 +626,7 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
   ATT_STAMP();  // PV done
   cbar();
   float* mypart = p.att_part + ((long)grp * ATT_UN + unit) * AG * HD;
+#pragma unroll 1
   for (int i = threadIdx.x; i < G * HD; i += 256) {
     float s = 0.f;
 #pragma unroll
