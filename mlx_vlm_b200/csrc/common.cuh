@@ -101,6 +101,49 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// products of bf16 pairs as they are: d0 += lo * lo, d1 += hi * hi, each rounded once like an fp32 FMA of the unpacked values
+__device__ __forceinline__ void fma_bf2(float& d0, float& d1, uint32_t a, uint32_t b) {
+  asm("{\n\t.reg .b16 al, ah, bl, bh;\n\t"
+      "mov.b32 {al, ah}, %2;\n\tmov.b32 {bl, bh}, %3;\n\t"
+      "fma.rn.f32.bf16 %0, al, bl, %0;\n\tfma.rn.f32.bf16 %1, ah, bh, %1;\n\t}"
+      : "+f"(d0), "+f"(d1)
+      : "r"(a), "r"(b));
+}
+// both onto one sum, lo first
+__device__ __forceinline__ void dot_bf2(float& s, uint32_t a, uint32_t b) {
+  asm("{\n\t.reg .b16 al, ah, bl, bh;\n\t"
+      "mov.b32 {al, ah}, %1;\n\tmov.b32 {bl, bh}, %2;\n\t"
+      "fma.rn.f32.bf16 %0, al, bl, %0;\n\tfma.rn.f32.bf16 %0, ah, bh, %0;\n\t}"
+      : "+f"(s)
+      : "r"(a), "r"(b));
+}
+// a pair times one number: p is a bf16 value in fp32
+__device__ __forceinline__ void axpy_bf2(float& d0, float& d1, float p, uint32_t v) {
+  asm("{\n\t.reg .b16 pl, ph, vl, vh;\n\t"
+      "mov.b32 {pl, ph}, %2;\n\tmov.b32 {vl, vh}, %3;\n\t"
+      "fma.rn.f32.bf16 %0, ph, vl, %0;\n\tfma.rn.f32.bf16 %1, ph, vh, %1;\n\t}"
+      : "+f"(d0), "+f"(d1)
+      : "r"(__float_as_uint(p)), "r"(v));
+}
+// warp_sum of 8 values at once, by the same tree: lane L gets the sum of value L / 4
+__device__ __forceinline__ float warp_sum8(const float (&x)[8], int lane) {
+  float a[4], b[2];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const bool up = lane & 16;
+    a[k] = (up ? x[k + 4] : x[k]) + __shfl_xor_sync(0xffffffffu, up ? x[k] : x[k + 4], 16);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const bool up = lane & 8;
+    b[k] = (up ? a[k + 2] : a[k]) + __shfl_xor_sync(0xffffffffu, up ? a[k] : a[k + 2], 8);
+  }
+  const bool up = lane & 4;
+  float s = (up ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, up ? b[0] : b[1], 4);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  return s + __shfl_xor_sync(0xffffffffu, s, 1);
+}
+
 // ---- activation restatements (oracle/mlx_semantics.py) --------------------
 // 1 / (1 + e^-x) with the SFU exponential and reciprocal (branch-free, ~3 ulp): far below the bf16 rounding every
 // bf16 caller applies next and below the 2^-17 of the split-operand GEMMs on the fp32 paths (the libm expf + IEEE

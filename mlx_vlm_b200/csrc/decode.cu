@@ -58,17 +58,9 @@ __device__ __forceinline__ void mb_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void mb_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t done;
   const uint32_t addr = s_u32(bar);
-  do {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-  } while (!done);
+  uint32_t done = mbar_test(addr, parity);
+  while (!done) done = mbar_try(addr, parity);
 }
 // 1-D bulk copy global -> shared through the TMA engine, evict-first in L2
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar,
@@ -143,7 +135,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 2) k_stream(const StreamP p) {
   using T = StreamTraits<MODE>;
   extern __shared__ __align__(128) uint8_t sm[];
   __shared__ uint64_t full_bar[8], empty_bar[8];
-  __shared__ float red[2][8][2];
+  __shared__ float red[2][8][8];   // [batch][warp][sum of the batch]
   __shared__ float2 wstat[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_launch_dependents();
@@ -164,10 +156,10 @@ __global__ void __launch_bounds__(STREAM_THREADS, 2) k_stream(const StreamP p) {
     // ===== producer: independent of the previous kernel -> runs ahead under PDL =====
     if (lane == 0) {
       const uint64_t pol = policy_evict_first();
+      int s = 0;   // ring slot and the parity of its round
+      uint32_t ph = 0;
       for (int it = 0; it < my_tiles; ++it) {
         const int t = blockIdx.x + it * gridDim.x;
-        const int s = it % p.n_stages;
-        const uint32_t ph = (it / p.n_stages) & 1;
         mb_wait(&empty_bar[s], ph ^ 1);
         int rows = p.R;
         if (MODE != SM_QKV) rows = min(p.R, p.N - t * p.R);
@@ -177,6 +169,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 2) k_stream(const StreamP p) {
         bulk_g2s(dst, tile_src<MODE>(p, t, 0), bytes, &full_bar[s], pol);
         if (T::PAIR) bulk_g2s(dst + (long)p.R * rows_unit, tile_src<MODE>(p, t, 1), bytes,
                               &full_bar[s], pol);
+        if (++s == p.n_stages) s = 0, ph ^= 1;
       }
     }
     return;
@@ -234,84 +227,91 @@ __global__ void __launch_bounds__(STREAM_THREADS, 2) k_stream(const StreamP p) {
       xv[u].w = pack2(f[6], f[7]);
     }
   }
-  float run_m = -INFINITY, run_l = 0.f;  // HEAD: running logsumexp (lane 0 of slice-0 warps)
+  float run_m = -INFINITY, run_l = 0.f;  // HEAD: running logsumexp of the lane's rows (slice-0 warps)
   int ctx = 0, pos = 0;
   if (MODE == SM_QKV) {
     ctx = p.st->ctx;
     pos = p.st->pos;
   }
 
-  for (int it = 0; it < my_tiles; ++it) {
-    const int t = blockIdx.x + it * gridDim.x;
-    const int s = it % p.n_stages;
-    const uint32_t ph = (it / p.n_stages) & 1;
-    int rows = p.R;
-    if (MODE != SM_QKV) rows = min(p.R, p.N - t * p.R);
-    mb_wait(&full_bar[s], ph);
-    const uint8_t* base = sm + (long)s * p.stage_bytes + (long)rloc * rows_unit;
-    float acc[T::NRW];
-    {
+  // tiles TB at a time, as in k_mega (decode_mega.cu): mixed-precision FMAs, eight sums reduced over the warp together, one meeting of
+  // the warps that share a row (S > 1) and one epilogue, a tile per lane, for a batch; the slot is free when it has been read.  The
+  // head of 16384 rows of 3584 (tile by tile, with a logsumexp step of one lane in each): 54 us, so 28.
+  constexpr int TB = 8 / T::NRW, CU = (CHX > 6 ? 4 : 8) / T::NRW;   // row pieces of 16 bytes per lane in flight
+  int s = 0;
+  uint32_t ph = 0;
+#pragma unroll 1
+  for (int it0 = 0; it0 < my_tiles; it0 += TB) {
+    float sums[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) sums[k] = 0.f;
+    const int n_b = min(TB, my_tiles - it0);
+#pragma unroll 1
+    for (int i = 0; i < n_b; ++i) {
+      int rows = p.R;
+      if (MODE != SM_QKV) rows = min(p.R, p.N - ((int)blockIdx.x + (it0 + i) * (int)gridDim.x) * p.R);
+      mb_wait(&full_bar[s], ph);
+      const uint8_t* base = sm + (long)s * p.stage_bytes + (long)rloc * rows_unit;
+      const int end = rloc < rows ? ce : 0;
       // 8 independent partial sums per row: the FMAs of a chunk do not chain
       float a8[T::NRW][8];
 #pragma unroll
       for (int m = 0; m < T::NRW; ++m)
 #pragma unroll
         for (int j = 0; j < 8; ++j) a8[m][j] = 0.f;
-      if (rloc < rows) {
 #pragma unroll
-        for (int u0 = 0; u0 < CHX; u0 += 2) {  // two chunks (LDS.128) in flight per row
-          uint4 w4[T::NRW][2];
+      for (int u0 = 0; u0 < CHX; u0 += CU) {
+        uint4 w4[T::NRW][CU];
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const int c = cb + lane + 32 * (u0 + q);
+        for (int q = 0; q < CU; ++q) {
+          const int c = cb + lane + 32 * (u0 + q);
 #pragma unroll
-            for (int m = 0; m < T::NRW; ++m)
-              w4[m][q] = (u0 + q < CHX && c < ce)
-                             ? *reinterpret_cast<const uint4*>(base + (long)m * p.R * rows_unit +
-                                                               (long)c * 16)
-                             : make_uint4(0, 0, 0, 0);
-          }
+          for (int m = 0; m < T::NRW; ++m)
+            w4[m][q] = (u0 + q < CHX && c < end) ? *reinterpret_cast<const uint4*>(base + (long)m * p.R * rows_unit + (long)c * 16)
+                                                 : make_uint4(0, 0, 0, 0);
+        }
+        if (u0 + CU >= CHX) {
+          __syncwarp();
+          if (lane == 0) mb_arrive(&empty_bar[s]);  // this warp has read the stage
+        }
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            if (u0 + q < CHX) {
-              float xf[8];
-              unpack8(xv[u0 + q], xf);
+        for (int q = 0; q < CU; ++q)
+          if (u0 + q < CHX)
 #pragma unroll
-              for (int m = 0; m < T::NRW; ++m) {
-                float wf[8];
-                unpack8(w4[m][q], wf);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) a8[m][j] = fmaf(wf[j], xf[j], a8[m][j]);
-              }
+            for (int m = 0; m < T::NRW; ++m) {
+              fma_bf2(a8[m][0], a8[m][1], w4[m][q].x, xv[u0 + q].x);
+              fma_bf2(a8[m][2], a8[m][3], w4[m][q].y, xv[u0 + q].y);
+              fma_bf2(a8[m][4], a8[m][5], w4[m][q].z, xv[u0 + q].z);
+              fma_bf2(a8[m][6], a8[m][7], w4[m][q].w, xv[u0 + q].w);
             }
-          }
-        }
       }
+      if (++s == p.n_stages) s = 0, ph ^= 1;
 #pragma unroll
-      for (int m = 0; m < T::NRW; ++m)
-        acc[m] = ((a8[m][0] + a8[m][1]) + (a8[m][2] + a8[m][3])) +
-                 ((a8[m][4] + a8[m][5]) + (a8[m][6] + a8[m][7]));
+      for (int m = 0; m < T::NRW; ++m) {
+        const float a = ((a8[m][0] + a8[m][1]) + (a8[m][2] + a8[m][3])) + ((a8[m][4] + a8[m][5]) + (a8[m][6] + a8[m][7]));
+#pragma unroll
+        for (int k = m; k < 8; k += T::NRW) sums[k] = k == i * T::NRW + m ? a : sums[k];
+      }
     }
-#pragma unroll
-    for (int m = 0; m < T::NRW; ++m) acc[m] = warp_sum(acc[m]);
-    __syncwarp();
-    if (lane == 0) mb_arrive(&empty_bar[s]);  // this warp is done reading the stage
+    const float sum = warp_sum8(sums, lane);   // value lane / 4 of the batch
+    const int v = (lane & (TB - 1)) * T::NRW;   // the lane's tile of the batch, its first value
+    float acc[T::NRW];
     if (p.S > 1) {  // split-K: combine the slices of a row through shared memory
-      if (lane == 0) {
-#pragma unroll
-        for (int m = 0; m < T::NRW; ++m) red[it & 1][warp][m] = acc[m];
-      }
+      float (*rb)[8] = red[(it0 / TB) & 1];
+      if ((lane & 3) == 0) rb[warp][lane >> 2] = sum;
       asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (sub == 0) {
 #pragma unroll
-        for (int m = 0; m < T::NRW; ++m) {
-          float a = 0.f;
-          for (int q = 0; q < p.S; ++q) a += red[it & 1][rloc + q * p.R][m];
-          acc[m] = a;
-        }
-      }
+      for (int m = 0; m < T::NRW; ++m) acc[m] = 0.f;
+      if (sub == 0)
+        for (int q = 0; q < p.S; ++q)
+#pragma unroll
+          for (int m = 0; m < T::NRW; ++m) acc[m] += rb[rloc + q * p.R][v + m];
+    } else {
+#pragma unroll
+      for (int m = 0; m < T::NRW; ++m) acc[m] = __shfl_sync(0xffffffffu, sum, (v + m) * 4);
     }
-    if (sub == 0 && lane == 0 && rloc < rows) {
+    const int t = blockIdx.x + (it0 + lane) * gridDim.x;
+    if (sub == 0 && lane < n_b && (MODE == SM_QKV || t * p.R + rloc < p.N)) {
       if (MODE == SM_QKV) {
         const int half = p.hd >> 1;
         const int per_slot = half / p.R;
@@ -351,7 +351,8 @@ __global__ void __launch_bounds__(STREAM_THREADS, 2) k_stream(const StreamP p) {
     }
   }
   if (MODE == SM_HEAD) {
-    if (lane == 0) wstat[warp] = make_float2(run_m, run_l);
+    const float wm = warp_max(run_m), wl = warp_sum(run_l > 0.f ? run_l * expf(run_m - wm) : 0.f);
+    if (lane == 0) wstat[warp] = make_float2(wm, wl);
     asm volatile("bar.sync 1, 256;" ::: "memory");
     if (threadIdx.x == 0) {
       float M = -INFINITY;
