@@ -378,7 +378,13 @@ __device__ __forceinline__ void consume_phase(const MegaP& p, const MegaPhase& g
 // them because every later phase needs data from ALL CTAs of the phase before it (transitively
 // nobody can overwrite a word that a slower CTA still has to read), and the tag of a word is
 // unique per (step, layer).
-template <int CHH, int CHI, bool FLOW>
+// ATT: the attention that the kernel holds.  One that held all three forms had 217 KB instead of 162 and took 1011 us instead of 996 for
+// a token of the 2B model; the small models and the dataflow mode share a kernel (MA_ANY) all the same.
+enum { MA_ANY = 0, MA_64, MA_128, MA_128_PAIR };   // head dim; PAIR: at most two q heads a CTA
+__host__ __device__ __forceinline__ int mega_att(const MegaP& p) {
+  return p.d.hd == 64 ? MA_64 : (p.hsplit * 2 >= p.d.n_heads / p.d.n_kv ? MA_128_PAIR : MA_128);
+}
+template <int CHH, int CHI, bool FLOW, int ATT>
 __global__ void __launch_bounds__(MEGA_THREADS, 1) k_mega(const MegaP p) {
   extern __shared__ __align__(128) uint8_t sm[];
   __shared__ MegaShared sh;
@@ -463,8 +469,9 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_mega(const MegaP p) {
     if ((int)blockIdx.x < p.attn_ctas) {
       const AttnParts ap = {nullptr, nullptr, 0, p.qkv_w, ep};
       constexpr int AM = FLOW ? ATT_FLOW : ATT_PLAIN;
-      if (d.hd == 128) attn_phase<128, AM>(p, kc, vc, scratch, &sh, ctx + 1, l, ap,
-                                           (p.dbg && l == 5 && blockIdx.x < 2) ? p.dbg + 4096 + 128 + 32 * blockIdx.x : nullptr);
+      long long* td = p.dbg && l == 5 && blockIdx.x < 2 ? p.dbg + 4096 + 128 + 32 * blockIdx.x : nullptr;
+      if (ATT == MA_128_PAIR || (ATT == MA_ANY && mega_att(p) == MA_128_PAIR)) attn_phase<128, AM, 2>(p, kc, vc, scratch, &sh, ctx + 1, l, ap, td);
+      else if (ATT == MA_128 || (ATT == MA_ANY && d.hd == 128)) attn_phase<128, AM>(p, kc, vc, scratch, &sh, ctx + 1, l, ap, td);
       else attn_phase<64, AM>(p, kc, vc, scratch, &sh, ctx + 1, l, ap);
     }
     grid_barrier(p, &sh, bidx);
@@ -578,7 +585,7 @@ int mega_fill(MegaP& p, int sm_count) {
 
 static int mega_chx(const MegaPhase& g) { return cdiv(cdiv(g.K >> 3, g.S), 32); }
 
-template <int CHH, int CHI, bool FLOW>
+template <int CHH, int CHI, bool FLOW, int ATT>
 static int mega_launch_f(const MegaP& p, int grid, size_t smem, cudaStream_t s) {
   // the function attributes are per device (a second engine on another GPU of the same process
   // must opt in again)
@@ -586,9 +593,9 @@ static int mega_launch_f(const MegaP& p, int grid, size_t smem, cudaStream_t s) 
   int dev = 0;
   B200_CUDA(cudaGetDevice(&dev));
   if (!(set_mask >> (dev & 63) & 1ull)) {
-    B200_CUDA(cudaFuncSetAttribute(k_mega<CHH, CHI, FLOW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    B200_CUDA(cudaFuncSetAttribute(k_mega<CHH, CHI, FLOW, ATT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    227 * 1024 - 2048));
-    B200_CUDA(cudaFuncSetAttribute(k_mega<CHH, CHI, FLOW>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    B200_CUDA(cudaFuncSetAttribute(k_mega<CHH, CHI, FLOW, ATT>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                    cudaSharedmemCarveoutMaxShared));
     set_mask |= 1ull << (dev & 63);
   }
@@ -605,13 +612,19 @@ static int mega_launch_f(const MegaP& p, int grid, size_t smem, cudaStream_t s) 
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  B200_CUDA(cudaLaunchKernelEx(&cfg, k_mega<CHH, CHI, FLOW>, p));
+  B200_CUDA(cudaLaunchKernelEx(&cfg, k_mega<CHH, CHI, FLOW, ATT>, p));
   return B200_OK;
 }
 template <int CHH, int CHI>
 static int mega_launch_t(const MegaP& p, int grid, size_t smem, cudaStream_t s) {
-  return p.flow ? mega_launch_f<CHH, CHI, true>(p, grid, smem, s)
-                : mega_launch_f<CHH, CHI, false>(p, grid, smem, s);
+  if (p.flow) return mega_launch_f<CHH, CHI, true, MA_ANY>(p, grid, smem, s);
+  if constexpr (CHH > 2) {
+    const int att = mega_att(p);
+    if (att == MA_64) return mega_launch_f<CHH, CHI, false, MA_64>(p, grid, smem, s);
+    if (att == MA_128) return mega_launch_f<CHH, CHI, false, MA_128>(p, grid, smem, s);
+    return mega_launch_f<CHH, CHI, false, MA_128_PAIR>(p, grid, smem, s);
+  }
+  return mega_launch_f<CHH, CHI, false, MA_ANY>(p, grid, smem, s);
 }
 
 int mega_launch(const MegaP& p, int sm_count, cudaStream_t s) {

@@ -217,14 +217,19 @@ struct AttnParts {
 };
 
 enum { ATT_PLAIN = 0, ATT_PARTS = 1, ATT_FLOW = 2 };
-template <int HD, int AMODE>
+// GN: q heads that a CTA holds at most (2 or MEGA_ATT_G).  With two, half of the products of four are not made, and twice as many keys
+// and values are on their way: a long context is bound by the bytes in flight (6000 keys of 8 kv heads, four layers of 4,096: a step
+// of 472 us, so 431).
+template <int HD, int AMODE, int GN = MEGA_ATT_G>
 __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const bf16* vc,
                                            float* scratch, MegaShared* sh, int nkeys, int layer,
                                            const AttnParts& ap, long long* tdbg = nullptr) {
   int tn = 0;
 #define ATT_STAMP() do { if (tdbg && threadIdx.x == 0 && tn < 30) tdbg[tn++] = gtimer(); } while (0)
   ATT_STAMP();
-  constexpr int EPL = HD / 32, SEG = HD / 8, AG = MEGA_ATT_G, NV = SEG / 8, UNR = 2;
+  constexpr int EPL = HD / 32, SEG = HD / 8, AG = MEGA_ATT_G, NV = SEG / 8;
+  // trips of UNR x 4 keys a warp, of VB value rows
+  constexpr int UNR = GN <= 2 ? 4 : 2, VB = GN <= 2 ? 16 : 8;
   const DecodeDims& d = p.d;
   const int Gall = d.n_heads / d.n_kv;
   // q heads of a kv head are split over p.hsplit CTAs, Gc per CTA; the last part may hold fewer
@@ -251,11 +256,10 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
   const int seg = lane & 7, ksub = lane >> 3;
   // ---- all global requests of the phase are issued before the first use: q, the first
   // 2 x 4 keys of this warp, and the V rows of its first VPRE keys (one round trip) ----
-  constexpr int VPRE = 8;
-  uint4 qraw[AG][NV];
+  uint4 qraw[GN][NV];
   if (!PARTS) {
 #pragma unroll
-    for (int g = 0; g < AG; ++g)
+    for (int g = 0; g < GN; ++g)
 #pragma unroll
       for (int v = 0; v < NV; ++v)
         qraw[g][v] = (g < G) ? ldcg16(p.qbuf + (long)(h0 + g) * HD + seg * SEG + v * 8)
@@ -272,18 +276,21 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
         kvn[q][v] = (j < u1g) ? ldcg16(kb + (long)j * HD + seg * SEG + v * 8) : make_uint4(0, 0, 0, 0);
     }
   }
-  uint2 vraw[VPRE];
+  uint2 vraw[VB];
+  auto load_v = [&](int j0) {   // rows j0, j0 + 8, ..
 #pragma unroll
-  for (int q = 0; q < VPRE; ++q) {
-    const int j = u0 + warp + 8 * q;
-    vraw[q] = make_uint2(0, 0);
-    if (j < u1g) {
-      const bf16* vr = vb + (long)j * HD + lane * EPL;
-      if (EPL == 4) vraw[q] = __ldcg(reinterpret_cast<const uint2*>(vr));
-      else vraw[q].x = __ldcg(reinterpret_cast<const uint32_t*>(vr));
+    for (int q = 0; q < VB; ++q) {
+      const int j = j0 + 8 * q;
+      vraw[q] = make_uint2(0, 0);
+      if (j < u1g) {
+        const bf16* vr = vb + (long)j * HD + lane * EPL;
+        if (EPL == 4) vraw[q] = __ldcg(reinterpret_cast<const uint2*>(vr));
+        else vraw[q].x = __ldcg(reinterpret_cast<const uint32_t*>(vr));
+      }
     }
-  }
-  uint32_t qp[AG][SEG / 2];   // q * scale, rounded to bf16: pairs, as the keys lie
+  };
+  load_v(u0 + warp);
+  uint32_t qp[GN][SEG / 2];   // q * scale, rounded to bf16: pairs, as the keys lie
   if (AMODE == ATT_FLOW) {
     // poll the finished q (x scale) / new k / new v pairs published by the qkv phase
     const int half = HD / 2;
@@ -316,7 +323,7 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
     }
     cbar();
 #pragma unroll
-    for (int g = 0; g < AG; ++g)
+    for (int g = 0; g < GN; ++g)
 #pragma unroll
       for (int i = 0; i < SEG / 2; ++i)
         qp[g][i] = (g < G) ? pack2(qs[(long)g * HD + seg * SEG + 2 * i], qs[(long)g * HD + seg * SEG + 2 * i + 1]) : 0u;
@@ -357,13 +364,13 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
       }
     }
 #pragma unroll
-    for (int g = 0; g < AG; ++g)
+    for (int g = 0; g < GN; ++g)
 #pragma unroll
       for (int i = 0; i < SEG / 2; ++i)
         qp[g][i] = (g < G) ? pack2(qs[(long)g * HD + seg * SEG + 2 * i], qs[(long)g * HD + seg * SEG + 2 * i + 1]) : 0u;
   } else {
 #pragma unroll
-    for (int g = 0; g < AG; ++g)
+    for (int g = 0; g < GN; ++g)
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
         const uint32_t w[4] = {qraw[g][v].x, qraw[g][v].y, qraw[g][v].z, qraw[g][v].w};
@@ -373,9 +380,9 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
   }
   ATT_STAMP();  // q loaded
   // ---- 1. scores of the own range (software-pipelined over trips of 2 x 4 keys) ----
-  float lm[AG];
+  float lm[GN];
 #pragma unroll
-  for (int g = 0; g < AG; ++g) lm[g] = -INFINITY;
+  for (int g = 0; g < GN; ++g) lm[g] = -INFINITY;
 #pragma unroll 1
   for (int j0 = u0 + warp * 4; j0 < u1g; j0 += 32 * UNR) {
     uint4 kv[UNR][NV];
@@ -396,13 +403,13 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
 #pragma unroll
     for (int q = 0; q < UNR; ++q) {
       const int j = j0 + 32 * q + ksub;
-      float s[AG];
+      float s[GN];
 #pragma unroll
-      for (int g = 0; g < AG; ++g) s[g] = 0.f;
+      for (int g = 0; g < GN; ++g) s[g] = 0.f;
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
 #pragma unroll
-        for (int g = 0; g < AG; ++g) {
+        for (int g = 0; g < GN; ++g) {
           dot_bf2(s[g], qp[g][v * 4], kv[q][v].x);
           dot_bf2(s[g], qp[g][v * 4 + 1], kv[q][v].y);
           dot_bf2(s[g], qp[g][v * 4 + 2], kv[q][v].z);
@@ -412,10 +419,10 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
 #pragma unroll
       for (int o = 1; o < 8; o <<= 1)
 #pragma unroll
-        for (int g = 0; g < AG; ++g) s[g] += __shfl_xor_sync(0xffffffffu, s[g], o);
+        for (int g = 0; g < GN; ++g) s[g] += __shfl_xor_sync(0xffffffffu, s[g], o);
       if (j < u1g && seg == 0) {
 #pragma unroll
-        for (int g = 0; g < AG; ++g) {
+        for (int g = 0; g < GN; ++g) {
           const float r = rbf(s[g]);
           sc[(long)g * ucap + (j - u0)] = r;
           lm[g] = fmaxf(lm[g], r);
@@ -425,7 +432,7 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
   }
   if (PARTS && owner && warp == 0) {  // the new key: q . k from shared memory
 #pragma unroll
-    for (int g = 0; g < AG; ++g) {
+    for (int g = 0; g < GN; ++g) {
       float s = 0.f;
 #pragma unroll
       for (int e = 0; e < EPL; ++e)
@@ -438,14 +445,14 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
   }
   ATT_STAMP();  // scores done
 #pragma unroll
-  for (int g = 0; g < AG; ++g) {
+  for (int g = 0; g < GN; ++g) {
     lm[g] = warp_max(lm[g]);
     if (lane == 0) sh->s_m[warp][g] = lm[g];
   }
   cbar();
-  float ml[AG], ls[AG];
+  float ml[GN], ls[GN];
 #pragma unroll
-  for (int g = 0; g < AG; ++g) {
+  for (int g = 0; g < GN; ++g) {
     float m = -INFINITY;
 #pragma unroll
     for (int w = 0; w < 8; ++w) m = fmaxf(m, sh->s_m[w][g]);
@@ -455,10 +462,10 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
 #pragma unroll 1
   for (int j = threadIdx.x; j < u1 - u0; j += 256) {
 #pragma unroll
-    for (int g = 0; g < AG; ++g) ls[g] += expf(sc[(long)g * ucap + j] - ml[g]);
+    for (int g = 0; g < GN; ++g) ls[g] += expf(sc[(long)g * ucap + j] - ml[g]);
   }
 #pragma unroll
-  for (int g = 0; g < AG; ++g) {
+  for (int g = 0; g < GN; ++g) {
     ls[g] = warp_sum(ls[g]);
     if (lane == 0) sh->s_l[warp][g] = ls[g];
   }
@@ -476,11 +483,15 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
     const uint32_t epoch = (uint32_t)(sh->att_base + (unsigned long long)layer + 1ull);
     if (warp == 0) {
       if (lane < AG) {
-        float l = 0.f;
+        float l = 0.f, mm = -INFINITY;
+        if (lane < GN)   // (the slots of more heads take part with nothing)
 #pragma unroll
-        for (int w = 0; w < 8; ++w) l += sh->s_l[w][lane];
+          for (int w = 0; w < 8; ++w) {
+            l += sh->s_l[w][lane];
+            mm = fmaxf(mm, sh->s_m[w][lane]);
+          }
         const float lv = (u1 > u0) ? l : 0.f;
-        const unsigned long long wm = ((unsigned long long)__float_as_uint(ml[lane]) << 32) | epoch;
+        const unsigned long long wm = ((unsigned long long)__float_as_uint(mm) << 32) | epoch;
         const unsigned long long wl = ((unsigned long long)__float_as_uint(lv) << 32) | epoch;
         asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(gw + (long)(unit * AG + lane) * 2),
                      "l"(wm), "l"(wl)
@@ -511,9 +522,9 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
   }
   cbar();
   ATT_STAMP();  // statistics exchanged
-  float M[AG], L[AG];
+  float M[GN], L[GN];
 #pragma unroll
-  for (int g = 0; g < AG; ++g) {
+  for (int g = 0; g < GN; ++g) {
     M[g] = sh->s_m[0][g];
     L[g] = sh->s_l[0][g];
   }
@@ -521,55 +532,29 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
 #pragma unroll 1
   for (int j = threadIdx.x; j < u1 - u0; j += 256) {
 #pragma unroll
-    for (int g = 0; g < AG; ++g)
+    for (int g = 0; g < GN; ++g)
       sc[(long)g * ucap + j] = rbf(expf(sc[(long)g * ucap + j] - M[g]) / L[g]);
   }
   cbar();
   ATT_STAMP();  // global stats read
-  float acc[AG][EPL];
+  float acc[GN][EPL];
 #pragma unroll
-  for (int g = 0; g < AG; ++g)
+  for (int g = 0; g < GN; ++g)
 #pragma unroll
     for (int e = 0; e < EPL; ++e) acc[g][e] = 0.f;
-#pragma unroll
-  for (int q = 0; q < VPRE; ++q) {
-    const int j = u0 + warp + 8 * q;
-    if (j < u1g) {
-#pragma unroll
-      for (int g = 0; g < AG; ++g) {
-        const float pj = sc[(long)g * ucap + (j - u0)];
-        axpy_bf2(acc[g][0], acc[g][1], pj, vraw[q].x);
-        if (EPL == 4) axpy_bf2(acc[g][EPL - 2], acc[g][EPL - 1], pj, vraw[q].y);
-      }
-    }
-  }
-  if (PARTS && owner && warp == 0) {  // the new value row comes from shared memory
-#pragma unroll
-    for (int g = 0; g < AG; ++g) {
-      const float pj = sc[(long)g * ucap + (nkeys - 1 - u0)];
-#pragma unroll
-      for (int e = 0; e < EPL; ++e) acc[g][e] = fmaf(pj, vn[lane * EPL + e], acc[g][e]);
-    }
-  }
+  // (the rows of the next trip are on their way while those of this one are multiplied)
 #pragma unroll 1
-  for (int j0 = u0 + warp + 8 * VPRE; j0 < u1g; j0 += 32) {  // 4 keys per trip, loads first
-    uint2 vw[4];
+  for (int j0 = u0 + warp; j0 < u1g; j0 += 8 * VB) {
+    uint2 vw[VB];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int j = j0 + 8 * q;
-      vw[q] = make_uint2(0, 0);
-      if (j < u1g) {
-        const bf16* vr = vb + (long)j * HD + lane * EPL;
-        if (EPL == 4) vw[q] = __ldcg(reinterpret_cast<const uint2*>(vr));
-        else vw[q].x = __ldcg(reinterpret_cast<const uint32_t*>(vr));
-      }
-    }
+    for (int q = 0; q < VB; ++q) vw[q] = vraw[q];
+    if (j0 + 8 * VB < u1g) load_v(j0 + 8 * VB);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < VB; ++q) {
       const int j = j0 + 8 * q;
       if (j < u1g) {
 #pragma unroll
-        for (int g = 0; g < AG; ++g) {
+        for (int g = 0; g < GN; ++g) {
           const float pj = sc[(long)g * ucap + (j - u0)];
           axpy_bf2(acc[g][0], acc[g][1], pj, vw[q].x);
           if (EPL == 4) axpy_bf2(acc[g][EPL - 2], acc[g][EPL - 1], pj, vw[q].y);
@@ -577,8 +562,16 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
       }
     }
   }
+  if (PARTS && owner && warp == 0) {  // the new value row comes from shared memory
 #pragma unroll
-  for (int g = 0; g < AG; ++g)
+    for (int g = 0; g < GN; ++g) {
+      const float pj = sc[(long)g * ucap + (nkeys - 1 - u0)];
+#pragma unroll
+      for (int e = 0; e < EPL; ++e) acc[g][e] = fmaf(pj, vn[lane * EPL + e], acc[g][e]);
+    }
+  }
+#pragma unroll
+  for (int g = 0; g < GN; ++g)
 #pragma unroll
     for (int e = 0; e < EPL; ++e) red[((long)warp * AG + g) * HD + lane * EPL + e] = acc[g][e];
   ATT_STAMP();  // PV done
