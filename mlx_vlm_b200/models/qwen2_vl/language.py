@@ -216,37 +216,44 @@ class LanguageModel:
         pools = {id(c[0]._pool) for c in caches}
         if len(pools) != 1 or any(int(c[0].offset) != 0 for c in caches):
             raise ValueError("prefill_rows: fresh prompts in rows of one pool only")
-        lens, pos, embs, deltas = [], [], [], []
+        ids_all, embs, lens = [], [], []
         for g in range(n):
             ids = _np(ids_list[g])
             if ids.ndim == 1:
                 ids = ids[None]
-            L = ids.shape[1]
+            e = embeds_list[g].reshape(-1, embeds_list[g].shape[-1])
+            assert e.shape[0] == ids.shape[1] and e.dtype == torch.bfloat16 and e.is_cuda
+            ids_all.append(ids)
+            embs.append(e)
+            lens.append(ids.shape[1])
+        # The embeddings are gathered on the device while the host works out the positions (the device has nothing else to do
+        # then; one fill for all paddings and one array for all positions: eight prompts of 608 tokens 4073 -> 3970 us a call).
+        with torch.cuda.stream(eng.stream):
+            parts, zeros = [], None
+            for e in embs:
+                parts.append(e)
+                pad = (-e.shape[0]) % 8            # sequences start at multiples of 8 tokens in the concatenated batch
+                if pad:
+                    zeros = torch.zeros(7, e.shape[1], dtype=e.dtype, device=e.device) if zeros is None else zeros
+                    parts.append(zeros[:pad])
+            emb = torch.cat(parts, 0) if len(parts) > 1 else parts[0].contiguous()
+        pos, deltas, at = np.zeros((3, emb.shape[0]), dtype=np.int32), [], 0
+        for g, ids in enumerate(ids_all):
             self._rope_deltas, self._position_ids = None, None
             p3, d0 = self.resolve_position_ids(
                 ids, 0, None if position_ids_list is None else position_ids_list[g], None, None, None,
                 None if rope_deltas_list is None else rope_deltas_list[g])
             if rope_deltas_list is not None and rope_deltas_list[g] is not None:
                 d0 = int(np.asarray(rope_deltas_list[g]).reshape(-1)[0])
-            e = embeds_list[g].reshape(-1, embeds_list[g].shape[-1])
-            assert e.shape[0] == L and e.dtype == torch.bfloat16 and e.is_cuda
-            pad = (-L) % 8            # sequences start at multiples of 8 tokens in the concatenated batch
-            p3 = np.asarray(p3)[:, 0, :].astype(np.int32)
-            lens.append(L)
-            pos.append(np.ascontiguousarray(np.pad(p3, ((0, 0), (0, pad)))))
-            embs.append((e, pad))
+            p3 = np.asarray(p3)[:, 0, :]
+            assert p3.shape == (3, lens[g])
+            pos[:, at:at + lens[g]] = p3
+            at += (lens[g] + 7) // 8 * 8
             deltas.append(d0)
         need = max(max(lens), reserve_tokens)
         self._bind(caches[0], need)
-        pos3 = torch.from_numpy(np.ascontiguousarray(np.concatenate(pos, axis=1)))
         with torch.cuda.stream(eng.stream):
-            pos3 = pos3.to(eng.device)
-            parts = []
-            for e, pad in embs:
-                parts.append(e)
-                if pad:
-                    parts.append(torch.zeros(pad, e.shape[1], dtype=e.dtype, device=e.device))
-            emb = torch.cat(parts, 0) if len(parts) > 1 else parts[0].contiguous()
+            pos3 = torch.from_numpy(pos).to(eng.device)
         start = eng.tokens_launched
         eng.prefill_batch(emb, pos3, lens, [int(c[0]._row or 0) for c in caches])
         for g in range(n):
