@@ -920,9 +920,11 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
 // the NEXT block applies to h (RMSNorm / LayerNorm with the oracle's rounding points).  One CTA
 // per token row; the split-K partials are added in split order (deterministic).
 // ---------------------------------------------------------------------------------------------
-// <256 threads, 8 vectors> for sequences (one CTA per row, many rows) and <1024, 2> for the few rows of a batched
-// decode step: there the kernel is a chain of L2 round trips, and 1024 threads issue every load of a row at once
-constexpr int FIN_N_MAX = 8192;  // N <= FIN_THREADS * 4 * FIN_MAXV in both shapes
+// <threads, vectors of 4 a thread> as the row's width and the number of rows ask for (finish_rows): a chain of L2 round trips, so a
+// thread has one vector where it can, the loads of a row go out together, and those of the weights ahead of the wait for the product.
+// Against <256, 8> for all sequences, weights behind the sums: one picture through four vision blocks (2 - 7 partials of 1280 a row)
+// 255 -> 251 us, 272 tokens through four 2B layers 227 -> 224; the few rows of a decode step (1024 threads) take the same time.
+constexpr int FIN_N_MAX = 8192;  // N <= FIN_THREADS * 4 * FIN_MAXV in the widest shapes
 
 template <int FIN_THREADS>
 __device__ __forceinline__ float fin_block_sum(float v, float* red) {
@@ -945,9 +947,18 @@ finish_rows_kernel(const float* __restrict__ P, int S, const bf16* __restrict__ 
                    bf16* __restrict__ xn, long ldx, int T, int N) {
   __shared__ float red[FIN_THREADS / 32];
   w_pdl_launch();
-  w_pdl_wait();
   const int t = blockIdx.x;
   const int nv = N >> 2;
+  if (FIN_THREADS == 1024) w_pdl_wait();   // (a step's blocks wait long for their product, beside its weight stream)
+  uint2 wb[FIN_MAXV], wn[FIN_MAXV], wnb[FIN_MAXV];   // bias, norm weight and bias: of no kernel before this one
+#pragma unroll
+  for (int u = 0; u < FIN_MAXV; ++u) {
+    const int c = threadIdx.x + FIN_THREADS * u;
+    wb[u] = bias && c < nv ? __ldg(reinterpret_cast<const uint2*>(bias + c * 4)) : make_uint2(0, 0);
+    wn[u] = norm_kind != B200_NORM_NONE && nw && c < nv ? __ldg(reinterpret_cast<const uint2*>(nw + c * 4)) : make_uint2(0, 0);
+    wnb[u] = norm_kind != B200_NORM_NONE && norm_kind != B200_NORM_RMS && nb && c < nv ? __ldg(reinterpret_cast<const uint2*>(nb + c * 4)) : make_uint2(0, 0);
+  }
+  if (FIN_THREADS < 1024) w_pdl_wait();
   float4 h[FIN_MAXV];
   float s1 = 0.f, s2 = 0.f;
 #pragma unroll
@@ -956,7 +967,9 @@ finish_rows_kernel(const float* __restrict__ P, int S, const bf16* __restrict__ 
     h[u] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c < nv) {
       // the split-K partials of this chunk: up to 8 loads in flight, added in split order
+      const uint2 rv = resid ? *reinterpret_cast<const uint2*>(resid + (long)t * ldr + c * 4) : make_uint2(0, 0);
       float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
       for (int s0 = 0; s0 < S; s0 += 8) {
         float4 v[8];
 #pragma unroll
@@ -970,13 +983,13 @@ finish_rows_kernel(const float* __restrict__ P, int S, const bf16* __restrict__ 
       }
       if (bias) {
         float bb[4];
-        unpack4(*reinterpret_cast<const uint2*>(bias + c * 4), bb);
+        unpack4(wb[u], bb);
         a.x += bb[0]; a.y += bb[1]; a.z += bb[2]; a.w += bb[3];
       }
       a.x = rbf(a.x); a.y = rbf(a.y); a.z = rbf(a.z); a.w = rbf(a.w);
       if (resid) {
         float rr[4];
-        unpack4(*reinterpret_cast<const uint2*>(resid + (long)t * ldr + c * 4), rr);
+        unpack4(rv, rr);
         a.x = rbf(rr[0] + a.x); a.y = rbf(rr[1] + a.y); a.z = rbf(rr[2] + a.z); a.w = rbf(rr[3] + a.w);
       }
       h[u] = a;
@@ -995,7 +1008,7 @@ finish_rows_kernel(const float* __restrict__ P, int S, const bf16* __restrict__ 
       const int c = threadIdx.x + FIN_THREADS * u;
       if (c < nv) {
         float w[4];
-        unpack4(*reinterpret_cast<const uint2*>(nw + c * 4), w);
+        unpack4(wn[u], w);
         const float4 a = h[u];
         *reinterpret_cast<uint2*>(xn + (long)t * ldx + c * 4) =
             make_uint2(pack2(rbf(rbf(a.x * rs) * w[0]), rbf(rbf(a.y * rs) * w[1])),
@@ -1027,13 +1040,13 @@ finish_rows_kernel(const float* __restrict__ P, int S, const bf16* __restrict__ 
                     rbf((a.w - mu) * rstd)};
       if (nw) {
         float w[4];
-        unpack4(*reinterpret_cast<const uint2*>(nw + c * 4), w);
+        unpack4(wn[u], w);
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[e] = rbf(o[e] * w[e]);
       }
       if (nb) {
         float b[4];
-        unpack4(*reinterpret_cast<const uint2*>(nb + c * 4), b);
+        unpack4(wnb[u], b);
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[e] = rbf(o[e] + b[e]);
       }
@@ -1628,23 +1641,21 @@ int finish_rows(const float* P, int S, const void* bias, const void* resid, long
   B200_REQUIRE((ldr % 4) == 0 && (ldh % 4) == 0 && (ldx % 4) == 0, "finish_rows: strides must be multiples of 4");
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(T);
-  const bool few_rows = T <= 32;
-  lc.blockDim = dim3(few_rows ? 1024 : 256);
   lc.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   lc.attrs = at;
   lc.numAttrs = g_wt_pdl ? 1 : 0;
-  if (few_rows) {
-    B200_CUDA(cudaLaunchKernelEx(&lc, finish_rows_kernel<1024, 2>, P, S, (const bf16*)bias, (const bf16*)resid, ldr,
-                                 (bf16*)h_out, ldh, norm_kind, (const bf16*)nw, (const bf16*)nb, eps,
-                                 (bf16*)xn, ldx, T, N));
-  } else {
-    B200_CUDA(cudaLaunchKernelEx(&lc, finish_rows_kernel<256, 8>, P, S, (const bf16*)bias, (const bf16*)resid, ldr,
-                                 (bf16*)h_out, ldh, norm_kind, (const bf16*)nw, (const bf16*)nb, eps,
-                                 (bf16*)xn, ldx, T, N));
-  }
+  auto go = [&](auto kern, int threads) {
+    lc.blockDim = dim3(threads);
+    return cudaLaunchKernelEx(&lc, kern, P, S, (const bf16*)bias, (const bf16*)resid, ldr, (bf16*)h_out, ldh, norm_kind, (const bf16*)nw,
+                              (const bf16*)nb, eps, (bf16*)xn, ldx, T, N);
+  };
+  if (T <= 32) B200_CUDA(N <= 4096 ? go(finish_rows_kernel<1024, 1>, 1024) : go(finish_rows_kernel<1024, 2>, 1024));
+  else if (N <= 1536) B200_CUDA(go(finish_rows_kernel<384, 1>, 384));
+  else if (N <= 4096) B200_CUDA(go(finish_rows_kernel<512, 2>, 512));
+  else B200_CUDA(go(finish_rows_kernel<512, 4>, 512));
   return B200_OK;
 }
 

@@ -170,3 +170,31 @@ def test_vision_qkv_post(lib):
     cmp_bf16(d[:, :2], want[:, :2], "qkv_post q (scaled), k", max_mismatch=0.01)
     assert torch.equal(d[:, 2].cpu().float(), qkv[:, 2]), "V must stay untouched"
     assert torch.equal(vt[:, :, :N].cpu().float(), qkv[:, 2].permute(1, 2, 0)), "V^T must be an exact transpose"
+
+
+@pytest.mark.parametrize("T,N", [(33, 4), (40, 1536), (33, 1540), (64, 4096), (35, 4100), (33, 8192), (32, 4096), (2, 4100), (32, 8192), (1, 8)])
+@pytest.mark.parametrize("kind", [0, 1, 2])
+def test_finish_rows_shapes(lib, T, N, kind):
+    """the widths and row counts at which finish_rows changes its threads and vectors; bound: every rounding of the oracle's chain is
+    repeated, the fp32 sums of the norm differ in their order (2^-20), so a bf16 rounding may fall the other way: 2^-8 of an element"""
+    from mlx_vlm_b200 import _native as Nn
+    g = torch.Generator(device="cuda").manual_seed(T * N + kind)
+    S = 3
+    part = torch.randn(S, T, N, generator=g, device="cuda")
+    bias, resid, nw, nb = (torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16) for s in ((N,), (T, N), (N,), (N,)))
+    h, xn = torch.zeros(T, N, dtype=torch.bfloat16, device="cuda"), torch.zeros(T, N, dtype=torch.bfloat16, device="cuda")
+    Nn.check(lib.b200_finish_rows(part.data_ptr(), S, bias.data_ptr(), resid.data_ptr(), N, h.data_ptr(), N, kind, nw.data_ptr(), nb.data_ptr(),
+                                  1e-5, xn.data_ptr(), N, T, N, 0), "finish_rows")
+    torch.cuda.synchronize()
+    r = lambda t: t.to(torch.bfloat16).float()
+    want = r(resid.float() + r(part[0] + part[1] + part[2] + bias.float()))
+    assert torch.equal(h.float(), want)
+    if kind == 1:
+        y = r(r(want * torch.rsqrt((want * want).mean(-1, keepdim=True) + 1e-5)) * nw.float())
+    elif kind == 2:
+        d = want - want.mean(-1, keepdim=True)
+        y = r(r(r(d * torch.rsqrt((d * d).mean(-1, keepdim=True) + 1e-5)) * nw.float()) + nb.float())
+    else:
+        assert bool((xn == 0).all())
+        return
+    assert float((xn.float() - y).norm() / y.norm()) <= 2.0 ** -8
