@@ -9,18 +9,20 @@
 // 1024 of 72 (a register-tiled FMA kernel: 5.2e-7, 6.5e-7).
 //
 // One CTA = 128 query rows of one head of one segment, tiles of 64 keys:
-//   warps 8..10  load the fp32 keys and values of a tile, split them, store the parts as no-swizzle K-major core matrices (8
+//   warps 8..14  load the fp32 keys and values of a tile, split them, store the parts as no-swizzle K-major core matrices (8
 //                rows x 16 bytes).  A block of 8 columns is 16 bytes longer than its rows need, so that the eight lanes of a
 //                store that share a row (K: a key) or a column (V: 8 keys) hit different banks.  V is transposed on the way
 //                (a thread holds 8 keys x 4 dims): as an MN-major operand it took the tensor core 138 cycles per
 //                128 x 64 x 16 product instead of about 40.
-//   warp 11      issues S[g] = Q.K^T and O[g] = P[g].V; P is an operand in tensor memory, no shared memory is touched by it
+//   warp 15      issues S[g] = Q.K^T and O[g] = P[g].V; P is an operand in tensor memory, no shared memory is touched by it
 //   warps 0..7   two groups of 128 threads, thread = query row: group g takes the tiles j = g mod 2 with its own score, P and
 //                O buffers in tensor memory and its own running maximum, sum and output, so the tensor core works on one
 //                group's tile while the other group is at its exponentials.  At the end the groups merge through shared memory.
-// Bound by the issuing thread's products and by the loading warps alike (about 2700 of 3700 cycles a tile are products: S at
-// 52 cycles each, which is what its two operands take to leave shared memory, P.V at 56).  Per block, fp32 FMA kernel ->
-// this one: CLIP-L, 8 pictures (16 heads of 64, 577 tokens) 417 -> 148 us, SigLIP, 4 of 1024 tokens (16 of 72) 790 -> 240,
+// With three loading warps they were what bounds it (without their splitting 319 -> 260 us for two blocks of the first of these, with
+// a sixth of the products 264): seven of them, the registers shared out between the roles (setmaxnreg), took CLIP-L, 8 pictures (16
+// heads of 64, 577 tokens) from 159 to 136 us a block, SigLIP, 4 of 1024 tokens (16 of 72) from 235 to 183, 64 latents on 1088 keys
+// of 96 from 73 to 54.  What is left: products (S at 52 cycles each, which is what its two operands take to leave shared memory, P.V
+// at 56) and the softmax between them.  Per block, fp32 FMA kernel -> the form with three loading warps: CLIP-L 417 -> 148 us, SigLIP 790 -> 240,
 // 64 latents on 1088 keys of 96 160 -> 75, one frame of 1564 (16 of 80) 583 -> 170, 25 windows of 64 41 -> 33; windows of 32
 // tokens cost the same (56, 58).
 #include <type_traits>
@@ -33,8 +35,12 @@ namespace b200 {
 namespace {
 
 constexpr int TC_ROWS = 128, TC_KEYS = 64;
-constexpr int TC_LOADERS = 96;
-constexpr int TC_THREADS = 256 + TC_LOADERS + 32;   // 8 softmax, 3 loading and 1 MMA warp: three warps and 168 registers per scheduler
+constexpr int TC_LOADERS = 224;
+constexpr int TC_THREADS = 256 + TC_LOADERS + 32;   // 8 softmax, 7 loading and 1 MMA warp
+constexpr int TC_MMA = TC_THREADS / 32 - 1;         // the last warp
+// registers of a softmax thread and of the others: together what the block is launched with, 512 x 128
+constexpr int TC_REGS_SOFTMAX = 152, TC_REGS_OTHER = 104;
+static_assert(256 * TC_REGS_SOFTMAX + (TC_THREADS - 256) * TC_REGS_OTHER <= TC_THREADS * 128, "a larger share would be waited for without end");
 constexpr int TC_QB = TC_ROWS * 16 + 16, TC_KB = TC_KEYS * 16 + 16;   // bytes of a block of 8 dims
 constexpr int TC_P0 = 128, TC_O0 = 320, TC_GB = 96;   // TMEM columns: S 2 x 64 | P 2 x (3 x 32) | O 2 x 96
 
@@ -271,7 +277,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 11) {
+  if (warp == TC_MMA) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(t_u32(&tmem_slot)), "r"(512u)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -282,8 +288,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
   const uint32_t tmem = tmem_slot;
   // (the next kernel may start from here on, not before: it may ask for tensor memory too, and would hold what this one still needs)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-
-  if (warp == 11) {
+  if (warp == TC_MMA) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TC_REGS_OTHER));
     if (lane == 0) {  // ===== MMA issuer =====
       // D = f32, A = B = bf16, both K-major, M = 128; N = keys of the tile / dims
       constexpr uint32_t ID = (1u << 4) | (1u << 7) | (1u << 10) | (8u << 24);
@@ -343,6 +349,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
       }
     }
   } else if (warp >= 8) {  // ===== keys and values of a tile =====
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TC_REGS_OTHER));
     const int t = tid - 256;
     const float* kb = p.k + k_first * p.k_ts + (long)kvh * p.k_hs;
     const float* vb = p.v + k_first * p.v_ts + (long)kvh * p.v_hs;
@@ -375,6 +382,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
       t_arrive(&bars.v_full[s]);
     }
   } else {  // ===== softmax: thread = query row; group g = tiles j = g mod 2 =====
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TC_REGS_SOFTMAX));
     for (int i0 = tid; i0 < TC_ROWS * HDP / 8; i0 += 4 * 256) {
       float4 a[4], b[4];
       load_items<HDP, TC_ROWS, 4, 256, true>(a, b, i0, p.q + (q_first + q0) * p.q_ts + (long)h * p.q_hs, p.q_ts, min(TC_ROWS, Lq - q0),
@@ -565,7 +573,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
   t_fence_before();
   __syncthreads();
   if (tid == 0 && failed) g_f32_wait_failed = B200_WAIT_TOWER;
-  if (warp == 11) {
+  if (warp == TC_MMA) {
     t_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
