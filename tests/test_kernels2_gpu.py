@@ -198,3 +198,27 @@ def test_finish_rows_shapes(lib, T, N, kind):
         assert bool((xn == 0).all())
         return
     assert float((xn.float() - y).norm() / y.norm()) <= 2.0 ** -8
+
+
+_CHILD_TOWER = """
+import sys, torch, numpy as np
+sys.path.insert(0, {root!r})
+import perf.cases as C
+case = {{"kind": "vit", "grids": {grids!r}, "depth": 1}}
+got = C.run(C.prepare(case, 3)).double()
+want = C.exact(case, 3)
+e = float((got - want).norm() / want.norm())
+print(e)
+assert e <= 0.012, e     # 0.009 measured for the roundings of these layers (one block: less), as before this kernel
+"""
+
+
+@pytest.mark.parametrize("grids", ["1x2x2", "1x6x10", "1x8x66", "2x4x14,1x18x34", "1x46x46,1x20x26"])
+def test_tower_rotary_over_token_tiles(grids):
+    """the tower's rotary kernel where token tiles end and where a CTA takes one head, several, an odd number: a block against float64"""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _CHILD_TOWER.format(root=root, grids=grids)], capture_output=True, text=True, timeout=300, cwd=root)
+    assert r.returncode == 0, r.stdout + r.stderr
