@@ -288,98 +288,99 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
   const uint32_t tmem = tmem_slot;
   // (the next kernel may start from here on, not before: it may ask for tensor memory too, and would hold what this one still needs)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (warp == TC_MMA) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TC_REGS_OTHER));
-    if (lane == 0) {  // ===== MMA issuer =====
-      // D = f32, A = B = bf16, both K-major, M = 128; N = keys of the tile / dims
-      constexpr uint32_t ID = (1u << 4) | (1u << 7) | (1u << 10) | (8u << 24);
-      constexpr uint32_t ID_O = ID | ((uint32_t)(HDP >> 3) << 17);
-      // (part of A, part of B), the smallest product first; 0 = h, 1 = m, 2 = l
-      constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
-      constexpr int KS = HDP / 16, VL = HDP * 16 + 16;
-      const uint32_t q_lo = t_desc(t_u32(Qs), TC_QB), k_lo = t_desc(t_u32(Ks), TC_KB), v_lo = t_desc(t_u32(Vs), VL);
-      bool dead = false;
-      auto keys16 = [&](int j) { return min(TC_KEYS, (S - j * TC_KEYS + 15) & ~15); };
-      auto issue_s = [&](int j) {
-        const int s = j & 1;
-        mbar_wait_issuer(&bars.k_full[s], (j >> 1) & 1, dead);
-        t_fence_after();
-        const uint32_t idesc = ID | ((uint32_t)(keys16(j) >> 3) << 17), d = tmem + (uint32_t)s * TC_KEYS;
-        const uint32_t ka = k_lo + s * (3 * KP >> 4);
-        t_mma_ss<false>(d, q_lo + (PA[0] * QP >> 4), ka + (PB[0] * KP >> 4), idesc);
+  if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TC_REGS_OTHER));   // (one instruction for both roles: a warpgroup executes it together)
+    if (warp == TC_MMA) {
+      if (lane == 0) {  // ===== MMA issuer =====
+        // D = f32, A = B = bf16, both K-major, M = 128; N = keys of the tile / dims
+        constexpr uint32_t ID = (1u << 4) | (1u << 7) | (1u << 10) | (8u << 24);
+        constexpr uint32_t ID_O = ID | ((uint32_t)(HDP >> 3) << 17);
+        // (part of A, part of B), the smallest product first; 0 = h, 1 = m, 2 = l
+        constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
+        constexpr int KS = HDP / 16, VL = HDP * 16 + 16;
+        const uint32_t q_lo = t_desc(t_u32(Qs), TC_QB), k_lo = t_desc(t_u32(Ks), TC_KB), v_lo = t_desc(t_u32(Vs), VL);
+        bool dead = false;
+        auto keys16 = [&](int j) { return min(TC_KEYS, (S - j * TC_KEYS + 15) & ~15); };
+        auto issue_s = [&](int j) {
+          const int s = j & 1;
+          mbar_wait_issuer(&bars.k_full[s], (j >> 1) & 1, dead);
+          t_fence_after();
+          const uint32_t idesc = ID | ((uint32_t)(keys16(j) >> 3) << 17), d = tmem + (uint32_t)s * TC_KEYS;
+          const uint32_t ka = k_lo + s * (3 * KP >> 4);
+          t_mma_ss<false>(d, q_lo + (PA[0] * QP >> 4), ka + (PB[0] * KP >> 4), idesc);
 #pragma unroll
-        for (int i = 1; i < 6 * KS; ++i) {
-          const int t = i / KS, ks = i % KS;
-          t_mma_ss<true>(d, q_lo + ((PA[t] * QP + ks * 2 * TC_QB) >> 4), ka + ((PB[t] * KP + ks * 2 * TC_KB) >> 4), idesc);
-        }
-        t_commit(dead ? &bars.dropped : &bars.k_empty[s]);
-        t_commit(dead ? &bars.dropped : &bars.s_full[s]);
-      };
-      mbar_wait_issuer(&bars.q_full, 0, dead);
-      issue_s(0);
-      if (n_tiles > 1) issue_s(1);
-      for (int j = 0; j < n_tiles; ++j) {
-        const int s = j & 1;
-        mbar_wait_issuer(&bars.p_full[s], (j >> 1) & 1, dead);
-        mbar_wait_issuer(&bars.v_full[s], (j >> 1) & 1, dead);
-        t_fence_after();
-        const uint32_t d = tmem + TC_O0 + s * TC_GB, pa = tmem + TC_P0 + s * TC_GB, va = v_lo + s * (3 * VP >> 4);
-        t_mma_ts<false>(d, pa + PA[0] * 32, va + (PB[0] * VP >> 4), ID_O);
-        if (S - j * TC_KEYS > 48) {
-#pragma unroll
-          for (int i = 1; i < 24; ++i) {
-            const int t = i >> 2, ks = i & 3;
-            t_mma_ts<true>(d, pa + PA[t] * 32 + ks * 8, va + ((PB[t] * VP + ks * 2 * VL) >> 4), ID_O);
+          for (int i = 1; i < 6 * KS; ++i) {
+            const int t = i / KS, ks = i % KS;
+            t_mma_ss<true>(d, q_lo + ((PA[t] * QP + ks * 2 * TC_QB) >> 4), ka + ((PB[t] * KP + ks * 2 * TC_KB) >> 4), idesc);
           }
-        } else {   // groups of 16 keys that lie wholly behind the last key are left out
-          const int steps = keys16(j) >> 4;
+          t_commit(dead ? &bars.dropped : &bars.k_empty[s]);
+          t_commit(dead ? &bars.dropped : &bars.s_full[s]);
+        };
+        mbar_wait_issuer(&bars.q_full, 0, dead);
+        issue_s(0);
+        if (n_tiles > 1) issue_s(1);
+        for (int j = 0; j < n_tiles; ++j) {
+          const int s = j & 1;
+          mbar_wait_issuer(&bars.p_full[s], (j >> 1) & 1, dead);
+          mbar_wait_issuer(&bars.v_full[s], (j >> 1) & 1, dead);
+          t_fence_after();
+          const uint32_t d = tmem + TC_O0 + s * TC_GB, pa = tmem + TC_P0 + s * TC_GB, va = v_lo + s * (3 * VP >> 4);
+          t_mma_ts<false>(d, pa + PA[0] * 32, va + (PB[0] * VP >> 4), ID_O);
+          if (S - j * TC_KEYS > 48) {
 #pragma unroll
-          for (int t = 0; t < 6; ++t)
-            for (int ks = t == 0 ? 1 : 0; ks < steps; ++ks)
-              t_mma_ts<true>(d, pa + PA[t] * 32 + ks * 8, va + ((PB[t] * VP) >> 4) + ks * (2 * VL >> 4), ID_O);
+            for (int i = 1; i < 24; ++i) {
+              const int t = i >> 2, ks = i & 3;
+              t_mma_ts<true>(d, pa + PA[t] * 32 + ks * 8, va + ((PB[t] * VP + ks * 2 * VL) >> 4), ID_O);
+            }
+          } else {   // groups of 16 keys that lie wholly behind the last key are left out
+            const int steps = keys16(j) >> 4;
+#pragma unroll
+            for (int t = 0; t < 6; ++t)
+              for (int ks = t == 0 ? 1 : 0; ks < steps; ++ks)
+                t_mma_ts<true>(d, pa + PA[t] * 32 + ks * 8, va + ((PB[t] * VP) >> 4) + ks * (2 * VL >> 4), ID_O);
+          }
+          t_commit(dead ? &bars.dropped : &bars.v_empty[s]);
+          t_commit(dead ? &bars.dropped : &bars.o_full[s]);
+          if (j + 2 < n_tiles) issue_s(j + 2);   // (the group has read S of tile j: it has stored its P)
         }
-        t_commit(dead ? &bars.dropped : &bars.v_empty[s]);
-        t_commit(dead ? &bars.dropped : &bars.o_full[s]);
-        if (j + 2 < n_tiles) issue_s(j + 2);   // (the group has read S of tile j: it has stored its P)
+        if (dead) {   // no product is left in flight; the threads that wait for what was dropped give up as well
+          *static_cast<volatile int*>(&failed) = 1;
+          t_commit(&bars.drained);
+          mbar_drain(&bars.drained, 0);
+        }
       }
-      if (dead) {   // no product is left in flight; the threads that wait for what was dropped give up as well
-        *static_cast<volatile int*>(&failed) = 1;
-        t_commit(&bars.drained);
-        mbar_drain(&bars.drained, 0);
-      }
-    }
-  } else if (warp >= 8) {  // ===== keys and values of a tile =====
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TC_REGS_OTHER));
-    const int t = tid - 256;
-    const float* kb = p.k + k_first * p.k_ts + (long)kvh * p.k_hs;
-    const float* vb = p.v + k_first * p.v_ts + (long)kvh * p.v_hs;
-    constexpr int U = (TC_KEYS * HDP / 8 + TC_LOADERS - 1) / TC_LOADERS;
-    constexpr int VU = (HDP / 16 + TC_LOADERS / 32 - 1) / (TC_LOADERS / 32);   // blocks of 16 dims per warp
-    const int wv = warp - 8;
-    float4 ka[U], kc[U], x[VU][8];   // the loads of one operand are in flight while the other is split
-    load_items<HDP, TC_KEYS, U, TC_LOADERS, false>(ka, kc, t, kb, p.k_ts, min(TC_KEYS, S), p.hd);
-    for (int j = 0; j < n_tiles; ++j) {
-      const int s = j & 1, rows = min(TC_KEYS, S - j * TC_KEYS);
-      const uint32_t free_parity = ((j >> 1) & 1) ^ 1;
+    } else {  // ===== keys and values of a tile =====
+      const int t = tid - 256;
+      const float* kb = p.k + k_first * p.k_ts + (long)kvh * p.k_hs;
+      const float* vb = p.v + k_first * p.v_ts + (long)kvh * p.v_hs;
+      constexpr int U = (TC_KEYS * HDP / 8 + TC_LOADERS - 1) / TC_LOADERS;
+      constexpr int VU = (HDP / 16 + TC_LOADERS / 32 - 1) / (TC_LOADERS / 32);   // blocks of 16 dims per warp
+      const int wv = warp - 8;
+      float4 ka[U], kc[U], x[VU][8];   // the loads of one operand are in flight while the other is split
+      load_items<HDP, TC_KEYS, U, TC_LOADERS, false>(ka, kc, t, kb, p.k_ts, min(TC_KEYS, S), p.hd);
+      for (int j = 0; j < n_tiles; ++j) {
+        const int s = j & 1, rows = min(TC_KEYS, S - j * TC_KEYS);
+        const uint32_t free_parity = ((j >> 1) & 1) ^ 1;
 #pragma unroll
-      for (int u = 0; u < VU; ++u)
-        if ((wv + u * (TC_LOADERS / 32)) * 16 < HDP) load_values(x[u], vb + (long)j * TC_KEYS * p.v_ts, p.v_ts, rows, p.hd, (wv + u * (TC_LOADERS / 32)) * 16, lane);
-      if (p.flags & 1) break;   // (nothing is loaded: every wait for it runs out)
-      if (!mbar_wait(&bars.k_empty[s], free_parity, &failed)) break;
-      store_items<HDP, TC_KEYS, U, TC_LOADERS>(Ks + s * 3 * KP, KP, ka, kc, t, 1.f);
-      t_fence_async();
-      t_arrive(&bars.k_full[s]);
-      if (j + 1 < n_tiles)
-        load_items<HDP, TC_KEYS, U, TC_LOADERS, false>(ka, kc, t, kb + (long)(j + 1) * TC_KEYS * p.k_ts, p.k_ts,
-                                                min(TC_KEYS, S - (j + 1) * TC_KEYS), p.hd);
-      if (!mbar_wait(&bars.v_empty[s], free_parity, &failed)) break;
+        for (int u = 0; u < VU; ++u)
+          if ((wv + u * (TC_LOADERS / 32)) * 16 < HDP) load_values(x[u], vb + (long)j * TC_KEYS * p.v_ts, p.v_ts, rows, p.hd, (wv + u * (TC_LOADERS / 32)) * 16, lane);
+        if (p.flags & 1) break;   // (nothing is loaded: every wait for it runs out)
+        if (!mbar_wait(&bars.k_empty[s], free_parity, &failed)) break;
+        store_items<HDP, TC_KEYS, U, TC_LOADERS>(Ks + s * 3 * KP, KP, ka, kc, t, 1.f);
+        t_fence_async();
+        t_arrive(&bars.k_full[s]);
+        if (j + 1 < n_tiles)
+          load_items<HDP, TC_KEYS, U, TC_LOADERS, false>(ka, kc, t, kb + (long)(j + 1) * TC_KEYS * p.k_ts, p.k_ts,
+                                                  min(TC_KEYS, S - (j + 1) * TC_KEYS), p.hd);
+        if (!mbar_wait(&bars.v_empty[s], free_parity, &failed)) break;
 #pragma unroll
-      for (int u = 0; u < VU; ++u) {
-        const int dim = (wv + u * (TC_LOADERS / 32)) * 16;
-        if (dim < HDP) store_values<HDP>(Vs + s * 3 * VP, VP, x[u], dim, lane);
+        for (int u = 0; u < VU; ++u) {
+          const int dim = (wv + u * (TC_LOADERS / 32)) * 16;
+          if (dim < HDP) store_values<HDP>(Vs + s * 3 * VP, VP, x[u], dim, lane);
+        }
+        t_fence_async();
+        t_arrive(&bars.v_full[s]);
       }
-      t_fence_async();
-      t_arrive(&bars.v_full[s]);
     }
   } else {  // ===== softmax: thread = query row; group g = tiles j = g mod 2 =====
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TC_REGS_SOFTMAX));
