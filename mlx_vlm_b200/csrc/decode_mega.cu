@@ -424,8 +424,8 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) k_mega(const MegaP p) {
         // the qkv/attention/o_proj chain is latency-bound (~20 us with ~11 MB of weights):
         // use it to pull this CTA's share of the layer's MLP weights (82 MB chip-wide,
         // fits the 126 MB L2) into L2, so the ring later refills at L2 speed.
-        // (measured: no gain — gate/up is consumer-bound at 8 warps — and a
-        // straggler CTA in the down phase; kept behind a switch)
+        // (measured: no gain while gate / up was bound by its eight warps, a step of
+        // the 2B model 1090 -> 1166 us since; kept behind a switch)
         if (p.l2_prefetch == 1) {
           l2_prefetch_phase<PH_GATEUP>(p.ph[PH_GATEUP], lw.wgu, lw.wgu + (long)d.inter * d.hidden);
           l2_prefetch_phase<PH_DRES>(p.ph[PH_DRES], lw.wd, nullptr);
