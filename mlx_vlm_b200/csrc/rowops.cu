@@ -506,6 +506,13 @@ __global__ void vision_rope_table_kernel(const int* __restrict__ pos_hw, const f
   cs[idx] = make_float2(cosf(ang), sinf(ang));
 }
 
+// bf16 of a * c + b * d, pairs, each product and the sum rounded.  (add.rn.f32x2 of two mul.rn.f32x2 becomes one product and one FMA:
+// single values came out a bf16 unit off, which the layers behind them spread to 0.5 % of the tower's output.  The same time.)
+__device__ __forceinline__ uint32_t rot_pair(uint64_t a, uint64_t c, uint64_t b, uint64_t d) {
+  return pack2(__fadd_rn(__fmul_rn(f2_lo(a), f2_lo(c)), __fmul_rn(f2_lo(b), f2_lo(d))),
+               __fadd_rn(__fmul_rn(f2_hi(a), f2_hi(c)), __fmul_rn(f2_hi(b), f2_hi(d))));
+}
+
 // The tower's form (V is read where it lies, cos / sin come from the table): a CTA takes 32 tokens x a group of heads; thread (token,
 // chunk of 8 rotary pairs) reads its 8 cos / sin once for q and k of all of them, two heads in flight, and works on pairs.  Bound by
 // memory: 2 B read and written per element of q and k.  A head a CTA, cos / sin read for q and for k of each (as many bytes as the
@@ -547,8 +554,8 @@ vision_rope_rows_kernel(bf16* __restrict__ qkv, const float2* __restrict__ cs, i
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
           const uint64_t y1 = unpack_bf2(x1[w]), y2 = unpack_bf2(x2[w]);
-          x1[w] = pack_bf2(add2(mul2(y1, co[w]), mul2(y2, ns[w])));
-          x2[w] = pack_bf2(add2(mul2(y2, co[w]), mul2(y1, si[w])));
+          x1[w] = rot_pair(y1, co[w], y2, ns[w]);
+          x2[w] = rot_pair(y2, co[w], y1, si[w]);
           if ((i & 1) == 0) {
             x1[w] = pack_bf2(mul2(unpack_bf2(x1[w]), scale2));
             x2[w] = pack_bf2(mul2(unpack_bf2(x2[w]), scale2));

@@ -222,3 +222,26 @@ def test_tower_rotary_over_token_tiles(grids):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", _CHILD_TOWER.format(root=root, grids=grids)], capture_output=True, text=True, timeout=300, cwd=root)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("T,nh,hd", [(1, 1, 16), (31, 3, 80), (32, 16, 80), (33, 5, 64), (577, 16, 80), (130, 7, 128), (2400, 16, 96), (19000, 2, 32)])
+def test_tower_rotary_of_rows(lib, T, nh, hd):
+    """the tower's own kernel (cos / sin from a table, heads in groups of a CTA: one, two, an odd number) against the general one, which
+    test_vision_qkv_post holds to the oracle: the same roundings, so the same bits; V is left alone"""
+    from mlx_vlm_b200 import _native as Nn
+    post, table = lib._ZN4b20015vision_qkv_postEPvPKiPKfiiifS0_iP11CUstream_stPKv, lib._ZN4b20017vision_rope_tableEPKiPKfiiPvP11CUstream_st
+    post.argtypes = [C.c_void_p] * 3 + [C.c_int] * 3 + [C.c_float, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]
+    table.argtypes = [C.c_void_p] * 2 + [C.c_int] * 2 + [C.c_void_p] * 2
+    g = torch.Generator(device="cuda").manual_seed(T)
+    qkv = torch.randn(T, 3, nh, hd, generator=g, device="cuda").to(torch.bfloat16)
+    pos = torch.randint(0, 70, (T, 2), generator=g, device="cuda", dtype=torch.int32)
+    inv = (1.0 / (10000.0 ** (torch.arange(0, hd // 2, 2, dtype=torch.float32) / (hd // 2)))).cuda()
+    cs = torch.empty(T, hd // 2, 2, device="cuda")
+    a, b = qkv.clone(), qkv.clone()
+    torch.cuda.synchronize()
+    Nn.check(table(pos.data_ptr(), inv.data_ptr(), T, hd, cs.data_ptr(), 0), "table")
+    Nn.check(post(a.data_ptr(), pos.data_ptr(), inv.data_ptr(), T, nh, hd, hd ** -0.5, 0, 0, 0, cs.data_ptr()), "rows")
+    Nn.check(post(b.data_ptr(), pos.data_ptr(), inv.data_ptr(), T, nh, hd, hd ** -0.5, 0, 0, 0, 0), "general")
+    torch.cuda.synchronize()
+    assert torch.equal(a, b), float((a.double() - b.double()).abs().max())
+    assert torch.equal(a[:, 2], qkv[:, 2]) and not torch.equal(a[:, :2], qkv[:, :2])
