@@ -926,16 +926,31 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
 // 255 -> 251 us, 272 tokens through four 2B layers 227 -> 224; the few rows of a decode step (1024 threads) take the same time.
 constexpr int FIN_N_MAX = 8192;  // N <= FIN_THREADS * 4 * FIN_MAXV in the widest shapes
 
-template <int FIN_THREADS>
-__device__ __forceinline__ float fin_block_sum(float v, float* red) {
-  v = warp_sum(v);
+// Sum of a row's vectors (q[u]: vector thread + FIN_THREADS * u).  1024 threads: as they lie.  Fewer: as 256 threads of up to 8 vectors
+// each would add them, so that a row's bits do not depend on the shape: the threads from 256 on hand theirs over, ahead of the
+// barrier that `red` needs anyway.
+template <int FIN_THREADS, int FIN_MAXV>
+__device__ __forceinline__ float fin_block_sum(const float (&q)[FIN_MAXV], float* red, float (*ex)[256]) {
+  constexpr int SUMS = FIN_THREADS == 1024 ? 1024 : 256;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x >= SUMS)
+#pragma unroll
+    for (int u = 0; u < FIN_MAXV; ++u) ex[u][threadIdx.x - SUMS] = q[u];
   __syncthreads();
-  if (lane == 0) red[warp] = v;
+  if (threadIdx.x < SUMS) {
+    float v = 0.f;
+#pragma unroll
+    for (int u = 0; u < FIN_MAXV; ++u) {
+      v += q[u];
+      if (threadIdx.x + SUMS < FIN_THREADS) v += ex[u][threadIdx.x];
+    }
+    v = warp_sum(v);
+    if (lane == 0) red[warp] = v;
+  }
   __syncthreads();
   float t = 0.f;
 #pragma unroll
-  for (int w = 0; w < FIN_THREADS / 32; ++w) t += red[w];
+  for (int w = 0; w < SUMS / 32; ++w) t += red[w];
   return t;
 }
 
@@ -945,7 +960,7 @@ finish_rows_kernel(const float* __restrict__ P, int S, const bf16* __restrict__ 
                    const bf16* __restrict__ resid, long ldr, bf16* __restrict__ h_out, long ldh,
                    int norm_kind, const bf16* __restrict__ nw, const bf16* __restrict__ nb, float eps,
                    bf16* __restrict__ xn, long ldx, int T, int N) {
-  __shared__ float red[FIN_THREADS / 32];
+  __shared__ float red[FIN_THREADS / 32], ex[FIN_MAXV][256];
   w_pdl_launch();
   const int t = blockIdx.x;
   const int nv = N >> 2;
@@ -960,11 +975,12 @@ finish_rows_kernel(const float* __restrict__ P, int S, const bf16* __restrict__ 
   }
   if (FIN_THREADS < 1024) w_pdl_wait();
   float4 h[FIN_MAXV];
-  float s1 = 0.f, s2 = 0.f;
+  float s1[FIN_MAXV], s2[FIN_MAXV];   // of a vector
 #pragma unroll
   for (int u = 0; u < FIN_MAXV; ++u) {
     const int c = threadIdx.x + FIN_THREADS * u;
     h[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    s1[u] = s2[u] = 0.f;
     if (c < nv) {
       // the split-K partials of this chunk: up to 8 loads in flight, added in split order
       const uint2 rv = resid ? *reinterpret_cast<const uint2*>(resid + (long)t * ldr + c * 4) : make_uint2(0, 0);
@@ -995,13 +1011,13 @@ finish_rows_kernel(const float* __restrict__ P, int S, const bf16* __restrict__ 
       h[u] = a;
       if (h_out)
         *reinterpret_cast<uint2*>(h_out + (long)t * ldh + c * 4) = make_uint2(pack2(a.x, a.y), pack2(a.z, a.w));
-      s1 += (a.x + a.y) + (a.z + a.w);
-      s2 += (a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w);
+      s1[u] = (a.x + a.y) + (a.z + a.w);
+      s2[u] = (a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w);
     }
   }
   if (norm_kind == B200_NORM_NONE) return;
   if (norm_kind == B200_NORM_RMS) {
-    const float tot = fin_block_sum<FIN_THREADS>(s2, red);
+    const float tot = fin_block_sum<FIN_THREADS>(s2, red, ex);
     const float rs = 1.0f / sqrtf(tot / (float)N + eps);
 #pragma unroll
     for (int u = 0; u < FIN_MAXV; ++u) {
@@ -1018,18 +1034,19 @@ finish_rows_kernel(const float* __restrict__ P, int S, const bf16* __restrict__ 
     return;
   }
   // LayerNorm: fp32 mean / variance (two passes over the registers), cast, * w, + b
-  const float mu = fin_block_sum<FIN_THREADS>(s1, red) / (float)N;
-  float v = 0.f;
+  const float mu = fin_block_sum<FIN_THREADS>(s1, red, ex) / (float)N;
+  float v[FIN_MAXV];
 #pragma unroll
   for (int u = 0; u < FIN_MAXV; ++u) {
     const int c = threadIdx.x + FIN_THREADS * u;
+    v[u] = 0.f;
     if (c < nv) {
       const float4 a = h[u];
       const float d0 = a.x - mu, d1 = a.y - mu, d2 = a.z - mu, d3 = a.w - mu;
-      v += (d0 * d0 + d1 * d1) + (d2 * d2 + d3 * d3);
+      v[u] = (d0 * d0 + d1 * d1) + (d2 * d2 + d3 * d3);
     }
   }
-  const float var = fin_block_sum<FIN_THREADS>(v, red) / (float)N;
+  const float var = fin_block_sum<FIN_THREADS>(v, red, ex) / (float)N;
   const float rstd = 1.0f / sqrtf(var + eps);
 #pragma unroll
   for (int u = 0; u < FIN_MAXV; ++u) {

@@ -200,6 +200,49 @@ def test_finish_rows_shapes(lib, T, N, kind):
     assert float((xn.float() - y).norm() / y.norm()) <= 2.0 ** -8
 
 
+@pytest.mark.parametrize("T,N", [(33, 1280), (40, 1536), (33, 1540), (35, 3584), (64, 4096), (35, 4100), (33, 8192)])
+def test_finish_rows_adds_a_row_as_256_threads_would(lib, T, N):
+    """whatever shape a width takes: 256 partial sums of every 256th vector, a butterfly over 32, eight warps in turn.  Rows of large numbers
+    that cancel and ones between them: the mean is what the order of the fp32 sums leaves, and (1 - mean) / deviation of the ones shows it."""
+    from mlx_vlm_b200 import _native as Nn
+    rng = np.random.default_rng(N)
+    nv = N // 4
+    x = np.ones((T, N), np.float32)
+    for row in x:
+        at = rng.permutation(N)[:N // 4 * 2]
+        big = np.ldexp(1.0 + rng.integers(0, 128, size=N // 4) / 128.0, rng.integers(0, 45, size=N // 4)).astype(np.float32)    # bf16 values
+        row[at] = np.concatenate([big, -big])
+
+    def mean(row, threads):
+        v = row.reshape(nv, 4)
+        q = (v[:, 0] + v[:, 1]) + (v[:, 2] + v[:, 3])
+        q = np.concatenate([q, np.zeros(-nv % threads, np.float32)]).reshape(-1, threads)
+        s = np.zeros(threads, np.float32)
+        for part in q:
+            s = s + part
+        s = s.reshape(-1, 32)
+        for o in (16, 8, 4, 2, 1):
+            s = s + s[:, np.arange(32) ^ o]
+        t = np.float32(0)
+        for w in s[:, 0]:
+            t = t + w
+        return t / np.float32(N)
+
+    part = torch.from_numpy(x[None].copy()).cuda()
+    h, xn = (torch.zeros(T, N, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    Nn.check(lib.b200_finish_rows(part.data_ptr(), 1, 0, 0, 0, h.data_ptr(), N, 2, 0, 0, 0.0, xn.data_ptr(), N, T, N, 0), "finish_rows")
+    torch.cuda.synchronize()
+    got, differ = xn.double().cpu().numpy(), 0
+    for t in range(T):
+        mu, other = float(mean(x[t], 256)), float(mean(x[t], 512 if N > 1536 else 384))
+        sd = np.sqrt(((x[t].astype(np.float64) - mu) ** 2).mean())
+        want = (1.0 - mu) / sd
+        ones = got[t][x[t] == 1.0]
+        assert np.abs(ones - want).max() <= 2.0 ** -8 * abs(want), t      # a rounding to bf16
+        differ += abs(other - mu) > 2.0 ** -6 * abs(1.0 - mu)
+    assert differ >= T // 2, differ      # (the rows tell the orders apart)
+
+
 _CHILD_TOWER = """
 import sys, torch, numpy as np
 sys.path.insert(0, {root!r})
