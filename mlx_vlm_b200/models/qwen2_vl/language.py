@@ -209,7 +209,7 @@ class LanguageModel:
         batched pool: all prompts are prefilled in one pass over the weights (tokens concatenated, block-diagonal
         causal attention, every token scattered to its own row / position of the pool).  `caches[g]` are the
         per-layer row caches of prompt g (`make_cache_row`); returns the first greedy token of every prompt
-        (host ints; one device->host fetch for the whole group)."""
+        (host ints; one device->host fetch for the whole group).  The embeddings are read behind the caller's current stream."""
         eng = self._engine()
         n = len(ids_list)
         assert n == len(embeds_list) == len(caches) and n > 0
@@ -228,6 +228,8 @@ class LanguageModel:
             lens.append(ids.shape[1])
         # The embeddings are gathered on the device while the host works out the positions (the device has nothing else to do
         # then; one fill for all paddings and one array for all positions: eight prompts of 608 tokens 4073 -> 3970 us a call).
+        # The engine's stream has no order of its own with the caller's, on which the embeddings may still be on their way.
+        eng.stream.wait_stream(torch.cuda.current_stream(eng.device))
         with torch.cuda.stream(eng.stream):
             parts, zeros = [], None
             for e in embs:

@@ -314,6 +314,39 @@ def test_first_tokens_of_a_batched_prefill(n):
     assert eng.device_error() == 0
 
 
+@pytest.mark.parametrize("n,pieces", [(1, 1), (3, 1), (2, 2)])
+def test_batched_prefill_reads_embeddings_behind_the_callers_stream(n, pieces):
+    """embeddings that the caller's stream still has to write when the call is made (and, in pieces, to join): the logits are bit for
+    bit those of embeddings that lay there"""
+    c, W, model, req = _build("wide2", 10, (56, 56))
+    lm, eng = model.language_model, model.engine
+    rng = np.random.default_rng(5)
+    L = 48
+    ids = [rng.integers(0, 900, size=(1, L)) for _ in range(n)]
+    H = c.text.hidden_size
+    embs = [torch.randn(1, L, H, device="cuda").to(torch.bfloat16) for _ in range(n)]
+
+    rows = lm.make_batch_cache(n, 256)[0]
+
+    def prefill(embeds):
+        return lm.prefill_rows(ids, embeds, [lm.make_cache_row(rows.pool, b) for b in range(n)], reserve_tokens=256), _left(eng)
+
+    torch.cuda.synchronize()
+    prefill(embs)                                       # (choices are measured, buffers laid out)
+    toks, left = prefill(embs)
+    late = [torch.zeros(pieces, 2 * L // pieces, H, device="cuda", dtype=torch.bfloat16) for _ in range(n)]
+    torch.cuda.synchronize()
+    torch.cuda._sleep(100_000_000)                      # some 50 ms of the caller's stream
+    views = []
+    for e, b in zip(embs, late):
+        v = b[:, :L // pieces]
+        v.copy_(e.view(pieces, L // pieces, H))
+        views.append(v)
+    toks2, left2 = prefill(views)
+    assert toks2 == toks and all(torch.equal(a, b) for a, b in zip(left, left2))
+    assert eng.device_error() == 0
+
+
 def _left(eng):
     """(logits, log-probabilities) that the engine goes on from, on the host"""
     lg, lp = eng.snapshot("logits"), eng.logprobs_view()
