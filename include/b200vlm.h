@@ -87,7 +87,9 @@ int b200_gemm_bf16_tn(const void* A, long lda, const void* W, const void* bias,
  * B200_WT_PARTIAL: fp32 tiles partial[split][T][N] (bias / residual applied by
  * b200_finish_rows); B200_WT_SWIGLU: W = [gate; up] (N == 2*inter), C[T][inter] =
  * swiglu (mlp.py:9-15, activations.py:8-10).  cfg4 = {TN, k-blocks per stage, stages,
- * splits} or NULL / {0} for the automatic choice.  flags: debugging aids, pass 0 (2: nothing is loaded; with CTA pairs the
+ * splits} or NULL / {0} for the automatic choice.  W may be requested while the kernel ahead of the call still runs, if that one
+ * lets its successor start early, as this library's do: it must not be what that kernel writes.  X, bias and residual may be.
+ * flags: debugging aids, pass 0 (2: nothing is loaded; with CTA pairs the
  * waits for it then run out: NaN, b200_wait_error). */
 int b200_gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void* residual,
                  long ldr, void* C, long ldc, float* partial, int T, int N, int K, int epilogue,

@@ -529,8 +529,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   __syncthreads();
   w_fence_after();
   const uint32_t tmem_base = tmem_slot;
-  const float bias = wt_bias<TOWER>(p, n0, threadIdx.x);
-  w_pdl_wait();  // everything the previous kernels wrote (X, residual) is visible from here on
+  w_pdl_wait();  // everything the previous kernels wrote (X, residual, the bias) is visible from here on
 
   if (warp == 0) {
     if (lane == 0) {  // ===== TMA producer =====
@@ -581,6 +580,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   __syncwarp();
 
   // ===== epilogue (all 8 warps): warp w reads TMEM lane quarter w % 4, token half w / 4 =====
+  const float bias = wt_bias<TOWER>(p, n0, threadIdx.x);   // (on its way while the products are)
   w_mbar_wait(&tmem_full, 0);
   w_fence_after();
   wt_store_tile<TOWER>(p, WtTile{tmem_base, n0, t0, cg, split, (int)threadIdx.x, bias, false});
@@ -921,7 +921,8 @@ gemm_wt_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
 // per token row; the split-K partials are added in split order (deterministic).
 // ---------------------------------------------------------------------------------------------
 // <threads, vectors of 4 a thread> as the row's width and the number of rows ask for (finish_rows): a chain of L2 round trips, so a
-// thread has one vector where it can, the loads of a row go out together, and those of the weights ahead of the wait for the product.
+// thread has one vector where it can, and the loads of a row and of the weights go out together.  (Weights ahead of the wait for the
+// product, as a caller who makes them on the device right before may not have it: the same times.)
 // Against <256, 8> for all sequences, weights behind the sums: one picture through four vision blocks (2 - 7 partials of 1280 a row)
 // 255 -> 251 us, 272 tokens through four 2B layers 227 -> 224; the few rows of a decode step (1024 threads) take the same time.
 constexpr int FIN_N_MAX = 8192;  // N <= FIN_THREADS * 4 * FIN_MAXV in the widest shapes
@@ -964,8 +965,8 @@ finish_rows_kernel(const float* __restrict__ P, int S, const bf16* __restrict__ 
   w_pdl_launch();
   const int t = blockIdx.x;
   const int nv = N >> 2;
-  if (FIN_THREADS == 1024) w_pdl_wait();   // (a step's blocks wait long for their product, beside its weight stream)
-  uint2 wb[FIN_MAXV], wn[FIN_MAXV], wnb[FIN_MAXV];   // bias, norm weight and bias: of no kernel before this one
+  w_pdl_wait();
+  uint2 wb[FIN_MAXV], wn[FIN_MAXV], wnb[FIN_MAXV];   // bias, norm weight and bias
 #pragma unroll
   for (int u = 0; u < FIN_MAXV; ++u) {
     const int c = threadIdx.x + FIN_THREADS * u;
@@ -973,7 +974,6 @@ finish_rows_kernel(const float* __restrict__ P, int S, const bf16* __restrict__ 
     wn[u] = norm_kind != B200_NORM_NONE && nw && c < nv ? __ldg(reinterpret_cast<const uint2*>(nw + c * 4)) : make_uint2(0, 0);
     wnb[u] = norm_kind != B200_NORM_NONE && norm_kind != B200_NORM_RMS && nb && c < nv ? __ldg(reinterpret_cast<const uint2*>(nb + c * 4)) : make_uint2(0, 0);
   }
-  if (FIN_THREADS < 1024) w_pdl_wait();
   float4 h[FIN_MAXV];
   float s1[FIN_MAXV], s2[FIN_MAXV];   // of a vector
 #pragma unroll

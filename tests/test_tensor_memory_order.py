@@ -67,3 +67,14 @@ def test_columns_are_allocated_before_the_next_kernel_may_start(name, kernel):
     assert "512u" in body[alloc:alloc + 200]
     signals = [m.start() for m in re.finditer(r"griddepcontrol\.launch_dependents|w_pdl_launch\(\)", body)]
     assert len(signals) == 1 and signals[0] > body.index("__syncthreads()", alloc), name
+
+
+@pytest.mark.parametrize("kernel,reads", [("gemm_wt_kernel", r"wt_bias<|p\.(?:bias|residual|res32)\b"), ("gemm_wt_pair_kernel", r"wt_bias<|p\.(?:bias|residual|res32)\b"),
+                                          ("finish_rows_kernel", r"\b(?:P|bias|resid|nw|nb)\b")])
+def test_operands_of_the_epilogue_are_read_behind_the_kernel_before(kernel, reads):
+    """A kernel that starts while the one before it still runs reads nothing that a caller may have made on the device right ahead of the
+    call until griddepcontrol.wait, whatever role its warps have (only the weight matrices are requested earlier)"""
+    body = _body("gemm_wt.cu", kernel)
+    waits = [m.start() for m in re.finditer(r"w_pdl_wait\(\)", body)]
+    seen = [m.start() for m in re.finditer(reads, body)]
+    assert waits and seen and min(seen) > max(waits), kernel
