@@ -40,7 +40,9 @@ constexpr int TC_THREADS = 256 + TC_LOADERS + 32;   // 8 softmax, 7 loading and 
 constexpr int TC_MMA = TC_THREADS / 32 - 1;         // the last warp
 // registers of a softmax thread and of the others: together what the block is launched with, 512 x 128
 constexpr int TC_REGS_SOFTMAX = 152, TC_REGS_OTHER = 104;
-static_assert(256 * TC_REGS_SOFTMAX + (TC_THREADS - 256) * TC_REGS_OTHER <= TC_THREADS * 128, "a larger share would be waited for without end");
+// (a larger share would be waited for without end: tc_launch asks what the kernel was compiled with, the launch bounds only limit it)
+constexpr bool tc_shares_fit(int regs) { return 256 * TC_REGS_SOFTMAX + (TC_THREADS - 256) * TC_REGS_OTHER <= TC_THREADS * regs; }
+static_assert(tc_shares_fit(128) && !tc_shares_fit(127), "the shares are those of 128 registers a thread");
 constexpr int TC_QB = TC_ROWS * 16 + 16, TC_KB = TC_KEYS * 16 + 16;   // bytes of a block of 8 dims
 constexpr int TC_P0 = 128, TC_O0 = 320, TC_GB = 96;   // TMEM columns: S 2 x 64 | P 2 x (3 x 32) | O 2 x 96
 
@@ -583,8 +585,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const _
 template <int HDP>
 int tc_launch(const AttnF32P& p, dim3 grid, cudaStream_t st) {
   static unsigned long long attr_mask = 0ull;
-  if (FirstUse first{&attr_mask})
+  if (FirstUse first{&attr_mask}) {
+    cudaFuncAttributes attr;
+    B200_CUDA(cudaFuncGetAttributes(&attr, attention_f32_tc_kernel<HDP>));
+    if (!tc_shares_fit(attr.numRegs)) first.bit = 0ull;   // (no call gets past this)
+    B200_REQUIRE(tc_shares_fit(attr.numRegs), "attention_f32_tc: compiled with %d registers a thread, fewer than its roles share out", attr.numRegs);
     B200_CUDA(cudaFuncSetAttribute(attention_f32_tc_kernel<HDP>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem<HDP>()));
+  }
   // Launched plainly, it waits for nothing itself.  As a dependent launch its blocks sat on the SMs that the product before it left
   // and ran longer: the whole SigLIP tower on four pictures 19.0 ms, plainly 18.5; three CLIP blocks on one picture 434 us, 423;
   // on three 641, 650; on eight the same.

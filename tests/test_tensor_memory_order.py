@@ -78,3 +78,17 @@ def test_operands_of_the_epilogue_are_read_behind_the_kernel_before(kernel, read
     waits = [m.start() for m in re.finditer(r"w_pdl_wait\(\)", body)]
     seen = [m.start() for m in re.finditer(reads, body)]
     assert waits and seen and min(seen) > max(waits), kernel
+
+
+@pytest.mark.parametrize("name", sorted(n for n in os.listdir(CSRC) if n.endswith(".cu")))
+def test_register_shares_are_checked_before_a_launch(name):
+    """setmaxnreg.inc waits without end for registers that the block was not launched with; launch bounds are only an upper limit, so
+    the host asks what the kernel was compiled with, and a refusal is not remembered as a first use"""
+    with open(os.path.join(CSRC, name)) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    if "setmaxnreg.inc" not in text:
+        return
+    launches = [m.start() for m in re.finditer(r"<<<", text)]
+    assert len(launches) == 1
+    asked, refused, unset = (text.index(w) for w in (".numRegs", "B200_REQUIRE(tc_shares_fit(", "first.bit = 0ull"))
+    assert text.index("cudaFuncGetAttributes") < asked < unset < refused < launches[0]
