@@ -1170,6 +1170,19 @@ static int round16(int x) { return (x + 15) & ~15; }
 constexpr int WP_PAIRS = 74;   // pairs of SMs
 constexpr int WT_KS_WIDE = -1; // WtConfig::KS of a pair with 512 weight rows (0: 256)
 static bool wt_swiglu(int mode) { return mode == B200_WT_SWIGLU || mode == B200_WT_SWIGLU_SPLIT; }
+constexpr size_t WT_SMEM_MAX = 227 * 1024 - 1024;
+static size_t wt_smem(const WtConfig& c) {
+  const int stage = c.KS <= 0 ? (c.KS == WT_KS_WIDE ? 2 : 1) * WT_WBLK + c.TN * 64 : c.KS * (WT_WBLK + c.TN * 128);
+  return (size_t)c.stages * stage + 1024;
+}
+// what gemm_wt takes as the choice of a product (whatever its operands are)
+static bool wt_takes(const WtConfig& c, int K, int mode, int col_groups) {
+  const bool pair = c.KS <= 0;
+  const int kb = cdiv(K, WT_BK);
+  return K > 0 && c.TN >= 16 && c.TN <= 256 && c.TN % (pair ? 32 : 16) == 0 && c.KS >= (col_groups > 0 ? 1 : WT_KS_WIDE) && c.KS <= WT_MAX_STAGES &&
+         c.stages >= 2 && c.stages <= (pair ? WP_MAX_STAGES : WT_MAX_STAGES) && wt_smem(c) <= WT_SMEM_MAX && c.split >= 1 && c.split <= kb &&
+         cdiv(kb, cdiv(kb, c.split)) == c.split && (mode == B200_WT_PARTIAL ? c.KS != WT_KS_WIDE : c.split == 1);
+}
 
 // Tile / pipeline configuration for (T, row blocks, K): a small cost model calibrated on a
 // sweep (profiles/r2_gemm_wt_sweep.txt, B200):
@@ -1311,9 +1324,8 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
   B200_REQUIRE(!grouped || (mode == B200_WT_F32 && ext->n_groups > 0 && cfg.split == 1 && !bias),
                "gemm_wt: grouped products are fp32-output, unsplit, without bias");
   B200_REQUIRE(!pair || (!grouped && !heads), "gemm_wt: pairs take no groups");
-  const int stage = pair ? (wide ? 2 : 1) * WT_WBLK + cfg.TN * 64 : cfg.KS * (WT_WBLK + cfg.TN * 128);
-  const size_t smem = (size_t)cfg.stages * stage + 1024;
-  B200_REQUIRE(smem <= 227 * 1024 - 1024, "gemm_wt: %zu B of shared memory", smem);
+  const size_t smem = wt_smem(cfg);
+  B200_REQUIRE(smem <= WT_SMEM_MAX, "gemm_wt: %zu B of shared memory", smem);
   CUtensorMap tw, tx;
   int rc = wt_tmap(W, (long)(ext && ext->ldw > 0 ? ext->ldw : k_w),
                    grouped ? ext->n_groups * N : (heads && !w_cols ? ext->col_groups * N : (swiglu ? inter : N)),
@@ -1325,14 +1337,14 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
   int dev = 0;
   B200_CUDA(cudaGetDevice(&dev));
   if (!(set_mask >> (dev & 63) & 1ull)) {
-    B200_CUDA(cudaFuncSetAttribute(gemm_wt_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024));
+    B200_CUDA(cudaFuncSetAttribute(gemm_wt_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, WT_SMEM_MAX));
     B200_CUDA(cudaFuncSetAttribute(gemm_wt_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                    cudaSharedmemCarveoutMaxShared));
-    B200_CUDA(cudaFuncSetAttribute(gemm_wt_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024));
+    B200_CUDA(cudaFuncSetAttribute(gemm_wt_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, WT_SMEM_MAX));
     B200_CUDA(cudaFuncSetAttribute(gemm_wt_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                    cudaSharedmemCarveoutMaxShared));
     for (auto kern : {gemm_wt_pair_kernel<false, 1>, gemm_wt_pair_kernel<true, 1>, gemm_wt_pair_kernel<false, 2>, gemm_wt_pair_kernel<true, 2>})
-      B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024));
+      B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WT_SMEM_MAX));
     set_mask |= 1ull << (dev & 63);
   }
   const int row_blocks = swiglu ? cdiv(inter, 64) : cdiv(N, WT_ROWS);
@@ -1439,9 +1451,8 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
           while (fgets(line, sizeof line, fp)) {
             int tb, n, k, md, so, tn, ks, stg, sp, g = 0;
             if (sscanf(line, "%d %d %d %d %d %d %d %d %d %d", &tb, &n, &k, &md, &so, &tn, &ks, &stg, &sp, &g) < 9) continue;
-            if (tn >= 16 && tn <= 256 && tn % (ks > 0 ? 16 : 32) == 0 && ks >= (g > 0 ? 1 : WT_KS_WIDE) && stg >= 2 &&
-                stg <= (ks > 0 ? WT_MAX_STAGES : WP_MAX_STAGES) && sp >= 1)
-              cache[TuneKey{tb, n, k, md, so, g, dev}] = WtConfig{tn, ks, stg, sp};
+            const WtConfig c{tn, ks, stg, sp};   // (a line that no call takes is passed over: its product is measured)
+            if (wt_takes(c, k, md, g)) cache[TuneKey{tb, n, k, md, so, g, dev}] = c;
           }
           fclose(fp);
         }

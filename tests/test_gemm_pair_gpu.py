@@ -251,3 +251,45 @@ def test_a_wait_of_wide_pairs_that_runs_out_is_told(T, n, K):
     child = _CHILD_WAIT.replace("cfg, 8 | flags", "cfg, 16 | flags")
     r = subprocess.run([sys.executable, "-c", child.format(root=root, T=T, n=n, K=K)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+_CHILD_LINES = """
+import sys, torch
+sys.path.insert(0, {root!r})
+sys.path.insert(0, {root!r} + "/tests")
+from mlx_vlm_b200 import _native as N
+lib = N.lib()
+stream = torch.cuda.Stream()       # (choices are measured under capture, which the default stream does not take)
+g = torch.Generator(device="cuda").manual_seed(21)
+for T, n, K in ((300, 264, 128), (577, 1152, 640), (130, 136, 192)):
+    x = torch.randn(T, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(n, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    out = torch.zeros(T, n, device="cuda")
+    torch.cuda.synchronize()
+    N.check(lib.b200_gemm_wt_f32(x.data_ptr(), K, w.data_ptr(), K, 0, 0, 0, out.data_ptr(), n, 0, 0, 0, T, n, K, 1, 0, 3, stream.cuda_stream), "f32")
+    torch.cuda.synchronize()
+    want = x.double() @ w.double().T
+    assert float((out.double() - want).norm() / want.norm()) <= 2e-6
+from test_engine_gpu import _build
+c, W, model, req = _build("wide1", 20, (56, 56))
+lm = model.language_model
+ids = torch.arange(20)[None].numpy()
+logits = lm(ids, inputs_embeds=model.get_input_embeddings(ids).inputs_embeds, cache=lm.make_cache(), logits_to_keep=1).logits
+torch.cuda.synchronize()
+assert bool(torch.isfinite(logits.float()).all())
+"""
+
+
+def test_lines_that_no_call_takes_are_passed_over(tmp_path):
+    """a file of choices may name what gemm_wt refuses: splits outside the partial mode, more shared memory than there is, splits without a
+    k-block, wide pairs that would write partial tiles; such products are measured, the others' lines are kept"""
+    bad = ["5 264 128 3 0 160 -1 4 2", "10 1152 640 3 0 256 2 6 1", "3 136 192 3 0 96 1 4 3", "1 1536 1536 1 1 64 -1 4 1"]
+    good = "1 1536 8960 1 1 32 1 4 3"
+    path = tmp_path / "choices.txt"
+    path.write_text("\n".join(bad + [good]) + "\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _CHILD_LINES.format(root=root)], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, B200_WT_TUNE_FILE=str(path)))
+    assert r.returncode == 0, r.stdout + r.stderr
+    added = [line.split()[:5] for line in path.read_text().splitlines()[len(bad) + 1:]]
+    assert all(line.split()[:5] in added for line in bad) and good.split()[:5] not in added, added
