@@ -1385,7 +1385,7 @@ int gemm_wt(const void* X, long ldx, const void* W, const void* bias, const void
 // ---------------------------------------------------------------------------------------------
 // Measured configuration choice ("measure, don't guess"): the first call for a problem class
 // (tokens rounded up to 64, N, K, mode) times a short list of candidate configurations on the
-// caller's stream with the call's own operands (CUDA events, one warm-up + two timed launches
+// caller's stream with the call's own operands (CUDA events, a warm-up and one or two timed replays
 // each) and caches the winner; later calls cost one hash lookup.  Candidates follow what that
 // sweep showed matters: token tile {96,128,144,192,256}, one CTA per SM with 2 k-blocks
 // per stage vs two CTAs per SM with 1, split-K to one or two waves, and CTA pairs.  The list is ordered and
@@ -1575,8 +1575,11 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
       ext_copy.res32 = nullptr;
       ext_t = &ext_copy;
     }
-    // each candidate is replayed from a small captured graph (6 launches): the measurement sees the
-    // kernel back to back with its programmatic dependent launch, not the host's launch overhead
+    // each candidate is replayed from a small captured graph (16 launches): the measurement sees the
+    // kernel back to back with its programmatic dependent launch, not the host's launch overhead.  One replay behind the warm-up where
+    // the candidate before took a millisecond for it, else two: a caller waits for all this at the first prompt of a new length (three
+    // models of a layer, 17 lengths of 300 - 2048 tokens in all, medians: 7.7 s with the candidates before wide pairs, 7.9 with those,
+    // 5.9 so; the chosen products take the same time, 13.3 / 13.2 / 13.1 ms for the second passes together)
     cudaEvent_t e0, e1;
     B200_CUDA(cudaEventCreate(&e0));
     B200_CUDA(cudaEventCreate(&e1));
@@ -1604,15 +1607,15 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
         rc = B200_ERR_CUDA;
         break;
       }
+      const int runs = i > 0 && ms[i - 1] * REP >= 1.f ? 1 : 2;
       cudaGraphLaunch(gx, st);  // warm-up
       cudaEventRecord(e0, st);
-      cudaGraphLaunch(gx, st);
-      cudaGraphLaunch(gx, st);
+      for (int r = 0; r < runs; ++r) cudaGraphLaunch(gx, st);
       cudaEventRecord(e1, st);
       if (cudaEventSynchronize(e1) != cudaSuccess) rc = B200_ERR_CUDA;
       float t = 0.f;
       cudaEventElapsedTime(&t, e0, e1);
-      ms[i] = t / (2.f * REP);
+      ms[i] = t / (float)(runs * REP);
       cudaGraphExecDestroy(gx);
     }
     cudaEventDestroy(e0);
