@@ -1,8 +1,11 @@
-"""One decoded token of one layer against float64, for every form of the decode kernels: two q heads a CTA (Mistral), three and four of
-four slots (Qwen2-VL-2B, 7B), the per-phase kernels (32 kv heads); contexts at which a CTA's trips over keys and values begin and end
-(its share is an eighth of the keys, a trip 64 or 128 of them); a vocabulary whose tiles fill no whole batch of any CTA.
+"""One decoded token of one layer against float64, for the forms of the decode kernels: heads of 128 with two q heads a CTA (Mistral),
+three and four of four slots (Qwen2-VL-2B, 7B), heads of 64 with two and four, the dataflow mode, the per-phase kernels (32 kv heads);
+contexts at which a CTA's trips over keys and values begin and end (its share is an eighth of the keys, a trip 64 or 128 of them).
 
-Bound: the bf16 roundings of such layers leave 0.016 - 0.036 of the result over two to four of them; 0.04 here."""
+`test_token` is the call as a program makes it, random keys and values, a vocabulary whose tiles fill no whole batch of any CTA: bf16
+roundings of such layers leave 0.016 - 0.036 of the result over two to four of them, 0.04 is its bound, and a key left out would
+pass.  `test_keys_at_the_edges` is for that: the first and last keys of every share and trip carry nearly all of the attention's output."""
+import numpy as np
 import pytest
 import torch
 
@@ -21,3 +24,109 @@ def test_token(geometry, ctx):
     for name in ("logits", "kv"):
         a, b = got[name].double(), want[name].double().reshape(got[name].shape)
         assert float((a - b).norm() / b.norm()) <= 0.04, name
+
+
+# (hidden, mlp, heads, kv heads, mode of the decode step)
+FORMS = {"two heads": (4096, 14336, 32, 8, 1), "three of four": (1536, 8960, 12, 2, 1), "four": (3584, 18944, 28, 4, 1), "per phase": (4096, 11008, 32, 32, 1),
+         "64 wide, four": (1024, 2816, 16, 2, 1), "64 wide, two": (1536, 4096, 24, 12, 1), "64 wide, 512": (512, 1536, 8, 2, 1),
+         "dataflow, two heads": (2048, 4096, 16, 4, 4), "dataflow, three of four": (1536, 8960, 12, 2, 4), "dataflow, 64 wide": (1024, 2816, 16, 2, 4)}
+EDGES = {"two heads": (8, 1023, 1024, 1025, 2049, 5000), "three of four": (7, 511, 513, 1030, 2600), "four": (3, 512, 1100), "per phase": (300, 2200),
+         "64 wide, four": (1, 130, 511, 513, 1025, 3000), "64 wide, two": (510, 1024, 2049), "64 wide, 512": (513, 1025),
+         "dataflow, two heads": (9, 1023, 1024, 2600), "dataflow, three of four": (511, 1030), "dataflow, 64 wide": (512, 1025)}
+VOCAB = 1531
+# q, k, the scores, p, the attention's output, o_proj, the sum, two roundings of the norm and the logits: each 2^-9 at most and 2^-9 / sqrt(3)
+# on the average, together some 2^-9 x sqrt(10 / 3) = 0.0036; twice that
+BOUND = 0.0072
+
+
+def _model(form, v_std, r):
+    """a layer whose attention shows: the MLP adds nothing (its last matrix is zero), the new value is as large as those at the edges"""
+    from mlx_vlm_b200.models.qwen2_vl import Model
+    from mlx_vlm_b200.models.qwen2_vl.config import ModelConfig, TextConfig, VisionConfig
+    H, I, nh, nkv, mode = form
+    hd = H // nh
+    text = TextConfig(model_type="qwen2_vl", hidden_size=H, num_hidden_layers=1, intermediate_size=I, num_attention_heads=nh, rms_norm_eps=1e-6,
+                      vocab_size=VOCAB, num_key_value_heads=nkv, rope_theta=1000000.0,
+                      rope_scaling={"type": "mrope", "mrope_section": [16, 24, 24] if hd == 128 else [8, 12, 12]}, tie_word_embeddings=True)
+    w = C._lm_weights(r, "form", 1, VOCAB)
+    q = "language_model.model.layers.0."
+    w[q + "mlp.down_proj.weight"].zero_()
+    w[q + "self_attn.k_proj.weight"].mul_(0.125)
+    w[q + "self_attn.v_proj.bias"].copy_(r(nkv * hd, std=v_std, dtype=torch.bfloat16))
+    lw = dict(w)
+    lw.update(C._vit_weights(r, 1, C.VIT["embed_dim"], H))
+    model = Model(ModelConfig(text_config=text, vision_config=VisionConfig(depth=1, embed_dim=C.VIT["embed_dim"], hidden_size=H,
+                                                                           num_heads=C.VIT["num_heads"]), model_type="qwen2_vl", vocab_size=VOCAB),
+                  device="cuda:0")
+    model.load_weights(lw)
+    model.engine.set_mega(mode)
+    return model, w
+
+
+def _edges(S):
+    """first and last key of the shares of eight CTAs and of their trips"""
+    per, at = -(-S // 8), set()
+    for u0 in range(0, S, per):
+        u1 = min(S, u0 + per)
+        at |= {u0, u1 - 1} | {u0 + o + d for o in range(64, per, 64) for d in (-1, 0) if u0 + o + d < u1}
+    return sorted(at)
+
+
+@pytest.mark.parametrize("name,ctx", [(n, c) for n, cs in EDGES.items() for c in cs])
+def test_keys_at_the_edges(monkeypatch, name, ctx):
+    """A kv head has its share of the edges (and the new key), whose values are so large that the result misses BOUND twice over where
+    one of them is left out for that head alone, which is shown here for every one; what lies behind the last key is larger still."""
+    H, I, nh, nkv, _ = form = FORMS[name]
+    monkeypatch.setitem(C.GEOMETRY, "form", form[:4])
+    hd, S, r = H // nh, ctx + 1, C._Rand(ctx)
+    edges = _edges(S)
+    share = min(nkv, 16)
+    mine = [sorted(set(edges[g % share::share]) | {ctx}) for g in range(nkv)]
+    v_std = S / (len(edges) / share) ** 0.5
+    model, w = _model(form, v_std, r)
+    lm = model.language_model
+    cache = lm.make_cache()
+    pool = cache[0]._pool
+    pool.reserve(ctx + 256)
+    kv = r(2, nkv, ctx, hd)
+    kv[0].mul_(0.125)
+    for g in range(nkv):
+        kv[1][g, [e for e in mine[g] if e < ctx]] *= v_std
+    kv = kv.to(torch.bfloat16)
+    pool.buf.fill_(4.0 * S)
+    pool.buf[0, :, 0, :, :ctx] = kv
+    tok = int(r.ints(0, VOCAB, 1)[0])
+    torch.cuda.synchronize()
+    for c in cache:
+        c.offset = ctx
+    out = lm(np.array([[tok]]), cache=cache, position_ids=np.full((3, 1, 1), ctx), rope_deltas=np.zeros((1, 1)))
+    torch.cuda.synchronize()
+    assert model.engine.device_error() == 0
+    # ---- float64
+    p, d = "language_model.model.", {n: t.double() for n, t in w.items()}
+    q_ = p + "layers.0.self_attn."
+    x = d[p + "embed_tokens.weight"][tok]
+    n1 = C._rms(x, w[p + "layers.0.input_layernorm.weight"], 1e-6)
+    ang = ctx * 1000000.0 ** (-torch.arange(0, hd, 2, device="cuda", dtype=torch.float64) / hd)
+    q, kn, vn = ((d[q_ + c + "_proj.weight"] @ n1 + d[q_ + c + "_proj.bias"]).view(-1, hd) for c in "qkv")
+    q, kn = C._rotate(q, ang), C._rotate(kn, ang)
+    got_kv = pool.buf[0, :, 0, :, ctx].double()
+    assert float((got_kv - torch.stack([kn, vn])).norm() / torch.stack([kn, vn]).norm()) <= 2.0 ** -8
+    k, v = torch.cat([kv[0].double(), kn[:, None]], 1), torch.cat([kv[1].double(), vn[:, None]], 1)     # (kv heads, S, hd)
+    rep = nh // nkv
+    pr = torch.softmax(torch.einsum("gqd,gsd->gqs", q.view(nkv, rep, hd), k) * hd ** -0.5, -1)
+    att = pr @ v                                                                                          # (kv heads, rep, hd)
+
+    def logits(a):
+        return C._rms(x + a.reshape(-1, H) @ d[q_ + "o_proj.weight"].T, w[p + "norm.weight"], 1e-6) @ d[p + "embed_tokens.weight"].T
+
+    want = logits(att)[0]
+    if ctx:                                               # without key e of kv head g
+        for g in range(nkv):
+            pe = pr[g][:, mine[g]].T[:, :, None]                                                          # (edges, rep, 1)
+            less = att.expand(len(mine[g]), -1, -1, -1).clone()
+            less[:, g] = (att[g] - pe * v[g, mine[g]][:, None]) / (1.0 - pe)
+            off = (logits(less) - want).norm(dim=1) / want.norm()
+            assert float(off.min()) >= 2 * BOUND, (g, float(off.min()))
+    got = out.logits.double().reshape(-1)
+    assert float((got - want).norm() / want.norm()) <= BOUND

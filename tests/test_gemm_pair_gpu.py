@@ -293,3 +293,17 @@ def test_lines_that_no_call_takes_are_passed_over(tmp_path):
     assert r.returncode == 0, r.stdout + r.stderr
     added = [line.split()[:5] for line in path.read_text().splitlines()[len(bad) + 1:]]
     assert all(line.split()[:5] in added for line in bad) and good.split()[:5] not in added, added
+
+
+@pytest.mark.parametrize("ks,tn", [(1, 128), (2, 96), (0, 160), (-1, 192)])
+def test_split_outputs_of_an_odd_number_of_rows(tmp_path, ks, tn):
+    """[hi | lo] pairs whose rows are written feature by feature: one CTA, pairs and wide pairs, configurations given by a file"""
+    cases = [(300, 263, 128, 4, 0), (577, 131, 584, 4, 2), (65, 77, 72, 4, 0), (200, 999, 1152, 4, 2)]
+    lines = [f"{(T + 63) // 64} {n} {2 * ((K + 63) // 64 * 64)} {mode} 0 {tn} {ks} 3 1" for T, n, K, mode, _ in cases]
+    path = tmp_path / "choices.txt"
+    path.write_text("\n".join(lines) + "\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _CHILD.format(root=root, cases=cases)], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, B200_WT_TUNE_FILE=str(path)))
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert path.read_text() == "\n".join(lines) + "\n"        # nothing was measured: the file's choices ran
