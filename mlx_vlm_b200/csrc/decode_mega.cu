@@ -11,10 +11,11 @@
 //   * warps 0..7 are CONSUMERS that execute the phases in order, separated by a
 //     software grid barrier (one atomic + acquire spin, ~1 us) instead of a kernel
 //     boundary; activations cross CTAs through L2 (ld.global.cg).
-// A layer runs through some 90 KB of code once, in the 33 us that it takes, and what of it is not in the instruction cache any more
-// is a wait in the middle of a phase.  So the loops here are rolled, and a phase calls its epilogue in one place (it is inlined): the
-// kernel for 1,536 wide models 233 -> 189 KB, its step at a context of 700 1079 -> 1005 us, four layers of 4,096 behind 6000 keys 514
-// -> 472, with the products of mega_common.cuh (fma_bf2) and batched warp sums; with the tile loop unrolled eight times 1284.
+// A layer runs once through most of the kernel's code, in the 33 us that it takes, and what of it is not in the instruction cache any
+// more is a wait in the middle of a phase.  So the loops here are rolled, and a phase calls its epilogue in one place (it is inlined):
+// the kernel for 1,536 wide models went from 233 KB to 189, its step at a context of 700 from 1079 to 1005 us, four layers of 4,096
+// behind 6000 keys from 514 to 472, with the products of common.cuh (fma_bf2) and batched warp sums; with the tile loop unrolled
+// eight times 1284.  With one form of the attention each (MA_*) it has 164 KB now.
 // Rounding points follow oracle/qwen2vl.py::lm_layers_forward (same device
 // functions as the multi-kernel path in decode.cu).
 #include <climits>
@@ -378,8 +379,8 @@ __device__ __forceinline__ void consume_phase(const MegaP& p, const MegaPhase& g
 // them because every later phase needs data from ALL CTAs of the phase before it (transitively
 // nobody can overwrite a word that a slower CTA still has to read), and the tag of a word is
 // unique per (step, layer).
-// ATT: the attention that the kernel holds.  One that held all three forms had 217 KB instead of 162 and took 1011 us instead of 996 for
-// a token of the 2B model; the small models and the dataflow mode share a kernel (MA_ANY) all the same.
+// ATT: the attention that the kernel holds.  One that holds all three forms has 219 KB instead of 158 - 164 and took 1011 us instead of
+// 996 for a token of the 2B model; the small models and the dataflow mode share a kernel (MA_ANY) all the same.
 enum { MA_ANY = 0, MA_64, MA_128, MA_128_PAIR };   // head dim; PAIR: at most two q heads a CTA
 __host__ __device__ __forceinline__ int mega_att(const MegaP& p) {
   return p.d.hd == 64 ? MA_64 : (p.hsplit * 2 >= p.d.n_heads / p.d.n_kv ? MA_128_PAIR : MA_128);
@@ -623,8 +624,9 @@ static int mega_launch_t(const MegaP& p, int grid, size_t smem, cudaStream_t s) 
     if (att == MA_64) return mega_launch_f<CHH, CHI, false, MA_64>(p, grid, smem, s);
     if (att == MA_128) return mega_launch_f<CHH, CHI, false, MA_128>(p, grid, smem, s);
     return mega_launch_f<CHH, CHI, false, MA_128_PAIR>(p, grid, smem, s);
+  } else {
+    return mega_launch_f<CHH, CHI, false, MA_ANY>(p, grid, smem, s);
   }
-  return mega_launch_f<CHH, CHI, false, MA_ANY>(p, grid, smem, s);
 }
 
 int mega_launch(const MegaP& p, int sm_count, cudaStream_t s) {
