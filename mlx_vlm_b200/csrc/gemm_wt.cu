@@ -1628,7 +1628,7 @@ int gemm_wt_tuned(const void* X, long ldx, const void* W, const void* bias, cons
     }
     // Back to back a pair does not show what it costs in a sequence: all of an SM's shared memory, so the next kernel's set-up
     // and weight loads wait for it, and code of its own to fetch.  It has to win by 8 % (a 2048 x 2048 x 2048 product measured 3 %
-    // faster alone and was 4 us of 26 slower between row kernels), or 4 us: the cost does not grow with the product (with 8 % of
+    // faster alone and was 4 us of 26 slower between row kernels), or by those 4 us: set-up and code do not grow with the product (with 8 % of
     // everything one-CTA tiles took 4096 x 4096 x 28672 in fp32 at 827 us, where wide pairs take 685).
     for (size_t i = 0; i < cand.size(); ++i)
       if (cand[i].KS <= 0) ms[i] += std::min(0.08f * ms[i], 0.004f);

@@ -247,7 +247,7 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
   float* vn = kn + HD;                                     //        [HD] new value
   const int seg = lane & 7, ksub = lane >> 3;
   // ---- all global requests of the phase are issued before the first use: q, the first
-  // 2 x 4 keys of this warp, and the V rows of its first VPRE keys (one round trip) ----
+  // UNR x 4 keys of this warp, and its first VB value rows (one round trip) ----
   uint4 qraw[GN][NV];
   if (!PARTS) {
 #pragma unroll
@@ -371,7 +371,7 @@ __device__ __forceinline__ void attn_phase(const MegaP& p, const bf16* kc, const
       }
   }
   ATT_STAMP();  // q loaded
-  // ---- 1. scores of the own range (software-pipelined over trips of 2 x 4 keys) ----
+  // ---- 1. scores of the own range (software-pipelined over trips of UNR x 4 keys) ----
   float lm[GN];
 #pragma unroll
   for (int g = 0; g < GN; ++g) lm[g] = -INFINITY;

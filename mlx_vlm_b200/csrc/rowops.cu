@@ -491,10 +491,7 @@ int mrope_kv_write(void* qkv, const int* pos3, const float* inv_freq, const int*
 
 // ---------------------------------------------------------------------------
 // Vision tower, after the qkv GEMM: 2-D rotary on q and k in place (same arithmetic as
-// vision_rope_kernel), q pre-scaled for the SDPA (qs = bf16(q * bf16(scale))), and, where vt is given, V written
-// TRANSPOSED ([head][dim][token], tokens contiguous) through a shared-memory tile (the tower itself passes none: its
-// attention reads V from the qkv rows).
-// grid (ceil(T / 32), heads), 256 threads.
+// vision_rope_kernel), q pre-scaled for the SDPA (qs = bf16(q * bf16(scale))).  First the cos / sin table of a tower call.
 __global__ void vision_rope_table_kernel(const int* __restrict__ pos_hw, const float* __restrict__ inv_freq, int T,
                                         int half, float2* __restrict__ cs) {
   pdl_prologue();
@@ -514,7 +511,7 @@ __device__ __forceinline__ uint32_t rot_pair(uint64_t a, uint64_t c, uint64_t b,
 }
 
 // The tower's form (V is read where it lies, cos / sin come from the table): a CTA takes 32 tokens x a group of heads; thread (token,
-// chunk of 8 rotary pairs) reads its 8 cos / sin once for q and k of all of them, two heads in flight, and works on pairs.  Bound by
+// chunk of 8 rotary pairs) reads its 8 cos / sin once for q and k of all of them, two heads in flight.  Bound by
 // memory: 2 B read and written per element of q and k.  A head a CTA, cos / sin read for q and for k of each (as many bytes as the
 // data), element by element: two vision blocks of 6012 patches, 16 heads of 80, 971 -> 947 us (the two launches 54 -> 35), four of 576
 // 253 -> 251, one at a time 452 -> 435.
@@ -568,6 +565,10 @@ vision_rope_rows_kernel(bf16* __restrict__ qkv, const float2* __restrict__ cs, i
   }
 }
 
+// The general form: cos / sin worked out per element, any head dim that is a multiple of 8, and where vt is given, V written
+// TRANSPOSED ([head][dim][token], tokens contiguous) through a shared-memory tile (b200_vision_qkv_post; the tower comes here only
+// with head dims that are no multiple of 16).
+// grid (ceil(T / 32), heads), 256 threads.
 __global__ void vision_qkv_post_kernel(bf16* __restrict__ qkv, const int* __restrict__ pos_hw,
                                        const float* __restrict__ inv_freq, int T, int n_heads, int hd,
                                        float scale_bf, bf16* __restrict__ vt, int t_ld) {
