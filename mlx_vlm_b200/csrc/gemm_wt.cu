@@ -957,22 +957,23 @@ __device__ __forceinline__ float fin_block_sum(const float (&q)[FIN_MAXV], float
 
 template <int FIN_THREADS, int FIN_MAXV>
 __global__ void __launch_bounds__(FIN_THREADS)
-finish_rows_kernel(const float* __restrict__ P, int S, const bf16* __restrict__ bias,
-                   const bf16* __restrict__ resid, long ldr, bf16* __restrict__ h_out, long ldh,
-                   int norm_kind, const bf16* __restrict__ nw, const bf16* __restrict__ nb, float eps,
-                   bf16* __restrict__ xn, long ldx, int T, int N) {
+finish_rows_kernel(const float* __restrict__ P, int S, const bf16* bias, const bf16* resid, long ldr, bf16* h_out, long ldh,
+                   int norm_kind, const bf16* nw, const bf16* nb, float eps, bf16* xn, long ldx, int T, int N) {
   __shared__ float red[FIN_THREADS / 32], ex[FIN_MAXV][256];
   w_pdl_launch();
   const int t = blockIdx.x;
   const int nv = N >> 2;
   w_pdl_wait();
-  uint2 wb[FIN_MAXV], wn[FIN_MAXV], wnb[FIN_MAXV];   // bias, norm weight and bias
+  // residual, bias, norm weight and bias (plain loads of pointers that may alias: the compiler may move neither these nor those of a
+  // read-only path ahead of the wait)
+  uint2 rv[FIN_MAXV], wb[FIN_MAXV], wn[FIN_MAXV], wnb[FIN_MAXV];
 #pragma unroll
   for (int u = 0; u < FIN_MAXV; ++u) {
     const int c = threadIdx.x + FIN_THREADS * u;
-    wb[u] = bias && c < nv ? __ldg(reinterpret_cast<const uint2*>(bias + c * 4)) : make_uint2(0, 0);
-    wn[u] = norm_kind != B200_NORM_NONE && nw && c < nv ? __ldg(reinterpret_cast<const uint2*>(nw + c * 4)) : make_uint2(0, 0);
-    wnb[u] = norm_kind != B200_NORM_NONE && norm_kind != B200_NORM_RMS && nb && c < nv ? __ldg(reinterpret_cast<const uint2*>(nb + c * 4)) : make_uint2(0, 0);
+    rv[u] = resid && c < nv ? *reinterpret_cast<const uint2*>(resid + (long)t * ldr + c * 4) : make_uint2(0, 0);
+    wb[u] = bias && c < nv ? *reinterpret_cast<const uint2*>(bias + c * 4) : make_uint2(0, 0);
+    wn[u] = norm_kind != B200_NORM_NONE && nw && c < nv ? *reinterpret_cast<const uint2*>(nw + c * 4) : make_uint2(0, 0);
+    wnb[u] = norm_kind != B200_NORM_NONE && norm_kind != B200_NORM_RMS && nb && c < nv ? *reinterpret_cast<const uint2*>(nb + c * 4) : make_uint2(0, 0);
   }
   float4 h[FIN_MAXV];
   float s1[FIN_MAXV], s2[FIN_MAXV];   // of a vector
@@ -983,7 +984,6 @@ finish_rows_kernel(const float* __restrict__ P, int S, const bf16* __restrict__ 
     s1[u] = s2[u] = 0.f;
     if (c < nv) {
       // the split-K partials of this chunk: up to 8 loads in flight, added in split order
-      const uint2 rv = resid ? *reinterpret_cast<const uint2*>(resid + (long)t * ldr + c * 4) : make_uint2(0, 0);
       float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
       for (int s0 = 0; s0 < S; s0 += 8) {
@@ -1005,7 +1005,7 @@ finish_rows_kernel(const float* __restrict__ P, int S, const bf16* __restrict__ 
       a.x = rbf(a.x); a.y = rbf(a.y); a.z = rbf(a.z); a.w = rbf(a.w);
       if (resid) {
         float rr[4];
-        unpack4(rv, rr);
+        unpack4(rv[u], rr);
         a.x = rbf(rr[0] + a.x); a.y = rbf(rr[1] + a.y); a.z = rbf(rr[2] + a.z); a.w = rbf(rr[3] + a.w);
       }
       h[u] = a;
