@@ -517,7 +517,7 @@ __device__ __forceinline__ uint32_t rot_pair(uint64_t a, uint64_t c, uint64_t b,
 // 253 -> 251, one at a time 452 -> 435.
 // grid (ceil(T / 32), head groups), 32 x (hd / 16) threads.
 __global__ void __launch_bounds__(256)
-vision_rope_rows_kernel(bf16* __restrict__ qkv, const float2* __restrict__ cs, int T, int n_heads, int hd, float scale_bf, int heads_per_cta) {
+vision_rope_rows_kernel(bf16* __restrict__ qkv, const float2* cs, int T, int n_heads, int hd, float scale_bf, int heads_per_cta) {
   pdl_prologue();
   const int half = hd >> 1, nc = half >> 3;
   const int c = threadIdx.x % nc, t = blockIdx.x * 32 + threadIdx.x / nc;
@@ -526,7 +526,7 @@ vision_rope_rows_kernel(bf16* __restrict__ qkv, const float2* __restrict__ cs, i
   uint64_t co[4], si[4], ns[4];   // cos, sin, -sin of pairs
 #pragma unroll
   for (int w = 0; w < 4; ++w) {
-    const float4 f = __ldg(tab + w);
+    const float4 f = tab[w];   // (a plain load: the table may be that of the kernel before the last, which the wait covers)
     co[w] = f2(f.x, f.z);
     si[w] = f2(f.y, f.w);
     ns[w] = f2(-f.y, -f.w);
