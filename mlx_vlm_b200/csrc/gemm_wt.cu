@@ -239,42 +239,63 @@ __device__ __forceinline__ void wt_groups(const WtTile& c, int tokens, Residual 
   }
 }
 
-// bf16 rows
+// Does the warp's last feature stand alone (an odd number of features, two to a word)?  It has a loop of its own: one more predicate per
+// store in the other's is 2 - 3 % of a vision block.  (Rows of an odd number element by element took 11 - 20 % longer where the
+// stores show: 300 x 32003 x 1024 31.5 us, 25.8 so; 600 x 1153 x 1152 18.0 and 15.0.)
+__device__ __forceinline__ bool wt_odd_end(const WtParams& p, const WtTile& c) {
+  return (p.N & 1) && c.n0 + (c.tid >> 5 & 3) * 32 + 32 > p.N;
+}
+template <bool TAIL>
+__device__ __forceinline__ void wt_put_word(bf16* d, uint32_t v, bool both) {
+  if (!TAIL || both) *reinterpret_cast<uint32_t*>(d) = v;
+  else *reinterpret_cast<unsigned short*>(d) = (unsigned short)v;
+}
+
+// bf16 rows, two features of a token as one word
+template <int EPI, bool TAIL>
+__device__ __forceinline__ void wt_store_words(const WtParams& p, const WtTile& c, int tokens) {
+  const int lane = c.tid & 31, n = c.n0 + (c.tid >> 5 & 3) * 32 + (lane & ~1), odd = lane & 1;
+  const uint32_t sel = odd ? 0x3276u : 0x5410u;
+  const bool store = n < p.N && !(p.flags & 4u), both = n + 1 < p.N;
+  bf16* const d0 = p.C + (long)(c.t0 + odd) * p.ldc + n;
+  const bf16* const s0 = p.residual + (long)(c.t0 + odd) * p.ldr + n;
+  auto body = [&](int cc, uint32_t (&a)[8], uint32_t (&r)[8], auto with_res) {
+    const int nv = store ? tokens - cc - odd : 0;
+    bf16* d = d0 + (long)cc * p.ldc;
+#pragma unroll
+    for (int i = 0; i < 4; ++i, d += 2 * p.ldc) {
+      uint32_t v = wt_swap(wt_act_bf16<EPI>(a[2 * i], a[2 * i + 1], c.bias), 1, sel);
+      if constexpr (decltype(with_res)::value) v = pack_bf2(add2(unpack_bf2(r[i]), unpack_bf2(v)));
+      if (2 * i < nv) wt_put_word<TAIL>(d, v, both);
+    }
+  };
+  if (p.residual) {
+    wt_groups(c, tokens, [&](int cc, uint32_t (&r)[8]) {
+      const int nv = store ? tokens - cc - odd : 0;
+      const bf16* s = s0 + (long)cc * p.ldr;
+#pragma unroll
+      for (int i = 0; i < 4; ++i, s += 2 * p.ldr) {
+        r[i] = 0u;
+        if (2 * i < nv) r[i] = !TAIL || both ? *reinterpret_cast<const uint32_t*>(s) : *reinterpret_cast<const unsigned short*>(s);
+      }
+    }, [&](int cc, uint32_t (&a)[8], uint32_t (&r)[8]) { body(cc, a, r, std::true_type{}); });
+  } else {
+    wt_groups(c, tokens, [](int, uint32_t (&)[8]) {}, [&](int cc, uint32_t (&a)[8], uint32_t (&r)[8]) { body(cc, a, r, std::false_type{}); });
+  }
+}
+
 template <int EPI>
 __device__ __forceinline__ void wt_store_bf16(const WtParams& p, const WtTile& c, int tokens) {
-  const int lane = c.tid & 31, n = c.n0 + (c.tid >> 5 & 3) * 32 + lane, odd = lane & 1;
-  const uint32_t sel = odd ? 0x3276u : 0x5410u;
-  const bool store = n < p.N && !(p.flags & 4u);
   const bool res = p.residual != nullptr;
-  auto none = [](int, uint32_t (&)[8]) {};
-  // two features of a token as one word
-  if ((p.N & 1) == 0 && ((p.ldc | (res ? p.ldr : 0)) & 1) == 0 &&
+  if (((p.ldc | (res ? p.ldr : 0)) & 1) == 0 &&
       ((reinterpret_cast<uintptr_t>(p.C) | (res ? reinterpret_cast<uintptr_t>(p.residual) : 0)) & 3) == 0) {
-    bf16* const d0 = p.C + (long)(c.t0 + odd) * p.ldc + (n & ~1);
-    const bf16* const s0 = p.residual + (long)(c.t0 + odd) * p.ldr + (n & ~1);
-    auto body = [&](int cc, uint32_t (&a)[8], uint32_t (&r)[8], auto with_res) {
-      const int nv = store ? tokens - cc - odd : 0;
-      bf16* d = d0 + (long)cc * p.ldc;
-#pragma unroll
-      for (int i = 0; i < 4; ++i, d += 2 * p.ldc) {
-        uint32_t v = wt_swap(wt_act_bf16<EPI>(a[2 * i], a[2 * i + 1], c.bias), 1, sel);
-        if constexpr (decltype(with_res)::value) v = pack_bf2(add2(unpack_bf2(r[i]), unpack_bf2(v)));
-        if (2 * i < nv) *reinterpret_cast<uint32_t*>(d) = v;
-      }
-    };
-    if (res) {
-      wt_groups(c, tokens, [&](int cc, uint32_t (&r)[8]) {
-        const int nv = store ? tokens - cc - odd : 0;
-        const bf16* s = s0 + (long)cc * p.ldr;
-#pragma unroll
-        for (int i = 0; i < 4; ++i, s += 2 * p.ldr) r[i] = 2 * i < nv ? *reinterpret_cast<const uint32_t*>(s) : 0u;
-      }, [&](int cc, uint32_t (&a)[8], uint32_t (&r)[8]) { body(cc, a, r, std::true_type{}); });
-    } else {
-      wt_groups(c, tokens, none, [&](int cc, uint32_t (&a)[8], uint32_t (&r)[8]) { body(cc, a, r, std::false_type{}); });
-    }
+    if (wt_odd_end(p, c)) wt_store_words<EPI, true>(p, c, tokens);
+    else wt_store_words<EPI, false>(p, c, tokens);
     return;
   }
-  wt_groups(c, tokens, none, [&](int cc, uint32_t (&a)[8], uint32_t (&)[8]) {
+  const int n = c.n0 + (c.tid >> 5 & 3) * 32 + (c.tid & 31);
+  const bool store = n < p.N && !(p.flags & 4u);
+  wt_groups(c, tokens, [](int, uint32_t (&)[8]) {}, [&](int cc, uint32_t (&a)[8], uint32_t (&)[8]) {
     const int nv = store ? tokens - cc : 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -288,10 +309,36 @@ __device__ __forceinline__ void wt_store_bf16(const WtParams& p, const WtTile& c
   });
 }
 
-// fp32 rows, or [hi | lo]: hi = bf16(v), lo = bf16(v - hi)
+// [hi | lo]: hi = bf16(v), lo = bf16(v - hi), two features to a word (rows and parts lie 8-feature aligned)
+template <int EPI, bool TAIL>
+__device__ __forceinline__ void wt_store_split(const WtParams& p, const WtTile& c, int tokens) {
+  const int lane = c.tid & 31, n = c.n0 + (c.tid >> 5 & 3) * 32 + (lane & ~1), odd = lane & 1;
+  const uint32_t sel = odd ? 0x3276u : 0x5410u;
+  const bool store = n < p.N && !(p.flags & 4u), both = n + 1 < p.N;
+  bf16* const d0 = p.Csplit + (long)(c.t0 + odd) * p.ld_split + n;
+  wt_groups(c, tokens, [](int, uint32_t (&)[8]) {}, [&](int cc, uint32_t (&a)[8], uint32_t (&)[8]) {
+    const int nv = store ? tokens - cc - odd : 0;
+    bf16* d = d0 + (long)cc * p.ld_split;
+#pragma unroll
+    for (int i = 0; i < 4; ++i, d += 2 * p.ld_split) {
+      wt_act_f32<EPI>(a[2 * i], a[2 * i + 1], c.bias);
+      const float x0 = __uint_as_float(a[2 * i]), x1 = __uint_as_float(a[2 * i + 1]);
+      uint32_t hi = pack2(x0, x1);
+      uint32_t lo = pack2(x0 - __uint_as_float(hi << 16), x1 - __uint_as_float(hi & 0xffff0000u));
+      hi = wt_swap(hi, 1, sel);
+      lo = wt_swap(lo, 1, sel);
+      if (2 * i < nv) {
+        wt_put_word<TAIL>(d, hi, both);
+        wt_put_word<TAIL>(d + p.n_pad, lo, both);
+      }
+    }
+  });
+}
+
+// fp32 rows, or [hi | lo]
 template <int EPI>
 __device__ __forceinline__ void wt_store_f32(const WtParams& p, const WtTile& c, int tokens) {
-  const int lane = c.tid & 31, n = c.n0 + (c.tid >> 5 & 3) * 32 + lane, odd = lane & 1;
+  const int n = c.n0 + (c.tid >> 5 & 3) * 32 + (c.tid & 31);
   const bool store = n < p.N && !(p.flags & 4u);
   auto none = [](int, uint32_t (&)[8]) {};
   if (p.mode == B200_WT_F32) {
@@ -321,32 +368,8 @@ __device__ __forceinline__ void wt_store_f32(const WtParams& p, const WtTile& c,
     }
     return;
   }
-  const uint32_t sel = odd ? 0x3276u : 0x5410u;
-  const bool pairs = (p.N & 1) == 0;   // two features of a token as one word
-  bf16* const d0 = p.Csplit + (long)(c.t0 + (pairs ? odd : 0)) * p.ld_split + (pairs ? n & ~1 : n);
-  wt_groups(c, tokens, none, [&](int cc, uint32_t (&a)[8], uint32_t (&)[8]) {
-    const int nv = store ? tokens - cc - (pairs ? odd : 0) : 0;
-    bf16* d = d0 + (long)cc * p.ld_split;
-#pragma unroll
-    for (int i = 0; i < 4; ++i, d += 2 * p.ld_split) {
-      wt_act_f32<EPI>(a[2 * i], a[2 * i + 1], c.bias);
-      const float x0 = __uint_as_float(a[2 * i]), x1 = __uint_as_float(a[2 * i + 1]);
-      uint32_t hi = pack2(x0, x1);
-      uint32_t lo = pack2(x0 - __uint_as_float(hi << 16), x1 - __uint_as_float(hi & 0xffff0000u));
-      if (pairs) {
-        hi = wt_swap(hi, 1, sel);
-        lo = wt_swap(lo, 1, sel);
-        if (2 * i < nv) {
-          *reinterpret_cast<uint32_t*>(d) = hi;
-          *reinterpret_cast<uint32_t*>(d + p.n_pad) = lo;
-        }
-      } else {
-        unsigned short* w = reinterpret_cast<unsigned short*>(d);
-        if (2 * i < nv) w[0] = (unsigned short)hi, w[p.n_pad] = (unsigned short)lo;
-        if (2 * i + 1 < nv) w[p.ld_split] = (unsigned short)(hi >> 16), w[p.ld_split + p.n_pad] = (unsigned short)(lo >> 16);
-      }
-    }
-  });
+  if (wt_odd_end(p, c)) wt_store_split<EPI, true>(p, c, tokens);
+  else wt_store_split<EPI, false>(p, c, tokens);
 }
 
 // SwiGLU: the tile's rows are gate and up of its channels in turn (w_tma_3d), so neighbouring lanes hold a channel: one swap gives

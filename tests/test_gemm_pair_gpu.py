@@ -307,3 +307,33 @@ def test_split_outputs_of_an_odd_number_of_rows(tmp_path, ks, tn):
                        env=dict(os.environ, B200_WT_TUNE_FILE=str(path)))
     assert r.returncode == 0, r.stdout + r.stderr
     assert path.read_text() == "\n".join(lines) + "\n"        # nothing was measured: the file's choices ran
+
+
+@pytest.mark.parametrize("T,N,K,cfg,flag", [(1, 65, 64, (16, 1, 3, 1), 0), (65, 77, 72, (96, 2, 2, 1), 0), (300, 263, 192, (128, 1, 3, 1), 0),
+                                            (300, 257, 192, (160, 1, 4, 1), PAIR), (577, 1031, 128, (224, 1, 4, 1), WIDE)])
+@pytest.mark.parametrize("epi", [0, 1, 2])
+def test_rows_of_an_odd_number_of_features(lib, T, N, K, cfg, flag, epi):
+    """even row strides: two features to a word, the last ones alone; with and without a residual, in place, and nothing behind the last
+    feature is written or taken"""
+    import ctypes
+    from mlx_vlm_b200 import _native as Nn
+    x, w, b = _rand(T, K, seed=31), _rand(N, K, seed=32, std=K ** -0.5), _rand(N, seed=33)
+    y = (x.double() @ w.double().T + b.double()).to(torch.bfloat16).double()
+    if epi == 1:
+        y = y * torch.sigmoid((1.703125 * y).to(torch.bfloat16).double()).to(torch.bfloat16).double()
+    if epi == 2:
+        y = torch.nn.functional.gelu(y)
+    ld = N + 1 + T % 2 * 2
+    for res in (None, _rand(T, ld, seed=34)):
+        out = torch.full((T, ld), 9.0, dtype=torch.bfloat16, device="cuda")
+        if res is not None:
+            res[:, N:] = float("nan")
+            out[:, :N] = res[:, :N]
+        r = None if res is None else out                  # (the output is its own residual)
+        Nn.check(lib.b200_gemm_wt(x.data_ptr(), K, w.data_ptr(), b.data_ptr(), Nn.ptr(r), ld, out.data_ptr(), ld, 0, T, N, K, epi, 0, 0,
+                                  (ctypes.c_int * 4)(*cfg), flag, 0), "gemm_wt")
+        torch.cuda.synchronize()
+        want = y if res is None else y.to(torch.bfloat16).double() + res[:, :N].double()
+        # the unit's own roundings to bf16: the exact GELU has five, the fast one three, most of them shared with the reference's
+        assert rl2(out[:, :N], want) <= (2.0 ** -8 if epi == 0 else 2.0 ** -7)
+        assert bool((out[:, N:] == 9.0).all())
