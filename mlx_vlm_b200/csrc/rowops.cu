@@ -503,11 +503,10 @@ __global__ void vision_rope_table_kernel(const int* __restrict__ pos_hw, const f
   cs[idx] = make_float2(cosf(ang), sinf(ang));
 }
 
-// bf16 of a * c + b * d, pairs, each product and the sum rounded.  (add.rn.f32x2 of two mul.rn.f32x2 becomes one product and one FMA:
-// single values came out a bf16 unit off, which the layers behind them spread to 0.5 % of the tower's output.  The same time.)
-__device__ __forceinline__ uint32_t rot_pair(uint64_t a, uint64_t c, uint64_t b, uint64_t d) {
-  return pack2(__fadd_rn(__fmul_rn(f2_lo(a), f2_lo(c)), __fmul_rn(f2_lo(b), f2_lo(d))),
-               __fadd_rn(__fmul_rn(f2_hi(a), f2_hi(c)), __fmul_rn(f2_hi(b), f2_hi(d))));
+// bf16 pair of a * c + b * d, each product and the sum rounded.  (On pairs, add.rn.f32x2 of two mul.rn.f32x2 becomes one product and one
+// FMA: single values came out a bf16 unit off, which the layers behind them spread to 0.5 % of the tower's output.  The same time.)
+__device__ __forceinline__ uint32_t rot_pair(uint64_t a, float c0, float c1, uint64_t b, float d0, float d1) {
+  return pack2(__fadd_rn(__fmul_rn(f2_lo(a), c0), __fmul_rn(f2_lo(b), d0)), __fadd_rn(__fmul_rn(f2_hi(a), c1), __fmul_rn(f2_hi(b), d1)));
 }
 
 // The tower's form (V is read where it lies, cos / sin come from the table): a CTA takes 32 tokens x a group of heads; thread (token,
@@ -523,14 +522,9 @@ vision_rope_rows_kernel(bf16* __restrict__ qkv, const float2* cs, int T, int n_h
   const int c = threadIdx.x % nc, t = blockIdx.x * 32 + threadIdx.x / nc;
   if (t >= T) return;
   const float4* tab = reinterpret_cast<const float4*>(cs + (long)t * half + c * 8);
-  uint64_t co[4], si[4], ns[4];   // cos, sin, -sin of pairs
+  float4 cs2[4];   // cos, sin of two pairs (plain loads: the table may be that of the kernel before the last, which the wait covers)
 #pragma unroll
-  for (int w = 0; w < 4; ++w) {
-    const float4 f = tab[w];   // (a plain load: the table may be that of the kernel before the last, which the wait covers)
-    co[w] = f2(f.x, f.z);
-    si[w] = f2(f.y, f.w);
-    ns[w] = f2(-f.y, -f.w);
-  }
+  for (int w = 0; w < 4; ++w) cs2[w] = tab[w];
   const uint64_t scale2 = f2(scale_bf, scale_bf);
   const int h0 = blockIdx.y * heads_per_cta, h1 = min(n_heads, h0 + heads_per_cta);
   bf16* row = qkv + (long)t * 3 * n_heads * hd + c * 8;
@@ -551,8 +545,9 @@ vision_rope_rows_kernel(bf16* __restrict__ qkv, const float2* cs, int T, int n_h
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
           const uint64_t y1 = unpack_bf2(x1[w]), y2 = unpack_bf2(x2[w]);
-          x1[w] = rot_pair(y1, co[w], y2, ns[w]);
-          x2[w] = rot_pair(y2, co[w], y1, si[w]);
+          const float4 f = cs2[w];
+          x1[w] = rot_pair(y1, f.x, f.z, y2, -f.y, -f.w);
+          x2[w] = rot_pair(y2, f.x, f.z, y1, f.y, f.w);
           if ((i & 1) == 0) {
             x1[w] = pack_bf2(mul2(unpack_bf2(x1[w]), scale2));
             x2[w] = pack_bf2(mul2(unpack_bf2(x2[w]), scale2));
