@@ -293,18 +293,25 @@ __device__ __forceinline__ void wt_store_bf16(const WtParams& p, const WtTile& c
     else wt_store_words<EPI, false>(p, c, tokens);
     return;
   }
+  // odd strides or bases: element by element, the residuals on their way like the accumulators (read where they are added, 2048 x 4608 x
+  // 3584 on pairs took 115 us and 576 x 3840 x 1280 31; so 51 and 13)
   const int n = c.n0 + (c.tid >> 5 & 3) * 32 + (c.tid & 31);
   const bool store = n < p.N && !(p.flags & 4u);
-  wt_groups(c, tokens, [](int, uint32_t (&)[8]) {}, [&](int cc, uint32_t (&a)[8], uint32_t (&)[8]) {
-    const int nv = store ? tokens - cc : 0;
+  wt_groups(c, tokens, [&](int cc, uint32_t (&r)[8]) {
+    const int nv = store && res ? tokens - cc : 0;
+    const bf16* s = p.residual + (long)(c.t0 + cc) * p.ldr + n;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint32_t v = wt_act_bf16<EPI>(a[j], a[j], c.bias);
-      if (j >= nv) continue;
-      const long t = c.t0 + cc + j;
-      float x = __uint_as_float(v << 16);
-      if (res) x = rbf(bf2f(p.residual[t * p.ldr + n]) + x);
-      p.C[t * p.ldc + n] = f2bf(x);
+    for (int j = 0; j < 8; ++j, s += p.ldr) r[j] = j < nv ? *reinterpret_cast<const unsigned short*>(s) : 0u;
+  }, [&](int cc, uint32_t (&a)[8], uint32_t (&r)[8]) {
+    const int nv = store ? tokens - cc : 0;
+    bf16* d = p.C + (long)(c.t0 + cc) * p.ldc + n;
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      uint32_t v = wt_act_bf16<EPI>(a[j], a[j + 1], c.bias);
+      if (res) v = pack_bf2(add2(unpack_bf2(r[j] | (r[j + 1] << 16)), unpack_bf2(v)));
+#pragma unroll
+      for (int e = 0; e < 2; ++e, d += p.ldc)
+        if (j + e < nv) *reinterpret_cast<unsigned short*>(d) = (unsigned short)(v >> (16 * e));
     }
   });
 }

@@ -311,10 +311,10 @@ def test_split_outputs_of_an_odd_number_of_rows(tmp_path, ks, tn):
 
 @pytest.mark.parametrize("T,N,K,cfg,flag", [(1, 65, 64, (16, 1, 3, 1), 0), (65, 77, 72, (96, 2, 2, 1), 0), (300, 263, 192, (128, 1, 3, 1), 0),
                                             (300, 257, 192, (160, 1, 4, 1), PAIR), (577, 1031, 128, (224, 1, 4, 1), WIDE)])
-@pytest.mark.parametrize("epi", [0, 1, 2])
-def test_rows_of_an_odd_number_of_features(lib, T, N, K, cfg, flag, epi):
-    """even row strides: two features to a word, the last ones alone; with and without a residual, in place, and nothing behind the last
-    feature is written or taken"""
+@pytest.mark.parametrize("epi,even", [(0, True), (1, True), (2, True), (0, False), (1, False), (2, False)])
+def test_rows_of_an_odd_number_of_features(lib, T, N, K, cfg, flag, epi, even):
+    """even row strides: two features to a word, the last one alone; odd ones: feature by feature; with and without a residual, in place,
+    and nothing behind the last feature is written or taken"""
     import ctypes
     from mlx_vlm_b200 import _native as Nn
     x, w, b = _rand(T, K, seed=31), _rand(N, K, seed=32, std=K ** -0.5), _rand(N, seed=33)
@@ -323,7 +323,7 @@ def test_rows_of_an_odd_number_of_features(lib, T, N, K, cfg, flag, epi):
         y = y * torch.sigmoid((1.703125 * y).to(torch.bfloat16).double()).to(torch.bfloat16).double()
     if epi == 2:
         y = torch.nn.functional.gelu(y)
-    ld = N + 1 + T % 2 * 2
+    ld = N + 1 + T % 2 * 2 if even else N + T % 2 * 2
     for res in (None, _rand(T, ld, seed=34)):
         out = torch.full((T, ld), 9.0, dtype=torch.bfloat16, device="cuda")
         if res is not None:
